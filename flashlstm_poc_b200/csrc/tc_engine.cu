@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "engine.h"
 #include "kernels.h"
+#include "tc_cluster.cuh"
 #include "tc_common.cuh"
 #include "tc_kernels.h"
 
@@ -40,10 +41,17 @@ struct TcState {
     BwdPlan bwd{};
     bool bwd_ok = false;
     StepPlan step{};
+    ClusterFwdPlan cfwd{};
+    ClusterBwdPlan cbwd{};
     float *dh_parts = nullptr;  // wide-batch path: fp32 (L, splits, B, H) partial sums of dG_t W_hh
     std::vector<TcLayer> layers;
     unsigned int *err_host = nullptr;  // pinned mirror of the device error word
 };
+
+// Estimated cycles per step above which the grid-wide schedules are faster.  Measured crossings: H = 640 at 64 sequences
+// in both directions; beyond 64 sequences the grid-wide forward takes a fifth longer itself (512 x 128 still wins).
+constexpr int grid_fwd_cycles(int B) { return B <= 64 ? 5600 : 6500; }
+constexpr int kGridBwdCycles = 6500;
 
 TcState *state(Engine &e) { return static_cast<TcState *>(e.tc_state); }
 
@@ -135,22 +143,28 @@ int init(Engine &e) {
     int optin = 0;
     FLSTM_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e.device));
     st->smem_limit = (size_t)optin;
-    FLSTM_TRY(plan_step((int)e.cfg.batch, (int)e.cfg.hidden_size, st->sms, st->smem_limit, &st->step));
     void *raw = nullptr;
-    if (st->step.use) {
-        st->bwd_ok = e.cfg.training != 0;
+    const int B = (int)e.cfg.batch, H = (int)e.cfg.hidden_size;
+    // Each direction takes the cluster-resident kernel while its estimated step is shorter than the grid-wide ones'.
+    // FLSTM_STEP_MIN_BATCH asks for one of the grid-wide schedules by name.
+    if (!std::getenv("FLSTM_STEP_MIN_BATCH")) {
+        FLSTM_TRY(plan_cluster_fwd(B, H, st->sms, st->smem_limit, &st->cfwd, true));
+        if (st->cfwd.cycles > grid_fwd_cycles(B)) st->cfwd.use = false;
         if (e.cfg.training) {
-            const size_t n = e.layers.size() * (size_t)st->step.splits * e.cfg.batch * e.cfg.hidden_size;
-            FLSTM_CUDA_TRY(cudaMalloc(&raw, n * sizeof(float)));
-            st->dh_parts = static_cast<float *>(raw);
-        }
-    } else {
-        FLSTM_TRY(plan_fwd((int)e.cfg.batch, (int)e.cfg.hidden_size, st->sms, st->smem_limit, &st->fwd));
-        if (e.cfg.training) {
-            FLSTM_TRY(plan_bwd((int)e.cfg.batch, (int)e.cfg.hidden_size, st->sms, st->smem_limit, &st->bwd));
-            st->bwd_ok = true;
+            FLSTM_TRY(plan_cluster_bwd(B, H, st->sms, st->smem_limit, &st->cbwd, true));
+            if (st->cbwd.cycles > kGridBwdCycles) st->cbwd.use = false;
         }
     }
+    const bool grid_fwd = !st->cfwd.use, grid_bwd = e.cfg.training && !st->cbwd.use;
+    st->bwd_ok = e.cfg.training != 0;
+    if (grid_fwd || grid_bwd) FLSTM_TRY(plan_step(B, H, st->sms, st->smem_limit, &st->step));
+    if (st->step.use && grid_bwd) {
+        const size_t n = e.layers.size() * (size_t)st->step.splits * e.cfg.batch * e.cfg.hidden_size;
+        FLSTM_CUDA_TRY(cudaMalloc(&raw, n * sizeof(float)));
+        st->dh_parts = static_cast<float *>(raw);
+    }
+    if (!st->step.use && grid_fwd) FLSTM_TRY(plan_fwd(B, H, st->sms, st->smem_limit, &st->fwd));
+    if (!st->step.use && grid_bwd) FLSTM_TRY(plan_bwd(B, H, st->sms, st->smem_limit, &st->bwd));
     st->layers.resize(e.layers.size());
     FLSTM_CUDA_TRY(cudaMalloc(&raw, 1024 * sizeof(unsigned int)));
     e.sync_words = static_cast<unsigned int *>(raw);
@@ -180,6 +194,8 @@ int on_capacity_change(Engine &e) {
     for (size_t li = 0; li < e.layers.size(); ++li) {
         auto &l = e.layers[li];
         auto &t = st->layers[li];
+        const bool grid_fwd = !st->cfwd.use, grid_bwd = e.cfg.training && l.dg && !st->cbwd.use;
+        if (!grid_fwd && !grid_bwd) continue;  // the cluster kernels use plain loads
         FLSTM_TRY(make_tensor_map_2d(&t.tm_w, l.w_hh, 4 * H, H, H, 64, 64, true));
         if (st->step.use) {
             FLSTM_TRY(make_tensor_map_3d(&t.tm_hs3, l.hs, cap + 1, B, H, H, B * H, 128, 64, true));
@@ -187,13 +203,15 @@ int on_capacity_change(Engine &e) {
             FLSTM_TRY(make_tensor_map_3d_tile(&t.tm_g_ep, l.gates, 2, cap, B, 4 * H, 32, 64));
             FLSTM_TRY(make_tensor_map_3d_tile(&t.tm_c_ep, l.cs, 4, cap + 1, B, H, 32, 16));
             FLSTM_TRY(make_tensor_map_3d_tile(&t.tm_h_ep, l.hs, 2, cap + 1, B, H, 32, 16));
-            if (e.cfg.training && l.dg)
+            if (grid_bwd)
                 FLSTM_TRY(make_tensor_map_3d(&t.tm_dg3, l.dg, dg_steps, B, 4 * H, 4 * H, B * 4 * H, 128, 64, true));
             continue;
         }
-        FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->fwd.pair ? st->fwd.BT / 2 : st->fwd.BT, st->fwd.ch));
-        FLSTM_TRY(make_tensor_map_3d(&t.tm_g, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwd.BT, 64, false));
-        if (e.cfg.training && l.dg)
+        if (grid_fwd) {
+            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->fwd.pair ? st->fwd.BT / 2 : st->fwd.BT, st->fwd.ch));
+            FLSTM_TRY(make_tensor_map_3d(&t.tm_g, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwd.BT, 64, false));
+        }
+        if (grid_bwd)
             FLSTM_TRY(make_tensor_map_chunked(&t.tm_dg, l.dg, dg_steps, B, 4 * H, st->bwd.BT, st->bwd.ch));
     }
     return FLSTM_OK;
@@ -236,6 +254,31 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     FLSTM_TRY(gemm(e.cfg.dtype, e.cfg.dtype, n * B, 4 * H, l.in_size, byte_ptr(x_l) + t0 * B * l.in_size * es, l.in_size, false,
                    l.w_ih, l.in_size, false, byte_ptr(l.gates) + t0 * B * 4 * H * es, 4 * H, l.bias, 0, err, st->sms, s));
     size_t m1 = e.timer.mark(s);
+    if (st->cfwd.use) {
+        ClusterFwdParams cp{};
+        cp.w_hh = l.w_hh;
+        cp.cs = l.cs;
+        cp.hs = l.hs;
+        cp.y = y_out;
+        cp.gates = l.gates;
+        cp.err = err;
+        cp.T = (int)n;
+        cp.t0 = (int)t0;
+        cp.B = (int)B;
+        cp.H = (int)H;
+        cp.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
+        cp.trace = (li == 0 && t0 == 0) ? e.trace : nullptr;
+        cp.trace_steps = e.trace_steps;
+        cp.wait_ns = e.wait_limit_ns;
+        cp.extra_arrivals = e.selftest_missing_arrivals;
+        FLSTM_TRY(lstm_forward_cluster(e.cfg.dtype, st->cfwd, cp, s));
+        size_t m2 = e.timer.mark(s);
+        e.timer.span(PH_PROJ, m0, m1);
+        e.timer.span(PH_RECUR_FWD, m1, m2);
+        e.launches += 2;
+        FLSTM_CUDA_TRY(cudaMemcpyAsync(st->err_host, err, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+        return FLSTM_OK;
+    }
     if (st->step.use) {
         CUtensorMap tm_y;
         if (y_out) FLSTM_TRY(make_tensor_map_3d_tile(&tm_y, y_out, 2, t1, B, H, 32, 16));
@@ -368,8 +411,33 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     // with activation checkpoints `T` and the range are segment-local; only the segment that starts the sequence
     // finishes the recurrence (dh0 / dc0) and the layer's gradients
     const bool finalize = t0 == 0 && (!e.seg.active || e.seg.final_segment);
-    if (st->step.use) FLSTM_TRY(backward_steps(e, li, T, t0, t1, dy_l, dhn_l, dcn_l, dh0_l, dc0_l, finalize, s));
-    else {
+    if (st->cbwd.use) {
+        ClusterBwdParams cp{};
+        cp.w_hh = l.w_hh;
+        cp.cs = l.cs;
+        cp.gates = l.gates;
+        cp.dg = l.dg;
+        cp.dy = dy_l;
+        cp.dhn = dhn_l;
+        cp.dcn = dcn_l;
+        cp.dh0 = dh0_l;
+        cp.dc0 = dc0_l;
+        cp.dc = e.dc_layers + (size_t)li * B * H;
+        cp.err = err;
+        cp.T = (int)T;
+        cp.s0 = (int)(T - t1);
+        cp.s1 = (int)(T - t0) + (finalize ? 1 : 0);
+        cp.B = (int)B;
+        cp.H = (int)H;
+        cp.trace = (li == 0 && e.trace && t1 == T) ? e.trace + (size_t)e.trace_steps * 16 : nullptr;
+        cp.trace_steps = e.trace_steps;
+        cp.wait_ns = e.wait_limit_ns;
+        cp.extra_arrivals = e.selftest_missing_arrivals;
+        FLSTM_TRY(lstm_backward_cluster(e.cfg.dtype, st->cbwd, cp, s));
+        e.launches += 1;
+    } else if (st->step.use) {
+        FLSTM_TRY(backward_steps(e, li, T, t0, t1, dy_l, dhn_l, dcn_l, dh0_l, dc0_l, finalize, s));
+    } else {
     FLSTM_CUDA_TRY(cudaMemsetAsync(e.sync_words + 1, 0, (size_t)st->bwd.ngroups * sizeof(unsigned int), s));
     BwdParams p{};
     p.cs = l.cs;

@@ -44,6 +44,8 @@ struct TcState {
     ClusterFwdPlan cfwd{};
     ClusterBwdPlan cbwd{};
     float *dh_parts = nullptr;  // wide-batch path: fp32 (L, splits, B, H) partial sums of dG_t W_hh
+    float *dw_parts = nullptr;  // split-K partial products of the weight-gradient GEMMs
+    size_t dw_floats = 0, dw_layers = 1;
     std::vector<TcLayer> layers;
     unsigned int *err_host = nullptr;  // pinned mirror of the device error word
 };
@@ -165,6 +167,13 @@ int init(Engine &e) {
     }
     if (!st->step.use && grid_fwd) FLSTM_TRY(plan_fwd(B, H, st->sms, st->smem_limit, &st->fwd));
     if (!st->step.use && grid_bwd) FLSTM_TRY(plan_bwd(B, H, st->sms, st->smem_limit, &st->bwd));
+    if (e.cfg.training) {  // a split GEMM has at most one 128 x 128 tile per SM
+        st->dw_floats = (size_t)st->sms * 128 * 128;
+        // one per layer where the cross-layer wavefront can run two layers' GEMMs at once
+        st->dw_layers = st->step.use ? e.layers.size() : 1;
+        FLSTM_CUDA_TRY(cudaMalloc(&raw, st->dw_layers * st->dw_floats * sizeof(float)));
+        st->dw_parts = static_cast<float *>(raw);
+    }
     st->layers.resize(e.layers.size());
     FLSTM_CUDA_TRY(cudaMalloc(&raw, 1024 * sizeof(unsigned int)));
     e.sync_words = static_cast<unsigned int *>(raw);
@@ -183,6 +192,7 @@ void destroy(Engine &e) {
     if (!st) return;
     if (st->err_host) cudaFreeHost(st->err_host);
     if (st->dh_parts) cudaFree(st->dh_parts);
+    if (st->dw_parts) cudaFree(st->dw_parts);
     delete st;
     e.tc_state = nullptr;
 }
@@ -483,6 +493,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
         const size_t steps = e.seg.active ? n : T;
         const bool acc = e.seg.active && !e.seg.first_segment, last = !e.seg.active || e.seg.final_segment;
         const size_t n_ih = 4 * H * l.in_size;
+        float *parts = st->dw_parts + (st->dw_layers > 1 ? (size_t)li * st->dw_floats : 0);
         // Opt-in (FLSTM_DW_SIDE_BY_SIDE=1, without a communicator): the two GEMMs run SIDE BY SIDE, each on its share of
         // the SMs.  Their 128 x 256 tiles run for milliseconds (K = T*B), so a last, partly filled round of tiles is
         // expensive -- config 3: 512 tiles each, 4 + 4 rounds on 148 SMs one after the other, 7 rounds on 74 + 74 SMs.
@@ -511,10 +522,10 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
             FLSTM_CUDA_TRY(cudaStreamWaitEvent(s, e.aux_join, 0));
         } else {
             FLSTM_TRY(gemm(e.cfg.dtype, FLSTM_DTYPE_F32, 4 * H, l.in_size, steps * B, l.dg, 4 * H, true, x_l, l.in_size, true,
-                           l.dw_ih, l.in_size, nullptr, (int)H, err, st->sms, s, acc));
+                           l.dw_ih, l.in_size, nullptr, (int)H, err, st->sms, s, acc, parts, st->dw_floats));
             if (last) FLSTM_TRY(e.reduce_grads(l.grad_offset, n_ih, s));
             FLSTM_TRY(gemm(e.cfg.dtype, FLSTM_DTYPE_F32, 4 * H, H, steps * B, l.dg, 4 * H, true, l.hs, H, true, l.dw_hh, H,
-                           nullptr, (int)H, err, st->sms, s, acc));
+                           nullptr, (int)H, err, st->sms, s, acc, parts, st->dw_floats));
         }
         FLSTM_TRY(simt::column_sum_two_pass(e.cfg.dtype, l.dg, steps * B, 4 * H,
                                             e.db_part + (size_t)li * simt::column_sum_scratch_floats(4 * H), l.db, (int)H, s,

@@ -9,7 +9,7 @@
 //                          next tile's main loop through the second accumulator
 // The grid is persistent (one CTA per SM, static round-robin over output tiles).
 //
-// Two tile shapes.  gemm_kernel: one CTA per 128 x BN tile (BN 128 / 256).  gemm_pair_kernel: a cluster of two
+// Two tile shapes.  gemm_kernel: one CTA per 128 x BN tile (BN 64 / 128 / 256).  gemm_pair_kernel: a cluster of two
 // CTAs per 256 x 256 tile (tcgen05 cta_group::2): each CTA stages 128 rows of A and 128 rows of B per K block
 // (32 KB instead of the 48 KB a lone CTA needs for 128 x 256) and the pair's UMMA reads both halves of B, so the
 // shared-memory traffic per FLOP -- what bounds the one-CTA kernel at about 2/3 of the tensor peak -- drops by a
@@ -25,6 +25,7 @@
 // These replace the reference's CUTLASS mma.sync instantiations (src/lstm_internal.h:48-68,
 // flashlstm_v2/src/gemm.cu:208-359) and its per-32-step chunked dW/dX GEMMs with beta=1
 // (flashlstm_v2/src/lstm_backward.cu:1112-1171).
+#include <algorithm>
 #include <cstdlib>
 
 #include <cuda_bf16.h>
@@ -44,7 +45,7 @@ constexpr int kGemmThreads = 192;
 
 template <int BN>
 struct GemmShape {
-    static constexpr int kStages = (BN == 256) ? 4 : 6;
+    static constexpr int kStages = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
     static constexpr int kABytes = BM * BK * 2;
     static constexpr int kBBytes = BN * BK * 2;
     static constexpr int kStageBytes = kABytes + kBBytes;
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
             const __grid_constant__ CUtensorMap tm_d, void *__restrict__ D,
             size_t ldd, const float *__restrict__ bias, int M, int N, int K, uint32_t idesc, int unperm_h,
-            unsigned int *__restrict__ err_word, int accumulate) {
+            unsigned int *__restrict__ err_word, int accumulate, int splits) {
     using S = GemmShape<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -196,16 +197,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     const uint32_t tmem_base = *tmem_slot;
 
     const int num_m = (M + BM - 1) / BM, num_n = (N + BN - 1) / BN;
-    const int tiles = num_m * num_n, kblocks = (K + BK - 1) / BK;
+    // split K: work item = (tile, split); split z contracts over its share of the K blocks and writes an M x N partial
+    // product of its own behind D (fp32 output only)
+    const int items = num_m * num_n * splits, kblocks = (K + BK - 1) / BK, kper = (kblocks + splits - 1) / splits;
 
     if (warp == 0) {
         if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
-            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            for (int item = blockIdx.x; item < items; item += gridDim.x) {
+                const int tile = item / splits, kb0 = item % splits * kper, kb1 = kb0 + kper < kblocks ? kb0 + kper : kblocks;
                 const int m0 = (tile / num_n) * BM, n0 = (tile % num_n) * BN;
                 bool ok = true;
-                for (int kb = 0; kb < kblocks && ok; ++kb) {
+                for (int kb = kb0; kb < kb1 && ok; ++kb) {
                     ok = mbar_wait(&empty[stage], phase ^ 1, abort_w);
                     if (!ok) break;
                     uint8_t *sa = smem + stage * S::kStageBytes, *sb = sa + S::kABytes;
@@ -232,14 +236,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             int stage = 0;
             uint32_t phase = 0;
             int it = 0;
-            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+            for (int item = blockIdx.x; item < items; item += gridDim.x, ++it) {
+                const int kb0 = item % splits * kper, kb1 = kb0 + kper < kblocks ? kb0 + kper : kblocks;
                 const int buf = it & 1;
                 const uint32_t bphase = (it >> 1) & 1;
                 if (!mbar_wait(&tempty[buf], bphase ^ 1, abort_w)) break;
                 tcgen05_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 bool ok = true;
-                for (int kb = 0; kb < kblocks; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     ok = mbar_wait(&full[stage], phase, abort_w);
                     if (!ok) break;
                     tcgen05_fence_after();
@@ -250,7 +255,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                                                  : umma_desc_kmajor_sw128(a_base + k * 32);
                         const uint64_t db = B_MN ? umma_desc_mnmajor_sw128(b_base + k * 2048, 8192)
                                                  : umma_desc_kmajor_sw128(b_base + k * 32);
-                        umma_f16(d_tmem, da, db, idesc, (kb | k) != 0);
+                        umma_f16(d_tmem, da, db, idesc, kb != kb0 || k != 0);
                     }
                     umma_commit(&empty[stage]);
                     if (++stage == S::kStages) { stage = 0; phase ^= 1; }
@@ -262,7 +267,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     } else {
         const int q = warp & 3;  // TMEM lane quadrant this warp may access
         int it = 0, out_idx = 0;
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+        for (int item = blockIdx.x; item < items; item += gridDim.x, ++it) {
+            const int tile = item / splits;
             const int buf = it & 1;
             const uint32_t bphase = (it >> 1) & 1;
             const int m0 = (tile / num_n) * BM, n0 = (tile % num_n) * BN;
@@ -300,7 +306,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             }
             const size_t esz = (MODE == OUT_F32) ? 4 : 2;
             const int out_row = (unperm_h && row < M) ? unpermute_gate_row(row, unperm_h) : row;
-            char *dst_row = static_cast<char *>(D) + (size_t)out_row * ldd * esz;
+            char *dst_row = static_cast<char *>(D) + ((size_t)(item % splits) * M + out_row) * ldd * esz;
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
                 uint32_t acc[32];
@@ -320,6 +326,34 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, S::kTmemCols);
     if (threadIdx.x == 0 && *abort_w) atomicExch(err_word, 1u);
+}
+
+// D (rows in torch gate order when unperm_h) = or += the sum of the split-K partial products, in a fixed order.
+__global__ void __launch_bounds__(256) sum_splits_kernel(const float *__restrict__ parts, int splits, int M, int N,
+                                                         float *__restrict__ D, size_t ldd, int unperm_h, int accumulate) {
+    const size_t plane = (size_t)M * N;
+    const int lane = threadIdx.x & 31;
+    const bool vec = N % 4 == 0 && ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0;
+    for (int r = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); r < M; r += (int)(gridDim.x * (blockDim.x >> 5))) {
+        const float *src = parts + (size_t)r * N;
+        float *dst = D + (size_t)(unperm_h ? unpermute_gate_row(r, unperm_h) : r) * ldd;
+        if (vec) {
+            for (int c = lane * 4; c < N; c += 128) {
+                float4 v = accumulate ? *reinterpret_cast<const float4 *>(dst + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int z = 0; z < splits; ++z) {
+                    const float4 p = *reinterpret_cast<const float4 *>(src + z * plane + c);
+                    v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+                }
+                *reinterpret_cast<float4 *>(dst + c) = v;
+            }
+        } else {
+            for (int c = lane; c < N; c += 32) {
+                float v = accumulate ? dst[c] : 0.f;
+                for (int z = 0; z < splits; ++z) v += src[z * plane + c];
+                dst[c] = v;
+            }
+        }
+    }
 }
 
 // ------------------------------------------------------------------ CTA-pair kernel (256 x 256 tiles)
@@ -532,6 +566,8 @@ struct GemmArgs {
     unsigned int *err;
     int sms;
     int accumulate;
+    int splits;    // K splits; the partial products then go to `parts`
+    float *parts;
     cudaStream_t s;
     bool pair;  // 256 x 256 tiles on CTA pairs (gemm_pair_kernel)
 };
@@ -552,10 +588,15 @@ int launch_one(const GemmArgs &g) {
     using S = GemmShape<BN>;
     auto kern = gemm_kernel<BN, MODE, HAS_BIAS, A_MN, B_MN, TMA_OUT>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)S::kSmemBytes));
-    const int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
+    const int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) * g.splits;
     const int grid = tiles < g.sms ? tiles : g.sms;
-    kern<<<grid, kGemmThreads, S::kSmemBytes, g.s>>>(g.ta, g.tb, g.td, g.D, g.ldd, g.bias, g.M, g.N, g.K, g.idesc,
-                                                    g.unperm_h, g.err, g.accumulate);
+    const bool split = g.splits > 1;
+    kern<<<grid, kGemmThreads, S::kSmemBytes, g.s>>>(g.ta, g.tb, g.td, split ? g.parts : g.D, split ? (size_t)g.N : g.ldd, g.bias, g.M,
+                                                    g.N, g.K, g.idesc, split ? 0 : g.unperm_h, g.err, split ? 0 : g.accumulate,
+                                                    g.splits);
+    if (split)
+        sum_splits_kernel<<<(g.M + 7) / 8, 256, 0, g.s>>>(g.parts, g.splits, g.M, g.N, static_cast<float *>(g.D), g.ldd, g.unperm_h,
+                                                         g.accumulate);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "tc gemm launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
@@ -633,7 +674,7 @@ int dispatch(int out_dtype, bool a_mn, bool b_mn, const GemmArgs &g) {
 
 int gemm(int dtype, int out_dtype, size_t M, size_t N, size_t K, const void *A, size_t lda, bool a_mn, const void *B,
          size_t ldb, bool b_mn, void *D, size_t ldd, const float *bias, int unperm_h, unsigned int *err_word, int sms,
-         cudaStream_t s, bool accumulate) {
+         cudaStream_t s, bool accumulate, float *scratch, size_t scratch_floats) {
     if (accumulate && out_dtype != FLSTM_DTYPE_F32)
         return set_error(FLSTM_ERR_UNSUPPORTED, "accumulating GEMM output must be fp32");
     if (dtype != FLSTM_DTYPE_F16 && dtype != FLSTM_DTYPE_BF16)
@@ -641,7 +682,21 @@ int gemm(int dtype, int out_dtype, size_t M, size_t N, size_t K, const void *A, 
     if (M == 0 || N == 0 || K == 0) return FLSTM_OK;
     if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
         return set_error(FLSTM_ERR_UNSUPPORTED, "tensor-core GEMM needs 16-byte aligned operands and row pitches");
-    const int BN = (N > 128) ? 256 : 128;
+    // Tile width: the widest whose tiles still give most SMs one; a CTA takes in about 60 bytes per cycle, so a grid of few
+    // wide tiles runs at the rate of few SMs (weight gradient 2048 x 512 x 5550 on 32 tiles of 128 x 256: 41 us).
+    // Contractions that are long enough are split along K instead while that keeps the SMs busy (fp32 output and a
+    // scratch buffer; at least 8 K blocks per split).
+    const size_t rows = (M + BM - 1) / BM, enough = (size_t)sms * 3 / 4, kblocks = (K + BK - 1) / BK;
+    int BN = (N > 128) ? 256 : 128, splits = 1;
+    while (BN > 64 && rows * ((N + BN - 1) / BN) < enough) {
+        const size_t tiles = rows * ((N + BN - 1) / BN), most = std::min<size_t>(std::min<size_t>(sms / tiles, kblocks / 8), 16);
+        if (BN == 128 && out_dtype == FLSTM_DTYPE_F32 && scratch && most >= 2 && most * M * N <= scratch_floats) {
+            const size_t per = (kblocks + most - 1) / most;
+            splits = (int)((kblocks + per - 1) / per);
+            break;
+        }
+        BN /= 2;
+    }
     GemmArgs g{};
     // measured on B200 (bf16) inside the engine's step: pairs win for K-major A from K = 2048 on (config 3:
     // projection 1465 -> 1529, input gradient 1507 -> 1540 TFLOP/s; 8192^3 1159 -> 1377).  With K = 1024 and the
@@ -650,6 +705,12 @@ int gemm(int dtype, int out_dtype, size_t M, size_t N, size_t K, const void *A, 
     // neutral in isolation (1158 -> 1205) and 2 % slower inside the step, so both stay on lone CTAs.
     g.pair = pair_enabled() && !a_mn && K >= 2048 && M >= 256 && N % 256 == 0 && sms >= 2;
     if (pair_forced()) g.pair = M >= 256 && N % 256 == 0 && sms >= 2;
+    // ... and only with enough tiles for the pairs
+    if (g.pair && !pair_forced() && (M + 2 * BM - 1) / (2 * BM) * (N / 256) < (size_t)sms / 4) g.pair = false;
+    if (g.pair) {
+        BN = 256;
+        splits = 1;
+    }
     // K-major: (rows, K) with K contiguous, box rows x 64.  MN-major: stored (K, rows), 64 x 64 boxes.
     if (!a_mn) FLSTM_TRY(make_tensor_map_2d(&g.ta, A, M, K, lda, BM, BK, true));
     else FLSTM_TRY(make_tensor_map_2d(&g.ta, A, K, M, lda, BK, 64, true));
@@ -672,8 +733,12 @@ int gemm(int dtype, int out_dtype, size_t M, size_t N, size_t K, const void *A, 
     g.err = err_word;
     g.sms = sms;
     g.accumulate = accumulate ? 1 : 0;
+    g.splits = splits;
+    g.parts = scratch;
     g.s = s;
-    return BN == 256 ? dispatch<256>(out_dtype, a_mn, b_mn, g) : dispatch<128>(out_dtype, a_mn, b_mn, g);
+    return BN == 256 ? dispatch<256>(out_dtype, a_mn, b_mn, g)
+           : BN == 128 ? dispatch<128>(out_dtype, a_mn, b_mn, g)
+                       : dispatch<64>(out_dtype, a_mn, b_mn, g);
 }
 
 // ------------------------------------------------------------------ tensor-map encoding (host)

@@ -219,28 +219,58 @@ int Engine::ensure_capacity(size_t T) {
     return allocate(T);
 }
 
-int Engine::set_weights(int layer, const float *w_ih, const float *w_hh, const float *b_ih, const float *b_hh,
-                        cudaStream_t s) {
-    if (layer < 0 || layer >= (int)layers.size()) return set_error(FLSTM_ERR_INVALID, "layer %d out of range", layer);
-    if (!w_ih || !w_hh || !b_ih || !b_hh) return set_error(FLSTM_ERR_INVALID, "null parameter pointer");
-    auto &l = layers[layer];
+int Engine::set_weights(int first, int count, const float *const *params, cudaStream_t s) {
+    if (first < 0 || count < 1 || first + count > (int)layers.size())
+        return set_error(FLSTM_ERR_INVALID, "layer %d out of range", count == 1 ? first : first + count - 1);
+    for (int i = 0; i < 4 * count; ++i)
+        if (!params[i]) return set_error(FLSTM_ERR_INVALID, "null parameter pointer");
     const size_t H = cfg.hidden_size;
     if (backend == FLSTM_BACKEND_TC) {
-        FLSTM_TRY(tc::set_weights(*this, layer, w_ih, w_hh, b_ih, b_hh, s));
-        launches += 5;
+        FLSTM_TRY(tc::set_weights(*this, first, count, params, s));
     } else {
-        FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, w_ih, cfg.dtype, l.w_ih, 4 * H * l.in_size, s));
-        FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, w_hh, cfg.dtype, l.w_hh, 4 * H * H, s));
-        FLSTM_TRY(simt::bias_sum(b_ih, b_hh, l.bias, 4 * H, s));
-        launches += 3;
+        for (int i = 0; i < count; ++i) {
+            auto &l = layers[first + i];
+            FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, params[4 * i], cfg.dtype, l.w_ih, 4 * H * l.in_size, s));
+            FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, params[4 * i + 1], cfg.dtype, l.w_hh, 4 * H * H, s));
+            FLSTM_TRY(simt::bias_sum(params[4 * i + 2], params[4 * i + 3], l.bias, 4 * H, s));
+            launches += 3;
+        }
     }
-    l.weights_set = true;
+    for (int i = 0; i < count; ++i) layers[first + i].weights_set = true;
     return FLSTM_OK;
 }
 
 int Engine::forward(size_t T, const void *x, const void *h0, const void *c0, void *y, void *hn, void *cn,
                     cudaStream_t s) {
     return forward_range(T, 0, T, x, h0, c0, y, hn, cn, s);
+}
+
+// The states that enter a sequence, into slot 0 of every layer's state tensors (layers [first, last)).
+static void add_states_in(Engine &e, CopyBatch &batch, int first, int last, const void *h0, const void *c0) {
+    const size_t B = e.cfg.batch, H = e.cfg.hidden_size, es = dtype_size(e.cfg.dtype);
+    const size_t ces = e.cell_io_f32 ? sizeof(float) : es;
+    const int c_dtype = e.cell_io_f32 ? (int)FLSTM_DTYPE_F32 : e.cfg.dtype;
+    for (int li = first; li < last; ++li) {
+        auto &l = e.layers[li];
+        batch.dense(h0 ? byte_ptr(h0) + li * B * H * es : nullptr, e.cfg.dtype, l.hs, e.cfg.dtype, B, H);
+        batch.dense(c0 ? byte_ptr(c0) + li * B * H * ces : nullptr, c_dtype, l.cs, FLSTM_DTYPE_F32, B, H);
+    }
+}
+
+// The states in slot `slot` of one layer to the caller's h_n / c_n (either may be null).
+static void add_states_out(Engine &e, CopyBatch &batch, int li, size_t slot, void *hn, void *cn) {
+    const size_t B = e.cfg.batch, H = e.cfg.hidden_size, slab = B * H, es = dtype_size(e.cfg.dtype);
+    const size_t ces = e.cell_io_f32 ? sizeof(float) : es;
+    const int c_dtype = e.cell_io_f32 ? (int)FLSTM_DTYPE_F32 : e.cfg.dtype;
+    auto &l = e.layers[li];
+    if (hn) batch.dense(byte_ptr(l.hs) + slot * slab * es, e.cfg.dtype, byte_ptr(hn) + li * slab * es, e.cfg.dtype, B, H);
+    if (cn) batch.dense(l.cs + slot * slab, FLSTM_DTYPE_F32, byte_ptr(cn) + li * slab * ces, c_dtype, B, H);
+}
+
+// The device error word to its host mirror, with the last copies of a call.
+static void add_error_mirror(Engine &e, CopyBatch &batch) {
+    batch.err = e.sync_words;  // null on the per-step CUDA-core path, which has no waits
+    batch.err_host = e.backend == FLSTM_BACKEND_TC ? tc::error_mirror(e) : e.simt_err_host;
 }
 
 // Steps [t0, t1) of a T-step forward.  Ranges must be issued in ascending order starting at 0; x and
@@ -270,16 +300,10 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
     } else if (fwd_progress != t0) {
         return set_error(FLSTM_ERR_INVALID, "forward ranges must be contiguous and ascending (expected start %zu, got %zu)", fwd_progress, t0);
     }
+    CopyBatch batch;
     if (t0 == 0) {
-        // initial state -> slot 0 of the state tensors
-        for (int li = 0; li < L; ++li) {
-            auto &l = layers[li];
-            if (h0) FLSTM_CUDA_TRY(cudaMemcpyAsync(l.hs, byte_ptr(h0) + li * slab * es, slab * es, cudaMemcpyDeviceToDevice, s));
-            else FLSTM_CUDA_TRY(cudaMemsetAsync(l.hs, 0, slab * es, s));
-            const size_t ces = cell_io_f32 ? sizeof(float) : es;
-            if (c0) { FLSTM_TRY(simt::convert(cell_io_f32 ? FLSTM_DTYPE_F32 : cfg.dtype, byte_ptr(c0) + li * slab * ces, FLSTM_DTYPE_F32, l.cs, slab, s)); ++launches; }
-            else FLSTM_CUDA_TRY(cudaMemsetAsync(l.cs, 0, slab * sizeof(float), s));
-        }
+        add_states_in(*this, batch, 0, L, h0, c0);
+        FLSTM_TRY(batch.run(s, &launches));
     }
     const size_t wave = backend == FLSTM_BACKEND_TC ? tc::wavefront_chunk(*this, t1 - t0) : 0;
     if (wave) {
@@ -321,8 +345,6 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
                 size_t m1 = timer.mark(s);
                 if (simt_grid) {
                     FLSTM_TRY(simt_check_error());
-                    const size_t tiles = (size_t)simt::persistent_batch_tiles(B);
-                    FLSTM_CUDA_TRY(cudaMemsetAsync(sync_words + 32, 0, tiles * sizeof(unsigned int), s));
                     simt::PersistentFwdParams pp{};
                     pp.w_hh = l.w_hh;
                     pp.hs = l.hs;
@@ -330,6 +352,7 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
                     pp.gates = l.gates;
                     pp.y = y_out;
                     pp.counters = sync_words + 32;
+                    pp.exits = sync_words + 1;
                     pp.err = sync_words;
                     pp.B = (int)B;
                     pp.H = (int)H;
@@ -339,7 +362,6 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
                     pp.wait_ns = wait_limit_ns;
                     pp.extra_arrivals = selftest_missing_arrivals;
                     FLSTM_TRY(simt::persistent_forward(cfg.dtype, simt_grid, pp, s));
-                    FLSTM_CUDA_TRY(cudaMemcpyAsync(simt_err_host, sync_words, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
                     ++launches;
                 } else {
                     for (size_t t = t0; t < t1; ++t) {
@@ -356,14 +378,10 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
             }
         }
     }
-    if (t1 == T) {
-        const size_t ces = cell_io_f32 ? sizeof(float) : es;
-        for (int li = 0; li < L; ++li) {
-            auto &l = layers[li];
-            if (hn) FLSTM_CUDA_TRY(cudaMemcpyAsync(byte_ptr(hn) + li * slab * es, byte_ptr(l.hs) + T * slab * es, slab * es, cudaMemcpyDeviceToDevice, s));
-            if (cn) { FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, l.cs + T * slab, cell_io_f32 ? FLSTM_DTYPE_F32 : cfg.dtype, byte_ptr(cn) + li * slab * ces, slab, s)); ++launches; }
-        }
-    }
+    if (t1 == T)
+        for (int li = 0; li < L; ++li) add_states_out(*this, batch, li, T, hn, cn);
+    add_error_mirror(*this, batch);
+    FLSTM_TRY(batch.run(s, &launches));
     fwd_progress = t1;
     if (t1 == T) {
         last_T = T;
@@ -384,37 +402,40 @@ int Engine::forward_checkpointed(size_t T, const void *x, const void *h0, const 
     timer.reset();
     x_saved = x;
     last_T = 0;
-    const size_t R = buf_steps, ces = cell_io_f32 ? sizeof(float) : es;
+    const size_t R = buf_steps;
+    CopyBatch batch;
     struct Restore { Engine &e; ~Restore() { e.seg = SegmentMode{}; } } restore{*this};  // also on early error returns
     seg.keep_gates = false;
     int st = FLSTM_OK;
     for (int li = 0; li < L && st == FLSTM_OK; ++li) {
         auto &l = layers[li];
-        if (h0) FLSTM_CUDA_TRY(cudaMemcpyAsync(l.hs, byte_ptr(h0) + li * slab * es, slab * es, cudaMemcpyDeviceToDevice, s));
-        else FLSTM_CUDA_TRY(cudaMemsetAsync(l.hs, 0, slab * es, s));
-        if (c0) { FLSTM_TRY(simt::convert(cell_io_f32 ? FLSTM_DTYPE_F32 : cfg.dtype, byte_ptr(c0) + li * slab * ces, FLSTM_DTYPE_F32, l.cs, slab, s)); ++launches; }
-        else FLSTM_CUDA_TRY(cudaMemsetAsync(l.cs, 0, slab * sizeof(float), s));
+        add_states_in(*this, batch, li, li + 1, h0, c0);
+        FLSTM_TRY(batch.run(s, &launches));
         const void *x_l = li == 0 ? x : layers[li - 1].y_all;
         void *y_l = (li == L - 1) ? y : l.y_all;
         size_t k = 0;
         for (size_t seg0 = 0; seg0 < T && st == FLSTM_OK; seg0 += R, ++k) {
             const size_t n = T - seg0 < R ? T - seg0 : R;
             // checkpoint k: the state entering the segment (slot 0)
-            FLSTM_CUDA_TRY(cudaMemcpyAsync(byte_ptr(l.ck_h) + k * slab * es, l.hs, slab * es, cudaMemcpyDeviceToDevice, s));
-            FLSTM_CUDA_TRY(cudaMemcpyAsync(l.ck_c + k * slab, l.cs, slab * sizeof(float), cudaMemcpyDeviceToDevice, s));
+            batch.dense(l.hs, cfg.dtype, byte_ptr(l.ck_h) + k * slab * es, cfg.dtype, B, H);
+            batch.dense(l.cs, FLSTM_DTYPE_F32, l.ck_c + k * slab, FLSTM_DTYPE_F32, B, H);
+            FLSTM_TRY(batch.run(s, &launches));
             st = tc::forward_layer(*this, li, 0, n, byte_ptr(x_l) + seg0 * B * l.in_size * es,
                                    y_l ? byte_ptr(y_l) + seg0 * slab * es : nullptr, s);
             if (st != FLSTM_OK) break;
             // the state leaving the segment enters the next one
-            FLSTM_CUDA_TRY(cudaMemcpyAsync(l.hs, byte_ptr(l.hs) + n * slab * es, slab * es, cudaMemcpyDeviceToDevice, s));
-            FLSTM_CUDA_TRY(cudaMemcpyAsync(l.cs, l.cs + n * slab, slab * sizeof(float), cudaMemcpyDeviceToDevice, s));
+            batch.dense(byte_ptr(l.hs) + n * slab * es, cfg.dtype, l.hs, cfg.dtype, B, H);
+            batch.dense(l.cs + n * slab, FLSTM_DTYPE_F32, l.cs, FLSTM_DTYPE_F32, B, H);
+            FLSTM_TRY(batch.run(s, &launches));
         }
         if (st != FLSTM_OK) break;
-        if (hn) FLSTM_CUDA_TRY(cudaMemcpyAsync(byte_ptr(hn) + li * slab * es, l.hs, slab * es, cudaMemcpyDeviceToDevice, s));
-        if (cn) { FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, l.cs, cell_io_f32 ? FLSTM_DTYPE_F32 : cfg.dtype, byte_ptr(cn) + li * slab * ces, slab, s)); ++launches; }
+        add_states_out(*this, batch, li, 0, hn, cn);
+        FLSTM_TRY(batch.run(s, &launches));
     }
     seg.keep_gates = true;
     FLSTM_TRY(st);
+    add_error_mirror(*this, batch);
+    FLSTM_TRY(batch.run(s, &launches));
     fwd_progress = T;
     last_T = T;
     bwd_progress = T;
@@ -440,8 +461,10 @@ int Engine::backward_checkpointed(size_t T, const void *dy, const void *dhn, con
         const size_t T_loc = (kk == K - 1) ? n : n + 1;  // slot n of dG then holds the step after the segment
         for (int li = L - 1; li >= 0 && st == FLSTM_OK; --li) {
             auto &l = layers[li];
-            FLSTM_CUDA_TRY(cudaMemcpyAsync(l.hs, byte_ptr(l.ck_h) + kk * slab * es, slab * es, cudaMemcpyDeviceToDevice, s));
-            FLSTM_CUDA_TRY(cudaMemcpyAsync(l.cs, l.ck_c + kk * slab, slab * sizeof(float), cudaMemcpyDeviceToDevice, s));
+            CopyBatch restore_state;
+            restore_state.dense(byte_ptr(l.ck_h) + kk * slab * es, cfg.dtype, l.hs, cfg.dtype, B, H);
+            restore_state.dense(l.ck_c + kk * slab, FLSTM_DTYPE_F32, l.cs, FLSTM_DTYPE_F32, B, H);
+            FLSTM_TRY(restore_state.run(s, &launches));
             const void *x_seg = li == 0 ? byte_ptr(x_saved) + seg0 * B * l.in_size * es
                                         : byte_ptr(layers[li - 1].y_all) + seg0 * slab * es;
             st = tc::forward_layer(*this, li, 0, n, x_seg, nullptr, s);  // recompute
@@ -458,6 +481,9 @@ int Engine::backward_checkpointed(size_t T, const void *dy, const void *dhn, con
     }
     seg = SegmentMode{};
     FLSTM_TRY(st);
+    CopyBatch batch;
+    add_error_mirror(*this, batch);
+    FLSTM_TRY(batch.run(s, &launches));
     if (comm) {
         FLSTM_CUDA_TRY(cudaEventRecord(comm_join, comm_stream));
         FLSTM_CUDA_TRY(cudaStreamWaitEvent(s, comm_join, 0));
@@ -521,6 +547,9 @@ int Engine::backward_segment(size_t n, bool last_in_time, bool first_in_time, co
             FLSTM_CUDA_TRY(cudaMemcpyAsync(byte_ptr(l.dg) + buf_steps * B * 4 * H * es, l.dg, B * 4 * H * es,
                                            cudaMemcpyDeviceToDevice, s));
     }
+    CopyBatch batch;
+    add_error_mirror(*this, batch);
+    FLSTM_TRY(batch.run(s, &launches));
     if (comm && first_in_time) {
         FLSTM_CUDA_TRY(cudaEventRecord(comm_join, comm_stream));
         FLSTM_CUDA_TRY(cudaStreamWaitEvent(s, comm_join, 0));
@@ -586,6 +615,9 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
             }
             c1s = c0s;
         }
+        CopyBatch batch;
+        add_error_mirror(*this, batch);
+        FLSTM_TRY(batch.run(s, &launches));
         if (comm && t0 == 0) {
             FLSTM_CUDA_TRY(cudaEventRecord(comm_join, comm_stream));
             FLSTM_CUDA_TRY(cudaStreamWaitEvent(s, comm_join, 0));
@@ -613,8 +645,6 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
             }
             if (simt_grid) {
                 FLSTM_TRY(simt_check_error());
-                const size_t tiles = (size_t)simt::persistent_batch_tiles(B);
-                FLSTM_CUDA_TRY(cudaMemsetAsync(sync_words + 32, 0, tiles * sizeof(unsigned int), s));
                 simt::PersistentBwdParams pp{};
                 pp.w_hh = l.w_hh;
                 pp.cs = l.cs;
@@ -626,6 +656,7 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
                 pp.dh0 = dh0_l;
                 pp.dc0 = dc0_l;
                 pp.counters = sync_words + 32;
+                pp.exits = sync_words + 1;
                 pp.err = sync_words;
                 pp.B = (int)B;
                 pp.H = (int)H;
@@ -635,7 +666,6 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
                 pp.wait_ns = wait_limit_ns;
                 pp.extra_arrivals = selftest_missing_arrivals;
                 FLSTM_TRY(simt::persistent_backward(cfg.dtype, simt_grid, pp, s));
-                FLSTM_CUDA_TRY(cudaMemcpyAsync(simt_err_host, sync_words, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
                 ++launches;
             } else {
                 for (size_t step = 0; step < n; ++step) {
@@ -678,6 +708,9 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
         // starts its reductions itself, block by block, as the weight-gradient kernels finish)
         if (t0 == 0 && backend != FLSTM_BACKEND_TC) FLSTM_TRY(reduce_grads(l.grad_offset, l.grad_count, s));
     }
+    CopyBatch batch;
+    add_error_mirror(*this, batch);
+    FLSTM_TRY(batch.run(s, &launches));
     if (comm && t0 == 0) {
         FLSTM_CUDA_TRY(cudaEventRecord(comm_join, comm_stream));
         FLSTM_CUDA_TRY(cudaStreamWaitEvent(s, comm_join, 0));
@@ -847,7 +880,14 @@ int flstm_engine_set_weights(flstm_engine *engine, int layer, const float *w_ih,
                              const float *b_ih, const float *b_hh, void *stream) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
     DeviceScope scope(engine->impl.device);
-    return engine->impl.set_weights(layer, w_ih, w_hh, b_ih, b_hh, static_cast<cudaStream_t>(stream));
+    const float *params[4] = {w_ih, w_hh, b_ih, b_hh};
+    return engine->impl.set_weights(layer, 1, params, static_cast<cudaStream_t>(stream));
+}
+
+int flstm_engine_set_all_weights(flstm_engine *engine, const float *const *params, void *stream) {
+    if (!engine || !params) return set_error(FLSTM_ERR_INVALID, "null argument");
+    DeviceScope scope(engine->impl.device);
+    return engine->impl.set_weights(0, engine->impl.cfg.layers, params, static_cast<cudaStream_t>(stream));
 }
 
 int flstm_engine_forward(flstm_engine *engine, size_t seq_len, const void *x, const void *h0, const void *c0,
@@ -895,6 +935,27 @@ int flstm_engine_grad_ptrs(flstm_engine *engine, int layer, float **dw_ih, float
     if (dw_hh) *dw_hh = l.dw_hh;
     if (db) *db = l.db;
     return FLSTM_OK;
+}
+
+int flstm_engine_export_grads(flstm_engine *engine, float *const *grads, const float *dh0, const float *dc0, void *dh0_out,
+                              void *dc0_out, void *stream) {
+    if (!engine || !grads) return set_error(FLSTM_ERR_INVALID, "null argument");
+    Engine &e = engine->impl;
+    DeviceScope scope(e.device);
+    const size_t H = e.cfg.hidden_size, rows = e.cfg.layers * e.cfg.batch;
+    flstm_b200::CopyBatch batch;
+    for (size_t li = 0; li < e.layers.size(); ++li, grads += 4) {
+        auto &l = e.layers[li];
+        for (int i = 0; i < 4; ++i)
+            if (!grads[i]) return set_error(FLSTM_ERR_INVALID, "null gradient pointer");
+        batch.dense(l.dw_ih, FLSTM_DTYPE_F32, grads[0], FLSTM_DTYPE_F32, 4 * H, l.in_size);
+        batch.dense(l.dw_hh, FLSTM_DTYPE_F32, grads[1], FLSTM_DTYPE_F32, 4 * H, H);
+        batch.dense(l.db, FLSTM_DTYPE_F32, grads[2], FLSTM_DTYPE_F32, 1, 4 * H);
+        batch.dense(l.db, FLSTM_DTYPE_F32, grads[3], FLSTM_DTYPE_F32, 1, 4 * H);
+    }
+    if (dh0 && dh0_out) batch.dense(dh0, FLSTM_DTYPE_F32, dh0_out, e.cfg.dtype, rows, H);
+    if (dc0 && dc0_out) batch.dense(dc0, FLSTM_DTYPE_F32, dc0_out, e.cfg.dtype, rows, H);
+    return batch.run(static_cast<cudaStream_t>(stream), &e.launches);
 }
 
 int flstm_engine_grad_buffer(flstm_engine *engine, float **flat, size_t *count) {

@@ -51,6 +51,28 @@ struct LayerBuffers {
     bool weights_set = false;
 };
 
+// Copies of small strided matrices (states in and out of the engine's buffers, padding, the error word), collected and
+// run as one launch: with one memcpy / memset / conversion per state and layer a call of a small model spent more time
+// on its launches than on its recurrence.
+struct CopyJob {
+    const void *src;  // null: zeros
+    void *dst;
+    size_t rows, src_pitch, dst_pitch;  // pitches in elements
+    int src_cols, dst_cols;             // columns [src_cols, dst_cols) of the destination become zero
+    int src_dtype, dst_dtype;
+};
+struct CopyBatch {
+    std::vector<CopyJob> jobs;
+    const unsigned int *err = nullptr;  // device error word, mirrored to err_host by the next launch when non-zero
+    unsigned int *err_host = nullptr;
+    void add(const void *src, int src_dtype, size_t src_pitch, int src_cols, void *dst, int dst_dtype, size_t dst_pitch,
+             int dst_cols, size_t rows);
+    void dense(const void *src, int src_dtype, void *dst, int dst_dtype, size_t rows, size_t cols) {
+        add(src, src_dtype, cols, (int)cols, dst, dst_dtype, cols, (int)cols, rows);
+    }
+    int run(cudaStream_t s, unsigned long long *launches);
+};
+
 struct Engine {
     flstm_engine_config cfg{};
     int backend = FLSTM_BACKEND_SIMT;
@@ -119,8 +141,8 @@ struct Engine {
     int allocate(size_t t_cap);
     void release_time_buffers();
     int ensure_capacity(size_t T);
-    int set_weights(int layer, const float *w_ih, const float *w_hh, const float *b_ih, const float *b_hh,
-                    cudaStream_t s);
+    // parameters of layers [first, first + count): w_ih, w_hh, b_ih, b_hh of each
+    int set_weights(int first, int count, const float *const *params, cudaStream_t s);
     int forward(size_t T, const void *x, const void *h0, const void *c0, void *y, void *hn, void *cn,
                 cudaStream_t s);
     int backward(size_t T, const void *dy, const void *dhn, const void *dcn, void *dx, float *dh0,
@@ -155,8 +177,8 @@ int init(Engine &e);
 void destroy(Engine &e);
 int on_capacity_change(Engine &e);
 int poll_error(Engine &e);  // reports (and clears) a device-side wait that expired in an earlier launch
-int set_weights(Engine &e, int layer, const float *w_ih, const float *w_hh, const float *b_ih,
-                const float *b_hh, cudaStream_t s);
+int set_weights(Engine &e, int first, int count, const float *const *params, cudaStream_t s);
+unsigned int *error_mirror(Engine &e);
 int forward_layer(Engine &e, int layer, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s);
 // `dx_ready` (optional) is recorded on `s` once dx_l of the range is complete, before the weight gradients
 int backward_layer(Engine &e, int layer, size_t T, size_t t0, size_t t1, const void *x_l, const void *dy_l,

@@ -49,7 +49,8 @@ struct PersistentFwdParams {
     float *cs;               // (T+1, B, H) fp32
     void *gates;             // (T, B, 4H): projection in, activated gates out (when store_gates)
     void *y;                 // optional (T, B, H) copy of h_t
-    unsigned int *counters;  // one per batch tile of 8 sequences, zeroed before the launch
+    unsigned int *counters;  // one per batch tile of 8 sequences, zero between launches
+    unsigned int *exits;     // CTAs that have left, zero between launches
     unsigned int *err;       // error word (a bounded wait expired)
     int B, H;
     int t0, T;               // first step and number of steps of this launch
@@ -66,7 +67,7 @@ struct PersistentBwdParams {
     const void *dhn;         // (B, H) or null: added at the last time step
     float *dc;               // (B, H) fp32 cell-gradient carry: read at launch start, written at its end
     float *dh0, *dc0;        // (B, H) fp32 or null, written by the iteration s == T
-    unsigned int *counters, *err;
+    unsigned int *counters, *exits, *err;
     int B, H;
     int T;                   // length of the whole sequence
     int s0, s1;              // reverse iterations [s0, s1): iteration s is time T-1-s

@@ -100,6 +100,7 @@ persistent_forward_kernel(PersistentFwdParams p) {
         if (tid == 0) red_release_gpu_add(counter, 1u);
     }
     if (tid == 0 && abort_w) atomicCAS(p.err, 0u, 1u);
+    if (tid == 0) tc::leave_counters(p.counters, (int)gridDim.x / unit_tiles, p.exits);
 }
 
 template <typename T>
@@ -182,6 +183,7 @@ persistent_backward_kernel(PersistentBwdParams p) {
     }
     if (owner) p.dc[idx] = dc_keep;  // a later launch continues the recurrence from here
     if (tid == 0 && abort_w) atomicCAS(p.err, 0u, 1u);
+    if (tid == 0) tc::leave_counters(p.counters, (int)gridDim.x / unit_tiles, p.exits);
 }
 
 template <typename Kern>

@@ -55,35 +55,44 @@ struct TcState {
 constexpr int grid_fwd_cycles(int B) { return B <= 64 ? 5600 : 6500; }
 constexpr int kGridBwdCycles = 6500;
 
+constexpr int kExitsWord = 1000;  // of Engine::sync_words: CTAs of the running launch that have left (see leave_counters)
+
 TcState *state(Engine &e) { return static_cast<TcState *>(e.tc_state); }
 
-__device__ __forceinline__ int interleaved_to_torch_row(int r, int H) {
-    const int tile = r >> 6, g = (r >> 4) & 3, u = r & 15;
-    return g * H + tile * 16 + u;
-}
+struct PackJobs {
+    PackJob job[kPackJobs];
+};
 
+// A warp packs one output row: 16-byte stores of 8 columns per lane, 32-byte loads where the source row allows them.
+// One launch for both matrices of up to 8 layers: three launches per layer with one element per thread took 14 us per
+// 4096 x 1024 matrix and more than the whole recurrence of a small model.
 template <typename T>
-__global__ void pack_rows_kernel(const float *__restrict__ w, int H, int K, T *__restrict__ out) {
-    const size_t total = (size_t)4 * H * K;
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (; i < total; i += stride) {
-        const int r = (int)(i / K), k = (int)(i % K);
-        st(out + i, w[(size_t)interleaved_to_torch_row(r, H) * K + k]);
+__global__ void __launch_bounds__(256) pack_weights_kernel(const __grid_constant__ PackJobs jobs) {
+    const PackJob &j = jobs.job[blockIdx.y];
+    const int lane = threadIdx.x & 31, rows = 4 * j.Hp;
+    const bool vec = j.K % 4 == 0 && (reinterpret_cast<uintptr_t>(j.w) & 15) == 0;
+    for (int r = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); r < rows; r += (int)(gridDim.x * (blockDim.x >> 5))) {
+        const int u = (r >> 6) * 16 + (r & 15), row = ((r >> 4) & 3) * j.H + u;
+        const bool real = u < j.H;
+        const float *src = j.w + (size_t)row * j.K;
+        T *dst = static_cast<T *>(j.out) + (size_t)r * j.Kp;
+        for (int k = lane * 8; k < j.Kp; k += 256) {
+            float v[8];
+            if (real && vec && k + 8 <= j.K) {
+                const float4 a = *reinterpret_cast<const float4 *>(src + k), b = *reinterpret_cast<const float4 *>(src + k + 4);
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+                v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = real && k + e < j.K ? src[k + e] : 0.f;
+            }
+            __align__(16) T o[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) st(o + e, v[e]);
+            *reinterpret_cast<uint4 *>(dst + k) = *reinterpret_cast<const uint4 *>(o);
+        }
+        if (lane == 0 && j.bias) j.bias[r] = real ? j.b_ih[row] + j.b_hh[row] : 0.f;
     }
-}
-
-__global__ void pack_bias_kernel(const float *__restrict__ a, const float *__restrict__ b, int H, float *__restrict__ out) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < 4 * H) {
-        const int o = interleaved_to_torch_row(r, H);
-        out[r] = a[o] + b[o];
-    }
-}
-
-__global__ void unpermute_kernel(const float *__restrict__ in, int H, float *__restrict__ out) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < 4 * H) out[interleaved_to_torch_row(r, H)] = in[r];
 }
 
 int check_launch(const char *what) {
@@ -97,23 +106,21 @@ inline const char *byte_ptr(const void *p) { return static_cast<const char *>(p)
 
 }  // namespace
 
-int pack_weights_interleaved(int dtype, const float *w, size_t H, size_t K, void *out, cudaStream_t s) {
-    const size_t total = 4 * H * K;
-    int grid = (int)((total + 255) / 256);
-    if (grid > 148 * 16) grid = 148 * 16;
-    if (dtype == FLSTM_DTYPE_F16) pack_rows_kernel<<<grid, 256, 0, s>>>(w, (int)H, (int)K, static_cast<__half *>(out));
-    else pack_rows_kernel<<<grid, 256, 0, s>>>(w, (int)H, (int)K, static_cast<__nv_bfloat16 *>(out));
-    return check_launch("pack_weights");
-}
-
-int pack_bias_interleaved(const float *b_ih, const float *b_hh, size_t H, float *out, cudaStream_t s) {
-    pack_bias_kernel<<<(int)((4 * H + 255) / 256), 256, 0, s>>>(b_ih, b_hh, (int)H, out);
-    return check_launch("pack_bias");
-}
-
-int unpermute_vector(const float *in, size_t H, float *out, cudaStream_t s) {
-    unpermute_kernel<<<(int)((4 * H + 255) / 256), 256, 0, s>>>(in, (int)H, out);
-    return check_launch("unpermute");
+int pack_weights(int dtype, const PackJob *jobs, int count, cudaStream_t s) {
+    for (int first = 0; first < count; first += kPackJobs) {
+        PackJobs args{};
+        const int n = count - first < kPackJobs ? count - first : kPackJobs;
+        int rows = 0;
+        for (int i = 0; i < n; ++i) {
+            args.job[i] = jobs[first + i];
+            if (4 * jobs[first + i].Hp > rows) rows = 4 * jobs[first + i].Hp;
+        }
+        const dim3 grid((rows + 7) / 8 < 1184 ? (rows + 7) / 8 : 1184, n);
+        if (dtype == FLSTM_DTYPE_F16) pack_weights_kernel<__half><<<grid, 256, 0, s>>>(args);
+        else pack_weights_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(args);
+        FLSTM_TRY(check_launch("pack_weights"));
+    }
+    return FLSTM_OK;
 }
 
 bool supported(const flstm_engine_config &cfg) {
@@ -227,18 +234,21 @@ int on_capacity_change(Engine &e) {
     return FLSTM_OK;
 }
 
-int set_weights(Engine &e, int layer, const float *w_ih, const float *w_hh, const float *b_ih, const float *b_hh,
-                cudaStream_t s) {
-    auto &l = e.layers[layer];
-    const size_t H = e.cfg.hidden_size;
-    FLSTM_TRY(pack_weights_interleaved(e.cfg.dtype, w_ih, H, l.in_size, l.w_ih, s));
-    FLSTM_TRY(pack_weights_interleaved(e.cfg.dtype, w_hh, H, H, l.w_hh, s));
-    FLSTM_TRY(pack_bias_interleaved(b_ih, b_hh, H, l.bias, s));
-    return FLSTM_OK;
+int set_weights(Engine &e, int first, int count, const float *const *params, cudaStream_t s) {
+    std::vector<PackJob> jobs;
+    const int H = (int)e.cfg.hidden_size;
+    for (int li = first; li < first + count; ++li, params += 4) {
+        auto &l = e.layers[li];
+        const int K = (int)l.in_size;
+        jobs.push_back({params[0], l.w_ih, params[2], params[3], l.bias, H, H, K, K});
+        jobs.push_back({params[1], l.w_hh, nullptr, nullptr, nullptr, H, H, H, H});
+    }
+    e.launches += (jobs.size() + kPackJobs - 1) / kPackJobs;
+    return pack_weights(e.cfg.dtype, jobs.data(), (int)jobs.size(), s);
 }
 
-// Deferred error reporting: the device error word is mirrored into pinned host memory after each
-// layer; a non-zero mirror fails the NEXT call (and flstm_engine_synchronize reports it at once).
+// Deferred error reporting: the device error word is mirrored into pinned host memory at the end of every call (by the
+// launch that copies the final states, see CopyBatch); a non-zero mirror fails the NEXT call.
 static int check_async_error(Engine &e) {
     TcState *st = state(e);
     if (st && *st->err_host) {
@@ -251,6 +261,8 @@ static int check_async_error(Engine &e) {
 }
 
 int poll_error(Engine &e) { return check_async_error(e); }
+
+unsigned int *error_mirror(Engine &e) { return state(e)->err_host; }
 
 int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s) {
     TcState *st = state(e);
@@ -286,7 +298,6 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         e.timer.span(PH_PROJ, m0, m1);
         e.timer.span(PH_RECUR_FWD, m1, m2);
         e.launches += 2;
-        FLSTM_CUDA_TRY(cudaMemcpyAsync(st->err_host, err, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         return FLSTM_OK;
     }
     if (st->step.use) {
@@ -297,10 +308,10 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         // cross-layer wavefront): two cooperative grids that each need most of the machine must not be in flight
         // at once, each could hold SMs the other is waiting for
         if (st->step.fwd_persistent && wavefront_chunk(e, (size_t)-1) == 0) {
-            FLSTM_CUDA_TRY(cudaMemsetAsync(e.sync_words + 1, 0, sizeof(unsigned int), s));
             WideFwdParams wp{};
             wp.err = err;
             wp.counter = e.sync_words + 1;
+            wp.exits = e.sync_words + kExitsWord;
             wp.t0 = (int)t0;
             wp.nsteps = (int)n;
             wp.B = (int)B;
@@ -313,7 +324,6 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
             e.timer.span(PH_PROJ, m0, m1);
             e.timer.span(PH_RECUR_FWD, m1, m2);
             e.launches += 2;
-            FLSTM_CUDA_TRY(cudaMemcpyAsync(st->err_host, err, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
             return FLSTM_OK;
         }
         for (size_t step = t0; step < t1; ++step) {
@@ -329,16 +339,15 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         e.timer.span(PH_PROJ, m0, m1);
         e.timer.span(PH_RECUR_FWD, m1, m2);
         e.launches += 1 + n;
-        FLSTM_CUDA_TRY(cudaMemcpyAsync(st->err_host, err, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         return FLSTM_OK;
     }
-    FLSTM_CUDA_TRY(cudaMemsetAsync(e.sync_words + 1, 0, (size_t)st->fwd.ngroups * sizeof(unsigned int), s));
     FwdParams p{};
     p.cs = l.cs;
     p.hs = l.hs;
     p.y = y_out;
     p.gates = l.gates;
     p.counters = e.sync_words + 1;
+    p.exits = e.sync_words + kExitsWord;
     p.err = err;
     p.T = (int)n;
     p.t0 = (int)t0;
@@ -354,7 +363,6 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     e.timer.span(PH_PROJ, m0, m1);
     e.timer.span(PH_RECUR_FWD, m1, m2);
     e.launches += 2;
-    FLSTM_CUDA_TRY(cudaMemcpyAsync(st->err_host, err, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     return FLSTM_OK;
 }
 
@@ -448,7 +456,6 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     } else if (st->step.use) {
         FLSTM_TRY(backward_steps(e, li, T, t0, t1, dy_l, dhn_l, dcn_l, dh0_l, dc0_l, finalize, s));
     } else {
-    FLSTM_CUDA_TRY(cudaMemsetAsync(e.sync_words + 1, 0, (size_t)st->bwd.ngroups * sizeof(unsigned int), s));
     BwdParams p{};
     p.cs = l.cs;
     p.gates = l.gates;
@@ -462,6 +469,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.trace = (li == 0 && e.trace && t1 == T) ? e.trace + (size_t)e.trace_steps * 16 : nullptr;
     p.trace_steps = e.trace_steps;
     p.counters = e.sync_words + 1;
+    p.exits = e.sync_words + kExitsWord;
     p.err = err;
     p.T = (int)T;
     p.s0 = (int)(T - t1);
@@ -554,7 +562,6 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
         e.timer.span(PH_XGRAD, m2, m3);
     }
     e.timer.span(PH_BPTT, m0, m1);
-    FLSTM_CUDA_TRY(cudaMemcpyAsync(st->err_host, err, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     return FLSTM_OK;
 }
 

@@ -42,7 +42,8 @@ struct FwdParams {
     void *hs;             // 16-bit (T+1, B, H) hidden states, slot 0 = h0
     void *y;              // optional 16-bit (T, B, H) copy of h_t for the caller
     void *gates;          // 16-bit (T, B, 4H): holds P on entry, the activated gates on exit
-    unsigned int *counters;  // one step counter per batch group, zeroed before the launch
+    unsigned int *counters;  // one step counter per batch group, zero between launches
+    unsigned int *exits;     // CTAs that have left, zero between launches (leave_counters)
     unsigned int *err;    // error word: non-zero after a bounded wait expired
     int T, B, H;          // T = number of steps this launch runs
     int t0;               // first (absolute) time step of this launch; the state of step t0 is in slot t0 of hs/cs
@@ -86,7 +87,7 @@ struct BwdParams {
     const void *dcn;      // 16-bit (B, H) or null
     float *dh0, *dc0;     // fp32 (B, H) or null
     float *dc;            // fp32 (B, H) scratch for the cell-gradient carry (used when nt > 1)
-    unsigned int *counters;
+    unsigned int *counters, *exits;  // as in FwdParams
     unsigned int *err;
     long long *trace;     // optional per-step clock64() stamps of CTA 0 (see FwdParams)
     int trace_steps;
@@ -138,7 +139,7 @@ struct StepFwdMaps {
 // a counter barrier in global memory separates the steps (same tensor maps as lstm_step_forward).
 struct WideFwdParams {
     unsigned int *err;
-    unsigned int *counter;  // zeroed before the launch
+    unsigned int *counter, *exits;  // zero between launches
     int t0, nsteps;
     int B, H;
     int store_gates;
@@ -160,10 +161,17 @@ int lstm_step_backward_pointwise(int dtype, const void *gates_t, const float *c_
 int sum_parts(const float *parts, int nparts, size_t n, float *out, cudaStream_t s);
 
 // fp32 (4H, K) torch-ordered rows -> 16-bit tile-interleaved rows; bias likewise (b_ih + b_hh)
-int pack_weights_interleaved(int dtype, const float *w, size_t H, size_t K, void *out, cudaStream_t s);
-int pack_bias_interleaved(const float *b_ih, const float *b_hh, size_t H, float *out, cudaStream_t s);
-// out[g*H + u] = in[tile-interleaved index of (g,u)]
-int unpermute_vector(const float *in, size_t H, float *out, cudaStream_t s);
+// One matrix of one layer from fp32 torch order (4H, K) to the 16-bit tile-interleaved order (4Hp, Kp), padding zero;
+// with b_ih / b_hh also the layer's summed bias (4Hp).  One launch packs up to kPackJobs of them.
+struct PackJob {
+    const float *w;
+    void *out;
+    const float *b_ih, *b_hh;
+    float *bias;
+    int H, Hp, K, Kp;
+};
+constexpr int kPackJobs = 16;
+int pack_weights(int dtype, const PackJob *jobs, int count, cudaStream_t s);
 
 }  // namespace tc
 }  // namespace flstm_b200

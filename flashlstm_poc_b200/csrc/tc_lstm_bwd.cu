@@ -459,6 +459,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     }
     if (warp == 5) tmem_dealloc(tmem_base, kTmemCols);
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
+    if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / (p.jt * KS), p.exits);
 }
 
 // ------------------------------------------------------------------ host side

@@ -511,7 +511,7 @@ struct WideFwdArgs {
     int t0, nsteps;    // first absolute time step and number of steps of this launch
     uint32_t idesc;
     unsigned int *err;
-    unsigned int *counter;        // step barrier, zeroed before the launch
+    unsigned int *counter, *exits;  // step barrier and CTAs that have left, zero between launches (leave_counters)
     int has_y, store_gates;
     unsigned long long wait_ns;   // limit of every wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path: arrivals nobody makes
@@ -804,6 +804,7 @@ wide_fwd_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         tmem_dealloc(tmem_base, S::kTmemCols);
     }
     if (threadIdx.x == 0 && *abort_w) atomicCAS(a.err, 0u, 1u);
+    if (threadIdx.x == 0) leave_counters(a.counter, 1, a.exits);
 }
 
 // Pointwise backward of one time step for 4 hidden units of one sequence per thread:
@@ -1059,6 +1060,7 @@ int lstm_wide_forward(int dtype, const StepPlan &plan, const StepFwdMaps &m, con
     a.idesc = umma_idesc_f16(plan.fwd_pair ? 2 * BM : BM, plan.bn_fwd, bf16 ? 1 : 0, 0, 0);
     a.err = p.err;
     a.counter = p.counter;
+    a.exits = p.exits;
     a.has_y = m.y ? 1 : 0;
     a.store_gates = p.store_gates;
     a.wait_ns = p.wait_ns;

@@ -71,6 +71,16 @@ __device__ __forceinline__ bool wait_counter(const unsigned int *ctr, unsigned i
     return true;
 }
 
+// End of a kernel whose CTAs met at step counters: the CTA that leaves last clears them for the next launch (one thread
+// of every CTA calls this once it makes no further waits or arrivals, after an abort too).  It replaces a memset node
+// in front of every launch.
+__device__ __forceinline__ void leave_counters(unsigned int *counters, int n, unsigned int *exits) {
+    __threadfence();
+    if (atomicAdd(exits, 1u) != gridDim.x - 1) return;
+    for (int i = 0; i < n; ++i) counters[i] = 0;
+    *exits = 0;
+}
+
 template <bool BF16>
 __device__ __forceinline__ float load16(const uint16_t *p) {
     if (BF16) return __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(p));

@@ -79,6 +79,18 @@ class Engine:
         check(self.lib.flstm_engine_set_weights(self._h, layer, w_ih.data_ptr(), w_hh.data_ptr(), b_ih.data_ptr(),
                                                 b_hh.data_ptr(), self._stream()))
 
+    def set_all_weights(self, params: Sequence[torch.Tensor]) -> None:
+        """set_weights for every layer at once: w_ih, w_hh, b_ih, b_hh of layer 0, then of layer 1, ..."""
+        H, checked = self.hidden_size, []
+        for i, p in enumerate(params):
+            I = self.input_size if i < 4 else H
+            shape = ((4 * H, I), (4 * H, H), (4 * H,), (4 * H,))[i % 4]
+            if p.dtype != torch.float32 or p.shape != shape or p.device != self.device or not p.is_contiguous():
+                p = self._check_tensor(p.detach(), shape, ("w_ih", "w_hh", "b_ih", "b_hh")[i % 4], torch.float32)
+            checked.append(p)
+        ptrs = (ctypes.c_void_p * (4 * self.layers))(*[p.data_ptr() for p in checked])
+        check(self.lib.flstm_engine_set_all_weights(self._h, ptrs, self._stream()))
+
     def forward(self, x: torch.Tensor, h0: Optional[torch.Tensor] = None, c0: Optional[torch.Tensor] = None,
                 want_states: bool = True):
         T = x.shape[0]
@@ -190,6 +202,21 @@ class Engine:
         I = self.input_size if layer == 0 else H
         return (self._wrap(a.value, (4 * H, I), torch.float32), self._wrap(b.value, (4 * H, H), torch.float32),
                 self._wrap(c.value, (4 * H,), torch.float32))
+
+    def export_grads(self, dh0: Optional[torch.Tensor] = None, dc0: Optional[torch.Tensor] = None):
+        """New tensors with the gradients of every layer (dW_ih, dW_hh, db_ih, db_hh of layer 0, then of layer 1, ...)
+        and, where given, dh0 / dc0 of the last backward converted to the engine dtype."""
+        H, out = self.hidden_size, []
+        for l in range(self.layers):
+            I = self.input_size if l == 0 else H
+            for shape in ((4 * H, I), (4 * H, H), (4 * H,), (4 * H,)):
+                out.append(torch.empty(shape, dtype=torch.float32, device=self.device))
+        dh0_out = None if dh0 is None else torch.empty(dh0.shape, dtype=self.torch_dtype, device=self.device)
+        dc0_out = None if dc0 is None else torch.empty(dc0.shape, dtype=self.torch_dtype, device=self.device)
+        ptrs = (ctypes.c_void_p * len(out))(*[t.data_ptr() for t in out])
+        check(self.lib.flstm_engine_export_grads(self._h, ptrs, _ptr(dh0), _ptr(dc0), _ptr(dh0_out), _ptr(dc0_out),
+                                                 self._stream()))
+        return out, dh0_out, dc0_out
 
     def grad_buffer(self) -> torch.Tensor:
         p, n = ctypes.c_void_p(), ctypes.c_size_t()

@@ -18,26 +18,21 @@ class _LSTMFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, module, x, h0, c0, *params):
         eng = module._engine_for(x)
-        for l in range(module.num_layers):
-            eng.set_weights(l, *params[4 * l:4 * l + 4])
+        eng.set_all_weights(params)
         y, hn, cn = eng.forward(x, h0, c0)
-        ctx.module, ctx.engine = module, eng
+        ctx.module, ctx.engine, ctx.y_shape = module, eng, y.shape
         ctx.has_h0, ctx.has_c0 = h0 is not None, c0 is not None
-        ctx.state_dtype = x.dtype
+        ctx.set_materialize_grads(False)  # absent gradients of y / h_n / c_n stay None
         return y, hn, cn
 
     @staticmethod
     def backward(ctx, dy, dhn, dcn):
         eng = ctx.engine
-        if dy is None:
-            raise RuntimeError("LSTM backward needs a gradient for y")
-        dx, dh0, dc0 = eng.backward(dy.contiguous(), dhn, dcn)
-        grads = []
-        for l in range(ctx.module.num_layers):
-            dw_ih, dw_hh, db = eng.grads(l)
-            grads += [dw_ih.clone(), dw_hh.clone(), db.clone(), db.clone()]
-        return (None, dx, dh0.to(ctx.state_dtype) if ctx.has_h0 else None,
-                dc0.to(ctx.state_dtype) if ctx.has_c0 else None, *grads)
+        if dy is None:  # only h_n / c_n were used
+            dy = torch.zeros(ctx.y_shape, dtype=eng.torch_dtype, device=eng.device)
+        dx, dh0, dc0 = eng.backward(dy.contiguous(), dhn, dcn, want_dstates=ctx.has_h0 or ctx.has_c0)
+        grads, dh0, dc0 = eng.export_grads(dh0 if ctx.has_h0 else None, dc0 if ctx.has_c0 else None)
+        return (None, dx, dh0, dc0, *grads)
 
 
 class LSTM(nn.Module):

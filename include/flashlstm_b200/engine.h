@@ -71,6 +71,9 @@ int flstm_engine_destroy(flstm_engine *engine);
 int flstm_engine_set_weights(flstm_engine *engine, int layer, const float *w_ih, const float *w_hh,
                              const float *b_ih, const float *b_hh, void *stream);
 
+/* The same for every layer at once: params[4 l + {0,1,2,3}] = w_ih, w_hh, b_ih, b_hh of layer l. */
+int flstm_engine_set_all_weights(flstm_engine *engine, const float *const *params, void *stream);
+
 /* y (T,B,H), h_n/c_n (L,B,H) may be NULL when not wanted; h0/c0 NULL = zeros.
  * Asynchronous on `stream`.  In training mode x must stay valid and unchanged until the
  * matching flstm_engine_backward has been enqueued (it is re-read for dW_ih). */
@@ -100,6 +103,11 @@ int flstm_engine_backward_range(flstm_engine *engine, size_t seq_len, size_t t0,
 /* Device pointers into the flat gradient buffer of one layer: dW_ih (4H,I_l), dW_hh (4H,H),
  * db (4H) (db_ih == db_hh == db, as in flashlstm_v2/src/lstm_backward.cu:1218-1231). */
 int flstm_engine_grad_ptrs(flstm_engine *engine, int layer, float **dw_ih, float **dw_hh, float **db);
+/* Copies of every layer's gradients in one launch: grads[4 l + {0,1,2,3}] receives dW_ih, dW_hh, db_ih, db_hh of layer
+ * l.  dh0 / dc0 (fp32 (L,B,H), as written by flstm_engine_backward) are converted to the engine dtype into dh0_out /
+ * dc0_out on the way; each pair may be NULL. */
+int flstm_engine_export_grads(flstm_engine *engine, float *const *grads, const float *dh0, const float *dc0, void *dh0_out,
+                              void *dc0_out, void *stream);
 /* The whole flat buffer, layer after layer as [dW_ih | dW_hh | db]. */
 int flstm_engine_grad_buffer(flstm_engine *engine, float **flat, size_t *count);
 

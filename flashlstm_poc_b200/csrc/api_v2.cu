@@ -173,7 +173,7 @@ struct V2Context {
         cfg.training = 1;
         cfg.backend = FLSTM_BACKEND_AUTO;
         FLSTM_TRY(flstm_engine_create(&cfg, &seg_engine));
-        if (flstm_engine_backend(seg_engine) != FLSTM_BACKEND_TC) {
+        if (flstm_engine_backend(seg_engine) != FLSTM_BACKEND_TC || seg_engine->impl.inner) {
             flstm_engine_destroy(seg_engine);
             seg_engine = nullptr;
             return set_error(FLSTM_ERR_UNSUPPORTED, "host streaming in segments needs the tensor-core backend (H %% 64 == 0, I %% 8 == 0)");

@@ -79,6 +79,20 @@ __device__ __forceinline__ float tanh_fast(float a) {
 }
 __device__ __forceinline__ float sigmoid_fast(float a) { return fmaf(0.5f, tanh_fast(0.5f * a), 0.5f); }
 
+// 16-bit shapes that the tensor-core path cannot tile ran in the CUDA-core kernels with expf / tanhf; padded onto the
+// tensor-core path (engine_padded.cu) their gate functions keep an error far below a 16-bit rounding step (about 1e-7
+// absolute), the ACCURATE form here.
+template <bool ACCURATE>
+__device__ __forceinline__ float sigmoid_sel(float a) {
+    return ACCURATE ? __fdividef(1.f, 1.f + __expf(-a)) : sigmoid_fast(a);
+}
+template <bool ACCURATE>
+__device__ __forceinline__ float tanh_sel(float a) {
+    if (!ACCURATE) return tanh_fast(a);
+    const float e = __expf(-2.f * fabsf(a));
+    return copysignf(__fdividef(1.f - e, 1.f + e), a);
+}
+
 inline int ceil_div(size_t a, size_t b) { return static_cast<int>((a + b - 1) / b); }
 
 // Opt-in dynamic shared memory above 48 KB.  cudaFuncSetAttribute acts on the CURRENT device only, so the

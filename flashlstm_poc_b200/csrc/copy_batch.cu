@@ -16,6 +16,13 @@ struct CopyArgs {
     unsigned int *err_host;
 };
 
+template <int BYTES>
+struct Piece;
+template <> struct Piece<16> { using type = uint4; };
+template <> struct Piece<8> { using type = uint2; };
+template <> struct Piece<4> { using type = uint32_t; };
+template <> struct Piece<2> { using type = uint16_t; };
+
 // V consecutive elements of a row, converted; columns from src_cols on (or all, without a source) are zero
 template <typename TI, typename TO, int V>
 __device__ __forceinline__ void copy_job(const CopyJob &j) {
@@ -28,35 +35,28 @@ __device__ __forceinline__ void copy_job(const CopyJob &j) {
         const int c = (int)(i - r * per_row) * V;
         const TI *from = src + r * j.src_pitch + c;
         TO *to = dst + r * j.dst_pitch + c;
+        using In = typename Piece<V * sizeof(TI)>::type;
+        using Out = typename Piece<V * sizeof(TO)>::type;
         __align__(16) TI in[V];
-        if (!src || c >= j.src_cols) {
-#pragma unroll
-            for (int e = 0; e < V; ++e) st(in + e, 0.f);
-        } else if (V > 1) {
-            if (sizeof(in) == 16) *reinterpret_cast<uint4 *>(in) = *reinterpret_cast<const uint4 *>(from);
-            else *reinterpret_cast<uint2 *>(in) = *reinterpret_cast<const uint2 *>(from);
-        } else {
-            in[0] = from[0];
-        }
+        if (!src || c >= j.src_cols) *reinterpret_cast<In *>(in) = In{};
+        else *reinterpret_cast<In *>(in) = *reinterpret_cast<const In *>(from);
         __align__(16) TO out[V];
 #pragma unroll
         for (int e = 0; e < V; ++e) st(out + e, ld(in + e));
-        if (V > 1) {
-            if (sizeof(out) == 16) *reinterpret_cast<uint4 *>(to) = *reinterpret_cast<const uint4 *>(out);
-            else *reinterpret_cast<uint2 *>(to) = *reinterpret_cast<const uint2 *>(out);
-        } else {
-            to[0] = out[0];
-        }
+        *reinterpret_cast<Out *>(to) = *reinterpret_cast<const Out *>(out);
     }
 }
 
 template <typename TI, typename TO>
 __device__ __forceinline__ void copy_any(const CopyJob &j) {
-    // four elements at a time where columns, pitches and addresses allow it
-    const bool four = ((j.src_cols | j.dst_cols) & 3) == 0 && ((j.src_pitch | j.dst_pitch) & 3) == 0 &&
-                      (reinterpret_cast<uintptr_t>(j.src) & (4 * sizeof(TI) - 1)) == 0 &&
-                      (reinterpret_cast<uintptr_t>(j.dst) & (4 * sizeof(TO) - 1)) == 0;
-    if (four) copy_job<TI, TO, 4>(j);
+    // four or two elements at a time where columns, pitches and addresses allow it
+    auto allows = [&](int v) {
+        return (((size_t)j.src_cols | (size_t)j.dst_cols | j.src_pitch | j.dst_pitch) & (v - 1)) == 0 &&
+               (reinterpret_cast<uintptr_t>(j.src) & (v * sizeof(TI) - 1)) == 0 &&
+               (reinterpret_cast<uintptr_t>(j.dst) & (v * sizeof(TO) - 1)) == 0;
+    };
+    if (allows(4)) copy_job<TI, TO, 4>(j);
+    else if (allows(2)) copy_job<TI, TO, 2>(j);
     else copy_job<TI, TO, 1>(j);
 }
 

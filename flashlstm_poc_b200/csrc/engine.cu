@@ -75,7 +75,62 @@ inline const char *byte_ptr(const void *p) { return static_cast<const char *>(p)
 
 }  // namespace
 
+// Workspace for cfg / backend on the current device.  An engine with an `inner` one owns the logical gradients only.
+int Engine::init() {
+    const size_t H = cfg.hidden_size, B = cfg.batch, es = dtype_size(cfg.dtype);
+    layers.resize(cfg.layers);
+    size_t total = 0;
+    for (int li = 0; li < cfg.layers; ++li) {
+        auto &l = layers[li];
+        l.in_size = li == 0 ? cfg.input_size : H;
+        l.grad_offset = total;
+        l.grad_count = 4 * H * l.in_size + 4 * H * H + 4 * H;
+        total += l.grad_count;
+    }
+    grad_count = total;
+    FLSTM_TRY(dev_alloc(&grads, total * sizeof(float)));
+    FLSTM_CUDA_TRY(cudaMemset(grads, 0, total * sizeof(float)));
+    for (auto &l : layers) {
+        l.dw_ih = grads + l.grad_offset;
+        l.dw_hh = l.dw_ih + 4 * H * l.in_size;
+        l.db = l.dw_hh + 4 * H * H;
+    }
+    if (inner) return FLSTM_OK;
+    FLSTM_TRY(dev_alloc(&dc_layers, (size_t)cfg.layers * B * H * sizeof(float)));
+    for (auto &l : layers) {
+        FLSTM_TRY(dev_alloc(&l.w_ih, 4 * H * l.in_size * es));
+        FLSTM_TRY(dev_alloc(&l.w_hh, 4 * H * H * es));
+        FLSTM_TRY(dev_alloc(&l.bias, 4 * H * sizeof(float)));
+    }
+    if (backend == FLSTM_BACKEND_TC) {
+        FLSTM_TRY(tc::init(*this));
+    } else {
+        if (cfg.training) {
+            // room for up to 8 partial products of the largest weight gradient, at most 64 MiB
+            const size_t widest = cfg.input_size > H ? cfg.input_size : H;
+            size_t floats = 8 * 4 * H * widest;
+            if (floats > (size_t)16 << 20) floats = (size_t)16 << 20;
+            if (dev_alloc(&simt_scratch, floats * sizeof(float)) == FLSTM_OK) simt_scratch_floats = floats;
+            else cudaGetLastError();  // the GEMMs then run unsplit
+        }
+        int grid = 0;
+        if (simt::persistent_fits(cfg.dtype, B, H, cfg.training != 0, &grid)) {
+            const size_t words = 32 + (size_t)simt::persistent_batch_tiles(B);
+            FLSTM_TRY(dev_alloc(&sync_words, words * sizeof(unsigned int)));
+            FLSTM_CUDA_TRY(cudaMemset(sync_words, 0, words * sizeof(unsigned int)));
+            void *raw = nullptr;
+            FLSTM_CUDA_TRY(cudaMallocHost(&raw, sizeof(unsigned int)));
+            simt_err_host = static_cast<unsigned int *>(raw);
+            *simt_err_host = 0;
+            simt_grid = grid;
+        }
+    }
+    return allocate(cfg.max_seq_len ? cfg.max_seq_len : 1);
+}
+
 Engine::~Engine() {
+    padded_release();
+    delete inner;
     tc::destroy(*this);
     release_time_buffers();
     for (auto &l : layers) {
@@ -199,8 +254,8 @@ int Engine::allocate(size_t cap) {
 }
 
 int Engine::set_recompute(size_t R) {
-    if (R && backend != FLSTM_BACKEND_TC)
-        return set_error(FLSTM_ERR_UNSUPPORTED, "activation checkpoints need the tensor-core backend (f16/bf16, H %% 64 == 0)");
+    if (R && (backend != FLSTM_BACKEND_TC || inner))
+        return set_error(FLSTM_ERR_UNSUPPORTED, "activation checkpoints need the tensor-core backend (f16/bf16, H %% 64 == 0, I %% 8 == 0)");
     if (R == recompute) return FLSTM_OK;
     FLSTM_CUDA_TRY(cudaDeviceSynchronize());
     const size_t cap = t_cap ? t_cap : 1;
@@ -225,7 +280,9 @@ int Engine::set_weights(int first, int count, const float *const *params, cudaSt
     for (int i = 0; i < 4 * count; ++i)
         if (!params[i]) return set_error(FLSTM_ERR_INVALID, "null parameter pointer");
     const size_t H = cfg.hidden_size;
-    if (backend == FLSTM_BACKEND_TC) {
+    if (inner) {
+        FLSTM_TRY(inner->set_weights(first, count, params, s));
+    } else if (backend == FLSTM_BACKEND_TC) {
         FLSTM_TRY(tc::set_weights(*this, first, count, params, s));
     } else {
         for (int i = 0; i < count; ++i) {
@@ -282,6 +339,7 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
     if (T == 0 || B == 0 || H == 0) return FLSTM_OK;  // zero-sized problem: silent no-op (lstm_forward.cu:493-495)
     if (!x) return set_error(FLSTM_ERR_INVALID, "x is null");
     if (t0 >= t1 || t1 > T) return set_error(FLSTM_ERR_INVALID, "bad step range [%zu, %zu) of %zu", t0, t1, T);
+    if (inner) return padded_forward_range(T, t0, t1, x, h0, c0, y, hn, cn, s);
     if (recompute) {
         if (t0 != 0 || t1 != T)
             return set_error(FLSTM_ERR_UNSUPPORTED, "step ranges are not available with activation checkpoints");
@@ -510,7 +568,7 @@ int Engine::backward_segment(size_t n, bool last_in_time, bool first_in_time, co
     const size_t B = cfg.batch, H = cfg.hidden_size, es = dtype_size(cfg.dtype), slab = B * H;
     const int L = (int)layers.size();
     if (!cfg.training) return set_error(FLSTM_ERR_INVALID, "engine was created with training = 0");
-    if (backend != FLSTM_BACKEND_TC || !recompute)
+    if (backend != FLSTM_BACKEND_TC || inner || !recompute)
         return set_error(FLSTM_ERR_UNSUPPORTED, "segment backward needs the tensor-core backend with a recompute interval set");
     if (n == 0 || n > buf_steps) return set_error(FLSTM_ERR_INVALID, "segment of %zu steps does not fit the %zu-step buffers", n, buf_steps);
     if (!x_seg || !dy_seg) return set_error(FLSTM_ERR_INVALID, "null pointer argument");
@@ -567,6 +625,7 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
     if (T == 0 || B == 0 || H == 0) return FLSTM_OK;
     if (!cfg.training) return set_error(FLSTM_ERR_INVALID, "engine was created with training = 0");
     if (comm_aborted) return set_error(FLSTM_ERR_COMM, "the communicator was aborted after a step missed its deadline; attach a new one");
+    if (inner) return padded_backward_range(T, t0, t1, dy, dhn, dcn, dx, dh0, dc0, s);
     if (last_T != T) return set_error(FLSTM_ERR_INVALID, "backward(T=%zu) does not follow a forward of the same length (last T=%zu)", T, last_T);
     if (!dy) return set_error(FLSTM_ERR_INVALID, "dy is null");
     if (t0 >= t1 || t1 > T) return set_error(FLSTM_ERR_INVALID, "bad step range [%zu, %zu) of %zu", t0, t1, T);
@@ -799,71 +858,13 @@ int flstm_engine_create(const flstm_engine_config *config, flstm_engine **out) {
                          "batch %% 8 == 0 on an sm_100 device");
     }
     e.backend = (config->backend == FLSTM_BACKEND_AUTO) ? (tc_ok ? FLSTM_BACKEND_TC : FLSTM_BACKEND_SIMT) : config->backend;
-    const size_t H = config->hidden_size, B = config->batch, es = flstm_b200::dtype_size(config->dtype);
-    e.layers.resize(config->layers);
-    size_t total = 0;
-    for (int li = 0; li < config->layers; ++li) {
-        auto &l = e.layers[li];
-        l.in_size = li == 0 ? config->input_size : H;
-        l.grad_offset = total;
-        l.grad_count = 4 * H * l.in_size + 4 * H * H + 4 * H;
-        total += l.grad_count;
-    }
-    e.grad_count = total;
     int st = FLSTM_OK;
-    auto fail = [&](int code) { delete h; return code; };
-    {
-        void *raw = nullptr;
-        if (cudaMalloc(&raw, total * sizeof(float)) != cudaSuccess) return fail(set_error(FLSTM_ERR_CUDA, "cudaMalloc of the gradient buffer failed"));
-        e.grads = static_cast<float *>(raw);
-        cudaMemset(raw, 0, total * sizeof(float));
-        if (cudaMalloc(&raw, (size_t)config->layers * B * H * sizeof(float)) != cudaSuccess) return fail(set_error(FLSTM_ERR_CUDA, "cudaMalloc failed"));
-        e.dc_layers = static_cast<float *>(raw);
+    if (config->backend == FLSTM_BACKEND_AUTO && !tc_ok) st = e.padded_create();
+    if (st == FLSTM_OK) st = e.init();
+    if (st != FLSTM_OK) {
+        delete h;
+        return st;
     }
-    for (auto &l : e.layers) {
-        l.dw_ih = e.grads + l.grad_offset;
-        l.dw_hh = l.dw_ih + 4 * H * l.in_size;
-        l.db = l.dw_hh + 4 * H * H;
-        void *raw = nullptr;
-        if (cudaMalloc(&raw, 4 * H * l.in_size * es) != cudaSuccess) return fail(set_error(FLSTM_ERR_CUDA, "cudaMalloc failed"));
-        l.w_ih = raw;
-        if (cudaMalloc(&raw, 4 * H * H * es) != cudaSuccess) return fail(set_error(FLSTM_ERR_CUDA, "cudaMalloc failed"));
-        l.w_hh = raw;
-        if (cudaMalloc(&raw, 4 * H * sizeof(float)) != cudaSuccess) return fail(set_error(FLSTM_ERR_CUDA, "cudaMalloc failed"));
-        l.bias = static_cast<float *>(raw);
-    }
-    if (e.backend == FLSTM_BACKEND_TC) {
-        st = flstm_b200::tc::init(e);
-        if (st != FLSTM_OK) return fail(st);
-    } else {
-        if (config->training) {
-            // room for up to 8 partial products of the largest weight gradient, at most 64 MiB
-            size_t widest = config->input_size > H ? config->input_size : H;
-            size_t floats = 8 * 4 * H * widest;
-            if (floats > (size_t)16 << 20) floats = (size_t)16 << 20;
-            void *raw = nullptr;
-            if (cudaMalloc(&raw, floats * sizeof(float)) == cudaSuccess) {
-                e.simt_scratch = static_cast<float *>(raw);
-                e.simt_scratch_floats = floats;
-            } else {
-                cudaGetLastError();  // the GEMMs then run unsplit
-            }
-        }
-        int grid = 0;
-        if (flstm_b200::simt::persistent_fits(config->dtype, B, H, config->training != 0, &grid)) {
-            void *raw = nullptr;
-            const size_t words = 32 + (size_t)flstm_b200::simt::persistent_batch_tiles(B);
-            if (cudaMalloc(&raw, words * sizeof(unsigned int)) != cudaSuccess) return fail(set_error(FLSTM_ERR_CUDA, "cudaMalloc failed"));
-            e.sync_words = static_cast<unsigned int *>(raw);
-            cudaMemset(raw, 0, words * sizeof(unsigned int));
-            if (cudaMallocHost(&raw, sizeof(unsigned int)) != cudaSuccess) return fail(set_error(FLSTM_ERR_CUDA, "cudaMallocHost failed"));
-            e.simt_err_host = static_cast<unsigned int *>(raw);
-            *e.simt_err_host = 0;
-            e.simt_grid = grid;
-        }
-    }
-    st = e.allocate(config->max_seq_len ? config->max_seq_len : 1);
-    if (st != FLSTM_OK) return fail(st);
     *out = h;
     return FLSTM_OK;
 }
@@ -969,6 +970,11 @@ int flstm_engine_cache_ptrs(flstm_engine *engine, int layer, void **gates, float
                             int *gate_layout) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
     if (layer < 0 || layer >= (int)engine->impl.layers.size()) return set_error(FLSTM_ERR_INVALID, "layer out of range");
+    if (engine->impl.inner) {
+        if (gate_layout) *gate_layout = 0;
+        DeviceScope scope(engine->impl.device);
+        return engine->impl.padded_cache_ptrs(layer, gates, cells, hiddens);
+    }
     auto &l = engine->impl.layers[layer];
     if (gates) *gates = l.gates;
     if (cells) *cells = l.cs;
@@ -1009,7 +1015,11 @@ int flstm_engine_set_recompute_interval(flstm_engine *engine, size_t interval) {
     return engine->impl.set_recompute(interval);
 }
 
-size_t flstm_engine_workspace_bytes(const flstm_engine *engine) { return engine ? engine->impl.workspace_bytes : 0; }
+size_t flstm_engine_workspace_bytes(const flstm_engine *engine) {
+    if (!engine) return 0;
+    const Engine &e = engine->impl;
+    return e.inner ? e.inner->workspace_bytes + e.pad.time_bytes + e.pad.state_bytes + e.pad.mirror_bytes : e.workspace_bytes;
+}
 
 int flstm_engine_abort_comm(flstm_engine *engine) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
@@ -1049,14 +1059,14 @@ int flstm_engine_wait(flstm_engine *engine, cudaStream_t stream, unsigned int ti
         return set_error(FLSTM_ERR_TIMEOUT, "the step did not finish within %u ms%s", timeout_ms,
                          had_comm ? "; the communicator was aborted" : "");
     }
-    if (e.backend == FLSTM_BACKEND_TC) FLSTM_TRY(flstm_b200::tc::poll_error(e));
+    if (e.backend == FLSTM_BACKEND_TC) FLSTM_TRY(flstm_b200::tc::poll_error(e.core()));
     else FLSTM_TRY(e.simt_check_error());
     return FLSTM_OK;
 }
 
 int flstm_engine_enable_trace(flstm_engine *engine, int steps) {
     if (!engine || steps < 0) return set_error(FLSTM_ERR_INVALID, "bad argument");
-    Engine &e = engine->impl;
+    Engine &e = engine->impl.core();
     DeviceScope scope(e.device);
     cudaDeviceSynchronize();
     if (e.trace) cudaFree(e.trace);
@@ -1074,7 +1084,7 @@ int flstm_engine_enable_trace(flstm_engine *engine, int steps) {
 
 int flstm_engine_read_trace(flstm_engine *engine, long long *out_host, size_t count) {
     if (!engine || !out_host) return set_error(FLSTM_ERR_INVALID, "null argument");
-    Engine &e = engine->impl;
+    Engine &e = engine->impl.core();
     DeviceScope scope(e.device);
     const size_t have = (size_t)2 * e.trace_steps * 16;
     if (!e.trace || count > have) return set_error(FLSTM_ERR_INVALID, "trace holds %zu values", have);
@@ -1085,31 +1095,32 @@ int flstm_engine_read_trace(flstm_engine *engine, long long *out_host, size_t co
 
 int flstm_engine_enable_timing(flstm_engine *engine, int enabled) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
-    engine->impl.timer.enabled = enabled != 0;
-    engine->impl.timer.reset();
+    engine->impl.core().timer.enabled = enabled != 0;
+    engine->impl.core().timer.reset();
     return FLSTM_OK;
 }
 
 int flstm_engine_phase_ms(flstm_engine *engine, float *out6) {
     if (!engine || !out6) return set_error(FLSTM_ERR_INVALID, "null argument");
     DeviceScope scope(engine->impl.device);
-    return engine->impl.timer.totals(out6);
+    return engine->impl.core().timer.totals(out6);
 }
 
 int flstm_engine_set_wait_limit(flstm_engine *engine, unsigned long long limit_us) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
-    engine->impl.wait_limit_ns = limit_us * 1000ull;
+    engine->impl.core().wait_limit_ns = limit_us * 1000ull;
     return FLSTM_OK;
 }
 
 int flstm_engine_selftest_missing_arrivals(flstm_engine *engine, unsigned int arrivals) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
-    engine->impl.selftest_missing_arrivals = arrivals;
+    engine->impl.core().selftest_missing_arrivals = arrivals;
     return FLSTM_OK;
 }
 
 unsigned long long flstm_engine_launch_count(const flstm_engine *engine) {
-    return engine ? engine->impl.launches : 0ull;
+    if (!engine) return 0ull;
+    return engine->impl.launches + (engine->impl.inner ? engine->impl.inner->launches : 0ull);
 }
 
 int flstm_bias_grad(int dtype, const void *dg, size_t rows, size_t cols, int interleaved_h, float *db, void *stream) {

@@ -105,6 +105,29 @@ struct Engine {
     // the timeout self-test: a step barrier that waits for this many arrivals which nobody makes.
     unsigned long long wait_limit_ns = 0;
     unsigned int selftest_missing_arrivals = 0;
+    // A 16-bit shape that the tensor-core path cannot tile runs there zero-padded (engine_padded.cu): this engine then
+    // only owns the logical gradients and staging tensors, `inner` has the padded sizes and does the work.
+    Engine *inner = nullptr;
+    int logical_h = 0, logical_in = 0;  // of an inner engine: the sizes of the parameters it is given (0: its own)
+    bool accurate = false;              // accurate gate functions (see common.cuh)
+    struct Padding {
+        void *x = nullptr, *dy = nullptr, *dx = nullptr;            // (T, B, .) padded, as needed
+        void *h0 = nullptr, *dhn = nullptr, *dcn = nullptr;         // (L, B, Hp) engine dtype
+        float *c0 = nullptr, *dh0 = nullptr, *dc0 = nullptr;        // (L, B, Hp) fp32
+        void *gates = nullptr, *hs = nullptr;                       // logical copies behind flstm_engine_cache_ptrs
+        float *cs = nullptr;
+        size_t t_cap = 0, t_mirror = 0;
+        size_t time_bytes = 0, state_bytes = 0, mirror_bytes = 0;
+    } pad;
+    Engine &core() { return inner ? *inner : *this; }
+    int padded_create();
+    void padded_release();
+    int padded_forward_range(size_t T, size_t t0, size_t t1, const void *x, const void *h0, const void *c0, void *y, void *hn,
+                             void *cn, cudaStream_t s);
+    int padded_backward_range(size_t T, size_t t0, size_t t1, const void *dy, const void *dhn, const void *dcn, void *dx,
+                              float *dh0, float *dc0, cudaStream_t s);
+    int padded_cache_ptrs(int layer, void **gates, float **cells, void **hiddens);
+    int padded_mirror(size_t t0, size_t t1, cudaStream_t s);
     bool cell_io_f32 = false;       // c0 / c_n cross the API as fp32 instead of the engine dtype
     const void *x_saved = nullptr;  // layer-0 input of the last forward (caller keeps it alive)
     PhaseTimer timer;
@@ -141,6 +164,7 @@ struct Engine {
     int allocate(size_t t_cap);
     void release_time_buffers();
     int ensure_capacity(size_t T);
+    int init();  // workspace, plans and backend state for cfg / backend / device
     // parameters of layers [first, first + count): w_ih, w_hh, b_ih, b_hh of each
     int set_weights(int first, int count, const float *const *params, cudaStream_t s);
     int forward(size_t T, const void *x, const void *h0, const void *c0, void *y, void *hn, void *cn,

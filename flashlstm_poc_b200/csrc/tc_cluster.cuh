@@ -58,20 +58,6 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
     return r;
 }
 
-// Gate functions.  ACCURATE: shapes whose recurrence used to run in the CUDA-core kernels with expf / tanhf keep an
-// error far below a 16-bit rounding step (about 1e-7 absolute); the others take the single-instruction form, whose
-// 2^-11 relative error is one fp16 rounding step.
-template <bool ACCURATE>
-__device__ __forceinline__ float sigmoid_sel(float a) {
-    return ACCURATE ? __fdividef(1.f, 1.f + __expf(-a)) : sigmoid_fast(a);
-}
-template <bool ACCURATE>
-__device__ __forceinline__ float tanh_sel(float a) {
-    if (!ACCURATE) return tanh_fast(a);
-    const float e = __expf(-2.f * fabsf(a));
-    return copysignf(__fdividef(1.f - e, 1.f + e), a);
-}
-
 // shared-memory row of `bytes` (a multiple of 64), padded so that the 16-byte fragment reads of 8 rows do not conflict
 __host__ __device__ constexpr int cluster_row_bytes(int bytes) { return bytes % 128 ? bytes : bytes + 64; }
 

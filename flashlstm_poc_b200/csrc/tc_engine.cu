@@ -236,12 +236,12 @@ int on_capacity_change(Engine &e) {
 
 int set_weights(Engine &e, int first, int count, const float *const *params, cudaStream_t s) {
     std::vector<PackJob> jobs;
-    const int H = (int)e.cfg.hidden_size;
+    const int Hp = (int)e.cfg.hidden_size, H = e.logical_h ? e.logical_h : Hp;
     for (int li = first; li < first + count; ++li, params += 4) {
         auto &l = e.layers[li];
-        const int K = (int)l.in_size;
-        jobs.push_back({params[0], l.w_ih, params[2], params[3], l.bias, H, H, K, K});
-        jobs.push_back({params[1], l.w_hh, nullptr, nullptr, nullptr, H, H, H, H});
+        const int Kp = (int)l.in_size, K = !e.logical_h ? Kp : li == 0 ? e.logical_in : H;
+        jobs.push_back({params[0], l.w_ih, params[2], params[3], l.bias, H, Hp, K, Kp});
+        jobs.push_back({params[1], l.w_hh, nullptr, nullptr, nullptr, H, Hp, H, Hp});
     }
     e.launches += (jobs.size() + kPackJobs - 1) / kPackJobs;
     return pack_weights(e.cfg.dtype, jobs.data(), (int)jobs.size(), s);
@@ -289,6 +289,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         cp.B = (int)B;
         cp.H = (int)H;
         cp.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
+        cp.accurate = e.accurate ? 1 : 0;
         cp.trace = (li == 0 && t0 == 0) ? e.trace : nullptr;
         cp.trace_steps = e.trace_steps;
         cp.wait_ns = e.wait_limit_ns;
@@ -317,6 +318,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
             wp.B = (int)B;
             wp.H = (int)H;
             wp.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
+            wp.accurate = e.accurate ? 1 : 0;
             wp.wait_ns = e.wait_limit_ns;
             wp.extra_arrivals = e.selftest_missing_arrivals;
             FLSTM_TRY(lstm_wide_forward(e.cfg.dtype, st->step, maps, wp, st->sms, s));
@@ -333,6 +335,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
             sp.B = (int)B;
             sp.H = (int)H;
             sp.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
+            sp.accurate = e.accurate ? 1 : 0;
             FLSTM_TRY(lstm_step_forward(e.cfg.dtype, st->step, maps, sp, st->sms, s));
         }
         size_t m2 = e.timer.mark(s);
@@ -354,6 +357,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.B = (int)B;
     p.H = (int)H;
     p.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
+    p.accurate = e.accurate ? 1 : 0;
     p.trace = (li == 0 && t0 == 0) ? e.trace : nullptr;
     p.trace_steps = e.trace_steps;
     p.wait_ns = e.wait_limit_ns;
@@ -388,7 +392,7 @@ static int backward_steps(Engine &e, int li, size_t T, size_t t0, size_t t1, con
         const int nparts = (step == T - 1) ? 1 : splits;
         FLSTM_TRY(lstm_step_backward_pointwise(e.cfg.dtype, byte_ptr(l.gates) + step * B * 4 * H * es, l.cs + (step + 1) * slab,
                                                l.cs + step * slab, byte_ptr(dy_l) + step * slab * es, parts, nparts, dc,
-                                               byte_ptr(l.dg) + step * B * 4 * H * es, (int)B, (int)H, s));
+                                               byte_ptr(l.dg) + step * B * 4 * H * es, (int)B, (int)H, e.accurate, s));
         ++e.launches;
         if (step > 0 || dh0_l || !finalize) {  // the product at step 0 is dh0, or the carry into the segment before
             FLSTM_TRY(lstm_step_backward_gemm(e.cfg.dtype, st->step, t.tm_dg3, t.tm_w, (int)step, (int)B, (int)H, parts,
@@ -441,6 +445,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
         cp.dh0 = dh0_l;
         cp.dc0 = dc0_l;
         cp.dc = e.dc_layers + (size_t)li * B * H;
+        cp.accurate = e.accurate ? 1 : 0;
         cp.err = err;
         cp.T = (int)T;
         cp.s0 = (int)(T - t1);
@@ -466,6 +471,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.dh0 = dh0_l;
     p.dc0 = dc0_l;
     p.dc = e.dc_layers + (size_t)li * B * H;
+    p.accurate = e.accurate ? 1 : 0;
     p.trace = (li == 0 && e.trace && t1 == T) ? e.trace + (size_t)e.trace_steps * 16 : nullptr;
     p.trace_steps = e.trace_steps;
     p.counters = e.sync_words + 1;

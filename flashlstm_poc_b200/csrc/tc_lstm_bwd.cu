@@ -405,7 +405,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         if (PREFETCH) v = in[k];
                         else load_pair(q, i, v);
                         const float dh = v.dy + dh_in[k];
-                        const float tc = tanh_fast(v.ct);
+                        const float tc = p.accurate ? tanh_sel<true>(v.ct) : tanh_fast(v.ct);
                         const float d_o = dh * tc;
                         const float dcv = dc_in[k] + dh * v.go * (1.f - tc * tc);
                         const float dai = dcv * v.gg * v.gi * (1.f - v.gi);

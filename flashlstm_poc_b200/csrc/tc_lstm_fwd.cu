@@ -417,9 +417,16 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         const float af = ex[(1 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 1 * 16 + u);
                         const float ag = ex[(2 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 2 * 16 + u);
                         const float ao = ex[(3 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 3 * 16 + u);
-                        const float gi = sigmoid_fast(ai), gf = sigmoid_fast(af), gg = tanh_fast(ag), go = sigmoid_fast(ao);
-                        const float c = fmaf(gf, c_prev[i], gi * gg);
-                        const float h = go * tanh_fast(c);
+                        float gi, gf, gg, go, c, h;
+                        if (p.accurate) {
+                            gi = sigmoid_sel<true>(ai); gf = sigmoid_sel<true>(af); gg = tanh_sel<true>(ag); go = sigmoid_sel<true>(ao);
+                            c = fmaf(gf, c_prev[i], gi * gg);
+                            h = go * tanh_sel<true>(c);
+                        } else {
+                            gi = sigmoid_fast(ai); gf = sigmoid_fast(af); gg = tanh_fast(ag); go = sigmoid_fast(ao);
+                            c = fmaf(gf, c_prev[i], gi * gg);
+                            h = go * tanh_fast(c);
+                        }
                         c_keep[i] = c;
                         act[i][0] = gi; act[i][1] = gf; act[i][2] = gg; act[i][3] = go;
                         h16[i] = to16<BF16>(h);

@@ -18,6 +18,7 @@
 // Replaces, for large batches, the same reference code as the persistent kernels: the per-step
 // recurrent launches of flashlstm_v2/src/lstm_forward.cu:744-830 and lstm_backward.cu:806-1110.
 #include <cstdlib>
+#include <type_traits>
 #include <utility>
 
 #include <cuda_bf16.h>
@@ -71,6 +72,7 @@ struct StepArgs {
     int t;             // time step: projection / gate cache and y at slot t, states read at slot t, written at t+1
     int has_y;         // also store h_t into the caller's y
     int store_gates;   // write the activated gates back (the gate cache)
+    int accurate;      // accurate gate functions (see common.cuh)
     int early;         // fetch the first weight blocks ahead of the previous kernel's completion (FLSTM_PDL_EARLY=0: off)
 };
 
@@ -144,7 +146,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // Outputs overwrite the inputs in place (gates over the projection, c_t over c_{t-1}).
 template <bool BF16>
 __device__ __forceinline__ void lstm_cell_16(const uint32_t (&acc)[64], uint8_t *sP, uint8_t *sC, uint8_t *sH, int r,
-                                             int store_gates) {
+                                             int store_gates, int accurate_gates) {
     uint8_t *prow = sP + r * 128, *crow = sC + r * 64, *hrow = sH + r * 32;
     const int xp = r & 7, xc = (r >> 1) & 3, xh = (r >> 2) & 1;
 #pragma unroll
@@ -166,15 +168,20 @@ __device__ __forceinline__ void lstm_cell_16(const uint32_t (&acc)[64], uint8_t 
                 act[g][2 * k + 1] = __uint_as_float(acc[g * 16 + ub * 8 + 2 * k + 1]) + pp.y;
             }
         }
+        auto cell = [&](auto accurate) {
+            constexpr bool ACC = decltype(accurate)::value;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const float gi = sigmoid_fast(act[0][u]), gf = sigmoid_fast(act[1][u]);
-            const float gg = tanh_fast(act[2][u]), go = sigmoid_fast(act[3][u]);
-            const float c = fmaf(gf, cp[u], gi * gg);
-            cn[u] = c;
-            hn[u] = go * tanh_fast(c);
-            act[0][u] = gi; act[1][u] = gf; act[2][u] = gg; act[3][u] = go;
-        }
+            for (int u = 0; u < 8; ++u) {
+                const float gi = sigmoid_sel<ACC>(act[0][u]), gf = sigmoid_sel<ACC>(act[1][u]);
+                const float gg = tanh_sel<ACC>(act[2][u]), go = sigmoid_sel<ACC>(act[3][u]);
+                const float c = fmaf(gf, cp[u], gi * gg);
+                cn[u] = c;
+                hn[u] = go * tanh_sel<ACC>(c);
+                act[0][u] = gi; act[1][u] = gf; act[2][u] = gg; act[3][u] = go;
+            }
+        };
+        if (accurate_gates) cell(std::true_type{});
+        else cell(std::false_type{});
         *reinterpret_cast<uint4 *>(hrow + ((ub ^ xh) << 4)) =
             make_uint4(pack2<BF16>(hn[0], hn[1]), pack2<BF16>(hn[2], hn[3]), pack2<BF16>(hn[4], hn[5]), pack2<BF16>(hn[6], hn[7]));
         *reinterpret_cast<float4 *>(crow + (((ub * 2) ^ xc) << 4)) = make_float4(cn[0], cn[1], cn[2], cn[3]);
@@ -441,7 +448,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     if (!ok) break;
                     ldphase ^= 1u << buf;
                     uint8_t *sP = wb + buf * kEpiPBytes, *sC = wb + 2 * kEpiPBytes + buf * kEpiCBytes;
-                    lstm_cell_16<BF16>(acc, sP, sC, sH, lane, a.store_gates);
+                    lstm_cell_16<BF16>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -512,7 +519,7 @@ struct WideFwdArgs {
     uint32_t idesc;
     unsigned int *err;
     unsigned int *counter, *exits;  // step barrier and CTAs that have left, zero between launches (leave_counters)
-    int has_y, store_gates;
+    int has_y, store_gates, accurate;
     unsigned long long wait_ns;   // limit of every wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path: arrivals nobody makes
 };
@@ -763,7 +770,7 @@ wide_fwd_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                     if (!good) continue;
                     ldphase ^= 1u << buf;
                     uint8_t *sP = wb + buf * kEpiPBytes, *sC = wb + 2 * kEpiPBytes + buf * kEpiCBytes;
-                    lstm_cell_16<BF16>(acc, sP, sC, sH, lane, a.store_gates);
+                    lstm_cell_16<BF16>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -814,7 +821,7 @@ __global__ void __launch_bounds__(256)
 step_bwd_pointwise_kernel(const uint16_t *__restrict__ gates_t, const float *__restrict__ c_t,
                           const float *__restrict__ c_prev, const uint16_t *__restrict__ dy_t,
                           const float *__restrict__ parts, int nparts, float *__restrict__ dc,
-                          uint16_t *__restrict__ dg_t, int B, int H, int early) {
+                          uint16_t *__restrict__ dg_t, int B, int H, int early, int accurate) {
     const int quads = H >> 2;
     const size_t total = (size_t)B * quads, slab = (size_t)B * H;
     // The split-K GEMM that follows may start its prologue and fetch its first weight blocks while this kernel
@@ -854,7 +861,7 @@ step_bwd_pointwise_kernel(const uint16_t *__restrict__ gates_t, const float *__r
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const float gi = gate[0][u], gf = gate[1][u], gg = gate[2][u], go = gate[3][u];
-            const float tc = tanh_fast(ct[u]);
+            const float tc = accurate ? tanh_sel<true>(ct[u]) : tanh_fast(ct[u]);
             const float d_o = dh[u] * tc;
             const float dcu = dcin[u] + dh[u] * go * (1.f - tc * tc);
             da[0][u] = dcu * gg * gi * (1.f - gi);
@@ -1012,6 +1019,7 @@ int lstm_step_forward(int dtype, const StepPlan &plan, const StepFwdMaps &m, con
     a.t = p.t;
     a.has_y = m.y ? 1 : 0;
     a.store_gates = p.store_gates;
+    a.accurate = p.accurate;
     const EpilogueMaps em{m.gates, m.cs, m.hs_out, m.y ? m.y : m.hs_out};
     if (plan.bn_fwd == 256)
         return bf16 ? launch_step<256, EPI_LSTM_FWD, false, true>(plan.pair, *m.hs, *m.w, em, a, sms, s)
@@ -1063,6 +1071,7 @@ int lstm_wide_forward(int dtype, const StepPlan &plan, const StepFwdMaps &m, con
     a.exits = p.exits;
     a.has_y = m.y ? 1 : 0;
     a.store_gates = p.store_gates;
+    a.accurate = p.accurate;
     a.wait_ns = p.wait_ns;
     a.extra_arrivals = p.extra_arrivals;
     if (plan.fwd_pair) {
@@ -1096,15 +1105,15 @@ int lstm_step_backward_gemm(int dtype, const StepPlan &plan, const CUtensorMap &
 }
 
 int lstm_step_backward_pointwise(int dtype, const void *gates_t, const float *c_t, const float *c_prev, const void *dy_t,
-                                 const float *parts, int nparts, float *dc, void *dg_t, int B, int H, cudaStream_t s) {
+                                 const float *parts, int nparts, float *dc, void *dg_t, int B, int H, bool accurate, cudaStream_t s) {
     const size_t total = (size_t)B * (H / 4);
     int grid = (int)((total + 255) / 256);
     if (grid > 148 * 16) grid = 148 * 16;
     const uint16_t *g16 = static_cast<const uint16_t *>(gates_t), *dy16 = static_cast<const uint16_t *>(dy_t);
     uint16_t *dg16 = static_cast<uint16_t *>(dg_t);
     cudaError_t e = dtype == FLSTM_DTYPE_BF16
-                        ? launch_chained(step_bwd_pointwise_kernel<true>, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0)
-                        : launch_chained(step_bwd_pointwise_kernel<false>, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0);
+                        ? launch_chained(step_bwd_pointwise_kernel<true>, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0, accurate ? 1 : 0)
+                        : launch_chained(step_bwd_pointwise_kernel<false>, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0, accurate ? 1 : 0);
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "step pointwise launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
 }

@@ -1,0 +1,69 @@
+"""16-bit shapes that the tensor-core path runs zero-padded (engine_padded.cu), against the oracle: odd widths around the
+padding's edges, each recurrent schedule behind it (clusters, grid-wide persistent, wide batch), the caches in logical
+layout, step ranges, and tensors that start off a 16-byte boundary."""
+import numpy as np
+import pytest
+import torch
+
+from flashlstm_poc_b200.engine import TORCH_DTYPES, Engine
+from flashlstm_poc_b200.workloads import Workload, make_inputs
+from oracle import lstm_oracle as orc
+from tests.gpu_helpers import assert_parity, run_engine, run_oracle
+from tests.helpers import to_np
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,L,T,B,I,H", [
+    ("f16", 2, 6, 20, 650, 650), ("bf16", 1, 5, 3, 5, 5), ("f16", 3, 4, 7, 63, 65), ("bf16", 1, 7, 33, 12, 100),
+    ("f16", 2, 5, 9, 3, 64),       # only the input is padded
+    ("bf16", 2, 4, 40, 130, 1217),  # grid-wide persistent kernels
+    ("f16", 1, 3, 150, 64, 1270),   # wide batch
+])
+def test_padded_shapes_match_the_oracle(dtype, L, T, B, I, H):
+    w = Workload("t", dtype, L, I, H, B, T, seed=51, state_std=0.3)
+    inp = make_inputs(w)
+    gen = torch.Generator().manual_seed(5)
+    dhn, dcn = torch.randn(L, B, H, generator=gen), torch.randn(L, B, H, generator=gen)
+    td = TORCH_DTYPES[dtype]
+    dhn, dcn = dhn.to(td).float(), dcn.to(td).float()
+    got, eng = run_engine(w, inp, dhn=dhn, dcn=dcn, repeat=2)
+    assert eng.backend == "tc"
+    ref = run_oracle(inp, dhn=dhn, dcn=dcn)
+    assert_parity(got, ref, dtype)
+    for l in range(L):
+        assert orc.max_abs_err(to_np(eng.gate_cache(l, T)), ref["gates"][l]) < 2e-2  # gates in (-1, 1), 16-bit h behind them
+        assert np.isfinite(to_np(eng.cell_states(l, T))).all()
+    eng.close()
+
+
+def test_padded_ranges_and_unaligned_tensors():
+    T, B, I, H = 7, 5, 33, 70
+    w = Workload("t", "f16", 2, I, H, B, T, seed=52, state_std=0.3)
+    inp = make_inputs(w)
+    dev, td = torch.device("cuda", 0), torch.float16
+    eng = Engine("f16", 2, B, I, H, T, device=dev)
+    for l in range(2):
+        eng.set_weights(l, inp.w_ih[l].to(dev), inp.w_hh[l].to(dev), inp.b_ih[l].to(dev), inp.b_hh[l].to(dev))
+
+    def odd(t):  # the same values one element past an aligned start
+        flat = torch.zeros(t.numel() + 1, dtype=t.dtype, device=dev)
+        flat[1:] = t.to(dev).flatten()
+        return flat[1:].view(t.shape)
+
+    x, h0, c0, dy = (t.to(dev, td) for t in (inp.x, inp.h0, inp.c0, inp.dy))
+    y, hn, cn = eng.forward(x, h0, c0)
+    dx, dh0, dc0 = eng.backward(dy)
+    cells = eng.cell_states(1, T).clone()
+    want = [t.clone() for t in (y, hn, cn, dx, dh0, dc0, *eng.grads(0), *eng.grads(1))]
+    x2, dy2, y2, dx2 = odd(x), odd(dy), odd(torch.zeros_like(y)), odd(torch.zeros_like(dx))
+    hn2, cn2, dh2, dc2 = torch.zeros_like(hn), torch.zeros_like(cn), torch.zeros_like(dh0), torch.zeros_like(dc0)
+    for t0, t1 in ((0, 2), (2, 3), (3, 7)):
+        eng.forward_range_into(T, t0, t1, x2, h0, c0, y2, hn2, cn2)
+    for t0, t1 in ((4, 7), (0, 4)):
+        eng.backward_range_into(T, t0, t1, dy2, None, None, dx2, dh2, dc2)
+    torch.cuda.synchronize()
+    for a, b in zip(want, (y2, hn2, cn2, dx2, dh2, dc2, *eng.grads(0), *eng.grads(1))):
+        assert torch.equal(a, b)
+    assert torch.equal(cells, eng.cell_states(1, T))  # the logical copy follows the later calls
+    eng.close()

@@ -8,6 +8,7 @@
 // asynchronously on the caller's stream.
 #include "engine.h"
 
+#include <algorithm>
 #include <chrono>
 #include <cstring>
 #include <map>
@@ -53,18 +54,6 @@ cudaError_t ensure_smem_limit(const void *kernel, int bytes) {
 namespace {
 
 template <typename P>
-int dev_alloc(P **p, size_t bytes) {
-    *p = nullptr;
-    if (bytes == 0) return FLSTM_OK;
-    void *raw = nullptr;
-    cudaError_t e = cudaMalloc(&raw, bytes);
-    if (e != cudaSuccess)
-        return set_error(FLSTM_ERR_CUDA, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
-    *p = static_cast<P *>(raw);
-    return FLSTM_OK;
-}
-
-template <typename P>
 void dev_free(P *&p) {
     if (p) cudaFree(p);
     p = nullptr;
@@ -74,6 +63,72 @@ inline char *byte_ptr(void *p) { return static_cast<char *>(p); }
 inline const char *byte_ptr(const void *p) { return static_cast<const char *>(p); }
 
 }  // namespace
+
+int Arena::commit() {
+    size_t total = 0;
+    for (auto &r : requests) total += (r.bytes + 255) / 256 * 256;
+    const cudaError_t e = total ? cudaMalloc(&base, total) : cudaSuccess;
+    if (e != cudaSuccess) {
+        base = nullptr;
+        return set_error(FLSTM_ERR_CUDA, "cudaMalloc(%zu bytes) failed: %s", total, cudaGetErrorString(e));
+    }
+    char *next = static_cast<char *>(base);
+    for (auto &r : requests) {
+        *r.p = r.bytes ? next : nullptr;
+        next += (r.bytes + 255) / 256 * 256;
+    }
+    return FLSTM_OK;
+}
+
+void Arena::release() {
+    if (base) cudaFree(base);
+    for (auto &r : requests) *r.p = nullptr;
+    requests.clear();
+    base = nullptr;
+}
+
+namespace {
+struct HostWords {
+    static constexpr int kWords = 1024;
+    std::mutex mu;
+    unsigned int *slab = nullptr;  // lives as long as the process
+    std::vector<unsigned int *> free_words;
+};
+HostWords &host_words() {
+    static HostWords *w = new HostWords();
+    return *w;
+}
+}  // namespace
+
+unsigned int *host_word_acquire() {
+    HostWords &w = host_words();
+    std::lock_guard<std::mutex> lock(w.mu);
+    if (!w.slab) {
+        void *raw = nullptr;
+        if (cudaHostAlloc(&raw, HostWords::kWords * sizeof(unsigned int), cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        w.slab = static_cast<unsigned int *>(raw);
+        for (int i = HostWords::kWords; i-- > 0;) w.free_words.push_back(w.slab + i);
+    }
+    unsigned int *word = nullptr;
+    if (!w.free_words.empty()) {
+        word = w.free_words.back();
+        w.free_words.pop_back();
+    } else {  // more engines alive than the slab has words
+        void *raw = nullptr;
+        if (cudaHostAlloc(&raw, sizeof(unsigned int), cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        word = static_cast<unsigned int *>(raw);
+    }
+    *word = 0;
+    return word;
+}
+
+void host_word_release(unsigned int *word) {
+    if (!word) return;
+    HostWords &w = host_words();
+    std::lock_guard<std::mutex> lock(w.mu);
+    if (word >= w.slab && word < w.slab + HostWords::kWords) w.free_words.push_back(word);
+    else cudaFreeHost(word);
+}
 
 // Workspace for cfg / backend on the current device.  An engine with an `inner` one owns the logical gradients only.
 int Engine::init() {
@@ -88,66 +143,55 @@ int Engine::init() {
         total += l.grad_count;
     }
     grad_count = total;
-    FLSTM_TRY(dev_alloc(&grads, total * sizeof(float)));
+    fixed.want(&grads, total * sizeof(float));
+    if (!inner) {
+        fixed.want(&dc_layers, (size_t)cfg.layers * B * H * sizeof(float));
+        for (auto &l : layers) {
+            fixed.want(&l.w_ih, 4 * H * l.in_size * es);
+            fixed.want(&l.w_hh, 4 * H * H * es);
+            fixed.want(&l.bias, 4 * H * sizeof(float));
+        }
+    }
+    size_t words = 0;
+    if (!inner && backend == FLSTM_BACKEND_TC) {
+        FLSTM_TRY(tc::init(*this));
+        words = tc::kSyncWords;
+    } else if (!inner) {
+        if (cfg.training) {
+            // room for up to 8 partial products of the largest weight gradient, at most 64 MiB
+            const size_t widest = cfg.input_size > H ? cfg.input_size : H;
+            simt_scratch_floats = std::min(8 * 4 * H * widest, (size_t)16 << 20);
+            fixed.want(&simt_scratch, simt_scratch_floats * sizeof(float));
+        }
+        if (simt::persistent_fits(cfg.dtype, B, H, cfg.training != 0, &simt_grid)) {
+            words = 32 + (size_t)simt::persistent_batch_tiles(B);
+            simt_err_host = host_word_acquire();
+            if (!simt_err_host) return set_error(FLSTM_ERR_CUDA, "pinned allocation failed");
+        }
+    }
+    if (words) fixed.want(&sync_words, words * sizeof(unsigned int));
+    FLSTM_TRY(fixed.commit());
     FLSTM_CUDA_TRY(cudaMemset(grads, 0, total * sizeof(float)));
+    if (words) FLSTM_CUDA_TRY(cudaMemset(sync_words, 0, words * sizeof(unsigned int)));
     for (auto &l : layers) {
         l.dw_ih = grads + l.grad_offset;
         l.dw_hh = l.dw_ih + 4 * H * l.in_size;
         l.db = l.dw_hh + 4 * H * H;
     }
-    if (inner) return FLSTM_OK;
-    FLSTM_TRY(dev_alloc(&dc_layers, (size_t)cfg.layers * B * H * sizeof(float)));
-    for (auto &l : layers) {
-        FLSTM_TRY(dev_alloc(&l.w_ih, 4 * H * l.in_size * es));
-        FLSTM_TRY(dev_alloc(&l.w_hh, 4 * H * H * es));
-        FLSTM_TRY(dev_alloc(&l.bias, 4 * H * sizeof(float)));
-    }
-    if (backend == FLSTM_BACKEND_TC) {
-        FLSTM_TRY(tc::init(*this));
-    } else {
-        if (cfg.training) {
-            // room for up to 8 partial products of the largest weight gradient, at most 64 MiB
-            const size_t widest = cfg.input_size > H ? cfg.input_size : H;
-            size_t floats = 8 * 4 * H * widest;
-            if (floats > (size_t)16 << 20) floats = (size_t)16 << 20;
-            if (dev_alloc(&simt_scratch, floats * sizeof(float)) == FLSTM_OK) simt_scratch_floats = floats;
-            else cudaGetLastError();  // the GEMMs then run unsplit
-        }
-        int grid = 0;
-        if (simt::persistent_fits(cfg.dtype, B, H, cfg.training != 0, &grid)) {
-            const size_t words = 32 + (size_t)simt::persistent_batch_tiles(B);
-            FLSTM_TRY(dev_alloc(&sync_words, words * sizeof(unsigned int)));
-            FLSTM_CUDA_TRY(cudaMemset(sync_words, 0, words * sizeof(unsigned int)));
-            void *raw = nullptr;
-            FLSTM_CUDA_TRY(cudaMallocHost(&raw, sizeof(unsigned int)));
-            simt_err_host = static_cast<unsigned int *>(raw);
-            *simt_err_host = 0;
-            simt_grid = grid;
-        }
-    }
-    return allocate(cfg.max_seq_len ? cfg.max_seq_len : 1);
+    return inner ? FLSTM_OK : allocate(cfg.max_seq_len ? cfg.max_seq_len : 1);
 }
 
 Engine::~Engine() {
     padded_release();
     delete inner;
-    tc::destroy(*this);
     release_time_buffers();
-    for (auto &l : layers) {
-        dev_free(l.w_ih);
-        dev_free(l.w_hh);
-        dev_free(l.bias);
-    }
-    dev_free(grads);
-    dev_free(dc_layers);
-    dev_free(db_part);
-    dev_free(sync_words);
+    fixed.release();  // before the objects whose pointers it clears
+    tc::destroy(*this);
     dev_free(trace);
     for (size_t i = 1; i < lanes.size(); ++i)
         if (lanes[i]) cudaStreamDestroy(lanes[i]);
     for (auto ev : lane_events) cudaEventDestroy(ev);
-    if (simt_err_host) cudaFreeHost(simt_err_host);
-    dev_free(simt_scratch);
+    host_word_release(simt_err_host);
     if (comm) comm_destroy(comm);
     if (comm_stream) cudaStreamDestroy(comm_stream);
     if (comm_fork) cudaEventDestroy(comm_fork);
@@ -208,16 +252,7 @@ cudaEvent_t Engine::next_lane_event() {
 }
 
 void Engine::release_time_buffers() {
-    for (auto &l : layers) {
-        dev_free(l.gates);
-        dev_free(l.hs);
-        dev_free(l.cs);
-        dev_free(l.dg);
-        dev_free(l.dx);
-        dev_free(l.y_all);
-        dev_free(l.ck_h);
-        dev_free(l.ck_c);
-    }
+    timed.release();
     t_cap = 0;
     buf_steps = 0;
     workspace_bytes = 0;
@@ -229,23 +264,24 @@ int Engine::allocate(size_t cap) {
     const size_t bs = (recompute && recompute < cap) ? recompute : cap;  // steps the gate-sized buffers span
     const size_t segments = (cap + bs - 1) / bs;
     size_t total = 0;
-    auto sized = [&](auto **p, size_t bytes) { total += bytes; return dev_alloc(p, bytes); };
+    auto sized = [&](auto **p, size_t bytes) { total += bytes; timed.want(p, bytes); };
     for (size_t li = 0; li < layers.size(); ++li) {
         auto &l = layers[li];
-        FLSTM_TRY(sized(&l.gates, bs * B * 4 * H * es));
-        FLSTM_TRY(sized(&l.hs, (bs + 1) * B * H * es));
-        FLSTM_TRY(sized(&l.cs, (bs + 1) * B * H * sizeof(float)));
+        sized(&l.gates, bs * B * 4 * H * es);
+        sized(&l.hs, (bs + 1) * B * H * es);
+        sized(&l.cs, (bs + 1) * B * H * sizeof(float));
         if (cfg.training) {
             // with checkpoints one more slot: dG of the first step of the segment processed before
-            FLSTM_TRY(sized(&l.dg, (bs + (recompute ? 1 : 0)) * B * 4 * H * es));
-            if (li > 0) FLSTM_TRY(sized(&l.dx, cap * B * l.in_size * es));
+            sized(&l.dg, (bs + (recompute ? 1 : 0)) * B * 4 * H * es);
+            if (li > 0) sized(&l.dx, cap * B * l.in_size * es);
         }
         if (recompute) {
-            if (li + 1 < layers.size()) FLSTM_TRY(sized(&l.y_all, cap * B * H * es));
-            FLSTM_TRY(sized(&l.ck_h, segments * B * H * es));
-            FLSTM_TRY(sized(&l.ck_c, segments * B * H * sizeof(float)));
+            if (li + 1 < layers.size()) sized(&l.y_all, cap * B * H * es);
+            sized(&l.ck_h, segments * B * H * es);
+            sized(&l.ck_c, segments * B * H * sizeof(float));
         }
     }
+    FLSTM_TRY(timed.commit());
     t_cap = cap;
     buf_steps = bs;
     workspace_bytes = total;

@@ -73,8 +73,23 @@ struct CopyBatch {
     int run(cudaStream_t s, unsigned long long *launches);
 };
 
+// Buffers that live and die together come from ONE cudaMalloc: each costs about 0.4 ms here, and an engine has dozens.
+struct Arena {
+    struct Request { void **p; size_t bytes; };
+    std::vector<Request> requests;
+    void *base = nullptr;
+    template <typename P>
+    void want(P **p, size_t bytes) { requests.push_back({reinterpret_cast<void **>(p), bytes}); }
+    int commit();   // allocates what was asked for since the last commit (at most one allocation at a time)
+    void release();
+};
+// A pinned host word for an engine's error mirror, from a small process-wide slab (cudaMallocHost takes milliseconds).
+unsigned int *host_word_acquire();
+void host_word_release(unsigned int *word);
+
 struct Engine {
     flstm_engine_config cfg{};
+    Arena fixed, timed;  // weights, gradients, scratch; buffers sized by the sequence length
     int backend = FLSTM_BACKEND_SIMT;
     int device = 0;
     size_t t_cap = 0;  // longest sequence the engine is currently sized for
@@ -112,6 +127,7 @@ struct Engine {
     bool accurate = false;              // accurate gate functions (see common.cuh)
     struct Padding {
         void *x = nullptr, *dy = nullptr, *dx = nullptr;            // (T, B, .) padded, as needed
+        void *odd_x = nullptr, *odd_dy = nullptr, *odd_dx = nullptr;  // for callers' tensors off a 16-byte boundary
         void *h0 = nullptr, *dhn = nullptr, *dcn = nullptr;         // (L, B, Hp) engine dtype
         float *c0 = nullptr, *dh0 = nullptr, *dc0 = nullptr;        // (L, B, Hp) fp32
         void *gates = nullptr, *hs = nullptr;                       // logical copies behind flstm_engine_cache_ptrs
@@ -122,6 +138,7 @@ struct Engine {
     Engine &core() { return inner ? *inner : *this; }
     int padded_create();
     void padded_release();
+    int padded_reserve(size_t T);
     int padded_forward_range(size_t T, size_t t0, size_t t1, const void *x, const void *h0, const void *c0, void *y, void *hn,
                              void *cn, cudaStream_t s);
     int padded_backward_range(size_t T, size_t t0, size_t t1, const void *dy, const void *dhn, const void *dcn, void *dx,
@@ -196,6 +213,7 @@ namespace flstm_b200 {
 
 // Tensor-core path entry points (tc_engine.cu).  `supported` decides AUTO resolution.
 namespace tc {
+constexpr size_t kSyncWords = 1024;  // step counters, exit counter and error word of an engine
 bool supported(const flstm_engine_config &cfg);
 int init(Engine &e);
 void destroy(Engine &e);

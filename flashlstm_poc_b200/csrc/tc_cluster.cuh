@@ -125,10 +125,14 @@ struct ClusterBwdParams {
     int dy_aligned;  // dY starts on a 16-byte boundary
 };
 
-// Plans for a shape, or use = false.  check_device: ask the occupancy calculator how many clusters run at once;
-// otherwise the numbers measured on a B200 (148 SMs) are used.
-int plan_cluster_fwd(int B, int H, int sms, size_t smem_limit, ClusterFwdPlan *plan, bool check_device);
-int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *plan, bool check_device);
+// Plans for a shape, or use = false.  With `check` the occupancy calculator is asked how many clusters of the kernel run
+// at once; otherwise the numbers measured on a B200 (148 SMs) are used.  Clusters never wait on one another, so a wrong
+// number costs a second wave and nothing else.
+struct ClusterCheck {
+    bool bf16, accurate;  // which kernel will be launched
+};
+int plan_cluster_fwd(int B, int H, int sms, size_t smem_limit, ClusterFwdPlan *plan, const ClusterCheck *check);
+int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *plan, const ClusterCheck *check);
 int lstm_forward_cluster(int dtype, const ClusterFwdPlan &plan, ClusterFwdParams p, cudaStream_t s);
 int lstm_backward_cluster(int dtype, const ClusterBwdPlan &plan, ClusterBwdParams p, cudaStream_t s);
 bool cluster_enabled();  // FLSTM_CLUSTER=0 keeps the grid-wide kernels

@@ -480,20 +480,23 @@ int bwd_smem(const ClusterBwdPlan &pl) {
 }  // namespace
 
 // Like plan_cluster_fwd over the rows of kBwdShapes; a step moves H fp32 partial sums per group of four sequences.
-int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *plan, bool check_device) {
+int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *plan, const ClusterCheck *check) {
     *plan = ClusterBwdPlan{};
     if (!cluster_enabled() || H % 64 || H > 768) return FLSTM_OK;
     const char *env = std::getenv("FLSTM_CLUSTER_SIZE");
     const int only = env ? std::atoi(env) : 0;
     const int blocks = H / 8, tiles16 = H / 16;
-    for (int C = 1; C <= 16; C *= 2) {
-        if (only && C != only) continue;
-        const int nub = (blocks + C - 1) / C;
-        for (const BwdShape &r : kBwdShapes) {
-            const int cover = r.W / r.KSB * r.MT;
-            if (r.NKB * r.KSB != nub || cover < tiles16 || cover > tiles16 + r.MT * 2) continue;
-            int slots = cluster_slots(C, sms);
-            for (int pass = 0; pass < 2 && slots > 0; ++pass) {
+    int slots[5];
+    for (int n = 0; n < 5; ++n) slots[n] = cluster_slots(1 << n, sms);
+    for (int tries = 0; tries < 8; ++tries) {
+        *plan = ClusterBwdPlan{};
+        const BwdShape *shape = nullptr;
+        for (int n = 0; n < 5; ++n) {
+            const int C = 1 << n, nub = (blocks + C - 1) / C;
+            if ((only && C != only) || slots[n] < 1) continue;
+            for (const BwdShape &r : kBwdShapes) {
+                const int cover = r.W / r.KSB * r.MT;
+                if (r.NKB * r.KSB != nub || cover < tiles16 || cover > tiles16 + r.MT * 2) continue;
                 ClusterBwdPlan pl{};
                 pl.C = C;
                 pl.nub = nub;
@@ -502,21 +505,14 @@ int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *p
                 pl.MT = r.MT;
                 pl.NKB = r.NKB;
                 pl.KSB = r.KSB;
-                pl.seqs = (B + slots - 1) / slots;
+                pl.seqs = (B + slots[n] - 1) / slots[n];
                 const int tiles = (pl.seqs + 7) / 8;
-                if (tiles > 4) break;
+                if (tiles > 4) continue;
                 pl.NT = tiles <= 1 ? 1 : tiles <= 2 ? 2 : 4;
                 pl.threads = r.W * 32;
                 pl.smem_bytes = bwd_smem(pl);
-                if ((size_t)pl.smem_bytes + 1024 > smem_limit) break;
+                if ((size_t)pl.smem_bytes + 1024 > smem_limit) continue;
                 pl.clusters = (B + pl.seqs - 1) / pl.seqs;
-                if (check_device) {
-                    const int have = cluster_count(reinterpret_cast<const void *>(r.kernels[nt_index(pl.NT)][0][0]), C, pl.threads, pl.smem_bytes);
-                    if (have < pl.clusters) {
-                        slots = have;
-                        continue;
-                    }
-                }
                 const int frags = r.MT * r.NKB, chain = r.NKB * 40, pairs = cluster_bwd_pairs(r.W, 8 * nub, pl.NT);
                 const int busy = (r.W + 3) / 4 * frags * pl.NT * 16;
                 const int in_smem = frags - cluster_bwd_reg_frags(r.W, r.MT, r.NKB, pl.NT, pairs);
@@ -524,11 +520,20 @@ int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *p
                 pl.cycles = (busy > chain ? busy : chain) + r.W * in_smem * 8 + (C == 1 ? 300 : 580 + 6 * C + incoming / 14) + 500 +
                             pairs * (250 + 6 * pl.peers * r.KSB) + r.MT * pl.NT * 40;
                 pl.use = true;
-                if (!plan->use || pl.cycles < plan->cycles) *plan = pl;
-                break;
+                if (!plan->use || pl.cycles < plan->cycles) {
+                    *plan = pl;
+                    shape = &r;
+                }
             }
         }
+        if (!plan->use || !check) return FLSTM_OK;
+        const int have = cluster_count(reinterpret_cast<const void *>(shape->kernels[nt_index(plan->NT)][check->bf16][check->accurate]),
+                                       plan->C, plan->threads, plan->smem_bytes);
+        if (have >= plan->clusters) return FLSTM_OK;
+        for (int n = 0; n < 5; ++n)
+            if (plan->C == 1 << n) slots[n] = have;
     }
+    plan->use = false;
     return FLSTM_OK;
 }
 

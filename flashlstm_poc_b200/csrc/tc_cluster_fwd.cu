@@ -465,53 +465,55 @@ bool cluster_enabled() {
 // weights that fit the registers (shared memory for what is left) and the estimated cycles of a step; the cheapest
 // wins.  The terms: 8 cycles per mma and sub-partition or 20 per dependent pair, 4 cycles per 512 B of weights read
 // from shared memory, the exchange as measured (tc_cluster.cuh), the gate functions per own slot.
-int plan_cluster_fwd(int B, int H, int sms, size_t smem_limit, ClusterFwdPlan *plan, bool check_device) {
+int plan_cluster_fwd(int B, int H, int sms, size_t smem_limit, ClusterFwdPlan *plan, const ClusterCheck *check) {
     *plan = ClusterFwdPlan{};
     if (!cluster_enabled() || H % 64 || H > 768) return FLSTM_OK;
     const char *env = std::getenv("FLSTM_CLUSTER_SIZE");
     const int only = env ? std::atoi(env) : 0;
     const int blocks = H / 8, chunks = H / 32;
-    for (int C = 1; C <= 16; C *= 2) {
-        if (only && C != only) continue;
-        ClusterFwdPlan best{};
-        int slots = cluster_slots(C, sms);
-        for (int pass = 0; pass < 2 && slots > 0; ++pass) {
-            best = ClusterFwdPlan{};
-            for (int ks = 1; ks <= 4 && ks <= chunks; ks *= 2)
-                for (int kr : {8, 6, 5, 4, 3, 2, 1}) {
-                    ClusterFwdPlan pl{};
-                    pl.C = C;
-                    pl.nub = (blocks + C - 1) / C;
-                    pl.peers = (blocks + pl.nub - 1) / pl.nub;
-                    pl.seqs = (B + slots - 1) / slots;
-                    const int tiles = (pl.seqs + 7) / 8, kc = (chunks + ks - 1) / ks;
-                    pl.NT = tiles <= 1 ? 1 : tiles <= 2 ? 2 : 4;
-                    const int warps = pl.nub * ks;
-                    if (tiles > 4 || kr > kc || warps > 16 || warps * 32 > cluster_fwd_max_threads(kr, pl.NT, ks)) continue;
-                    pl.ks = ks;
-                    pl.kr = kr;
-                    pl.nsm = kc - kr;
-                    pl.threads = warps * 32;
-                    pl.smem_bytes = fwd_smem(pl);
-                    if ((size_t)pl.smem_bytes + 1024 > smem_limit) continue;
-                    pl.clusters = (B + pl.seqs - 1) / pl.seqs;
-                    const int busy = (warps + 3) / 4 * kc * pl.NT * 32, chain = kc * 40, own = (2 * pl.NT + ks - 1) / ks;
-                    const int incoming = H * 2 * pl.seqs;
-                    const int exchange = C == 1 ? 600 : 540 + 10 * C + (pl.seqs < kRowSeqs ? incoming / 6 : 250 + incoming / 14);
-                    pl.cycles = (busy > chain ? busy : chain) + warps * pl.nsm * 16 + exchange + 300 + (warps + 3) / 4 * 100 + 200 * own +
-                                (ks > 1 ? 70 + 10 * ks : 0);
-                    pl.use = true;
-                    if (!best.use || pl.cycles < best.cycles) best = pl;
-                }
-            if (!best.use || !check_device) break;
-            const int have = cluster_count(reinterpret_cast<const void *>(fwd_kernel(best.kr, best.NT, best.ks, false, false)), C, best.threads,
-                                           best.smem_bytes);
-            if (have >= best.clusters) break;
-            slots = have;  // fewer clusters run at once than assumed: more sequences for each
-            best.use = false;
+    int slots[5];  // clusters of 1, 2, 4, 8, 16 CTAs that run at once
+    for (int n = 0; n < 5; ++n) slots[n] = cluster_slots(1 << n, sms);
+    for (int tries = 0; tries < 8; ++tries) {
+        *plan = ClusterFwdPlan{};
+        for (int n = 0; n < 5; ++n) {
+            const int C = 1 << n;
+            if ((only && C != only) || slots[n] < 1) continue;
+        for (int ks = 1; ks <= 4 && ks <= chunks; ks *= 2)
+            for (int kr : {8, 6, 5, 4, 3, 2, 1}) {
+                ClusterFwdPlan pl{};
+                pl.C = C;
+                pl.nub = (blocks + C - 1) / C;
+                pl.peers = (blocks + pl.nub - 1) / pl.nub;
+                pl.seqs = (B + slots[n] - 1) / slots[n];
+                const int tiles = (pl.seqs + 7) / 8, kc = (chunks + ks - 1) / ks;
+                pl.NT = tiles <= 1 ? 1 : tiles <= 2 ? 2 : 4;
+                const int warps = pl.nub * ks;
+                if (tiles > 4 || kr > kc || warps > 16 || warps * 32 > cluster_fwd_max_threads(kr, pl.NT, ks)) continue;
+                pl.ks = ks;
+                pl.kr = kr;
+                pl.nsm = kc - kr;
+                pl.threads = warps * 32;
+                pl.smem_bytes = fwd_smem(pl);
+                if ((size_t)pl.smem_bytes + 1024 > smem_limit) continue;
+                pl.clusters = (B + pl.seqs - 1) / pl.seqs;
+                const int busy = (warps + 3) / 4 * kc * pl.NT * 32, chain = kc * 40, own = (2 * pl.NT + ks - 1) / ks;
+                const int incoming = H * 2 * pl.seqs;
+                const int exchange = C == 1 ? 600 : 540 + 10 * C + (pl.seqs < kRowSeqs ? incoming / 6 : 250 + incoming / 14);
+                pl.cycles = (busy > chain ? busy : chain) + warps * pl.nsm * 16 + exchange + 300 + (warps + 3) / 4 * 100 + 200 * own +
+                            (ks > 1 ? 70 + 10 * ks : 0);
+                pl.use = true;
+                if (!plan->use || pl.cycles < plan->cycles) *plan = pl;
+            }
         }
-        if (best.use && (!plan->use || best.cycles < plan->cycles)) *plan = best;
+        if (!plan->use || !check) return FLSTM_OK;
+        // only the winner's occupancy is asked for: a query loads the kernel and takes about a millisecond
+        const int have = cluster_count(reinterpret_cast<const void *>(fwd_kernel(plan->kr, plan->NT, plan->ks, check->bf16, check->accurate)),
+                                       plan->C, plan->threads, plan->smem_bytes);
+        if (have >= plan->clusters) return FLSTM_OK;
+        for (int n = 0; n < 5; ++n)
+            if (plan->C == 1 << n) slots[n] = have;  // fewer run at once than assumed: more sequences for each
     }
+    plan->use = false;
     return FLSTM_OK;
 }
 

@@ -152,15 +152,15 @@ int init(Engine &e) {
     int optin = 0;
     FLSTM_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e.device));
     st->smem_limit = (size_t)optin;
-    void *raw = nullptr;
     const int B = (int)e.cfg.batch, H = (int)e.cfg.hidden_size;
     // Each direction takes the cluster-resident kernel while its estimated step is shorter than the grid-wide ones'.
     // FLSTM_STEP_MIN_BATCH asks for one of the grid-wide schedules by name.
     if (!std::getenv("FLSTM_STEP_MIN_BATCH")) {
-        FLSTM_TRY(plan_cluster_fwd(B, H, st->sms, st->smem_limit, &st->cfwd, true));
+        const ClusterCheck check{e.cfg.dtype == FLSTM_DTYPE_BF16, e.accurate};
+        FLSTM_TRY(plan_cluster_fwd(B, H, st->sms, st->smem_limit, &st->cfwd, &check));
         if (st->cfwd.cycles > grid_fwd_cycles(B)) st->cfwd.use = false;
         if (e.cfg.training) {
-            FLSTM_TRY(plan_cluster_bwd(B, H, st->sms, st->smem_limit, &st->cbwd, true));
+            FLSTM_TRY(plan_cluster_bwd(B, H, st->sms, st->smem_limit, &st->cbwd, &check));
             if (st->cbwd.cycles > kGridBwdCycles) st->cbwd.use = false;
         }
     }
@@ -169,8 +169,7 @@ int init(Engine &e) {
     if (grid_fwd || grid_bwd) FLSTM_TRY(plan_step(B, H, st->sms, st->smem_limit, &st->step));
     if (st->step.use && grid_bwd) {
         const size_t n = e.layers.size() * (size_t)st->step.splits * e.cfg.batch * e.cfg.hidden_size;
-        FLSTM_CUDA_TRY(cudaMalloc(&raw, n * sizeof(float)));
-        st->dh_parts = static_cast<float *>(raw);
+        e.fixed.want(&st->dh_parts, n * sizeof(float));
     }
     if (!st->step.use && grid_fwd) FLSTM_TRY(plan_fwd(B, H, st->sms, st->smem_limit, &st->fwd));
     if (!st->step.use && grid_bwd) FLSTM_TRY(plan_bwd(B, H, st->sms, st->smem_limit, &st->bwd));
@@ -178,28 +177,20 @@ int init(Engine &e) {
         st->dw_floats = (size_t)st->sms * 128 * 128;
         // one per layer where the cross-layer wavefront can run two layers' GEMMs at once
         st->dw_layers = st->step.use ? e.layers.size() : 1;
-        FLSTM_CUDA_TRY(cudaMalloc(&raw, st->dw_layers * st->dw_floats * sizeof(float)));
-        st->dw_parts = static_cast<float *>(raw);
+        e.fixed.want(&st->dw_parts, st->dw_layers * st->dw_floats * sizeof(float));
     }
     st->layers.resize(e.layers.size());
-    FLSTM_CUDA_TRY(cudaMalloc(&raw, 1024 * sizeof(unsigned int)));
-    e.sync_words = static_cast<unsigned int *>(raw);
-    FLSTM_CUDA_TRY(cudaMemset(raw, 0, 1024 * sizeof(unsigned int)));
     // one bias-gradient scratch per layer: with the cross-layer wavefront two layers may reduce at once
-    FLSTM_CUDA_TRY(cudaMalloc(&raw, e.layers.size() * (size_t)simt::column_sum_scratch_floats(4 * e.cfg.hidden_size) * sizeof(float)));
-    e.db_part = static_cast<float *>(raw);
-    FLSTM_CUDA_TRY(cudaMallocHost(&raw, sizeof(unsigned int)));
-    st->err_host = static_cast<unsigned int *>(raw);
-    *st->err_host = 0;
+    if (e.cfg.training) e.fixed.want(&e.db_part, e.layers.size() * (size_t)simt::column_sum_scratch_floats(4 * e.cfg.hidden_size) * sizeof(float));
+    st->err_host = host_word_acquire();
+    if (!st->err_host) return set_error(FLSTM_ERR_CUDA, "pinned allocation failed");
     return FLSTM_OK;
 }
 
 void destroy(Engine &e) {
     TcState *st = state(e);
     if (!st) return;
-    if (st->err_host) cudaFreeHost(st->err_host);
-    if (st->dh_parts) cudaFree(st->dh_parts);
-    if (st->dw_parts) cudaFree(st->dw_parts);
+    host_word_release(st->err_host);
     delete st;
     e.tc_state = nullptr;
 }

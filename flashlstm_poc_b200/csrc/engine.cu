@@ -163,7 +163,16 @@ int Engine::init() {
             simt_scratch_floats = std::min(8 * 4 * H * widest, (size_t)16 << 20);
             fixed.want(&simt_scratch, simt_scratch_floats * sizeof(float));
         }
-        if (simt::persistent_fits(cfg.dtype, B, H, cfg.training != 0, &simt_grid)) {
+        if (cfg.dtype == FLSTM_DTYPE_F32) {
+            int sms = 0, optin = 0;
+            FLSTM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+            FLSTM_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+            FLSTM_TRY(simt::plan_cluster_f32(true, (int)B, (int)H, sms, (size_t)optin, &f32_fwd));
+            if (cfg.training) FLSTM_TRY(simt::plan_cluster_f32(false, (int)B, (int)H, sms, (size_t)optin, &f32_bwd));
+        }
+        const bool rest = !f32_fwd.use || (cfg.training && !f32_bwd.use);
+        if (rest && !simt::persistent_fits(cfg.dtype, B, H, cfg.training != 0, &simt_grid)) simt_grid = 0;
+        if (simt_grid || f32_fwd.use || f32_bwd.use) {
             words = 32 + (size_t)simt::persistent_batch_tiles(B);
             simt_err_host = host_word_acquire();
             if (!simt_err_host) return set_error(FLSTM_ERR_CUDA, "pinned allocation failed");
@@ -437,8 +446,25 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
                                      l.bias, s));
                 ++launches;
                 size_t m1 = timer.mark(s);
-                if (simt_grid) {
-                    FLSTM_TRY(simt_check_error());
+                FLSTM_TRY(simt_check_error());
+                if (f32_fwd.use) {
+                    simt::ClusterF32FwdParams cp{};
+                    cp.w_hh = static_cast<const float *>(l.w_hh);
+                    cp.hs = static_cast<float *>(l.hs);
+                    cp.cs = l.cs;
+                    cp.gates = static_cast<float *>(l.gates);
+                    cp.y = static_cast<float *>(y_out);
+                    cp.err = sync_words;
+                    cp.B = (int)B;
+                    cp.H = (int)H;
+                    cp.t0 = (int)t0;
+                    cp.T = (int)(t1 - t0);
+                    cp.store_gates = cfg.training ? 1 : 0;
+                    cp.wait_ns = wait_limit_ns;
+                    cp.extra_arrivals = selftest_missing_arrivals;
+                    FLSTM_TRY(simt::cluster_f32_forward(f32_fwd, cp, s));
+                    ++launches;
+                } else if (simt_grid) {
                     simt::PersistentFwdParams pp{};
                     pp.w_hh = l.w_hh;
                     pp.hs = l.hs;
@@ -734,12 +760,34 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
         } else {
             float *dc_l = dc_layers + li * slab;  // the carry survives between ranges, one per layer
             size_t m0 = timer.mark(s);
-            if (t1 == T) {
+            FLSTM_TRY(simt_check_error());
+            if (t1 == T && !f32_bwd.use) {
                 if (dcn_l) { FLSTM_TRY(simt::convert(cfg.dtype, dcn_l, FLSTM_DTYPE_F32, dc_l, slab, s)); ++launches; }
                 else FLSTM_CUDA_TRY(cudaMemsetAsync(dc_l, 0, slab * sizeof(float), s));
             }
-            if (simt_grid) {
-                FLSTM_TRY(simt_check_error());
+            if (f32_bwd.use) {
+                simt::ClusterF32BwdParams cp{};
+                cp.w_hh = static_cast<const float *>(l.w_hh);
+                cp.cs = l.cs;
+                cp.gates = static_cast<const float *>(l.gates);
+                cp.dg = static_cast<float *>(l.dg);
+                cp.dy = static_cast<const float *>(dy_l);
+                cp.dhn = static_cast<const float *>(dhn_l);
+                cp.dc_init = static_cast<const float *>(dcn_l);
+                cp.dc = dc_l;
+                cp.dh0 = dh0_l;
+                cp.dc0 = dc0_l;
+                cp.err = sync_words;
+                cp.B = (int)B;
+                cp.H = (int)H;
+                cp.T = (int)T;
+                cp.s0 = (int)(T - t1);
+                cp.s1 = (int)(T - t0) + ((t0 == 0 && (dh0_l || dc0_l)) ? 1 : 0);  // the last range also forms dh0 / dc0
+                cp.wait_ns = wait_limit_ns;
+                cp.extra_arrivals = selftest_missing_arrivals;
+                FLSTM_TRY(simt::cluster_f32_backward(f32_bwd, cp, s));
+                ++launches;
+            } else if (simt_grid) {
                 simt::PersistentBwdParams pp{};
                 pp.w_hh = l.w_hh;
                 pp.cs = l.cs;
@@ -775,7 +823,7 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
             }
             size_t m1 = timer.mark(s), m2 = m1;
             if (t0 == 0) {
-                if (!simt_grid) {
+                if (!simt_grid && !f32_bwd.use) {
                     if (dh0_l) { FLSTM_TRY(simt::final_dh(cfg.dtype, B, H, l.dg, l.w_hh, dh0_l, s)); ++launches; }
                     if (dc0_l) FLSTM_CUDA_TRY(cudaMemcpyAsync(dc0_l, dc_l, slab * sizeof(float), cudaMemcpyDeviceToDevice, s));
                 }

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "flashlstm_b200/engine.h"
+#include "kernels.h"
 
 namespace flstm_b200 {
 
@@ -161,6 +162,7 @@ struct Engine {
     int trace_steps = 0;
     void *tc_state = nullptr;  // tensor-core path: cached tensor maps etc. (tc_engine.cu)
     // CUDA-core path: persistent recurrent kernels when the shape fits (simt_persistent.cu)
+    simt::ClusterF32Plan f32_fwd{}, f32_bwd{};  // fp32: recurrences inside thread-block clusters (simt_cluster.cu)
     int simt_grid = 0;                       // 0: one launch per step
     unsigned int *simt_err_host = nullptr;   // pinned mirror of the error word
     int simt_check_error();

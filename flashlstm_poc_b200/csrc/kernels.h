@@ -80,6 +80,42 @@ int persistent_batch_tiles(size_t B);
 int persistent_forward(int dtype, int grid, PersistentFwdParams p, cudaStream_t s);
 int persistent_backward(int dtype, int grid, PersistentBwdParams p, cudaStream_t s);
 
+// ---- cluster-resident fp32 recurrent kernels (simt_cluster.cu): fp32 storage, H <= 512
+struct ClusterF32Plan {
+    bool use;
+    int C, peers, nub;     // CTAs per cluster, those that own units, units per CTA (a multiple of 4)
+    int seqs, clusters;    // sequences per cluster, clusters
+    int kr, nsm;           // groups of 16 weights per thread in registers / in shared memory
+    int ahead;             // steps the inputs are fetched early
+    int threads, smem_bytes;
+    int cycles;            // estimated cycles per step
+};
+struct ClusterF32FwdParams {
+    const float *w_hh;     // (4H, H), torch row order
+    float *hs, *cs;        // (T+1, B, H)
+    float *gates;          // (T, B, 4H): projection in, activated gates out
+    float *y;              // optional (T, B, H)
+    unsigned int *err;
+    int B, H, t0, T, store_gates;
+    unsigned long long wait_ns;
+    unsigned int extra_arrivals;
+    int C, peers, nub, nsm, seqs, ahead;  // from the plan
+};
+struct ClusterF32BwdParams {
+    const float *w_hh, *cs, *gates;
+    float *dg;
+    const float *dy, *dhn, *dc_init;  // dc_init: gradient of c_n or null
+    float *dc, *dh0, *dc0;
+    unsigned int *err;
+    int B, H, T, s0, s1;
+    unsigned long long wait_ns;
+    unsigned int extra_arrivals;
+    int C, peers, nub, nsm, seqs, ahead;
+};
+int plan_cluster_f32(bool forward, int B, int H, int sms, size_t smem_limit, ClusterF32Plan *plan);
+int cluster_f32_forward(const ClusterF32Plan &plan, ClusterF32FwdParams p, cudaStream_t s);
+int cluster_f32_backward(const ClusterF32Plan &plan, ClusterF32BwdParams p, cudaStream_t s);
+
 // out[n] = sum_r dg[r, n] over R rows (deterministic order)
 int column_sum(int dtype, const void *dg, size_t R, size_t N, float *out, cudaStream_t s);
 

@@ -28,6 +28,7 @@
 // lstm_backward.cu:188-197).  Packed weights are kept across calls while the caller says they have not
 // changed (flstm_v2_set_weight_version); without that promise they are re-packed on every call, as the
 // reference does (lstm_forward.cu:605).
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -263,9 +264,6 @@ int get_context(size_t B, size_t I, size_t H, V2Context **out) {
     } else {
         c = it->second;
     }
-    c->budget = device_budget() + c->device_bytes();  // what is free now plus what this context already holds
-    if (const char *env = std::getenv("FLSTM_V2_DEVICE_BUDGET_BYTES"))
-        if (std::atoll(env) > 0) c->budget = (size_t)std::atoll(env);
     c->last_use = ++g_use_counter;
     *out = c;
     return FLSTM_OK;
@@ -299,17 +297,24 @@ int set_weights_cached(flstm_engine *e, V2Context::Packed &last, const float *w_
     return FLSTM_OK;
 }
 
-// Host tensors move in chunks of whole time steps so that copies overlap the recurrence: about eight
-// chunks per sequence, at least 16 steps each (the reference uses fixed 32-step chunks,
-// flashlstm_v2/src/lstm_forward.cu:515).  FLSTM_STREAM_CHUNK overrides the number of steps.
-size_t chunk_steps(size_t T) {
-    if (const char *env = std::getenv("FLSTM_STREAM_CHUNK")) {
-        const long v = std::atol(env);
-        if (v > 0) return (size_t)v < T ? (size_t)v : T;
-    }
-    size_t n = (T + 7) / 8;
-    if (n < 16) n = 16;
-    return n < T ? n : T;
+// Host tensors move in chunks of whole time steps so that copies overlap the recurrence: about eight chunks per
+// sequence, at least 16 steps and about a megabyte each (the reference uses fixed 32-step chunks,
+// flashlstm_v2/src/lstm_forward.cu:515), the first and the last of long ones a quarter as long: nothing runs while the
+// first chunk arrives or the last one leaves (config H = 1024, B = 64, T = 512: 155 us each with equal chunks).
+// FLSTM_STREAM_CHUNK overrides the number of steps.  Returns the bounds 0 = b[0] < ... < b[n] = T.
+std::vector<size_t> chunk_bounds(size_t T, size_t step_bytes) {
+    size_t n = std::max<size_t>({(T + 7) / 8, 16, ((size_t)1 << 20) / std::max<size_t>(step_bytes, 1)}), edge = 0;
+    const char *env = std::getenv("FLSTM_STREAM_CHUNK");
+    if (env && std::atol(env) > 0) n = (size_t)std::atol(env);
+    else if (n * step_bytes >= ((size_t)4 << 20) && T > 4 * n) edge = n / 4;
+    std::vector<size_t> bounds{0};
+    if (edge) bounds.push_back(edge);
+    const size_t from = edge, to = T - edge;
+    const size_t pieces = edge ? 6 : (to - from + n - 1) / n, len = edge ? (to - from + pieces - 1) / pieces : n;
+    for (size_t t = from + len; t < to; t += len) bounds.push_back(t);
+    if (edge) bounds.push_back(to);
+    bounds.push_back(T);
+    return bounds;
 }
 
 bool is_device_pointer(const void *p) {
@@ -473,15 +478,10 @@ int backward_streaming(V2Context *c, size_t T, size_t R, const __half *x_host, f
     return FLSTM_OK;
 }
 
-int copy_gradients_out(flstm_engine *e, size_t I, size_t H, float *dw_ih, float *dw_hh, float *db_ih, float *db_hh,
+int copy_gradients_out(flstm_engine *e, float *dw_ih, float *dw_hh, float *db_ih, float *db_hh,
                        cudaStream_t sc) {
-    float *g_ih = nullptr, *g_hh = nullptr, *g_b = nullptr;
-    FLSTM_TRY(flstm_engine_grad_ptrs(e, 0, &g_ih, &g_hh, &g_b));
-    FLSTM_CUDA_TRY(cudaMemcpyAsync(dw_ih, g_ih, 4 * H * I * sizeof(float), cudaMemcpyDeviceToDevice, sc));
-    FLSTM_CUDA_TRY(cudaMemcpyAsync(dw_hh, g_hh, 4 * H * H * sizeof(float), cudaMemcpyDeviceToDevice, sc));
-    FLSTM_CUDA_TRY(cudaMemcpyAsync(db_ih, g_b, 4 * H * sizeof(float), cudaMemcpyDeviceToDevice, sc));
-    FLSTM_CUDA_TRY(cudaMemcpyAsync(db_hh, g_b, 4 * H * sizeof(float), cudaMemcpyDeviceToDevice, sc));
-    return FLSTM_OK;
+    float *const out[4] = {dw_ih, dw_hh, db_ih, db_hh};
+    return flstm_engine_export_grads(e, out, nullptr, nullptr, nullptr, nullptr, sc);
 }
 
 int sync_three(cudaStream_t sc, cudaStream_t sh, cudaStream_t sd) {
@@ -494,8 +494,13 @@ int sync_three(cudaStream_t sc, cudaStream_t sh, cudaStream_t sd) {
 // Whether this call runs in streaming mode; reserves what the chosen mode needs.  `stateless_backward`: a backward
 // call that cannot use the resident engine's gate cache consumes the caller's checkpoints segment by segment.
 int choose_mode(V2Context *c, size_t T, size_t R, bool stateless_backward, bool *streaming) {
-    const bool over_budget = c->resident_bytes(T, R) > c->budget;
     *streaming = false;
+    // A sequence that the resident buffers already hold needs no look at the free memory (0.1 ms a call).
+    const char *env = std::getenv("FLSTM_V2_DEVICE_BUDGET_BYTES");
+    const bool fixed_budget = env && std::atoll(env) > 0, held = c->engine && T <= c->t_cap && (T + R - 1) / R <= c->chk_cap;
+    if (fixed_budget) c->budget = (size_t)std::atoll(env);
+    else if (!held || stateless_backward) c->budget = device_budget() + c->device_bytes();  // free now + held already
+    const bool over_budget = (fixed_budget || !held) && c->resident_bytes(T, R) > c->budget;
     if (over_budget || stateless_backward) {
         int st = c->reserve_streaming(pick_segment(*c, T, R), R);
         if (st == FLSTM_OK) {
@@ -549,10 +554,11 @@ int forward_impl(size_t T, size_t B, size_t I, size_t H, size_t R, const __half 
     // Chunk pipeline over the caller's three streams: x chunk k+1 travels host->device while chunk k
     // runs (projection GEMM + persistent recurrence over the chunk's steps), and y / checkpoint rows
     // of chunk k travel device->host while chunk k+1 runs.
-    const size_t cs_steps = chunk_steps(T), nchunks = (T + cs_steps - 1) / cs_steps;
+    const std::vector<size_t> bounds = chunk_bounds(T, B * std::max(I, H) * 2);
+    const size_t nchunks = bounds.size() - 1;
     if (!x_on_device) {
         for (size_t k = 0; k < nchunks; ++k) {
-            const size_t t0 = k * cs_steps, t1 = (t0 + cs_steps < T) ? t0 + cs_steps : T;
+            const size_t t0 = bounds[k], t1 = bounds[k + 1];
             FLSTM_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(c->x) + t0 * B * I * 2,
                                            reinterpret_cast<const char *>(x_host) + t0 * B * I * 2, (t1 - t0) * B * I * 2,
                                            cudaMemcpyHostToDevice, sh));
@@ -562,7 +568,7 @@ int forward_impl(size_t T, size_t B, size_t I, size_t H, size_t R, const __half 
         }
     }
     for (size_t k = 0; k < nchunks; ++k) {
-        const size_t t0 = k * cs_steps, t1 = (t0 + cs_steps < T) ? t0 + cs_steps : T;
+        const size_t t0 = bounds[k], t1 = bounds[k + 1];
         cudaEvent_t ev_x, ev_done;
         FLSTM_TRY(c->event(2 * k, &ev_x));
         FLSTM_TRY(c->event(2 * k + 1, &ev_done));
@@ -630,19 +636,20 @@ int backward_impl(size_t T, size_t B, size_t I, size_t H, size_t R, const __half
     if (streaming) {
         int st = backward_streaming(c, T, R, x_host, cache, hd, cd, dy_host, d_hn, d_cn, h0, c0, w_ih, w_hh, b_ih, b_hh, dx_host,
                                     dh0, dc0, sc, sh, sd);
-        if (st == FLSTM_OK) st = copy_gradients_out(c->seg_engine, I, H, dw_ih, dw_hh, db_ih, db_hh, sc);
+        if (st == FLSTM_OK) st = copy_gradients_out(c->seg_engine, dw_ih, dw_hh, db_ih, db_hh, sc);
         int sy = sync_three(sc, sh, sd);
         return st != FLSTM_OK ? st : sy;
     }
     const bool dy_on_device = is_device_pointer(dy_host), dx_on_device = is_device_pointer(dx_host);
     const void *dy_dev = dy_on_device ? (const void *)dy_host : c->dy;
     void *dx_dev = dx_on_device ? (void *)dx_host : c->dx;
-    const size_t cs_steps = chunk_steps(T), nchunks = (T + cs_steps - 1) / cs_steps;
+    const std::vector<size_t> bounds = chunk_bounds(T, B * std::max(I, H) * 2);
+    const size_t nchunks = bounds.size() - 1;
     // dY chunks travel host->device in the order the reverse recurrence consumes them: last chunk first
     if (!dy_on_device) {
         for (size_t r = 0; r < nchunks; ++r) {
             const size_t k = nchunks - 1 - r;
-            const size_t t0 = k * cs_steps, t1 = (t0 + cs_steps < T) ? t0 + cs_steps : T;
+            const size_t t0 = bounds[k], t1 = bounds[k + 1];
             FLSTM_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(c->dy) + t0 * slab * 2,
                                            reinterpret_cast<const char *>(dy_host) + t0 * slab * 2, (t1 - t0) * slab * 2,
                                            cudaMemcpyHostToDevice, sh));
@@ -666,7 +673,7 @@ int backward_impl(size_t T, size_t B, size_t I, size_t H, size_t R, const __half
     // chunk k+1 leaves; the weight / bias gradients are formed over the whole sequence by the last chunk
     for (size_t r = 0; r < nchunks; ++r) {
         const size_t k = nchunks - 1 - r;
-        const size_t t0 = k * cs_steps, t1 = (t0 + cs_steps < T) ? t0 + cs_steps : T;
+        const size_t t0 = bounds[k], t1 = bounds[k + 1];
         cudaEvent_t ev_dy, ev_done;
         FLSTM_TRY(c->event(2 * k, &ev_dy));
         FLSTM_TRY(c->event(2 * k + 1, &ev_done));
@@ -680,7 +687,7 @@ int backward_impl(size_t T, size_t B, size_t I, size_t H, size_t R, const __half
                                            cudaMemcpyDeviceToHost, sd));
         }
     }
-    FLSTM_TRY(copy_gradients_out(c->engine, I, H, dw_ih, dw_hh, db_ih, db_hh, sc));
+    FLSTM_TRY(copy_gradients_out(c->engine, dw_ih, dw_hh, db_ih, db_hh, sc));
     FLSTM_TRY(sync_three(sc, sh, sd));
     c->cache_valid = false;  // a cache is consumed once
     return FLSTM_OK;

@@ -63,7 +63,7 @@ __host__ __device__ inline BwdSmemLayout bwd_smem_layout(int BT, int H, int KS, 
     return l;
 }
 
-template <int BT, int KS, bool W_RESIDENT, bool BF16>
+template <int BT, int KS, bool W_RESIDENT, bool BF16, bool ACCURATE>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_dg, BwdParams p) {
     constexpr int UPO = 64 / KS;            // units this CTA owns after the reduce-scatter
@@ -405,7 +405,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         if (PREFETCH) v = in[k];
                         else load_pair(q, i, v);
                         const float dh = v.dy + dh_in[k];
-                        const float tc = p.accurate ? tanh_sel<true>(v.ct) : tanh_fast(v.ct);
+                        const float tc = tanh_sel<ACCURATE>(v.ct);
                         const float d_o = dh * tc;
                         const float dcv = dc_in[k] + dh * v.go * (1.f - tc * tc);
                         const float dai = dcv * v.gg * v.gi * (1.f - v.gi);
@@ -463,10 +463,10 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 }
 
 // ------------------------------------------------------------------ host side
-template <int BT, int KS, bool RES, bool BF16>
-static int launch_bwd(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes,
+template <int BT, int KS, bool RES, bool BF16, bool ACC>
+static int launch_bwd_one(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes,
                       cudaStream_t s) {
-    auto kern = lstm_bwd_kernel<BT, KS, RES, BF16>;
+    auto kern = lstm_bwd_kernel<BT, KS, RES, BF16, ACC>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -501,9 +501,15 @@ static int launch_bwd(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdPa
     return FLSTM_OK;
 }
 
+template <int BT, int KS, bool RES, bool BF16>
+static int launch_bwd(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes, cudaStream_t s) {
+    return p.accurate ? launch_bwd_one<BT, KS, RES, BF16, true>(tw, tdg, p, grid, smem_bytes, s)
+                      : launch_bwd_one<BT, KS, RES, BF16, false>(tw, tdg, p, grid, smem_bytes, s);
+}
+
 template <int BT, int KS, bool RES>
 static int max_clusters(int smem_bytes, int grid) {
-    auto kern = lstm_bwd_kernel<BT, KS, RES, false>;
+    auto kern = lstm_bwd_kernel<BT, KS, RES, false, false>;
     if (ensure_smem_limit(kern, (size_t)smem_bytes) != cudaSuccess) {
         cudaGetLastError();
         return -1;

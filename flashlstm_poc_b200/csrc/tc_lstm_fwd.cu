@@ -77,7 +77,7 @@ __host__ __device__ inline FwdSmemLayout fwd_smem_layout(int BT, int H, int rt, 
 // Only the leader (rank 0) issues UMMAs; both CTAs' loads are counted on the leader's barriers, its commits
 // signal both CTAs.  Each CTA finds its 64 x BT accumulator in its own tensor memory, sequences [0, BT/2) in lanes
 // 0-63 and [BT/2, BT) in lanes 64-127 (BT/2 columns).  Nothing is multicast.
-template <int BT, bool W_RESIDENT, bool BF16, bool PAIR>
+template <int BT, bool W_RESIDENT, bool BF16, bool PAIR, bool ACCURATE>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_h,
                 const __grid_constant__ CUtensorMap tm_g, FwdParams p) {
@@ -417,16 +417,10 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         const float af = ex[(1 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 1 * 16 + u);
                         const float ag = ex[(2 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 2 * 16 + u);
                         const float ao = ex[(3 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 3 * 16 + u);
-                        float gi, gf, gg, go, c, h;
-                        if (p.accurate) {
-                            gi = sigmoid_sel<true>(ai); gf = sigmoid_sel<true>(af); gg = tanh_sel<true>(ag); go = sigmoid_sel<true>(ao);
-                            c = fmaf(gf, c_prev[i], gi * gg);
-                            h = go * tanh_sel<true>(c);
-                        } else {
-                            gi = sigmoid_fast(ai); gf = sigmoid_fast(af); gg = tanh_fast(ag); go = sigmoid_fast(ao);
-                            c = fmaf(gf, c_prev[i], gi * gg);
-                            h = go * tanh_fast(c);
-                        }
+                        const float gi = sigmoid_sel<ACCURATE>(ai), gf = sigmoid_sel<ACCURATE>(af);
+                        const float gg = tanh_sel<ACCURATE>(ag), go = sigmoid_sel<ACCURATE>(ao);
+                        const float c = fmaf(gf, c_prev[i], gi * gg);
+                        const float h = go * tanh_sel<ACCURATE>(c);
                         c_keep[i] = c;
                         act[i][0] = gi; act[i][1] = gf; act[i][2] = gg; act[i][3] = go;
                         h16[i] = to16<BF16>(h);
@@ -484,10 +478,10 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 }
 
 // ------------------------------------------------------------------ host launcher
-template <int BT, bool RES, bool BF16, bool PAIR>
-static int launch_fwd(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdParams &p, int grid,
+template <int BT, bool RES, bool BF16, bool PAIR, bool ACC>
+static int launch_fwd_one(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdParams &p, int grid,
                       int smem_bytes, cudaStream_t s) {
-    auto kern = lstm_fwd_kernel<BT, RES, BF16, PAIR>;
+    auto kern = lstm_fwd_kernel<BT, RES, BF16, PAIR, ACC>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -506,6 +500,13 @@ static int launch_fwd(const CUtensorMap &tw, const CUtensorMap &th, const CUtens
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, th, tg, p);
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "recurrent forward launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
+}
+
+template <int BT, bool RES, bool BF16, bool PAIR>
+static int launch_fwd(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdParams &p, int grid,
+                      int smem_bytes, cudaStream_t s) {
+    return p.accurate ? launch_fwd_one<BT, RES, BF16, PAIR, true>(tw, th, tg, p, grid, smem_bytes, s)
+                      : launch_fwd_one<BT, RES, BF16, PAIR, false>(tw, th, tg, p, grid, smem_bytes, s);
 }
 
 // FLSTM_FWD_PAIR=0: no CTA pairs in the forward kernel

@@ -159,10 +159,10 @@ class _StreamingLSTMFunction(torch.autograd.Function):
         grad_cy, grad_cy_ptr = state_grad(grad_cy, "grad_cy")
 
         dx_host = _host_like(x_host, tuple(x_host.shape), torch.float16)
-        dw_ih = torch.zeros_like(weight_ih, memory_format=torch.contiguous_format)
-        dw_hh = torch.zeros_like(weight_hh, memory_format=torch.contiguous_format)
-        db_ih = torch.zeros_like(bias_ih, memory_format=torch.contiguous_format)
-        db_hh = torch.zeros_like(bias_hh, memory_format=torch.contiguous_format)
+        # written whole by the native call, which leaves an empty problem alone
+        new = torch.empty_like if T * B * I * H > 0 else torch.zeros_like
+        dw_ih, dw_hh, db_ih, db_hh = (new(p, memory_format=torch.contiguous_format)
+                                      for p in (weight_ih, weight_hh, bias_ih, bias_hh))
         dh0 = torch.empty((B, H), device="cuda", dtype=torch.float32)
         dc0 = torch.empty_like(dh0)
         w_ih, w_hh = weight_ih.detach().contiguous(), weight_hh.detach().contiguous()

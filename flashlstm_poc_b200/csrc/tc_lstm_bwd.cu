@@ -309,6 +309,20 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         else dc_in[k] = (b < p.B) ? p.dc[idx] : 0.f;
                         if (PREFETCH) load_pair(q, i, in[k]);
                     }
+                // dG and the carried dc are linear in dh and dc: everything else is formed ahead of the wait
+                struct Factors {
+                    float dy, ka, ki, kf, kg, ko, gf;
+                };
+                auto factors = [](const PairIn &v) {
+                    const float tc = tanh_sel<ACCURATE>(v.ct);
+                    return Factors{v.dy, v.go * (1.f - tc * tc), v.gg * v.gi * (1.f - v.gi), v.cp * v.gf * (1.f - v.gf),
+                                   v.gi * (1.f - v.gg * v.gg), tc * v.go * (1.f - v.go), v.gf};
+                };
+                Factors fac[PREFETCH ? PAIRS : 1];
+                if (PREFETCH) {
+#pragma unroll
+                    for (int k = 0; k < (PREFETCH ? PAIRS : 1); ++k) fac[k] = factors(in[k]);
+                }
                 // dh contribution from the step above: reduce-scattered partial products
                 float dh_in[PAIRS];
                 if (s == 0) {
@@ -401,18 +415,18 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                             if (p.dc0) p.dc0[idx] = dc_in[k];
                             continue;
                         }
-                        PairIn v;
-                        if (PREFETCH) v = in[k];
-                        else load_pair(q, i, v);
-                        const float dh = v.dy + dh_in[k];
-                        const float tc = tanh_sel<ACCURATE>(v.ct);
-                        const float d_o = dh * tc;
-                        const float dcv = dc_in[k] + dh * v.go * (1.f - tc * tc);
-                        const float dai = dcv * v.gg * v.gi * (1.f - v.gi);
-                        const float daf = dcv * v.cp * v.gf * (1.f - v.gf);
-                        const float dag = dcv * v.gi * (1.f - v.gg * v.gg);
-                        const float dao = d_o * v.go * (1.f - v.go);
-                        const float dcp = dcv * v.gf;
+                        Factors f;
+                        if (PREFETCH) {
+                            f = fac[PREFETCH ? k : 0];
+                        } else {
+                            PairIn v;
+                            load_pair(q, i, v);
+                            f = factors(v);
+                        }
+                        const float dh = f.dy + dh_in[k];
+                        const float dcv = fmaf(dh, f.ka, dc_in[k]);
+                        const float dai = dcv * f.ki, daf = dcv * f.kf, dag = dcv * f.kg, dao = dh * f.ko;
+                        const float dcp = dcv * f.gf;
                         if (keep_dc) dc_keep[k] = dcp;
                         else p.dc[idx] = dcp;
                         uint16_t *drow = dg + ((size_t)t * p.B + b) * G + (size_t)(U >> 4) * 64 + (U & 15);

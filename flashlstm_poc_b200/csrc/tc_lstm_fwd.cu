@@ -354,7 +354,23 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     }
                     // No thread leaves between here and the named barrier below, whatever its waits return: the
                     // barrier ORs the failures, so that all 256 threads go on or give up together.
-                    bool good = mbar_wait(&tfull[buf], (wi >> 1) & 1, abort_w, wait_ns);
+                    // The projection tile landed long before the accumulator: its values go to registers here, off the
+                    // serial chain (they and the result addresses stood behind the barrier before; 3.66 -> see plan_fwd).
+                    bool good = mbar_wait(&pfull[pb], (wi >> 1) & 1, abort_w, wait_ns);
+                    float proj[PAIRS][4];
+                    {
+                        const uint16_t *ptile = reinterpret_cast<const uint16_t *>(s_p + pb * BT * 128) + nb * 64 + u;
+#pragma unroll
+                        for (int i = 0; i < PAIRS; ++i)
+#pragma unroll
+                            for (int g = 0; g < 4; ++g) proj[i][g] = load16<BF16>(ptile + i * 1024 + g * 16);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&pempty[pb]);  // this warp is done with the P tile
+                    const size_t idx0 = (size_t)(b0 + nb) * p.H + j * 16 + u;
+                    uint16_t *h_out = hs + (size_t)(t + 1) * slab + idx0;
+                    const int rows_left = p.B - b0 - nb;
+                    good = mbar_wait(&tfull[buf], (wi >> 1) & 1, abort_w, wait_ns) && good;
                     if (tid == 0) FLSTM_STAMP(tt, 5);
                     tcgen05_fence_after();
                     float *ex = s_ex + (wi & 1) * 64 * EXS;
@@ -400,23 +416,19 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster_relaxed(tempty_c + 8u * (uint32_t)buf);
                     }
-                    if (good) good = mbar_wait(&pfull[pb], (wi >> 1) & 1, abort_w, wait_ns);
                     if (named_barrier_or(1, kFwdEpilogueThreads, !good)) {
                         ok = false;
                         break;
                     }
                     if (tid == 0) FLSTM_STAMP(tt, 6);
                     // phase B: one thread per (unit, sequence) pair does the whole pointwise update
-                    const uint16_t *ptile = reinterpret_cast<const uint16_t *>(s_p + pb * BT * 128);
                     float act[PAIRS][4];
                     uint16_t h16[PAIRS];
+                    const float *exu = ex + u * EXS + nb;
 #pragma unroll
                     for (int i = 0; i < PAIRS; ++i) {
-                        const int nn = nb + 16 * i;
-                        const float ai = ex[(0 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 0 * 16 + u);
-                        const float af = ex[(1 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 1 * 16 + u);
-                        const float ag = ex[(2 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 2 * 16 + u);
-                        const float ao = ex[(3 * 16 + u) * EXS + nn] + load16<BF16>(ptile + nn * 64 + 3 * 16 + u);
+                        const float ai = exu[16 * i] + proj[i][0], af = exu[16 * EXS + 16 * i] + proj[i][1];
+                        const float ag = exu[32 * EXS + 16 * i] + proj[i][2], ao = exu[48 * EXS + 16 * i] + proj[i][3];
                         const float gi = sigmoid_sel<ACCURATE>(ai), gf = sigmoid_sel<ACCURATE>(af);
                         const float gg = tanh_sel<ACCURATE>(ag), go = sigmoid_sel<ACCURATE>(ao);
                         const float c = fmaf(gf, c_prev[i], gi * gg);
@@ -425,10 +437,8 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                         act[i][0] = gi; act[i][1] = gf; act[i][2] = gg; act[i][3] = go;
                         h16[i] = to16<BF16>(h);
                         // h_t first: it is what the other CTAs wait for
-                        if (b0 + nn < p.B) hs[(size_t)(t + 1) * slab + (size_t)(b0 + nn) * p.H + j * 16 + u] = h16[i];
+                        if (16 * i < rows_left) h_out[(size_t)(16 * i) * p.H] = h16[i];
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&pempty[pb]);  // this warp is done with the P tile
                     if (last_item) {
                         if (tid == 0) FLSTM_STAMP(tt, 7);
                         // publish h_t: after the named barrier thread 0's release is cumulative over every epilogue

@@ -330,13 +330,15 @@ int Engine::set_weights(int first, int count, const float *const *params, cudaSt
     } else if (backend == FLSTM_BACKEND_TC) {
         FLSTM_TRY(tc::set_weights(*this, first, count, params, s));
     } else {
+        CopyBatch batch;
         for (int i = 0; i < count; ++i) {
             auto &l = layers[first + i];
-            FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, params[4 * i], cfg.dtype, l.w_ih, 4 * H * l.in_size, s));
-            FLSTM_TRY(simt::convert(FLSTM_DTYPE_F32, params[4 * i + 1], cfg.dtype, l.w_hh, 4 * H * H, s));
+            batch.dense(params[4 * i], FLSTM_DTYPE_F32, l.w_ih, cfg.dtype, 4 * H, l.in_size);
+            batch.dense(params[4 * i + 1], FLSTM_DTYPE_F32, l.w_hh, cfg.dtype, 4 * H, H);
             FLSTM_TRY(simt::bias_sum(params[4 * i + 2], params[4 * i + 3], l.bias, 4 * H, s));
-            launches += 3;
+            ++launches;
         }
+        FLSTM_TRY(batch.run(s, &launches));
     }
     for (int i = 0; i < count; ++i) layers[first + i].weights_set = true;
     return FLSTM_OK;
@@ -832,8 +834,11 @@ int Engine::backward_range(size_t T, size_t t0, size_t t1, const void *dy, const
                                      l.in_size, false, l.dw_ih, l.in_size, nullptr, s, simt_scratch, simt_scratch_floats));
                 FLSTM_TRY(simt::gemm(cfg.dtype, FLSTM_DTYPE_F32, 4 * H, H, T * B, l.dg, 4 * H, false, l.hs, H, false,
                                      l.dw_hh, H, nullptr, s, simt_scratch, simt_scratch_floats));
-                FLSTM_TRY(simt::column_sum(cfg.dtype, l.dg, T * B, 4 * H, l.db, s));
-                launches += 3;
+                if (simt_scratch_floats >= (size_t)simt::column_sum_scratch_floats(4 * H))
+                    FLSTM_TRY(simt::column_sum_two_pass(cfg.dtype, l.dg, T * B, 4 * H, simt_scratch, l.db, 0, s));
+                else
+                    FLSTM_TRY(simt::column_sum(cfg.dtype, l.dg, T * B, 4 * H, l.db, s));
+                launches += 4;
                 m2 = timer.mark(s);
             }
             if (dx_l) {

@@ -47,15 +47,37 @@ __global__ void gather_slabs_kernel(const TI *__restrict__ src, size_t slab, siz
 }
 
 // ---------------------------------------------------------------- tiled fp32-accumulate GEMM
-constexpr int BM = 64, BN = 64, BK = 16;
+// 256 threads, BM x BN output tile, BM/16 x BN/16 sums per thread (in groups of four rows and columns 64 apart, so that the
+// 16-byte reads of shared memory do not conflict), K in blocks of 16 through two shared-memory buffers, the next block on
+// its way to registers meanwhile.  64 x 64 tiles with 4 x 4 sums and one buffer, as before, read shared memory for every
+// second FMA and stood at the barriers: 4096 x 1024 x 256 took 75 us.
+constexpr int BK = 16;
 
-template <typename TAB, typename TC, bool A_KC, bool B_KC>
-__global__ void __launch_bounds__(256)
+// four consecutive elements of an operand tile: K-contiguous (row, k..k+3) or row-contiguous (row..row+3, k)
+template <typename T, bool KC>
+__device__ __forceinline__ void load_quad(const T *__restrict__ X, size_t ld_x, int row, int rows, int k, int K, bool vec, float (&v)[4]) {
+    const T *src = KC ? X + (size_t)row * ld_x + k : X + (size_t)k * ld_x + row;
+    const bool whole = KC ? row < rows && k + 3 < K : k < K && row + 3 < rows;
+    if (vec && whole) {
+        __align__(16) T q[4];
+        if (sizeof(T) == 4) *reinterpret_cast<uint4 *>(q) = *reinterpret_cast<const uint4 *>(src);
+        else *reinterpret_cast<uint2 *>(q) = *reinterpret_cast<const uint2 *>(src);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = ld(q + j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = (KC ? row < rows && k + j < K : k < K && row + j < rows) ? ld(src + j) : 0.f;
+    }
+}
+
+template <typename TAB, typename TC, bool A_KC, bool B_KC, int BM, int BN>
+__global__ void __launch_bounds__(256, 2)
 gemm_kernel(int M, int N, int K_total, const TAB *__restrict__ A, size_t lda, const TAB *__restrict__ B,
             size_t ldb, TC *__restrict__ C, size_t ldc, const float *__restrict__ bias, int k_per_split,
-            size_t c_split_stride) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Bs[BK][BN + 4];
+            size_t c_split_stride, int vec_a, int vec_b) {
+    constexpr int TM = BM / 16, TN = BN / 16, AQ = BM / 64, BQ = BN / 64;  // quads per thread and block
+    __shared__ __align__(16) float As[2][BK][BM + 4];
+    __shared__ __align__(16) float Bs[2][BK][BN + 4];
     const int tid = threadIdx.x;
     const int tx = tid % 16, ty = tid / 16;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -63,53 +85,91 @@ gemm_kernel(int M, int N, int K_total, const TAB *__restrict__ A, size_t lda, co
     const int kz0 = blockIdx.z * k_per_split;
     const int K = (kz0 + k_per_split < K_total) ? kz0 + k_per_split : K_total;
     C += (size_t)blockIdx.z * c_split_stride;
-    float acc[4][4] = {};
-    for (int k0 = kz0; k0 < K; k0 += BK) {
+    float ra[AQ][4], rb[BQ][4];
+    auto place = [&](int e, int R, bool kc, int *r, int *k) {
+        *r = kc ? e >> 2 : e % (R / 4) * 4;
+        *k = kc ? (e & 3) * 4 : e / (R / 4);
+    };
+    auto fetch = [&](int k0) {
+        int r, k;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int e = tid + i * 256;
-            int m, k;
-            if (A_KC) { m = e / BK; k = e % BK; } else { k = e / BM; m = e % BM; }
-            int gm = m0 + m, gk = k0 + k;
-            float v = 0.f;
-            if (gm < M && gk < K) v = A_KC ? ld(A + (size_t)gm * lda + gk) : ld(A + (size_t)gk * lda + gm);
-            As[k][m] = v;
+        for (int i = 0; i < AQ; ++i) {
+            place(tid + i * 256, BM, A_KC, &r, &k);
+            load_quad<TAB, A_KC>(A, lda, m0 + r, M, k0 + k, K, vec_a, ra[i]);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int e = tid + i * 256;
-            int n, k;
-            if (B_KC) { n = e / BK; k = e % BK; } else { k = e / BN; n = e % BN; }
-            int gn = n0 + n, gk = k0 + k;
-            float v = 0.f;
-            if (gn < N && gk < K) v = B_KC ? ld(B + (size_t)gn * ldb + gk) : ld(B + (size_t)gk * ldb + gn);
-            Bs[k][n] = v;
+        for (int i = 0; i < BQ; ++i) {
+            place(tid + i * 256, BN, B_KC, &r, &k);
+            load_quad<TAB, B_KC>(B, ldb, n0 + r, N, k0 + k, K, vec_b, rb[i]);
         }
-        __syncthreads();
+    };
+    auto stage = [&](int buf) {
+        int r, k;
+#pragma unroll
+        for (int i = 0; i < AQ; ++i) {
+            place(tid + i * 256, BM, A_KC, &r, &k);
+            if (A_KC) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) As[buf][k + j][r] = ra[i][j];
+            } else {
+                *reinterpret_cast<float4 *>(&As[buf][k][r]) = make_float4(ra[i][0], ra[i][1], ra[i][2], ra[i][3]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < BQ; ++i) {
+            place(tid + i * 256, BN, B_KC, &r, &k);
+            if (B_KC) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) Bs[buf][k + j][r] = rb[i][j];
+            } else {
+                *reinterpret_cast<float4 *>(&Bs[buf][k][r]) = make_float4(rb[i][0], rb[i][1], rb[i][2], rb[i][3]);
+            }
+        }
+    };
+    float acc[TM][TN] = {};
+    fetch(kz0);
+    stage(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = kz0; k0 < K; k0 += BK, buf ^= 1) {
+        const bool more = k0 + BK < K;
+        if (more) fetch(k0 + BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
-            float a[4], b[4];
+            float a[TM], b[TN];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
+            for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4 *>(a + i) = *reinterpret_cast<const float4 *>(&As[buf][k][i * 16 + ty * 4]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[k][tx * 4 + j];
+            for (int j = 0; j < TN; j += 4) *reinterpret_cast<float4 *>(b + j) = *reinterpret_cast<const float4 *>(&Bs[buf][k][j * 16 + tx * 4]);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
-        __syncthreads();
+        if (more) {
+            stage(buf ^ 1);
+            __syncthreads();
+        }
     }
+    const bool vec_c = sizeof(TC) == 4 && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int gm = m0 + ty * 4 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int gm = m0 + (i / 4) * 64 + ty * 4 + i % 4;
         if (gm >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int gn = n0 + tx * 4 + j;
-            if (gn >= N) continue;
-            float v = acc[i][j] + (bias ? bias[gn] : 0.f);
-            st(C + (size_t)gm * ldc + gn, v);
+        for (int j = 0; j < TN; j += 4) {
+            const int gn = n0 + (j / 4) * 64 + tx * 4;
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = acc[i][j + e] + (bias && gn + e < N ? bias[gn + e] : 0.f);
+            TC *dst = C + (size_t)gm * ldc + gn;
+            if (vec_c && gn + 3 < N) {
+                *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (gn + e < N) st(dst + e, v[e]);
+            }
         }
     }
 }
@@ -338,11 +398,12 @@ __global__ void sum_splits_kernel(const float *__restrict__ parts, int splits, s
     }
 }
 
-template <typename TAB, typename TC>
-int gemm_typed(size_t M, size_t N, size_t K, const TAB *A, size_t lda, bool akc, const TAB *B, size_t ldb,
-               bool bkc, TC *C, size_t ldc, const float *bias, cudaStream_t s, int splits = 1, float *parts = nullptr) {
-    dim3 grid(ceil_div(N, BN), ceil_div(M, BM), splits);
+template <typename TAB, typename TC, int BM, int BN>
+int gemm_tiled(size_t M, size_t N, size_t K, const TAB *A, size_t lda, bool akc, const TAB *B, size_t ldb,
+               bool bkc, TC *C, size_t ldc, const float *bias, cudaStream_t s, int splits, float *parts) {
     const int kper = splits > 1 ? (int)(((K + splits - 1) / splits + BK - 1) / BK * BK) : (int)K;
+    if (splits > 1) splits = (int)((K + kper - 1) / kper);
+    dim3 grid(ceil_div(N, BN), ceil_div(M, BM), splits);
     TC *out = C;
     size_t out_ld = ldc, stride = 0;
     if (splits > 1) {  // partial products go to the scratch buffer (only instantiated for fp32 C)
@@ -350,10 +411,11 @@ int gemm_typed(size_t M, size_t N, size_t K, const TAB *A, size_t lda, bool akc,
         out_ld = N;
         stride = M * N;
     }
-    if (akc && bkc) gemm_kernel<TAB, TC, true, true><<<grid, 256, 0, s>>>((int)M, (int)N, (int)K, A, lda, B, ldb, out, out_ld, bias, kper, stride);
-    else if (akc && !bkc) gemm_kernel<TAB, TC, true, false><<<grid, 256, 0, s>>>((int)M, (int)N, (int)K, A, lda, B, ldb, out, out_ld, bias, kper, stride);
-    else if (!akc && bkc) gemm_kernel<TAB, TC, false, true><<<grid, 256, 0, s>>>((int)M, (int)N, (int)K, A, lda, B, ldb, out, out_ld, bias, kper, stride);
-    else gemm_kernel<TAB, TC, false, false><<<grid, 256, 0, s>>>((int)M, (int)N, (int)K, A, lda, B, ldb, out, out_ld, bias, kper, stride);
+    auto vec = [](const void *p, size_t ld_x) { return ld_x % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & (4 * sizeof(TAB) - 1)) == 0 ? 1 : 0; };
+    auto kern = akc && bkc ? gemm_kernel<TAB, TC, true, true, BM, BN>
+                : akc ? gemm_kernel<TAB, TC, true, false, BM, BN>
+                : bkc ? gemm_kernel<TAB, TC, false, true, BM, BN> : gemm_kernel<TAB, TC, false, false, BM, BN>;
+    kern<<<grid, 256, 0, s>>>((int)M, (int)N, (int)K, A, lda, B, ldb, out, out_ld, bias, kper, stride, vec(A, lda), vec(B, ldb));
     FLSTM_TRY(check_launch("gemm"));
     if (splits > 1) {
         sum_splits_kernel<<<grid_1d(M * N), 256, 0, s>>>(parts, splits, M, N, reinterpret_cast<float *>(C), ldc);
@@ -362,24 +424,34 @@ int gemm_typed(size_t M, size_t N, size_t K, const TAB *A, size_t lda, bool akc,
     return FLSTM_OK;
 }
 
+// The largest tile that still gives about two thirds of the SMs one, splitting long contractions (the weight gradients:
+// fp32 C, no bias, scratch given) along K into partial products that are added in a fixed order.
+template <typename TAB, typename TC>
+int gemm_typed(size_t M, size_t N, size_t K, const TAB *A, size_t lda, bool akc, const TAB *B, size_t ldb, bool bkc, TC *C,
+               size_t ldc, const float *bias, cudaStream_t s, float *scratch, size_t scratch_floats) {
+    auto splits_for = [&](size_t tiles) {
+        size_t n = 1;
+        if (sizeof(TC) == 4 && scratch && !bias && K >= 1024)
+            while (n < 16 && tiles * n * 2 <= 296 && K / (n * 2) >= 256 && n * 2 * M * N <= scratch_floats) n *= 2;
+        return n;
+    };
+    auto tiles = [&](int bm, int bn) { return (size_t)ceil_div(M, bm) * ceil_div(N, bn); };
+    const size_t enough = 100;
+    if (tiles(128, 128) * splits_for(tiles(128, 128)) >= enough)
+        return gemm_tiled<TAB, TC, 128, 128>(M, N, K, A, lda, akc, B, ldb, bkc, C, ldc, bias, s, (int)splits_for(tiles(128, 128)), scratch);
+    if (tiles(128, 64) * splits_for(tiles(128, 64)) >= enough)
+        return gemm_tiled<TAB, TC, 128, 64>(M, N, K, A, lda, akc, B, ldb, bkc, C, ldc, bias, s, (int)splits_for(tiles(128, 64)), scratch);
+    return gemm_tiled<TAB, TC, 64, 64>(M, N, K, A, lda, akc, B, ldb, bkc, C, ldc, bias, s, (int)splits_for(tiles(64, 64)), scratch);
+}
+
 template <typename TAB>
 int gemm_ab(int c_dtype, size_t M, size_t N, size_t K, const TAB *A, size_t lda, bool akc, const TAB *B,
             size_t ldb, bool bkc, void *C, size_t ldc, const float *bias, cudaStream_t s, float *scratch,
             size_t scratch_floats) {
-    if (c_dtype == FLSTM_DTYPE_F32) {
-        // long contractions with few output tiles (the weight gradients): split K over grid.z into the scratch
-        // buffer, then add the partial products in a fixed order
-        int splits = 1;
-        const size_t tiles = (size_t)ceil_div(N, BN) * ceil_div(M, BM);
-        if (scratch && !bias && K >= 1024 && tiles < 148) {
-            while (splits < 8 && tiles * splits * 2 <= 296 && K / (splits * 2) >= 256 &&
-                   (size_t)(splits * 2) * M * N <= scratch_floats)
-                splits *= 2;
-        }
-        return gemm_typed(M, N, K, A, lda, akc, B, ldb, bkc, (float *)C, ldc, bias, s, splits, scratch);
-    }
+    if (c_dtype == FLSTM_DTYPE_F32)
+        return gemm_typed(M, N, K, A, lda, akc, B, ldb, bkc, (float *)C, ldc, bias, s, scratch, scratch_floats);
     // a 16-bit C has the same type as A and B
-    return gemm_typed(M, N, K, A, lda, akc, B, ldb, bkc, (TAB *)C, ldc, bias, s);
+    return gemm_typed(M, N, K, A, lda, akc, B, ldb, bkc, (TAB *)C, ldc, bias, s, nullptr, 0);
 }
 
 }  // namespace

@@ -144,7 +144,8 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // 32-sequence block.  TMA wrote the tiles with the swizzle of their row size: 16-byte chunk j of row r sits at
 // chunk j ^ (r & 7) (128 B rows), j ^ ((r >> 1) & 3) (64 B rows), j ^ ((r >> 2) & 1) (32 B rows).
 // Outputs overwrite the inputs in place (gates over the projection, c_t over c_{t-1}).
-template <bool BF16>
+// ACCURATE: 0 / 1 = fast / accurate gate functions, 2 = as `accurate_gates` says (the branch costs the epilogue time)
+template <bool BF16, int ACCURATE>
 __device__ __forceinline__ void lstm_cell_16(const uint32_t (&acc)[64], uint8_t *sP, uint8_t *sC, uint8_t *sH, int r,
                                              int store_gates, int accurate_gates) {
     uint8_t *prow = sP + r * 128, *crow = sC + r * 64, *hrow = sH + r * 32;
@@ -180,7 +181,7 @@ __device__ __forceinline__ void lstm_cell_16(const uint32_t (&acc)[64], uint8_t 
                 act[0][u] = gi; act[1][u] = gf; act[2][u] = gg; act[3][u] = go;
             }
         };
-        if (accurate_gates) cell(std::true_type{});
+        if (ACCURATE == 1 || (ACCURATE == 2 && accurate_gates)) cell(std::true_type{});
         else cell(std::false_type{});
         *reinterpret_cast<uint4 *>(hrow + ((ub ^ xh) << 4)) =
             make_uint4(pack2<BF16>(hn[0], hn[1]), pack2<BF16>(hn[2], hn[3]), pack2<BF16>(hn[4], hn[5]), pack2<BF16>(hn[6], hn[7]));
@@ -448,7 +449,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     if (!ok) break;
                     ldphase ^= 1u << buf;
                     uint8_t *sP = wb + buf * kEpiPBytes, *sC = wb + 2 * kEpiPBytes + buf * kEpiCBytes;
-                    lstm_cell_16<BF16>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
+                    lstm_cell_16<BF16, 2>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -524,7 +525,7 @@ struct WideFwdArgs {
     unsigned int extra_arrivals;  // self-test of the timeout path: arrivals nobody makes
 };
 
-template <int BN, bool BF16, bool PAIR>
+template <int BN, bool BF16, bool PAIR, bool ACCURATE>
 __global__ void __launch_bounds__(kStepThreads, 1)
 wide_fwd_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                 const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_c,
@@ -770,7 +771,7 @@ wide_fwd_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                     if (!good) continue;
                     ldphase ^= 1u << buf;
                     uint8_t *sP = wb + buf * kEpiPBytes, *sC = wb + 2 * kEpiPBytes + buf * kEpiCBytes;
-                    lstm_cell_16<BF16>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
+                    lstm_cell_16<BF16, ACCURATE ? 1 : 0>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -816,12 +817,12 @@ wide_fwd_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 
 // Pointwise backward of one time step for 4 hidden units of one sequence per thread:
 //   dh = dy_t + sum of the fp32 partial products dG_{t+1} W_hh;  dc, dG_t as in the persistent BPTT kernel.
-template <bool BF16>
+template <bool BF16, bool ACCURATE>
 __global__ void __launch_bounds__(256)
 step_bwd_pointwise_kernel(const uint16_t *__restrict__ gates_t, const float *__restrict__ c_t,
                           const float *__restrict__ c_prev, const uint16_t *__restrict__ dy_t,
                           const float *__restrict__ parts, int nparts, float *__restrict__ dc,
-                          uint16_t *__restrict__ dg_t, int B, int H, int early, int accurate) {
+                          uint16_t *__restrict__ dg_t, int B, int H, int early) {
     const int quads = H >> 2;
     const size_t total = (size_t)B * quads, slab = (size_t)B * H;
     // The split-K GEMM that follows may start its prologue and fetch its first weight blocks while this kernel
@@ -861,7 +862,7 @@ step_bwd_pointwise_kernel(const uint16_t *__restrict__ gates_t, const float *__r
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const float gi = gate[0][u], gf = gate[1][u], gg = gate[2][u], go = gate[3][u];
-            const float tc = accurate ? tanh_sel<true>(ct[u]) : tanh_fast(ct[u]);
+            const float tc = tanh_sel<ACCURATE>(ct[u]);
             const float d_o = dh[u] * tc;
             const float dcu = dcin[u] + dh[u] * go * (1.f - tc * tc);
             da[0][u] = dcu * gg * gi * (1.f - gi);
@@ -1034,7 +1035,7 @@ int lstm_step_forward(int dtype, const StepPlan &plan, const StepFwdMaps &m, con
 template <int BN, bool BF16, bool PAIR>
 static int launch_wide_fwd(const StepFwdMaps &m, const WideFwdArgs &a, int sms, cudaStream_t s) {
     using S = StepShape<BN, EPI_LSTM_FWD, PAIR>;
-    auto kern = wide_fwd_kernel<BN, BF16, PAIR>;
+    auto kern = a.accurate ? wide_fwd_kernel<BN, BF16, PAIR, true> : wide_fwd_kernel<BN, BF16, PAIR, false>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)S::kSmemBytes));
     const int rows = PAIR ? 2 * BM : BM, workers = PAIR ? sms / 2 : sms;
     const int tiles = ((a.M + rows - 1) / rows) * (a.N / BN);
@@ -1111,9 +1112,9 @@ int lstm_step_backward_pointwise(int dtype, const void *gates_t, const float *c_
     if (grid > 148 * 16) grid = 148 * 16;
     const uint16_t *g16 = static_cast<const uint16_t *>(gates_t), *dy16 = static_cast<const uint16_t *>(dy_t);
     uint16_t *dg16 = static_cast<uint16_t *>(dg_t);
-    cudaError_t e = dtype == FLSTM_DTYPE_BF16
-                        ? launch_chained(step_bwd_pointwise_kernel<true>, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0, accurate ? 1 : 0)
-                        : launch_chained(step_bwd_pointwise_kernel<false>, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0, accurate ? 1 : 0);
+    auto kern = dtype == FLSTM_DTYPE_BF16 ? (accurate ? step_bwd_pointwise_kernel<true, true> : step_bwd_pointwise_kernel<true, false>)
+                                          : (accurate ? step_bwd_pointwise_kernel<false, true> : step_bwd_pointwise_kernel<false, false>);
+    cudaError_t e = launch_chained(kern, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0);
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "step pointwise launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
 }

@@ -405,6 +405,11 @@ int Engine::forward_range(size_t T, size_t t0, size_t t1, const void *x, const v
     } else if (fwd_progress != t0) {
         return set_error(FLSTM_ERR_INVALID, "forward ranges must be contiguous and ascending (expected start %zu, got %zu)", fwd_progress, t0);
     }
+    if (t0 == 0 && t1 == T && tc::cell_path(*this, T, x, h0, c0, y, hn, cn)) {
+        FLSTM_TRY(tc::forward_cells(*this, T, x, h0, c0, y, hn, cn, s));
+        fwd_progress = last_T = bwd_progress = T;
+        return FLSTM_OK;
+    }
     CopyBatch batch;
     if (t0 == 0) {
         add_states_in(*this, batch, 0, L, h0, c0);

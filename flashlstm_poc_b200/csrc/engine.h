@@ -230,6 +230,9 @@ int backward_layer(Engine &e, int layer, size_t T, size_t t0, size_t t1, const v
                    cudaEvent_t dx_ready = nullptr);
 // steps per wavefront chunk for a range of n steps; 0 = no cross-layer wavefront for this engine
 size_t wavefront_chunk(const Engine &e, size_t n);
+// whether a T-step inference call runs step by step (tc_cell.cu), and that call
+bool cell_path(const Engine &e, size_t T, const void *x, const void *h0, const void *c0, const void *y, const void *hn, const void *cn);
+int forward_cells(Engine &e, size_t T, const void *x, const void *h0, const void *c0, void *y, void *hn, void *cn, cudaStream_t s);
 }  // namespace tc
 
 // Communicator (comm.cu): NCCL loaded at run time with dlopen.

@@ -361,6 +361,70 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     return FLSTM_OK;
 }
 
+// Inference over a few steps: a launch per layer and step reads the layer's weights once, against projection GEMM, state copies
+// and the weight loads of a persistent kernel, all of which a few steps do not repay.  One call, us, cells / before:
+//   H = 1024, 2 layers, B = 1:  T = 1 23 / 47, T = 4 49 / 66, T = 8 98 / 94;   H = 512, B = 8:  14 / 23, 25 / 29, 49 / 31
+//   H = 4096, B = 8:  T = 1 55 / 80, T = 2 110 / 94;   H = 2048, 2 layers, B = 32:  T = 1 52 / 66, T = 2 104 / 74
+// From the second step on weights that stay in L2 (half of its 126 MB) are what pays; beyond that only T = 1 does.
+// A result that overlaps an input keeps to the other path, which has read all of x, h0 and c0 before it writes any.
+bool cell_path(const Engine &e, size_t T, const void *x, const void *h0, const void *c0, const void *y, const void *hn, const void *cn) {
+    if (e.backend != FLSTM_BACKEND_TC || e.cfg.training || T > 4 || e.cfg.batch > (size_t)kCellBatch || e.trace) return false;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(h0)) & 15) return false;
+    const size_t B = e.cfg.batch, H = e.cfg.hidden_size, states = e.layers.size() * B * H, ces = e.cell_io_f32 ? sizeof(float) : 2;
+    const struct { const void *p; size_t bytes; } in[] = {{x, T * B * e.cfg.input_size * 2}, {h0, states * 2}, {c0, states * ces}},
+                                                  out[] = {{y, T * B * H * 2}, {hn, states * 2}, {cn, states * ces}};
+    for (const auto &o : out)
+        for (const auto &i : in) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(o.p), b = reinterpret_cast<uintptr_t>(i.p);
+            if (a && b && a < b + i.bytes && b < a + o.bytes) return false;
+        }
+    size_t weights = 0;
+    for (const auto &l : e.layers) weights += 8 * H * (l.in_size + H);
+    return T == 1 || weights <= ((size_t)64 << 20);
+}
+
+int forward_cells(Engine &e, size_t T, const void *x, const void *h0, const void *c0, void *y, void *hn, void *cn, cudaStream_t s) {
+    FLSTM_TRY(check_async_error(e));
+    const size_t B = e.cfg.batch, H = e.cfg.hidden_size, slab = B * H, L = e.layers.size();
+    const size_t ces = e.cell_io_f32 ? sizeof(float) : 2;
+    size_t m0 = e.timer.mark(s);
+    for (size_t t = 0; t < T; ++t)
+        for (size_t li = 0; li < L; ++li) {
+            auto &l = e.layers[li];
+            CellParams p{};
+            p.w_ih = l.w_ih;
+            p.w_hh = l.w_hh;
+            p.bias = l.bias;
+            p.x = li == 0 ? byte_ptr(x) + t * B * l.in_size * 2 : byte_ptr(e.layers[li - 1].hs) + (t + 1) * slab * 2;
+            if (t > 0) {
+                p.h_prev = byte_ptr(l.hs) + t * slab * 2;
+                p.c_prev = l.cs + t * slab;
+                p.c_prev_f32 = 1;
+            } else {
+                p.h_prev = h0 ? byte_ptr(h0) + li * slab * 2 : nullptr;
+                p.c_prev = c0 ? byte_ptr(c0) + li * slab * ces : nullptr;
+                p.c_prev_f32 = e.cell_io_f32 ? 1 : 0;
+                p.h_first = l.hs;
+                p.c_first = l.cs;
+            }
+            p.h_out = byte_ptr(l.hs) + (t + 1) * slab * 2;
+            p.c_out = l.cs + (t + 1) * slab;
+            p.y = (li == L - 1 && y) ? byte_ptr(y) + t * slab * 2 : nullptr;
+            if (t == T - 1) {
+                p.hn = hn ? byte_ptr(hn) + li * slab * 2 : nullptr;
+                p.cn = cn ? byte_ptr(cn) + li * slab * ces : nullptr;
+                p.cn_f32 = e.cell_io_f32 ? 1 : 0;
+            }
+            p.B = (int)B;
+            p.I = (int)l.in_size;
+            p.H = (int)H;
+            FLSTM_TRY(lstm_cell_step(e.cfg.dtype, e.accurate, p, s));
+            ++e.launches;
+        }
+    e.timer.span(PH_RECUR_FWD, m0, e.timer.mark(s));
+    return FLSTM_OK;
+}
+
 // Wide-batch BPTT over the steps [t0, t1), descending: per step one pointwise kernel (dG_t, cell-gradient
 // carry) and one split-K GEMM (the fp32 partial sums of dG_t W_hh that step t-1 adds to its dy).
 static int backward_steps(Engine &e, int li, size_t T, size_t t0, size_t t1, const void *dy_l, const void *dhn_l,

@@ -165,6 +165,24 @@ int lstm_step_backward_pointwise(int dtype, const void *gates_t, const float *c_
 int sum_parts(const float *parts, int nparts, size_t n, float *out, cudaStream_t s);
 
 // fp32 (4H, K) torch-ordered rows -> 16-bit tile-interleaved rows; bias likewise (b_ih + b_hh)
+// One time step of one layer in one launch (tc_cell.cu); B <= 32, 16-byte aligned x and h_prev.
+struct CellParams {
+    const void *w_ih, *w_hh;  // 16-bit, rows tile-interleaved: (4H, I), (4H, H)
+    const float *bias;        // (4H), same order
+    const void *x;            // (B, I)
+    const void *h_prev;       // (B, H) or null: zeros
+    const void *c_prev;       // (B, H) fp32 or 16-bit, or null: zeros
+    void *h_out;              // (B, H)
+    float *c_out;             // (B, H)
+    void *y, *hn, *cn;        // optional further copies for the caller
+    void *h_first;            // where the state that enters a sequence is kept, or null
+    float *c_first;
+    int c_prev_f32, cn_f32;
+    int B, I, H;
+};
+constexpr int kCellBatch = 32;
+int lstm_cell_step(int dtype, bool accurate, const CellParams &p, cudaStream_t s);
+
 // One matrix of one layer from fp32 torch order (4H, K) to the 16-bit tile-interleaved order (4Hp, Kp), padding zero;
 // with b_ih / b_hh also the layer's summed bias (4Hp).  One launch packs up to kPackJobs of them.
 struct PackJob {

@@ -355,7 +355,7 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     // No thread leaves between here and the named barrier below, whatever its waits return: the
                     // barrier ORs the failures, so that all 256 threads go on or give up together.
                     // The projection tile landed long before the accumulator: its values go to registers here, off the
-                    // serial chain (they and the result addresses stood behind the barrier before; 3.66 -> see plan_fwd).
+                    // serial chain (they and the result addresses stood behind the barrier before; H = 1024, B = 64, T = 512: 1825 -> 1783 us).
                     bool good = mbar_wait(&pfull[pb], (wi >> 1) & 1, abort_w, wait_ns);
                     float proj[PAIRS][4];
                     {

@@ -39,6 +39,7 @@ class Engine:
             check(self.lib.flstm_engine_create(ctypes.byref(cfg), ctypes.byref(handle)))
         self._h = handle
         self._saved_x = None
+        self._index = torch.cuda.current_device() if self.device.index is None else self.device.index
 
     def close(self) -> None:
         if getattr(self, "_h", None):
@@ -56,7 +57,11 @@ class Engine:
         return BACKEND_NAMES[self.lib.flstm_engine_backend(self._h)]
 
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return torch.cuda.current_stream(self._index).cuda_stream
+
+    def _accepts(self, t: torch.Tensor, shape: Tuple[int, ...]) -> bool:
+        """The common case of _check_tensor at a fraction of its cost: a call of a few steps is bound by its host work."""
+        return t.dtype is self.torch_dtype and t.shape == shape and t.device == self.device and t.is_contiguous()
 
     def _check_tensor(self, t: torch.Tensor, shape: Tuple[int, ...], name: str, dtype=None) -> torch.Tensor:
         dtype = dtype or self.torch_dtype
@@ -95,14 +100,17 @@ class Engine:
                 want_states: bool = True):
         T = x.shape[0]
         L, B, H = self.layers, self.batch, self.hidden_size
-        x = self._check_tensor(x, (T, B, self.input_size), "x")
-        if h0 is not None:
+        if not self._accepts(x, (T, B, self.input_size)):
+            x = self._check_tensor(x, (T, B, self.input_size), "x")
+        if h0 is not None and not self._accepts(h0, (L, B, H)):
             h0 = self._check_tensor(h0, (L, B, H), "h0")
-        if c0 is not None:
+        if c0 is not None and not self._accepts(c0, (L, B, H)):
             c0 = self._check_tensor(c0, (L, B, H), "c0")
-        y = torch.empty((T, B, H), dtype=self.torch_dtype, device=self.device)
-        hn = torch.empty((L, B, H), dtype=self.torch_dtype, device=self.device) if want_states else None
-        cn = torch.empty((L, B, H), dtype=self.torch_dtype, device=self.device) if want_states else None
+        y = torch.empty_like(x) if self.input_size == H else x.new_empty((T, B, H))
+        hn = cn = None
+        if want_states:  # empty_like is the cheapest of the allocating calls
+            hn = torch.empty_like(h0) if h0 is not None else x.new_empty((L, B, H))
+            cn = torch.empty_like(hn)
         check(self.lib.flstm_engine_forward(self._h, T, x.data_ptr(), _ptr(h0), _ptr(c0), y.data_ptr(), _ptr(hn),
                                             _ptr(cn), self._stream()))
         self._saved_x = x  # re-read by backward for dW_ih

@@ -459,7 +459,7 @@ const BwdShape kBwdShapes[] = {
     FLSTM_CL_ROW(16, 2, 4, 1),   // H = 512, 16 CTAs
     FLSTM_CL_ROW(12, 3, 5, 1),   // H = 576, 15 of 16 CTAs
     FLSTM_CL_ROW(8, 5, 5, 1),    // H = 640, 16 CTAs
-    FLSTM_CL_ROW(12, 4, 6, 1),   // H = 704, 768, 15 / 16 of 16 CTAs
+    FLSTM_CL_ROW(8, 6, 6, 1),    // H = 704, 768, 15 / 16 of 16 CTAs: with 12 warps fewer fragments fit into registers, too many for shared memory
 };
 
 int nt_index(int NT) { return NT == 1 ? 0 : NT == 2 ? 1 : 2; }

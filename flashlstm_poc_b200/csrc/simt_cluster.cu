@@ -42,6 +42,8 @@ __device__ __forceinline__ void ring_wait(int ahead, int younger) {
     }
 }
 
+// floats per row of the forward kernel's staging: the units of a CTA plus two, which spreads 16 rows over the banks
+__host__ __device__ constexpr int f32_out_row(int threads) { return threads / 16 + 2; }
 constexpr int f32_fwd_max_threads(int KR) { return KR <= 4 ? 512 : KR <= 6 ? 384 : 256; }
 constexpr int f32_bwd_max_threads(int UR) { return UR <= 4 ? 512 : UR <= 6 ? 384 : 256; }
 
@@ -71,9 +73,10 @@ __global__ void __launch_bounds__(f32_fwd_max_threads(KR), 1) f32_cluster_fwd_ke
     uint8_t *s_h = smem;                                                    // 2 x [sequence][Kp]
     float4 *s_w = reinterpret_cast<float4 *>(s_h + 2 * h_bytes);            // [warp][nsm][4 gates][32 lanes]
     float *s_send = reinterpret_cast<float *>(s_w + (size_t)warps * p.nsm * 128);  // 2 x [sequence][nub]
-    float *s_p = s_send + 2 * p.seqs * p.nub;                               // [ahead][block][thread] projections
-    float *s_act = s_p + p.ahead * max_blocks * threads;                    // [block][thread] activated gates
-    float *s_c = s_act + max_blocks * threads;                              // [block][thread] cell states
+    float *s_p = s_send + 2 * p.seqs * p.nub;                               // [ahead][block][16 rows][unit] projections
+    const int nw = threads / 16, row = f32_out_row(threads);                // units per CTA with the partly used warp, floats per row
+    float *s_out = s_p + p.ahead * max_blocks * 16 * row;                   // 2 x [block][16 gate rows, 4 cell rows][unit]
+    float *s_c = s_out + 2 * max_blocks * 20 * row;                         // [block][thread] cell states
 
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) mbar_init(&full[i], 1);
@@ -112,36 +115,44 @@ __global__ void __launch_bounds__(f32_fwd_max_threads(KR), 1) f32_cluster_fwd_ke
 
     if (active) {
         const size_t G = (size_t)4 * H, gate_step = (size_t)p.B * G;
-        // this lane's gate of its unit in sequence sq of a block; the state it stores: h, c or y by gate lane 0, 1, 2
-        const size_t first = (size_t)p.t0 * p.B + b0 + sq;
-        float *g_ptr = p.gates + first * G + (size_t)gl * H + u;
-        const float *p_src = g_ptr;
-        float *s_ptr = gl == 0 ? p.hs + slab : gl == 1 ? p.cs + slab : gl == 2 ? p.y : nullptr;
-        if (s_ptr) s_ptr += first * H + u;
         auto mine = [&](int blk) { return real && blk * 4 + sq < nvalid; };
+        // What goes to or comes from global memory moves in rows: thread = unit tid % nw of row (sequence * 4 + gate) tid / nw of a block, so a
+        // warp touches one or two runs of neighbouring floats.  (Each lane fetching and storing its own (unit, sequence, gate) took
+        // 16 sectors per instruction ahead of the next wait; H = 256, B = 32, T = 128: 936 -> 918 us a training step.)
+        // The state a row stores: h, c or y by gate 0, 1, 2.
+        const int fu = tid % nw, frow = tid / nw, fg = frow & 3, fsq = frow >> 2;
+        const size_t first = (size_t)p.t0 * p.B + b0 + fsq;
+        float *g_ptr = p.gates + first * G + (size_t)fg * H + u0 + fu;
+        const float *p_src = g_ptr;
+        float *s_ptr = fg == 0 ? p.hs + slab : fg == 1 ? p.cs + slab : fg == 2 ? p.y : nullptr;
+        if (s_ptr) s_ptr += first * H + u0 + fu;
+        auto moved = [&](int blk) { return fu < own && blk * 4 + fsq < nvalid; };
+        int slot_in = 0, slot = 0;  // of the next fetch, of this step
         auto fetch = [&](int tt) {
             if (tt < p.T)
                 for (int blk = 0; blk < blocks; ++blk)
-                    if (mine(blk)) cp_async_4(s_p + ((tt % p.ahead) * max_blocks + blk) * threads + tid, p_src + (size_t)blk * 4 * G);
+                    if (moved(blk)) cp_async_4(s_p + ((slot_in * max_blocks + blk) * 16 + frow) * row + fu, p_src + (size_t)blk * 4 * G);
             cp_async_commit();
             p_src += gate_step;
+            slot_in = slot_in + 1 == p.ahead ? 0 : slot_in + 1;
         };
         for (int blk = 0; blk < blocks; ++blk)
             s_c[blk * threads + tid] = mine(blk) ? p.cs[(size_t)p.t0 * slab + (size_t)(b0 + blk * 4 + sq) * H + u] : 0.f;
         for (int tt = 0; tt < p.ahead; ++tt) fetch(tt);
+        ring_wait(p.ahead, p.ahead - 1);
+        named_barrier_sync(1, threads);
         const int quads = (own + 3) / 4, pieces = nvalid * quads;
         const uint32_t h_local = smem_u32(s_h), bar_off = smem_u32(full) - h_local;
         const int e_seq = lane / quads, e_quad = lane % quads;  // this lane's first piece
         const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
         for (int tt = 0; tt < p.T; ++tt) {
-            ring_wait(p.ahead, p.ahead - 1);
             bool ok = true;
             if (tt > 0) {
                 ok = mbar_wait_cluster(&full[tt & 1], (uint32_t)(tt - 1) >> 1 & 1u, &abort_w, wait_ns);
                 if (ok && tid == 0 && tt + 2 < p.T) mbar_expect_tx(&full[tt & 1], step_bytes);
             }
             ok = __all_sync(0xffffffffu, ok);
-            float *send = s_send + (tt & 1) * p.seqs * p.nub;
+            float *send = s_send + (tt & 1) * p.seqs * p.nub, *out = s_out + (tt & 1) * max_blocks * 20 * row;
             const float *hb = reinterpret_cast<const float *>(s_h + (tt & 1) * h_bytes) + slice * 4;
             for (int blk = 0; blk < blocks; ++blk) {
                 const int ns = nvalid - blk * 4;
@@ -194,7 +205,7 @@ __global__ void __launch_bounds__(f32_fwd_max_threads(KR), 1) f32_cluster_fwd_ke
                 const float y1 = (b1 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, b1 ? v[1] : v[3], 2);
                 const float sum = (b0s ? y1 : y0) + __shfl_xor_sync(0xffffffffu, b0s ? y0 : y1, 1);
                 const bool ours = mine(blk);
-                const float a = ours ? sum + s_p[((tt % p.ahead) * max_blocks + blk) * threads + tid] : 0.f;
+                const float a = ours ? sum + s_p[((slot * max_blocks + blk) * 16 + sq * 4 + gl) * row + ul] : 0.f;
                 const float act = gl == 2 ? tanh_acc(a) : sigmoid_acc(a);
                 const int base = lane & 19;  // unit and sequence of this lane, gate 0
                 const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 4);
@@ -202,9 +213,11 @@ __global__ void __launch_bounds__(f32_fwd_max_threads(KR), 1) f32_cluster_fwd_ke
                 const float c = fmaf(gf, s_c[blk * threads + tid], gi * gg);
                 const float h = go * tanh_acc(c);
                 s_c[blk * threads + tid] = c;
-                s_act[blk * threads + tid] = act;
+                out[(blk * 20 + sq * 4 + gl) * row + ul] = act;
+                if (gl == 1) out[(blk * 20 + 16 + sq) * row + ul] = c;
                 if (ours && gl == 0) send[(blk * 4 + sq) * p.nub + ul] = h;
             }
+            ring_wait(p.ahead, p.ahead - 2);  // the projections of the next step; the barrier shows them to the other threads
             if (named_barrier_or(1, threads, !ok)) break;
             if (tt + 1 < p.T) {
                 const uint32_t to = (uint32_t)(((tt + 1) & 1) * h_bytes) + (uint32_t)u0 * 4u, bar = bar_off + ((tt + 1) & 1) * 8u;
@@ -223,10 +236,12 @@ __global__ void __launch_bounds__(f32_fwd_max_threads(KR), 1) f32_cluster_fwd_ke
             }
             // everything nobody waits for
             for (int blk = 0; blk < blocks; ++blk)
-                if (mine(blk)) {
-                    if (p.store_gates) g_ptr[(size_t)blk * 4 * G] = s_act[blk * threads + tid];
-                    if (s_ptr) s_ptr[(size_t)blk * 4 * H] = gl == 1 ? s_c[blk * threads + tid] : send[(blk * 4 + sq) * p.nub + ul];
+                if (moved(blk)) {
+                    if (p.store_gates) g_ptr[(size_t)blk * 4 * G] = out[(blk * 20 + frow) * row + fu];
+                    if (s_ptr)
+                        s_ptr[(size_t)blk * 4 * H] = fg == 1 ? out[(blk * 20 + 16 + fsq) * row + fu] : send[(blk * 4 + fsq) * p.nub + fu];
                 }
+            slot = slot + 1 == p.ahead ? 0 : slot + 1;
             g_ptr += gate_step;
             if (s_ptr) s_ptr += slab;
             fetch(tt + p.ahead);
@@ -529,7 +544,7 @@ bool fill(ClusterF32Plan &pl, bool forward, int need, size_t smem_limit) {
             pl.ahead = ahead;
             const size_t weights = (size_t)pl.threads / 32 * pl.nsm * 2048;
             const size_t bytes = forward ? 2 * (size_t)pl.seqs * need * 256 + weights + 2 * (size_t)pl.seqs * pl.nub * 4 +
-                                               (size_t)(ahead + 2) * blocks * pl.threads * 4
+                                               (size_t)blocks * ((16 * ahead + 40) * f32_out_row(pl.threads) + pl.threads) * 4
                                          : 2 * (size_t)pl.peers * pl.seqs * pl.nub * 4 + 2 * (size_t)pl.seqs * pl.nub * 16 +
                                                (size_t)(ahead + 1) * pl.seqs * pl.nub * 32 + (size_t)pl.seqs * pl.nub * 16 + weights;
             pl.smem_bytes = (int)bytes;

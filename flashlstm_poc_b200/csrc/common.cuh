@@ -80,17 +80,16 @@ __device__ __forceinline__ float tanh_fast(float a) {
 __device__ __forceinline__ float sigmoid_fast(float a) { return fmaf(0.5f, tanh_fast(0.5f * a), 0.5f); }
 
 // 16-bit shapes that the tensor-core path cannot tile ran in the CUDA-core kernels with expf / tanhf; padded onto the
-// tensor-core path (engine_padded.cu) their gate functions keep an error far below a 16-bit rounding step (about 1e-7
-// absolute), the ACCURATE form here.
+// tensor-core path (engine_padded.cu) they keep those functions, the ACCURATE form here.  A quotient of __expf stands in
+// for tanhf only as long as nobody looks near zero: (1 - e) / (1 + e) is off by 6e-8 absolute, a whole fp16 rounding step
+// of a result below 1e-4.
 template <bool ACCURATE>
 __device__ __forceinline__ float sigmoid_sel(float a) {
-    return ACCURATE ? __fdividef(1.f, 1.f + __expf(-a)) : sigmoid_fast(a);
+    return ACCURATE ? sigmoid_acc(a) : sigmoid_fast(a);
 }
 template <bool ACCURATE>
 __device__ __forceinline__ float tanh_sel(float a) {
-    if (!ACCURATE) return tanh_fast(a);
-    const float e = __expf(-2.f * fabsf(a));
-    return copysignf(__fdividef(1.f - e, 1.f + e), a);
+    return ACCURATE ? tanh_acc(a) : tanh_fast(a);
 }
 
 inline int ceil_div(size_t a, size_t b) { return static_cast<int>((a + b - 1) / b); }

@@ -67,3 +67,29 @@ def test_padded_ranges_and_unaligned_tensors():
         assert torch.equal(a, b)
     assert torch.equal(cells, eng.cell_states(1, T))  # the logical copy follows the later calls
     eng.close()
+
+
+@pytest.mark.parametrize("dtype,B,I,H,training", [
+    ("f16", 9, 8, 70, True), ("bf16", 9, 8, 70, True),  # clusters
+    ("bf16", 40, 16, 1217, True),                       # grid-wide persistent kernels
+    ("f16", 150, 64, 1270, True),                       # wide batch
+    ("bf16", 5, 8, 70, False),                          # one launch per step
+])
+def test_padded_gate_functions_keep_their_relative_accuracy_near_zero(dtype, B, I, H, training):
+    """Only the cell candidate has a pre-activation, exact in 16 bits and down to 2^-13 (f16) or 2^-20 (bf16), so that
+    c_1 = tanh(a) / 2.  tanhf is good to 2 units in the last place and sigmoid(0) = 1/2 is exact: 2^-22 relative."""
+    dev, td = torch.device("cuda", 0), TORCH_DTYPES[dtype]
+    u = torch.arange(H)
+    low = 13 if dtype == "f16" else 20
+    a = (128 + (37 * u) % 128) / 128 * torch.pow(2.0, -(4 + u % (low - 3)).float()) * torch.where(u % 2 == 0, 1.0, -1.0)
+    w_ih, w_hh, b = torch.zeros(4 * H, I), torch.zeros(4 * H, H), torch.zeros(4 * H)
+    w_ih[2 * H:3 * H, 0] = a * 64
+    x = torch.zeros(1, B, I)
+    x[..., 0] = 1 / 64
+    eng = Engine(dtype, 1, B, I, H, 1, training=training, device=dev)
+    eng.set_weights(0, w_ih.to(dev), w_hh.to(dev), b.to(dev), b.to(dev))
+    eng.forward(x.to(dev, td))
+    got = eng.cell_states(0, 1)[1].double().cpu()
+    eng.close()
+    want = (torch.tanh(a.double()) / 2).expand(B, H)
+    assert float(((got - want) / want).abs().max()) < 2 ** -22

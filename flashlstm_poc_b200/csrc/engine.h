@@ -124,8 +124,7 @@ struct Engine {
     // A 16-bit shape that the tensor-core path cannot tile runs there zero-padded (engine_padded.cu): this engine then
     // only owns the logical gradients and staging tensors, `inner` has the padded sizes and does the work.
     Engine *inner = nullptr;
-    int logical_h = 0, logical_in = 0;  // of an inner engine: the sizes of the parameters it is given (0: its own)
-    bool accurate = false;              // accurate gate functions (see common.cuh)
+    int logical_h = 0, logical_in = 0;  // of an inner engine: the sizes of the parameters it is given (0: not one)
     struct Padding {
         void *x = nullptr, *dy = nullptr, *dx = nullptr;            // (T, B, .) padded, as needed
         void *odd_x = nullptr, *odd_dy = nullptr, *odd_dx = nullptr;  // for callers' tensors off a 16-byte boundary

@@ -1,8 +1,10 @@
 // 16-bit shapes that the tensor-core path cannot tile (hidden size not a multiple of 64 or input width not a multiple of
 // 8) run on it zero-padded: an inner engine has the padded sizes Hp and Ip, this one copies the caller's tensors in and
-// out.  A padded hidden unit has zero weights and bias and starts from zero states, so it stays at c = h = 0 (its gates
-// are sigmoid(0) and tanh(0) = 0) and receives no gradient; padded input columns meet zero weights.  The weights are
-// packed straight into the padded layout.
+// out.  A padded hidden unit starts from zero states and the kernels take its pre-activations and its dh as zero, so it
+// stays at c = h = 0 (its gates are sigmoid(0) and tanh(0) = 0) and passes no gradient on.  Its zero weights alone would
+// not do: one infinite input, which leaves the real units' gates saturated and finite, made it 0 * inf = NaN and from
+// the next step on the whole sequence.  Padded input columns meet zero weights.  The weights are packed straight into
+// the padded layout.
 //
 // Before, such shapes ran in the CUDA-core kernels, one launch per step once W_hh outgrew shared memory: two layers of
 // H = I = 650, B = 20, T = 35 forward + backward took 6.9 ms.
@@ -62,7 +64,6 @@ int Engine::padded_create() {
     inner->backend = FLSTM_BACKEND_TC;
     inner->logical_h = (int)cfg.hidden_size;
     inner->logical_in = (int)cfg.input_size;
-    inner->accurate = true;
     backend = FLSTM_BACKEND_TC;
     const size_t n = cfg.layers * cfg.batch * padded.hidden_size;
     if (padded.hidden_size != cfg.hidden_size) {

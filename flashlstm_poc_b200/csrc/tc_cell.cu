@@ -74,8 +74,9 @@ __global__ void __launch_bounds__(512, 1) cell_step_kernel(const CellParams p) {
         const int n = e >> 3, uu = blockIdx.x * 8 + (e & 7);
         if (n >= p.B) continue;
         const float *v = sums + (n >> 3) * 256 + (e & 7) * 8 + (n & 7);
-        const float gi = sigmoid_sel<ACCURATE>(v[0]), gf = sigmoid_sel<ACCURATE>(v[64]);
-        const float gg = tanh_sel<ACCURATE>(v[128]), go = sigmoid_sel<ACCURATE>(v[192]);
+        const bool pad = ACCURATE && uu >= p.real_units;
+        const float gi = sigmoid_sel<ACCURATE>(pad ? 0.f : v[0]), gf = sigmoid_sel<ACCURATE>(pad ? 0.f : v[64]);
+        const float gg = tanh_sel<ACCURATE>(pad ? 0.f : v[128]), go = sigmoid_sel<ACCURATE>(pad ? 0.f : v[192]);
         const size_t idx = (size_t)n * H + uu;
         const float c_prev = !p.c_prev ? 0.f : p.c_prev_f32 ? static_cast<const float *>(p.c_prev)[idx]
                                                             : load16<BF16>(static_cast<const uint16_t *>(p.c_prev) + idx);
@@ -98,10 +99,10 @@ __global__ void __launch_bounds__(512, 1) cell_step_kernel(const CellParams p) {
 
 }  // namespace
 
-int lstm_cell_step(int dtype, bool accurate, const CellParams &p, cudaStream_t s) {
+int lstm_cell_step(int dtype, const CellParams &p, cudaStream_t s) {
     const int NT = p.B <= 8 ? 1 : p.B <= 16 ? 2 : 4, chunks = (p.I + 31) / 32 + p.H / 32;
     const int warps = chunks >= 32 ? 16 : 8;
-    const bool bf16 = dtype == FLSTM_DTYPE_BF16;
+    const bool bf16 = dtype == FLSTM_DTYPE_BF16, accurate = p.real_units > 0;
 #define FLSTM_CELL(NT_) \
     (bf16 ? (accurate ? cell_step_kernel<NT_, true, true> : cell_step_kernel<NT_, true, false>) \
           : (accurate ? cell_step_kernel<NT_, false, true> : cell_step_kernel<NT_, false, false>))

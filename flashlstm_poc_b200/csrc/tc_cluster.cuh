@@ -89,7 +89,7 @@ struct ClusterFwdParams {
     unsigned int *err;
     int T, t0, B, H;
     int store_gates;
-    int accurate;
+    int real_units;  // see FwdParams
     long long *trace;
     int trace_steps;
     unsigned long long wait_ns;
@@ -116,7 +116,7 @@ struct ClusterBwdParams {
     float *dh0, *dc0, *dc;
     unsigned int *err;
     int T, s0, s1, B, H;
-    int accurate;
+    int real_units;  // see FwdParams
     long long *trace;
     int trace_steps;
     unsigned long long wait_ns;

@@ -373,6 +373,11 @@ cluster_bwd_kernel(const ClusterBwdParams p) {
                     dh[k] += (d0 + d1) + (d2 + d3);
                 }
             }
+            if (ACCURATE) {
+#pragma unroll
+                for (int k = 0; k < PP; ++k)
+                    if (u0 + unit_of(k) >= p.real_units) dh[k] = 0.f;
+            }
             if (t < 0) {
                 if (good) {
 #pragma unroll
@@ -544,7 +549,7 @@ int lstm_backward_cluster(int dtype, const ClusterBwdPlan &pl, ClusterBwdParams 
     p.peers = pl.peers;
     p.seqs = pl.seqs;
     p.dy_aligned = reinterpret_cast<uintptr_t>(p.dy) % 16 == 0;
-    return cluster_launch(reinterpret_cast<const void *>(r->kernels[nt_index(pl.NT)][dtype == FLSTM_DTYPE_BF16 ? 1 : 0][p.accurate ? 1 : 0]), pl.C,
+    return cluster_launch(reinterpret_cast<const void *>(r->kernels[nt_index(pl.NT)][dtype == FLSTM_DTYPE_BF16 ? 1 : 0][p.real_units ? 1 : 0]), pl.C,
                           pl.clusters * pl.C, pl.threads, pl.smem_bytes, &p, s, "cluster BPTT");
 }
 

@@ -95,6 +95,7 @@ cluster_fwd_kernel(const ClusterFwdParams p) {
         s_to[e] = (b >> 2) * CHUNK + n * 64 + (b & 3) * 16;
     }
     const int u = ub * 8 + i8;  // this thread's unit
+    const bool pad = ACCURATE && u >= p.real_units;
     auto load_w = [&](int c, int g) {  // 8 consecutive columns of gate row g of the unit
         const int k0 = (kq * KC + c) * 32 + 8 * q;
         if (!active || k0 >= H) return make_uint4(0, 0, 0, 0);
@@ -269,8 +270,10 @@ cluster_fwd_kernel(const ClusterFwdParams p) {
             if (kq < OWNERS) {
 #pragma unroll
                 for (int j = 0; j < OWN; ++j) {
-                    const float gi = sigmoid_sel<ACCURATE>(sum[j].x + proj[j][0]), gf = sigmoid_sel<ACCURATE>(sum[j].y + proj[j][1]);
-                    const float gg = tanh_sel<ACCURATE>(sum[j].z + proj[j][2]), go = sigmoid_sel<ACCURATE>(sum[j].w + proj[j][3]);
+                    const float ai = pad ? 0.f : sum[j].x + proj[j][0], af = pad ? 0.f : sum[j].y + proj[j][1];
+                    const float ag = pad ? 0.f : sum[j].z + proj[j][2], ao = pad ? 0.f : sum[j].w + proj[j][3];
+                    const float gi = sigmoid_sel<ACCURATE>(ai), gf = sigmoid_sel<ACCURATE>(af);
+                    const float gg = tanh_sel<ACCURATE>(ag), go = sigmoid_sel<ACCURATE>(ao);
                     c_keep[j] = fmaf(gf, c_keep[j], gi * gg);
                     const uint16_t h16 = to16<BF16>(go * tanh_sel<ACCURATE>(c_keep[j]));
                     if (mine[j]) reinterpret_cast<uint16_t *>(send + (seq_of(j) * nb + blk) * 16)[i8] = h16;
@@ -525,7 +528,7 @@ int lstm_forward_cluster(int dtype, const ClusterFwdPlan &pl, ClusterFwdParams p
     p.nsm = pl.nsm;
     p.seqs = pl.seqs;
     p.y_aligned = reinterpret_cast<uintptr_t>(p.y) % 16 == 0;
-    FwdKernel kern = fwd_kernel(pl.kr, pl.NT, pl.ks, dtype == FLSTM_DTYPE_BF16, p.accurate != 0);
+    FwdKernel kern = fwd_kernel(pl.kr, pl.NT, pl.ks, dtype == FLSTM_DTYPE_BF16, p.real_units > 0);
     if (!kern) return set_error(FLSTM_ERR_UNSUPPORTED, "no cluster forward kernel for this plan");
     return cluster_launch(reinterpret_cast<const void *>(kern), pl.C, pl.clusters * pl.C, pl.threads, pl.smem_bytes, &p, s,
                           "cluster recurrent forward");

@@ -156,7 +156,7 @@ int init(Engine &e) {
     // Each direction takes the cluster-resident kernel while its estimated step is shorter than the grid-wide ones'.
     // FLSTM_STEP_MIN_BATCH asks for one of the grid-wide schedules by name.
     if (!std::getenv("FLSTM_STEP_MIN_BATCH")) {
-        const ClusterCheck check{e.cfg.dtype == FLSTM_DTYPE_BF16, e.accurate};
+        const ClusterCheck check{e.cfg.dtype == FLSTM_DTYPE_BF16, e.logical_h > 0};
         FLSTM_TRY(plan_cluster_fwd(B, H, st->sms, st->smem_limit, &st->cfwd, &check));
         if (st->cfwd.cycles > grid_fwd_cycles(B)) st->cfwd.use = false;
         if (e.cfg.training) {
@@ -280,7 +280,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         cp.B = (int)B;
         cp.H = (int)H;
         cp.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
-        cp.accurate = e.accurate ? 1 : 0;
+        cp.real_units = e.logical_h;
         cp.trace = (li == 0 && t0 == 0) ? e.trace : nullptr;
         cp.trace_steps = e.trace_steps;
         cp.wait_ns = e.wait_limit_ns;
@@ -309,7 +309,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
             wp.B = (int)B;
             wp.H = (int)H;
             wp.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
-            wp.accurate = e.accurate ? 1 : 0;
+            wp.real_units = e.logical_h;
             wp.wait_ns = e.wait_limit_ns;
             wp.extra_arrivals = e.selftest_missing_arrivals;
             FLSTM_TRY(lstm_wide_forward(e.cfg.dtype, st->step, maps, wp, st->sms, s));
@@ -326,7 +326,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
             sp.B = (int)B;
             sp.H = (int)H;
             sp.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
-            sp.accurate = e.accurate ? 1 : 0;
+            sp.real_units = e.logical_h;
             FLSTM_TRY(lstm_step_forward(e.cfg.dtype, st->step, maps, sp, st->sms, s));
         }
         size_t m2 = e.timer.mark(s);
@@ -348,7 +348,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.B = (int)B;
     p.H = (int)H;
     p.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
-    p.accurate = e.accurate ? 1 : 0;
+    p.real_units = e.logical_h;
     p.trace = (li == 0 && t0 == 0) ? e.trace : nullptr;
     p.trace_steps = e.trace_steps;
     p.wait_ns = e.wait_limit_ns;
@@ -418,7 +418,8 @@ int forward_cells(Engine &e, size_t T, const void *x, const void *h0, const void
             p.B = (int)B;
             p.I = (int)l.in_size;
             p.H = (int)H;
-            FLSTM_TRY(lstm_cell_step(e.cfg.dtype, e.accurate, p, s));
+            p.real_units = e.logical_h;
+            FLSTM_TRY(lstm_cell_step(e.cfg.dtype, p, s));
             ++e.launches;
         }
     e.timer.span(PH_RECUR_FWD, m0, e.timer.mark(s));
@@ -447,7 +448,7 @@ static int backward_steps(Engine &e, int li, size_t T, size_t t0, size_t t1, con
         const int nparts = (step == T - 1) ? 1 : splits;
         FLSTM_TRY(lstm_step_backward_pointwise(e.cfg.dtype, byte_ptr(l.gates) + step * B * 4 * H * es, l.cs + (step + 1) * slab,
                                                l.cs + step * slab, byte_ptr(dy_l) + step * slab * es, parts, nparts, dc,
-                                               byte_ptr(l.dg) + step * B * 4 * H * es, (int)B, (int)H, e.accurate, s));
+                                               byte_ptr(l.dg) + step * B * 4 * H * es, (int)B, (int)H, e.logical_h, s));
         ++e.launches;
         if (step > 0 || dh0_l || !finalize) {  // the product at step 0 is dh0, or the carry into the segment before
             FLSTM_TRY(lstm_step_backward_gemm(e.cfg.dtype, st->step, t.tm_dg3, t.tm_w, (int)step, (int)B, (int)H, parts,
@@ -500,7 +501,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
         cp.dh0 = dh0_l;
         cp.dc0 = dc0_l;
         cp.dc = e.dc_layers + (size_t)li * B * H;
-        cp.accurate = e.accurate ? 1 : 0;
+        cp.real_units = e.logical_h;
         cp.err = err;
         cp.T = (int)T;
         cp.s0 = (int)(T - t1);
@@ -526,7 +527,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.dh0 = dh0_l;
     p.dc0 = dc0_l;
     p.dc = e.dc_layers + (size_t)li * B * H;
-    p.accurate = e.accurate ? 1 : 0;
+    p.real_units = e.logical_h;
     p.trace = (li == 0 && e.trace && t1 == T) ? e.trace + (size_t)e.trace_steps * 16 : nullptr;
     p.trace_steps = e.trace_steps;
     p.counters = e.sync_words + 1;

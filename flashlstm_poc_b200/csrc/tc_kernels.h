@@ -48,7 +48,9 @@ struct FwdParams {
     int T, B, H;          // T = number of steps this launch runs
     int t0;               // first (absolute) time step of this launch; the state of step t0 is in slot t0 of hs/cs
     int store_gates;      // write the activated gates back (the gate cache)
-    int accurate;         // accurate gate functions (see common.cuh)
+    // 0: fast gate functions.  > 0: accurate ones (see common.cuh), and the units from this one on are padding
+    // (engine_padded.cu): their pre-activations count as zero, whatever 0 * inf made of them
+    int real_units;
     long long *trace;     // optional: CTA 0 stamps clock64() at 16 points of each of the first trace_steps steps
     int trace_steps;
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
@@ -90,7 +92,7 @@ struct BwdParams {
     float *dc;            // fp32 (B, H) scratch for the cell-gradient carry (used when nt > 1)
     unsigned int *counters, *exits;  // as in FwdParams
     unsigned int *err;
-    int accurate;         // accurate gate functions (see common.cuh)
+    int real_units;       // as in FwdParams; a padding unit's dh counts as zero
     long long *trace;     // optional per-step clock64() stamps of CTA 0 (see FwdParams)
     int trace_steps;
     int T, B, H;          // T = length of the whole sequence
@@ -127,7 +129,7 @@ struct StepFwdParams {
     int t;            // absolute time step: h_{t-1} / c_{t-1} in slot t of the state tensors, results in slot t+1
     int B, H;
     int store_gates;  // overwrite the projection with the activated gates (the gate cache)
-    int accurate;     // accurate gate functions (see common.cuh)
+    int real_units;   // as in FwdParams
 };
 
 // Tensor maps of the forward step kernel.  Operands: hs (T+1, B, H) as a 3-D map with 1 x 128 x 64 boxes and
@@ -146,7 +148,7 @@ struct WideFwdParams {
     int t0, nsteps;
     int B, H;
     int store_gates;
-    int accurate;
+    int real_units;
     unsigned long long wait_ns;
     unsigned int extra_arrivals;
 };
@@ -161,7 +163,7 @@ int lstm_step_backward_gemm(int dtype, const StepPlan &plan, const CUtensorMap &
                             int B, int H, float *parts, unsigned int *err, int sms, cudaStream_t s);
 // dG_t and the cell-gradient carry from dh = dy_t + sum(parts[0..nparts)), the gate cache and the cell states.
 int lstm_step_backward_pointwise(int dtype, const void *gates_t, const float *c_t, const float *c_prev, const void *dy_t,
-                                 const float *parts, int nparts, float *dc, void *dg_t, int B, int H, bool accurate, cudaStream_t s);
+                                 const float *parts, int nparts, float *dc, void *dg_t, int B, int H, int real_units, cudaStream_t s);
 int sum_parts(const float *parts, int nparts, size_t n, float *out, cudaStream_t s);
 
 // fp32 (4H, K) torch-ordered rows -> 16-bit tile-interleaved rows; bias likewise (b_ih + b_hh)
@@ -179,9 +181,10 @@ struct CellParams {
     float *c_first;
     int c_prev_f32, cn_f32;
     int B, I, H;
+    int real_units;           // as in FwdParams
 };
 constexpr int kCellBatch = 32;
-int lstm_cell_step(int dtype, bool accurate, const CellParams &p, cudaStream_t s);
+int lstm_cell_step(int dtype, const CellParams &p, cudaStream_t s);
 
 // One matrix of one layer from fp32 torch order (4H, K) to the 16-bit tile-interleaved order (4Hp, Kp), padding zero;
 // with b_ih / b_hh also the layer's summed bias (4Hp).  One launch packs up to kPackJobs of them.

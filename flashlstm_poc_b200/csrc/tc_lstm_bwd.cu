@@ -423,7 +423,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                             load_pair(q, i, v);
                             f = factors(v);
                         }
-                        const float dh = f.dy + dh_in[k];
+                        const float dh = ACCURATE && U >= p.real_units ? 0.f : f.dy + dh_in[k];
                         const float dcv = fmaf(dh, f.ka, dc_in[k]);
                         const float dai = dcv * f.ki, daf = dcv * f.kf, dag = dcv * f.kg, dao = dh * f.ko;
                         const float dcp = dcv * f.gf;
@@ -517,7 +517,7 @@ static int launch_bwd_one(const CUtensorMap &tw, const CUtensorMap &tdg, const B
 
 template <int BT, int KS, bool RES, bool BF16>
 static int launch_bwd(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes, cudaStream_t s) {
-    return p.accurate ? launch_bwd_one<BT, KS, RES, BF16, true>(tw, tdg, p, grid, smem_bytes, s)
+    return p.real_units ? launch_bwd_one<BT, KS, RES, BF16, true>(tw, tdg, p, grid, smem_bytes, s)
                       : launch_bwd_one<BT, KS, RES, BF16, false>(tw, tdg, p, grid, smem_bytes, s);
 }
 

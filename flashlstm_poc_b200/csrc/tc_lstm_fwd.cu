@@ -425,12 +425,13 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     float act[PAIRS][4];
                     uint16_t h16[PAIRS];
                     const float *exu = ex + u * EXS + nb;
+                    const bool pad = ACCURATE && j * 16 + u >= p.real_units;
 #pragma unroll
                     for (int i = 0; i < PAIRS; ++i) {
                         const float ai = exu[16 * i] + proj[i][0], af = exu[16 * EXS + 16 * i] + proj[i][1];
                         const float ag = exu[32 * EXS + 16 * i] + proj[i][2], ao = exu[48 * EXS + 16 * i] + proj[i][3];
-                        const float gi = sigmoid_sel<ACCURATE>(ai), gf = sigmoid_sel<ACCURATE>(af);
-                        const float gg = tanh_sel<ACCURATE>(ag), go = sigmoid_sel<ACCURATE>(ao);
+                        const float gi = sigmoid_sel<ACCURATE>(pad ? 0.f : ai), gf = sigmoid_sel<ACCURATE>(pad ? 0.f : af);
+                        const float gg = tanh_sel<ACCURATE>(pad ? 0.f : ag), go = sigmoid_sel<ACCURATE>(pad ? 0.f : ao);
                         const float c = fmaf(gf, c_prev[i], gi * gg);
                         const float h = go * tanh_sel<ACCURATE>(c);
                         c_keep[i] = c;
@@ -515,7 +516,7 @@ static int launch_fwd_one(const CUtensorMap &tw, const CUtensorMap &th, const CU
 template <int BT, bool RES, bool BF16, bool PAIR>
 static int launch_fwd(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdParams &p, int grid,
                       int smem_bytes, cudaStream_t s) {
-    return p.accurate ? launch_fwd_one<BT, RES, BF16, PAIR, true>(tw, th, tg, p, grid, smem_bytes, s)
+    return p.real_units ? launch_fwd_one<BT, RES, BF16, PAIR, true>(tw, th, tg, p, grid, smem_bytes, s)
                       : launch_fwd_one<BT, RES, BF16, PAIR, false>(tw, th, tg, p, grid, smem_bytes, s);
 }
 

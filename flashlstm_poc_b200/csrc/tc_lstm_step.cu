@@ -72,7 +72,7 @@ struct StepArgs {
     int t;             // time step: projection / gate cache and y at slot t, states read at slot t, written at t+1
     int has_y;         // also store h_t into the caller's y
     int store_gates;   // write the activated gates back (the gate cache)
-    int accurate;      // accurate gate functions (see common.cuh)
+    int real_units;    // see FwdParams
     int early;         // fetch the first weight blocks ahead of the previous kernel's completion (FLSTM_PDL_EARLY=0: off)
 };
 
@@ -144,10 +144,11 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // 32-sequence block.  TMA wrote the tiles with the swizzle of their row size: 16-byte chunk j of row r sits at
 // chunk j ^ (r & 7) (128 B rows), j ^ ((r >> 1) & 3) (64 B rows), j ^ ((r >> 2) & 1) (32 B rows).
 // Outputs overwrite the inputs in place (gates over the projection, c_t over c_{t-1}).
-// ACCURATE: 0 / 1 = fast / accurate gate functions, 2 = as `accurate_gates` says (the branch costs the epilogue time)
+// ACCURATE: 0 / 1 = fast / accurate gate functions, 2 = accurate where `real` is not negative (the branch costs the
+// epilogue time).  Accurate: units of the 16 from `real` on are padding (FwdParams::real_units).
 template <bool BF16, int ACCURATE>
 __device__ __forceinline__ void lstm_cell_16(const uint32_t (&acc)[64], uint8_t *sP, uint8_t *sC, uint8_t *sH, int r,
-                                             int store_gates, int accurate_gates) {
+                                             int store_gates, int real) {
     uint8_t *prow = sP + r * 128, *crow = sC + r * 64, *hrow = sH + r * 32;
     const int xp = r & 7, xc = (r >> 1) & 3, xh = (r >> 2) & 1;
 #pragma unroll
@@ -173,15 +174,16 @@ __device__ __forceinline__ void lstm_cell_16(const uint32_t (&acc)[64], uint8_t 
             constexpr bool ACC = decltype(accurate)::value;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const float gi = sigmoid_sel<ACC>(act[0][u]), gf = sigmoid_sel<ACC>(act[1][u]);
-                const float gg = tanh_sel<ACC>(act[2][u]), go = sigmoid_sel<ACC>(act[3][u]);
+                const bool pad = ACC && ub * 8 + u >= real;
+                const float gi = sigmoid_sel<ACC>(pad ? 0.f : act[0][u]), gf = sigmoid_sel<ACC>(pad ? 0.f : act[1][u]);
+                const float gg = tanh_sel<ACC>(pad ? 0.f : act[2][u]), go = sigmoid_sel<ACC>(pad ? 0.f : act[3][u]);
                 const float c = fmaf(gf, cp[u], gi * gg);
                 cn[u] = c;
                 hn[u] = go * tanh_sel<ACC>(c);
                 act[0][u] = gi; act[1][u] = gf; act[2][u] = gg; act[3][u] = go;
             }
         };
-        if (ACCURATE == 1 || (ACCURATE == 2 && accurate_gates)) cell(std::true_type{});
+        if (ACCURATE == 1 || (ACCURATE == 2 && real >= 0)) cell(std::true_type{});
         else cell(std::false_type{});
         *reinterpret_cast<uint4 *>(hrow + ((ub ^ xh) << 4)) =
             make_uint4(pack2<BF16>(hn[0], hn[1]), pack2<BF16>(hn[2], hn[3]), pack2<BF16>(hn[4], hn[5]), pack2<BF16>(hn[6], hn[7]));
@@ -449,7 +451,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     if (!ok) break;
                     ldphase ^= 1u << buf;
                     uint8_t *sP = wb + buf * kEpiPBytes, *sC = wb + 2 * kEpiPBytes + buf * kEpiCBytes;
-                    lstm_cell_16<BF16, 2>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
+                    lstm_cell_16<BF16, 2>(acc, sP, sC, sH, lane, a.store_gates, a.real_units ? max(a.real_units - (col0 >> 2), 0) : -1);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -520,7 +522,7 @@ struct WideFwdArgs {
     uint32_t idesc;
     unsigned int *err;
     unsigned int *counter, *exits;  // step barrier and CTAs that have left, zero between launches (leave_counters)
-    int has_y, store_gates, accurate;
+    int has_y, store_gates, real_units;
     unsigned long long wait_ns;   // limit of every wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path: arrivals nobody makes
 };
@@ -771,7 +773,7 @@ wide_fwd_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                     if (!good) continue;
                     ldphase ^= 1u << buf;
                     uint8_t *sP = wb + buf * kEpiPBytes, *sC = wb + 2 * kEpiPBytes + buf * kEpiCBytes;
-                    lstm_cell_16<BF16, ACCURATE ? 1 : 0>(acc, sP, sC, sH, lane, a.store_gates, a.accurate);
+                    lstm_cell_16<BF16, ACCURATE ? 1 : 0>(acc, sP, sC, sH, lane, a.store_gates, a.real_units - (col0 >> 2));
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -822,7 +824,7 @@ __global__ void __launch_bounds__(256)
 step_bwd_pointwise_kernel(const uint16_t *__restrict__ gates_t, const float *__restrict__ c_t,
                           const float *__restrict__ c_prev, const uint16_t *__restrict__ dy_t,
                           const float *__restrict__ parts, int nparts, float *__restrict__ dc,
-                          uint16_t *__restrict__ dg_t, int B, int H, int early) {
+                          uint16_t *__restrict__ dg_t, int B, int H, int real_units, int early) {
     const int quads = H >> 2;
     const size_t total = (size_t)B * quads, slab = (size_t)B * H;
     // The split-K GEMM that follows may start its prologue and fetch its first weight blocks while this kernel
@@ -857,6 +859,11 @@ step_bwd_pointwise_kernel(const uint16_t *__restrict__ gates_t, const float *__r
         for (int s = 0; s < nparts; ++s) {
             const float4 r = *reinterpret_cast<const float4 *>(parts + (size_t)s * slab + sidx);
             dh[0] += r.x; dh[1] += r.y; dh[2] += r.z; dh[3] += r.w;
+        }
+        if (ACCURATE) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (U0 + u >= real_units) dh[u] = 0.f;
         }
         float da[4][4], dcp[4];
 #pragma unroll
@@ -1020,7 +1027,7 @@ int lstm_step_forward(int dtype, const StepPlan &plan, const StepFwdMaps &m, con
     a.t = p.t;
     a.has_y = m.y ? 1 : 0;
     a.store_gates = p.store_gates;
-    a.accurate = p.accurate;
+    a.real_units = p.real_units;
     const EpilogueMaps em{m.gates, m.cs, m.hs_out, m.y ? m.y : m.hs_out};
     if (plan.bn_fwd == 256)
         return bf16 ? launch_step<256, EPI_LSTM_FWD, false, true>(plan.pair, *m.hs, *m.w, em, a, sms, s)
@@ -1035,7 +1042,7 @@ int lstm_step_forward(int dtype, const StepPlan &plan, const StepFwdMaps &m, con
 template <int BN, bool BF16, bool PAIR>
 static int launch_wide_fwd(const StepFwdMaps &m, const WideFwdArgs &a, int sms, cudaStream_t s) {
     using S = StepShape<BN, EPI_LSTM_FWD, PAIR>;
-    auto kern = a.accurate ? wide_fwd_kernel<BN, BF16, PAIR, true> : wide_fwd_kernel<BN, BF16, PAIR, false>;
+    auto kern = a.real_units ? wide_fwd_kernel<BN, BF16, PAIR, true> : wide_fwd_kernel<BN, BF16, PAIR, false>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)S::kSmemBytes));
     const int rows = PAIR ? 2 * BM : BM, workers = PAIR ? sms / 2 : sms;
     const int tiles = ((a.M + rows - 1) / rows) * (a.N / BN);
@@ -1072,7 +1079,7 @@ int lstm_wide_forward(int dtype, const StepPlan &plan, const StepFwdMaps &m, con
     a.exits = p.exits;
     a.has_y = m.y ? 1 : 0;
     a.store_gates = p.store_gates;
-    a.accurate = p.accurate;
+    a.real_units = p.real_units;
     a.wait_ns = p.wait_ns;
     a.extra_arrivals = p.extra_arrivals;
     if (plan.fwd_pair) {
@@ -1106,15 +1113,15 @@ int lstm_step_backward_gemm(int dtype, const StepPlan &plan, const CUtensorMap &
 }
 
 int lstm_step_backward_pointwise(int dtype, const void *gates_t, const float *c_t, const float *c_prev, const void *dy_t,
-                                 const float *parts, int nparts, float *dc, void *dg_t, int B, int H, bool accurate, cudaStream_t s) {
+                                 const float *parts, int nparts, float *dc, void *dg_t, int B, int H, int real_units, cudaStream_t s) {
     const size_t total = (size_t)B * (H / 4);
     int grid = (int)((total + 255) / 256);
     if (grid > 148 * 16) grid = 148 * 16;
     const uint16_t *g16 = static_cast<const uint16_t *>(gates_t), *dy16 = static_cast<const uint16_t *>(dy_t);
     uint16_t *dg16 = static_cast<uint16_t *>(dg_t);
-    auto kern = dtype == FLSTM_DTYPE_BF16 ? (accurate ? step_bwd_pointwise_kernel<true, true> : step_bwd_pointwise_kernel<true, false>)
-                                          : (accurate ? step_bwd_pointwise_kernel<false, true> : step_bwd_pointwise_kernel<false, false>);
-    cudaError_t e = launch_chained(kern, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, pdl_early_enabled() ? 1 : 0);
+    auto kern = dtype == FLSTM_DTYPE_BF16 ? (real_units ? step_bwd_pointwise_kernel<true, true> : step_bwd_pointwise_kernel<true, false>)
+                                          : (real_units ? step_bwd_pointwise_kernel<false, true> : step_bwd_pointwise_kernel<false, false>);
+    cudaError_t e = launch_chained(kern, grid, 256, 0, s, 1, g16, c_t, c_prev, dy16, parts, nparts, dc, dg16, B, H, real_units, pdl_early_enabled() ? 1 : 0);
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "step pointwise launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
 }

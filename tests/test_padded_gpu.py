@@ -93,3 +93,38 @@ def test_padded_gate_functions_keep_their_relative_accuracy_near_zero(dtype, B, 
     eng.close()
     want = (torch.tanh(a.double()) / 2).expand(B, H)
     assert float(((got - want) / want).abs().max()) < 2 ** -22
+
+
+@pytest.mark.parametrize("dtype,T,B,I,H", [
+    ("f16", 5, 9, 10, 70), ("bf16", 4, 5, 16, 100),  # clusters
+    ("bf16", 4, 40, 16, 1217),                       # grid-wide persistent kernels
+    ("f16", 3, 150, 64, 1270),                       # wide batch
+])
+@pytest.mark.parametrize("training", [True, False])
+def test_an_infinite_input_stays_out_of_the_padding(dtype, T, B, I, H, training):
+    """An infinite x or h0 saturates the real units' gates, which leaves every result finite; a padding unit must not make
+    NaN of it (0 * inf) and hand that to the next step.  An infinite dy makes its own row's dG infinite, and nothing else."""
+    if not training:
+        T = min(T, 4)  # with B <= 32 one launch per step
+    w = Workload("t", dtype, 1, I, H, B, T, seed=53, state_std=0.3, training=training)
+    inp = make_inputs(w)
+    inp.x[1, 2, 3], inp.x[0, 4, 1], inp.h0[0, 3, 2] = float("inf"), float("-inf"), float("inf")
+    if not training:
+        inp.dy = None
+    got, eng = run_engine(w, inp)
+    with np.errstate(over="ignore"):
+        ref = run_oracle(inp)
+    keys = ("y", "hn", "cn") + (("dx", "dh0", "dc0") if training else ())
+    assert_parity(got, ref, dtype, keys=keys)
+    if training:
+        inp.dy[T - 1, 1, 0] = float("inf")
+        dev, td = torch.device("cuda", 0), TORCH_DTYPES[dtype]
+        x = inp.x.to(dev, td)
+        eng.forward(x, inp.h0.to(dev, td), inp.c0.to(dev, td))
+        dx, dh0, dc0 = (to_np(t) for t in eng.backward(inp.dy.to(dev, td)))
+        rest = [b for b in range(B) if b != 1]
+        clean = {"dx": dx[:, rest], "dh0": dh0[:, rest], "dc0": dc0[:, rest]}
+        want = {"dx": got["dx"][:, rest], "dh0": got["dh0"][:, rest], "dc0": got["dc0"][:, rest]}
+        for k in clean:
+            assert np.array_equal(clean[k], want[k]), k
+    eng.close()

@@ -187,7 +187,8 @@ int Engine::init() {
         l.dw_hh = l.dw_ih + 4 * H * l.in_size;
         l.db = l.dw_hh + 4 * H * H;
     }
-    return inner ? FLSTM_OK : allocate(cfg.max_seq_len ? cfg.max_seq_len : 1);
+    const size_t cap = cfg.max_seq_len ? cfg.max_seq_len : 1;
+    return inner ? padded_reserve(cap) : allocate(cap);
 }
 
 Engine::~Engine() {

@@ -126,8 +126,7 @@ struct Engine {
     Engine *inner = nullptr;
     int logical_h = 0, logical_in = 0;  // of an inner engine: the sizes of the parameters it is given (0: not one)
     struct Padding {
-        void *x = nullptr, *dy = nullptr, *dx = nullptr;            // (T, B, .) padded, as needed
-        void *odd_x = nullptr, *odd_dy = nullptr, *odd_dx = nullptr;  // for callers' tensors off a 16-byte boundary
+        void *x = nullptr, *dy = nullptr, *dx = nullptr;            // (T, B, .) padded
         void *h0 = nullptr, *dhn = nullptr, *dcn = nullptr;         // (L, B, Hp) engine dtype
         float *c0 = nullptr, *dh0 = nullptr, *dc0 = nullptr;        // (L, B, Hp) fp32
         void *gates = nullptr, *hs = nullptr;                       // logical copies behind flstm_engine_cache_ptrs

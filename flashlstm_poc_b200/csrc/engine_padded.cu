@@ -81,39 +81,27 @@ int Engine::padded_create() {
 }
 
 void Engine::padded_release() {
-    drop(pad.odd_x);
-    drop(pad.odd_dy);
-    drop(pad.odd_dx);
     drop(pad.gates);
     drop(pad.hs);
     drop(pad.cs);
 }
 
-// Staging tensors for sequences of up to T steps.
+// Staging tensors for sequences of up to T steps: for max_seq_len steps when the engine is made, so that a call within it
+// allocates nothing (it may be captured).  A tensor whose width needs no padding has one too: the caller's may start off a
+// 16-byte boundary.
 int Engine::padded_reserve(size_t T) {
     if (T <= pad.t_cap) return FLSTM_OK;
     if (pad.t_cap) FLSTM_CUDA_TRY(cudaDeviceSynchronize());
-    drop(pad.odd_x);
-    drop(pad.odd_dy);
-    drop(pad.odd_dx);
     timed.release();
     pad.t_cap = 0;
     const size_t cap = std::max(T, cfg.max_seq_len), B = cfg.batch;
-    const size_t x_bytes = inner->cfg.input_size != cfg.input_size ? cap * B * inner->cfg.input_size * 2 : 0;
-    const size_t y_bytes = inner->cfg.hidden_size != cfg.hidden_size && cfg.training ? cap * B * inner->cfg.hidden_size * 2 : 0;
+    const size_t x_bytes = cap * B * inner->cfg.input_size * 2, y_bytes = cfg.training ? cap * B * inner->cfg.hidden_size * 2 : 0;
     timed.want(&pad.x, x_bytes);
     timed.want(&pad.dx, cfg.training ? x_bytes : 0);
     timed.want(&pad.dy, y_bytes);
     FLSTM_TRY(timed.commit());
     pad.time_bytes = x_bytes * (cfg.training ? 2 : 1) + y_bytes;
     pad.t_cap = cap;
-    return FLSTM_OK;
-}
-
-// A staging tensor: the padded one, or (same width, but the caller's tensor starts off a 16-byte boundary) one of its own.
-static int staging(void *padded, void **odd, size_t n, size_t *total, void **out) {
-    if (!padded && !*odd) FLSTM_TRY(grab(odd, n, total));
-    *out = padded ? padded : *odd;
     return FLSTM_OK;
 }
 
@@ -130,18 +118,16 @@ int Engine::padded_forward_range(size_t T, size_t t0, size_t t1, const void *x, 
     } else if (in.fwd_progress != t0 || t1 > pad.t_cap) {
         return set_error(FLSTM_ERR_INVALID, "forward ranges must be contiguous and ascending (expected start %zu, got %zu)", in.fwd_progress, t0);
     }
-    void *x_pad = nullptr;
-    if (pad_x) FLSTM_TRY(staging(pad.x, &pad.odd_x, pad.t_cap * B * Ip * es, &pad.time_bytes, &x_pad));
     CopyBatch batch;
     if (pad_x)
-        batch.add(bytes(x) + t0 * B * I * es, dt, I, (int)I, bytes(x_pad) + t0 * B * Ip * es, dt, Ip, (int)Ip, (t1 - t0) * B);
+        batch.add(bytes(x) + t0 * B * I * es, dt, I, (int)I, bytes(pad.x) + t0 * B * Ip * es, dt, Ip, (int)Ip, (t1 - t0) * B);
     if (pad_h && t0 == 0) {
         if (h0) batch.add(h0, dt, H, (int)H, pad.h0, dt, Hp, (int)Hp, L * B);
         if (c0) batch.add(c0, c_dtype, H, (int)H, pad.c0, FLSTM_DTYPE_F32, Hp, (int)Hp, L * B);
     }
     FLSTM_TRY(batch.run(s, &launches));
     in.cell_io_f32 = pad_h || cell_io_f32;
-    FLSTM_TRY(in.forward_range(T, t0, t1, pad_x ? x_pad : x, pad_h && h0 ? pad.h0 : h0, pad_h && c0 ? pad.c0 : c0,
+    FLSTM_TRY(in.forward_range(T, t0, t1, pad_x ? pad.x : x, pad_h && h0 ? pad.h0 : h0, pad_h && c0 ? pad.c0 : c0,
                                pad_y ? nullptr : y, pad_h ? nullptr : hn, pad_h ? nullptr : cn, s));
     if (y && pad_y)
         batch.add(bytes(in.layers.back().hs) + (t0 + 1) * B * Hp * es, dt, Hp, (int)H, bytes(y) + t0 * B * H * es, dt, H, (int)H,
@@ -164,22 +150,19 @@ int Engine::padded_backward_range(size_t T, size_t t0, size_t t1, const void *dy
     const size_t B = cfg.batch, H = cfg.hidden_size, Hp = in.cfg.hidden_size, I = cfg.input_size, Ip = in.cfg.input_size, es = 2;
     if (!dy) return set_error(FLSTM_ERR_INVALID, "dy is null");
     const bool pad_h = Hp != H, pad_dy = pad_h || !aligned16(dy), pad_dx = dx && (Ip != I || !aligned16(dx));
-    void *dy_pad = nullptr, *dx_pad = nullptr;
     CopyBatch batch;
     // the inner engine checks the order of the ranges; a wrong one must not write past the staging tensors
     if (cfg.training && in.last_T == T && t0 < t1 && t1 <= T) {
-        if (pad_dy) FLSTM_TRY(staging(pad.dy, &pad.odd_dy, pad.t_cap * B * Hp * es, &pad.time_bytes, &dy_pad));
-        if (pad_dx) FLSTM_TRY(staging(pad.dx, &pad.odd_dx, pad.t_cap * B * Ip * es, &pad.time_bytes, &dx_pad));
         if (pad_dy)
-            batch.add(bytes(dy) + t0 * B * H * es, dt, H, (int)H, bytes(dy_pad) + t0 * B * Hp * es, dt, Hp, (int)Hp, (t1 - t0) * B);
+            batch.add(bytes(dy) + t0 * B * H * es, dt, H, (int)H, bytes(pad.dy) + t0 * B * Hp * es, dt, Hp, (int)Hp, (t1 - t0) * B);
         if (pad_h && dhn && t1 == T) batch.add(dhn, dt, H, (int)H, pad.dhn, dt, Hp, (int)Hp, L * B);
         if (pad_h && dcn && t1 == T) batch.add(dcn, dt, H, (int)H, pad.dcn, dt, Hp, (int)Hp, L * B);
         FLSTM_TRY(batch.run(s, &launches));
     }
-    FLSTM_TRY(in.backward_range(T, t0, t1, pad_dy ? dy_pad : dy, pad_h && dhn ? pad.dhn : dhn, pad_h && dcn ? pad.dcn : dcn,
-                                pad_dx ? dx_pad : dx, pad_h && dh0 ? pad.dh0 : dh0, pad_h && dc0 ? pad.dc0 : dc0, s));
+    FLSTM_TRY(in.backward_range(T, t0, t1, pad_dy ? pad.dy : dy, pad_h && dhn ? pad.dhn : dhn, pad_h && dcn ? pad.dcn : dcn,
+                                pad_dx ? pad.dx : dx, pad_h && dh0 ? pad.dh0 : dh0, pad_h && dc0 ? pad.dc0 : dc0, s));
     if (pad_dx)
-        batch.add(bytes(dx_pad) + t0 * B * Ip * es, dt, Ip, (int)I, bytes(dx) + t0 * B * I * es, dt, I, (int)I, (t1 - t0) * B);
+        batch.add(bytes(pad.dx) + t0 * B * Ip * es, dt, Ip, (int)I, bytes(dx) + t0 * B * I * es, dt, I, (int)I, (t1 - t0) * B);
     if (t0 == 0) {
         if (pad_h && dh0) batch.add(pad.dh0, FLSTM_DTYPE_F32, Hp, (int)H, dh0, FLSTM_DTYPE_F32, H, (int)H, L * B);
         if (pad_h && dc0) batch.add(pad.dc0, FLSTM_DTYPE_F32, Hp, (int)H, dc0, FLSTM_DTYPE_F32, H, (int)H, L * B);

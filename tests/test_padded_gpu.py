@@ -128,3 +128,62 @@ def test_an_infinite_input_stays_out_of_the_padding(dtype, T, B, I, H, training)
         for k in clean:
             assert np.array_equal(clean[k], want[k]), k
     eng.close()
+
+
+@pytest.mark.parametrize("I,H", [(33, 70), (64, 70), (33, 64)])
+def test_padded_calls_allocate_nothing_and_can_be_captured(I, H):
+    """An engine's workspace is sized for max_seq_len when it is made: neither its first call nor the first one with tensors
+    off a 16-byte boundary allocates, so either may be the one that a stream capture records."""
+    T, B, dev, td = 6, 64, torch.device("cuda", 0), torch.float16
+    w = Workload("t", "f16", 1, I, H, B, T, seed=54, state_std=0.3)
+    inp = make_inputs(w)
+
+    def odd(t):
+        flat = torch.zeros(t.numel() + 1, dtype=t.dtype, device=dev)
+        flat[1:] = t.to(dev).flatten()
+        return flat[1:].view(t.shape)
+
+    x, dy, h0, c0 = (t.to(dev, td) for t in (inp.x, inp.dy, inp.h0, inp.c0))
+    inputs = {"even": (x, dy), "odd": (odd(x), odd(dy))}
+    out = {k: [f(torch.zeros(s, dtype=td, device=dev)) for f, s in ((make, (T, B, H)), (make, (T, B, I)))]
+           for k, make in (("even", lambda t: t), ("odd", odd))}
+    states = [torch.zeros(1, B, H, dtype=t, device=dev) for t in (td, td, torch.float32, torch.float32)]
+    params = [p[0].to(dev) for p in (inp.w_ih, inp.w_hh, inp.b_ih, inp.b_hh)]
+
+    def made():
+        eng = Engine("f16", 1, B, I, H, T, device=dev)
+        eng.set_weights(0, *params)
+        return eng
+
+    def step(eng, kind):
+        (xk, dyk), (y, dx) = inputs[kind], out[kind]
+        eng.forward_into(T, xk, h0, c0, y, states[0], states[1])
+        eng.backward_into(T, dyk, None, None, dx, states[2], states[3])
+
+    eng = made()  # loads the kernels
+    for kind in ("even", "odd"):
+        step(eng, kind)
+    torch.cuda.synchronize()
+    want = [t.clone() for t in (*out["even"], *states, *eng.grads(0))]
+    eng.close()
+    eng = made()
+    torch.cuda.synchronize()
+    held, free = eng.workspace_bytes, torch.cuda.mem_get_info()[0]
+    for kind in ("even", "odd"):
+        step(eng, kind)
+        torch.cuda.synchronize()
+        assert eng.workspace_bytes == held
+        assert torch.cuda.mem_get_info()[0] == free
+    eng.close()
+    eng = made()
+    for t in out["odd"] + states:
+        t.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step(eng, "odd")
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(want, (*out["odd"], *states, *eng.grads(0))):
+        assert torch.equal(a, b)
+    del graph
+    eng.close()

@@ -70,6 +70,7 @@ int Arena::commit() {
     const cudaError_t e = total ? cudaMalloc(&base, total) : cudaSuccess;
     if (e != cudaSuccess) {
         base = nullptr;
+        cudaGetLastError();  // the caller may do with less
         return set_error(FLSTM_ERR_CUDA, "cudaMalloc(%zu bytes) failed: %s", total, cudaGetErrorString(e));
     }
     char *next = static_cast<char *>(base);
@@ -179,7 +180,13 @@ int Engine::init() {
         }
     }
     if (words) fixed.want(&sync_words, words * sizeof(unsigned int));
-    FLSTM_TRY(fixed.commit());
+    int st = fixed.commit();
+    if (st != FLSTM_OK && simt_scratch_floats) {  // the weight-gradient GEMMs then run unsplit
+        fixed.forget(&simt_scratch);
+        simt_scratch_floats = 0;
+        st = fixed.commit();
+    }
+    FLSTM_TRY(st);
     FLSTM_CUDA_TRY(cudaMemset(grads, 0, total * sizeof(float)));
     if (words) FLSTM_CUDA_TRY(cudaMemset(sync_words, 0, words * sizeof(unsigned int)));
     for (auto &l : layers) {

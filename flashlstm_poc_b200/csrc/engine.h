@@ -81,6 +81,11 @@ struct Arena {
     void *base = nullptr;
     template <typename P>
     void want(P **p, size_t bytes) { requests.push_back({reinterpret_cast<void **>(p), bytes}); }
+    template <typename P>
+    void forget(P **p) {  // a request that is not committed
+        for (size_t i = requests.size(); i-- > 0;)
+            if (requests[i].p == reinterpret_cast<void **>(p)) requests.erase(requests.begin() + i);
+    }
     int commit();   // allocates what was asked for since the last commit (at most one allocation at a time)
     void release();
 };

@@ -963,6 +963,11 @@ int flstm_engine_create(const flstm_engine_config *config, flstm_engine **out) {
     int st = FLSTM_OK;
     if (config->backend == FLSTM_BACKEND_AUTO && !tc_ok) st = e.padded_create();
     if (st == FLSTM_OK) st = e.init();
+    if (st != FLSTM_OK && e.inner) {
+        // padding takes up to 64 / hidden_size times the memory: what only fits as it is runs on the CUDA cores
+        e.padded_drop();
+        st = e.init();
+    }
     if (st != FLSTM_OK) {
         delete h;
         return st;

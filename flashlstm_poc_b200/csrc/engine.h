@@ -142,6 +142,7 @@ struct Engine {
     Engine &core() { return inner ? *inner : *this; }
     int padded_create();
     void padded_release();
+    void padded_drop();  // back to the CUDA-core path, before anything has run
     int padded_reserve(size_t T);
     int padded_forward_range(size_t T, size_t t0, size_t t1, const void *x, const void *h0, const void *c0, void *y, void *hn,
                              void *cn, cudaStream_t s);

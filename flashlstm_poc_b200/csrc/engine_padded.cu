@@ -86,6 +86,16 @@ void Engine::padded_release() {
     drop(pad.cs);
 }
 
+void Engine::padded_drop() {
+    padded_release();
+    timed.release();
+    fixed.release();
+    delete inner;
+    inner = nullptr;
+    pad = Padding{};
+    backend = FLSTM_BACKEND_SIMT;
+}
+
 // Staging tensors for sequences of up to T steps: for max_seq_len steps when the engine is made, so that a call within it
 // allocates nothing (it may be captured).  A tensor whose width needs no padding has one too: the caller's may start off a
 // 16-byte boundary.

@@ -187,3 +187,23 @@ def test_padded_calls_allocate_nothing_and_can_be_captured(I, H):
         assert torch.equal(a, b)
     del graph
     eng.close()
+
+
+def test_what_fits_only_unpadded_runs_on_the_cuda_cores():
+    """H = 65 pads to 128 and twice the memory.  Here the padded workspace takes 225 GB, the plain one 114 GB."""
+    B, H, dev, td = 80000, 65, torch.device("cuda", 0), torch.float16
+    torch.cuda.empty_cache()
+    w = Workload("t", "f16", 1, 8, H, 9, 2, seed=55, state_std=0.3)
+    inp = make_inputs(w)
+    want, small = run_engine(w, inp)
+    assert small.backend == "tc"
+    small.close()
+    eng = Engine("f16", 1, B, 8, H, 1000, device=dev)
+    assert eng.backend == "simt"
+    eng.set_weights(0, *(p[0].to(dev) for p in (inp.w_ih, inp.w_hh, inp.b_ih, inp.b_hh)))
+    x, h0, c0 = (torch.zeros(n, B, k, dtype=td, device=dev) for n, k in ((2, 8), (1, H), (1, H)))
+    x[:, :9], h0[:, :9], c0[:, :9] = (t.to(dev, td) for t in (inp.x, inp.h0, inp.c0))
+    y, hn, cn = eng.forward(x, h0, c0)
+    got = {"y": to_np(y[:, :9]), "hn": to_np(hn[:, :9]), "cn": to_np(cn[:, :9])}
+    eng.close()
+    assert_parity(got, want, "f16", keys=("y", "hn", "cn"))

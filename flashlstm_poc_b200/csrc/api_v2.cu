@@ -153,7 +153,8 @@ struct V2Context {
             resident_staging_bytes = T * (2 * B * I * 2 + 2 * slab * 2) + nchk * slab * 8;
             cache_valid = false;
         }
-        return FLSTM_OK;
+        // now, and not inside the call: the checkpoints are gathered from state tensors whose addresses it takes first
+        return engine->impl.reserve(T);
     }
     // Streaming needs the tensor-core backend (segment backward); returns FLSTM_ERR_UNSUPPORTED otherwise.
     int reserve_streaming(size_t S, size_t R) {

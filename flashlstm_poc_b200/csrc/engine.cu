@@ -327,6 +327,12 @@ int Engine::ensure_capacity(size_t T) {
     return allocate(T);
 }
 
+int Engine::reserve(size_t T) {
+    if (!inner) return ensure_capacity(T);
+    FLSTM_TRY(padded_reserve(T));
+    return inner->ensure_capacity(T);
+}
+
 int Engine::set_weights(int first, int count, const float *const *params, cudaStream_t s) {
     if (first < 0 || count < 1 || first + count > (int)layers.size())
         return set_error(FLSTM_ERR_INVALID, "layer %d out of range", count == 1 ? first : first + count - 1);

@@ -187,6 +187,7 @@ struct Engine {
     int allocate(size_t t_cap);
     void release_time_buffers();
     int ensure_capacity(size_t T);
+    int reserve(size_t T);  // the same, padded or not; buffers handed out before (cache_ptrs) are gone when they grow
     int init();  // workspace, plans and backend state for cfg / backend / device
     // parameters of layers [first, first + count): w_ih, w_hh, b_ih, b_hh of each
     int set_weights(int first, int count, const float *const *params, cudaStream_t s);

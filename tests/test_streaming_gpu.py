@@ -18,7 +18,7 @@ from flashlstm_poc_b200.engine import TORCH_DTYPES, Engine
 from flashlstm_poc_b200.workloads import Workload, make_inputs
 from oracle import lstm_oracle as orc
 from tests.gpu_helpers import assert_parity, run_oracle
-from tests.helpers import to_np
+from tests.helpers import params_from_inputs, to_np
 
 pytestmark = pytest.mark.gpu
 
@@ -131,3 +131,25 @@ def test_v2_surface_streams_when_the_sequence_exceeds_the_device_budget(R, monke
         for e in range(1, (T + R - 1) // R):
             assert orc.rel_l2_err(got["ch"][e], y_ref[e * R - 1].detach().numpy()) < 1e-2
     assert footprints[0] == footprints[1] and 0 < footprints[0] <= (6 << 20)
+
+
+@pytest.mark.parametrize("I,H", [(64, 128), (33, 70)])
+def test_v2_checkpoints_of_a_longer_sequence_after_a_shorter_one(I, H):
+    """The resident engine grows with the second call; the checkpoints come from its new state tensors."""
+    lib, B, R = _lib.load(), 6, 4
+    for T in (9, 75):
+        w = Workload("stream", "f16", 1, I, H, B, T, seed=22, state_std=0.3)
+        inp = make_inputs(w)
+        lstm = torch.nn.LSTM(I, H)
+        with torch.no_grad():
+            for p, v in zip(lstm.parameters(), (inp.w_ih[0], inp.w_hh[0], inp.b_ih[0], inp.b_hh[0])):
+                p.copy_(v)
+        x, dy = inp.x.half().pin_memory(), inp.dy.half().pin_memory()
+        got, _, streaming = _v2_step(lib, T, B, I, H, R, lstm, x, inp.h0[0].half(), inp.c0[0].half(), dy, False)
+        assert streaming == 0
+        ref = run_oracle(inp)
+        for k in ("y", "dx"):
+            assert orc.rel_l2_err(got[k], ref[k]) < 1e-2, (T, k)
+        fwd = orc.lstm_forward(inp.x.numpy(), params_from_inputs(inp), inp.h0.numpy(), inp.c0.numpy(), dtype=np.float32)
+        for k, states in (("ch", fwd.caches[0].h_s), ("cc", fwd.caches[0].c_s)):
+            assert orc.rel_l2_err(got[k], states[:T:R]) < 1e-2, (T, k)  # entry e: the state that enters step e R

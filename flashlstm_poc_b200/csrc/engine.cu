@@ -307,7 +307,10 @@ int Engine::allocate(size_t cap) {
 }
 
 int Engine::set_recompute(size_t R) {
-    if (R && (backend != FLSTM_BACKEND_TC || inner))
+    if (R && inner)
+        return set_error(FLSTM_ERR_UNSUPPORTED, "activation checkpoints need hidden_size %% 64 == 0 and input_size %% 8 == 0: this shape "
+                         "runs zero-padded on the tensor-core backend");
+    if (R && backend != FLSTM_BACKEND_TC)
         return set_error(FLSTM_ERR_UNSUPPORTED, "activation checkpoints need the tensor-core backend (f16/bf16, H %% 64 == 0, I %% 8 == 0)");
     if (R == recompute) return FLSTM_OK;
     FLSTM_CUDA_TRY(cudaDeviceSynchronize());

@@ -128,7 +128,8 @@ int flstm_engine_set_cell_io_f32(flstm_engine *engine, int enabled);
  * sequence) and the backward re-runs the forward of one R-step segment at a time to rebuild its gates, so
  * the (T,B,4H) gate cache and dG shrink to (R,B,4H): 16 -> 2 bytes per (step, sequence, gate) at R = 8.
  * Outputs and state gradients are bit-identical to R = 0; weight gradients are summed segment by segment
- * (fp32) instead of in one pass.  Tensor-core backend only; whole-sequence calls only (no step ranges).
+ * (fp32) instead of in one pass.  Tensor-core backend only, without padding
+ * (hidden_size % 64 == 0, input_size % 8 == 0); whole-sequence calls only (no step ranges).
  * Call between sequences; it re-allocates the time-sized buffers.  flstm_engine_workspace_bytes returns
  * the bytes those buffers take now. */
 int flstm_engine_set_recompute_interval(flstm_engine *engine, size_t interval);
@@ -153,7 +154,8 @@ int flstm_engine_backward_segment(flstm_engine *engine, size_t steps, int last_i
                                   const void *h_in, const float *c_in, const void *dy_seg, const void *d_hn, const void *d_cn,
                                   void *dx_seg, float *dh0, float *dc0, void *stream);
 
-/* Which backend the engine resolved to (flstm_backend, never AUTO). */
+/* Which backend the engine resolved to (flstm_backend, never AUTO).  FLSTM_BACKEND_TC also for a 16-bit shape that AUTO
+ * runs there zero-padded (hidden_size % 64 or input_size % 8 not 0). */
 int flstm_engine_backend(const flstm_engine *engine);
 
 /* Batch-sharded data parallelism: one engine per GPU/process.  flstm_comm_unique_id fills a

@@ -86,3 +86,13 @@ def test_checkpoint_mode_limits():
     eng.forward_range_into(8, 4, 8, x, None, None, y, None, None)
     torch.cuda.synchronize()
     eng.close()
+
+
+def test_a_padded_shape_says_why_it_has_no_checkpoints():
+    from flashlstm_poc_b200._lib import FlashLstmError
+
+    eng = Engine("f16", 1, 4, 33, 70, 8, device=torch.device("cuda", 0))
+    assert eng.backend == "tc"
+    with pytest.raises(FlashLstmError, match="hidden_size % 64 == 0 and input_size % 8 == 0"):
+        eng.set_recompute_interval(4)
+    eng.close()

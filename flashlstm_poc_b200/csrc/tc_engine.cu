@@ -362,15 +362,24 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
 }
 
 // Inference over a few steps: a launch per layer and step reads the layer's weights once, against projection GEMM, state copies
-// and the weight loads of a persistent kernel, all of which a few steps do not repay.  One call, us, cells / before:
-//   H = 1024, 2 layers, B = 1:  T = 1 23 / 47, T = 4 49 / 66, T = 8 98 / 94;   H = 512, B = 8:  14 / 23, 25 / 29, 49 / 31
-//   H = 4096, B = 8:  T = 1 55 / 80, T = 2 110 / 94;   H = 2048, 2 layers, B = 32:  T = 1 52 / 66, T = 2 104 / 74
-// From the second step on weights that stay in L2 (half of its 126 MB) are what pays; beyond that only T = 1 does.
+// and the weight loads of a persistent kernel, all of which a few steps do not repay.  One call, cells / other path, us:
+//   2 layers, H = 128, B = 32:   T = 1 12 / 33    T = 2 24 / 33    T = 3 36 / 37    T = 4 46 / 37
+//   4 layers, H = 512, B = 8:    T = 1 25 / 74    T = 2 49 / 82    T = 3 74 / 82    T = 4 98 / 90
+//   3 layers, H = 1024, B = 24:  T = 1 25 / 64    T = 2 49 / 76    T = 3 74 / 83    T = 4 99 / 92
+//   1 layer, H = 1216, B = 16:   T = 1 12 / 33    T = 2 24 / 39    T = 3 36 / 45    T = 4 48 / 51
+//   1 layer, H = 1216, B = 24:   T = 1 16 / 31    T = 2 32 / 38    T = 3 47 / 45    T = 4 62 / 51
+//   1 layer, H = 2048, B = 16:   T = 1 15 / 37    T = 2 29 / 37    T = 3 43 / 41    T = 4 59 / 47
+//   1 layer, H = 2048, B = 32:   T = 1 23 / 31    T = 2 45 / 37    T = 3 68 / 41    T = 4 90 / 47
+//   1 layer, B = 24, T = 1:      H = 3072 49 / 55   H = 4096 79 / 74
+// From the second step on weights that stay in L2 (half of its 126 MB) are what pays; beyond that only T = 1 does.  More than
+// 16 sequences take twice the operand loads per step, which wide layers do not repay.  A fourth step is repaid least: beyond
+// 16 sequences in a single layer, up to 16 in stacks of 512 units altogether or where the other path is the grid-wide
+// kernel (H > 512 at these batches).
 // A result that overlaps an input keeps to the other path, which has read all of x, h0 and c0 before it writes any.
 bool cell_path(const Engine &e, size_t T, const void *x, const void *h0, const void *c0, const void *y, const void *hn, const void *cn) {
     if (e.backend != FLSTM_BACKEND_TC || e.cfg.training || T > 4 || e.cfg.batch > (size_t)kCellBatch || e.trace) return false;
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(h0)) & 15) return false;
-    const size_t B = e.cfg.batch, H = e.cfg.hidden_size, states = e.layers.size() * B * H, ces = e.cell_io_f32 ? sizeof(float) : 2;
+    const size_t B = e.cfg.batch, H = e.cfg.hidden_size, L = e.layers.size(), states = L * B * H, ces = e.cell_io_f32 ? sizeof(float) : 2;
     const struct { const void *p; size_t bytes; } in[] = {{x, T * B * e.cfg.input_size * 2}, {h0, states * 2}, {c0, states * ces}},
                                                   out[] = {{y, T * B * H * 2}, {hn, states * 2}, {cn, states * ces}};
     for (const auto &o : out)
@@ -380,7 +389,11 @@ bool cell_path(const Engine &e, size_t T, const void *x, const void *h0, const v
         }
     size_t weights = 0;
     for (const auto &l : e.layers) weights += 8 * H * (l.in_size + H);
-    return T == 1 || weights <= ((size_t)64 << 20);
+    const bool wide = B > 16;
+    if (T == 1) return !wide || H <= 3072;
+    if (weights > ((size_t)64 << 20)) return false;
+    if (T == 4) return wide ? L == 1 && H <= 1152 : H <= 1280 && (H > 512 || L * H <= 512);
+    return !wide || H <= (T == 2 ? 1280 : 1152);
 }
 
 int forward_cells(Engine &e, size_t T, const void *x, const void *h0, const void *c0, void *y, void *hn, void *cn, cudaStream_t s) {

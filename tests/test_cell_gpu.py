@@ -59,3 +59,28 @@ def test_states_updated_in_place():
     for a, b in zip(want, (y, h, c)):  # fp32 sums of 1088 terms in another order, rounded to bf16
         assert torch.allclose(a.float(), b.float(), rtol=2 ** -7, atol=2 ** -9)
     eng.close()
+
+
+@pytest.mark.parametrize("L,T,B,I,H,cells", [
+    (1, 1, 16, 64, 3136, True), (1, 1, 32, 64, 3072, True), (1, 1, 17, 64, 3136, False),
+    (1, 2, 16, 64, 1344, True), (1, 2, 32, 64, 1280, True), (1, 2, 17, 64, 1344, False),
+    (1, 3, 16, 64, 1216, True), (1, 3, 32, 64, 1152, True), (1, 3, 17, 64, 1216, False),
+    (1, 4, 16, 64, 512, True), (2, 4, 8, 64, 512, False), (4, 4, 8, 64, 128, True), (2, 4, 16, 64, 576, True),
+    (1, 4, 17, 64, 1152, True), (2, 4, 17, 64, 64, False), (1, 4, 17, 64, 1216, False), (1, 4, 8, 64, 1344, False),
+    (1, 5, 1, 64, 64, False), (1, 2, 1, 2048, 2112, False),
+])
+def test_which_calls_run_step_by_step(L, T, B, I, H, cells):
+    """The edges of the rule, by the launches of a call: one per layer and step, or the other path's (states in, a projection
+    and a recurrence per layer, states out).  Both give the oracle's results."""
+    w = Workload("t", "f16", L, I, H, B, T, seed=94, state_std=0.3, training=False)
+    inp = make_inputs(w)
+    inp.dy = None
+    got, eng = run_engine(w, inp)
+    dev, td = torch.device("cuda", 0), TORCH_DTYPES["f16"]
+    before = eng.launch_count
+    eng.forward(inp.x.to(dev, td), inp.h0.to(dev, td), inp.c0.to(dev, td))
+    torch.cuda.synchronize()
+    launches = eng.launch_count - before
+    eng.close()
+    assert launches == (L * T if cells else 2 * L + 2)
+    assert_parity(got, run_oracle(inp), "f16")

@@ -437,15 +437,14 @@ using BwdKernel = void (*)(ClusterBwdParams);
 
 struct BwdShape {
     int W, MT, NKB, KSB;
-    BwdKernel kernels[3][2][2];  // NT = 1, 2, 4; f16, bf16; fast, accurate gate functions
+    BwdKernel kernels[2][2][2];  // NT = 1, 2; f16, bf16; fast, accurate gate functions
 };
 #define FLSTM_CL_K(W, MT, NKB, KSB, NT, BF) \
     {cluster_bwd_kernel<W, MT, NKB, KSB, NT, BF, false>, cluster_bwd_kernel<W, MT, NKB, KSB, NT, BF, true>}
 #define FLSTM_CL_ROW(W, MT, NKB, KSB)                                                                \
     {W, MT, NKB, KSB,                                                                                \
      {{FLSTM_CL_K(W, MT, NKB, KSB, 1, false), FLSTM_CL_K(W, MT, NKB, KSB, 1, true)},                 \
-      {FLSTM_CL_K(W, MT, NKB, KSB, 2, false), FLSTM_CL_K(W, MT, NKB, KSB, 2, true)},                 \
-      {FLSTM_CL_K(W, MT, NKB, KSB, 4, false), FLSTM_CL_K(W, MT, NKB, KSB, 4, true)}}}
+      {FLSTM_CL_K(W, MT, NKB, KSB, 2, false), FLSTM_CL_K(W, MT, NKB, KSB, 2, true)}}}
 // warps, 16-unit tiles and K chunks per warp, K groups: one row per width (multiple of 64) and cluster size in use
 const BwdShape kBwdShapes[] = {
     FLSTM_CL_ROW(8, 1, 4, 2),    // H = 64,  1 CTA
@@ -466,8 +465,6 @@ const BwdShape kBwdShapes[] = {
     FLSTM_CL_ROW(8, 5, 5, 1),    // H = 640, 16 CTAs
     FLSTM_CL_ROW(8, 6, 6, 1),    // H = 704, 768, 15 / 16 of 16 CTAs: with 12 warps fewer fragments fit into registers, too many for shared memory
 };
-
-int nt_index(int NT) { return NT == 1 ? 0 : NT == 2 ? 1 : 2; }
 
 const BwdShape *shape_of(const ClusterBwdPlan &pl) {
     for (const BwdShape &r : kBwdShapes)
@@ -512,8 +509,8 @@ int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *p
                 pl.KSB = r.KSB;
                 pl.seqs = (B + slots[n] - 1) / slots[n];
                 const int tiles = (pl.seqs + 7) / 8;
-                if (tiles > 4) continue;
-                pl.NT = tiles <= 1 ? 1 : tiles <= 2 ? 2 : 4;
+                if (tiles > 2) continue;  // with more the estimate below exceeds the grid-wide kernels at every width
+                pl.NT = tiles <= 1 ? 1 : 2;
                 pl.threads = r.W * 32;
                 pl.smem_bytes = bwd_smem(pl);
                 if ((size_t)pl.smem_bytes + 1024 > smem_limit) continue;
@@ -532,7 +529,7 @@ int plan_cluster_bwd(int B, int H, int sms, size_t smem_limit, ClusterBwdPlan *p
             }
         }
         if (!plan->use || !check) return FLSTM_OK;
-        const int have = cluster_count(reinterpret_cast<const void *>(shape->kernels[nt_index(plan->NT)][check->bf16][check->accurate]),
+        const int have = cluster_count(reinterpret_cast<const void *>(shape->kernels[plan->NT - 1][check->bf16][check->accurate]),
                                        plan->C, plan->threads, plan->smem_bytes);
         if (have >= plan->clusters) return FLSTM_OK;
         for (int n = 0; n < 5; ++n)
@@ -549,7 +546,7 @@ int lstm_backward_cluster(int dtype, const ClusterBwdPlan &pl, ClusterBwdParams 
     p.peers = pl.peers;
     p.seqs = pl.seqs;
     p.dy_aligned = reinterpret_cast<uintptr_t>(p.dy) % 16 == 0;
-    return cluster_launch(reinterpret_cast<const void *>(r->kernels[nt_index(pl.NT)][dtype == FLSTM_DTYPE_BF16 ? 1 : 0][p.real_units ? 1 : 0]), pl.C,
+    return cluster_launch(reinterpret_cast<const void *>(r->kernels[pl.NT - 1][dtype == FLSTM_DTYPE_BF16 ? 1 : 0][p.real_units ? 1 : 0]), pl.C,
                           pl.clusters * pl.C, pl.threads, pl.smem_bytes, &p, s, "cluster BPTT");
 }
 

@@ -389,7 +389,6 @@ FwdKernel fwd_kernel_ks(int kr, int NT, int ks) {
     switch (ks) {
         case 1: return fwd_kernel_nt<1, BF16, ACC>(kr, NT);
         case 2: return fwd_kernel_nt<2, BF16, ACC>(kr, NT);
-        case 4: return fwd_kernel_nt<4, BF16, ACC>(kr, NT);
     }
     return nullptr;
 }
@@ -481,7 +480,7 @@ int plan_cluster_fwd(int B, int H, int sms, size_t smem_limit, ClusterFwdPlan *p
         for (int n = 0; n < 5; ++n) {
             const int C = 1 << n;
             if ((only && C != only) || slots[n] < 1) continue;
-        for (int ks = 1; ks <= 4 && ks <= chunks; ks *= 2)
+        for (int ks = 1; ks <= 2 && ks <= chunks; ks *= 2)  // (4 is the cheapest plan of no shape)
             for (int kr : {8, 6, 5, 4, 3, 2, 1}) {
                 ClusterFwdPlan pl{};
                 pl.C = C;

@@ -300,8 +300,9 @@ int set_weights_cached(flstm_engine *e, V2Context::Packed &last, const float *w_
 
 // Host tensors move in chunks of whole time steps so that copies overlap the recurrence: about eight chunks per
 // sequence, at least 16 steps and about a megabyte each (the reference uses fixed 32-step chunks,
-// flashlstm_v2/src/lstm_forward.cu:515), the first and the last of long ones a quarter as long: nothing runs while the
-// first chunk arrives or the last one leaves (config H = 1024, B = 64, T = 512: 155 us each with equal chunks).
+// flashlstm_v2/src/lstm_forward.cu:515).  Where such a chunk has 4 MB or more and there are more than four, the first and
+// the last are a quarter as long, with six equal ones between them whatever their length: nothing runs while the first
+// chunk arrives or the last one leaves (H = 1024, B = 64, T = 512: 155 us each with equal chunks).
 // FLSTM_STREAM_CHUNK overrides the number of steps.  Returns the bounds 0 = b[0] < ... < b[n] = T.
 std::vector<size_t> chunk_bounds(size_t T, size_t step_bytes) {
     size_t n = std::max<size_t>({(T + 7) / 8, 16, ((size_t)1 << 20) / std::max<size_t>(step_bytes, 1)}), edge = 0;

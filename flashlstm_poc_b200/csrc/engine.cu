@@ -1148,6 +1148,26 @@ int flstm_engine_abort_comm(flstm_engine *engine) {
     return FLSTM_OK;
 }
 
+int flstm_engine_path(flstm_engine *engine, int backward, int *path, int *ctas, int *seqs) {
+    if (!engine || !path) return set_error(FLSTM_ERR_INVALID, "null argument");
+    const Engine &e = engine->impl.core();
+    if (backward && !e.cfg.training) return set_error(FLSTM_ERR_INVALID, "engine was created with training = 0");
+    int c = 0, n = 0;
+    if (e.backend == FLSTM_BACKEND_TC) {
+        *path = flstm_b200::tc::recurrent_path(e, backward != 0, &c, &n);
+    } else {
+        const auto &plan = backward ? e.f32_bwd : e.f32_fwd;
+        *path = plan.use ? FLSTM_PATH_CLUSTER : e.simt_grid ? FLSTM_PATH_GRID : FLSTM_PATH_STEPS;
+        if (plan.use) {
+            c = plan.C;
+            n = plan.seqs;
+        }
+    }
+    if (ctas) *ctas = c;
+    if (seqs) *seqs = n;
+    return FLSTM_OK;
+}
+
 int flstm_engine_wait(flstm_engine *engine, cudaStream_t stream, unsigned int timeout_ms) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
     Engine &e = engine->impl;

@@ -255,6 +255,16 @@ int poll_error(Engine &e) { return check_async_error(e); }
 
 unsigned int *error_mirror(Engine &e) { return state(e)->err_host; }
 
+int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs) {
+    const TcState *st = static_cast<const TcState *>(e.tc_state);
+    const bool cluster = backward ? st->cbwd.use : st->cfwd.use;
+    *ctas = !cluster ? 0 : backward ? st->cbwd.C : st->cfwd.C;
+    *seqs = !cluster ? 0 : backward ? st->cbwd.seqs : st->cfwd.seqs;
+    if (cluster) return FLSTM_PATH_CLUSTER;
+    if (!st->step.use) return FLSTM_PATH_GRID;
+    return !backward && st->step.fwd_persistent && wavefront_chunk(e, (size_t)-1) == 0 ? FLSTM_PATH_GRID : FLSTM_PATH_STEPS;
+}
+
 int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s) {
     TcState *st = state(e);
     FLSTM_TRY(check_async_error(e));

@@ -166,7 +166,6 @@ int lstm_step_backward_pointwise(int dtype, const void *gates_t, const float *c_
                                  const float *parts, int nparts, float *dc, void *dg_t, int B, int H, int real_units, cudaStream_t s);
 int sum_parts(const float *parts, int nparts, size_t n, float *out, cudaStream_t s);
 
-// fp32 (4H, K) torch-ordered rows -> 16-bit tile-interleaved rows; bias likewise (b_ih + b_hh)
 // One time step of one layer in one launch (tc_cell.cu); B <= 32, 16-byte aligned x and h_prev.
 struct CellParams {
     const void *w_ih, *w_hh;  // 16-bit, rows tile-interleaved: (4H, I), (4H, H)

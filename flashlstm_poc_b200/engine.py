@@ -56,6 +56,12 @@ class Engine:
     def backend(self) -> str:
         return BACKEND_NAMES[self.lib.flstm_engine_backend(self._h)]
 
+    def recurrent_path(self, backward: bool = False) -> Tuple[str, int, int]:
+        """Which kernels run a sequence: ("steps" | "grid" | "cluster", CTAs per cluster, sequences per cluster)."""
+        path, ctas, seqs = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+        check(self.lib.flstm_engine_path(self._h, int(backward), ctypes.byref(path), ctypes.byref(ctas), ctypes.byref(seqs)))
+        return ("steps", "grid", "cluster")[path.value], ctas.value, seqs.value
+
     def _stream(self) -> int:
         return torch.cuda.current_stream(self._index).cuda_stream
 

@@ -158,6 +158,12 @@ int flstm_engine_backward_segment(flstm_engine *engine, size_t steps, int last_i
  * runs there zero-padded (hidden_size % 64 or input_size % 8 not 0). */
 int flstm_engine_backend(const flstm_engine *engine);
 
+/* Which kernels run a sequence's recurrence (backward = 0) or its BPTT (1; training engines): launches per time step, one
+ * grid-wide launch per layer, or one launch of thread-block clusters that each run their own sequences; for those `ctas` is
+ * the CTAs of a cluster and `seqs` its sequences (else 0).  Either of them may be NULL. */
+typedef enum { FLSTM_PATH_STEPS = 0, FLSTM_PATH_GRID = 1, FLSTM_PATH_CLUSTER = 2 } flstm_path;
+int flstm_engine_path(flstm_engine *engine, int backward, int *path, int *ctas, int *seqs);
+
 /* Batch-sharded data parallelism: one engine per GPU/process.  flstm_comm_unique_id fills a
  * 128-byte id on rank 0 (send it to the other ranks by any means); every rank then calls
  * flstm_engine_attach_comm.  The only collective is one sum-allreduce per layer over that
@@ -217,6 +223,7 @@ typedef struct {
     int fwd_pair;      /* persistent forward kernel: neighbouring row-tile CTAs form cta_group::2 pairs */
     int step_fwd_pair; /* wide batches: the all-steps forward kernel runs on CTA pairs (256-sequence tiles) */
 } flstm_tc_plan_info;
+/* (Engines try the cluster-resident kernels first where hidden_size <= 768: see flstm_engine_path.) */
 int flstm_tc_plan(size_t batch, size_t hidden_size, int training, int sm_count, size_t smem_limit,
                   flstm_tc_plan_info *out);
 

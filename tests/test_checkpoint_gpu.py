@@ -37,15 +37,7 @@ def _run(w, inp, interval, dhn, dcn, repeat=1):
     return out, bytes_
 
 
-@pytest.mark.parametrize("dtype,L,T,B,I,H,R,step_path", [
-    ("f16", 2, 23, 16, 64, 64, 5, False),     # persistent kernels, ragged last segment, stacked layers
-    ("bf16", 1, 12, 32, 128, 128, 1, False),  # R = 1: a checkpoint at every step
-    ("f16", 1, 9, 8, 64, 128, 16, False),     # R >= T: a single segment
-    ("bf16", 2, 9, 256, 128, 128, 4, True),   # per-step GEMM path (wide batch), dh carried as fp32 partial sums
-    ("f16", 1, 7, 300, 64, 256, 3, True),     # per-step path, ragged batch tile, K split
-])
-def test_checkpoint_mode_matches_full_cache(dtype, L, T, B, I, H, R, step_path, monkeypatch):
-    monkeypatch.setenv("FLSTM_STEP_MIN_BATCH", "1" if step_path else "0")
+def _compare(dtype, L, T, B, I, H, R):
     w = Workload("ck", dtype, L, I, H, B, T, seed=77, state_std=0.3)
     inp = make_inputs(w)
     torch.manual_seed(9)
@@ -62,6 +54,29 @@ def test_checkpoint_mode_matches_full_cache(dtype, L, T, B, I, H, R, step_path, 
     assert_parity(ck, ref, dtype)
     if R < T:
         assert ck_bytes < full_bytes
+
+
+@pytest.mark.parametrize("dtype,L,T,B,I,H,R,step_path", [
+    ("f16", 2, 23, 16, 64, 64, 5, False),     # persistent kernels, ragged last segment, stacked layers
+    ("bf16", 1, 12, 32, 128, 128, 1, False),  # R = 1: a checkpoint at every step
+    ("f16", 1, 9, 8, 64, 128, 16, False),     # R >= T: a single segment
+    ("bf16", 2, 9, 256, 128, 128, 4, True),   # per-step GEMM path (wide batch), dh carried as fp32 partial sums
+    ("f16", 1, 7, 300, 64, 256, 3, True),     # per-step path, ragged batch tile, K split
+])
+def test_checkpoint_mode_matches_full_cache(dtype, L, T, B, I, H, R, step_path, monkeypatch):
+    monkeypatch.setenv("FLSTM_STEP_MIN_BATCH", "1" if step_path else "0")
+    _compare(dtype, L, T, B, I, H, R)
+
+
+@pytest.mark.parametrize("dtype,L,T,B,I,H,R", [
+    ("f16", 2, 23, 16, 64, 64, 5), ("bf16", 1, 12, 37, 128, 256, 1), ("f16", 1, 9, 20, 64, 512, 16), ("bf16", 2, 10, 300, 64, 256, 4),
+])
+def test_checkpoint_mode_on_clusters(dtype, L, T, B, I, H, R):
+    """The same on the cluster-resident kernels: a segment's backward continues from the dG of the step after it."""
+    eng = Engine(dtype, L, B, I, H, T, device=torch.device("cuda", 0))
+    assert eng.recurrent_path()[0] == eng.recurrent_path(backward=True)[0] == "cluster"
+    eng.close()
+    _compare(dtype, L, T, B, I, H, R)
 
 
 def test_checkpoint_mode_limits():

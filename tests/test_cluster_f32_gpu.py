@@ -49,3 +49,33 @@ def test_f32_ranges_equal_one_call(B, H):
     for a, b in zip(want, (*out, *eng.grads(0))):
         assert torch.equal(a, b)
     eng.close()
+
+
+@pytest.mark.parametrize("cluster,L,B,I,H", SHAPES)
+def test_the_shapes_above_run_on_clusters(cluster, L, B, I, H, monkeypatch):
+    if cluster:
+        monkeypatch.setenv("FLSTM_CLUSTER_SIZE", str(cluster))
+    eng = Engine("f32", L, B, I, H, 1, device=torch.device("cuda", 0))
+    paths = [eng.recurrent_path(b) for b in (False, True)]
+    eng.close()
+    assert all(p[0] == "cluster" and p[1] == (cluster or p[1]) for p in paths)
+
+
+@pytest.mark.parametrize("L,B,I,H,path", [(1, 8, 24, 520, "grid"), (2, 5, 16, 800, "grid"), (1, 40, 16, 700, "steps"), (1, 3, 16, 1100, "steps"),
+                                          (1, 9, 8, 256, "grid-small"), (1, 300, 8, 200, "steps-small")])
+def test_f32_beyond_the_clusters(L, B, I, H, path, monkeypatch):
+    """The kernels of fp32 layers wider than 512: one grid-wide launch while its CTAs fit the machine at once, else a launch per
+    step; small widths reach them with the clusters switched off."""
+    path, _, small = path.partition("-")
+    if small:
+        monkeypatch.setenv("FLSTM_CLUSTER", "0")
+    w = Workload("t", "f32", L, I, H, B, 5, seed=73, state_std=0.3)
+    inp = make_inputs(w)
+    gen = torch.Generator().manual_seed(7)
+    dhn, dcn = torch.randn(L, B, H, generator=gen), torch.randn(L, B, H, generator=gen)
+    got, eng = run_engine(w, inp, dhn=dhn, dcn=dcn, repeat=2)
+    paths = [eng.recurrent_path(b)[0] for b in (False, True)]
+    eng.close()
+    assert paths == [path, path]
+    # fp32 sums of up to 4400 terms of order 1/sqrt(H) and 1500-term weight gradients: errors of order 1e-5
+    assert_parity(got, run_oracle(inp, dhn=dhn, dcn=dcn), "f32", fp32_max_abs=1e-4)

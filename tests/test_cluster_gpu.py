@@ -1,6 +1,6 @@
 """The cluster-resident recurrent kernels (tc_cluster_fwd.cu, tc_cluster_bwd.cu) against the oracle, at the edges of
-their tiling: every width / cluster size they are built for, one to four tiles of 8 sequences per cluster, partly
-filled tiles and clusters, CTAs of a cluster that own no units, weights partly in shared memory, both ways of sending
+their tiling: every width and most cluster sizes they are built for, one, two and four tiles of 8 sequences per cluster
+(BPTT: one and two), partly filled tiles and clusters, CTAs of a cluster that own no units, weights partly in shared memory, both ways of sending
 h_t (from 4 sequences per cluster on whole rows), and step ranges that continue an earlier launch."""
 import pytest
 import torch
@@ -57,3 +57,27 @@ def test_ranges_and_an_unaligned_gradient(B, H):
     eng.close()
     for a, b in zip(want, (y2, hn2, cn2, dx2, dh2, dc2)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("cluster,B,H", SHAPES)
+def test_the_shapes_above_run_on_clusters(cluster, B, H, monkeypatch):
+    monkeypatch.setenv("FLSTM_CLUSTER_SIZE", str(cluster))
+    eng = Engine("f16", 1, B, 64, H, 1, device=torch.device("cuda", 0))
+    forward, backward = eng.recurrent_path(), eng.recurrent_path(backward=True)
+    eng.close()
+    assert forward[:2] == ("cluster", cluster)
+    # the BPTT kernel has no form for 4 CTAs at H = 64
+    assert backward[:2] == (("grid", 0) if (cluster, H) == (4, 64) else ("cluster", cluster))
+
+
+@pytest.mark.parametrize("B,H,tiles,backward_tiles", [(2400, 64, 4, 0), (1250, 64, 2, 2), (600, 192, 4, 2), (600, 256, 4, 0), (300, 256, 2, 2),
+                                                      (130, 320, 2, 2), (128, 512, 4, 0), (60, 512, 2, 2)])
+def test_several_tiles_of_sequences_per_cluster(B, H, tiles, backward_tiles):
+    """Batches at which the planner itself gives a cluster more than 8 or 16 sequences."""
+    w = Workload("t", "bf16" if H % 128 else "f16", 1, 32, H, B, 3, seed=43, state_std=0.3)
+    inp = make_inputs(w)
+    got, eng = run_engine(w, inp, repeat=2)
+    per_cluster = [eng.recurrent_path(b)[2] for b in (False, True)]
+    eng.close()
+    assert [(n + 7) // 8 if n <= 16 else 4 for n in per_cluster] == [tiles, backward_tiles]
+    assert_parity(got, run_oracle(inp), w.dtype)

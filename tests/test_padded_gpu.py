@@ -207,3 +207,28 @@ def test_what_fits_only_unpadded_runs_on_the_cuda_cores():
     got = {"y": to_np(y[:, :9]), "hn": to_np(hn[:, :9]), "cn": to_np(cn[:, :9])}
     eng.close()
     assert_parity(got, want, "f16", keys=("y", "hn", "cn"))
+
+
+@pytest.mark.parametrize("dtype,L,T,B,I,H", [("f16", 2, 6, 20, 40, 70), ("bf16", 2, 4, 40, 130, 1217)])
+def test_padded_state_caches_match_the_oracle(dtype, L, T, B, I, H):
+    """The logical copies of the cell and hidden states behind flstm_engine_cache_ptrs, slot by slot, of every layer."""
+    import ctypes
+
+    from flashlstm_poc_b200._lib import check
+    from tests.helpers import params_from_inputs
+
+    w = Workload("t", dtype, L, I, H, B, T, seed=56, state_std=0.3)
+    inp = make_inputs(w)
+    got, eng = run_engine(w, inp)
+    fwd = orc.lstm_forward(inp.x.numpy(), params_from_inputs(inp), inp.h0.numpy(), inp.c0.numpy(), dtype=np.float32)
+    for l in range(L):
+        ptr = ctypes.c_void_p()
+        check(eng.lib.flstm_engine_cache_ptrs(eng._h, l, None, None, ctypes.byref(ptr), None))
+        hs = to_np(eng._wrap(ptr.value, (T + 1, B, H), TORCH_DTYPES[dtype]))
+        cs = to_np(eng.cell_states(l, T))
+        for t in range(T + 1):
+            assert orc.rel_l2_err(hs[t], fwd.caches[l].h_s[t]) < 1e-2, (l, t)
+            assert orc.rel_l2_err(cs[t], fwd.caches[l].c_s[t]) < 1e-2, (l, t)
+        assert np.array_equal(hs[T], got["hn"][l])
+    assert np.array_equal(hs[1:], got["y"])
+    eng.close()

@@ -42,10 +42,12 @@ def _step(eng, inp, dev, td):
     ("bf16", "tc", "forward-wide"),  # 96 sequences at H = 1024: the wide-batch forward kernel (all steps in one launch)
     # H = 2048: W_hh is streamed, and part of it is fetched into the ring ahead of the barrier that then fails
     ("bf16", "tc", "forward-streamed"), ("bf16", "tc", "backward-streamed"),
+    # clusters of several CTAs in either direction (H = 64: BPTT on one CTA)
+    ("f16", "tc", "forward-several"), ("bf16", "tc", "backward-several"),
 ])
 def test_step_barrier_timeout_returns_and_engine_recovers(dtype, backend, where):
     where, _, variant = where.partition("-")
-    shape = {"": (64, 64, 8), "wide": (128, 1024, 96), "streamed": (128, 2048, 8)}[variant]
+    shape = {"": (64, 64, 8), "wide": (128, 1024, 96), "streamed": (128, 2048, 8), "several": (64, 512, 8)}[variant]
     w = Workload("timeout", dtype, 1, *shape, 4, seed=11, state_std=0.1)
     inp = make_inputs(w)
     td = TORCH_DTYPES[dtype]
@@ -77,3 +79,31 @@ def test_step_barrier_timeout_returns_and_engine_recovers(dtype, backend, where)
     eng.close()
     for a, b in zip(before, after):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,backend,where", [
+    ("f16", "tc", "forward"), ("f16", "tc", "backward"), ("bf16", "tc", "forward"), ("bf16", "tc", "backward"),
+    ("f32", "simt", "forward"), ("f32", "simt", "backward"), ("f16", "simt", "forward"), ("bf16", "simt", "backward"),
+])
+def test_grid_wide_kernels_return_and_recover(dtype, backend, where, monkeypatch):
+    """The grid-wide kernels with resident weights, whose CTAs clear the step counters on their way out (after an abort too):
+    the shape above runs on clusters unless they are switched off."""
+    monkeypatch.setenv("FLSTM_CLUSTER", "0")
+    eng = Engine(dtype, 1, 8, 64, 64, 4, backend=backend, device=torch.device("cuda", 0))
+    assert eng.recurrent_path()[0] == eng.recurrent_path(backward=True)[0] == "grid"
+    eng.close()
+    test_step_barrier_timeout_returns_and_engine_recovers(dtype, backend, where)
+
+
+def test_which_kernels_the_cases_above_time_out():
+    dev = torch.device("cuda", 0)
+    for dtype, shape, forward, backward in (("f16", (64, 64, 8), "cluster", "cluster"), ("f32", (64, 64, 8), "cluster", "cluster"),
+                                            ("f16", (64, 512, 8), "cluster", "cluster"), ("bf16", (128, 1024, 96), "grid", "steps"),
+                                            ("bf16", (128, 2048, 8), "grid", "grid")):
+        I, H, B = shape
+        eng = Engine(dtype, 1, B, I, H, 4, device=dev)
+        paths = eng.recurrent_path(), eng.recurrent_path(backward=True)
+        eng.close()
+        assert [p[0] for p in paths] == [forward, backward]
+        if H == 512:
+            assert all(p[1] == 16 for p in paths)

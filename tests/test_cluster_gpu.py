@@ -70,7 +70,7 @@ def test_the_shapes_above_run_on_clusters(cluster, B, H, monkeypatch):
     assert backward[:2] == (("grid", 0) if (cluster, H) == (4, 64) else ("cluster", cluster))
 
 
-@pytest.mark.parametrize("B,H,tiles,backward_tiles", [(2400, 64, 4, 0), (1250, 64, 2, 2), (600, 192, 4, 2), (600, 256, 4, 0), (300, 256, 2, 2),
+@pytest.mark.parametrize("B,H,tiles,backward_tiles", [(2400, 64, 4, 0), (1250, 64, 2, 2), (600, 192, 2, 2), (600, 256, 4, 0), (300, 256, 2, 2),
                                                       (130, 320, 2, 2), (128, 512, 4, 0), (60, 512, 2, 2)])
 def test_several_tiles_of_sequences_per_cluster(B, H, tiles, backward_tiles):
     """Batches at which the planner itself gives a cluster more than 8 or 16 sequences."""

@@ -77,7 +77,7 @@ def test_padded_ranges_and_unaligned_tensors():
 ])
 def test_padded_gate_functions_keep_their_relative_accuracy_near_zero(dtype, B, I, H, training):
     """Only the cell candidate has a pre-activation, exact in 16 bits and down to 2^-13 (f16) or 2^-20 (bf16), so that
-    c_1 = tanh(a) / 2.  tanhf is good to 2 units in the last place and sigmoid(0) = 1/2 is exact: 2^-22 relative."""
+    c_1 = tanh(a) / 2.  tanh is good to 2 units in the last place there and sigmoid(0) = 1/2 is exact: 2^-22 relative."""
     dev, td = torch.device("cuda", 0), TORCH_DTYPES[dtype]
     u = torch.arange(H)
     low = 13 if dtype == "f16" else 20

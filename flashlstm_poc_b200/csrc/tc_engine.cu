@@ -27,6 +27,7 @@ struct TcLayer {
     CUtensorMap tm_h;   // hs (Tcap+1, B, H), 1 x BT x 64 boxes, 128B swizzle
     CUtensorMap tm_g;   // gates (Tcap, B, 4H), 1 x BT x 64 boxes, no swizzle
     CUtensorMap tm_dg;  // dG (Tcap, B, 4H), 1 x BT x 64 boxes, 128B swizzle (BPTT operand)
+    BwdTmMaps dg_tm;    // dG for the tensor-memory BPTT kernel
     // wide-batch path (one GEMM launch per step)
     CUtensorMap tm_hs3;    // hs (Tcap+1, B, H), 1 x 128 x 64 boxes, 128B swizzle
     CUtensorMap tm_wstep;  // w_hh (4H, H), bn_fwd x 64 boxes, 128B swizzle
@@ -38,7 +39,9 @@ struct TcState {
     int sms = 0;
     size_t smem_limit = 0;
     FwdPlan fwd{};
+    FwdTmPlan fwdtm{};
     BwdPlan bwd{};
+    BwdTmPlan bwdtm{};
     bool bwd_ok = false;
     StepPlan step{};
     ClusterFwdPlan cfwd{};
@@ -163,8 +166,14 @@ int init(Engine &e) {
             FLSTM_TRY(plan_cluster_bwd(B, H, st->sms, st->smem_limit, &st->cbwd, &check));
             if (st->cbwd.cycles > kGridBwdCycles) st->cbwd.use = false;
         }
+        // the cross-layer wavefront would put two cooperative grids side by side
+        const char *wave = std::getenv("FLSTM_WAVE_CHUNK");
+        const bool wavefront = wave && std::atoi(wave) > 0;
+        if (!st->cfwd.use && !wavefront) FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &st->fwdtm));
+        if (e.cfg.training && !st->cbwd.use && !wavefront)
+            FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &st->bwdtm, /*check_device=*/true));
     }
-    const bool grid_fwd = !st->cfwd.use, grid_bwd = e.cfg.training && !st->cbwd.use;
+    const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use, grid_bwd = e.cfg.training && !st->cbwd.use && !st->bwdtm.use;
     st->bwd_ok = e.cfg.training != 0;
     if (grid_fwd || grid_bwd) FLSTM_TRY(plan_step(B, H, st->sms, st->smem_limit, &st->step));
     if (st->step.use && grid_bwd) {
@@ -202,9 +211,15 @@ int on_capacity_change(Engine &e) {
     for (size_t li = 0; li < e.layers.size(); ++li) {
         auto &l = e.layers[li];
         auto &t = st->layers[li];
-        const bool grid_fwd = !st->cfwd.use, grid_bwd = e.cfg.training && l.dg && !st->cbwd.use;
-        if (!grid_fwd && !grid_bwd) continue;  // the cluster kernels use plain loads
+        const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use, tm_bwd = e.cfg.training && l.dg && st->bwdtm.use;
+        const bool grid_bwd = e.cfg.training && l.dg && !st->cbwd.use && !st->bwdtm.use;
+        if (!grid_fwd && !grid_bwd && !st->fwdtm.use && !tm_bwd) continue;  // the cluster kernels use plain loads
         FLSTM_TRY(make_tensor_map_2d(&t.tm_w, l.w_hh, 4 * H, H, H, 64, 64, true));
+        if (tm_bwd) FLSTM_TRY(make_bwd_tm_maps(&t.dg_tm, st->bwdtm, l.dg, dg_steps, B, H));
+        if (st->fwdtm.use) {
+            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->fwdtm.S * st->fwdtm.BT / 2, st->fwdtm.ch));
+            FLSTM_TRY(make_tensor_map_3d(&t.tm_g, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwdtm.BT, 64, false));
+        }
         if (st->step.use) {
             FLSTM_TRY(make_tensor_map_3d(&t.tm_hs3, l.hs, cap + 1, B, H, H, B * H, 128, 64, true));
             FLSTM_TRY(make_tensor_map_2d(&t.tm_wstep, l.w_hh, 4 * H, H, H, (st->step.pair || st->step.fwd_pair) ? st->step.bn_fwd / 2 : st->step.bn_fwd, 64, true));
@@ -261,7 +276,7 @@ int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs) {
     *ctas = !cluster ? 0 : backward ? st->cbwd.C : st->cfwd.C;
     *seqs = !cluster ? 0 : backward ? st->cbwd.seqs : st->cfwd.seqs;
     if (cluster) return FLSTM_PATH_CLUSTER;
-    if (!st->step.use) return FLSTM_PATH_GRID;
+    if (!st->step.use || (backward ? st->bwdtm.use : st->fwdtm.use)) return FLSTM_PATH_GRID;
     return !backward && st->step.fwd_persistent && wavefront_chunk(e, (size_t)-1) == 0 ? FLSTM_PATH_GRID : FLSTM_PATH_STEPS;
 }
 
@@ -302,7 +317,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         e.launches += 2;
         return FLSTM_OK;
     }
-    if (st->step.use) {
+    if (st->step.use && !st->fwdtm.use) {
         CUtensorMap tm_y;
         if (y_out) FLSTM_TRY(make_tensor_map_3d_tile(&tm_y, y_out, 2, t1, B, H, 32, 16));
         const StepFwdMaps maps{&t.tm_hs3, &t.tm_wstep, &t.tm_g_ep, &t.tm_c_ep, &t.tm_h_ep, y_out ? &tm_y : nullptr};
@@ -363,7 +378,9 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.trace_steps = e.trace_steps;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    FLSTM_TRY(lstm_forward_persistent(e.cfg.dtype, st->fwd, t.tm_w, t.tm_h, t.tm_g, p, s));
+    p.w_hh = l.w_hh;
+    if (st->fwdtm.use) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_h, t.tm_g, p, s));
+    else FLSTM_TRY(lstm_forward_persistent(e.cfg.dtype, st->fwd, t.tm_w, t.tm_h, t.tm_g, p, s));
     size_t m2 = e.timer.mark(s);
     e.timer.span(PH_PROJ, m0, m1);
     e.timer.span(PH_RECUR_FWD, m1, m2);
@@ -491,7 +508,7 @@ static int backward_steps(Engine &e, int li, size_t T, size_t t0, size_t t1, con
 // layer-by-layer schedule.
 size_t wavefront_chunk(const Engine &e, size_t n) {
     TcState *st = static_cast<TcState *>(e.tc_state);
-    if (!st || !st->step.use || e.layers.size() < 2 || e.timer.enabled) return 0;
+    if (!st || !st->step.use || st->fwdtm.use || st->bwdtm.use || e.layers.size() < 2 || e.timer.enabled) return 0;
     const char *env = std::getenv("FLSTM_WAVE_CHUNK");
     if (!env) return 0;
     const long v = std::atol(env);
@@ -537,7 +554,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
         cp.extra_arrivals = e.selftest_missing_arrivals;
         FLSTM_TRY(lstm_backward_cluster(e.cfg.dtype, st->cbwd, cp, s));
         e.launches += 1;
-    } else if (st->step.use) {
+    } else if (st->step.use && !st->bwdtm.use) {
         FLSTM_TRY(backward_steps(e, li, T, t0, t1, dy_l, dhn_l, dcn_l, dh0_l, dc0_l, finalize, s));
     } else {
     BwdParams p{};
@@ -563,7 +580,9 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.H = (int)H;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    FLSTM_TRY(lstm_backward_persistent(e.cfg.dtype, st->bwd, t.tm_w, t.tm_dg, p, s));
+    p.w_hh = l.w_hh;
+    if (st->bwdtm.use) FLSTM_TRY(lstm_backward_tm(e.cfg.dtype, st->bwdtm, t.tm_w, t.dg_tm, p, s));
+    else FLSTM_TRY(lstm_backward_persistent(e.cfg.dtype, st->bwd, t.tm_w, t.tm_dg, p, s));
     e.launches += 1;
     }
     size_t m1 = e.timer.mark(s);

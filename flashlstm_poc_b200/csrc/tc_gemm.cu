@@ -831,5 +831,20 @@ int make_tensor_map_chunked(CUtensorMap *out, const void *base, uint64_t steps, 
     return FLSTM_OK;
 }
 
+int make_tensor_map_halves(CUtensorMap *out, const void *base, uint64_t steps, uint64_t rows, uint64_t width, uint32_t box_rows,
+                           uint32_t half_chunks, uint32_t chunks) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return set_error(FLSTM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    cuuint64_t dims[5] = {64, rows, 2, half_chunks, steps};
+    cuuint64_t strides[4] = {width * 2, half_chunks * 128ull, 128, rows * width * 2};
+    cuuint32_t box[5] = {64, box_rows, 2, chunks, 1};
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 5, const_cast<void *>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(FLSTM_ERR_CUDA, "cuTensorMapEncodeTiled (halves) failed (%d)", (int)r);
+    return FLSTM_OK;
+}
+
 }  // namespace tc
 }  // namespace flstm_b200

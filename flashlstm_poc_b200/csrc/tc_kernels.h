@@ -55,6 +55,7 @@ struct FwdParams {
     int trace_steps;
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path: the step barrier waits for this many arrivals nobody makes
+    const void *w_hh;     // 16-bit (4H, H), rows tile-interleaved; read by the tensor-memory kernel beside its tensor map
     // filled by the launcher from the plan
     int rt, cta_rows, nt, stages, ch;
     uint32_t idesc;
@@ -68,6 +69,25 @@ bool wider_tile_enabled();  // 65..128 sequences as one 128-wide batch tile like
 // (T, B, 4H), box 1 x BT x 64, no swizzle.
 int lstm_forward_persistent(int dtype, const FwdPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_h,
                             const CUtensorMap &tm_g, FwdParams p, cudaStream_t s);
+
+// ------------------------------------------------------------------ the same with W_hh in tensor memory (tc_lstm_fwd_tm.cu)
+struct FwdTmPlan {
+    bool use;
+    int S;         // 2: K split over the lane halves, 64 gate rows per CTA; 1: 128 gate rows per CTA
+    int BT;        // sequences per batch group
+    int cta_rows;  // CTAs per batch group (row blocks)
+    int ngroups;
+    int kc;        // chunk-steps of 64 along K (per half for S = 2)
+    int ct, cs;    // of these, kept in tensor / shared memory; the others are streamed each step
+    int ch, hstages;  // chunk-steps of h per copy, copies in the ring
+    int wstages;   // ring of streamed chunk-steps of W_hh (0: nothing is streamed)
+    int smem_bytes;
+    int grid;
+};
+int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan);
+// tm_w: W_hh as for lstm_forward_persistent.  tm_h: chunked map with box rows S * BT / 2 and plan.ch chunks.  tm_g: box 1 x BT x 64.
+int lstm_forward_tm(int dtype, const FwdTmPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_h, const CUtensorMap &tm_g,
+                    const FwdParams &p, cudaStream_t s);
 
 // ------------------------------------------------------------------ persistent BPTT
 struct BwdPlan {
@@ -99,6 +119,7 @@ struct BwdParams {
     int s0, s1;           // reverse iterations [s0, s1) of this launch; iteration s is time T-1-s, s == T writes dh0/dc0
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path (see FwdParams)
+    const void *w_hh;     // as in FwdParams
     int jt, nt, stages, ch;
     uint32_t idesc;
 };
@@ -111,6 +132,28 @@ int plan_bwd(int B, int H, int sms, size_t smem_limit, BwdPlan *plan, bool check
 // with box rows BT and plan.ch chunks.
 int lstm_backward_persistent(int dtype, const BwdPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_dg,
                              BwdParams p, cudaStream_t s);
+
+// ------------------------------------------------------------------ the same with W_hh in tensor memory (tc_lstm_bwd_tm.cu)
+struct BwdTmPlan {
+    bool use;
+    int BT;        // sequences per batch group
+    int jt;        // unit tiles = H / 64, a cluster of four CTAs each
+    int ngroups;
+    int kp;        // chunk-steps of 64 per half of a CTA's K range
+    int left;      // 1: the range has an odd number of chunks, the last one runs by itself
+    int ct, cs;    // chunk-steps of W_hh in tensor / shared memory (all of them)
+    int ch, stages;  // chunk-steps of dG per copy, copies in the ring
+    int smem_bytes;
+    int grid;
+};
+struct BwdTmMaps {
+    CUtensorMap half[4];  // dG from the K range of each CTA of a cluster on (make_tensor_map_halves)
+    CUtensorMap chunk;    // single chunks of dG (make_tensor_map_chunked)
+};
+int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool check_device);
+int make_bwd_tm_maps(BwdTmMaps *maps, const BwdTmPlan &plan, const void *dg, size_t steps, size_t B, size_t H);
+int lstm_backward_tm(int dtype, const BwdTmPlan &plan, const CUtensorMap &tm_w, const BwdTmMaps &maps, const BwdParams &p,
+                     cudaStream_t s);
 
 // ------------------------------------------------------------------ wide-batch path: one GEMM launch per step
 struct StepPlan {

@@ -1,0 +1,524 @@
+// Persistent BPTT kernel with W_hh in TENSOR MEMORY: one launch runs the whole reverse recurrence of one layer.
+//
+// Same split as tc_lstm_bwd.cu: a cluster of four CTAs owns 64 hidden units, CTA kq contracts its quarter of K = 4H, the
+// partial sums are reduce-scattered through distributed shared memory, every CTA runs the pointwise backward of 16 units.
+// What bounded that kernel beyond H = 1024 was its slice of W_hh (256 KB per CTA and step at H = 2048, through an SM port of
+// about 60 B per cycle) and, at every H, UMMAs of M = 64 that read both operands from shared memory.  Here the slice is the A
+// operand in tensor memory (what does not fit its columns stays in shared memory, nothing is streamed), and the tiles are
+// M = 128: lanes 0-63 hold W_hh^T of the 64 units for the first half of the CTA's K range, lanes 64-127 for the second half.
+// The B operand has 2 BT rows (K half 0 and 1 of the BT sequences), the accumulator 128 lanes x 2 BT columns, of which the
+// blocks (half q, columns of half q) are partial sums and the other two are ignored.  A K range of an odd number of 64-wide
+// chunks leaves one chunk that runs as an instruction of N = BT from shared memory into the first half's block.
+//
+// Per step: the producer waits for the step barrier and fetches dG_{t+1} of the K range (both halves with one copy: a 5-D
+// map orders them as the B operand wants); the UMMA thread contracts; the 256 epilogue threads move the accumulator to shared
+// memory, add the halves, send them to the owners with st.async, add the four sources and do the pointwise update.
+// Every wait is bounded; the way out is that of tc_lstm_bwd.cu.
+//
+// Replaces the same reference launches (flashlstm_v2/src/lstm_backward.cu:158-227, 1057-1101).
+#include <cstdlib>
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "tc_common.cuh"
+#include "tc_kernels.h"
+#include "tc_recurrent.cuh"
+
+namespace flstm_b200 {
+namespace tc {
+
+namespace {
+
+constexpr int kThreads = 320;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA issuer
+constexpr int kEpilogueThreads = 256;
+constexpr int kStepBytesW = 2 * 64 * 128;  // one chunk-step of A: two blocks of 64 K rows x 64 units
+constexpr int kTmemColumns = 512;
+constexpr int KS = 4, UPO = 64 / KS;
+
+struct Layout {
+    int w, left_w, ring, left, ps, red, total;
+};
+
+__host__ __device__ inline Layout layout_of(const BwdTmPlan &pl) {
+    Layout l;
+    l.w = pl.cs * kStepBytesW;
+    l.left_w = pl.left ? kStepBytesW : 0;
+    l.ring = pl.stages * pl.ch * 2 * pl.BT * 128;
+    l.left = pl.left ? pl.BT * 128 : 0;
+    l.ps = 128 * (pl.BT + 4) * 4;
+    l.red = 2 * KS * UPO * (pl.BT + 4) * 4;
+    l.total = l.w + l.left_w + l.ring + l.left + l.ps + l.red + 1024 /*align*/ + 512 /*barriers*/;
+    return l;
+}
+
+template <int BT, bool BF16, bool ACCURATE>
+__global__ void __launch_bounds__(kThreads, 1)
+lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ BwdTmMaps maps,
+                   const __grid_constant__ BwdTmPlan pl, BwdParams p) {
+    constexpr int PAIRS = BT / 16;  // (unit, sequence) pairs per epilogue thread
+    constexpr int RS = BT + 4;      // row stride of the exchange and reduce buffers (floats), keeps float4 alignment
+    constexpr int N = 2 * BT;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const Layout L = layout_of(pl);
+    const int KP = pl.kp, CT = pl.ct, CS = pl.cs, CH = pl.ch, NLOAD = (KP + CH - 1) / CH, ST = pl.stages;
+    const int stage_bytes = CH * N * 128;
+    uint8_t *s_w = smem, *s_lw = s_w + L.w, *s_ring = s_lw + L.left_w, *s_left = s_ring + L.ring;
+    float *s_ps = reinterpret_cast<float *>(s_left + L.left), *s_red = s_ps + L.ps / 4;
+    uint64_t *full = reinterpret_cast<uint64_t *>(s_red + L.red / 4), *empty = full + ST;
+    uint64_t *lfull = empty + ST, *lempty = lfull + 1, *tfull = lempty + 1, *tempty = tfull + 1, *wbar = tempty + 1;
+    uint64_t *rbar = wbar + 1;  // [2] partial sums received
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(rbar + 2);
+    volatile uint32_t *abort_w = tmem_slot + 1;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kq = (int)cluster_ctarank();
+    const int cl = blockIdx.x / KS, ng = cl / pl.jt, j = cl % pl.jt;  // batch group, unit tile [64j, 64j+64)
+    const int b0 = ng * BT;
+    unsigned int *counter = p.counters + ng;
+    const int kcq = 2 * KP + pl.left, c_first = kq * kcq;  // 64-wide K chunks of this CTA
+    const CUtensorMap *tm_dg = &maps.half[kq];
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < ST; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        mbar_init(lfull, 1);
+        mbar_init(lempty, 1);
+        mbar_init(tfull, 1);
+        mbar_init(tempty, kEpilogueThreads / 32);
+        mbar_init(wbar, 1);
+        mbar_init(&rbar[0], 1);
+        mbar_init(&rbar[1], 1);
+        *abort_w = 0;
+        fence_barrier_init();
+        tma_prefetch_desc(&tm_w);
+        tma_prefetch_desc(tm_dg);
+        if (pl.left) tma_prefetch_desc(&maps.chunk);
+    }
+    if (warp == 5) {
+        tmem_alloc(tmem_slot, kTmemColumns);
+        tmem_relinquish();
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + N;
+    // W_hh^T into tensor memory: lane l takes unit l % 64 and K half l / 64, 32 columns of two K elements per chunk-step; the
+    // warps 0-3 take the even chunk-steps, 6-9 the odd ones (a warp reaches the lane quadrant warp % 4)
+    if (warp < 4 || warp > 5) {
+        const int quad = warp & 3, l = quad * 32 + lane;
+        const uint16_t *src = static_cast<const uint16_t *>(p.w_hh) + (size_t)(c_first + (l >> 6) * KP) * 64 * p.H + j * 64 + (l & 63);
+        for (int c = warp < 4 ? 0 : 1; c < CT; c += 2) {
+            uint32_t r[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const uint16_t *e = src + (size_t)(c * 64 + 2 * i) * p.H;
+                r[i] = (uint32_t)__ldg(e) | (uint32_t)__ldg(e + p.H) << 16;
+            }
+            tmem_st_32x32b_x32(tmem_a + ((uint32_t)(quad * 32) << 16) + c * 32, r);
+        }
+        tmem_st_wait();
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    cluster_sync_all();  // every CTA's barriers exist before any remote arrive
+    tcgen05_fence_after();
+    const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
+    const int s_first = p.s0 > 1 ? p.s0 : 1;  // iteration s handles time T-1-s and, from s = 1 on, contracts dG_{T-s}
+    const bool tracing = p.trace != nullptr && blockIdx.x == 0;
+#define FLSTM_STAMP(step, slot)                                                     \
+    do {                                                                            \
+        if (tracing && (step) < p.trace_steps) p.trace[(step) * 16 + (slot)] = clock64(); \
+    } while (0)
+
+    if (warp == 4) {
+        // ------------------------------------------------------------ producer
+        if (elect_one()) {
+            bool ok = true;
+            if (CS > 0 || pl.left) {
+                mbar_expect_tx(wbar, (uint32_t)(L.w + L.left_w));
+                for (int c = 0; c < CS; ++c)
+                    for (int h = 0; h < 2; ++h)
+                        tma_load_2d(s_w + c * kStepBytesW + h * 8192, &tm_w, j * 64, (c_first + h * KP + CT + c) * 64, wbar);
+                if (pl.left)  // the second block only feeds lanes whose results are ignored
+                    for (int h = 0; h < 2; ++h) tma_load_2d(s_lw + h * 8192, &tm_w, j * 64, (c_first + 2 * KP) * 64, wbar);
+            }
+            int stage = 0;
+            uint32_t phase = 0, lphase = 0;
+            uint32_t issued = 0, parity = 0;
+            bool left_issued = false;
+            for (int s = s_first; s < p.s1 && ok; ++s) {
+                const int t_src = p.T - s;
+                if (s > p.s0)
+                    ok = wait_counter(counter, (unsigned)(pl.jt * KS) * (unsigned)(s - p.s0) + p.extra_arrivals, p.err, abort_w, 3u, wait_ns);
+                if (!ok) break;
+                fence_proxy_async_global();
+                FLSTM_STAMP(s - p.s0, 0);
+                for (int ld = 0; ld < NLOAD; ++ld) {
+                    ok = mbar_wait(&empty[stage], phase ^ 1, abort_w, wait_ns);
+                    if (!ok) break;
+                    mbar_expect_tx(&full[stage], (uint32_t)stage_bytes);
+                    issued |= 1u << stage;
+                    parity = (parity & ~(1u << stage)) | (phase << stage);
+                    // (x, row, K half, chunk of the half, step); chunks beyond the half come as zeros (and are counted)
+                    tma_load_5d(s_ring + stage * stage_bytes, tm_dg, 0, b0, 0, ld * CH, t_src, &full[stage]);
+                    if (++stage == ST) { stage = 0; phase ^= 1; }
+                }
+                if (ok && pl.left) {
+                    ok = mbar_wait(lempty, lphase ^ 1, abort_w, wait_ns);
+                    if (!ok) break;
+                    mbar_expect_tx(lfull, BT * 128);
+                    tma_load_4d(s_left, &maps.chunk, 0, b0, c_first + 2 * KP, t_src, lfull);
+                    left_issued = true;
+                    lphase ^= 1;
+                }
+                FLSTM_STAMP(s - p.s0, 1);
+            }
+            // way out (normal or aborted): every copy this thread started must have landed before the CTA exits
+            if (CS > 0 || pl.left) mbar_drain(wbar, 0, wait_ns);
+            for (int i = 0; i < ST; ++i)
+                if (issued >> i & 1u) mbar_drain(&full[i], parity >> i & 1u, wait_ns);
+            if (left_issued) mbar_drain(lfull, lphase ^ 1, wait_ns);
+        }
+    } else if (warp == 5) {
+        // ------------------------------------------------------------ UMMA issuer
+        if (elect_one()) {
+            bool ok = (CS == 0 && !pl.left) || mbar_wait(wbar, 0, abort_w, wait_ns);
+            int stage = 0;
+            uint32_t phase = 0;
+            const uint32_t idesc_ts = umma_idesc_f16(128, N, BF16 ? 1 : 0, 0, 0), idesc_ss = umma_idesc_f16(128, N, BF16 ? 1 : 0, 1, 0);
+            const uint32_t idesc_left = umma_idesc_f16(128, BT, BF16 ? 1 : 0, 1, 0);
+            const uint64_t dw_res = umma_desc_mnmajor_sw128(smem_u32(s_w), 8192);
+            int committed = 0;
+            for (int s = s_first; s < p.s1 && ok; ++s) {
+                const uint32_t wi = (uint32_t)(s - s_first);
+                ok = mbar_wait(tempty, (wi & 1) ^ 1, abort_w, wait_ns);
+                if (!ok) break;
+                tcgen05_fence_after();
+                for (int ld = 0; ld < NLOAD; ++ld) {
+                    ok = mbar_wait(&full[stage], phase, abort_w, wait_ns);
+                    if (!ok) break;
+                    if (ld == 0) FLSTM_STAMP(s - p.s0, 2);
+                    if (ld == NLOAD - 1) FLSTM_STAMP(s - p.s0, 3);
+                    tcgen05_fence_after();
+                    uint64_t dd = umma_desc_kmajor_sw128(smem_u32(s_ring + stage * stage_bytes));
+                    const int c1 = (ld + 1) * CH < KP ? (ld + 1) * CH : KP;
+                    int c = ld * CH;
+                    const int ct1 = c1 < CT ? c1 : CT;
+                    uint32_t da = tmem_a + (uint32_t)c * 32;
+#pragma unroll 4
+                    for (; c < ct1; ++c) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) umma_f16_ts(tmem_base, da + 8 * k, dd + 2 * k, idesc_ts, (uint32_t)(c | k));
+                        da += 32;
+                        dd += (N * 128) >> 4;
+                    }
+                    for (; c < c1; ++c) {
+                        const uint64_t dw = dw_res + (uint64_t)((c - CT) * (kStepBytesW >> 4));
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) umma_f16(tmem_base, dw + 128 * k, dd + 2 * k, idesc_ss, (uint32_t)(c | k));
+                        dd += (N * 128) >> 4;
+                    }
+                    umma_commit(&empty[stage]);
+                    if (++stage == ST) { stage = 0; phase ^= 1; }
+                }
+                if (!ok) break;
+                if (pl.left) {
+                    ok = mbar_wait(lfull, wi & 1, abort_w, wait_ns);
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                    const uint64_t dw = umma_desc_mnmajor_sw128(smem_u32(s_lw), 8192), dd = umma_desc_kmajor_sw128(smem_u32(s_left));
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) umma_f16(tmem_base, dw + 128 * k, dd + 2 * k, idesc_left, 1u);
+                    umma_commit(lempty);
+                }
+                umma_commit(tfull);
+                ++committed;
+                FLSTM_STAMP(s - p.s0, 4);
+            }
+            // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
+            if (committed > 0) mbar_drain(tfull, (uint32_t)(committed - 1) & 1u, wait_ns);
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue (256 threads)
+        const int tid = warp < 4 ? threadIdx.x : threadIdx.x - 64;  // 0..255
+        const int u16 = tid & 15, nb = tid >> 4;  // unit u16 of the CTA's 16, sequences nb + 16 i
+        const int U = j * 64 + kq * UPO + u16;
+        const size_t slab = (size_t)p.B * p.H, G = (size_t)4 * p.H;
+        const uint16_t *gates = static_cast<const uint16_t *>(p.gates);
+        const uint16_t *dy = static_cast<const uint16_t *>(p.dy);
+        const uint16_t *dhn = static_cast<const uint16_t *>(p.dhn);
+        const uint16_t *dcn = static_cast<const uint16_t *>(p.dcn);
+        uint16_t *dg = static_cast<uint16_t *>(p.dg);
+        const int quad = warp & 3, col0 = warp < 4 ? 0 : BT / 2;  // lane quadrant, half of the columns
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (quad >> 1) * BT + col0;
+        const uint32_t red_local = smem_u32(s_red), rbar_local = smem_u32(rbar);
+        float dc_keep[PAIRS];
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            const int b = b0 + nb + 16 * i;
+            const size_t idx = (size_t)b * p.H + U;
+            dc_keep[i] = b >= p.B ? 0.f : p.s0 > 0 ? p.dc[idx] : dcn ? load16<BF16>(dcn + idx) : 0.f;
+        }
+        bool ok = true;
+        for (int s = p.s0; s < p.s1 && ok; ++s) {
+            const int t = p.T - 1 - s;  // time step whose dG is produced (t = -1: only dh0 / dc0)
+            // dG and the carried dc are linear in dh and dc: everything else is formed ahead of the wait
+            struct Factors {
+                float dy, ka, ki, kf, kg, ko, gf;
+            };
+            Factors fac[PAIRS];
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const int b = b0 + nb + 16 * i;
+                fac[i] = Factors{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                if (b < p.B && t >= 0) {
+                    const uint16_t *grow = gates + ((size_t)t * p.B + b) * G + (size_t)(U >> 4) * 64 + (U & 15);
+                    const size_t idx = (size_t)b * p.H + U;
+                    const float gi = load16<BF16>(grow), gf = load16<BF16>(grow + 16), gg = load16<BF16>(grow + 32), go = load16<BF16>(grow + 48);
+                    const float tc = tanh_sel<ACCURATE>(p.cs[(size_t)(t + 1) * slab + idx]), cp = p.cs[(size_t)t * slab + idx];
+                    fac[i] = Factors{load16<BF16>(dy + (size_t)t * slab + idx), go * (1.f - tc * tc), gg * gi * (1.f - gi),
+                                     cp * gf * (1.f - gf), gi * (1.f - gg * gg), tc * go * (1.f - go), gf};
+                }
+            }
+            // dh contribution from the step above: reduce-scattered partial products
+            float dh_in[PAIRS];
+            if (s == 0) {
+#pragma unroll
+                for (int i = 0; i < PAIRS; ++i) {
+                    const int b = b0 + nb + 16 * i;
+                    dh_in[i] = (dhn && b < p.B) ? load16<BF16>(dhn + (size_t)b * p.H + U) : 0.f;
+                }
+            } else {
+                const uint32_t wi = (uint32_t)(s - s_first);
+                const int rb = wi & 1;
+                // No thread leaves between here and the second named barrier below, whatever its waits return: the barriers
+                // OR the failures, so that all 256 threads go on or give up together.
+                bool good = __all_sync(0xffffffffu, mbar_wait(tfull, wi & 1, abort_w, wait_ns));
+                if (tid == 0) FLSTM_STAMP(s - p.s0, 5);
+                tcgen05_fence_after();
+                if (good) {
+                    uint32_t acc[BT / 2];
+                    if (BT == 32) tmem_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(&acc[0]));
+                    else tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&acc[0]));
+                    tmem_ld_wait();
+                    float4 *dst = reinterpret_cast<float4 *>(s_ps + (quad * 32 + lane) * RS + col0);
+#pragma unroll
+                    for (int i = 0; i < BT / 8; ++i)
+                        dst[i] = make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]),
+                                             __uint_as_float(acc[4 * i + 2]), __uint_as_float(acc[4 * i + 3]));
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(tempty);
+                const bool failed = named_barrier_or(1, kEpilogueThreads, !good);
+                if (!failed) {
+                    // UPO rows of BT sums for this CTA arrive from every CTA of the cluster, its own included
+                    if (tid == 0) mbar_expect_tx(&rbar[rb], (uint32_t)(KS * UPO * BT * 4));
+                    constexpr int V = BT / 4;  // 16-byte pieces of a row
+#pragma unroll
+                    for (int i = 0; i < 64 * V / kEpilogueThreads; ++i) {
+                        const int e = tid + i * kEpilogueThreads, row = e / V, v = e % V;
+                        const float4 a = *reinterpret_cast<const float4 *>(s_ps + row * RS + 4 * v);
+                        const float4 b = *reinterpret_cast<const float4 *>(s_ps + (64 + row) * RS + 4 * v);
+                        const uint32_t owner = row / UPO, off = (uint32_t)(((rb * KS + kq) * UPO + row % UPO) * RS + 4 * v) * 4u;
+                        st_async_v4(map_to_rank(red_local + off, owner), __float_as_uint(a.x + b.x), __float_as_uint(a.y + b.y),
+                                    __float_as_uint(a.z + b.z), __float_as_uint(a.w + b.w), map_to_rank(rbar_local + rb * 8, owner));
+                    }
+                    if (tid == 0) FLSTM_STAMP(s - p.s0, 9);
+                    good = mbar_wait_cluster(&rbar[rb], (wi >> 1) & 1, abort_w, wait_ns);
+                } else {
+                    good = false;
+                }
+                if (tid == 0) FLSTM_STAMP(s - p.s0, 10);
+                const float *red = s_red + (size_t)rb * KS * UPO * RS;
+#pragma unroll
+                for (int i = 0; i < PAIRS; ++i) {
+                    float acc = 0.f;
+#pragma unroll
+                    for (int src = 0; src < KS; ++src) acc += red[(src * UPO + u16) * RS + nb + 16 * i];
+                    dh_in[i] = acc;
+                }
+                // one warp's failure is everybody's
+                if (named_barrier_or(1, kEpilogueThreads, !good)) {
+                    ok = false;
+                    break;
+                }
+                if (tid == 0) FLSTM_STAMP(s - p.s0, 6);
+            }
+            // fused pointwise backward for the owned (unit, sequence) pairs
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const int b = b0 + nb + 16 * i;
+                if (b >= p.B) continue;
+                const size_t idx = (size_t)b * p.H + U;
+                if (t < 0) {
+                    if (p.dh0) p.dh0[idx] = dh_in[i];
+                    if (p.dc0) p.dc0[idx] = dc_keep[i];
+                    continue;
+                }
+                const Factors &f = fac[i];
+                const float dh = ACCURATE && U >= p.real_units ? 0.f : f.dy + dh_in[i];
+                const float dcv = fmaf(dh, f.ka, dc_keep[i]);
+                dc_keep[i] = dcv * f.gf;
+                uint16_t *drow = dg + ((size_t)t * p.B + b) * G + (size_t)(U >> 4) * 64 + (U & 15);
+                drow[0] = to16<BF16>(dcv * f.ki);
+                drow[16] = to16<BF16>(dcv * f.kf);
+                drow[32] = to16<BF16>(dcv * f.kg);
+                drow[48] = to16<BF16>(dh * f.ko);
+            }
+            if (t >= 0) {
+                if (tid == 0) FLSTM_STAMP(s - p.s0, 7);
+                // publish dG_t: ONE arrival per CTA; after the named barrier thread 0's release is cumulative over every
+                // epilogue warp's stores, the generic->async proxy fence is the consumer's
+                named_barrier_sync(2, kEpilogueThreads);
+                if (tid == 0) red_release_gpu_add(counter, 1u);
+                if (tid == 0) FLSTM_STAMP(s - p.s0, 8);
+            }
+        }
+        // a later launch continues the recurrence: leave the cell-gradient carry where it will look for it
+        if (ok && p.s1 <= p.T) {
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const int b = b0 + nb + 16 * i;
+                if (b < p.B) p.dc[(size_t)b * p.H + U] = dc_keep[i];
+            }
+        }
+    }
+#undef FLSTM_STAMP
+    tcgen05_fence_before();
+    __syncthreads();
+    cluster_sync_all();  // nobody leaves while a peer may still send into its shared memory
+    if (*abort_w) {
+        // after an abort this CTA may not have waited for partial sums that a peer sent before it reached the barrier
+        // above: give those asynchronous stores time to land before the shared memory is released
+        const unsigned long long t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < kAbortDrainNs) {}
+    }
+    if (warp == 5) tmem_dealloc(tmem_base, kTmemColumns);
+    if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
+    if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / (pl.jt * KS), p.exits);
+}
+
+void cluster_attr(cudaLaunchAttribute *a) {
+    a->id = cudaLaunchAttributeClusterDimension;
+    a->val.clusterDim.x = KS;
+    a->val.clusterDim.y = 1;
+    a->val.clusterDim.z = 1;
+}
+
+template <int BT, bool BF16, bool ACC>
+int launch_one(const CUtensorMap &tw, const BwdTmMaps &maps, const BwdTmPlan &pl, const BwdParams &p, cudaStream_t s) {
+    auto kern = lstm_bwd_tm_kernel<BT, BF16, ACC>;
+    FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)pl.smem_bytes));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = pl.smem_bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeCooperative;  // co-residency: CTAs wait on one another
+    attr[0].val.cooperative = 1;
+    cluster_attr(&attr[1]);
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, maps, pl, p);
+    if (e == cudaErrorNotSupported || e == cudaErrorInvalidValue) {
+        // as in tc_lstm_bwd.cu: planning has proved that every cluster is resident at once
+        cudaGetLastError();
+        cfg.attrs = attr + 1;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, kern, tw, maps, pl, p);
+    }
+    if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "BPTT launch failed: %s", cudaGetErrorString(e));
+    return FLSTM_OK;
+}
+
+// clusters of this plan that the current device holds at once, or -1
+template <int BT>
+int max_clusters(const BwdTmPlan &pl) {
+    auto kern = lstm_bwd_tm_kernel<BT, false, false>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = pl.smem_bytes;
+    cudaLaunchAttribute attr[1];
+    cluster_attr(attr);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (ensure_smem_limit(kern, (size_t)pl.smem_bytes) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    return n;
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ host side
+int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool check_device) {
+    *plan = BwdTmPlan{};
+    if (H % 64 != 0 || H < 256 || smem_limit < 160 * 1024) return FLSTM_OK;
+    const char *env = std::getenv("FLSTM_BWD_TM");
+    if (env && env[0] == '0') return FLSTM_OK;
+    BwdTmPlan pl{};
+    pl.jt = H / 64;
+    if (pl.jt * KS > sms) return FLSTM_OK;
+    const int groups = sms / (pl.jt * KS);
+    for (int bt = 32; bt <= 64 && !pl.BT; bt *= 2)
+        if ((B + bt - 1) / bt <= groups) pl.BT = bt;
+    if (!pl.BT) return FLSTM_OK;
+    pl.ngroups = (B + pl.BT - 1) / pl.BT;
+    const int kcq = H / 16 / KS;
+    pl.kp = kcq / 2;
+    pl.left = kcq % 2;
+    const int tmem_steps = (kTmemColumns - 2 * pl.BT) / 32, step_bytes = 2 * pl.BT * 128;
+    pl.ct = pl.kp < tmem_steps ? pl.kp : tmem_steps;
+    pl.cs = pl.kp - pl.ct;
+    // dG in copies of up to 64 KB, the whole tile at once if it fits
+    pl.ch = 65536 / step_bytes < pl.kp ? 65536 / step_bytes : pl.kp;
+    if (const char *e = std::getenv("FLSTM_TM_BCH")) pl.ch = std::atoi(e) < pl.kp ? std::atoi(e) : pl.kp;
+    pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
+    auto fits = [&]() { return (size_t)layout_of(pl).total <= smem_limit; };
+    while (!fits() && pl.ch > 1) {
+        pl.ch = pl.ch > 2 ? 2 : 1;
+        pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
+        while (!fits() && pl.stages > 2) --pl.stages;
+    }
+    if (!fits()) return FLSTM_OK;
+    pl.smem_bytes = layout_of(pl).total;
+    if (pl.smem_bytes < 120 * 1024) pl.smem_bytes = 120 * 1024;  // one CTA per SM: each allocates all of tensor memory
+    pl.grid = pl.jt * KS * pl.ngroups;
+    if (check_device && (pl.BT == 32 ? max_clusters<32>(pl) : max_clusters<64>(pl)) * KS < pl.grid) return FLSTM_OK;
+    pl.use = true;
+    *plan = pl;
+    return FLSTM_OK;
+}
+
+int make_bwd_tm_maps(BwdTmMaps *maps, const BwdTmPlan &pl, const void *dg, size_t steps, size_t B, size_t H) {
+    for (int kq = 0; kq < KS; ++kq)
+        FLSTM_TRY(make_tensor_map_halves(&maps->half[kq], static_cast<const char *>(dg) + (size_t)kq * (2 * pl.kp + pl.left) * 128, steps, B,
+                                         4 * H, pl.BT, pl.kp, pl.ch));
+    if (pl.left) FLSTM_TRY(make_tensor_map_chunked(&maps->chunk, dg, steps, B, 4 * H, pl.BT, 1));
+    return FLSTM_OK;
+}
+
+int lstm_backward_tm(int dtype, const BwdTmPlan &pl, const CUtensorMap &tw, const BwdTmMaps &maps, const BwdParams &p, cudaStream_t s) {
+    const bool bf16 = dtype == FLSTM_DTYPE_BF16, acc = p.real_units > 0;
+#define FLSTM_TM_CASE(BT_)                                                                                                \
+    if (pl.BT == BT_) {                                                                                                   \
+        if (bf16) return acc ? launch_one<BT_, true, true>(tw, maps, pl, p, s) : launch_one<BT_, true, false>(tw, maps, pl, p, s); \
+        return acc ? launch_one<BT_, false, true>(tw, maps, pl, p, s) : launch_one<BT_, false, false>(tw, maps, pl, p, s); \
+    }
+    FLSTM_TM_CASE(32) FLSTM_TM_CASE(64)
+#undef FLSTM_TM_CASE
+    return set_error(FLSTM_ERR_UNSUPPORTED, "no tensor-memory BPTT kernel for this plan");
+}
+
+}  // namespace tc
+}  // namespace flstm_b200

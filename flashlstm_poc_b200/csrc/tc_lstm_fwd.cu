@@ -284,27 +284,23 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     if (ld == 0) FLSTM_STAMP((int)(it / items_per_step), 2);
                     if (ld == NLOAD - 1) FLSTM_STAMP((int)(it / items_per_step), 3);
                     tcgen05_fence_after();
+                    // one descriptor per stage and operand, advanced by constants in an unrolled loop (see the BPTT kernel);
+                    // the further K steps of 16 elements advance the start-address field by 32 bytes
                     const uint32_t st_base = smem_u32(s_ring + stage * L.ring_stage_bytes);
+                    uint64_t dh = umma_desc_kmajor_sw128(st_base);
+                    uint64_t dw = umma_desc_kmajor_sw128(W_RESIDENT ? s_w_u32 + (uint32_t)(r * KC + ld * CH) * kChunkBytesW
+                                                                    : st_base + CH * BTH * 128);
+                    uint32_t acc = ld != 0;
+#pragma unroll 4
                     for (int c = 0; c < CH; ++c) {
-                        const int kc = ld * CH + c;
-                        const uint32_t h_base = st_base + c * BTH * 128;
-                        const uint32_t w_base = W_RESIDENT ? s_w_u32 + (uint32_t)(r * KC + kc) * kChunkBytesW
-                                                           : st_base + CH * BTH * 128 + c * kChunkBytesW;
-                        // one descriptor per chunk; the three further K steps of 16 elements advance the
-                        // start-address field by 32 bytes (2 in descriptor units)
-                        const uint64_t dw = umma_desc_kmajor_sw128(w_base), dh = umma_desc_kmajor_sw128(h_base);
-                        if (PAIR) {
-                            umma_f16_pair(d_tmem, dw, dh, idesc, kc != 0);
-                            umma_f16_pair(d_tmem, dw + 2, dh + 2, idesc, 1u);
-                            umma_f16_pair(d_tmem, dw + 4, dh + 4, idesc, 1u);
-                            umma_f16_pair(d_tmem, dw + 6, dh + 6, idesc, 1u);
-                        } else {
-                            if (kc == 0) umma_f16_imm<false>(d_tmem, dw, dh, idesc);
-                            else umma_f16_imm<true>(d_tmem, dw, dh, idesc);
-                            umma_f16_imm<true>(d_tmem, dw + 2, dh + 2, idesc);
-                            umma_f16_imm<true>(d_tmem, dw + 4, dh + 4, idesc);
-                            umma_f16_imm<true>(d_tmem, dw + 6, dh + 6, idesc);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if (PAIR) umma_f16_pair(d_tmem, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                            else umma_f16(d_tmem, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
                         }
+                        acc = 1u;
+                        dw += kChunkBytesW >> 4;
+                        dh += (BTH * 128) >> 4;
                     }
                     // the stage may be refilled (PAIR: in both CTAs) once these UMMAs have read it
                     if (PAIR) umma_commit_pair_both(empty_l + 8u * (uint32_t)stage);

@@ -1,0 +1,49 @@
+"""The recurrent kernels that hold W_hh in tensor memory (tc_lstm_fwd_tm.cu, tc_lstm_bwd_tm.cu) against the oracle, at the edges
+of their tiling: an odd and an even number of 64-wide K chunks per half, weights in tensor memory only, beside shared memory
+and streamed, every batch-tile width, partly filled tiles, one and two batch groups, and step ranges that continue a launch."""
+import pytest
+import torch
+
+from flashlstm_poc_b200.engine import TORCH_DTYPES, Engine
+from flashlstm_poc_b200.workloads import Workload, make_inputs
+from tests.gpu_helpers import assert_parity, run_engine, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+# batch, hidden size, training
+SHAPES = [(1, 1088, True), (70, 1088, True), (33, 1152, True), (100, 1152, True), (40, 1216, True), (32, 1280, True),
+          (5, 2048, True), (64, 2048, True), (31, 2304, True), (50, 2368, True),
+          (3, 2432, False), (16, 2496, False), (17, 3072, False), (33, 4096, False), (8, 4096, False), (64, 2560, False)]
+
+
+@pytest.mark.parametrize("B,H,training", SHAPES)
+def test_tensor_memory_kernels_match_the_oracle(B, H, training):
+    dtype = "bf16" if (B + H // 64) % 2 else "f16"
+    w = Workload("t", dtype, 1, 64, H, B, 5, seed=51, state_std=0.3, training=training)
+    inp = make_inputs(w)
+    got, eng = run_engine(w, inp, repeat=2)
+    eng.close()
+    assert_parity(got, run_oracle(inp), dtype)
+
+
+@pytest.mark.parametrize("B,H", [(7, 1088), (40, 2048)])
+def test_ranges_continue_one_another(B, H):
+    """Forward and backward in step ranges equal one call."""
+    w = Workload("t", "f16", 1, 64, H, B, 7, seed=52, state_std=0.3)
+    inp = make_inputs(w)
+    dev, td = torch.device("cuda", 0), TORCH_DTYPES["f16"]
+    eng = Engine("f16", 1, B, 64, H, 7, device=dev)
+    eng.set_weights(0, inp.w_ih[0].to(dev), inp.w_hh[0].to(dev), inp.b_ih[0].to(dev), inp.b_hh[0].to(dev))
+    x, h0, c0, dy = (t.to(dev, td) for t in (inp.x, inp.h0, inp.c0, inp.dy))
+    y, hn, cn = eng.forward(x, h0, c0)
+    dx, dh0, dc0 = eng.backward(dy)
+    want = [t.clone() for t in (y, hn, cn, dx, dh0, dc0)]
+    got = [torch.empty_like(t) for t in want]
+    for t0, t1 in ((0, 3), (3, 4), (4, 7)):
+        eng.forward_range_into(7, t0, t1, x, h0, c0, *got[:3])
+    for t0, t1 in ((5, 7), (1, 5), (0, 1)):
+        eng.backward_range_into(7, t0, t1, dy, None, None, *got[3:])
+    torch.cuda.synchronize()
+    eng.close()
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)

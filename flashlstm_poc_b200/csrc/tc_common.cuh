@@ -305,22 +305,13 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// The same with A in tensor memory, K-major: lane = row, a 32-bit column holds two consecutive K elements, so an
-// instruction (K = 16) reads 8 columns.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // The mbarrier gets one arrival when every UMMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+__device__ __forceinline__ void umma_commit_addr(uint32_t bar_local_addr) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_local_addr) : "memory");
 }
 
 // ------------------------------------------------------------------ CTA pairs (cta_group::2)
@@ -386,18 +377,6 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// A in the tensor memory of both CTAs (M = 256: each holds its 128 rows at the same columns)
-__device__ __forceinline__ void umma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 template <bool ACC>
 __device__ __forceinline__ void umma_f16_pair_imm(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
     umma_f16_pair(d_tmem, a_desc, b_desc, idesc, ACC ? 1u : 0u);
@@ -451,6 +430,45 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
         }
     }
     return true;
+}
+
+// ------------------------------------------------------------------ UMMA with descriptors by their low word
+// The issuing thread has to move every operand to uniform registers for each instruction.  Of a descriptor only the low word
+// changes from one instruction to the next (start address, leading byte offset): kept as a 32-bit value that advances by
+// constants in unrolled loops an instruction takes about 25 cycles to issue, against 45 to 100 with 64-bit descriptors formed in
+// the loop.
+constexpr uint32_t kUmmaDescHi = 0x40004040u;  // 8-row groups 1024 bytes apart, descriptor version, 128-byte swizzle
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes = 16) {
+    return ((smem_addr & 0x3FFFF) >> 4) | (lbo_bytes >> 4) << 16;
+}
+// D (+)= A B, both operands in shared memory
+template <bool PAIR>
+__device__ __forceinline__ void umma_lo_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    if (PAIR)
+        asm volatile(
+            "{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n}\n"
+            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
+    else
+        asm volatile(
+            "{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
+            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
+}
+// The same with A in tensor memory, K-major: lane = row, a 32-bit column holds two consecutive K elements, so an instruction
+// (K = 16) reads 8 columns.  PAIR: M = 256, each CTA holds its 128 rows at the same columns.
+template <bool PAIR>
+__device__ __forceinline__ void umma_lo_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    if (PAIR)
+        asm volatile(
+            "{\n.reg .pred p;\n.reg .b64 b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 b, {%2, %5};\n"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], b, %3, p;\n}\n"
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
+    else
+        asm volatile(
+            "{\n.reg .pred p;\n.reg .b64 b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 b, {%2, %5};\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n"
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
 }
 
 // ------------------------------------------------------------------ host: tensor maps

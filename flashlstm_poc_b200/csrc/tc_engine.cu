@@ -27,6 +27,7 @@ struct TcLayer {
     CUtensorMap tm_h;   // hs (Tcap+1, B, H), 1 x BT x 64 boxes, 128B swizzle
     CUtensorMap tm_g;   // gates (Tcap, B, 4H), 1 x BT x 64 boxes, no swizzle
     CUtensorMap tm_dg;  // dG (Tcap, B, 4H), 1 x BT x 64 boxes, 128B swizzle (BPTT operand)
+    CUtensorMap tm_ws;  // w_hh, 128 x 64 boxes (streamed part of the tensor-memory forward)
     BwdTmMaps dg_tm;    // dG for the tensor-memory BPTT kernel
     // wide-batch path (one GEMM launch per step)
     CUtensorMap tm_hs3;    // hs (Tcap+1, B, H), 1 x 128 x 64 boxes, 128B swizzle
@@ -219,6 +220,7 @@ int on_capacity_change(Engine &e) {
         if (st->fwdtm.use) {
             FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->fwdtm.S * st->fwdtm.BT / 2, st->fwdtm.ch));
             FLSTM_TRY(make_tensor_map_3d(&t.tm_g, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwdtm.BT, 64, false));
+            if (st->fwdtm.wstages) FLSTM_TRY(make_tensor_map_chunked(&t.tm_ws, l.w_hh, 1, 4 * H, H, 128, kFwdTmGroup));
         }
         if (st->step.use) {
             FLSTM_TRY(make_tensor_map_3d(&t.tm_hs3, l.hs, cap + 1, B, H, H, B * H, 128, 64, true));
@@ -379,7 +381,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
     p.w_hh = l.w_hh;
-    if (st->fwdtm.use) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_h, t.tm_g, p, s));
+    if (st->fwdtm.use) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h, t.tm_g, p, s));
     else FLSTM_TRY(lstm_forward_persistent(e.cfg.dtype, st->fwd, t.tm_w, t.tm_h, t.tm_g, p, s));
     size_t m2 = e.timer.mark(s);
     e.timer.span(PH_PROJ, m0, m1);

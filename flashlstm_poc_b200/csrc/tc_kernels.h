@@ -80,14 +80,16 @@ struct FwdTmPlan {
     int kc;        // chunk-steps of 64 along K (per half for S = 2)
     int ct, cs;    // of these, kept in tensor / shared memory; the others are streamed each step
     int ch, hstages;  // chunk-steps of h per copy, copies in the ring
-    int wstages;   // ring of streamed chunk-steps of W_hh (0: nothing is streamed)
+    int wstages;   // slots for copies of streamed W_hh (0: nothing is streamed)
+    int hring;     // 0: the copies of h hold a whole tile, they need no hand-back
     int smem_bytes;
     int grid;
 };
+constexpr int kFwdTmGroup = 3;  // streamed chunk-steps per copy
 int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan);
-// tm_w: W_hh as for lstm_forward_persistent.  tm_h: chunked map with box rows S * BT / 2 and plan.ch chunks.  tm_g: box 1 x BT x 64.
-int lstm_forward_tm(int dtype, const FwdTmPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_h, const CUtensorMap &tm_g,
-                    const FwdParams &p, cudaStream_t s);
+// tm_w: W_hh as for lstm_forward_persistent.  tm_ws: W_hh as a chunked map of one step, box rows 128, kFwdTmGroup chunks.  tm_h: chunked map with box rows S * BT / 2 and plan.ch chunks.  tm_g: box 1 x BT x 64.
+int lstm_forward_tm(int dtype, const FwdTmPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_ws, const CUtensorMap &tm_h,
+                    const CUtensorMap &tm_g, const FwdParams &p, cudaStream_t s);
 
 // ------------------------------------------------------------------ persistent BPTT
 struct BwdPlan {
@@ -143,6 +145,7 @@ struct BwdTmPlan {
     int left;      // 1: the range has an odd number of chunks, the last one runs by itself
     int ct, cs;    // chunk-steps of W_hh in tensor / shared memory (all of them)
     int ch, stages;  // chunk-steps of dG per copy, copies in the ring
+    int ring;      // 0: the copies hold a whole tile, they need no hand-back
     int smem_bytes;
     int grid;
 };

@@ -68,7 +68,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     uint8_t *s_w = smem, *s_lw = s_w + L.w, *s_ring = s_lw + L.left_w, *s_left = s_ring + L.ring;
     float *s_ps = reinterpret_cast<float *>(s_left + L.left), *s_red = s_ps + L.ps / 4;
     uint64_t *full = reinterpret_cast<uint64_t *>(s_red + L.red / 4), *empty = full + ST;
-    uint64_t *lfull = empty + ST, *lempty = lfull + 1, *tfull = lempty + 1, *tempty = tfull + 1, *wbar = tempty + 1;
+    uint64_t *lfull = empty + ST, *tfull = lfull + 1, *tempty = tfull + 1, *wbar = tempty + 1;
     uint64_t *rbar = wbar + 1;  // [2] partial sums received
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(rbar + 2);
     volatile uint32_t *abort_w = tmem_slot + 1;
@@ -87,7 +87,6 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             mbar_init(&empty[i], 1);
         }
         mbar_init(lfull, 1);
-        mbar_init(lempty, 1);
         mbar_init(tfull, 1);
         mbar_init(tempty, kEpilogueThreads / 32);
         mbar_init(wbar, 1);
@@ -159,7 +158,8 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 fence_proxy_async_global();
                 FLSTM_STAMP(s - p.s0, 0);
                 for (int ld = 0; ld < NLOAD; ++ld) {
-                    ok = mbar_wait(&empty[stage], phase ^ 1, abort_w, wait_ns);
+                    // (without a ring the tile is free: the step barrier came after the UMMAs that read it)
+                    if (pl.ring) ok = mbar_wait(&empty[stage], phase ^ 1, abort_w, wait_ns);
                     if (!ok) break;
                     mbar_expect_tx(&full[stage], (uint32_t)stage_bytes);
                     issued |= 1u << stage;
@@ -169,8 +169,6 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     if (++stage == ST) { stage = 0; phase ^= 1; }
                 }
                 if (ok && pl.left) {
-                    ok = mbar_wait(lempty, lphase ^ 1, abort_w, wait_ns);
-                    if (!ok) break;
                     mbar_expect_tx(lfull, BT * 128);
                     tma_load_4d(s_left, &maps.chunk, 0, b0, c_first + 2 * KP, t_src, lfull);
                     left_issued = true;
@@ -187,61 +185,67 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     } else if (warp == 5) {
         // ------------------------------------------------------------ UMMA issuer
         if (elect_one()) {
-            bool ok = (CS == 0 && !pl.left) || mbar_wait(wbar, 0, abort_w, wait_ns);
-            int stage = 0;
-            uint32_t phase = 0;
-            const uint32_t idesc_ts = umma_idesc_f16(128, N, BF16 ? 1 : 0, 0, 0), idesc_ss = umma_idesc_f16(128, N, BF16 ? 1 : 0, 1, 0);
-            const uint32_t idesc_left = umma_idesc_f16(128, BT, BF16 ? 1 : 0, 1, 0);
-            const uint64_t dw_res = umma_desc_mnmajor_sw128(smem_u32(s_w), 8192);
-            int committed = 0;
-            for (int s = s_first; s < p.s1 && ok; ++s) {
-                const uint32_t wi = (uint32_t)(s - s_first);
-                ok = mbar_wait(tempty, (wi & 1) ^ 1, abort_w, wait_ns);
+        bool ok = (CS == 0 && !pl.left) || mbar_wait(wbar, 0, abort_w, wait_ns);
+        int stage = 0;
+        uint32_t phase = 0;
+        constexpr uint32_t idesc_ts = umma_idesc_f16(128, N, BF16 ? 1 : 0, 0, 0), idesc_ss = umma_idesc_f16(128, N, BF16 ? 1 : 0, 1, 0);
+        constexpr uint32_t idesc_left = umma_idesc_f16(128, BT, BF16 ? 1 : 0, 1, 0);
+        constexpr uint32_t kStepG = (N * 128) >> 4, kStepW = kStepBytesW >> 4;  // descriptor units
+        const uint32_t dw_res = umma_desc_lo(smem_u32(s_w), 8192), dw_left = umma_desc_lo(smem_u32(s_lw), 8192);
+        const uint32_t dd_ring = umma_desc_lo(smem_u32(s_ring)), dd_left = umma_desc_lo(smem_u32(s_left));
+        const uint32_t empty_l = smem_u32(empty), tfull_l = smem_u32(tfull);
+        int committed = 0;
+        for (int s = s_first; s < p.s1 && ok; ++s) {
+            const uint32_t wi = (uint32_t)(s - s_first);
+            ok = mbar_wait(tempty, (wi & 1) ^ 1, abort_w, wait_ns);
+            if (!ok) break;
+            tcgen05_fence_after();
+            uint32_t acc = 0;  // the step's first instruction overwrites the accumulator
+            for (int ld = 0; ld < NLOAD; ++ld) {
+                ok = mbar_wait(&full[stage], phase, abort_w, wait_ns);
+                if (!ok) break;
+                if (ld == 0) FLSTM_STAMP(s - p.s0, 2);
+                if (ld == NLOAD - 1) FLSTM_STAMP(s - p.s0, 3);
+                tcgen05_fence_after();
+                uint32_t dd = dd_ring + (uint32_t)stage * (uint32_t)(stage_bytes >> 4);
+                const int c1 = (ld + 1) * CH < KP ? (ld + 1) * CH : KP;
+                int c = ld * CH;
+                const int ct1 = c1 < CT ? c1 : CT;
+                uint32_t da = tmem_a + (uint32_t)c * 32;
+#pragma unroll 4
+                for (; c < ct1; ++c) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) umma_lo_ts<false>(tmem_base, da + 8 * k, dd + 2 * k, idesc_ts, k ? 1u : acc);
+                    acc = 1u;
+                    da += 32;
+                    dd += kStepG;
+                }
+                uint32_t dw = dw_res + (uint32_t)(c - CT) * kStepW;
+#pragma unroll 2
+                for (; c < c1; ++c) {  // K steps of 16: +2048 bytes on the MN-major W_hh, +32 bytes on the K-major dG
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) umma_lo_ss<false>(tmem_base, dw + 128 * k, dd + 2 * k, idesc_ss, k ? 1u : acc);
+                    acc = 1u;
+                    dw += kStepW;
+                    dd += kStepG;
+                }
+                if (pl.ring) umma_commit_addr(empty_l + 8u * (uint32_t)stage);
+                if (++stage == ST) { stage = 0; phase ^= 1; }
+            }
+            if (!ok) break;
+            if (pl.left) {
+                ok = mbar_wait(lfull, wi & 1, abort_w, wait_ns);
                 if (!ok) break;
                 tcgen05_fence_after();
-                for (int ld = 0; ld < NLOAD; ++ld) {
-                    ok = mbar_wait(&full[stage], phase, abort_w, wait_ns);
-                    if (!ok) break;
-                    if (ld == 0) FLSTM_STAMP(s - p.s0, 2);
-                    if (ld == NLOAD - 1) FLSTM_STAMP(s - p.s0, 3);
-                    tcgen05_fence_after();
-                    uint64_t dd = umma_desc_kmajor_sw128(smem_u32(s_ring + stage * stage_bytes));
-                    const int c1 = (ld + 1) * CH < KP ? (ld + 1) * CH : KP;
-                    int c = ld * CH;
-                    const int ct1 = c1 < CT ? c1 : CT;
-                    uint32_t da = tmem_a + (uint32_t)c * 32;
-#pragma unroll 4
-                    for (; c < ct1; ++c) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) umma_f16_ts(tmem_base, da + 8 * k, dd + 2 * k, idesc_ts, (uint32_t)(c | k));
-                        da += 32;
-                        dd += (N * 128) >> 4;
-                    }
-                    for (; c < c1; ++c) {
-                        const uint64_t dw = dw_res + (uint64_t)((c - CT) * (kStepBytesW >> 4));
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) umma_f16(tmem_base, dw + 128 * k, dd + 2 * k, idesc_ss, (uint32_t)(c | k));
-                        dd += (N * 128) >> 4;
-                    }
-                    umma_commit(&empty[stage]);
-                    if (++stage == ST) { stage = 0; phase ^= 1; }
-                }
-                if (!ok) break;
-                if (pl.left) {
-                    ok = mbar_wait(lfull, wi & 1, abort_w, wait_ns);
-                    if (!ok) break;
-                    tcgen05_fence_after();
-                    const uint64_t dw = umma_desc_mnmajor_sw128(smem_u32(s_lw), 8192), dd = umma_desc_kmajor_sw128(smem_u32(s_left));
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_f16(tmem_base, dw + 128 * k, dd + 2 * k, idesc_left, 1u);
-                    umma_commit(lempty);
-                }
-                umma_commit(tfull);
-                ++committed;
-                FLSTM_STAMP(s - p.s0, 4);
+                for (int k = 0; k < 4; ++k) umma_lo_ss<false>(tmem_base, dw_left + 128 * k, dd_left + 2 * k, idesc_left, 1u);
             }
-            // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
-            if (committed > 0) mbar_drain(tfull, (uint32_t)(committed - 1) & 1u, wait_ns);
+            umma_commit_addr(tfull_l);
+            ++committed;
+            FLSTM_STAMP(s - p.s0, 4);
+        }
+        // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
+        if (committed > 0) mbar_drain(tfull, (uint32_t)(committed - 1) & 1u, wait_ns);
         }
     } else {
         // ------------------------------------------------------------ epilogue (256 threads)
@@ -470,7 +474,7 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
     pl.jt = H / 64;
     if (pl.jt * KS > sms) return FLSTM_OK;
     const int groups = sms / (pl.jt * KS);
-    for (int bt = 32; bt <= 64 && !pl.BT; bt *= 2)
+    for (int bt = 32; bt <= (H > 1024 ? 64 : 32) && !pl.BT; bt *= 2)
         if ((B + bt - 1) / bt <= groups) pl.BT = bt;
     if (!pl.BT) return FLSTM_OK;
     pl.ngroups = (B + pl.BT - 1) / pl.BT;
@@ -491,6 +495,7 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
         while (!fits() && pl.stages > 2) --pl.stages;
     }
     if (!fits()) return FLSTM_OK;
+    pl.ring = pl.stages * pl.ch < pl.kp;
     pl.smem_bytes = layout_of(pl).total;
     if (pl.smem_bytes < 120 * 1024) pl.smem_bytes = 120 * 1024;  // one CTA per SM: each allocates all of tensor memory
     pl.grid = pl.jt * KS * pl.ngroups;

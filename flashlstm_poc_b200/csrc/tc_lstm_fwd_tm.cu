@@ -14,8 +14,11 @@
 //   S = 1 (wider layers): a CTA owns 128 gate rows (32 units), the pair's B operand is BT sequences, each CTA stages BT / 2.
 // Either way a CTA stages half of what its rows need of h, and nothing is multicast.
 //
-// K runs in chunk-steps of 64 per half: [0, ct) from tensor memory, [ct, ct + cs) from shared memory, the rest streamed through
-// a ring of its own by a warp of its own, which does not wait for the step barrier.  Roles, step barrier, epilogue and the way
+// K runs in chunk-steps of 64 per half: [0, ct) from tensor memory, [ct, ct + cs) from shared memory.  The rest is streamed
+// through a ring of slots by a warp of its own, ascending in even steps of a launch and descending in odd ones: the slots then
+// still hold the chunk-steps that the next step starts with, and L2 is asked first for what it was given last (in one direction
+// 94 MB per step go round in its 126 MB and mostly miss).  A step takes the chunk-steps that the slots hold first, so that
+// copies start as soon as h is there, then those in tensor and shared memory, then the streamed ones.  Roles, step barrier, epilogue and the way
 // out after a bounded wait expired are the other forward kernel's (tc_lstm_fwd.cu): producer and UMMA threads break out of
 // their loops, the 256 epilogue threads leave together, an aborted pair lingers before its final cluster barrier.
 //
@@ -39,6 +42,7 @@ constexpr int kThreads = 352;  // warps 0-3 and 6-9 epilogue, 4 producer of h, 5
 constexpr int kEpilogueThreads = 256;
 constexpr int kStepBytesW = 128 * 128;  // one chunk-step of A: 128 rows x 64 16-bit elements
 constexpr int kTmemColumns = 512;
+constexpr int WCH = kFwdTmGroup;
 
 struct Layout {
     int w, wring, h, p, ex, total;
@@ -47,7 +51,7 @@ struct Layout {
 __host__ __device__ inline Layout layout_of(const FwdTmPlan &pl) {
     Layout l;
     l.w = pl.cs * kStepBytesW;
-    l.wring = pl.wstages * kStepBytesW;
+    l.wring = pl.wstages * WCH * kStepBytesW;
     l.h = pl.hstages * pl.ch * (pl.S * pl.BT / 2) * 128;
     l.p = 2 * (2 / pl.S) * pl.BT * 128;
     l.ex = 128 * (pl.BT + 4) * 4;
@@ -55,9 +59,25 @@ __host__ __device__ inline Layout layout_of(const FwdTmPlan &pl) {
     return l;
 }
 
+// The order in which a step takes its chunk-steps: up to three runs, each ascending or descending, each fetched in copies of
+// ch chunk-steps of h (a last copy brings chunk-steps that are not used).
+struct Run {
+    int lo, hi;  // chunk-steps [lo, hi)
+    __device__ int copies(int ch) const { return (hi - lo + ch - 1) / ch; }
+};
+template <bool STREAM>
+__device__ __forceinline__ Run run_of(const FwdTmPlan &pl, int which, bool down) {
+    const int first = pl.ct + pl.cs;  // first streamed chunk-step
+    if (!STREAM) return Run{0, which == 0 ? pl.kc : 0};
+    if (which == 1) return Run{0, first};
+    const int ring = pl.wstages * WCH, held = down ? pl.kc - ring : first;  // what the slots hold when the step begins
+    if (which == 0) return Run{held, held + ring};
+    return down ? Run{first, pl.kc - ring} : Run{first + ring, pl.kc};
+}
+
 template <int S, int BT, bool STREAM, bool BF16, bool ACCURATE>
 __global__ void __launch_bounds__(kThreads, 1)
-lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_h,
+lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_ws, const __grid_constant__ CUtensorMap tm_h,
                    const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ FwdTmPlan pl, FwdParams p) {
     constexpr int ROWS = 128 / S, UT = 2 / S;  // gate rows and 16-unit tiles of this CTA
     constexpr int N = S * BT, BROWS = N / 2;   // UMMA N, B rows a CTA stages
@@ -65,7 +85,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const Layout L = layout_of(pl);
-    const int KC = pl.kc, CT = pl.ct, CS = pl.cs, CH = pl.ch, NLOAD = (KC + CH - 1) / CH, HST = pl.hstages, WST = pl.wstages;
+    const int KC = pl.kc, CT = pl.ct, CS = pl.cs, CH = pl.ch, HST = pl.hstages, WST = pl.wstages;
     uint8_t *s_w = smem, *s_wr = s_w + L.w, *s_h = s_wr + L.wring, *s_p = s_h + L.h;
     float *s_ex = reinterpret_cast<float *>(s_p + L.p);
     uint64_t *hfull = reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(s_ex) + L.ex), *hempty = hfull + HST;
@@ -101,6 +121,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         *abort_w = 0;
         fence_barrier_init();
         tma_prefetch_desc(&tm_w);
+        if (STREAM) tma_prefetch_desc(&tm_ws);
         tma_prefetch_desc(&tm_h);
         tma_prefetch_desc(&tm_g);
     }
@@ -172,17 +193,25 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     fence_proxy_async_global();
                 }
                 FLSTM_STAMP(tt, 0);
-                for (int ld = 0; ld < NLOAD; ++ld) {
-                    ok = mbar_wait(&hempty[stage], phase ^ 1, abort_w, wait_ns);
-                    if (!ok) break;
-                    if (leader) mbar_expect_tx(&hfull[stage], 2 * hstage_bytes);
-                    h_issued |= 1u << stage;
-                    h_parity = (h_parity & ~(1u << stage)) | (phase << stage);
-                    // chunks beyond K come as zeros (and are counted)
-                    tma_load_4d_pair(s_h + stage * hstage_bytes, &tm_h, 0, S == 2 ? b0 : b0 + (int)rank * BROWS,
-                                     (S == 2 ? (int)rank * KC : 0) + ld * CH, t, hfull_c + 8u * (uint32_t)stage);
-                    if (++stage == HST) { stage = 0; phase ^= 1; }
+                const bool down = STREAM && (tt & 1);
+                for (int which = 0; which < (STREAM ? 3 : 1) && ok; ++which) {
+                    const Run run = run_of<STREAM>(pl, which, down);
+                    const bool desc = down && which != 1;
+                    for (int i = 0, n = run.copies(CH); i < n; ++i) {
+                        // (without a ring the tile is free: the step barrier came after the UMMAs that read it)
+                        if (STREAM || pl.hring) ok = mbar_wait(&hempty[stage], phase ^ 1, abort_w, wait_ns);
+                        if (!ok) break;
+                        if (leader) mbar_expect_tx(&hfull[stage], 2 * hstage_bytes);
+                        h_issued |= 1u << stage;
+                        h_parity = (h_parity & ~(1u << stage)) | (phase << stage);
+                        // chunks beyond K come as zeros (and are counted)
+                        const int c = desc ? run.hi - (i + 1) * CH : run.lo + i * CH;
+                        tma_load_4d_pair(s_h + stage * hstage_bytes, &tm_h, 0, S == 2 ? b0 : b0 + (int)rank * BROWS,
+                                         (S == 2 ? (int)rank * KC : 0) + c, t, hfull_c + 8u * (uint32_t)stage);
+                        if (++stage == HST) { stage = 0; phase ^= 1; }
+                    }
                 }
+                if (!ok) break;
                 FLSTM_STAMP(tt, 1);
             }
             // way out: every copy this thread started must have landed before the CTA exits (the peer's copies complete
@@ -200,79 +229,124 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 if (leader) mbar_expect_tx(wbar, 2u * (uint32_t)(CS * kStepBytesW));
                 for (int c = 0; c < CS; ++c) load_w(s_w + c * kStepBytesW, CT + c, wbar_c);
             }
-            int stage = 0;
-            uint32_t phase = 0, issued = 0, parity = 0;
-            for (int tt = 0; STREAM && tt < p.T && ok; ++tt)
-                for (int c = CT + CS; c < KC; ++c) {
-                    ok = mbar_wait(&wempty[stage], phase ^ 1, abort_w, wait_ns);
-                    if (!ok) break;
-                    if (leader) mbar_expect_tx(&wfull[stage], 2u * kStepBytesW);
-                    issued |= 1u << stage;
-                    parity = (parity & ~(1u << stage)) | (phase << stage);
-                    load_w(s_wr + stage * kStepBytesW, c, wfull_c + 8u * (uint32_t)stage);
-                    if (++stage == WST) { stage = 0; phase ^= 1; }
+            // group i of wch chunk-steps lives in slot i % WST; a load waits until the group WST before it (in the direction of the
+            // step) has been consumed
+            uint32_t loaded = 0, parity = 0, eparity = 0;
+            const int first = CT + CS, n = STREAM ? (KC - first) / WCH : 0, slot_bytes = WCH * kStepBytesW;
+            for (int tt = 0; STREAM && tt < p.T && ok; ++tt) {
+                const bool down = tt & 1;
+                for (int k = tt == 0 ? 0 : WST; k < n; ++k) {
+                    const int i = down ? n - 1 - k : k, slot = i % WST;
+                    if (k >= WST) {
+                        ok = mbar_wait(&wempty[slot], eparity >> slot & 1u, abort_w, wait_ns);
+                        if (!ok) break;
+                        eparity ^= 1u << slot;
+                    }
+                    if (leader) mbar_expect_tx(&wfull[slot], 2u * (uint32_t)slot_bytes);
+                    if (loaded >> slot & 1u) parity ^= 1u << slot;
+                    loaded |= 1u << slot;
+                    tma_load_4d_pair(s_wr + slot * slot_bytes, &tm_ws, 0, jr * ROWS, first + i * WCH, 0, wfull_c + 8u * (uint32_t)slot);
                 }
+            }
             if (CS > 0 && leader) mbar_drain(wbar, 0, wait_ns);
             for (int i = 0; i < WST && leader; ++i)
-                if (issued >> i & 1u) mbar_drain(&wfull[i], parity >> i & 1u, ok ? wait_ns : kAbortDrainNs);
+                if (loaded >> i & 1u) mbar_drain(&wfull[i], parity >> i & 1u, ok ? wait_ns : kAbortDrainNs);
         }
     } else if (warp == 5) {
         // ------------------------------------------------------------ UMMA issuer (the leader's)
         if (leader && elect_one()) {
             bool ok = CS == 0 || mbar_wait(wbar, 0, abort_w, wait_ns);
-            int hs = 0, ws = 0;
-            uint32_t hphase = 0, wphase = 0;
-            const uint32_t idesc = umma_idesc_f16(256, N, BF16 ? 1 : 0, 0, 0);
-            const uint32_t hempty_l = smem_u32(hempty), wempty_l = smem_u32(wempty);
-            const uint64_t dw_res = umma_desc_kmajor_sw128(smem_u32(s_w));
+            int hs = 0;
+            uint32_t hphase = 0, wparity = 0;
+            constexpr uint32_t idesc = umma_idesc_f16(256, N, BF16 ? 1 : 0, 0, 0);
+            constexpr uint32_t kStepH = (BROWS * 128) >> 4, kStepW = kStepBytesW >> 4;  // descriptor units
+            const uint32_t hempty_l = smem_u32(hempty), wempty_l = smem_u32(wempty), tfull_l = smem_u32(tfull);
+            const uint32_t dw_res = umma_desc_lo(smem_u32(s_w)), dw_ring = umma_desc_lo(smem_u32(s_wr)), dh_ring = umma_desc_lo(smem_u32(s_h));
+            const int first = CT + CS, ngroups = (KC - first) / WCH;
             int committed = 0;
             for (int tt = 0; tt < p.T && ok; ++tt) {
                 ok = mbar_wait_cluster(tempty, (tt & 1) ^ 1, abort_w, wait_ns);
                 if (!ok) break;
                 tcgen05_fence_after();
-                for (int ld = 0; ld < NLOAD && ok; ++ld) {
-                    ok = mbar_wait(&hfull[hs], hphase, abort_w, wait_ns);
-                    if (!ok) break;
-                    if (ld == 0) FLSTM_STAMP(tt, 2);
-                    if (ld == NLOAD - 1) FLSTM_STAMP(tt, 3);
-                    tcgen05_fence_after();
-                    uint64_t dh = umma_desc_kmajor_sw128(smem_u32(s_h + hs * hstage_bytes));
-                    const int c1 = (ld + 1) * CH < KC ? (ld + 1) * CH : KC;
-                    int c = ld * CH;
-                    const int ct1 = c1 < CT ? c1 : CT;
-                    uint32_t da = tmem_a + (uint32_t)c * 32;
-#pragma unroll 4
-                    for (; c < ct1; ++c) {
+                const bool down = STREAM && (tt & 1);
+                long long hwait = 0, wwait = 0;
+                uint32_t acc = 0;  // the step's first instruction overwrites the accumulator
+                for (int which = 0; which < (STREAM ? 3 : 1) && ok; ++which) {
+                    const Run run = run_of<STREAM>(pl, which, down);
+                    const bool desc = down && which != 1;
+                    FLSTM_STAMP(tt, (which == 0 ? 15 : 10 + which));
+                    int grp = desc ? (run.hi - first) / WCH - 1 : (run.lo - first) / WCH, slot = STREAM && which != 1 ? grp % WST : 0;
+                    for (int ld = 0, nld = run.copies(CH); ld < nld; ++ld) {
+                        long long q0 = clock64();
+                        ok = mbar_wait(&hfull[hs], hphase, abort_w, wait_ns);
+                        hwait += clock64() - q0;
+                        if (!ok) break;
+                        if (which == 0 && ld == 0) FLSTM_STAMP(tt, 2);
+                        FLSTM_STAMP(tt, 3);
+                        tcgen05_fence_after();
+                        uint32_t dh = dh_ring + (uint32_t)hs * (hstage_bytes >> 4);
+                        if (STREAM && which != 1) {
+                            const int left = run.hi - run.lo - ld * CH, cnt = (left < CH ? left : CH) / WCH;  // groups of this copy
+                            if (desc) dh += (uint32_t)(CH - WCH) * kStepH;
+                            for (int e = 0; e < cnt; ++e) {
+                                if (which == 2 || tt == 0) {
+                                    long long q1 = clock64();
+                                    ok = mbar_wait(&wfull[slot], wparity >> slot & 1u, abort_w, wait_ns);
+                                    wwait += clock64() - q1;
+                                    if (!ok) break;
+                                    wparity ^= 1u << slot;
+                                    tcgen05_fence_after();
+                                }
+                                uint32_t dw = dw_ring + (uint32_t)(slot * WCH) * kStepW;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) umma_f16_ts_pair(tmem_base, da + 8 * k, dh + 2 * k, idesc, (uint32_t)(c | k));
-                        da += 32;
-                        dh += (BROWS * 128) >> 4;
-                    }
-                    for (; c < c1; ++c) {
-                        uint64_t dw;
-                        const bool streamed = STREAM && c >= CT + CS;
-                        if (streamed) {
-                            ok = mbar_wait(&wfull[ws], wphase, abort_w, wait_ns);
+                                for (int c = 0; c < WCH; ++c) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) umma_lo_ss<true>(tmem_base, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                                    acc = 1u;
+                                    dw += kStepW;
+                                    dh += kStepH;
+                                }
+                                // what the next step begins with stays in its slot
+                                if (down ? grp >= WST : grp < ngroups - WST) umma_commit_pair_both(wempty_l + 8u * (uint32_t)slot);
+                                if (desc) {
+                                    dh -= 2u * (uint32_t)WCH * kStepH;
+                                    --grp;
+                                    slot = slot == 0 ? WST - 1 : slot - 1;
+                                } else {
+                                    ++grp;
+                                    slot = slot + 1 == WST ? 0 : slot + 1;
+                                }
+                            }
                             if (!ok) break;
-                            tcgen05_fence_after();
-                            dw = umma_desc_kmajor_sw128(smem_u32(s_wr + ws * kStepBytesW));
                         } else {
-                            dw = dw_res + (uint64_t)((c - CT) * (kStepBytesW >> 4));
-                        }
+                            int c = run.lo + ld * CH;
+                            const int c1 = c + CH < run.hi ? c + CH : run.hi, ct1 = c1 < CT ? c1 : CT;
+                            uint32_t da = tmem_a + (uint32_t)c * 32;
+#pragma unroll 4
+                            for (; c < ct1; ++c) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) umma_f16_pair(tmem_base, dw + 2 * k, dh + 2 * k, idesc, (uint32_t)(c | k));
-                        dh += (BROWS * 128) >> 4;
-                        if (streamed) {
-                            umma_commit_pair_both(wempty_l + 8u * (uint32_t)ws);
-                            if (++ws == WST) { ws = 0; wphase ^= 1; }
+                                for (int k = 0; k < 4; ++k) umma_lo_ts<true>(tmem_base, da + 8 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                                acc = 1u;
+                                da += 32;
+                                dh += kStepH;
+                            }
+                            uint32_t dw = dw_res + (uint32_t)(c - CT) * kStepW;
+#pragma unroll 2
+                            for (; c < c1; ++c) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_lo_ss<true>(tmem_base, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                                acc = 1u;
+                                dw += kStepW;
+                                dh += kStepH;
+                            }
                         }
+                        if (STREAM || pl.hring) umma_commit_pair_both(hempty_l + 8u * (uint32_t)hs);
+                        if (++hs == HST) { hs = 0; hphase ^= 1; }
                     }
-                    if (!ok) break;
-                    umma_commit_pair_both(hempty_l + 8u * (uint32_t)hs);
-                    if (++hs == HST) { hs = 0; hphase ^= 1; }
                 }
+                if (tracing && tt < p.trace_steps) { p.trace[tt*16+13] = hwait; p.trace[tt*16+14] = wwait; }
                 if (!ok) break;
-                umma_commit_pair_both(smem_u32(tfull));
+                umma_commit_pair_both(tfull_l);
                 ++committed;
                 FLSTM_STAMP(tt, 4);
             }
@@ -407,7 +481,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 }
 
 template <int S, int BT, bool STREAM, bool BF16, bool ACC>
-int launch_one(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdTmPlan &pl, const FwdParams &p,
+int launch_one(const CUtensorMap &tw, const CUtensorMap &tws, const CUtensorMap &th, const CUtensorMap &tg, const FwdTmPlan &pl, const FwdParams &p,
                cudaStream_t s) {
     auto kern = lstm_fwd_tm_kernel<S, BT, STREAM, BF16, ACC>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)pl.smem_bytes));
@@ -425,7 +499,7 @@ int launch_one(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, th, tg, pl, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tws, th, tg, pl, p);
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "recurrent forward launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
 }
@@ -452,36 +526,31 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
     const int N = pl.S * pl.BT, tmem_steps = (kTmemColumns - N) / 32, step_h = N / 2 * 128;
     pl.ct = pl.kc < tmem_steps ? pl.kc : tmem_steps;
     auto fits = [&]() { return (size_t)layout_of(pl).total <= smem_limit; };
-    // h in few large copies: the whole tile at once if it fits beside the rest of the weights, else two or more stages
-    pl.cs = pl.kc - pl.ct;
-    pl.ch = 65536 / step_h < pl.kc ? 65536 / step_h : pl.kc;
+    // h in copies of 16 KB, the whole tile at once if it fits beside the rest of the weights
+    const int rest = pl.kc - pl.ct;
+    pl.cs = rest;
+    pl.ch = 16384 / step_h < pl.kc ? 16384 / step_h : pl.kc;
     if (const char *e = std::getenv("FLSTM_TM_CH")) pl.ch = std::atoi(e) < pl.kc ? std::atoi(e) : pl.kc;
     pl.hstages = (pl.kc + pl.ch - 1) / pl.ch;
-    while (!fits() && pl.hstages > 2) --pl.hstages;
-    while (!fits() && pl.ch > 4) {
-        pl.ch /= 2;
-        pl.hstages = 2;
-        while (pl.hstages * pl.ch < pl.kc) {
-            ++pl.hstages;
-            if (!fits()) {
-                --pl.hstages;
-                break;
-            }
-        }
+    while (!fits() && pl.hstages > 2) {
+        --pl.hstages;
+        pl.hring = 1;
     }
     if (!fits()) {
-        // streamed: the ring keeps the copies going while a step waits for h, the rest of the room holds weights for good
+        // streamed: all the room goes to the slots, which keep what the next step begins with
         pl.cs = 0;
-        pl.ch = 16384 / step_h < pl.kc ? 16384 / step_h : pl.kc;
-        pl.hstages = 4;
+        pl.hring = 1;
+        pl.ch = (16384 / step_h) / WCH * WCH;
+        if (const char *e = std::getenv("FLSTM_TM_SCH")) pl.ch = std::atoi(e);
+        pl.hstages = 2;
         if (const char *e = std::getenv("FLSTM_TM_HST")) pl.hstages = std::atoi(e);
         if (!fits()) return FLSTM_OK;
         const int room = (int)((smem_limit - (size_t)layout_of(pl).total) / kStepBytesW);
-        if (room < 3) return FLSTM_OK;
-        int ring = 6;
-        if (const char *e = std::getenv("FLSTM_TM_RING")) ring = std::atoi(e);
-        pl.wstages = room < ring ? room : ring;
-        pl.cs = room - pl.wstages;
+        pl.wstages = (room - rest % WCH) / WCH;  // chunk-steps that make no whole group stay in shared memory
+        if (const char *e = std::getenv("FLSTM_TM_RING")) pl.wstages = std::atoi(e) < pl.wstages ? std::atoi(e) : pl.wstages;
+        if (pl.wstages < 2) return FLSTM_OK;
+        if (pl.wstages > rest / WCH) pl.wstages = rest / WCH;
+        pl.cs = rest % WCH;
     }
     pl.smem_bytes = layout_of(pl).total;
     if (pl.smem_bytes < 120 * 1024) pl.smem_bytes = 120 * 1024;  // one CTA per SM: each allocates all of tensor memory
@@ -491,15 +560,15 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
     return FLSTM_OK;
 }
 
-int lstm_forward_tm(int dtype, const FwdTmPlan &pl, const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg,
+int lstm_forward_tm(int dtype, const FwdTmPlan &pl, const CUtensorMap &tw, const CUtensorMap &tws, const CUtensorMap &th, const CUtensorMap &tg,
                     const FwdParams &p, cudaStream_t s) {
     const bool bf16 = dtype == FLSTM_DTYPE_BF16, acc = p.real_units > 0, stream = pl.wstages > 0;
 #define FLSTM_TM_CASE(S_, BT_, ST_)                                                                       \
     if (pl.S == S_ && pl.BT == BT_ && stream == ST_) {                                                    \
-        if (bf16) return acc ? launch_one<S_, BT_, ST_, true, true>(tw, th, tg, pl, p, s)                 \
-                             : launch_one<S_, BT_, ST_, true, false>(tw, th, tg, pl, p, s);               \
-        return acc ? launch_one<S_, BT_, ST_, false, true>(tw, th, tg, pl, p, s)                          \
-                   : launch_one<S_, BT_, ST_, false, false>(tw, th, tg, pl, p, s);                        \
+        if (bf16) return acc ? launch_one<S_, BT_, ST_, true, true>(tw, tws, th, tg, pl, p, s)                 \
+                             : launch_one<S_, BT_, ST_, true, false>(tw, tws, th, tg, pl, p, s);               \
+        return acc ? launch_one<S_, BT_, ST_, false, true>(tw, tws, th, tg, pl, p, s)                          \
+                   : launch_one<S_, BT_, ST_, false, false>(tw, tws, th, tg, pl, p, s);                        \
     }
     FLSTM_TM_CASE(2, 32, false) FLSTM_TM_CASE(2, 64, false)
     FLSTM_TM_CASE(1, 16, true) FLSTM_TM_CASE(1, 32, true) FLSTM_TM_CASE(1, 64, true)

@@ -170,7 +170,15 @@ int init(Engine &e) {
         // the cross-layer wavefront would put two cooperative grids side by side
         const char *wave = std::getenv("FLSTM_WAVE_CHUNK");
         const bool wavefront = wave && std::atoi(wave) > 0;
-        if (!st->cfwd.use && !wavefront) FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &st->fwdtm));
+        if (!st->cfwd.use && !wavefront) {
+            FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &st->fwdtm));
+            // 33 to 64 sequences per batch group: the K halves make an UMMA of N = 128, which takes longer than the other
+            // kernel's of N = 64 (H = 512, B = 250: 4.15 against 3.97 us a step; H = 640, B = 130: 4.16 against 3.98), so that one
+            // stays where its weights are resident and a CTA has one batch tile
+            FwdPlan f{};
+            if (st->fwdtm.use && st->fwdtm.BT == 64 && plan_fwd(B, H, st->sms, st->smem_limit, &f) == FLSTM_OK && f.resident && f.nt == 1)
+                st->fwdtm.use = false;
+        }
         if (e.cfg.training && !st->cbwd.use && !wavefront)
             FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &st->bwdtm, /*check_device=*/true));
     }
@@ -380,7 +388,6 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.trace_steps = e.trace_steps;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    p.w_hh = l.w_hh;
     if (st->fwdtm.use) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h, t.tm_g, p, s));
     else FLSTM_TRY(lstm_forward_persistent(e.cfg.dtype, st->fwd, t.tm_w, t.tm_h, t.tm_g, p, s));
     size_t m2 = e.timer.mark(s);
@@ -582,7 +589,6 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.H = (int)H;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    p.w_hh = l.w_hh;
     if (st->bwdtm.use) FLSTM_TRY(lstm_backward_tm(e.cfg.dtype, st->bwdtm, t.tm_w, t.dg_tm, p, s));
     else FLSTM_TRY(lstm_backward_persistent(e.cfg.dtype, st->bwd, t.tm_w, t.tm_dg, p, s));
     e.launches += 1;

@@ -55,7 +55,6 @@ struct FwdParams {
     int trace_steps;
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path: the step barrier waits for this many arrivals nobody makes
-    const void *w_hh;     // 16-bit (4H, H), rows tile-interleaved; read by the tensor-memory kernel beside its tensor map
     // filled by the launcher from the plan
     int rt, cta_rows, nt, stages, ch;
     uint32_t idesc;
@@ -121,7 +120,6 @@ struct BwdParams {
     int s0, s1;           // reverse iterations [s0, s1) of this launch; iteration s is time T-1-s, s == T writes dh0/dc0
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path (see FwdParams)
-    const void *w_hh;     // as in FwdParams
     int jt, nt, stages, ch;
     uint32_t idesc;
 };

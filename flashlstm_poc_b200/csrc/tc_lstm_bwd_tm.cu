@@ -35,6 +35,8 @@ constexpr int kThreads = 320;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA
 constexpr int kEpilogueThreads = 256;
 constexpr int kStepBytesW = 2 * 64 * 128;  // one chunk-step of A: two blocks of 64 K rows x 64 units
 constexpr int kTmemColumns = 512;
+constexpr int kBarrierBytes = 1024, kMinSmemBytes = 120 * 1024;
+constexpr int kFillSlots = (kMinSmemBytes - 1024 - kBarrierBytes) / kStepBytesW;
 constexpr int KS = 4, UPO = 64 / KS;
 
 struct Layout {
@@ -49,7 +51,7 @@ __host__ __device__ inline Layout layout_of(const BwdTmPlan &pl) {
     l.left = pl.left ? pl.BT * 128 : 0;
     l.ps = 128 * (pl.BT + 4) * 4;
     l.red = 2 * KS * UPO * (pl.BT + 4) * 4;
-    l.total = l.w + l.left_w + l.ring + l.left + l.ps + l.red + 1024 /*align*/ + 512 /*barriers*/;
+    l.total = kBarrierBytes + l.w + l.left_w + l.ring + l.left + l.ps + l.red + 1024 /*align*/;
     return l;
 }
 
@@ -65,12 +67,13 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const Layout L = layout_of(pl);
     const int KP = pl.kp, CT = pl.ct, CS = pl.cs, CH = pl.ch, NLOAD = (KP + CH - 1) / CH, ST = pl.stages;
     const int stage_bytes = CH * N * 128;
-    uint8_t *s_w = smem, *s_lw = s_w + L.w, *s_ring = s_lw + L.left_w, *s_left = s_ring + L.ring;
+    uint8_t *s_w = smem + kBarrierBytes, *s_lw = s_w + L.w, *s_ring = s_lw + L.left_w, *s_left = s_ring + L.ring;
     float *s_ps = reinterpret_cast<float *>(s_left + L.left), *s_red = s_ps + L.ps / 4;
-    uint64_t *full = reinterpret_cast<uint64_t *>(s_red + L.red / 4), *empty = full + ST;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + ST;
     uint64_t *lfull = empty + ST, *tfull = lfull + 1, *tempty = tfull + 1, *wbar = tempty + 1;
     uint64_t *rbar = wbar + 1;  // [2] partial sums received
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(rbar + 2);
+    uint64_t *ffull = rbar + 2, *fempty = ffull + kFillSlots;  // while W_hh moves into tensor memory
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fempty + kFillSlots);
     volatile uint32_t *abort_w = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,6 +95,10 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         mbar_init(wbar, 1);
         mbar_init(&rbar[0], 1);
         mbar_init(&rbar[1], 1);
+        for (int i = 0; i < kFillSlots; ++i) {
+            mbar_init(&ffull[i], 1);
+            mbar_init(&fempty[i], 4);
+        }
         *abort_w = 0;
         fence_barrier_init();
         tma_prefetch_desc(&tm_w);
@@ -106,19 +113,36 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + N;
-    // W_hh^T into tensor memory: lane l takes unit l % 64 and K half l / 64, 32 columns of two K elements per chunk-step; the
-    // warps 0-3 take the even chunk-steps, 6-9 the odd ones (a warp reaches the lane quadrant warp % 4)
-    if (warp < 4 || warp > 5) {
-        const int quad = warp & 3, l = quad * 32 + lane;
-        const uint16_t *src = static_cast<const uint16_t *>(p.w_hh) + (size_t)(c_first + (l >> 6) * KP) * 64 * p.H + j * 64 + (l & 63);
+    const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
+    // W_hh^T into tensor memory, by way of the shared memory that the rings will use (as in tc_lstm_fwd_tm.cu): lane l takes unit
+    // l % 64 and K half l / 64, 32 columns of two K elements per chunk-step; the warps 0-3 take the even chunk-steps, 6-9 the
+    // odd ones
+    if (warp == 4 && elect_one()) {
+        for (int c = 0; c < CT; ++c) {
+            const int slot = c % kFillSlots;
+            if (c >= kFillSlots && !mbar_wait(&fempty[slot], (uint32_t)(c / kFillSlots - 1) & 1u, abort_w, wait_ns)) break;
+            mbar_expect_tx(&ffull[slot], kStepBytesW);
+            for (int h = 0; h < 2; ++h)
+                tma_load_2d(s_w + slot * kStepBytesW + h * 8192, &tm_w, j * 64, (c_first + h * KP + c) * 64, &ffull[slot]);
+        }
+    } else if (warp < 4 || warp > 5) {
+        const int quad = warp & 3, l = quad * 32 + lane, un = l & 63;
+        const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
         for (int c = warp < 4 ? 0 : 1; c < CT; c += 2) {
+            const int slot = c % kFillSlots;
+            if (!__all_sync(0xffffffffu, mbar_wait(&ffull[slot], (uint32_t)(c / kFillSlots) & 1u, abort_w, wait_ns))) break;
+            const uint8_t *tile = s_w + slot * kStepBytesW + (l >> 6) * 8192 + (un & 7) * 2;
             uint32_t r[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-                const uint16_t *e = src + (size_t)(c * 64 + 2 * i) * p.H;
-                r[i] = (uint32_t)__ldg(e) | (uint32_t)__ldg(e + p.H) << 16;
+                const int k = 2 * i;
+                const uint32_t lo = *reinterpret_cast<const uint16_t *>(tile + k * 128 + (((un >> 3) ^ (k & 7)) * 16));
+                const uint32_t hi = *reinterpret_cast<const uint16_t *>(tile + (k + 1) * 128 + (((un >> 3) ^ ((k + 1) & 7)) * 16));
+                r[i] = lo | hi << 16;
             }
-            tmem_st_32x32b_x32(tmem_a + ((uint32_t)(quad * 32) << 16) + c * 32, r);
+            tmem_st_32x32b_x32(dst + c * 32, r);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&fempty[slot]);
         }
         tmem_st_wait();
     }
@@ -126,7 +150,6 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     __syncthreads();
     cluster_sync_all();  // every CTA's barriers exist before any remote arrive
     tcgen05_fence_after();
-    const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
     const int s_first = p.s0 > 1 ? p.s0 : 1;  // iteration s handles time T-1-s and, from s = 1 on, contracts dG_{T-s}
     const bool tracing = p.trace != nullptr && blockIdx.x == 0;
 #define FLSTM_STAMP(step, slot)                                                     \
@@ -468,7 +491,7 @@ int max_clusters(const BwdTmPlan &pl) {
 int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool check_device) {
     *plan = BwdTmPlan{};
     if (H % 64 != 0 || H < 256 || smem_limit < 160 * 1024) return FLSTM_OK;
-    const char *env = std::getenv("FLSTM_BWD_TM");
+    const char *env = std::getenv("FLSTM_TMEM");
     if (env && env[0] == '0') return FLSTM_OK;
     BwdTmPlan pl{};
     pl.jt = H / 64;
@@ -486,7 +509,6 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
     pl.cs = pl.kp - pl.ct;
     // dG in copies of up to 64 KB, the whole tile at once if it fits
     pl.ch = 65536 / step_bytes < pl.kp ? 65536 / step_bytes : pl.kp;
-    if (const char *e = std::getenv("FLSTM_TM_BCH")) pl.ch = std::atoi(e) < pl.kp ? std::atoi(e) : pl.kp;
     pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
     auto fits = [&]() { return (size_t)layout_of(pl).total <= smem_limit; };
     while (!fits() && pl.ch > 1) {
@@ -497,7 +519,7 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
     if (!fits()) return FLSTM_OK;
     pl.ring = pl.stages * pl.ch < pl.kp;
     pl.smem_bytes = layout_of(pl).total;
-    if (pl.smem_bytes < 120 * 1024) pl.smem_bytes = 120 * 1024;  // one CTA per SM: each allocates all of tensor memory
+    if (pl.smem_bytes < kMinSmemBytes) pl.smem_bytes = kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
     pl.grid = pl.jt * KS * pl.ngroups;
     if (check_device && (pl.BT == 32 ? max_clusters<32>(pl) : max_clusters<64>(pl)) * KS < pl.grid) return FLSTM_OK;
     pl.use = true;

@@ -42,6 +42,8 @@ constexpr int kThreads = 352;  // warps 0-3 and 6-9 epilogue, 4 producer of h, 5
 constexpr int kEpilogueThreads = 256;
 constexpr int kStepBytesW = 128 * 128;  // one chunk-step of A: 128 rows x 64 16-bit elements
 constexpr int kTmemColumns = 512;
+constexpr int kBarrierBytes = 1024, kMinSmemBytes = 120 * 1024;
+constexpr int kFillSlots = (kMinSmemBytes - 1024 - kBarrierBytes) / kStepBytesW;
 constexpr int WCH = kFwdTmGroup;
 
 struct Layout {
@@ -55,7 +57,7 @@ __host__ __device__ inline Layout layout_of(const FwdTmPlan &pl) {
     l.h = pl.hstages * pl.ch * (pl.S * pl.BT / 2) * 128;
     l.p = 2 * (2 / pl.S) * pl.BT * 128;
     l.ex = 128 * (pl.BT + 4) * 4;
-    l.total = l.w + l.wring + l.h + l.p + l.ex + 1024 /*align*/ + 1024 /*barriers*/;
+    l.total = kBarrierBytes + l.w + l.wring + l.h + l.p + l.ex + 1024 /*align*/;
     return l;
 }
 
@@ -86,13 +88,14 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const Layout L = layout_of(pl);
     const int KC = pl.kc, CT = pl.ct, CS = pl.cs, CH = pl.ch, HST = pl.hstages, WST = pl.wstages;
-    uint8_t *s_w = smem, *s_wr = s_w + L.w, *s_h = s_wr + L.wring, *s_p = s_h + L.h;
+    uint8_t *s_w = smem + kBarrierBytes, *s_wr = s_w + L.w, *s_h = s_wr + L.wring, *s_p = s_h + L.h;
     float *s_ex = reinterpret_cast<float *>(s_p + L.p);
-    uint64_t *hfull = reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(s_ex) + L.ex), *hempty = hfull + HST;
+    uint64_t *hfull = reinterpret_cast<uint64_t *>(smem), *hempty = hfull + HST;
     uint64_t *wfull = hempty + HST, *wempty = wfull + WST;
     uint64_t *tfull = wempty + WST, *tempty = tfull + 1, *wbar = tempty + 1;
     uint64_t *pfull = wbar + 1, *pempty = pfull + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(pempty + 2);
+    uint64_t *ffull = pempty + 2, *fempty = ffull + kFillSlots;  // while W_hh moves into tensor memory
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fempty + kFillSlots);
     volatile uint32_t *abort_w = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -118,6 +121,10 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             mbar_init(&pfull[i], 1);
             mbar_init(&pempty[i], kEpilogueThreads / 32);
         }
+        for (int i = 0; i < kFillSlots; ++i) {
+            mbar_init(&ffull[i], 1);
+            mbar_init(&fempty[i], 4);
+        }
         *abort_w = 0;
         fence_barrier_init();
         tma_prefetch_desc(&tm_w);
@@ -133,21 +140,36 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + N;
-    // W_hh into tensor memory: lane l of the CTA takes row l % ROWS, K half l / ROWS, 32 columns of two elements per
-    // chunk-step; the warps 0-3 take the even chunk-steps, 6-9 the odd ones (a warp reaches the lane quadrant warp % 4)
-    if (warp != 4 && warp != 5 && warp != 10) {
-        const int quad = warp & 3, l = quad * 32 + lane, part = l / ROWS;
-        const uint4 *src = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(p.w_hh) +
-                                                           (size_t)(jr * ROWS + l % ROWS) * p.H + (size_t)part * KC * 64);
+    const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
+    // W_hh into tensor memory, by way of the shared memory that the rings will use: lane l of the CTA takes row l % ROWS, K half
+    // l / ROWS, 32 columns of two elements per chunk-step; the warps 0-3 take the even chunk-steps, 6-9 the odd ones (a warp
+    // reaches the lane quadrant warp % 4).  Loads straight from global memory, a row of 128 bytes per lane, took 10 us more per
+    // launch at H = 1024.  A wait that expires raises the abort word, on which every role below gives up.
+    if (warp == 4 && elect_one()) {
+        for (int c = 0; c < CT; ++c) {
+            const int slot = c % kFillSlots;
+            uint8_t *dst = s_w + slot * kStepBytesW;
+            if (c >= kFillSlots && !mbar_wait(&fempty[slot], (uint32_t)(c / kFillSlots - 1) & 1u, abort_w, wait_ns)) break;
+            mbar_expect_tx(&ffull[slot], kStepBytesW);
+            tma_load_2d(dst, &tm_w, c * 64, jr * ROWS, &ffull[slot]);
+            tma_load_2d(dst + 8192, &tm_w, (S == 2 ? KC + c : c) * 64, jr * ROWS + (S == 2 ? 0 : 64), &ffull[slot]);
+        }
+    } else if (warp != 4 && warp != 5 && warp != 10) {
+        const int quad = warp & 3, l = quad * 32 + lane;
+        const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
         for (int c = warp < 4 ? 0 : 1; c < CT; c += 2) {
+            const int slot = c % kFillSlots;
+            if (!__all_sync(0xffffffffu, mbar_wait(&ffull[slot], (uint32_t)(c / kFillSlots) & 1u, abort_w, wait_ns))) break;
+            const uint8_t *row = s_w + slot * kStepBytesW + l * 128;
             uint32_t r[32];
-            const bool there = (part * KC + c) * 64 < p.H;  // an odd number of chunks: the second half is one short
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const uint4 v = there ? __ldg(src + c * 8 + i) : make_uint4(0, 0, 0, 0);
+                const uint4 v = *reinterpret_cast<const uint4 *>(row + ((i ^ (l & 7)) * 16));
                 r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
             }
-            tmem_st_32x32b_x32(tmem_a + ((uint32_t)(quad * 32) << 16) + c * 32, r);
+            tmem_st_32x32b_x32(dst + c * 32, r);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&fempty[slot]);
         }
         tmem_st_wait();
     }
@@ -164,7 +186,6 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         tma_load_2d_pair(dst + 8192, &tm_w, (S == 2 ? KC + c : c) * 64, jr * ROWS + (S == 2 ? 0 : 64), bar);
     };
 
-    const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
     const bool tracing = p.trace != nullptr && blockIdx.x == 0;
 #define FLSTM_STAMP(step, slot)                                                     \
     do {                                                                            \
@@ -269,17 +290,13 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 if (!ok) break;
                 tcgen05_fence_after();
                 const bool down = STREAM && (tt & 1);
-                long long hwait = 0, wwait = 0;
                 uint32_t acc = 0;  // the step's first instruction overwrites the accumulator
                 for (int which = 0; which < (STREAM ? 3 : 1) && ok; ++which) {
                     const Run run = run_of<STREAM>(pl, which, down);
                     const bool desc = down && which != 1;
-                    FLSTM_STAMP(tt, (which == 0 ? 15 : 10 + which));
                     int grp = desc ? (run.hi - first) / WCH - 1 : (run.lo - first) / WCH, slot = STREAM && which != 1 ? grp % WST : 0;
                     for (int ld = 0, nld = run.copies(CH); ld < nld; ++ld) {
-                        long long q0 = clock64();
                         ok = mbar_wait(&hfull[hs], hphase, abort_w, wait_ns);
-                        hwait += clock64() - q0;
                         if (!ok) break;
                         if (which == 0 && ld == 0) FLSTM_STAMP(tt, 2);
                         FLSTM_STAMP(tt, 3);
@@ -290,9 +307,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                             if (desc) dh += (uint32_t)(CH - WCH) * kStepH;
                             for (int e = 0; e < cnt; ++e) {
                                 if (which == 2 || tt == 0) {
-                                    long long q1 = clock64();
                                     ok = mbar_wait(&wfull[slot], wparity >> slot & 1u, abort_w, wait_ns);
-                                    wwait += clock64() - q1;
                                     if (!ok) break;
                                     wparity ^= 1u << slot;
                                     tcgen05_fence_after();
@@ -344,7 +359,6 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                         if (++hs == HST) { hs = 0; hphase ^= 1; }
                     }
                 }
-                if (tracing && tt < p.trace_steps) { p.trace[tt*16+13] = hwait; p.trace[tt*16+14] = wwait; }
                 if (!ok) break;
                 umma_commit_pair_both(tfull_l);
                 ++committed;
@@ -510,9 +524,8 @@ int launch_one(const CUtensorMap &tw, const CUtensorMap &tws, const CUtensorMap 
 int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
     *plan = FwdTmPlan{};
     if (H % 64 != 0 || H < 64 || smem_limit < 160 * 1024) return FLSTM_OK;
-    const char *env = std::getenv("FLSTM_FWD_TM");
-    if (env && env[0] == '0') return FLSTM_OK;
-    if (H <= 1024 && !(env && env[0] == '1')) return FLSTM_OK;
+    const char *env = std::getenv("FLSTM_TMEM"), *pair = std::getenv("FLSTM_FWD_PAIR");  // =0: weights in shared memory, lone CTAs
+    if ((env && env[0] == '0') || (pair && pair[0] == '0')) return FLSTM_OK;
     FwdTmPlan pl{};
     pl.S = H / 16 <= sms ? 2 : 1;
     pl.cta_rows = pl.S == 2 ? H / 16 : H / 32;
@@ -530,7 +543,6 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
     const int rest = pl.kc - pl.ct;
     pl.cs = rest;
     pl.ch = 16384 / step_h < pl.kc ? 16384 / step_h : pl.kc;
-    if (const char *e = std::getenv("FLSTM_TM_CH")) pl.ch = std::atoi(e) < pl.kc ? std::atoi(e) : pl.kc;
     pl.hstages = (pl.kc + pl.ch - 1) / pl.ch;
     while (!fits() && pl.hstages > 2) {
         --pl.hstages;
@@ -541,19 +553,16 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
         pl.cs = 0;
         pl.hring = 1;
         pl.ch = (16384 / step_h) / WCH * WCH;
-        if (const char *e = std::getenv("FLSTM_TM_SCH")) pl.ch = std::atoi(e);
         pl.hstages = 2;
-        if (const char *e = std::getenv("FLSTM_TM_HST")) pl.hstages = std::atoi(e);
         if (!fits()) return FLSTM_OK;
         const int room = (int)((smem_limit - (size_t)layout_of(pl).total) / kStepBytesW);
         pl.wstages = (room - rest % WCH) / WCH;  // chunk-steps that make no whole group stay in shared memory
-        if (const char *e = std::getenv("FLSTM_TM_RING")) pl.wstages = std::atoi(e) < pl.wstages ? std::atoi(e) : pl.wstages;
         if (pl.wstages < 2) return FLSTM_OK;
         if (pl.wstages > rest / WCH) pl.wstages = rest / WCH;
         pl.cs = rest % WCH;
     }
     pl.smem_bytes = layout_of(pl).total;
-    if (pl.smem_bytes < 120 * 1024) pl.smem_bytes = 120 * 1024;  // one CTA per SM: each allocates all of tensor memory
+    if (pl.smem_bytes < kMinSmemBytes) pl.smem_bytes = kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
     pl.grid = pl.cta_rows * pl.ngroups;
     pl.use = true;
     *plan = pl;

@@ -226,7 +226,26 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[
                  : "r"(taddr)
                  : "memory");
 }
-// the reverse of the loads: thread i of the warp writes 32 columns of lane (base_lane + i)
+// 16 lanes x 8 N columns of 32 bits, as mma accumulator fragments: thread i gets, per 8 columns, columns 2 (i % 4) and + 1 of lane
+// base_lane + i / 4 (r[0], r[1]) and of lane base_lane + 8 + i / 4 (r[2], r[3])
+template <int N>
+__device__ __forceinline__ void tmem_ld_16x256b(uint32_t taddr, uint32_t (&r)[4 * N]) {
+    static_assert(N == 2 || N == 4, "instantiated forms");
+    if constexpr (N == 2)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr)
+                     : "memory");
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr)
+            : "memory");
+}
+// the reverse of the 32x32b loads: thread i of the warp writes 32 columns of lane (base_lane + i)
 __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -365,6 +384,13 @@ __device__ __forceinline__ void tma_load_4d_pair(void *smem_dst, const CUtensorM
         ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w)
         : "memory");
 }
+__device__ __forceinline__ void tma_load_5d_pair(void *smem_dst, const CUtensorMap *m, int x, int y, int z, int w, int v,
+                                                 uint32_t bar_cluster_addr) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v)
+        : "memory");
+}
 // D[tmem of both CTAs] (+)= A * B over the pair; issued by ONE thread of the leader CTA
 __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                               uint32_t accumulate) {
@@ -493,6 +519,9 @@ int make_tensor_map_chunked(CUtensorMap *out, const void *base, uint64_t steps, 
 // 2 box_rows rows, the rows of the first run above those of the second.  Chunks beyond a run come as zeros.
 int make_tensor_map_halves(CUtensorMap *out, const void *base, uint64_t steps, uint64_t rows, uint64_t width, uint32_t box_rows,
                            uint32_t half_chunks, uint32_t chunks);
+// W_hh (4H, H) with tile-interleaved rows as (H / 16 tiles, 2 unit halves, 4 gates, 8 units, H): a box of 1 x 2 x 4 x 8 x 64 lands as
+// a K-major operand tile of 64 rows in the order (unit half, gate, unit).
+int make_tensor_map_gate_rows(CUtensorMap *out, const void *base, uint64_t H);
 
 }  // namespace tc
 }  // namespace flstm_b200

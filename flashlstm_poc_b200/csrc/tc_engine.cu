@@ -27,7 +27,7 @@ struct TcLayer {
     CUtensorMap tm_h;   // hs (Tcap+1, B, H), 1 x BT x 64 boxes, 128B swizzle
     CUtensorMap tm_g;   // gates (Tcap, B, 4H), 1 x BT x 64 boxes, no swizzle
     CUtensorMap tm_dg;  // dG (Tcap, B, 4H), 1 x BT x 64 boxes, 128B swizzle (BPTT operand)
-    CUtensorMap tm_ws;  // w_hh, 128 x 64 boxes (streamed part of the tensor-memory forward)
+    CUtensorMap tm_ws;  // w_hh, 128 x 64 boxes (streamed part of the tensor-memory forward), or its gate-row form (wide forward)
     BwdTmMaps dg_tm;    // dG for the tensor-memory BPTT kernel
     // wide-batch path (one GEMM launch per step)
     CUtensorMap tm_hs3;    // hs (Tcap+1, B, H), 1 x 128 x 64 boxes, 128B swizzle
@@ -41,6 +41,7 @@ struct TcState {
     size_t smem_limit = 0;
     FwdPlan fwd{};
     FwdTmPlan fwdtm{};
+    FwdWidePlan wide{};
     BwdPlan bwd{};
     BwdTmPlan bwdtm{};
     bool bwd_ok = false;
@@ -176,13 +177,14 @@ int init(Engine &e) {
             // kernel's of N = 64 (H = 512, B = 250: 4.15 against 3.97 us a step; H = 640, B = 130: 4.16 against 3.98), so that one
             // stays where its weights are resident and a CTA has one batch tile
             FwdPlan f{};
-            if (st->fwdtm.use && st->fwdtm.BT == 64 && plan_fwd(B, H, st->sms, st->smem_limit, &f) == FLSTM_OK && f.resident && f.nt == 1)
-                st->fwdtm.use = false;
+            const bool one_tile = plan_fwd(B, H, st->sms, st->smem_limit, &f) == FLSTM_OK && f.resident && f.nt == 1 && f.BT <= 64;
+            if (st->fwdtm.BT == 64 && one_tile) st->fwdtm.use = false;
+            else if (!st->fwdtm.use) FLSTM_TRY(plan_fwd_wide(B, H, st->sms, st->smem_limit, &st->wide));
         }
         if (e.cfg.training && !st->cbwd.use && !wavefront)
             FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &st->bwdtm, /*check_device=*/true));
     }
-    const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use, grid_bwd = e.cfg.training && !st->cbwd.use && !st->bwdtm.use;
+    const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use && !st->wide.use, grid_bwd = e.cfg.training && !st->cbwd.use && !st->bwdtm.use;
     st->bwd_ok = e.cfg.training != 0;
     if (grid_fwd || grid_bwd) FLSTM_TRY(plan_step(B, H, st->sms, st->smem_limit, &st->step));
     if (st->step.use && grid_bwd) {
@@ -220,11 +222,15 @@ int on_capacity_change(Engine &e) {
     for (size_t li = 0; li < e.layers.size(); ++li) {
         auto &l = e.layers[li];
         auto &t = st->layers[li];
-        const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use, tm_bwd = e.cfg.training && l.dg && st->bwdtm.use;
+        const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use && !st->wide.use, tm_bwd = e.cfg.training && l.dg && st->bwdtm.use;
         const bool grid_bwd = e.cfg.training && l.dg && !st->cbwd.use && !st->bwdtm.use;
-        if (!grid_fwd && !grid_bwd && !st->fwdtm.use && !tm_bwd) continue;  // the cluster kernels use plain loads
+        if (!grid_fwd && !grid_bwd && !st->fwdtm.use && !st->wide.use && !tm_bwd) continue;  // the cluster kernels use plain loads
         FLSTM_TRY(make_tensor_map_2d(&t.tm_w, l.w_hh, 4 * H, H, H, 64, 64, true));
         if (tm_bwd) FLSTM_TRY(make_bwd_tm_maps(&t.dg_tm, st->bwdtm, l.dg, dg_steps, B, H));
+        if (st->wide.use) {
+            FLSTM_TRY(make_tensor_map_gate_rows(&t.tm_ws, l.w_hh, H));
+            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->wide.BT / 2, 2));
+        }
         if (st->fwdtm.use) {
             FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->fwdtm.S * st->fwdtm.BT / 2, st->fwdtm.ch));
             FLSTM_TRY(make_tensor_map_3d(&t.tm_g, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwdtm.BT, 64, false));
@@ -286,7 +292,7 @@ int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs) {
     *ctas = !cluster ? 0 : backward ? st->cbwd.C : st->cfwd.C;
     *seqs = !cluster ? 0 : backward ? st->cbwd.seqs : st->cfwd.seqs;
     if (cluster) return FLSTM_PATH_CLUSTER;
-    if (!st->step.use || (backward ? st->bwdtm.use : st->fwdtm.use)) return FLSTM_PATH_GRID;
+    if (!st->step.use || (backward ? st->bwdtm.use : st->fwdtm.use || st->wide.use)) return FLSTM_PATH_GRID;
     return !backward && st->step.fwd_persistent && wavefront_chunk(e, (size_t)-1) == 0 ? FLSTM_PATH_GRID : FLSTM_PATH_STEPS;
 }
 
@@ -327,7 +333,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         e.launches += 2;
         return FLSTM_OK;
     }
-    if (st->step.use && !st->fwdtm.use) {
+    if (st->step.use && !st->fwdtm.use && !st->wide.use) {
         CUtensorMap tm_y;
         if (y_out) FLSTM_TRY(make_tensor_map_3d_tile(&tm_y, y_out, 2, t1, B, H, 32, 16));
         const StepFwdMaps maps{&t.tm_hs3, &t.tm_wstep, &t.tm_g_ep, &t.tm_c_ep, &t.tm_h_ep, y_out ? &tm_y : nullptr};
@@ -388,7 +394,8 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.trace_steps = e.trace_steps;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    if (st->fwdtm.use) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h, t.tm_g, p, s));
+    if (st->wide.use) FLSTM_TRY(lstm_forward_wide(e.cfg.dtype, st->wide, t.tm_ws, t.tm_h, p, s));
+    else if (st->fwdtm.use) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h, t.tm_g, p, s));
     else FLSTM_TRY(lstm_forward_persistent(e.cfg.dtype, st->fwd, t.tm_w, t.tm_h, t.tm_g, p, s));
     size_t m2 = e.timer.mark(s);
     e.timer.span(PH_PROJ, m0, m1);
@@ -517,7 +524,7 @@ static int backward_steps(Engine &e, int li, size_t T, size_t t0, size_t t1, con
 // layer-by-layer schedule.
 size_t wavefront_chunk(const Engine &e, size_t n) {
     TcState *st = static_cast<TcState *>(e.tc_state);
-    if (!st || !st->step.use || st->fwdtm.use || st->bwdtm.use || e.layers.size() < 2 || e.timer.enabled) return 0;
+    if (!st || !st->step.use || st->fwdtm.use || st->wide.use || st->bwdtm.use || e.layers.size() < 2 || e.timer.enabled) return 0;
     const char *env = std::getenv("FLSTM_WAVE_CHUNK");
     if (!env) return 0;
     const long v = std::atol(env);

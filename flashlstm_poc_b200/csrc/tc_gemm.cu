@@ -846,5 +846,19 @@ int make_tensor_map_halves(CUtensorMap *out, const void *base, uint64_t steps, u
     return FLSTM_OK;
 }
 
+int make_tensor_map_gate_rows(CUtensorMap *out, const void *base, uint64_t H) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return set_error(FLSTM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    cuuint64_t dims[5] = {H, 8, 4, 2, H / 16};
+    cuuint64_t strides[4] = {H * 2, 16 * H * 2, 8 * H * 2, 64 * H * 2};
+    cuuint32_t box[5] = {64, 8, 4, 2, 1};
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 5, const_cast<void *>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(FLSTM_ERR_CUDA, "cuTensorMapEncodeTiled (gate rows) failed (%d)", (int)r);
+    return FLSTM_OK;
+}
+
 }  // namespace tc
 }  // namespace flstm_b200

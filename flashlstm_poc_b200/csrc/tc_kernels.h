@@ -90,6 +90,25 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan);
 int lstm_forward_tm(int dtype, const FwdTmPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_ws, const CUtensorMap &tm_h,
                     const CUtensorMap &tm_g, const FwdParams &p, cudaStream_t s);
 
+// ------------------------------------------------------------------ wide batches with W_hh on the chip (tc_lstm_fwd_wide.cu)
+struct FwdWidePlan {
+    bool use;
+    int BT;        // sequences per batch tile: 64 or 128
+    int cta_rows;  // CTAs per batch group = H / 16
+    int ngroups;
+    int nt;        // batch tiles that a CTA takes in turn
+    int kc;        // 64-wide chunks of K
+    int ct, cs;    // of these, kept in tensor / shared memory (all of them)
+    int hstages;   // copies of h in the ring
+    int smem_bytes;
+    int grid;
+};
+constexpr int kMaxStepCounters = 900;  // words of Engine::sync_words that step barriers may take
+int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan);
+// tm_w: make_tensor_map_gate_rows.  tm_h: chunked map with box rows BT / 2 and 2 chunks.
+int lstm_forward_wide(int dtype, const FwdWidePlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_h, const FwdParams &p,
+                      cudaStream_t s);
+
 // ------------------------------------------------------------------ persistent BPTT
 struct BwdPlan {
     int BT;        // sequences per batch tile

@@ -1,0 +1,399 @@
+// Persistent recurrent forward kernel for wide batches: one launch runs all T time steps of one layer, W_hh stays on the chip
+// and a CTA works on several batch tiles in turn.
+//
+// What bounds an output-tiled step GEMM (tc_lstm_step.cu) is what an SM can take in: 768 KB of h and W_hh per CTA and step at
+// H = 2048, B = 256, through a port of about 60 B per cycle, and the chain from one step's stores to the next step's operands
+// stands between the steps.  Here a CTA pair (cta_group::2, M = 128: 64 gate rows, 16 units per CTA) keeps its rows of W_hh for
+// the whole sequence, in tensor memory (the A operand, held twice: lanes 0-63 and 64-127, as an M = 128 instruction over two CTAs
+// reads it) and what does not fit there in shared memory.  Only h is staged, half of a tile per CTA.  The batch tiles are
+// independent recurrences with a step barrier each, so the chain of one hides behind the UMMAs of the others.
+//
+// Per step and batch tile of BT sequences:
+//   producer warp : waits for the tile's step barrier, streams h_{t-1} through the ring (copies of two 64-wide chunks)
+//   UMMA thread   : M = 128, N = BT, accumulating over K = H into one of two accumulators (BT / 2 columns: sequences [0, BT/2) in
+//                   lanes 0-63, the others in lanes 64-127)
+//   8 other warps : the rows of A are ordered so that a lane quadrant holds the four gates of 8 units, 8 lanes each: two
+//                   tcgen05.ld of the 16x256b shape leave all four gate sums of a (unit, sequence) pair in one thread, and no
+//                   exchange through shared memory is needed.  Projections and cell states are read ahead of the wait; h_t is
+//                   stored and published first, cell states, gates and y follow.
+// Waits are bounded and the way out is that of tc_lstm_fwd.cu: producer and UMMA thread break out of their loops, the 256
+// epilogue threads leave together (the barrier behind their waits ORs the failures), an aborted pair lingers before the final
+// cluster barrier.
+//
+// Replaces the same reference launches as tc_lstm_fwd.cu (flashlstm_v2/src/lstm_forward.cu:744-830).
+#include <cstdlib>
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "tc_common.cuh"
+#include "tc_kernels.h"
+#include "tc_recurrent.cuh"
+
+namespace flstm_b200 {
+namespace tc {
+
+namespace {
+
+constexpr int kThreads = 320;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA issuer
+constexpr int kEpilogueThreads = 256;
+constexpr int kChunkBytesW = 64 * 128;  // 64 rows x 64 16-bit elements
+constexpr int kTmemColumns = 512;
+constexpr int kCh = 2;  // chunks per copy of h
+constexpr int kBarrierBytes = 1024, kMinSmemBytes = 120 * 1024;
+constexpr int kFillSlots = 14;
+static_assert(kBarrierBytes + kFillSlots * kChunkBytesW + 1024 <= kMinSmemBytes, "the fill slots fit every launch");
+
+__host__ __device__ inline int smem_of(const FwdWidePlan &pl) {
+    return kBarrierBytes + pl.cs * kChunkBytesW + pl.hstages * kCh * (pl.BT / 2) * 128 + 1024 /*align*/;
+}
+
+template <int BT, bool BF16, bool ACCURATE>
+__global__ void __launch_bounds__(kThreads, 1)
+lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_h,
+                     const __grid_constant__ FwdWidePlan pl, FwdParams p) {
+    constexpr int BTH = BT / 2;        // B rows a CTA stages, columns of an accumulator
+    constexpr int WC = BTH / 2;        // columns a warp finishes
+    constexpr int GROUPS = WC / 8;     // of 8 columns
+    constexpr int PAIRS = 2 * GROUPS;  // (unit, sequence) pairs per thread
+    constexpr int kStageBytes = kCh * BTH * 128;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int KC = pl.kc, CT = pl.ct, CS = pl.cs, NLOAD = (KC + kCh - 1) / kCh, HST = pl.hstages, NT = pl.nt;
+    uint8_t *s_w = smem + kBarrierBytes, *s_h = s_w + CS * kChunkBytesW;
+    uint64_t *hfull = reinterpret_cast<uint64_t *>(smem), *hempty = hfull + HST;
+    uint64_t *tfull = hempty + HST, *tempty = tfull + 2, *wbar = tempty + 2;
+    uint64_t *ffull = wbar + 1, *fempty = ffull + kFillSlots;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fempty + kFillSlots);
+    volatile uint32_t *abort_w = tmem_slot + 1;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ng = blockIdx.x / pl.cta_rows, jr = blockIdx.x % pl.cta_rows;  // batch group, 16-unit tile
+    const uint32_t rank = cluster_ctarank();
+    const bool leader = rank == 0;
+    const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < HST; ++i) {
+            mbar_init(&hfull[i], 1);
+            mbar_init(&hempty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], 2 * kEpilogueThreads / 32);  // the epilogue warps of both CTAs report to the leader
+        }
+        mbar_init(wbar, 1);
+        for (int i = 0; i < kFillSlots; ++i) {
+            mbar_init(&ffull[i], 1);
+            mbar_init(&fempty[i], 4);
+        }
+        *abort_w = 0;
+        fence_barrier_init();
+        tma_prefetch_desc(&tm_w);
+        tma_prefetch_desc(&tm_h);
+    }
+    if (warp == 5) {
+        tmem_alloc_pair(tmem_slot, kTmemColumns);
+        tmem_relinquish_pair();
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + 2 * BTH;
+    // W_hh into tensor memory by way of the shared memory that the ring will use: lanes l and l + 64 take row l of the tile in the
+    // map's order (unit half, gate, unit), 32 columns of two elements per chunk; the warps 0-3 take the even chunks, 6-9 the odd
+    // ones.  A wait that expires raises the abort word, on which every role below gives up.
+    if (warp == 4 && elect_one()) {
+        for (int c = 0; c < CT; ++c) {
+            const int slot = c % kFillSlots;
+            if (c >= kFillSlots && !mbar_wait(&fempty[slot], (uint32_t)(c / kFillSlots - 1) & 1u, abort_w, wait_ns)) break;
+            mbar_expect_tx(&ffull[slot], kChunkBytesW);
+            tma_load_5d(s_w + slot * kChunkBytesW, &tm_w, c * 64, 0, 0, 0, jr, &ffull[slot]);
+        }
+    } else if (warp != 4 && warp != 5) {
+        const int quad = warp & 3, row = (quad & 1) * 32 + lane;
+        const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
+        for (int c = warp < 4 ? 0 : 1; c < CT; c += 2) {
+            const int slot = c % kFillSlots;
+            if (!__all_sync(0xffffffffu, mbar_wait(&ffull[slot], (uint32_t)(c / kFillSlots) & 1u, abort_w, wait_ns))) break;
+            const uint8_t *src = s_w + slot * kChunkBytesW + row * 128;
+            uint32_t r[32];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(src + ((i ^ (row & 7)) * 16));
+                r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
+            }
+            tmem_st_32x32b_x32(dst + c * 32, r);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&fempty[slot]);
+        }
+        tmem_st_wait();
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    cluster_sync_all();  // both CTAs' barriers and tensor memory exist before anything crosses the pair
+    tcgen05_fence_after();
+    // barriers the loads of this CTA complete: the leader's at the same offsets
+    const uint32_t hfull_c = map_to_rank(smem_u32(hfull), 0), wbar_c = map_to_rank(smem_u32(wbar), 0);
+    const uint32_t tempty_c = map_to_rank(smem_u32(tempty), 0);
+
+    if (warp == 4) {
+        // ------------------------------------------------------------ producer
+        if (elect_one()) {
+            bool ok = true;
+            if (CS > 0) {
+                if (leader) mbar_expect_tx(wbar, 2u * (uint32_t)(CS * kChunkBytesW));
+                for (int c = 0; c < CS; ++c) tma_load_5d_pair(s_w + c * kChunkBytesW, &tm_w, (CT + c) * 64, 0, 0, 0, jr, wbar_c);
+            }
+            int stage = 0;
+            uint32_t phase = 0, issued = 0, parity = 0;
+            for (int tt = 0; tt < p.T && ok; ++tt)
+                for (int n = 0; n < NT && ok; ++n) {
+                    const int b0 = (ng * NT + n) * BT;
+                    if (b0 >= p.B) break;  // a group's last tiles may be empty
+                    if (tt > 0) {  // h_{t-1} of this tile is complete when every CTA of the group has arrived tt times
+                        ok = wait_counter(p.counters + ng * NT + n, (unsigned)pl.cta_rows * (unsigned)tt + p.extra_arrivals, p.err, abort_w,
+                                          2u, wait_ns);
+                        if (!ok) break;
+                        fence_proxy_async_global();
+                    }
+                    for (int ld = 0; ld < NLOAD; ++ld) {
+                        ok = mbar_wait(&hempty[stage], phase ^ 1, abort_w, wait_ns);
+                        if (!ok) break;
+                        if (leader) mbar_expect_tx(&hfull[stage], 2u * kStageBytes);
+                        issued |= 1u << stage;
+                        parity = (parity & ~(1u << stage)) | (phase << stage);
+                        // chunks beyond K come as zeros (and are counted)
+                        tma_load_4d_pair(s_h + stage * kStageBytes, &tm_h, 0, b0 + (int)rank * BTH, ld * kCh, p.t0 + tt,
+                                         hfull_c + 8u * (uint32_t)stage);
+                        if (++stage == HST) { stage = 0; phase ^= 1; }
+                    }
+                }
+            // way out: every copy this thread started must have landed before the CTA exits (the peer's copies complete
+            // the leader's barriers; after an abort the whole pair lingers, see below)
+            if (CS > 0 && leader) mbar_drain(wbar, 0, wait_ns);
+            for (int i = 0; i < HST && leader; ++i)
+                if (issued >> i & 1u) mbar_drain(&hfull[i], parity >> i & 1u, ok ? wait_ns : kAbortDrainNs);
+        }
+    } else if (warp == 5) {
+        // ------------------------------------------------------------ UMMA issuer (the leader's)
+        if (leader && elect_one()) {
+            bool ok = CS == 0 || mbar_wait(wbar, 0, abort_w, wait_ns);
+            int stage = 0;
+            uint32_t phase = 0, wi = 0;
+            constexpr uint32_t idesc = umma_idesc_f16(128, BT, BF16 ? 1 : 0, 0, 0);
+            constexpr uint32_t kStepH = (BTH * 128) >> 4, kStepW = kChunkBytesW >> 4;  // descriptor units
+            const uint32_t hempty_l = smem_u32(hempty), tfull_l = smem_u32(tfull);
+            const uint32_t dw_res = umma_desc_lo(smem_u32(s_w)), dh_ring = umma_desc_lo(smem_u32(s_h));
+            for (int tt = 0; tt < p.T && ok; ++tt)
+                for (int n = 0; n < NT && ok; ++n) {
+                    if ((ng * NT + n) * BT >= p.B) break;
+                    const uint32_t buf = wi & 1;
+                    ok = mbar_wait_cluster(&tempty[buf], ((wi >> 1) & 1) ^ 1, abort_w, wait_ns);
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                    const uint32_t d = tmem_base + buf * BTH;
+                    for (int ld = 0; ld < NLOAD; ++ld) {
+                        ok = mbar_wait(&hfull[stage], phase, abort_w, wait_ns);
+                        if (!ok) break;
+                        tcgen05_fence_after();
+                        const uint32_t dh = dh_ring + (uint32_t)stage * (kStageBytes >> 4);
+#pragma unroll
+                        for (int e = 0; e < kCh; ++e) {
+                            const int c = ld * kCh + e;
+                            if (c < CT) {
+                                const uint32_t da = tmem_a + (uint32_t)c * 32;
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_lo_ts<true>(d, da + 8 * k, dh + e * kStepH + 2 * k, idesc, (uint32_t)(c | k));
+                            } else if (c < KC) {
+                                const uint32_t dw = dw_res + (uint32_t)(c - CT) * kStepW;
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_lo_ss<true>(d, dw + 2 * k, dh + e * kStepH + 2 * k, idesc, (uint32_t)(c | k));
+                            }
+                        }
+                        umma_commit_pair_both(hempty_l + 8u * (uint32_t)stage);
+                        if (++stage == HST) { stage = 0; phase ^= 1; }
+                    }
+                    if (!ok) break;
+                    umma_commit_pair_both(tfull_l + 8u * buf);
+                    ++wi;
+                }
+            // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
+            if (wi > 0) mbar_drain(&tfull[(wi - 1) & 1], (wi - 1) >> 1 & 1u, wait_ns);
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue (256 threads)
+        const int tid = warp < 4 ? threadIdx.x : threadIdx.x - 64;
+        const int quad = warp & 3;
+        const int U = jr * 16 + (quad & 1) * 8 + (lane >> 2);                                   // this thread's unit
+        const int seq0 = (quad >> 1) * BTH + (warp < 4 ? 0 : WC) + 2 * (lane & 3);  // of a tile: pair (i, e) is sequence seq0 + 8 i + e
+        const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (warp < 4 ? 0 : WC);
+        const size_t slab = (size_t)p.B * p.H, G = (size_t)4 * p.H;
+        const bool pad = ACCURATE && U >= p.real_units;
+        uint16_t *hs = static_cast<uint16_t *>(p.hs);
+        uint16_t *y = static_cast<uint16_t *>(p.y);
+        uint16_t *gates = static_cast<uint16_t *>(p.gates);
+        uint32_t wi = 0;
+        bool ok = true;
+        for (int tt = 0; tt < p.T && ok; ++tt) {
+            const int t = p.t0 + tt;
+            for (int n = 0; n < NT && ok; ++n, ++wi) {
+                const int b0 = (ng * NT + n) * BT;
+                if (b0 >= p.B) break;
+                const uint32_t buf = wi & 1;
+                const int rows_left = p.B - b0 - seq0;  // pair (i, e) exists while 8 i + e < rows_left
+                const size_t row0 = (size_t)b0 + seq0;
+                uint16_t *grow = gates + ((size_t)t * p.B + row0) * G + (size_t)jr * 64 + (U & 15);
+                const size_t idx0 = row0 * p.H + U;
+                uint16_t proj[PAIRS][4];
+                float c_prev[PAIRS];
+#pragma unroll
+                for (int k = 0; k < PAIRS; ++k) {
+                    const int r = 8 * (k >> 1) + (k & 1);
+                    const bool there = r < rows_left;
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) proj[k][g] = there ? grow[(size_t)r * G + g * 16] : (uint16_t)0;
+                    c_prev[k] = there ? p.cs[(size_t)t * slab + idx0 + (size_t)r * p.H] : 0.f;
+                }
+                // No thread leaves between here and the named barrier below, whatever its wait returns: the barrier ORs the
+                // failures, so that all 256 threads go on or give up together.  A warp reads the accumulator only if all of
+                // its lanes saw it complete.
+                const bool good = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (wi >> 1) & 1, abort_w, wait_ns));
+                tcgen05_fence_after();
+                uint32_t lo[4 * GROUPS], hi[4 * GROUPS];  // gates i, f and g, o: per 8 columns two of each
+                if (good) {
+                    tmem_ld_16x256b<GROUPS>(taddr0 + buf * BTH, lo);
+                    tmem_ld_16x256b<GROUPS>(taddr0 + (16u << 16) + buf * BTH, hi);
+                    tmem_ld_wait();
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4 * GROUPS; ++i) lo[i] = hi[i] = 0u;
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                // relaxed: it orders the reuse of the accumulator only (a release would wait for the warp's global stores)
+                if (lane == 0) mbar_arrive_cluster_relaxed(tempty_c + 8u * buf);
+                uint16_t act[PAIRS][4], h16[PAIRS];
+                float c_new[PAIRS];
+                uint16_t *h_out = hs + (size_t)(t + 1) * slab + idx0;
+#pragma unroll
+                for (int k = 0; k < PAIRS; ++k) {
+                    const int i = k >> 1, e = k & 1, r = 8 * i + e;
+                    const float ai = __uint_as_float(lo[4 * i + e]) + load16<BF16>(&proj[k][0]), af = __uint_as_float(lo[4 * i + 2 + e]) + load16<BF16>(&proj[k][1]);
+                    const float ag = __uint_as_float(hi[4 * i + e]) + load16<BF16>(&proj[k][2]), ao = __uint_as_float(hi[4 * i + 2 + e]) + load16<BF16>(&proj[k][3]);
+                    const float gi = sigmoid_sel<ACCURATE>(pad ? 0.f : ai), gf = sigmoid_sel<ACCURATE>(pad ? 0.f : af);
+                    const float gg = tanh_sel<ACCURATE>(pad ? 0.f : ag), go = sigmoid_sel<ACCURATE>(pad ? 0.f : ao);
+                    c_new[k] = fmaf(gf, c_prev[k], gi * gg);
+                    h16[k] = to16<BF16>(go * tanh_sel<ACCURATE>(c_new[k]));
+                    act[k][0] = to16<BF16>(gi);
+                    act[k][1] = to16<BF16>(gf);
+                    act[k][2] = to16<BF16>(gg);
+                    act[k][3] = to16<BF16>(go);
+                    // h_t first: it is what the other CTAs wait for
+                    if (good && r < rows_left) h_out[(size_t)r * p.H] = h16[k];
+                }
+                if (named_barrier_or(1, kEpilogueThreads, !good)) {
+                    ok = false;
+                    break;
+                }
+                // publish h_t of the tile: after the named barrier thread 0's release is cumulative over every epilogue warp's
+                // stores; the generic->async proxy fence is the consumer's
+                if (tid == 0) red_release_gpu_add(p.counters + ng * NT + n, 1u);
+                // everything nobody waits for: cell state, gate cache, the caller's y
+#pragma unroll
+                for (int k = 0; k < PAIRS; ++k) {
+                    const int r = 8 * (k >> 1) + (k & 1);
+                    if (r >= rows_left) continue;
+                    p.cs[(size_t)(t + 1) * slab + idx0 + (size_t)r * p.H] = c_new[k];
+                    if (y) y[(size_t)t * slab + idx0 + (size_t)r * p.H] = h16[k];
+                    if (p.store_gates) {
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) grow[(size_t)r * G + g * 16] = act[k][g];
+                    }
+                }
+            }
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    // after an abort this CTA's own copies may still be landing on barriers it cannot see (the leader's)
+    if (*abort_w) {
+        const unsigned long long t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < kAbortDrainNs) {}
+    }
+    cluster_sync_all();  // the peer's shared and tensor memory stay valid until the leader's last UMMA is consumed
+    if (warp == 5) tmem_dealloc_pair(tmem_base, kTmemColumns);
+    if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
+    if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / pl.cta_rows * NT, p.exits);
+}
+
+template <int BT, bool BF16, bool ACC>
+int launch_one(const CUtensorMap &tw, const CUtensorMap &th, const FwdWidePlan &pl, const FwdParams &p, cudaStream_t s) {
+    auto kern = lstm_fwd_wide_kernel<BT, BF16, ACC>;
+    FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)pl.smem_bytes));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = pl.smem_bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs must be co-resident: they wait on one another
+    attr[0].val.cooperative = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, th, pl, p);
+    if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "recurrent forward launch failed: %s", cudaGetErrorString(e));
+    return FLSTM_OK;
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ host side
+int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan) {
+    *plan = FwdWidePlan{};
+    if (H % 64 != 0 || H < 64 || smem_limit < 160 * 1024) return FLSTM_OK;
+    const char *env = std::getenv("FLSTM_TMEM"), *pair = std::getenv("FLSTM_FWD_PAIR");  // as for plan_fwd_tm
+    if ((env && env[0] == '0') || (pair && pair[0] == '0')) return FLSTM_OK;
+    FwdWidePlan pl{};
+    pl.cta_rows = H / 16;
+    if (pl.cta_rows > sms || pl.cta_rows % 2) return FLSTM_OK;
+    const int groups = sms / pl.cta_rows;
+    // two tiles of 64 sequences in turn rather than one of 128, whose chain would stand alone
+    pl.BT = B <= 128 * groups ? 64 : 128;
+    const int tiles = (B + pl.BT - 1) / pl.BT;
+    pl.nt = (tiles + groups - 1) / groups;
+    pl.ngroups = (tiles + pl.nt - 1) / pl.nt;
+    if (pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
+    pl.kc = H / 64;
+    const int tmem_chunks = (kTmemColumns - pl.BT) / 32;
+    pl.ct = pl.kc < tmem_chunks ? pl.kc : tmem_chunks;
+    pl.cs = pl.kc - pl.ct;
+    pl.hstages = 16;
+    while (pl.hstages > 3 && (size_t)smem_of(pl) > smem_limit) --pl.hstages;
+    if ((size_t)smem_of(pl) > smem_limit) return FLSTM_OK;
+    pl.smem_bytes = smem_of(pl) > kMinSmemBytes ? smem_of(pl) : kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
+    pl.grid = pl.cta_rows * pl.ngroups;
+    pl.use = true;
+    *plan = pl;
+    return FLSTM_OK;
+}
+
+int lstm_forward_wide(int dtype, const FwdWidePlan &pl, const CUtensorMap &tw, const CUtensorMap &th, const FwdParams &p, cudaStream_t s) {
+    const bool bf16 = dtype == FLSTM_DTYPE_BF16, acc = p.real_units > 0;
+#define FLSTM_WIDE_CASE(BT_)                                                                                                \
+    if (pl.BT == BT_) {                                                                                                     \
+        if (bf16) return acc ? launch_one<BT_, true, true>(tw, th, pl, p, s) : launch_one<BT_, true, false>(tw, th, pl, p, s); \
+        return acc ? launch_one<BT_, false, true>(tw, th, pl, p, s) : launch_one<BT_, false, false>(tw, th, pl, p, s);       \
+    }
+    FLSTM_WIDE_CASE(64) FLSTM_WIDE_CASE(128)
+#undef FLSTM_WIDE_CASE
+    return set_error(FLSTM_ERR_UNSUPPORTED, "no wide forward kernel for this plan");
+}
+
+}  // namespace tc
+}  // namespace flstm_b200

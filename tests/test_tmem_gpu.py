@@ -1,6 +1,6 @@
-"""The recurrent kernels that hold W_hh in tensor memory (tc_lstm_fwd_tm.cu, tc_lstm_bwd_tm.cu) against the oracle, at the edges
+"""The recurrent kernels that hold W_hh in tensor memory (tc_lstm_fwd_tm.cu, tc_lstm_fwd_wide.cu, tc_lstm_bwd_tm.cu) against the oracle, at the edges
 of their tiling: an odd and an even number of 64-wide K chunks per half, weights in tensor memory only, beside shared memory
-and streamed, every batch-tile width, partly filled tiles, one and two batch groups, and step ranges that continue a launch."""
+and streamed, every batch-tile width, partly filled and empty tiles, one and two batch groups, one to four batch tiles in turn, and step ranges that continue a launch."""
 import pytest
 import torch
 
@@ -13,6 +13,8 @@ pytestmark = pytest.mark.gpu
 # batch, hidden size, training
 SHAPES = [(1, 1088, True), (70, 1088, True), (33, 1152, True), (100, 1152, True), (40, 1216, True), (32, 1280, True),
           (5, 2048, True), (64, 2048, True), (31, 2304, True), (50, 2368, True),
+          (140, 1024, True), (256, 1024, True), (259, 1024, False), (300, 704, True), (130, 1088, True), (65, 1984, False),
+          (100, 2048, True), (256, 2048, True), (150, 2176, False),  # the last nine: batch tiles in turn
           (3, 2432, False), (16, 2496, False), (17, 3072, False), (33, 4096, False), (8, 4096, False), (64, 2560, False)]
 
 
@@ -26,7 +28,7 @@ def test_tensor_memory_kernels_match_the_oracle(B, H, training):
     assert_parity(got, run_oracle(inp), dtype)
 
 
-@pytest.mark.parametrize("B,H", [(7, 1088), (40, 2048)])
+@pytest.mark.parametrize("B,H", [(7, 1088), (40, 2048), (140, 1024)])
 def test_ranges_continue_one_another(B, H):
     """Forward and backward in step ranges equal one call."""
     w = Workload("t", "f16", 1, 64, H, B, 7, seed=52, state_std=0.3)

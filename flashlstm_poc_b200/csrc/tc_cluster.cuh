@@ -51,12 +51,6 @@ __device__ __forceinline__ void cp_async_wait() {
 // Steps a kernel's inputs are fetched ahead of their use: a step takes 700..3000 cycles, a fetch from memory more than
 // the shortest of them (fetched one step ahead, H = 64 ran at 2300 cycles a step).
 constexpr int kClusterAhead = 4;
-// transpose of an 8x8 matrix of 16-bit elements spread over the warp (row = lane / 4, columns 2 (lane % 4) + {0, 1})
-__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
-    uint32_t r;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
-    return r;
-}
 
 // shared-memory row of `bytes` (a multiple of 64), padded so that the 16-byte fragment reads of 8 rows do not conflict
 __host__ __device__ constexpr int cluster_row_bytes(int bytes) { return bytes % 128 ? bytes : bytes + 64; }

@@ -42,6 +42,24 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// Transpose of an 8x8 matrix of 16-bit elements spread over the warp as an mma fragment (row = lane / 4, columns 2 (lane % 4) + {0, 1}).
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+// 4x4 transpose over the four lanes of a quad: lane q gets r[j] = r[q] of lane j.
+__device__ __forceinline__ void quad_transpose(uint32_t (&r)[4], int lane) {
+    const bool b0 = lane & 1, b1 = lane & 2;
+    const uint32_t x = __shfl_xor_sync(0xffffffffu, b0 ? r[0] : r[1], 1), y = __shfl_xor_sync(0xffffffffu, b0 ? r[2] : r[3], 1);
+    const uint32_t a = b0 ? x : r[0], b = b0 ? r[1] : x, c = b0 ? y : r[2], d = b0 ? r[3] : y;
+    const uint32_t u = __shfl_xor_sync(0xffffffffu, b1 ? a : c, 2), v = __shfl_xor_sync(0xffffffffu, b1 ? b : d, 2);
+    r[0] = b1 ? u : a;
+    r[1] = b1 ? v : b;
+    r[2] = b1 ? c : u;
+    r[3] = b1 ? d : v;
+}
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -12,13 +12,12 @@
 //   producer warp : waits for the tile's step barrier, streams h_{t-1} through the ring (copies of two 64-wide chunks)
 //   UMMA thread   : M = 128, N = BT, accumulating over K = H into one of two accumulators (BT / 2 columns: sequences [0, BT/2) in
 //                   lanes 0-63, the others in lanes 64-127)
-//   8 other warps : the rows of A are ordered so that a lane quadrant holds the four gates of 8 units, 8 lanes each: two
+//   8 warps       : the rows of A are ordered so that a lane quadrant holds the four gates of 8 units, 8 lanes each: two
 //                   tcgen05.ld of the 16x256b shape leave all four gate sums of a (unit, sequence) pair in one thread, and no
-//                   exchange through shared memory is needed.  Projections and cell states are read ahead of the wait; h_t is
-//                   stored and published first, cell states, gates and y follow.
-// Waits are bounded and the way out is that of tc_lstm_fwd.cu: producer and UMMA thread break out of their loops, the 256
-// epilogue threads leave together (the barrier behind their waits ORs the failures), an aborted pair lingers before the final
-// cluster barrier.
+//                   exchange through shared memory is needed.  Projections and cell states are read a tile ahead; h_t is stored
+//                   first, cell states, gates and y follow while a thread of its own publishes h_t.
+// Waits are bounded; producer, publisher, UMMA thread and each epilogue warp break out of their loops by themselves (no barrier of
+// threads lies inside the loops) and meet at the final __syncthreads; an aborted pair lingers before the final cluster barrier.
 //
 // Replaces the same reference launches as tc_lstm_fwd.cu (flashlstm_v2/src/lstm_forward.cu:744-830).
 #include <cstdlib>
@@ -36,8 +35,8 @@ namespace tc {
 
 namespace {
 
-constexpr int kThreads = 320;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA issuer
-constexpr int kEpilogueThreads = 256;
+constexpr int kThreads = 352;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA issuer, 10 publisher of h
+constexpr int kEpilogueWarps = 8;
 constexpr int kChunkBytesW = 64 * 128;  // 64 rows x 64 16-bit elements
 constexpr int kTmemColumns = 512;
 constexpr int kCh = 2;  // chunks per copy of h
@@ -60,16 +59,19 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     constexpr int kStageBytes = kCh * BTH * 128;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int KC = pl.kc, CT = pl.ct, CS = pl.cs, NLOAD = (KC + kCh - 1) / kCh, HST = pl.hstages, NT = pl.nt;
+    const int KC = pl.kc, CT = pl.ct, CS = pl.cs, NLOAD = (KC + kCh - 1) / kCh, HST = pl.hstages;
     uint8_t *s_w = smem + kBarrierBytes, *s_h = s_w + CS * kChunkBytesW;
     uint64_t *hfull = reinterpret_cast<uint64_t *>(smem), *hempty = hfull + HST;
-    uint64_t *tfull = hempty + HST, *tempty = tfull + 2, *wbar = tempty + 2;
+    uint64_t *tfull = hempty + HST, *tempty = tfull + 2, *hdone = tempty + 2, *wbar = hdone + 2;
     uint64_t *ffull = wbar + 1, *fempty = ffull + kFillSlots;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fempty + kFillSlots);
     volatile uint32_t *abort_w = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ng = blockIdx.x / pl.cta_rows, jr = blockIdx.x % pl.cta_rows;  // batch group, 16-unit tile
+    const int tile0 = ng * pl.nt, tiles = (p.B + BT - 1) / BT;
+    const int NT = tiles - tile0 < pl.nt ? tiles - tile0 : pl.nt;  // batch tiles of this group
+    unsigned int *counters = p.counters + tile0;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
     const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
@@ -81,7 +83,8 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&tfull[i], 1);
-            mbar_init(&tempty[i], 2 * kEpilogueThreads / 32);  // the epilogue warps of both CTAs report to the leader
+            mbar_init(&tempty[i], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs report to the leader
+            mbar_init(&hdone[i], kEpilogueWarps);
         }
         mbar_init(wbar, 1);
         for (int i = 0; i < kFillSlots; ++i) {
@@ -111,7 +114,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             mbar_expect_tx(&ffull[slot], kChunkBytesW);
             tma_load_5d(s_w + slot * kChunkBytesW, &tm_w, c * 64, 0, 0, 0, jr, &ffull[slot]);
         }
-    } else if (warp != 4 && warp != 5) {
+    } else if (warp != 4 && warp != 5 && warp != 10) {
         const int quad = warp & 3, row = (quad & 1) * 32 + lane;
         const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
         for (int c = warp < 4 ? 0 : 1; c < CT; c += 2) {
@@ -150,11 +153,9 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             uint32_t phase = 0, issued = 0, parity = 0;
             for (int tt = 0; tt < p.T && ok; ++tt)
                 for (int n = 0; n < NT && ok; ++n) {
-                    const int b0 = (ng * NT + n) * BT;
-                    if (b0 >= p.B) break;  // a group's last tiles may be empty
+                    const int b0 = (tile0 + n) * BT;
                     if (tt > 0) {  // h_{t-1} of this tile is complete when every CTA of the group has arrived tt times
-                        ok = wait_counter(p.counters + ng * NT + n, (unsigned)pl.cta_rows * (unsigned)tt + p.extra_arrivals, p.err, abort_w,
-                                          2u, wait_ns);
+                        ok = wait_counter(counters + n, (unsigned)pl.cta_rows * (unsigned)tt + p.extra_arrivals, p.err, abort_w, 2u, wait_ns);
                         if (!ok) break;
                         fence_proxy_async_global();
                     }
@@ -188,7 +189,6 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             const uint32_t dw_res = umma_desc_lo(smem_u32(s_w)), dh_ring = umma_desc_lo(smem_u32(s_h));
             for (int tt = 0; tt < p.T && ok; ++tt)
                 for (int n = 0; n < NT && ok; ++n) {
-                    if ((ng * NT + n) * BT >= p.B) break;
                     const uint32_t buf = wi & 1;
                     ok = mbar_wait_cluster(&tempty[buf], ((wi >> 1) & 1) ^ 1, abort_w, wait_ns);
                     if (!ok) break;
@@ -222,94 +222,150 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
             if (wi > 0) mbar_drain(&tfull[(wi - 1) & 1], (wi - 1) >> 1 & 1u, wait_ns);
         }
+    } else if (warp == 10) {
+        // ------------------------------------------------------------ publisher
+        // The release takes about a thousand cycles (it waits for the stores it covers); on a thread of its own the epilogue goes
+        // on meanwhile.  hdone orders it behind every epilogue warp's stores of h; the generic->async proxy fence is the consumer's.
+        if (elect_one()) {
+            uint32_t wi = 0;
+            bool ok = true;
+            for (int tt = 0; tt < p.T && ok; ++tt)
+                for (int n = 0; n < NT && ok; ++n, ++wi) {
+                    ok = mbar_wait(&hdone[wi & 1], (wi >> 1) & 1, abort_w, wait_ns);
+                    if (ok) red_release_gpu_add(counters + n, 1u);
+                }
+        }
     } else {
-        // ------------------------------------------------------------ epilogue (256 threads)
-        const int tid = warp < 4 ? threadIdx.x : threadIdx.x - 64;
-        const int quad = warp & 3;
-        const int U = jr * 16 + (quad & 1) * 8 + (lane >> 2);                                   // this thread's unit
-        const int seq0 = (quad >> 1) * BTH + (warp < 4 ? 0 : WC) + 2 * (lane & 3);  // of a tile: pair (i, e) is sequence seq0 + 8 i + e
+        // ------------------------------------------------------------ epilogue (8 warps, each on its own)
+        // Quadrant q of the lanes: unit half q & 1, sequences (q >> 1) BT / 2 of the tile, of which this warp takes WC columns, 8
+        // at a time.  An accumulator fragment is (unit lane / 4, sequences 2 (lane % 4) and + 1); 16-bit data move as (sequence
+        // lane / 4, 8 units of gate lane % 4: 16 bytes) and (sequence lane / 4, units 2 (lane % 4) and + 1 of h: 4 bytes), between
+        // which movmatrix and a transpose over quads translate.  As 2-byte accesses in fragment order they took 10 k cycles per
+        // tile of 128 sequences, four times the UMMAs.
+        const int quad = warp & 3, half = quad & 1, q = lane & 3, s8 = lane >> 2;
+        const int U = jr * 16 + half * 8 + s8;                           // unit of this thread's fragments
+        const int col0 = (quad >> 1) * BTH + (warp < 4 ? 0 : WC);        // first sequence of the warp within a tile
         const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (warp < 4 ? 0 : WC);
         const size_t slab = (size_t)p.B * p.H, G = (size_t)4 * p.H;
         const bool pad = ACCURATE && U >= p.real_units;
         uint16_t *hs = static_cast<uint16_t *>(p.hs);
         uint16_t *y = static_cast<uint16_t *>(p.y);
         uint16_t *gates = static_cast<uint16_t *>(p.gates);
+        const bool y_words = (reinterpret_cast<uintptr_t>(y) & 3) == 0;
+        const size_t gcol = (size_t)jr * 64 + q * 16 + half * 8;         // gate q, 8 units
+        const size_t hcol = (size_t)jr * 16 + half * 8 + 2 * q;          // two units of h
+        uint4 p_next[GROUPS];
+        float c_next[PAIRS];
+        auto fetch_p = [&](int t, int n) {
+            const int b = (tile0 + n) * BT + col0 + s8;
+#pragma unroll
+            for (int i = 0; i < GROUPS; ++i)
+                p_next[i] = b + 8 * i < p.B ? *reinterpret_cast<const uint4 *>(gates + ((size_t)t * p.B + b + 8 * i) * G + gcol) : make_uint4(0, 0, 0, 0);
+        };
+        auto fetch_c = [&](int t, int n) {
+            const int b = (tile0 + n) * BT + col0 + 2 * q;
+#pragma unroll
+            for (int k = 0; k < PAIRS; ++k) {
+                const int r = b + 8 * (k >> 1) + (k & 1);
+                c_next[k] = r < p.B ? p.cs[(size_t)t * slab + (size_t)r * p.H + U] : 0.f;
+            }
+        };
+        fetch_p(p.t0, 0);
+        fetch_c(p.t0, 0);
         uint32_t wi = 0;
         bool ok = true;
         for (int tt = 0; tt < p.T && ok; ++tt) {
             const int t = p.t0 + tt;
-            for (int n = 0; n < NT && ok; ++n, ++wi) {
-                const int b0 = (ng * NT + n) * BT;
-                if (b0 >= p.B) break;
+            for (int n = 0; n < NT; ++n, ++wi) {
                 const uint32_t buf = wi & 1;
-                const int rows_left = p.B - b0 - seq0;  // pair (i, e) exists while 8 i + e < rows_left
-                const size_t row0 = (size_t)b0 + seq0;
-                uint16_t *grow = gates + ((size_t)t * p.B + row0) * G + (size_t)jr * 64 + (U & 15);
-                const size_t idx0 = row0 * p.H + U;
-                uint16_t proj[PAIRS][4];
-                float c_prev[PAIRS];
+                const int b = (tile0 + n) * BT + col0;
+                uint32_t proj[GROUPS][4];
+                float c[PAIRS];
 #pragma unroll
-                for (int k = 0; k < PAIRS; ++k) {
-                    const int r = 8 * (k >> 1) + (k & 1);
-                    const bool there = r < rows_left;
+                for (int i = 0; i < GROUPS; ++i) {
+                    proj[i][0] = p_next[i].x; proj[i][1] = p_next[i].y; proj[i][2] = p_next[i].z; proj[i][3] = p_next[i].w;
+                    quad_transpose(proj[i], lane);
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) proj[k][g] = there ? grow[(size_t)r * G + g * 16] : (uint16_t)0;
-                    c_prev[k] = there ? p.cs[(size_t)t * slab + idx0 + (size_t)r * p.H] : 0.f;
+                    for (int g = 0; g < 4; ++g) proj[i][g] = movmatrix_trans(proj[i][g]);
                 }
-                // No thread leaves between here and the named barrier below, whatever its wait returns: the barrier ORs the
-                // failures, so that all 256 threads go on or give up together.  A warp reads the accumulator only if all of
-                // its lanes saw it complete.
-                const bool good = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (wi >> 1) & 1, abort_w, wait_ns));
+#pragma unroll
+                for (int k = 0; k < PAIRS; ++k) c[k] = c_next[k];
+                // the next tile's projections and, unless it is this one again, its cell states
+                const int n_next = n + 1 == NT ? 0 : n + 1, t_next = n + 1 == NT ? t + 1 : t;
+                const bool more = t_next < p.t0 + p.T;
+                if (more) fetch_p(t_next, n_next);
+                if (more && NT > 1) fetch_c(t_next, n_next);
+                // a warp reads the accumulator only if all of its lanes saw it complete
+                ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (wi >> 1) & 1, abort_w, wait_ns));
+                if (!ok) break;
                 tcgen05_fence_after();
                 uint32_t lo[4 * GROUPS], hi[4 * GROUPS];  // gates i, f and g, o: per 8 columns two of each
-                if (good) {
-                    tmem_ld_16x256b<GROUPS>(taddr0 + buf * BTH, lo);
-                    tmem_ld_16x256b<GROUPS>(taddr0 + (16u << 16) + buf * BTH, hi);
-                    tmem_ld_wait();
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4 * GROUPS; ++i) lo[i] = hi[i] = 0u;
-                }
+                tmem_ld_16x256b<GROUPS>(taddr0 + buf * BTH, lo);
+                tmem_ld_16x256b<GROUPS>(taddr0 + (16u << 16) + buf * BTH, hi);
+                tmem_ld_wait();
                 tcgen05_fence_before();
-                __syncwarp();
-                // relaxed: it orders the reuse of the accumulator only (a release would wait for the warp's global stores)
-                if (lane == 0) mbar_arrive_cluster_relaxed(tempty_c + 8u * buf);
-                uint16_t act[PAIRS][4], h16[PAIRS];
-                float c_new[PAIRS];
-                uint16_t *h_out = hs + (size_t)(t + 1) * slab + idx0;
+                uint32_t act[GROUPS][4], h2[GROUPS];
+                uint16_t *h_out = hs + (size_t)(t + 1) * slab + (size_t)(b + s8) * p.H + hcol;
 #pragma unroll
-                for (int k = 0; k < PAIRS; ++k) {
-                    const int i = k >> 1, e = k & 1, r = 8 * i + e;
-                    const float ai = __uint_as_float(lo[4 * i + e]) + load16<BF16>(&proj[k][0]), af = __uint_as_float(lo[4 * i + 2 + e]) + load16<BF16>(&proj[k][1]);
-                    const float ag = __uint_as_float(hi[4 * i + e]) + load16<BF16>(&proj[k][2]), ao = __uint_as_float(hi[4 * i + 2 + e]) + load16<BF16>(&proj[k][3]);
-                    const float gi = sigmoid_sel<ACCURATE>(pad ? 0.f : ai), gf = sigmoid_sel<ACCURATE>(pad ? 0.f : af);
-                    const float gg = tanh_sel<ACCURATE>(pad ? 0.f : ag), go = sigmoid_sel<ACCURATE>(pad ? 0.f : ao);
-                    c_new[k] = fmaf(gf, c_prev[k], gi * gg);
-                    h16[k] = to16<BF16>(go * tanh_sel<ACCURATE>(c_new[k]));
-                    act[k][0] = to16<BF16>(gi);
-                    act[k][1] = to16<BF16>(gf);
-                    act[k][2] = to16<BF16>(gg);
-                    act[k][3] = to16<BF16>(go);
+                for (int i = 0; i < GROUPS; ++i) {
+                    uint32_t pk[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        auto gate = [&](uint32_t acc, uint32_t pr) {
+                            const uint16_t v = (uint16_t)(e ? pr >> 16 : pr);
+                            return pad ? 0.f : __uint_as_float(acc) + load16<BF16>(&v);
+                        };
+                        const float gi = sigmoid_sel<ACCURATE>(gate(lo[4 * i + e], proj[i][0])), gf = sigmoid_sel<ACCURATE>(gate(lo[4 * i + 2 + e], proj[i][1]));
+                        const float gg = tanh_sel<ACCURATE>(gate(hi[4 * i + e], proj[i][2])), go = sigmoid_sel<ACCURATE>(gate(hi[4 * i + 2 + e], proj[i][3]));
+                        const float cn = fmaf(gf, c[2 * i + e], gi * gg);
+                        c[2 * i + e] = cn;
+                        pk[0] |= (uint32_t)to16<BF16>(gi) << (16 * e);
+                        pk[1] |= (uint32_t)to16<BF16>(gf) << (16 * e);
+                        pk[2] |= (uint32_t)to16<BF16>(gg) << (16 * e);
+                        pk[3] |= (uint32_t)to16<BF16>(go) << (16 * e);
+                        pk[4] |= (uint32_t)to16<BF16>(go * tanh_sel<ACCURATE>(cn)) << (16 * e);
+                    }
+                    h2[i] = movmatrix_trans(pk[4]);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) act[i][g] = pk[g];
                     // h_t first: it is what the other CTAs wait for
-                    if (good && r < rows_left) h_out[(size_t)r * p.H] = h16[k];
+                    if (b + 8 * i + s8 < p.B) *reinterpret_cast<uint32_t *>(h_out + (size_t)(8 * i) * p.H) = h2[i];
                 }
-                if (named_barrier_or(1, kEpilogueThreads, !good)) {
-                    ok = false;
-                    break;
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&hdone[buf]);
+                    // Behind hdone, so that nobody arrives there for the next tile of this buffer before all have for this one.
+                    // Relaxed: it orders the reuse of the accumulator only (a release would wait for the warp's global stores).
+                    mbar_arrive_cluster_relaxed(tempty_c + 8u * buf);
                 }
-                // publish h_t of the tile: after the named barrier thread 0's release is cumulative over every epilogue warp's
-                // stores; the generic->async proxy fence is the consumer's
-                if (tid == 0) red_release_gpu_add(p.counters + ng * NT + n, 1u);
                 // everything nobody waits for: cell state, gate cache, the caller's y
 #pragma unroll
                 for (int k = 0; k < PAIRS; ++k) {
-                    const int r = 8 * (k >> 1) + (k & 1);
-                    if (r >= rows_left) continue;
-                    p.cs[(size_t)(t + 1) * slab + idx0 + (size_t)r * p.H] = c_new[k];
-                    if (y) y[(size_t)t * slab + idx0 + (size_t)r * p.H] = h16[k];
+                    const int r = b + 2 * q + 8 * (k >> 1) + (k & 1);
+                    if (r < p.B) p.cs[(size_t)(t + 1) * slab + (size_t)r * p.H + U] = c[k];
+                }
+                if (NT == 1) {
+#pragma unroll
+                    for (int k = 0; k < PAIRS; ++k) c_next[k] = c[k];
+                }
+#pragma unroll
+                for (int i = 0; i < GROUPS; ++i) {
+                    const int r = b + 8 * i + s8;
                     if (p.store_gates) {
 #pragma unroll
-                        for (int g = 0; g < 4; ++g) grow[(size_t)r * G + g * 16] = act[k][g];
+                        for (int g = 0; g < 4; ++g) act[i][g] = movmatrix_trans(act[i][g]);
+                        quad_transpose(act[i], lane);
+                        if (r < p.B)
+                            *reinterpret_cast<uint4 *>(gates + ((size_t)t * p.B + r) * G + gcol) = make_uint4(act[i][0], act[i][1], act[i][2], act[i][3]);
+                    }
+                    if (y && r < p.B) {
+                        uint16_t *dst = y + (size_t)t * slab + (size_t)r * p.H + hcol;
+                        if (y_words) {
+                            *reinterpret_cast<uint32_t *>(dst) = h2[i];
+                        } else {
+                            dst[0] = (uint16_t)h2[i];
+                            dst[1] = (uint16_t)(h2[i] >> 16);
+                        }
                     }
                 }
             }
@@ -325,7 +381,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     cluster_sync_all();  // the peer's shared and tensor memory stay valid until the leader's last UMMA is consumed
     if (warp == 5) tmem_dealloc_pair(tmem_base, kTmemColumns);
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
-    if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / pl.cta_rows * NT, p.exits);
+    if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / pl.cta_rows * pl.nt, p.exits);
 }
 
 template <int BT, bool BF16, bool ACC>

@@ -104,6 +104,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + 2 * BTH;
+    // (ct is even: a copy of h never mixes tensor- and shared-memory chunks)
     // W_hh into tensor memory by way of the shared memory that the ring will use: lanes l and l + 64 take row l of the tile in the
     // map's order (unit half, gate, unit), 32 columns of two elements per chunk; the warps 0-3 take the even chunks, 6-9 the odd
     // ones.  A wait that expires raises the abort word, on which every role below gives up.
@@ -194,26 +195,43 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                     if (!ok) break;
                     tcgen05_fence_after();
                     const uint32_t d = tmem_base + buf * BTH;
-                    for (int ld = 0; ld < NLOAD; ++ld) {
+                    // copies of tensor-memory chunks, then of shared-memory ones: no decision stands between two instructions
+                    uint32_t da = tmem_a, dw = dw_res, acc = 0;
+                    auto landed = [&]() {
                         ok = mbar_wait(&hfull[stage], phase, abort_w, wait_ns);
-                        if (!ok) break;
-                        tcgen05_fence_after();
-                        const uint32_t dh = dh_ring + (uint32_t)stage * (kStageBytes >> 4);
-#pragma unroll
-                        for (int e = 0; e < kCh; ++e) {
-                            const int c = ld * kCh + e;
-                            if (c < CT) {
-                                const uint32_t da = tmem_a + (uint32_t)c * 32;
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) umma_lo_ts<true>(d, da + 8 * k, dh + e * kStepH + 2 * k, idesc, (uint32_t)(c | k));
-                            } else if (c < KC) {
-                                const uint32_t dw = dw_res + (uint32_t)(c - CT) * kStepW;
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) umma_lo_ss<true>(d, dw + 2 * k, dh + e * kStepH + 2 * k, idesc, (uint32_t)(c | k));
-                            }
-                        }
+                        return dh_ring + (uint32_t)stage * (kStageBytes >> 4);
+                    };
+                    auto consumed = [&]() {
                         umma_commit_pair_both(hempty_l + 8u * (uint32_t)stage);
                         if (++stage == HST) { stage = 0; phase ^= 1; }
+                    };
+                    for (int c = 0; c < CT; c += kCh) {
+                        const uint32_t dh = landed();
+                        if (!ok) break;
+#pragma unroll
+                        for (int e = 0; e < 4 * kCh; ++e)
+                            umma_lo_ts<true>(d, da + 8 * e, dh + (e >> 2) * kStepH + 2 * (e & 3), idesc, e ? 1u : acc);
+                        acc = 1;
+                        da += 32 * kCh;
+                        consumed();
+                    }
+                    int c = CT;
+                    for (; c + kCh <= KC && ok; c += kCh) {
+                        const uint32_t dh = landed();
+                        if (!ok) break;
+#pragma unroll
+                        for (int e = 0; e < 4 * kCh; ++e)
+                            umma_lo_ss<true>(d, dw + (e >> 2) * kStepW + 2 * (e & 3), dh + (e >> 2) * kStepH + 2 * (e & 3), idesc, e ? 1u : acc);
+                        acc = 1;
+                        dw += kCh * kStepW;
+                        consumed();
+                    }
+                    for (; c < KC && ok; c += kCh) {  // an odd last chunk
+                        const uint32_t dh = landed();
+                        if (!ok) break;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) umma_lo_ss<true>(d, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                        consumed();
                     }
                     if (!ok) break;
                     umma_commit_pair_both(tfull_l + 8u * buf);
@@ -427,7 +445,7 @@ int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan) {
     if (pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
     pl.kc = H / 64;
     const int tmem_chunks = (kTmemColumns - pl.BT) / 32;
-    pl.ct = pl.kc < tmem_chunks ? pl.kc : tmem_chunks;
+    pl.ct = (pl.kc < tmem_chunks ? pl.kc : tmem_chunks) / kCh * kCh;
     pl.cs = pl.kc - pl.ct;
     pl.hstages = 16;
     while (pl.hstages > 3 && (size_t)smem_of(pl) > smem_limit) --pl.hstages;

@@ -36,7 +36,9 @@ constexpr int kEpilogueThreads = 256;
 constexpr int kStepBytesW = 2 * 64 * 128;  // one chunk-step of A: two blocks of 64 K rows x 64 units
 constexpr int kTmemColumns = 512;
 constexpr int kBarrierBytes = 1024, kMinSmemBytes = 120 * 1024;
-constexpr int kFillSlots = (kMinSmemBytes - 1024 - kBarrierBytes) / kStepBytesW;
+// Even: a slot always belongs to the same set of warps.  A set that met a slot only every other time could find its first phase
+// still open, whose parity reads as that of the phase it waits for.
+constexpr int kFillSlots = (kMinSmemBytes - 1024 - kBarrierBytes) / kStepBytesW / 2 * 2;
 constexpr int KS = 4, UPO = 64 / KS;
 
 struct Layout {

@@ -43,7 +43,9 @@ constexpr int kEpilogueThreads = 256;
 constexpr int kStepBytesW = 128 * 128;  // one chunk-step of A: 128 rows x 64 16-bit elements
 constexpr int kTmemColumns = 512;
 constexpr int kBarrierBytes = 1024, kMinSmemBytes = 120 * 1024;
-constexpr int kFillSlots = (kMinSmemBytes - 1024 - kBarrierBytes) / kStepBytesW;
+// Even: a slot always belongs to the same set of warps.  A set that met a slot only every other time could find its first phase
+// still open, whose parity reads as that of the phase it waits for.
+constexpr int kFillSlots = (kMinSmemBytes - 1024 - kBarrierBytes) / kStepBytesW / 2 * 2;
 constexpr int WCH = kFwdTmGroup;
 
 struct Layout {

@@ -12,7 +12,7 @@
 //   producer warp : waits for the tile's step barrier, streams h_{t-1} through the ring (copies of two 64-wide chunks)
 //   UMMA thread   : M = 128, N = BT, accumulating over K = H into one of two accumulators (BT / 2 columns: sequences [0, BT/2) in
 //                   lanes 0-63, the others in lanes 64-127)
-//   8 warps       : the rows of A are ordered so that a lane quadrant holds the four gates of 8 units, 8 lanes each: two
+//   16 warps      : the rows of A are ordered so that a lane quadrant holds the four gates of 8 units, 8 lanes each: two
 //                   tcgen05.ld of the 16x256b shape leave all four gate sums of a (unit, sequence) pair in one thread, and no
 //                   exchange through shared memory is needed.  Projections and cell states are read a tile ahead; h_t is stored
 //                   first, cell states, gates and y follow while a thread of its own publishes h_t.
@@ -35,13 +35,14 @@ namespace tc {
 
 namespace {
 
-constexpr int kThreads = 352;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA issuer, 10 publisher of h
-constexpr int kEpilogueWarps = 8;
+// 16 epilogue warps: with 8 a tile of 128 sequences took them 5.3 k cycles of instruction latencies, more than its UMMAs
+constexpr int kEpilogueWarps = 16, kProducerWarp = 16, kUmmaWarp = 17, kPublisherWarp = 18;
+constexpr int kThreads = (kEpilogueWarps + 3) * 32;
 constexpr int kChunkBytesW = 64 * 128;  // 64 rows x 64 16-bit elements
 constexpr int kTmemColumns = 512;
 constexpr int kCh = 2;  // chunks per copy of h
 constexpr int kBarrierBytes = 1024, kMinSmemBytes = 120 * 1024;
-constexpr int kFillSlots = 14;
+constexpr int kFillSlots = 12;  // a multiple of 4: a slot always belongs to the same set of warps (see tc_lstm_fwd_tm.cu)
 static_assert(kBarrierBytes + kFillSlots * kChunkBytesW + 1024 <= kMinSmemBytes, "the fill slots fit every launch");
 
 __host__ __device__ inline int smem_of(const FwdWidePlan &pl) {
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_h,
                      const __grid_constant__ FwdWidePlan pl, FwdParams p) {
     constexpr int BTH = BT / 2;        // B rows a CTA stages, columns of an accumulator
-    constexpr int WC = BTH / 2;        // columns a warp finishes
+    constexpr int WC = BTH / 4;        // columns a warp finishes
     constexpr int GROUPS = WC / 8;     // of 8 columns
     constexpr int PAIRS = 2 * GROUPS;  // (unit, sequence) pairs per thread
     constexpr int kStageBytes = kCh * BTH * 128;
@@ -96,7 +97,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         tma_prefetch_desc(&tm_w);
         tma_prefetch_desc(&tm_h);
     }
-    if (warp == 5) {
+    if (warp == kUmmaWarp) {
         tmem_alloc_pair(tmem_slot, kTmemColumns);
         tmem_relinquish_pair();
     }
@@ -106,19 +107,19 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + 2 * BTH;
     // (ct is even: a copy of h never mixes tensor- and shared-memory chunks)
     // W_hh into tensor memory by way of the shared memory that the ring will use: lanes l and l + 64 take row l of the tile in the
-    // map's order (unit half, gate, unit), 32 columns of two elements per chunk; the warps 0-3 take the even chunks, 6-9 the odd
-    // ones.  A wait that expires raises the abort word, on which every role below gives up.
-    if (warp == 4 && elect_one()) {
+    // map's order (unit half, gate, unit), 32 columns of two elements per chunk; a warp reaches the lane quadrant warp % 4
+    // and takes every fourth chunk.  A wait that expires raises the abort word, on which every role below gives up.
+    if (warp == kProducerWarp && elect_one()) {
         for (int c = 0; c < CT; ++c) {
             const int slot = c % kFillSlots;
             if (c >= kFillSlots && !mbar_wait(&fempty[slot], (uint32_t)(c / kFillSlots - 1) & 1u, abort_w, wait_ns)) break;
             mbar_expect_tx(&ffull[slot], kChunkBytesW);
             tma_load_5d(s_w + slot * kChunkBytesW, &tm_w, c * 64, 0, 0, 0, jr, &ffull[slot]);
         }
-    } else if (warp != 4 && warp != 5 && warp != 10) {
+    } else if (warp < kEpilogueWarps) {
         const int quad = warp & 3, row = (quad & 1) * 32 + lane;
         const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
-        for (int c = warp < 4 ? 0 : 1; c < CT; c += 2) {
+        for (int c = warp >> 2; c < CT; c += 4) {
             const int slot = c % kFillSlots;
             if (!__all_sync(0xffffffffu, mbar_wait(&ffull[slot], (uint32_t)(c / kFillSlots) & 1u, abort_w, wait_ns))) break;
             const uint8_t *src = s_w + slot * kChunkBytesW + row * 128;
@@ -142,7 +143,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     const uint32_t hfull_c = map_to_rank(smem_u32(hfull), 0), wbar_c = map_to_rank(smem_u32(wbar), 0);
     const uint32_t tempty_c = map_to_rank(smem_u32(tempty), 0);
 
-    if (warp == 4) {
+    if (warp == kProducerWarp) {
         // ------------------------------------------------------------ producer
         if (elect_one()) {
             bool ok = true;
@@ -178,7 +179,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             for (int i = 0; i < HST && leader; ++i)
                 if (issued >> i & 1u) mbar_drain(&hfull[i], parity >> i & 1u, ok ? wait_ns : kAbortDrainNs);
         }
-    } else if (warp == 5) {
+    } else if (warp == kUmmaWarp) {
         // ------------------------------------------------------------ UMMA issuer (the leader's)
         if (leader && elect_one()) {
             bool ok = CS == 0 || mbar_wait(wbar, 0, abort_w, wait_ns);
@@ -240,7 +241,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
             if (wi > 0) mbar_drain(&tfull[(wi - 1) & 1], (wi - 1) >> 1 & 1u, wait_ns);
         }
-    } else if (warp == 10) {
+    } else if (warp == kPublisherWarp) {
         // ------------------------------------------------------------ publisher
         // The release takes about a thousand cycles (it waits for the stores it covers); on a thread of its own the epilogue goes
         // on meanwhile.  hdone orders it behind every epilogue warp's stores of h; the generic->async proxy fence is the consumer's.
@@ -254,7 +255,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                 }
         }
     } else {
-        // ------------------------------------------------------------ epilogue (8 warps, each on its own)
+        // ------------------------------------------------------------ epilogue (16 warps, each on its own)
         // Quadrant q of the lanes: unit half q & 1, sequences (q >> 1) BT / 2 of the tile, of which this warp takes WC columns, 8
         // at a time.  An accumulator fragment is (unit lane / 4, sequences 2 (lane % 4) and + 1); 16-bit data move as (sequence
         // lane / 4, 8 units of gate lane % 4: 16 bytes) and (sequence lane / 4, units 2 (lane % 4) and + 1 of h: 4 bytes), between
@@ -262,8 +263,8 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         // tile of 128 sequences, four times the UMMAs.
         const int quad = warp & 3, half = quad & 1, q = lane & 3, s8 = lane >> 2;
         const int U = jr * 16 + half * 8 + s8;                           // unit of this thread's fragments
-        const int col0 = (quad >> 1) * BTH + (warp < 4 ? 0 : WC);        // first sequence of the warp within a tile
-        const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (warp < 4 ? 0 : WC);
+        const int col0 = (quad >> 1) * BTH + (warp >> 2) * WC;           // first sequence of the warp within a tile
+        const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16) + (warp >> 2) * WC;
         const size_t slab = (size_t)p.B * p.H, G = (size_t)4 * p.H;
         const bool pad = ACCURATE && U >= p.real_units;
         uint16_t *hs = static_cast<uint16_t *>(p.hs);
@@ -397,7 +398,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         while (global_timer_ns() - t0 < kAbortDrainNs) {}
     }
     cluster_sync_all();  // the peer's shared and tensor memory stay valid until the leader's last UMMA is consumed
-    if (warp == 5) tmem_dealloc_pair(tmem_base, kTmemColumns);
+    if (warp == kUmmaWarp) tmem_dealloc_pair(tmem_base, kTmemColumns);
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / pl.cta_rows * pl.nt, p.exits);
 }

@@ -158,6 +158,7 @@ struct BwdTmPlan {
     int BT;        // sequences per batch group
     int jt;        // unit tiles = H / 64, a cluster of four CTAs each
     int ngroups;
+    int nt;        // batch tiles that a cluster takes in turn
     int kp;        // chunk-steps of 64 per half of a CTA's K range
     int left;      // 1: the range has an odd number of chunks, the last one runs by itself
     int ct, cs;    // chunk-steps of W_hh in tensor / shared memory (all of them)

@@ -31,7 +31,7 @@ namespace tc {
 
 namespace {
 
-constexpr int kThreads = 320;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA issuer
+constexpr int kThreads = 352;  // warps 0-3 and 6-9 epilogue, 4 producer, 5 UMMA issuer, 10 publisher of dG
 constexpr int kEpilogueThreads = 256;
 constexpr int kStepBytesW = 2 * 64 * 128;  // one chunk-step of A: two blocks of 64 K rows x 64 units
 constexpr int kTmemColumns = 512;
@@ -72,17 +72,19 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     uint8_t *s_w = smem + kBarrierBytes, *s_lw = s_w + L.w, *s_ring = s_lw + L.left_w, *s_left = s_ring + L.ring;
     float *s_ps = reinterpret_cast<float *>(s_left + L.left), *s_red = s_ps + L.ps / 4;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + ST;
-    uint64_t *lfull = empty + ST, *tfull = lfull + 1, *tempty = tfull + 1, *wbar = tempty + 1;
+    uint64_t *lfull = empty + ST, *lempty = lfull + 1, *tfull = lempty + 1, *tempty = tfull + 1, *wbar = tempty + 1;
     uint64_t *rbar = wbar + 1;  // [2] partial sums received
-    uint64_t *ffull = rbar + 2, *fempty = ffull + kFillSlots;  // while W_hh moves into tensor memory
+    uint64_t *gdone = rbar + 2, *pdone = gdone + 2;  // [2] dG stored by every warp / seen by the publisher
+    uint64_t *ffull = pdone + 2, *fempty = ffull + kFillSlots;  // while W_hh moves into tensor memory
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fempty + kFillSlots);
     volatile uint32_t *abort_w = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kq = (int)cluster_ctarank();
     const int cl = blockIdx.x / KS, ng = cl / pl.jt, j = cl % pl.jt;  // batch group, unit tile [64j, 64j+64)
-    const int b0 = ng * BT;
-    unsigned int *counter = p.counters + ng;
+    const int tile0 = ng * pl.nt, tiles = (p.B + BT - 1) / BT;
+    const int NT = tiles - tile0 < pl.nt ? tiles - tile0 : pl.nt;  // batch tiles of this group, taken in turn
+    unsigned int *counters = p.counters + tile0;
     const int kcq = 2 * KP + pl.left, c_first = kq * kcq;  // 64-wide K chunks of this CTA
     const CUtensorMap *tm_dg = &maps.half[kq];
 
@@ -92,11 +94,15 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             mbar_init(&empty[i], 1);
         }
         mbar_init(lfull, 1);
+        mbar_init(lempty, 1);
         mbar_init(tfull, 1);
         mbar_init(tempty, kEpilogueThreads / 32);
         mbar_init(wbar, 1);
-        mbar_init(&rbar[0], 1);
-        mbar_init(&rbar[1], 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&rbar[i], 1);
+            mbar_init(&gdone[i], kEpilogueThreads / 32);
+            mbar_init(&pdone[i], 1);
+        }
         for (int i = 0; i < kFillSlots; ++i) {
             mbar_init(&ffull[i], 1);
             mbar_init(&fempty[i], 4);
@@ -127,7 +133,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             for (int h = 0; h < 2; ++h)
                 tma_load_2d(s_w + slot * kStepBytesW + h * 8192, &tm_w, j * 64, (c_first + h * KP + c) * 64, &ffull[slot]);
         }
-    } else if (warp < 4 || warp > 5) {
+    } else if (warp != 4 && warp != 5 && warp != 10) {
         const int quad = warp & 3, l = quad * 32 + lane, un = l & 63;
         const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
         for (int c = warp < 4 ? 0 : 1; c < CT; c += 2) {
@@ -175,32 +181,36 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             uint32_t phase = 0, lphase = 0;
             uint32_t issued = 0, parity = 0;
             bool left_issued = false;
-            for (int s = s_first; s < p.s1 && ok; ++s) {
-                const int t_src = p.T - s;
-                if (s > p.s0)
-                    ok = wait_counter(counter, (unsigned)(pl.jt * KS) * (unsigned)(s - p.s0) + p.extra_arrivals, p.err, abort_w, 3u, wait_ns);
-                if (!ok) break;
-                fence_proxy_async_global();
-                FLSTM_STAMP(s - p.s0, 0);
-                for (int ld = 0; ld < NLOAD; ++ld) {
-                    // (without a ring the tile is free: the step barrier came after the UMMAs that read it)
-                    if (pl.ring) ok = mbar_wait(&empty[stage], phase ^ 1, abort_w, wait_ns);
+            for (int s = s_first; s < p.s1 && ok; ++s)
+                for (int n = 0; n < NT && ok; ++n) {
+                    const int t_src = p.T - s, b0 = (tile0 + n) * BT;
+                    if (s > p.s0)
+                        ok = wait_counter(counters + n, (unsigned)(pl.jt * KS) * (unsigned)(s - p.s0) + p.extra_arrivals, p.err, abort_w, 3u,
+                                          wait_ns);
                     if (!ok) break;
-                    mbar_expect_tx(&full[stage], (uint32_t)stage_bytes);
-                    issued |= 1u << stage;
-                    parity = (parity & ~(1u << stage)) | (phase << stage);
-                    // (x, row, K half, chunk of the half, step); chunks beyond the half come as zeros (and are counted)
-                    tma_load_5d(s_ring + stage * stage_bytes, tm_dg, 0, b0, 0, ld * CH, t_src, &full[stage]);
-                    if (++stage == ST) { stage = 0; phase ^= 1; }
+                    fence_proxy_async_global();
+                    if (n == 0) FLSTM_STAMP(s - p.s0, 0);
+                    for (int ld = 0; ld < NLOAD; ++ld) {
+                        // (without a ring the tile is free: the step barrier came after the UMMAs that read it)
+                        if (pl.ring) ok = mbar_wait(&empty[stage], phase ^ 1, abort_w, wait_ns);
+                        if (!ok) break;
+                        mbar_expect_tx(&full[stage], (uint32_t)stage_bytes);
+                        issued |= 1u << stage;
+                        parity = (parity & ~(1u << stage)) | (phase << stage);
+                        // (x, row, K half, chunk of the half, step); chunks beyond the half come as zeros (and are counted)
+                        tma_load_5d(s_ring + stage * stage_bytes, tm_dg, 0, b0, 0, ld * CH, t_src, &full[stage]);
+                        if (++stage == ST) { stage = 0; phase ^= 1; }
+                    }
+                    if (ok && pl.left) {
+                        if (pl.ring) ok = mbar_wait(lempty, lphase ^ 1, abort_w, wait_ns);
+                        if (!ok) break;
+                        mbar_expect_tx(lfull, BT * 128);
+                        tma_load_4d(s_left, &maps.chunk, 0, b0, c_first + 2 * KP, t_src, lfull);
+                        left_issued = true;
+                        lphase ^= 1;
+                    }
+                    if (n == 0) FLSTM_STAMP(s - p.s0, 1);
                 }
-                if (ok && pl.left) {
-                    mbar_expect_tx(lfull, BT * 128);
-                    tma_load_4d(s_left, &maps.chunk, 0, b0, c_first + 2 * KP, t_src, lfull);
-                    left_issued = true;
-                    lphase ^= 1;
-                }
-                FLSTM_STAMP(s - p.s0, 1);
-            }
             // way out (normal or aborted): every copy this thread started must have landed before the CTA exits
             if (CS > 0 || pl.left) mbar_drain(wbar, 0, wait_ns);
             for (int i = 0; i < ST; ++i)
@@ -218,10 +228,11 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         constexpr uint32_t kStepG = (N * 128) >> 4, kStepW = kStepBytesW >> 4;  // descriptor units
         const uint32_t dw_res = umma_desc_lo(smem_u32(s_w), 8192), dw_left = umma_desc_lo(smem_u32(s_lw), 8192);
         const uint32_t dd_ring = umma_desc_lo(smem_u32(s_ring)), dd_left = umma_desc_lo(smem_u32(s_left));
-        const uint32_t empty_l = smem_u32(empty), tfull_l = smem_u32(tfull);
+        const uint32_t empty_l = smem_u32(empty), lempty_l = smem_u32(lempty), tfull_l = smem_u32(tfull);
         int committed = 0;
-        for (int s = s_first; s < p.s1 && ok; ++s) {
-            const uint32_t wi = (uint32_t)(s - s_first);
+        const uint32_t items = (uint32_t)(p.s1 - s_first) * (uint32_t)NT;
+        for (uint32_t wi = 0; wi < items && ok; ++wi) {
+            const int s = s_first + (int)(wi / (uint32_t)NT);
             ok = mbar_wait(tempty, (wi & 1) ^ 1, abort_w, wait_ns);
             if (!ok) break;
             tcgen05_fence_after();
@@ -264,6 +275,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 tcgen05_fence_after();
 #pragma unroll
                 for (int k = 0; k < 4; ++k) umma_lo_ss<false>(tmem_base, dw_left + 128 * k, dd_left + 2 * k, idesc_left, 1u);
+                if (pl.ring) umma_commit_addr(lempty_l);
             }
             umma_commit_addr(tfull_l);
             ++committed;
@@ -271,6 +283,22 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         }
         // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
         if (committed > 0) mbar_drain(tfull, (uint32_t)(committed - 1) & 1u, wait_ns);
+        }
+    } else if (warp == 10) {
+        // ------------------------------------------------------------ publisher
+        // The release takes about a thousand cycles (it waits for the stores it covers), which the epilogue need not spend.  The
+        // generic->async proxy fence is the consumer's.
+        if (elect_one()) {
+            uint32_t gi = 0;
+            bool ok = true;
+            for (int s = p.s0; s < p.s1 && s < p.T && ok; ++s)
+                for (int n = 0; n < NT; ++n, ++gi) {
+                    ok = mbar_wait(&gdone[gi & 1], (gi >> 1) & 1, abort_w, wait_ns);
+                    if (!ok) break;
+                    mbar_arrive(&pdone[gi & 1]);
+                    red_release_gpu_add(counters + n, 1u);
+                    if (n == 0) FLSTM_STAMP(s - p.s0, 8);
+                }
         }
     } else {
         // ------------------------------------------------------------ epilogue (256 threads)
@@ -286,135 +314,152 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const int quad = warp & 3, col0 = warp < 4 ? 0 : BT / 2;  // lane quadrant, half of the columns
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (quad >> 1) * BT + col0;
         const uint32_t red_local = smem_u32(s_red), rbar_local = smem_u32(rbar);
-        float dc_keep[PAIRS];
+        // what the pointwise update of a tile reads, fetched a tile ahead
+        struct Inputs {
+            uint16_t gi, gf, gg, go, dy;
+            float ct, cp, dc;
+        };
+        Inputs next[PAIRS];
+        auto fetch = [&](int s, int n) {
+            const int t = p.T - 1 - s;
 #pragma unroll
-        for (int i = 0; i < PAIRS; ++i) {
-            const int b = b0 + nb + 16 * i;
-            const size_t idx = (size_t)b * p.H + U;
-            dc_keep[i] = b >= p.B ? 0.f : p.s0 > 0 ? p.dc[idx] : dcn ? load16<BF16>(dcn + idx) : 0.f;
-        }
+            for (int i = 0; i < PAIRS; ++i) {
+                const int b = (tile0 + n) * BT + nb + 16 * i;
+                const size_t idx = (size_t)b * p.H + U;
+                next[i].gi = next[i].gf = next[i].gg = next[i].go = next[i].dy = 0;
+                next[i].ct = next[i].cp = 0.f;
+                if (s == p.s0 || NT > 1) next[i].dc = b >= p.B ? 0.f : s > 0 ? p.dc[idx] : dcn ? load16<BF16>(dcn + idx) : 0.f;
+                if (b < p.B && t >= 0) {
+                    const uint16_t *grow = gates + ((size_t)t * p.B + b) * G + (size_t)(U >> 4) * 64 + (U & 15);
+                    next[i].gi = grow[0];
+                    next[i].gf = grow[16];
+                    next[i].gg = grow[32];
+                    next[i].go = grow[48];
+                    next[i].ct = p.cs[(size_t)(t + 1) * slab + idx];
+                    next[i].cp = p.cs[(size_t)t * slab + idx];
+                    next[i].dy = dy[(size_t)t * slab + idx];
+                }
+            }
+        };
+        fetch(p.s0, 0);
+        uint32_t wi = 0, gi = 0;  // tiles contracted, tiles published
         bool ok = true;
         for (int s = p.s0; s < p.s1 && ok; ++s) {
             const int t = p.T - 1 - s;  // time step whose dG is produced (t = -1: only dh0 / dc0)
-            // dG and the carried dc are linear in dh and dc: everything else is formed ahead of the wait
-            struct Factors {
-                float dy, ka, ki, kf, kg, ko, gf;
-            };
-            Factors fac[PAIRS];
+            for (int n = 0; n < NT; ++n) {
+                const int b0 = (tile0 + n) * BT;
+                // dG and the carried dc are linear in dh and dc: everything else is formed ahead of the wait
+                struct Factors {
+                    float dy, ka, ki, kf, kg, ko, gf, dc;
+                };
+                Factors fac[PAIRS];
 #pragma unroll
-            for (int i = 0; i < PAIRS; ++i) {
-                const int b = b0 + nb + 16 * i;
-                fac[i] = Factors{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (b < p.B && t >= 0) {
-                    const uint16_t *grow = gates + ((size_t)t * p.B + b) * G + (size_t)(U >> 4) * 64 + (U & 15);
-                    const size_t idx = (size_t)b * p.H + U;
-                    const float gi = load16<BF16>(grow), gf = load16<BF16>(grow + 16), gg = load16<BF16>(grow + 32), go = load16<BF16>(grow + 48);
-                    const float tc = tanh_sel<ACCURATE>(p.cs[(size_t)(t + 1) * slab + idx]), cp = p.cs[(size_t)t * slab + idx];
-                    fac[i] = Factors{load16<BF16>(dy + (size_t)t * slab + idx), go * (1.f - tc * tc), gg * gi * (1.f - gi),
-                                     cp * gf * (1.f - gf), gi * (1.f - gg * gg), tc * go * (1.f - go), gf};
+                for (int i = 0; i < PAIRS; ++i) {
+                    const Inputs &v = next[i];
+                    const float g0 = load16<BF16>(&v.gi), g1 = load16<BF16>(&v.gf), g2 = load16<BF16>(&v.gg), g3 = load16<BF16>(&v.go);
+                    const float tc = tanh_sel<ACCURATE>(v.ct);
+                    fac[i] = Factors{load16<BF16>(&v.dy), g3 * (1.f - tc * tc), g2 * g0 * (1.f - g0), v.cp * g1 * (1.f - g1),
+                                     g0 * (1.f - g2 * g2), tc * g3 * (1.f - g3), g1, v.dc};
                 }
-            }
-            // dh contribution from the step above: reduce-scattered partial products
-            float dh_in[PAIRS];
-            if (s == 0) {
+                const int n_next = n + 1 == NT ? 0 : n + 1, s_next = n + 1 == NT ? s + 1 : s;
+                if (s_next < p.s1) fetch(s_next, n_next);
+                // dh contribution from the step above: reduce-scattered partial products
+                float dh_in[PAIRS];
+                if (s == 0) {
+#pragma unroll
+                    for (int i = 0; i < PAIRS; ++i) {
+                        const int b = b0 + nb + 16 * i;
+                        dh_in[i] = (dhn && b < p.B) ? load16<BF16>(dhn + (size_t)b * p.H + U) : 0.f;
+                    }
+                } else {
+                    const int rb = wi & 1;
+                    // No thread leaves between here and the second named barrier below, whatever its waits return: the barriers
+                    // OR the failures, so that all 256 threads go on or give up together.
+                    bool good = __all_sync(0xffffffffu, mbar_wait(tfull, wi & 1, abort_w, wait_ns));
+                    if (tid == 0 && n == 0) FLSTM_STAMP(s - p.s0, 5);
+                    tcgen05_fence_after();
+                    if (good) {
+                        uint32_t acc[BT / 2];
+                        if (BT == 32) tmem_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(&acc[0]));
+                        else tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&acc[0]));
+                        tmem_ld_wait();
+                        float4 *dst = reinterpret_cast<float4 *>(s_ps + (quad * 32 + lane) * RS + col0);
+#pragma unroll
+                        for (int i = 0; i < BT / 8; ++i)
+                            dst[i] = make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]),
+                                                 __uint_as_float(acc[4 * i + 2]), __uint_as_float(acc[4 * i + 3]));
+                    }
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty);
+                    const bool failed = named_barrier_or(1, kEpilogueThreads, !good);
+                    if (!failed) {
+                        // UPO rows of BT sums for this CTA arrive from every CTA of the cluster, its own included
+                        if (tid == 0) mbar_expect_tx(&rbar[rb], (uint32_t)(KS * UPO * BT * 4));
+                        constexpr int V = BT / 4;  // 16-byte pieces of a row
+#pragma unroll
+                        for (int i = 0; i < 64 * V / kEpilogueThreads; ++i) {
+                            const int e = tid + i * kEpilogueThreads, row = e / V, v = e % V;
+                            const float4 a = *reinterpret_cast<const float4 *>(s_ps + row * RS + 4 * v);
+                            const float4 b = *reinterpret_cast<const float4 *>(s_ps + (64 + row) * RS + 4 * v);
+                            const uint32_t owner = row / UPO, off = (uint32_t)(((rb * KS + kq) * UPO + row % UPO) * RS + 4 * v) * 4u;
+                            st_async_v4(map_to_rank(red_local + off, owner), __float_as_uint(a.x + b.x), __float_as_uint(a.y + b.y),
+                                        __float_as_uint(a.z + b.z), __float_as_uint(a.w + b.w), map_to_rank(rbar_local + rb * 8, owner));
+                        }
+                        if (tid == 0 && n == 0) FLSTM_STAMP(s - p.s0, 9);
+                        good = mbar_wait_cluster(&rbar[rb], (wi >> 1) & 1, abort_w, wait_ns);
+                    } else {
+                        good = false;
+                    }
+                    if (tid == 0 && n == 0) FLSTM_STAMP(s - p.s0, 10);
+                    const float *red = s_red + (size_t)rb * KS * UPO * RS;
+#pragma unroll
+                    for (int i = 0; i < PAIRS; ++i) {
+                        float acc = 0.f;
+#pragma unroll
+                        for (int src = 0; src < KS; ++src) acc += red[(src * UPO + u16) * RS + nb + 16 * i];
+                        dh_in[i] = acc;
+                    }
+                    // one warp's failure is everybody's
+                    if (named_barrier_or(1, kEpilogueThreads, !good)) {
+                        ok = false;
+                        break;
+                    }
+                    if (tid == 0 && n == 0) FLSTM_STAMP(s - p.s0, 6);
+                    ++wi;
+                }
+                // fused pointwise backward for the owned (unit, sequence) pairs
 #pragma unroll
                 for (int i = 0; i < PAIRS; ++i) {
                     const int b = b0 + nb + 16 * i;
-                    dh_in[i] = (dhn && b < p.B) ? load16<BF16>(dhn + (size_t)b * p.H + U) : 0.f;
-                }
-            } else {
-                const uint32_t wi = (uint32_t)(s - s_first);
-                const int rb = wi & 1;
-                // No thread leaves between here and the second named barrier below, whatever its waits return: the barriers
-                // OR the failures, so that all 256 threads go on or give up together.
-                bool good = __all_sync(0xffffffffu, mbar_wait(tfull, wi & 1, abort_w, wait_ns));
-                if (tid == 0) FLSTM_STAMP(s - p.s0, 5);
-                tcgen05_fence_after();
-                if (good) {
-                    uint32_t acc[BT / 2];
-                    if (BT == 32) tmem_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(&acc[0]));
-                    else tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&acc[0]));
-                    tmem_ld_wait();
-                    float4 *dst = reinterpret_cast<float4 *>(s_ps + (quad * 32 + lane) * RS + col0);
-#pragma unroll
-                    for (int i = 0; i < BT / 8; ++i)
-                        dst[i] = make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]),
-                                             __uint_as_float(acc[4 * i + 2]), __uint_as_float(acc[4 * i + 3]));
-                }
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(tempty);
-                const bool failed = named_barrier_or(1, kEpilogueThreads, !good);
-                if (!failed) {
-                    // UPO rows of BT sums for this CTA arrive from every CTA of the cluster, its own included
-                    if (tid == 0) mbar_expect_tx(&rbar[rb], (uint32_t)(KS * UPO * BT * 4));
-                    constexpr int V = BT / 4;  // 16-byte pieces of a row
-#pragma unroll
-                    for (int i = 0; i < 64 * V / kEpilogueThreads; ++i) {
-                        const int e = tid + i * kEpilogueThreads, row = e / V, v = e % V;
-                        const float4 a = *reinterpret_cast<const float4 *>(s_ps + row * RS + 4 * v);
-                        const float4 b = *reinterpret_cast<const float4 *>(s_ps + (64 + row) * RS + 4 * v);
-                        const uint32_t owner = row / UPO, off = (uint32_t)(((rb * KS + kq) * UPO + row % UPO) * RS + 4 * v) * 4u;
-                        st_async_v4(map_to_rank(red_local + off, owner), __float_as_uint(a.x + b.x), __float_as_uint(a.y + b.y),
-                                    __float_as_uint(a.z + b.z), __float_as_uint(a.w + b.w), map_to_rank(rbar_local + rb * 8, owner));
+                    if (b >= p.B) continue;
+                    const size_t idx = (size_t)b * p.H + U;
+                    const Factors &f = fac[i];
+                    if (t < 0) {
+                        if (p.dh0) p.dh0[idx] = dh_in[i];
+                        if (p.dc0) p.dc0[idx] = f.dc;
+                        continue;
                     }
-                    if (tid == 0) FLSTM_STAMP(s - p.s0, 9);
-                    good = mbar_wait_cluster(&rbar[rb], (wi >> 1) & 1, abort_w, wait_ns);
-                } else {
-                    good = false;
+                    const float dh = ACCURATE && U >= p.real_units ? 0.f : f.dy + dh_in[i];
+                    const float dcv = fmaf(dh, f.ka, f.dc), dc_out = dcv * f.gf;
+                    uint16_t *drow = dg + ((size_t)t * p.B + b) * G + (size_t)(U >> 4) * 64 + (U & 15);
+                    drow[0] = to16<BF16>(dcv * f.ki);
+                    drow[16] = to16<BF16>(dcv * f.kf);
+                    drow[32] = to16<BF16>(dcv * f.kg);
+                    drow[48] = to16<BF16>(dh * f.ko);
+                    // the carry of a lone tile stays in its thread; a later launch looks for it in memory
+                    if (NT == 1) next[i].dc = dc_out;
+                    if (NT > 1 || s + 1 == p.s1) p.dc[idx] = dc_out;
                 }
-                if (tid == 0) FLSTM_STAMP(s - p.s0, 10);
-                const float *red = s_red + (size_t)rb * KS * UPO * RS;
-#pragma unroll
-                for (int i = 0; i < PAIRS; ++i) {
-                    float acc = 0.f;
-#pragma unroll
-                    for (int src = 0; src < KS; ++src) acc += red[(src * UPO + u16) * RS + nb + 16 * i];
-                    dh_in[i] = acc;
+                if (t >= 0) {
+                    if (tid == 0 && n == 0) FLSTM_STAMP(s - p.s0, 7);
+                    // publish dG_t: ONE arrival per CTA by a thread of its own, behind every warp's stores; no third tile may use
+                    // a gdone barrier before the publisher has seen this phase of it
+                    const bool seen = gi < 2 || mbar_wait(&pdone[gi & 1], ((gi >> 1) - 1) & 1, abort_w, wait_ns);
+                    __syncwarp();
+                    if (lane == 0 && seen) mbar_arrive(&gdone[gi & 1]);
+                    ++gi;
                 }
-                // one warp's failure is everybody's
-                if (named_barrier_or(1, kEpilogueThreads, !good)) {
-                    ok = false;
-                    break;
-                }
-                if (tid == 0) FLSTM_STAMP(s - p.s0, 6);
-            }
-            // fused pointwise backward for the owned (unit, sequence) pairs
-#pragma unroll
-            for (int i = 0; i < PAIRS; ++i) {
-                const int b = b0 + nb + 16 * i;
-                if (b >= p.B) continue;
-                const size_t idx = (size_t)b * p.H + U;
-                if (t < 0) {
-                    if (p.dh0) p.dh0[idx] = dh_in[i];
-                    if (p.dc0) p.dc0[idx] = dc_keep[i];
-                    continue;
-                }
-                const Factors &f = fac[i];
-                const float dh = ACCURATE && U >= p.real_units ? 0.f : f.dy + dh_in[i];
-                const float dcv = fmaf(dh, f.ka, dc_keep[i]);
-                dc_keep[i] = dcv * f.gf;
-                uint16_t *drow = dg + ((size_t)t * p.B + b) * G + (size_t)(U >> 4) * 64 + (U & 15);
-                drow[0] = to16<BF16>(dcv * f.ki);
-                drow[16] = to16<BF16>(dcv * f.kf);
-                drow[32] = to16<BF16>(dcv * f.kg);
-                drow[48] = to16<BF16>(dh * f.ko);
-            }
-            if (t >= 0) {
-                if (tid == 0) FLSTM_STAMP(s - p.s0, 7);
-                // publish dG_t: ONE arrival per CTA; after the named barrier thread 0's release is cumulative over every
-                // epilogue warp's stores, the generic->async proxy fence is the consumer's
-                named_barrier_sync(2, kEpilogueThreads);
-                if (tid == 0) red_release_gpu_add(counter, 1u);
-                if (tid == 0) FLSTM_STAMP(s - p.s0, 8);
-            }
-        }
-        // a later launch continues the recurrence: leave the cell-gradient carry where it will look for it
-        if (ok && p.s1 <= p.T) {
-#pragma unroll
-            for (int i = 0; i < PAIRS; ++i) {
-                const int b = b0 + nb + 16 * i;
-                if (b < p.B) p.dc[(size_t)b * p.H + U] = dc_keep[i];
             }
         }
     }
@@ -430,7 +475,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
     if (warp == 5) tmem_dealloc(tmem_base, kTmemColumns);
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
-    if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / (pl.jt * KS), p.exits);
+    if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / (pl.jt * KS) * pl.nt, p.exits);
 }
 
 void cluster_attr(cudaLaunchAttribute *a) {
@@ -498,11 +543,16 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
     BwdTmPlan pl{};
     pl.jt = H / 64;
     if (pl.jt * KS > sms) return FLSTM_OK;
+    // one tile of 32 sequences per group, of 64, or several of 64 in turn: the tiles are independent recurrences with a step
+    // barrier each, so the chain of one hides behind the others' contractions
     const int groups = sms / (pl.jt * KS);
-    for (int bt = 32; bt <= (H > 1024 ? 64 : 32) && !pl.BT; bt *= 2)
-        if ((B + bt - 1) / bt <= groups) pl.BT = bt;
-    if (!pl.BT) return FLSTM_OK;
-    pl.ngroups = (B + pl.BT - 1) / pl.BT;
+    pl.BT = B <= 32 * groups ? 32 : 64;
+    const int tiles = (B + pl.BT - 1) / pl.BT;
+    pl.nt = (tiles + groups - 1) / groups;
+    pl.ngroups = (tiles + pl.nt - 1) / pl.nt;
+    if (pl.BT == 64 && pl.nt == 1 && H <= 1024) return FLSTM_OK;  // a chain that stands alone: the other kernels are as fast
+    if (const char *e = std::getenv("FLSTM_BNT")) if (pl.nt > std::atoi(e)) return FLSTM_OK;
+    if (pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
     const int kcq = H / 16 / KS;
     pl.kp = kcq / 2;
     pl.left = kcq % 2;
@@ -513,13 +563,18 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
     pl.ch = 65536 / step_bytes < pl.kp ? 65536 / step_bytes : pl.kp;
     pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
     auto fits = [&]() { return (size_t)layout_of(pl).total <= smem_limit; };
+    if (pl.nt > 1) {  // copies of two chunk-steps, as many as fit: the next tile's arrive while this one is contracted
+        pl.ch = pl.kp < 2 ? 1 : 2;
+        pl.stages = 16;
+        while (!fits() && pl.stages > 3) --pl.stages;
+    }
     while (!fits() && pl.ch > 1) {
         pl.ch = pl.ch > 2 ? 2 : 1;
         pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
         while (!fits() && pl.stages > 2) --pl.stages;
     }
     if (!fits()) return FLSTM_OK;
-    pl.ring = pl.stages * pl.ch < pl.kp;
+    pl.ring = pl.nt > 1 || pl.stages * pl.ch < pl.kp;
     pl.smem_bytes = layout_of(pl).total;
     if (pl.smem_bytes < kMinSmemBytes) pl.smem_bytes = kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
     pl.grid = pl.jt * KS * pl.ngroups;

@@ -84,7 +84,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&tfull[i], 1);
-            mbar_init(&tempty[i], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs report to the leader
+            mbar_init(&tempty[i], 2 * (kEpilogueWarps + 1));  // epilogue warps and publishers of both CTAs report to the leader
             mbar_init(&hdone[i], kEpilogueWarps);
         }
         mbar_init(wbar, 1);
@@ -251,7 +251,10 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             for (int tt = 0; tt < p.T && ok; ++tt)
                 for (int n = 0; n < NT && ok; ++n, ++wi) {
                     ok = mbar_wait(&hdone[wi & 1], (wi >> 1) & 1, abort_w, wait_ns);
-                    if (ok) red_release_gpu_add(counters + n, 1u);
+                    if (!ok) break;
+                    // no third tile may use this hdone barrier before the publisher has seen this phase of it
+                    mbar_arrive_cluster_relaxed(tempty_c + 8u * (wi & 1));
+                    red_release_gpu_add(counters + n, 1u);
                 }
         }
     } else {
@@ -443,7 +446,9 @@ int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan) {
     const int tiles = (B + pl.BT - 1) / pl.BT;
     pl.nt = (tiles + groups - 1) / groups;
     pl.ngroups = (tiles + pl.nt - 1) / pl.nt;
-    if (pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
+    // Up to six tiles in turn: H = 1024, B = 1536 28.2 -> 23.4 us a step against the output-tiled kernel, H = 512, B = 2048 17.2 ->
+    // 15.0, H = 2048, B = 512 25.4 -> 24.2; eight are slower (H = 1024, B = 2048 30.3 -> 31.8), the epilogue then bounds it
+    if (pl.nt > 6 || pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
     pl.kc = H / 64;
     const int tmem_chunks = (kTmemColumns - pl.BT) / 32;
     pl.ct = (pl.kc < tmem_chunks ? pl.kc : tmem_chunks) / kCh * kCh;

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(1, 1088, True), (70, 1088, True), (33, 1152, True), (100, 1152, True), (40, 1216, True), (32, 1280, True),
           (5, 2048, True), (64, 2048, True), (31, 2304, True), (50, 2368, True),
           (140, 1024, True), (256, 1024, True), (259, 1024, False), (300, 704, True), (130, 1088, True), (65, 1984, False),
-          (100, 2048, True), (256, 2048, True), (150, 2176, False),  # the last nine: batch tiles in turn
+          (100, 2048, True), (256, 2048, True), (530, 320, True), (290, 576, True), (150, 2176, False),  # the last nine: batch tiles in turn
           (3, 2432, False), (16, 2496, False), (17, 3072, False), (33, 4096, False), (8, 4096, False), (64, 2560, False)]
 
 

@@ -535,38 +535,38 @@ int max_clusters(const BwdTmPlan &pl) {
 }  // namespace
 
 // ------------------------------------------------------------------ host side
-int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool check_device) {
-    *plan = BwdTmPlan{};
-    if (H % 64 != 0 || H < 256 || smem_limit < 160 * 1024) return FLSTM_OK;
-    const char *env = std::getenv("FLSTM_TMEM");
-    if (env && env[0] == '0') return FLSTM_OK;
+static int plan_groups(int B, int H, int groups, size_t smem_limit, BwdTmPlan *plan) {
     BwdTmPlan pl{};
     pl.jt = H / 64;
-    if (pl.jt * KS > sms) return FLSTM_OK;
     // one tile of 32 sequences per group, of 64, or several of 64 in turn: the tiles are independent recurrences with a step
     // barrier each, so the chain of one hides behind the others' contractions
-    const int groups = sms / (pl.jt * KS);
     pl.BT = B <= 32 * groups ? 32 : 64;
     const int tiles = (B + pl.BT - 1) / pl.BT;
     pl.nt = (tiles + groups - 1) / groups;
     pl.ngroups = (tiles + pl.nt - 1) / pl.nt;
     if (pl.BT == 64 && pl.nt == 1 && H <= 1024) return FLSTM_OK;  // a chain that stands alone: the other kernels are as fast
-    if (const char *e = std::getenv("FLSTM_BNT")) if (pl.nt > std::atoi(e)) return FLSTM_OK;
-    if (pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
+    // Tiles in turn against the step-by-step GEMMs (which exist for H % 128 == 0), backward pass in us a step with its GEMMs:
+    //   2 tiles: H = 512, B = 512 12.4 -> 8.7    H = 1024, B = 256 13.8 -> 9.8   H = 1536, B = 128 17.6 -> 10.9   H = 2048, B = 128 17.4 -> 16.0
+    //   3 tiles: H = 640, B = 512 16.2 -> 14.0   H = 1024, B = 384 16.4 -> 13.6  H = 1792, B = 192 21.4 -> 16.3   H = 2048, B = 190 21.9 -> 23.2
+    //   4 tiles: H = 512, B = 1024 16.3 -> 17.3  H = 1024, B = 512 18.6 -> 18.5  H = 1536, B = 256 20.4 -> 17.9   H = 1792, B = 256 23.1 -> 21.4
+    // Every tile brings its dG through the SM's port (H x 128 bytes) and its own pointwise pass, a step GEMM spreads them.  At other
+    // H the alternative takes several tiles per step one after the other (H = 1216, B = 200 25.4 -> 15.2).
+    const int most = H % 128 != 0 ? 6 : H > 1792 ? 2 : H > 1024 ? 4 : 3;
+    if (pl.nt > most || pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
     const int kcq = H / 16 / KS;
     pl.kp = kcq / 2;
     pl.left = kcq % 2;
     const int tmem_steps = (kTmemColumns - 2 * pl.BT) / 32, step_bytes = 2 * pl.BT * 128;
     pl.ct = pl.kp < tmem_steps ? pl.kp : tmem_steps;
     pl.cs = pl.kp - pl.ct;
-    // dG in copies of up to 64 KB, the whole tile at once if it fits
-    pl.ch = 65536 / step_bytes < pl.kp ? 65536 / step_bytes : pl.kp;
-    pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
     auto fits = [&]() { return (size_t)layout_of(pl).total <= smem_limit; };
     if (pl.nt > 1) {  // copies of two chunk-steps, as many as fit: the next tile's arrive while this one is contracted
         pl.ch = pl.kp < 2 ? 1 : 2;
         pl.stages = 16;
         while (!fits() && pl.stages > 3) --pl.stages;
+    } else {  // dG in copies of up to 64 KB, the whole tile at once if it fits
+        pl.ch = 65536 / step_bytes < pl.kp ? 65536 / step_bytes : pl.kp;
+        pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
     }
     while (!fits() && pl.ch > 1) {
         pl.ch = pl.ch > 2 ? 2 : 1;
@@ -578,9 +578,23 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
     pl.smem_bytes = layout_of(pl).total;
     if (pl.smem_bytes < kMinSmemBytes) pl.smem_bytes = kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
     pl.grid = pl.jt * KS * pl.ngroups;
-    if (check_device && (pl.BT == 32 ? max_clusters<32>(pl) : max_clusters<64>(pl)) * KS < pl.grid) return FLSTM_OK;
     pl.use = true;
     *plan = pl;
+    return FLSTM_OK;
+}
+
+int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool check_device) {
+    *plan = BwdTmPlan{};
+    if (H % 64 != 0 || H < 256 || smem_limit < 160 * 1024) return FLSTM_OK;
+    const char *env = std::getenv("FLSTM_TMEM");
+    if (env && env[0] == '0') return FLSTM_OK;
+    // as many batch groups as the device holds clusters for at once
+    for (int groups = sms / (H / 64 * KS); groups > 0; --groups) {
+        FLSTM_TRY(plan_groups(B, H, groups, smem_limit, plan));
+        if (!plan->use) return FLSTM_OK;
+        if (!check_device || (plan->BT == 32 ? max_clusters<32>(*plan) : max_clusters<64>(*plan)) * KS >= plan->grid) return FLSTM_OK;
+        *plan = BwdTmPlan{};
+    }
     return FLSTM_OK;
 }
 

@@ -75,7 +75,30 @@ PyObject *py_backward(PyObject *, PyObject *args) {
     return raise_if_failed();
 }
 
+// flstm_engine_forward for the Engine class: a call of a few steps is bound by its host work, of which the generic foreign
+// function call took a sixth.
+PyObject *py_engine_forward(PyObject *, PyObject *const *args, Py_ssize_t count) {
+    if (count != 9) {
+        PyErr_Format(PyExc_TypeError, "engine_forward expects 9 integer arguments");
+        return nullptr;
+    }
+    unsigned long long v[9];
+    for (Py_ssize_t i = 0; i < 9; ++i) {
+        v[i] = args[i] == Py_None ? 0 : PyLong_AsUnsignedLongLongMask(args[i]);
+        if (v[i] == (unsigned long long)-1 && PyErr_Occurred()) return nullptr;
+    }
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = flstm_engine_forward(as_ptr<flstm_engine *>(v[0]), (size_t)v[1], as_ptr<const void *>(v[2]), as_ptr<const void *>(v[3]),
+                                  as_ptr<const void *>(v[4]), as_ptr<void *>(v[5]), as_ptr<void *>(v[6]), as_ptr<void *>(v[7]),
+                                  as_ptr<void *>(v[8]));
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(status);
+}
+
 PyMethodDef kMethods[] = {
+    {"engine_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_engine_forward)), METH_FASTCALL,
+     "engine_forward(engine, T, x, h0, c0, y, hn, cn, stream) -> status"},
     {"streaming_lstm_forward", py_forward, METH_VARARGS,
      "streaming_lstm_forward(T,B,I,H,R, x_host,h0,c0, W_ih,W_hh,b_ih,b_hh, y_host, cache_h,cache_c, "
      "cache_h_dtype,cache_c_dtype, hy,cy, compute_stream,h2d_stream,d2h_stream) -> None"},

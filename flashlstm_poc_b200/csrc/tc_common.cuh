@@ -306,27 +306,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_f16(int m, int n, int ab_forma
     return (1u << 4) | ((uint32_t)ab_format << 7) | ((uint32_t)ab_format << 10) | ((uint32_t)a_mn_major << 15) |
            ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-// Same, with the accumulate flag known at compile time (no predicate set-up in the issue loop).
-template <bool ACC>
-__device__ __forceinline__ void umma_f16_imm(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-    if (ACC) {
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "setp.eq.u32 p, 1, 1;\n"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-            "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "setp.eq.u32 p, 1, 0;\n"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-            "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
-            : "memory");
-    }
-}
 // D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          uint32_t accumulate) {
@@ -417,10 +396,6 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
         "}\n"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
-}
-template <bool ACC>
-__device__ __forceinline__ void umma_f16_pair_imm(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-    umma_f16_pair(d_tmem, a_desc, b_desc, idesc, ACC ? 1u : 0u);
 }
 // One arrival on the mbarrier at this offset in BOTH CTAs of the pair when every UMMA issued so far by this
 // thread has completed (a commit is a signal, not a load: the operands are never multicast).  Two separate

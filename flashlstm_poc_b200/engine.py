@@ -9,6 +9,7 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 
 from . import _lib
+from ._flashlstm import engine_forward as _native_forward
 from ._lib import BACKEND_CODES, BACKEND_NAMES, DTYPE_CODES, EngineConfig, check
 
 TORCH_DTYPES = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
@@ -37,14 +38,14 @@ class Engine:
         handle = ctypes.c_void_p()
         with torch.cuda.device(self.device):
             check(self.lib.flstm_engine_create(ctypes.byref(cfg), ctypes.byref(handle)))
-        self._h = handle
+        self._h, self._address = handle, handle.value
         self._saved_x = None
         self._index = torch.cuda.current_device() if self.device.index is None else self.device.index
 
     def close(self) -> None:
         if getattr(self, "_h", None):
             self.lib.flstm_engine_destroy(self._h)
-            self._h = None
+            self._h = self._address = None  # the native side refuses a null engine
 
     def __del__(self):
         try:
@@ -63,7 +64,7 @@ class Engine:
         return ("steps", "grid", "cluster")[path.value], ctas.value, seqs.value
 
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self._index).cuda_stream
+        return torch._C._cuda_getCurrentRawStream(self._index)  # current_stream() makes a Stream object of it first
 
     def _accepts(self, t: torch.Tensor, shape: Tuple[int, ...]) -> bool:
         """The common case of _check_tensor at a fraction of its cost: a call of a few steps is bound by its host work."""
@@ -117,8 +118,8 @@ class Engine:
         if want_states:  # empty_like is the cheapest of the allocating calls
             hn = torch.empty_like(h0) if h0 is not None else x.new_empty((L, B, H))
             cn = torch.empty_like(hn)
-        check(self.lib.flstm_engine_forward(self._h, T, x.data_ptr(), _ptr(h0), _ptr(c0), y.data_ptr(), _ptr(hn),
-                                            _ptr(cn), self._stream()))
+        check(_native_forward(self._address, T, x.data_ptr(), _ptr(h0), _ptr(c0), y.data_ptr(), _ptr(hn), _ptr(cn),
+                              self._stream()))
         self._saved_x = x  # re-read by backward for dW_ih
         return y, hn, cn
 

@@ -28,21 +28,37 @@ __global__ void __launch_bounds__(512, 1) cell_step_kernel(const CellParams p) {
     const uint16_t *x = static_cast<const uint16_t *>(p.x), *h = static_cast<const uint16_t *>(p.h_prev);
     float acc[NT][2][4] = {};
     constexpr int DEPTH = NT == 1 ? 4 : 2;
-    for (int c0 = warp; c0 < chunks; c0 += warps * DEPTH) {
-        uint4 w[DEPTH][4], b[DEPTH][NT];
+    uint4 w[DEPTH][4];
+    auto load_w = [&](int c0) {
 #pragma unroll
         for (int d = 0; d < DEPTH; ++d) {
             const int c = c0 + d * warps;
             const bool of_x = c < x_chunks;
             const int k = (of_x ? c : c - x_chunks) * 32 + 8 * q, K = of_x ? I : H;
-            const bool in = c < chunks && k < K;
-            const uint16_t *wrow = (of_x ? w_ih : w_hh) + row0 * K + k, *brow = (of_x ? x : h) + k;
+            const uint16_t *wrow = (of_x ? w_ih : w_hh) + row0 * K + k;
 #pragma unroll
-            for (int g = 0; g < 4; ++g) w[d][g] = in ? __ldg(reinterpret_cast<const uint4 *>(wrow + (size_t)(16 * g) * K)) : make_uint4(0, 0, 0, 0);
+            for (int g = 0; g < 4; ++g)
+                w[d][g] = c < chunks && k < K ? __ldg(reinterpret_cast<const uint4 *>(wrow + (size_t)(16 * g) * K)) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    // Weights do not come from the launch before: the first rounds of them are under way before its results are waited for.  The
+    // next launch may start once this one has waited, so that whatever it finds here was complete before the first of them.
+    load_w(warp);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (int c0 = warp; c0 < chunks; c0 += warps * DEPTH) {
+        if (c0 != warp) load_w(c0);
+        uint4 b[DEPTH][NT];
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+            const int c = c0 + d * warps;
+            const bool of_x = c < x_chunks;
+            const int k = (of_x ? c : c - x_chunks) * 32 + 8 * q, K = of_x ? I : H;
+            const uint16_t *brow = (of_x ? x : h) + k;
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 const int n = nt * 8 + i8;
-                b[d][nt] = in && n < p.B ? *reinterpret_cast<const uint4 *>(brow + (size_t)n * K) : make_uint4(0, 0, 0, 0);
+                b[d][nt] = c < chunks && k < K && n < p.B ? *reinterpret_cast<const uint4 *>(brow + (size_t)n * K) : make_uint4(0, 0, 0, 0);
             }
         }
 #pragma unroll
@@ -110,8 +126,17 @@ int lstm_cell_step(int dtype, const CellParams &p, cudaStream_t s) {
 #undef FLSTM_CELL
     const size_t smem = (size_t)(warps + 1) * NT * 256 * sizeof(float);
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, smem));
-    kern<<<p.H / 8, warps * 32, smem, s>>>(p);
-    const cudaError_t e = cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.H / 8);
+    cfg.blockDim = dim3(warps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.follows ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "cell step launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
 }

@@ -171,18 +171,29 @@ int init(Engine &e) {
         // the cross-layer wavefront would put two cooperative grids side by side
         const char *wave = std::getenv("FLSTM_WAVE_CHUNK");
         const bool wavefront = wave && std::atoi(wave) > 0;
+        // Moving W_hh into tensor memory takes 2 us of a launch (BPTT 4 us), which few steps do not repay; where the other kernels
+        // exist in a good form (H % 128 == 0) they keep engines made for short sequences.  A forward launch, us, T = 1 / 2 / 4 / 8:
+        // H = 1024, B = 64 18.5 / 22.6 / 30.2 / 45.2 -> 20.2 / 23.2 / 30.8 / 44.9;  H = 2048, B = 40 20.6 / 26.7 / 39.0 / 65.7 -> 22.7 /
+        // 28.8 / 41.3 / 66.5;  in turn, H = 1024, B = 256 22.6 / 30.8 / 49.2 / 82.8 -> 24.6 / 30.8 / 43.1 / 69.7.  BPTT at H = 1024,
+        // B = 32, T = 8 / 16: 76 / 111 -> 80 / 116.
+        const size_t steps = e.cfg.max_seq_len;
+        const bool good = H % 128 == 0;
         if (!st->cfwd.use && !wavefront) {
             FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &st->fwdtm));
             // 33 to 64 sequences per batch group: the K halves make an UMMA of N = 128, which takes longer than the other
             // kernel's of N = 64 (H = 512, B = 250: 4.15 against 3.97 us a step; H = 640, B = 130: 4.16 against 3.98), so that one
-            // stays where its weights are resident and a CTA has one batch tile
+            // stays where its weights are resident and a CTA has one batch tile; beyond that the gain per step is small
             FwdPlan f{};
             const bool one_tile = plan_fwd(B, H, st->sms, st->smem_limit, &f) == FLSTM_OK && f.resident && f.nt == 1 && f.BT <= 64;
+            const bool fits_one = st->fwdtm.use;
             if (st->fwdtm.BT == 64 && one_tile) st->fwdtm.use = false;
-            else if (!st->fwdtm.use) FLSTM_TRY(plan_fwd_wide(B, H, st->sms, st->smem_limit, &st->wide));
+            if (st->fwdtm.S == 2 && good && f.nt == 1 && steps < (st->fwdtm.BT == 64 ? 32 : 5)) st->fwdtm.use = false;
+            if (!fits_one && steps > 1) FLSTM_TRY(plan_fwd_wide(B, H, st->sms, st->smem_limit, &st->wide));
         }
-        if (e.cfg.training && !st->cbwd.use && !wavefront)
+        if (e.cfg.training && !st->cbwd.use && !wavefront) {
             FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &st->bwdtm, /*check_device=*/true));
+            if (good && st->bwdtm.nt == 1 && H <= 1024 && steps < 24) st->bwdtm.use = false;
+        }
     }
     const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use && !st->wide.use, grid_bwd = e.cfg.training && !st->cbwd.use && !st->bwdtm.use;
     st->bwd_ok = e.cfg.training != 0;
@@ -475,6 +486,7 @@ int forward_cells(Engine &e, size_t T, const void *x, const void *h0, const void
             p.I = (int)l.in_size;
             p.H = (int)H;
             p.real_units = e.logical_h;
+            p.follows = t > 0 || li > 0;
             FLSTM_TRY(lstm_cell_step(e.cfg.dtype, p, s));
             ++e.launches;
         }

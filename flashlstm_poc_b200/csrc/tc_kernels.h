@@ -245,6 +245,7 @@ struct CellParams {
     int c_prev_f32, cn_f32;
     int B, I, H;
     int real_units;           // as in FwdParams
+    int follows;              // the launch before it in the stream is another cell step of the same call
 };
 constexpr int kCellBatch = 32;
 int lstm_cell_step(int dtype, const CellParams &p, cudaStream_t s);

@@ -10,18 +10,20 @@ from tests.gpu_helpers import assert_parity, run_engine, run_oracle
 
 pytestmark = pytest.mark.gpu
 
-# batch, hidden size, training
-SHAPES = [(1, 1088, True), (70, 1088, True), (33, 1152, True), (100, 1152, True), (40, 1216, True), (32, 1280, True),
-          (5, 2048, True), (64, 2048, True), (31, 2304, True), (50, 2368, True),
-          (140, 1024, True), (256, 1024, True), (259, 1024, False), (300, 704, True), (130, 1088, True), (65, 1984, False),
-          (100, 2048, True), (256, 2048, True), (530, 320, True), (290, 576, True), (150, 2176, False),  # the last nine: batch tiles in turn
-          (3, 2432, False), (16, 2496, False), (17, 3072, False), (33, 4096, False), (8, 4096, False), (64, 2560, False)]
+# batch, hidden size, training, steps
+SHAPES = [(1, 1088, True, 5), (70, 1088, True, 5), (33, 1152, True, 5), (100, 1152, True, 5), (40, 1216, True, 5), (32, 1280, True, 5),
+          (32, 1024, True, 25), (40, 768, True, 25), (5, 2048, True, 5), (64, 2048, True, 33), (31, 2304, True, 5), (50, 2368, True, 5),
+          # batch tiles in turn
+          (140, 1024, True, 5), (256, 1024, True, 5), (259, 1024, False, 5), (300, 704, True, 5), (130, 1088, True, 5), (65, 1984, False, 5),
+          (100, 2048, True, 5), (256, 2048, True, 5), (530, 320, True, 5), (290, 576, True, 5), (150, 2176, False, 5),
+          # streamed
+          (3, 2432, False, 5), (16, 2496, False, 5), (17, 3072, False, 5), (33, 4096, False, 5), (8, 4096, False, 5), (64, 2560, False, 5)]
 
 
-@pytest.mark.parametrize("B,H,training", SHAPES)
-def test_tensor_memory_kernels_match_the_oracle(B, H, training):
+@pytest.mark.parametrize("B,H,training,T", SHAPES)
+def test_tensor_memory_kernels_match_the_oracle(B, H, training, T):
     dtype = "bf16" if (B + H // 64) % 2 else "f16"
-    w = Workload("t", dtype, 1, 64, H, B, 5, seed=51, state_std=0.3, training=training)
+    w = Workload("t", dtype, 1, 64, H, B, T, seed=51, state_std=0.3, training=training)
     inp = make_inputs(w)
     got, eng = run_engine(w, inp, repeat=2)
     eng.close()

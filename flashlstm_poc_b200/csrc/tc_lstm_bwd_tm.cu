@@ -184,6 +184,16 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             for (int s = s_first; s < p.s1 && ok; ++s)
                 for (int n = 0; n < NT && ok; ++n) {
                     const int t_src = p.T - s, b0 = (tile0 + n) * BT;
+                    // Without a ring (one tile) the copies of a step are announced ahead of its barrier and follow it back to back,
+                    // see tc_lstm_fwd_tm.cu; the tile is free then: the barrier came after the UMMAs that read it
+                    const uint32_t step = (uint32_t)(s - s_first);
+                    for (int i = 0; !pl.ring && i < ST + pl.left; ++i) {
+                        uint64_t *bar = i < ST ? &full[i] : lfull;
+                        if (step > 0 && !mbar_wait(bar, (step - 1) & 1u, abort_w, wait_ns)) ok = false;
+                        if (!ok) break;
+                        mbar_expect_tx(bar, i < ST ? (uint32_t)stage_bytes : (uint32_t)(BT * 128));
+                    }
+                    if (!ok) break;
                     if (s > p.s0)
                         ok = wait_counter(counters + n, (unsigned)(pl.jt * KS) * (unsigned)(s - p.s0) + p.extra_arrivals, p.err, abort_w, 3u,
                                           wait_ns);
@@ -191,10 +201,11 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     fence_proxy_async_global();
                     if (n == 0) FLSTM_STAMP(s - p.s0, 0);
                     for (int ld = 0; ld < NLOAD; ++ld) {
-                        // (without a ring the tile is free: the step barrier came after the UMMAs that read it)
-                        if (pl.ring) ok = mbar_wait(&empty[stage], phase ^ 1, abort_w, wait_ns);
-                        if (!ok) break;
-                        mbar_expect_tx(&full[stage], (uint32_t)stage_bytes);
+                        if (pl.ring) {
+                            ok = mbar_wait(&empty[stage], phase ^ 1, abort_w, wait_ns);
+                            if (!ok) break;
+                            mbar_expect_tx(&full[stage], (uint32_t)stage_bytes);
+                        }
                         issued |= 1u << stage;
                         parity = (parity & ~(1u << stage)) | (phase << stage);
                         // (x, row, K half, chunk of the half, step); chunks beyond the half come as zeros (and are counted)
@@ -202,9 +213,11 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                         if (++stage == ST) { stage = 0; phase ^= 1; }
                     }
                     if (ok && pl.left) {
-                        if (pl.ring) ok = mbar_wait(lempty, lphase ^ 1, abort_w, wait_ns);
-                        if (!ok) break;
-                        mbar_expect_tx(lfull, BT * 128);
+                        if (pl.ring) {
+                            ok = mbar_wait(lempty, lphase ^ 1, abort_w, wait_ns);
+                            if (!ok) break;
+                            mbar_expect_tx(lfull, BT * 128);
+                        }
                         tma_load_4d(s_left, &maps.chunk, 0, b0, c_first + 2 * KP, t_src, lfull);
                         left_issued = true;
                         lphase ^= 1;

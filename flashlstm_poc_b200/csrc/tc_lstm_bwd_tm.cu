@@ -588,8 +588,9 @@ static int plan_groups(int B, int H, int groups, size_t smem_limit, BwdTmPlan *p
     }
     if (!fits()) return FLSTM_OK;
     pl.ring = pl.nt > 1 || pl.stages * pl.ch < pl.kp;
-    pl.smem_bytes = layout_of(pl).total;
-    if (pl.smem_bytes < kMinSmemBytes) pl.smem_bytes = kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
+    // All of shared memory: a CTA allocates all of tensor memory, so no other kernel that uses some (another engine's, on another
+    // stream) may share its SM; two grids that each held what the other's CTAs were waiting for would run into their limits
+    pl.smem_bytes = (int)smem_limit;
     pl.grid = pl.jt * KS * pl.ngroups;
     pl.use = true;
     *plan = pl;

@@ -578,8 +578,9 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
         if (pl.wstages > rest / WCH) pl.wstages = rest / WCH;
         pl.cs = rest % WCH;
     }
-    pl.smem_bytes = layout_of(pl).total;
-    if (pl.smem_bytes < kMinSmemBytes) pl.smem_bytes = kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
+    // All of shared memory: a CTA allocates all of tensor memory, so no other kernel that uses some (another engine's, on another
+    // stream) may share its SM; two grids that each held what the other's CTAs were waiting for would run into their limits
+    pl.smem_bytes = (int)smem_limit;
     pl.grid = pl.cta_rows * pl.ngroups;
     pl.use = true;
     *plan = pl;

@@ -456,7 +456,9 @@ int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan) {
     pl.hstages = 16;
     while (pl.hstages > 3 && (size_t)smem_of(pl) > smem_limit) --pl.hstages;
     if ((size_t)smem_of(pl) > smem_limit) return FLSTM_OK;
-    pl.smem_bytes = smem_of(pl) > kMinSmemBytes ? smem_of(pl) : kMinSmemBytes;  // one CTA per SM: each allocates all of tensor memory
+    // All of shared memory: a CTA allocates all of tensor memory, so no other kernel that uses some (another engine's, on another
+    // stream) may share its SM; two grids that each held what the other's CTAs were waiting for would run into their limits
+    pl.smem_bytes = (int)smem_limit;
     pl.grid = pl.cta_rows * pl.ngroups;
     pl.use = true;
     *plan = pl;

@@ -223,7 +223,8 @@ typedef struct {
     int fwd_pair;      /* persistent forward kernel: neighbouring row-tile CTAs form cta_group::2 pairs */
     int step_fwd_pair; /* wide batches: the all-steps forward kernel runs on CTA pairs (256-sequence tiles) */
 } flstm_tc_plan_info;
-/* (Engines try the cluster-resident kernels first where hidden_size <= 768: see flstm_engine_path.) */
+/* (Engines try the cluster-resident kernels first where hidden_size <= 768, see flstm_engine_path, and then the kernels that
+ * hold W_hh in tensor memory, which this function does not describe; FLSTM_TMEM=0 switches those off.) */
 int flstm_tc_plan(size_t batch, size_t hidden_size, int training, int sm_count, size_t smem_limit,
                   flstm_tc_plan_info *out);
 

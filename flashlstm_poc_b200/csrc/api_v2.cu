@@ -379,6 +379,7 @@ int forward_streaming(V2Context *c, size_t T, size_t R, const __half *x_host, co
             FLSTM_TRY(c->event(3 * (k - 2) + 2, &ev_prev));
             FLSTM_CUDA_TRY(cudaStreamWaitEvent(sc, ev_prev, 0));
         }
+        e->impl.seq_start = t0;
         FLSTM_TRY(flstm_engine_forward(e, n, sl.x[slot], sl.h_state[slot], sl.c_state[slot], sl.y[slot], sl.h_state[slot ^ 1],
                                        sl.c_state[slot ^ 1], sc));
         // checkpoints: entry e = state entering step e*R; this segment owns entries e0 .. e1-1.  Entry e0 is the
@@ -466,6 +467,7 @@ int backward_streaming(V2Context *c, size_t T, size_t R, const __half *x_host, f
             FLSTM_CUDA_TRY(cudaMemcpyAsync(sl.ck_h[slot], h0, slab * 2, cudaMemcpyDeviceToDevice, sc));
             FLSTM_TRY(simt::convert(FLSTM_DTYPE_F16, c0, FLSTM_DTYPE_F32, sl.ck_c[slot], slab, sc));
         }
+        e->impl.seq_start = t0;
         FLSTM_TRY(flstm_engine_backward_segment(e, n, r == 0, k == 0, sl.x[slot], sl.ck_h[slot], sl.ck_c[slot], sl.dy[slot], d_hn,
                                                 d_cn, sl.dx[slot], dh0, dc0, sc));
         FLSTM_CUDA_TRY(cudaEventRecord(ev_done, sc));

@@ -560,6 +560,7 @@ int Engine::forward_checkpointed(size_t T, const void *x, const void *h0, const 
         size_t k = 0;
         for (size_t seg0 = 0; seg0 < T && st == FLSTM_OK; seg0 += R, ++k) {
             const size_t n = T - seg0 < R ? T - seg0 : R;
+            seg.start = seg0;
             // checkpoint k: the state entering the segment (slot 0)
             batch.dense(l.hs, cfg.dtype, byte_ptr(l.ck_h) + k * slab * es, cfg.dtype, B, H);
             batch.dense(l.cs, FLSTM_DTYPE_F32, l.ck_c + k * slab, FLSTM_DTYPE_F32, B, H);
@@ -600,6 +601,7 @@ int Engine::backward_checkpointed(size_t T, const void *dy, const void *dhn, con
     int st = FLSTM_OK;
     for (size_t kk = K; kk-- > 0 && st == FLSTM_OK;) {
         const size_t seg0 = kk * R, n = T - seg0 < R ? T - seg0 : R;
+        seg.start = seg0;
         seg.final_segment = kk == 0;
         seg.first_segment = kk == K - 1;
         const size_t T_loc = (kk == K - 1) ? n : n + 1;  // slot n of dG then holds the step after the segment

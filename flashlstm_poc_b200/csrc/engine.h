@@ -111,6 +111,7 @@ struct Engine {
         bool final_segment = true;   // the segment that starts at t = 0: dh0/dc0 and the gradient allreduce follow it
         bool first_segment = true;   // the first one processed (the end of the sequence): weight gradients start from zero
         bool keep_gates = true;      // forward writes the activated gates back (off in the checkpointing forward pass)
+        size_t start = 0;            // number of the segment's first step within the call's sequence
     } seg;
     std::vector<LayerBuffers> layers;
     float *grads = nullptr;  // flat fp32: per layer [dW_ih | dW_hh | db]
@@ -151,6 +152,7 @@ struct Engine {
     int padded_cache_ptrs(int layer, void **gates, float **cells, void **hiddens);
     int padded_mirror(size_t t0, size_t t1, cudaStream_t s);
     bool cell_io_f32 = false;       // c0 / c_n cross the API as fp32 instead of the engine dtype
+    size_t seq_start = 0;           // number of the calls' first step within a sequence that is streamed from outside in segments
     const void *x_saved = nullptr;  // layer-0 input of the last forward (caller keeps it alive)
     PhaseTimer timer;
     Comm *comm = nullptr;

@@ -400,6 +400,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.B = (int)B;
     p.H = (int)H;
     p.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
+    p.odd = (int)((e.seq_start + e.seg.start + t0) & 1);
     p.real_units = e.logical_h;
     p.trace = (li == 0 && t0 == 0) ? e.trace : nullptr;
     p.trace_steps = e.trace_steps;

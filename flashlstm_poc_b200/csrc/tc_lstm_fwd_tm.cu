@@ -15,9 +15,10 @@
 // Either way a CTA stages half of what its rows need of h, and nothing is multicast.
 //
 // K runs in chunk-steps of 64 per half: [0, ct) from tensor memory, [ct, ct + cs) from shared memory.  The rest is streamed
-// through a ring of slots by a warp of its own, ascending in even steps of a launch and descending in odd ones: the slots then
+// through a ring of slots by a warp of its own, ascending in even steps of the sequence and descending in odd ones: the slots then
 // still hold the chunk-steps that the next step starts with, and L2 is asked first for what it was given last (in one direction
-// 94 MB per step go round in its 126 MB and mostly miss).  A step takes the chunk-steps that the slots hold first, so that
+// 94 MB per step go round in its 126 MB and mostly miss).  The direction is the order of the sums: it follows the step's number
+// in its sequence, so that a sequence cut into ranges or segments gives the bits of one launch.  A step takes the chunk-steps that the slots hold first, so that
 // copies start as soon as h is there, then those in tensor and shared memory, then the streamed ones.  Roles, step barrier, epilogue and the way
 // out after a bounded wait expired are the other forward kernel's (tc_lstm_fwd.cu): producer and UMMA threads break out of
 // their loops, the 256 epilogue threads leave together, an aborted pair lingers before its final cluster barrier.
@@ -232,7 +233,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     h_issued = (1u << HST) - 1u;
                     h_parity = tt & 1 ? h_issued : 0u;
                 }
-                const bool down = STREAM && (tt & 1);
+                const bool down = STREAM && ((tt + p.odd) & 1);
                 for (int which = 0; !whole && which < (STREAM ? 3 : 1) && ok; ++which) {
                     const Run run = run_of<STREAM>(pl, which, down);
                     const bool desc = down && which != 1;
@@ -272,7 +273,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             uint32_t loaded = 0, parity = 0, eparity = 0;
             const int first = CT + CS, n = STREAM ? (KC - first) / WCH : 0, slot_bytes = WCH * kStepBytesW;
             for (int tt = 0; STREAM && tt < p.T && ok; ++tt) {
-                const bool down = tt & 1;
+                const bool down = (tt + p.odd) & 1;
                 for (int k = tt == 0 ? 0 : WST; k < n; ++k) {
                     const int i = down ? n - 1 - k : k, slot = i % WST;
                     if (k >= WST) {
@@ -306,7 +307,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 ok = mbar_wait_cluster(tempty, (tt & 1) ^ 1, abort_w, wait_ns);
                 if (!ok) break;
                 tcgen05_fence_after();
-                const bool down = STREAM && (tt & 1);
+                const bool down = STREAM && ((tt + p.odd) & 1);
                 uint32_t acc = 0;  // the step's first instruction overwrites the accumulator
                 for (int which = 0; which < (STREAM ? 3 : 1) && ok; ++which) {
                     const Run run = run_of<STREAM>(pl, which, down);

@@ -149,7 +149,9 @@ size_t flstm_engine_workspace_bytes(const flstm_engine *engine);
  *             checkpoint (rebuilding its gate cache), runs the BPTT over it and keeps the dh / dc carries for
  *             the next call; d_hn / d_cn are read by the call with last_in_time, dh0 / dc0 are written and the
  *             weight gradients are complete (and reduced over the ranks) after the call with first_in_time.
- * Results equal a single whole-sequence call up to the fp32 summation order of dW / db.  Tensor-core backend. */
+ * Results equal a single whole-sequence call up to the fp32 summation order of dW / db (beyond hidden_size = 2368, where part
+ * of W_hh is streamed in a direction that alternates from step to step, with segments of an even number of steps; the
+ * bits of odd ones differ by the order of fp32 sums).  Tensor-core backend. */
 int flstm_engine_backward_segment(flstm_engine *engine, size_t steps, int last_in_time, int first_in_time, const void *x_seg,
                                   const void *h_in, const float *c_in, const void *dy_seg, const void *d_hn, const void *d_cn,
                                   void *dx_seg, float *dh0, float *dc0, void *stream);

@@ -79,6 +79,11 @@ def test_checkpoint_mode_on_clusters(dtype, L, T, B, I, H, R):
     _compare(dtype, L, T, B, I, H, R)
 
 
+def test_checkpoint_mode_with_streamed_weights():
+    """Segments that start at an odd step, at a width whose W_hh is streamed in alternating directions."""
+    _compare("bf16", 1, 7, 3, 64, 2432, 3)
+
+
 def test_checkpoint_mode_limits():
     from flashlstm_poc_b200._lib import FlashLstmError
 

@@ -51,3 +51,27 @@ def test_ranges_continue_one_another(B, H):
     eng.close()
     for a, b in zip(want, got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H,dtype", [(2432, "bf16"), (2496, "f16"), (4096, "f16")])
+def test_ranges_of_a_streamed_forward_continue_one_another(H, dtype):
+    """Part of W_hh is streamed in a direction that alternates from step to step: it goes by the step's number in the sequence,
+    whatever step a launch starts at."""
+    B, T = 3, 7
+    w = Workload("t", dtype, 1, 64, H, B, T, seed=53, state_std=0.3, training=False)
+    inp = make_inputs(w)
+    dev, td = torch.device("cuda", 0), TORCH_DTYPES[dtype]
+    eng = Engine(dtype, 1, B, 64, H, T, training=False, device=dev)
+    eng.set_weights(0, inp.w_ih[0].to(dev), inp.w_hh[0].to(dev), inp.b_ih[0].to(dev), inp.b_hh[0].to(dev))
+    x, h0, c0 = (t.to(dev, td) for t in (inp.x, inp.h0, inp.c0))
+    want = [t.clone() for t in eng.forward(x, h0, c0)]
+    got = [torch.empty_like(t) for t in want]
+    for ranges in (((0, 3), (3, 4), (4, 7)), ((0, 1), (1, 6), (6, 7))):
+        for t in got:
+            t.zero_()
+        for t0, t1 in ranges:
+            eng.forward_range_into(T, t0, t1, x, h0, c0, *got)
+        torch.cuda.synchronize()
+        for a, b in zip(want, got):
+            assert torch.equal(a, b)
+    eng.close()

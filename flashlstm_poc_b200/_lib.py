@@ -14,7 +14,7 @@ LIB_PATH = os.path.join(PKG, "libflashlstm_b200.so")
 ENGINE_SYMBOLS = [
     "flstm_engine_create", "flstm_engine_destroy", "flstm_engine_set_weights", "flstm_engine_set_all_weights", "flstm_engine_forward",
     "flstm_engine_backward", "flstm_engine_forward_range", "flstm_engine_backward_range", "flstm_engine_grad_ptrs", "flstm_engine_grad_buffer", "flstm_engine_export_grads", "flstm_engine_cache_ptrs",
-    "flstm_engine_set_cell_io_f32", "flstm_engine_backend", "flstm_engine_path", "flstm_comm_unique_id", "flstm_engine_attach_comm",
+    "flstm_engine_set_cell_io_f32", "flstm_engine_backend", "flstm_engine_path", "flstm_engine_kernel", "flstm_comm_unique_id", "flstm_engine_attach_comm",
     "flstm_engine_enable_timing", "flstm_engine_phase_ms", "flstm_engine_launch_count", "flstm_tc_gemm",
     "flstm_engine_enable_trace", "flstm_engine_read_trace", "flstm_bias_grad", "flstm_tc_plan", "flstm_engine_wait", "flstm_engine_abort_comm",
                   "flstm_engine_set_recompute_interval", "flstm_engine_workspace_bytes",
@@ -49,6 +49,11 @@ class TcPlanInfo(ctypes.Structure):
         "bwd_batch_tile", "bwd_cluster_size", "bwd_grid", "bwd_batch_groups", "bwd_tiles_per_group",
         "bwd_stages", "bwd_chunks_per_stage", "bwd_weights_resident", "bwd_smem_bytes",
         "step_path", "step_bn_fwd", "step_bn_bwd", "step_splits", "step_pair", "fwd_pair", "step_fwd_pair")]
+
+
+class KernelInfo(ctypes.Structure):
+    _fields_ = [("name", ctypes.c_char_p), *((n, ctypes.c_int) for n in (
+        "launches_per_step", "batch_tile", "tiles_in_turn", "batch_groups", "weights_streamed"))]
 
 
 class LstmBuffers(ctypes.Structure):
@@ -99,6 +104,7 @@ def load() -> ctypes.CDLL:
     lib.flstm_engine_set_cell_io_f32.argtypes = [vp, ci]
     lib.flstm_engine_backend.argtypes = [vp]
     lib.flstm_engine_path.argtypes = [vp, ci, *[ctypes.POINTER(ci)] * 3]
+    lib.flstm_engine_kernel.argtypes = [vp, ci, sz, ctypes.POINTER(KernelInfo)]
     lib.flstm_comm_unique_id.argtypes = [vp]
     lib.flstm_engine_attach_comm.argtypes = [vp, vp, ci, ci]
     lib.flstm_engine_enable_timing.argtypes = [vp, ci]

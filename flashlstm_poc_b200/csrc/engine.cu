@@ -1170,6 +1170,23 @@ int flstm_engine_path(flstm_engine *engine, int backward, int *path, int *ctas, 
     return FLSTM_OK;
 }
 
+int flstm_engine_kernel(flstm_engine *engine, int backward, size_t steps, flstm_kernel_info *out) {
+    if (!engine || !out) return set_error(FLSTM_ERR_INVALID, "null argument");
+    if (steps == 0) return set_error(FLSTM_ERR_INVALID, "a launch has at least one step");
+    const Engine &e = engine->impl.core();
+    if (backward && !e.cfg.training) return set_error(FLSTM_ERR_INVALID, "engine was created with training = 0");
+    *out = flstm_kernel_info{};
+    if (e.backend == FLSTM_BACKEND_TC) {
+        flstm_b200::tc::recurrent_kernel(e, backward != 0, steps, out);
+        return FLSTM_OK;
+    }
+    const auto &plan = backward ? e.f32_bwd : e.f32_fwd;
+    if (plan.use) *out = {backward ? "f32_cluster_bwd_kernel" : "f32_cluster_fwd_kernel", 0, plan.seqs, 1, 0, 0};
+    else if (e.simt_grid) *out = {backward ? "persistent_backward_kernel" : "persistent_forward_kernel", 0, 0, 1, 0, 0};
+    else *out = {backward ? "step_backward_kernel" : "step_forward_kernel", 1, 0, 1, 0, 1};
+    return FLSTM_OK;
+}
+
 int flstm_engine_wait(flstm_engine *engine, cudaStream_t stream, unsigned int timeout_ms) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
     Engine &e = engine->impl;

@@ -231,6 +231,7 @@ int poll_error(Engine &e);  // reports (and clears) a device-side wait that expi
 int set_weights(Engine &e, int first, int count, const float *const *params, cudaStream_t s);
 unsigned int *error_mirror(Engine &e);
 int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs);  // flstm_path
+void recurrent_kernel(const Engine &e, bool backward, size_t steps, flstm_kernel_info *out);
 int forward_layer(Engine &e, int layer, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s);
 // `dx_ready` (optional) is recorded on `s` once dx_l of the range is complete, before the weight gradients
 int backward_layer(Engine &e, int layer, size_t T, size_t t0, size_t t1, const void *x_l, const void *dy_l,

@@ -307,6 +307,24 @@ int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs) {
     return !backward && st->step.fwd_persistent && wavefront_chunk(e, (size_t)-1) == 0 ? FLSTM_PATH_GRID : FLSTM_PATH_STEPS;
 }
 
+void recurrent_kernel(const Engine &e, bool backward, size_t, flstm_kernel_info *out) {
+    const TcState *st = static_cast<const TcState *>(e.tc_state);
+    const bool steps_path = st->step.use && (backward || !st->step.fwd_persistent || wavefront_chunk(e, (size_t)-1) != 0);
+    if (!backward) {
+        if (st->cfwd.use) *out = {"cluster_fwd_kernel", 0, st->cfwd.seqs, 1, 0, 0};
+        else if (st->wide.use) *out = {"lstm_fwd_wide_kernel", 0, st->wide.BT, st->wide.nt, st->wide.ngroups, 0};
+        else if (st->fwdtm.use) *out = {"lstm_fwd_tm_kernel", 0, st->fwdtm.BT, 1, st->fwdtm.ngroups, st->fwdtm.wstages > 0};
+        else if (steps_path) *out = {"step_kernel", 1, 0, 1, 0, 1};
+        else if (st->step.use) *out = {"wide_fwd_kernel", 0, 0, 1, 0, 1};
+        else *out = {"lstm_fwd_kernel", 0, st->fwd.BT, st->fwd.nt, st->fwd.ngroups, !st->fwd.resident};
+    } else {
+        if (st->cbwd.use) *out = {"cluster_bwd_kernel", 0, st->cbwd.seqs, 1, 0, 0};
+        else if (st->bwdtm.use) *out = {"lstm_bwd_tm_kernel", 0, st->bwdtm.BT, st->bwdtm.nt, st->bwdtm.ngroups, 0};
+        else if (steps_path) *out = {"step_kernel", 2, 0, 1, 0, 1};  // step_bwd_pointwise_kernel and the GEMM
+        else *out = {"lstm_bwd_kernel", 0, st->bwd.BT, st->bwd.nt, st->bwd.ngroups, !st->bwd.resident};
+    }
+}
+
 int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s) {
     TcState *st = state(e);
     FLSTM_TRY(check_async_error(e));

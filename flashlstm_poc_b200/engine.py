@@ -4,7 +4,7 @@ device pointers across the C ABI.  PyTorch is used for device memory and streams
 from __future__ import annotations
 
 import ctypes
-from typing import List, Optional, Sequence, Tuple
+from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
@@ -62,6 +62,13 @@ class Engine:
         path, ctas, seqs = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         check(self.lib.flstm_engine_path(self._h, int(backward), ctypes.byref(path), ctypes.byref(ctas), ctypes.byref(seqs)))
         return ("steps", "grid", "cluster")[path.value], ctas.value, seqs.value
+
+    def recurrent_kernel(self, steps: int, backward: bool = False) -> Dict[str, object]:
+        """The kernel that runs a launch of `steps` time steps, and its batch layout (flstm_kernel_info)."""
+        info = _lib.KernelInfo()
+        check(self.lib.flstm_engine_kernel(self._h, int(backward), steps, ctypes.byref(info)))
+        out = {field: getattr(info, field) for field, _ in info._fields_}
+        return dict(out, name=info.name.decode())
 
     def _stream(self) -> int:
         return torch._C._cuda_getCurrentRawStream(self._index)  # current_stream() makes a Stream object of it first

@@ -165,6 +165,18 @@ int flstm_engine_backend(const flstm_engine *engine);
  * the CTAs of a cluster and `seqs` its sequences (else 0).  Either of them may be NULL. */
 typedef enum { FLSTM_PATH_STEPS = 0, FLSTM_PATH_GRID = 1, FLSTM_PATH_CLUSTER = 2 } flstm_path;
 int flstm_engine_path(flstm_engine *engine, int backward, int *path, int *ctas, int *seqs);
+/* The kernel that runs a launch of `steps` time steps of the recurrence (backward = 0) or the BPTT (1; training engines), and
+ * how it lays the batch out.  (Inference calls of a few steps may run cell by cell instead, which depends on the call's
+ * tensors: cell_step_kernel.) */
+typedef struct {
+    const char *name;      /* as in the library's sources and in a profiler's list; a static string */
+    int launches_per_step; /* 0: one launch runs all the steps of a range */
+    int batch_tile;        /* sequences that a CTA, pair or cluster works on at a time (0: not tiled by sequences) */
+    int tiles_in_turn;     /* batch tiles that it takes one after the other within a step */
+    int batch_groups;      /* groups of CTAs with batch tiles and a step barrier of their own (0: no such groups) */
+    int weights_streamed;  /* W_hh, or a part of it, is read again in every step */
+} flstm_kernel_info;
+int flstm_engine_kernel(flstm_engine *engine, int backward, size_t steps, flstm_kernel_info *out);
 
 /* Batch-sharded data parallelism: one engine per GPU/process.  flstm_comm_unique_id fills a
  * 128-byte id on rank 0 (send it to the other ranks by any means); every rank then calls

@@ -75,3 +75,45 @@ def test_ranges_of_a_streamed_forward_continue_one_another(H, dtype):
         for a, b in zip(want, got):
             assert torch.equal(a, b)
     eng.close()
+
+
+# batch, hidden size, training, steps, then (kernel, batch tile, tiles in turn) forward and backward.  More than 33 clusters of
+# four CTAs do not fit the GPU at once, so that from H = 1088 on the BPTT has one batch group.
+TM, WIDE, BACK = "lstm_fwd_tm_kernel", "lstm_fwd_wide_kernel", "lstm_bwd_tm_kernel"
+KERNELS = [
+    (1, 1088, True, 5, (TM, 32, 1), (BACK, 32, 1)), (70, 1088, True, 5, (TM, 64, 1), (BACK, 64, 2)),
+    (33, 1152, True, 5, (TM, 32, 1), (BACK, 64, 1)), (100, 1152, True, 5, (TM, 64, 1), (BACK, 64, 2)),
+    (40, 1216, True, 5, ("lstm_fwd_kernel", 64, 1), (BACK, 64, 1)), (32, 1280, True, 5, (TM, 32, 1), (BACK, 32, 1)),
+    (32, 1024, True, 25, (TM, 32, 1), (BACK, 32, 1)), (40, 768, True, 25, ("cluster_fwd_kernel", 6, 1), ("cluster_bwd_kernel", 6, 1)),
+    (5, 2048, True, 5, (TM, 32, 1), (BACK, 32, 1)), (64, 2048, True, 33, (TM, 64, 1), (BACK, 64, 1)),
+    # training at these widths needs more clusters than fit: CUDA cores
+    (31, 2304, True, 5, ("step_forward_kernel", 0, 1), ("step_backward_kernel", 0, 1)),
+    (50, 2368, True, 5, ("step_forward_kernel", 0, 1), ("step_backward_kernel", 0, 1)),
+    (31, 2304, False, 5, (TM, 32, 1), None), (50, 2368, False, 5, (TM, 64, 1), None),
+    # batch tiles in turn
+    (140, 1024, True, 5, (WIDE, 64, 2), (BACK, 64, 2)), (256, 1024, True, 5, (WIDE, 64, 2), (BACK, 64, 2)),
+    (259, 1024, False, 5, (WIDE, 128, 2), None), (300, 704, True, 5, (WIDE, 64, 2), (BACK, 64, 2)),
+    (130, 1088, True, 5, (WIDE, 64, 2), (BACK, 64, 3)), (65, 1984, False, 5, (WIDE, 64, 2), None),
+    (100, 2048, True, 5, (WIDE, 64, 2), (BACK, 64, 2)), (256, 2048, True, 5, (WIDE, 128, 2), ("step_kernel", 0, 1)),
+    (530, 320, True, 5, (WIDE, 64, 2), (BACK, 64, 2)), (290, 576, True, 5, (WIDE, 64, 2), (BACK, 64, 2)),
+    (150, 2176, False, 5, (WIDE, 128, 2), None),
+    # streamed
+    (3, 2432, False, 5, (TM, 16, 1), None), (16, 2496, False, 5, (TM, 16, 1), None), (17, 3072, False, 5, (TM, 32, 1), None),
+    (33, 4096, False, 5, (TM, 64, 1), None), (8, 4096, False, 5, (TM, 16, 1), None), (64, 2560, False, 5, (TM, 64, 1), None)]
+
+
+def check_kernels(table):
+    for B, H, training, T, forward, backward in table:
+        eng = Engine("f16", 1, B, 64, H, T, training=training, device=torch.device("cuda", 0))
+        for back, want in ((False, forward), (True, backward)):
+            if want is not None:
+                got = eng.recurrent_kernel(T, backward=back)
+                assert (got["name"], got["batch_tile"], got["tiles_in_turn"]) == want, (B, H, back)
+                if got["name"] in (TM, WIDE, BACK):
+                    assert bool(got["weights_streamed"]) == (H > 2368)
+        eng.close()
+
+
+def test_which_kernels_the_shapes_run():
+    assert set(SHAPES) <= {s[:4] for s in KERNELS}
+    check_kernels(KERNELS)

@@ -27,6 +27,7 @@ struct TcLayer {
     CUtensorMap tm_h;   // hs (Tcap+1, B, H), 1 x BT x 64 boxes, 128B swizzle
     CUtensorMap tm_g;   // gates (Tcap, B, 4H), 1 x BT x 64 boxes, no swizzle
     CUtensorMap tm_dg;  // dG (Tcap, B, 4H), 1 x BT x 64 boxes, 128B swizzle (BPTT operand)
+    CUtensorMap tm_h_tm, tm_g_tm;  // hs and gates with the boxes of the tensor-memory forward kernels
     CUtensorMap tm_ws;  // w_hh, 128 x 64 boxes (streamed part of the tensor-memory forward), or its gate-row form (wide forward)
     BwdTmMaps dg_tm;    // dG for the tensor-memory BPTT kernel
     // wide-batch path (one GEMM launch per step)
@@ -44,6 +45,7 @@ struct TcState {
     FwdWidePlan wide{};
     BwdPlan bwd{};
     BwdTmPlan bwdtm{};
+    size_t fwd_from = 0, bwd_from = 0;  // launches of fewer steps run without tensor memory
     bool bwd_ok = false;
     StepPlan step{};
     ClusterFwdPlan cfwd{};
@@ -63,6 +65,20 @@ constexpr int kGridBwdCycles = 6500;
 constexpr int kExitsWord = 1000;  // of Engine::sync_words: CTAs of the running launch that have left (see leave_counters)
 
 TcState *state(Engine &e) { return static_cast<TcState *>(e.tc_state); }
+
+// The kernel of a launch of n steps.
+enum class Kind { Cluster, Tmem, Wide, Steps, Grid };
+Kind fwd_kind(const TcState &st, size_t n) {
+    if (st.cfwd.use) return Kind::Cluster;
+    if (n >= st.fwd_from && st.wide.use) return Kind::Wide;
+    if (n >= st.fwd_from && st.fwdtm.use) return Kind::Tmem;
+    return st.step.use && !st.fwdtm.use ? Kind::Steps : Kind::Grid;
+}
+Kind bwd_kind(const TcState &st, size_t n) {
+    if (st.cbwd.use) return Kind::Cluster;
+    if (st.bwdtm.use) return n >= st.bwd_from ? Kind::Tmem : Kind::Grid;
+    return st.step.use ? Kind::Steps : Kind::Grid;
+}
 
 struct PackJobs {
     PackJob job[kPackJobs];
@@ -150,6 +166,52 @@ bool supported(const flstm_engine_config &cfg) {
     return true;
 }
 
+// The kernels with W_hh in tensor memory for a shape, and the launches they take.  Moving W_hh there takes 2 us of a launch (BPTT
+// 2 to 4 us), which few steps do not repay; where the other kernels exist in a good form (H % 128 == 0, one batch tile) they
+// keep short launches.  Those then sum the halves of K apart, so that a sequence cut into ranges or segments of any length
+// gives the bits of one launch.  Calls of n steps in us, other kernels -> these:
+//   forward, n = 1 / 2 / 4 / 8 / 16 / 24:
+//     H = 1024, B = 32, one tile of 32   23.7 / 26.7 / 33.5 / 47.2 / 76.9 / 107.8 -> 24.7 / 28.8 / 34.9 / 47.2 / 73.6 / 102.0
+//     H = 2048, B = 40, one tile of 64   26.5 / 30.8 / 45.2 / 70.8 / 123.1 / 168.3 -> 28.8 / 32.9 / 45.6 / 71.8 / 121.7 / 164.4
+//     H = 2048, B = 256, tiles in turn   35.9 / 53.2 / 84.6 / 154 / 282 / 404 -> 37.2 / 48.7 / 71.9 / 125 / 214 / 297
+//   backward, n = 1 / 2 / 4 / 8 / 16 / 24:
+//     H = 1024, B = 64   58.7 / 63.9 / 75.9 / 97.2 / 138.3 / 179.7 -> 61.6 / 66.5 / 79.2 / 98.0 / 139.1 / 179.9
+//     H = 2048, B = 5    104.4 / 107.5 / 121.4 / 146.0 / 196.5 / 246.4 -> 107.4 / 111.1 / 120.6 / 141.2 / 182.5 / 220.8
+//     H = 1280, B = 60   76.4 / 85.1 / 98.5 / 130.9 / 187.5 / 257.2 -> 78.2 / 87.1 / 98.1 / 126.8 / 179.0 / 239.4
+//     tiles in turn, H = 1024, B = 140   70.7 / 81.5 / 104 / 149 / 238 / 324 -> 68.0 / 77.0 / 92.3 / 123 / 182 / 241
+static int choose_tmem(int B, int H, bool fwd, bool bwd, int sms, size_t smem_limit, bool check_device, TcState *st) {
+    const bool good = H % 128 == 0;
+    if (fwd) {
+        FLSTM_TRY(plan_fwd_tm(B, H, sms, smem_limit, &st->fwdtm));
+        // 33 to 64 sequences per batch group: the K halves make an UMMA of N = 128, which takes longer than the other
+        // kernel's of N = 64 (H = 512, B = 250: 4.15 against 3.97 us a step; H = 640, B = 130: 4.16 against 3.98), so that one
+        // stays where its weights are resident and a CTA has one batch tile; beyond that the gain per step is small
+        FwdPlan f{};
+        const bool single = plan_fwd(B, H, sms, smem_limit, &f) == FLSTM_OK && f.nt == 1, fits_one = st->fwdtm.use;
+        if (st->fwdtm.BT == 64 && single && f.resident && f.BT <= 64) st->fwdtm.use = false;
+        if (st->fwdtm.use && st->fwdtm.S == 2 && good && single) {
+            st->fwd_from = st->fwdtm.BT == 64 ? 12 : 5;
+            st->fwd = f;
+            st->fwd.halves = true;
+        }
+        if (!fits_one) {
+            FLSTM_TRY(plan_fwd_wide(B, H, sms, smem_limit, &st->wide));
+            if (st->wide.use) st->fwd_from = 2;
+        }
+    }
+    if (bwd) {
+        FLSTM_TRY(plan_bwd_tm(B, H, sms, smem_limit, &st->bwdtm, check_device));
+        BwdPlan b{};
+        if (st->bwdtm.use && good && st->bwdtm.nt == 1 && plan_bwd(B, H, sms, smem_limit, &b, check_device) == FLSTM_OK &&
+            b.nt == 1 && b.KS == 4) {
+            st->bwd_from = H <= 1024 ? 24 : 4;
+            st->bwd = b;
+            st->bwd.halves = true;
+        }
+    }
+    return FLSTM_OK;
+}
+
 int init(Engine &e) {
     TcState *st = new TcState();
     e.tc_state = st;
@@ -171,33 +233,15 @@ int init(Engine &e) {
         // the cross-layer wavefront would put two cooperative grids side by side
         const char *wave = std::getenv("FLSTM_WAVE_CHUNK");
         const bool wavefront = wave && std::atoi(wave) > 0;
-        // Moving W_hh into tensor memory takes 2 us of a launch (BPTT 4 us), which few steps do not repay; where the other kernels
-        // exist in a good form (H % 128 == 0) they keep engines made for short sequences.  A forward launch, us, T = 1 / 2 / 4 / 8:
-        // H = 1024, B = 64 18.5 / 22.6 / 30.2 / 45.2 -> 20.2 / 23.2 / 30.8 / 44.9;  H = 2048, B = 40 20.6 / 26.7 / 39.0 / 65.7 -> 22.7 /
-        // 28.8 / 41.3 / 66.5;  in turn, H = 1024, B = 256 22.6 / 30.8 / 49.2 / 82.8 -> 24.6 / 30.8 / 43.1 / 69.7.  BPTT at H = 1024,
-        // B = 32, T = 8 / 16: 76 / 111 -> 80 / 116.
-        const size_t steps = e.cfg.max_seq_len;
-        const bool good = H % 128 == 0;
-        if (!st->cfwd.use && !wavefront) {
-            FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &st->fwdtm));
-            // 33 to 64 sequences per batch group: the K halves make an UMMA of N = 128, which takes longer than the other
-            // kernel's of N = 64 (H = 512, B = 250: 4.15 against 3.97 us a step; H = 640, B = 130: 4.16 against 3.98), so that one
-            // stays where its weights are resident and a CTA has one batch tile; beyond that the gain per step is small
-            FwdPlan f{};
-            const bool one_tile = plan_fwd(B, H, st->sms, st->smem_limit, &f) == FLSTM_OK && f.resident && f.nt == 1 && f.BT <= 64;
-            const bool fits_one = st->fwdtm.use;
-            if (st->fwdtm.BT == 64 && one_tile) st->fwdtm.use = false;
-            if (st->fwdtm.S == 2 && good && f.nt == 1 && steps < (st->fwdtm.BT == 64 ? 32 : 5)) st->fwdtm.use = false;
-            if (!fits_one && steps > 1) FLSTM_TRY(plan_fwd_wide(B, H, st->sms, st->smem_limit, &st->wide));
-        }
-        if (e.cfg.training && !st->cbwd.use && !wavefront) {
-            FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &st->bwdtm, /*check_device=*/true));
-            if (good && st->bwdtm.nt == 1 && H <= 1024 && steps < 24) st->bwdtm.use = false;
-        }
+        if (!wavefront)
+            FLSTM_TRY(choose_tmem(B, H, !st->cfwd.use, e.cfg.training && !st->cbwd.use, st->sms, st->smem_limit, /*check_device=*/true, st));
     }
-    const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use && !st->wide.use, grid_bwd = e.cfg.training && !st->cbwd.use && !st->bwdtm.use;
+    const bool tm_fwd = st->fwdtm.use || st->wide.use;
+    const bool grid_fwd = !st->cfwd.use && !tm_fwd, grid_bwd = e.cfg.training && !st->cbwd.use && !st->bwdtm.use;
+    const bool short_wide = st->wide.use && st->fwd_from > 1;
     st->bwd_ok = e.cfg.training != 0;
-    if (grid_fwd || grid_bwd) FLSTM_TRY(plan_step(B, H, st->sms, st->smem_limit, &st->step));
+    if (grid_fwd || grid_bwd || short_wide) FLSTM_TRY(plan_step(B, H, st->sms, st->smem_limit, &st->step));
+    if (short_wide && !st->step.use && plan_fwd(B, H, st->sms, st->smem_limit, &st->fwd) != FLSTM_OK) st->fwd_from = 0;
     if (st->step.use && grid_bwd) {
         const size_t n = e.layers.size() * (size_t)st->step.splits * e.cfg.batch * e.cfg.hidden_size;
         e.fixed.want(&st->dh_parts, n * sizeof(float));
@@ -207,7 +251,7 @@ int init(Engine &e) {
     if (e.cfg.training) {  // a split GEMM has at most one 128 x 128 tile per SM
         st->dw_floats = (size_t)st->sms * 128 * 128;
         // one per layer where the cross-layer wavefront can run two layers' GEMMs at once
-        st->dw_layers = st->step.use ? e.layers.size() : 1;
+        st->dw_layers = st->step.use && !tm_fwd && !st->bwdtm.use ? e.layers.size() : 1;
         e.fixed.want(&st->dw_parts, st->dw_layers * st->dw_floats * sizeof(float));
     }
     st->layers.resize(e.layers.size());
@@ -233,18 +277,18 @@ int on_capacity_change(Engine &e) {
     for (size_t li = 0; li < e.layers.size(); ++li) {
         auto &l = e.layers[li];
         auto &t = st->layers[li];
-        const bool grid_fwd = !st->cfwd.use && !st->fwdtm.use && !st->wide.use, tm_bwd = e.cfg.training && l.dg && st->bwdtm.use;
-        const bool grid_bwd = e.cfg.training && l.dg && !st->cbwd.use && !st->bwdtm.use;
-        if (!grid_fwd && !grid_bwd && !st->fwdtm.use && !st->wide.use && !tm_bwd) continue;  // the cluster kernels use plain loads
+        const bool bwd = e.cfg.training && l.dg;
+        const bool grid_fwd = st->fwd.BT > 0, grid_bwd = bwd && st->bwd.BT > 0, step_bwd = bwd && bwd_kind(*st, 1) == Kind::Steps;
+        if (st->cfwd.use && (!e.cfg.training || st->cbwd.use)) continue;  // the cluster kernels use plain loads
         FLSTM_TRY(make_tensor_map_2d(&t.tm_w, l.w_hh, 4 * H, H, H, 64, 64, true));
-        if (tm_bwd) FLSTM_TRY(make_bwd_tm_maps(&t.dg_tm, st->bwdtm, l.dg, dg_steps, B, H));
+        if (bwd && st->bwdtm.use) FLSTM_TRY(make_bwd_tm_maps(&t.dg_tm, st->bwdtm, l.dg, dg_steps, B, H));
         if (st->wide.use) {
             FLSTM_TRY(make_tensor_map_gate_rows(&t.tm_ws, l.w_hh, H));
-            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->wide.BT / 2, 2));
+            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->wide.BT / 2, 2));
         }
         if (st->fwdtm.use) {
-            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->fwdtm.S * st->fwdtm.BT / 2, st->fwdtm.ch));
-            FLSTM_TRY(make_tensor_map_3d(&t.tm_g, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwdtm.BT, 64, false));
+            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->fwdtm.S * st->fwdtm.BT / 2, st->fwdtm.ch));
+            FLSTM_TRY(make_tensor_map_3d(&t.tm_g_tm, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwdtm.BT, 64, false));
             if (st->fwdtm.wstages) FLSTM_TRY(make_tensor_map_chunked(&t.tm_ws, l.w_hh, 1, 4 * H, H, 128, kFwdTmGroup));
         }
         if (st->step.use) {
@@ -253,9 +297,8 @@ int on_capacity_change(Engine &e) {
             FLSTM_TRY(make_tensor_map_3d_tile(&t.tm_g_ep, l.gates, 2, cap, B, 4 * H, 32, 64));
             FLSTM_TRY(make_tensor_map_3d_tile(&t.tm_c_ep, l.cs, 4, cap + 1, B, H, 32, 16));
             FLSTM_TRY(make_tensor_map_3d_tile(&t.tm_h_ep, l.hs, 2, cap + 1, B, H, 32, 16));
-            if (grid_bwd)
+            if (step_bwd)
                 FLSTM_TRY(make_tensor_map_3d(&t.tm_dg3, l.dg, dg_steps, B, 4 * H, 4 * H, B * 4 * H, 128, 64, true));
-            continue;
         }
         if (grid_fwd) {
             FLSTM_TRY(make_tensor_map_chunked(&t.tm_h, l.hs, cap + 1, B, H, st->fwd.pair ? st->fwd.BT / 2 : st->fwd.BT, st->fwd.ch));
@@ -307,21 +350,26 @@ int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs) {
     return !backward && st->step.fwd_persistent && wavefront_chunk(e, (size_t)-1) == 0 ? FLSTM_PATH_GRID : FLSTM_PATH_STEPS;
 }
 
-void recurrent_kernel(const Engine &e, bool backward, size_t, flstm_kernel_info *out) {
-    const TcState *st = static_cast<const TcState *>(e.tc_state);
-    const bool steps_path = st->step.use && (backward || !st->step.fwd_persistent || wavefront_chunk(e, (size_t)-1) != 0);
+void recurrent_kernel(const Engine &e, bool backward, size_t steps, flstm_kernel_info *out) {
+    const TcState &st = *static_cast<const TcState *>(e.tc_state);
     if (!backward) {
-        if (st->cfwd.use) *out = {"cluster_fwd_kernel", 0, st->cfwd.seqs, 1, 0, 0};
-        else if (st->wide.use) *out = {"lstm_fwd_wide_kernel", 0, st->wide.BT, st->wide.nt, st->wide.ngroups, 0};
-        else if (st->fwdtm.use) *out = {"lstm_fwd_tm_kernel", 0, st->fwdtm.BT, 1, st->fwdtm.ngroups, st->fwdtm.wstages > 0};
-        else if (steps_path) *out = {"step_kernel", 1, 0, 1, 0, 1};
-        else if (st->step.use) *out = {"wide_fwd_kernel", 0, 0, 1, 0, 1};
-        else *out = {"lstm_fwd_kernel", 0, st->fwd.BT, st->fwd.nt, st->fwd.ngroups, !st->fwd.resident};
+        switch (fwd_kind(st, steps)) {
+            case Kind::Cluster: *out = {"cluster_fwd_kernel", 0, st.cfwd.seqs, 1, 0, 0}; break;
+            case Kind::Wide: *out = {"lstm_fwd_wide_kernel", 0, st.wide.BT, st.wide.nt, st.wide.ngroups, 0}; break;
+            case Kind::Tmem: *out = {"lstm_fwd_tm_kernel", 0, st.fwdtm.BT, 1, st.fwdtm.ngroups, st.fwdtm.wstages > 0}; break;
+            case Kind::Steps:
+                if (st.step.fwd_persistent && wavefront_chunk(e, (size_t)-1) == 0) *out = {"wide_fwd_kernel", 0, 0, 1, 0, 1};
+                else *out = {"step_kernel", 1, 0, 1, 0, 1};
+                break;
+            case Kind::Grid: *out = {"lstm_fwd_kernel", 0, st.fwd.BT, st.fwd.nt, st.fwd.ngroups, !st.fwd.resident}; break;
+        }
     } else {
-        if (st->cbwd.use) *out = {"cluster_bwd_kernel", 0, st->cbwd.seqs, 1, 0, 0};
-        else if (st->bwdtm.use) *out = {"lstm_bwd_tm_kernel", 0, st->bwdtm.BT, st->bwdtm.nt, st->bwdtm.ngroups, 0};
-        else if (steps_path) *out = {"step_kernel", 2, 0, 1, 0, 1};  // step_bwd_pointwise_kernel and the GEMM
-        else *out = {"lstm_bwd_kernel", 0, st->bwd.BT, st->bwd.nt, st->bwd.ngroups, !st->bwd.resident};
+        switch (bwd_kind(st, steps)) {
+            case Kind::Cluster: *out = {"cluster_bwd_kernel", 0, st.cbwd.seqs, 1, 0, 0}; break;
+            case Kind::Steps: *out = {"step_kernel", 2, 0, 1, 0, 1}; break;  // step_bwd_pointwise_kernel and the GEMM
+            case Kind::Grid: *out = {"lstm_bwd_kernel", 0, st.bwd.BT, st.bwd.nt, st.bwd.ngroups, !st.bwd.resident}; break;
+            default: *out = {"lstm_bwd_tm_kernel", 0, st.bwdtm.BT, st.bwdtm.nt, st.bwdtm.ngroups, 0}; break;
+        }
     }
 }
 
@@ -337,7 +385,8 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     FLSTM_TRY(gemm(e.cfg.dtype, e.cfg.dtype, n * B, 4 * H, l.in_size, byte_ptr(x_l) + t0 * B * l.in_size * es, l.in_size, false,
                    l.w_ih, l.in_size, false, byte_ptr(l.gates) + t0 * B * 4 * H * es, 4 * H, l.bias, 0, err, st->sms, s));
     size_t m1 = e.timer.mark(s);
-    if (st->cfwd.use) {
+    const Kind kind = fwd_kind(*st, n);
+    if (kind == Kind::Cluster) {
         ClusterFwdParams cp{};
         cp.w_hh = l.w_hh;
         cp.cs = l.cs;
@@ -362,7 +411,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
         e.launches += 2;
         return FLSTM_OK;
     }
-    if (st->step.use && !st->fwdtm.use && !st->wide.use) {
+    if (kind == Kind::Steps) {
         CUtensorMap tm_y;
         if (y_out) FLSTM_TRY(make_tensor_map_3d_tile(&tm_y, y_out, 2, t1, B, H, 32, 16));
         const StepFwdMaps maps{&t.tm_hs3, &t.tm_wstep, &t.tm_g_ep, &t.tm_c_ep, &t.tm_h_ep, y_out ? &tm_y : nullptr};
@@ -424,8 +473,8 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.trace_steps = e.trace_steps;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    if (st->wide.use) FLSTM_TRY(lstm_forward_wide(e.cfg.dtype, st->wide, t.tm_ws, t.tm_h, p, s));
-    else if (st->fwdtm.use) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h, t.tm_g, p, s));
+    if (kind == Kind::Wide) FLSTM_TRY(lstm_forward_wide(e.cfg.dtype, st->wide, t.tm_ws, t.tm_h_tm, p, s));
+    else if (kind == Kind::Tmem) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h_tm, t.tm_g_tm, p, s));
     else FLSTM_TRY(lstm_forward_persistent(e.cfg.dtype, st->fwd, t.tm_w, t.tm_h, t.tm_g, p, s));
     size_t m2 = e.timer.mark(s);
     e.timer.span(PH_PROJ, m0, m1);
@@ -576,7 +625,8 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     // with activation checkpoints `T` and the range are segment-local; only the segment that starts the sequence
     // finishes the recurrence (dh0 / dc0) and the layer's gradients
     const bool finalize = t0 == 0 && (!e.seg.active || e.seg.final_segment);
-    if (st->cbwd.use) {
+    const Kind kind = bwd_kind(*st, n);
+    if (kind == Kind::Cluster) {
         ClusterBwdParams cp{};
         cp.w_hh = l.w_hh;
         cp.cs = l.cs;
@@ -601,7 +651,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
         cp.extra_arrivals = e.selftest_missing_arrivals;
         FLSTM_TRY(lstm_backward_cluster(e.cfg.dtype, st->cbwd, cp, s));
         e.launches += 1;
-    } else if (st->step.use && !st->bwdtm.use) {
+    } else if (kind == Kind::Steps) {
         FLSTM_TRY(backward_steps(e, li, T, t0, t1, dy_l, dhn_l, dcn_l, dh0_l, dc0_l, finalize, s));
     } else {
     BwdParams p{};
@@ -627,7 +677,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.H = (int)H;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    if (st->bwdtm.use) FLSTM_TRY(lstm_backward_tm(e.cfg.dtype, st->bwdtm, t.tm_w, t.dg_tm, p, s));
+    if (kind == Kind::Tmem) FLSTM_TRY(lstm_backward_tm(e.cfg.dtype, st->bwdtm, t.tm_w, t.dg_tm, p, s));
     else FLSTM_TRY(lstm_backward_persistent(e.cfg.dtype, st->bwd, t.tm_w, t.tm_dg, p, s));
     e.launches += 1;
     }

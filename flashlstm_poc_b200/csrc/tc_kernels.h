@@ -33,6 +33,7 @@ struct FwdPlan {
     int ch;        // 64-wide K chunks per ring stage (one TMA copy each)
     bool resident; // W_hh slice stays in shared memory for the whole sequence
     bool pair;     // neighbouring row-tile CTAs form cta_group::2 pairs; the h map then has BT/2 rows per box
+    bool halves;   // the two halves of K are summed apart and added last, the order of the kernel that takes longer launches
     int smem_bytes;
     int grid;
 };
@@ -57,7 +58,7 @@ struct FwdParams {
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path: the step barrier waits for this many arrivals nobody makes
     // filled by the launcher from the plan
-    int rt, cta_rows, nt, stages, ch;
+    int rt, cta_rows, nt, stages, ch, halves;
     uint32_t idesc;
 };
 
@@ -118,6 +119,7 @@ struct BwdPlan {
     int ngroups, nt, stages;
     int ch;        // 64-wide K chunks per ring stage (one TMA copy each)
     bool resident;
+    bool halves;   // as in FwdPlan, of a CTA's part of K
     int smem_bytes;
     int grid;
 };
@@ -140,7 +142,7 @@ struct BwdParams {
     int s0, s1;           // reverse iterations [s0, s1) of this launch; iteration s is time T-1-s, s == T writes dh0/dc0
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path (see FwdParams)
-    int jt, nt, stages, ch;
+    int jt, nt, stages, ch, halves;
     uint32_t idesc;
 };
 

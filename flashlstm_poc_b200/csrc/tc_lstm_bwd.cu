@@ -93,6 +93,8 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     const int j = cl % p.jt;                 // unit tile: hidden units [64j, 64j+64)
     unsigned int *counter = p.counters + ng;
     constexpr int kTmemCols = (2 * BT < 32) ? 32 : 2 * BT;
+    // p.halves: a second pair of accumulators behind the first takes the second half of this CTA's K range
+    const uint32_t tmem_cols = p.halves ? 2 * kTmemCols : kTmemCols;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < L.stages; ++i) {
@@ -113,7 +115,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         tma_prefetch_desc(&tm_dg);
     }
     if (warp == 5) {
-        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_alloc(tmem_slot, tmem_cols);
         tmem_relinquish();
     }
     tcgen05_fence_before();
@@ -216,13 +218,14 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             uint32_t phase = 0;
             const uint32_t s_w_u32 = smem_u32(s_w), idesc = p.idesc;
             const uint32_t items = (uint32_t)(p.s1 - (p.s0 > 1 ? p.s0 : 1)) * nt_count;
+            const int half = p.halves ? KCper / 2 : KCper;  // the chunk that starts the second accumulator
             int last_commit = -1;
             for (uint32_t wi = 0; wi < items && ok; ++wi) {
                 const int buf = wi & 1;
                 ok = mbar_wait(&tempty[buf], ((wi >> 1) & 1) ^ 1, abort_w, wait_ns);
                 if (!ok) break;
                 tcgen05_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * BT;
+                uint32_t d_tmem = tmem_base + buf * BT;
                 for (int ld = 0; ld < NLOAD; ++ld) {
                     ok = mbar_wait(&full[stage], phase, abort_w, wait_ns);
                     if (!ok) break;
@@ -239,6 +242,10 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     uint32_t acc = ld != 0;
 #pragma unroll 4
                     for (int c = 0; c < CH; ++c) {
+                        if (ld * CH + c == half) {
+                            d_tmem += kTmemCols;
+                            acc = 0u;
+                        }
                         umma_f16(d_tmem, dw, dd, idesc, acc);
                         umma_f16(d_tmem, dw + 128, dd + 2, idesc, 1u);
                         umma_f16(d_tmem, dw + 256, dd + 4, idesc, 1u);
@@ -350,8 +357,16 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 #pragma unroll
                         for (int c0 = 0; c0 < BT; c0 += 32) {
                             uint32_t acc[32];
-                            tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(warp * 32) << 16) + buf * BT + c0, acc);
+                            const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + buf * BT + c0;
+                            tmem_ld_32x32b_x32(taddr, acc);
                             tmem_ld_wait();
+                            if (p.halves) {
+                                uint32_t more[32];
+                                tmem_ld_32x32b_x32(taddr + kTmemCols, more);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(more[i]));
+                            }
                             if (lane < 16) {
                                 const int row = warp * 16 + lane;        // unit within the tile
                                 const uint32_t owner = row / UPO, lu = row % UPO;
@@ -475,7 +490,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             while (global_timer_ns() - t0 < 20000ull) {}
         }
     }
-    if (warp == 5) tmem_dealloc(tmem_base, kTmemCols);
+    if (warp == 5) tmem_dealloc(tmem_base, tmem_cols);
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / (p.jt * KS), p.exits);
 }
@@ -635,6 +650,7 @@ int plan_bwd(int B, int H, int sms, size_t smem_limit, BwdPlan *plan, bool check
     plan->ch = ch;
     plan->BT = BT;
     plan->KS = KS;
+    plan->halves = false;
     plan->jt = jt;
     plan->ngroups = ngroups;
     plan->nt = nt;
@@ -669,6 +685,7 @@ int lstm_backward_persistent(int dtype, const BwdPlan &plan, const CUtensorMap &
     p.nt = plan.nt;
     p.stages = plan.stages;
     p.ch = plan.ch;
+    p.halves = plan.halves ? 1 : 0;
     p.idesc = umma_idesc_f16(64, plan.BT, bf16 ? 1 : 0, /*A MN-major*/ 1, /*B K-major*/ 0);
 #define FLSTM_BWD_CASE(BT_, KS_, RES_)                                                                         \
     if (plan.BT == BT_ && plan.KS == KS_ && plan.resident == RES_)                                             \

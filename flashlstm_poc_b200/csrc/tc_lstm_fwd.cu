@@ -105,6 +105,8 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     unsigned int *counter = p.counters + ng;
     constexpr int kAccCols = PAIR ? BT / 2 : BT;  // tensor-memory columns of one accumulator
     constexpr int kTmemCols = (2 * kAccCols < 32) ? 32 : 2 * kAccCols;
+    // p.halves: a second pair of accumulators behind the first takes the second half of K, and the epilogue adds the two
+    const uint32_t tmem_cols = p.halves ? 2 * kTmemCols : kTmemCols;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     const bool leader = rank == 0;
 
@@ -128,10 +130,10 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     }
     if (warp == 5) {
         if (PAIR) {
-            tmem_alloc_pair(tmem_slot, kTmemCols);
+            tmem_alloc_pair(tmem_slot, tmem_cols);
             tmem_relinquish_pair();
         } else {
-            tmem_alloc(tmem_slot, kTmemCols);
+            tmem_alloc(tmem_slot, tmem_cols);
             tmem_relinquish();
         }
     }
@@ -269,6 +271,7 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             const uint32_t s_w_u32 = smem_u32(s_w), idesc = p.idesc;
             const uint32_t empty_l = smem_u32(empty), tfull_l = smem_u32(tfull);
             const uint32_t total_items = (uint32_t)p.T * items_per_step;
+            const int half = p.halves ? KC / 2 : KC;  // the chunk that starts the second accumulator
             int last_commit = -1;
             for (uint32_t it = 0; it < total_items && ok; ++it, ++wi) {
                 const int r = (it % items_per_step) / nt_count;
@@ -277,7 +280,7 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                           : mbar_wait(&tempty[buf], ((wi >> 1) & 1) ^ 1, abort_w, wait_ns);
                 if (!ok) break;
                 tcgen05_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * kAccCols;
+                uint32_t d_tmem = tmem_base + buf * kAccCols;
                 for (int ld = 0; ld < NLOAD; ++ld) {
                     ok = mbar_wait(&full[stage], phase, abort_w, wait_ns);
                     if (!ok) break;
@@ -293,6 +296,10 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     uint32_t acc = ld != 0;
 #pragma unroll 4
                     for (int c = 0; c < CH; ++c) {
+                        if (ld * CH + c == half) {
+                            d_tmem += kTmemCols;
+                            acc = 0u;
+                        }
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             if (PAIR) umma_f16_pair(d_tmem, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
@@ -376,8 +383,16 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 #pragma unroll
                         for (int c0 = 0; c0 < BT; c0 += 32) {
                             uint32_t acc[32];
-                            tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(warp * 32) << 16) + buf * BT + c0, acc);
+                            const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + buf * BT + c0;
+                            tmem_ld_32x32b_x32(taddr, acc);
                             tmem_ld_wait();
+                            if (p.halves) {
+                                uint32_t more[32];
+                                tmem_ld_32x32b_x32(taddr + kTmemCols, more);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(more[i]));
+                            }
                             if (lane < 16) {
                                 float4 *dst = reinterpret_cast<float4 *>(ex + (warp * 16 + lane) * EXS + c0);
 #pragma unroll
@@ -402,6 +417,14 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                             if (W16 == 16) tmem_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(&acc[0]));
                             else tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&acc[0]));
                             tmem_ld_wait();
+                            if (p.halves) {
+                                uint32_t more[W16];
+                                if (W16 == 16) tmem_ld_32x32b_x16(taddr + kTmemCols, *reinterpret_cast<uint32_t(*)[16]>(&more[0]));
+                                else tmem_ld_32x32b_x32(taddr + kTmemCols, *reinterpret_cast<uint32_t(*)[32]>(&more[0]));
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int i = 0; i < W16; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(more[i]));
+                            }
                             float4 *dst = reinterpret_cast<float4 *>(ex + row * EXS + seq0 + c0);
 #pragma unroll
                             for (int i = 0; i < W16 / 4; ++i)
@@ -476,9 +499,9 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             while (global_timer_ns() - t0 < kAbortDrainNs) {}
         }
         cluster_sync_all();  // the peer's shared and tensor memory stay valid until the leader's last UMMA is consumed
-        if (warp == 5) tmem_dealloc_pair(tmem_base, kTmemCols);
+        if (warp == 5) tmem_dealloc_pair(tmem_base, tmem_cols);
     } else if (warp == 5) {
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc(tmem_base, tmem_cols);
     }
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / p.cta_rows, p.exits);
@@ -617,6 +640,7 @@ int plan_fwd(int B, int H, int sms, size_t smem_limit, FwdPlan *plan) {
     }
     plan->ch = ch;
     plan->pair = pair;
+    plan->halves = false;
     plan->BT = BT;
     plan->rt = rt;
     plan->cta_rows = cta_rows;
@@ -637,6 +661,7 @@ int lstm_forward_persistent(int dtype, const FwdPlan &plan, const CUtensorMap &t
     p.nt = plan.nt;
     p.stages = plan.stages;
     p.ch = plan.ch;
+    p.halves = plan.halves ? 1 : 0;
     p.idesc = umma_idesc_f16(plan.pair ? 128 : 64, plan.BT, bf16 ? 1 : 0, 0, 0);
 #define FLSTM_FWD_CASE(BT_, RES_)                                                                                  \
     if (plan.BT == BT_ && plan.resident == RES_) {                                                                 \

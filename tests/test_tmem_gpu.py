@@ -117,3 +117,56 @@ def check_kernels(table):
 def test_which_kernels_the_shapes_run():
     assert set(SHAPES) <= {s[:4] for s in KERNELS}
     check_kernels(KERNELS)
+
+
+@pytest.mark.parametrize("dtype,B,H,short_fwd,long_fwd,short_bwd,long_bwd", [
+    ("f16", 32, 1024, "lstm_fwd_kernel", "lstm_fwd_tm_kernel", "lstm_bwd_kernel", "lstm_bwd_tm_kernel"),
+    ("bf16", 64, 1024, "lstm_fwd_kernel", "lstm_fwd_tm_kernel", "lstm_bwd_kernel", "lstm_bwd_tm_kernel"),
+    ("bf16", 40, 768, "lstm_fwd_kernel", "lstm_fwd_tm_kernel", "lstm_bwd_kernel", "lstm_bwd_tm_kernel"),
+    ("f16", 33, 1152, "lstm_fwd_kernel", "lstm_fwd_tm_kernel", "lstm_bwd_tm_kernel", "lstm_bwd_tm_kernel"),
+    ("f16", 32, 1280, "lstm_fwd_kernel", "lstm_fwd_tm_kernel", "lstm_bwd_kernel", "lstm_bwd_tm_kernel"),
+    ("bf16", 40, 2048, "lstm_fwd_kernel", "lstm_fwd_tm_kernel", "lstm_bwd_kernel", "lstm_bwd_tm_kernel"),
+    ("f16", 140, 1024, "lstm_fwd_kernel", "lstm_fwd_wide_kernel", "lstm_bwd_tm_kernel", "lstm_bwd_tm_kernel"),
+    ("bf16", 256, 2048, "wide_fwd_kernel", "lstm_fwd_wide_kernel", "step_kernel", "step_kernel"),
+])
+def test_the_length_of_a_launch_chooses_its_kernel_and_not_its_bits(dtype, B, H, short_fwd, long_fwd, short_bwd, long_bwd, monkeypatch):
+    """Short launches run other kernels than long ones, whatever length the engine was made for, and every way to cut a sequence
+    gives the same bits."""
+    monkeypatch.setenv("FLSTM_CLUSTER", "0")
+    I, T = 64, 40
+    w = Workload("t", dtype, 1, I, H, B, T, seed=54, state_std=0.3)
+    inp = make_inputs(w)
+    dev, td = torch.device("cuda", 0), TORCH_DTYPES[dtype]
+    params = [p[0].to(dev) for p in (inp.w_ih, inp.w_hh, inp.b_ih, inp.b_hh)]
+    x, h0, c0, dy = (t.to(dev, td) for t in (inp.x, inp.h0, inp.c0, inp.dy))
+
+    def made_for(steps):
+        eng = Engine(dtype, 1, B, I, H, steps, device=dev)
+        eng.set_weights(0, *params)
+        return eng
+
+    def whole(eng):
+        out = [t.clone() for t in eng.forward(x, h0, c0)]
+        out += [t.clone() for t in eng.backward(dy)]
+        return out + [t.clone() for t in eng.grads(0)]
+
+    long = made_for(T)
+    want = whole(long)
+    short = made_for(2)
+    short.forward(x[:2].contiguous(), h0, c0)
+    for eng in (long, short):
+        assert eng.recurrent_kernel(1)["name"] == short_fwd and eng.recurrent_kernel(T)["name"] == long_fwd
+        assert eng.recurrent_kernel(1, backward=True)["name"] == short_bwd
+        assert eng.recurrent_kernel(T, backward=True)["name"] == long_bwd
+    for a, b in zip(want, whole(short)):  # the engine has grown
+        assert torch.equal(a, b)
+    short.close()
+    got = [torch.zeros_like(t) for t in want[:6]]
+    for t0, t1 in ((0, 1), (1, 4), (4, 36), (36, 40)):
+        long.forward_range_into(T, t0, t1, x, h0, c0, *got[:3])
+    for t0, t1 in ((39, 40), (30, 39), (5, 30), (0, 5)):
+        long.backward_range_into(T, t0, t1, dy, None, None, *got[3:])
+    torch.cuda.synchronize()
+    for a, b in zip(want, got + list(long.grads(0))):
+        assert torch.equal(a, b)
+    long.close()

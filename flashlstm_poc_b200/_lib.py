@@ -16,7 +16,7 @@ ENGINE_SYMBOLS = [
     "flstm_engine_backward", "flstm_engine_forward_range", "flstm_engine_backward_range", "flstm_engine_grad_ptrs", "flstm_engine_grad_buffer", "flstm_engine_export_grads", "flstm_engine_cache_ptrs",
     "flstm_engine_set_cell_io_f32", "flstm_engine_backend", "flstm_engine_path", "flstm_engine_kernel", "flstm_comm_unique_id", "flstm_engine_attach_comm",
     "flstm_engine_enable_timing", "flstm_engine_phase_ms", "flstm_engine_launch_count", "flstm_tc_gemm",
-    "flstm_engine_enable_trace", "flstm_engine_read_trace", "flstm_bias_grad", "flstm_tc_plan", "flstm_engine_wait", "flstm_engine_abort_comm",
+    "flstm_engine_enable_trace", "flstm_engine_read_trace", "flstm_bias_grad", "flstm_tc_plan", "flstm_tmem_plan", "flstm_engine_wait", "flstm_engine_abort_comm",
                   "flstm_engine_set_recompute_interval", "flstm_engine_workspace_bytes",
     "flstm_bias_grad_static", "flstm_engine_set_wait_limit", "flstm_engine_selftest_missing_arrivals",
     "flstm_engine_backward_segment",
@@ -49,6 +49,13 @@ class TcPlanInfo(ctypes.Structure):
         "bwd_batch_tile", "bwd_cluster_size", "bwd_grid", "bwd_batch_groups", "bwd_tiles_per_group",
         "bwd_stages", "bwd_chunks_per_stage", "bwd_weights_resident", "bwd_smem_bytes",
         "step_path", "step_bn_fwd", "step_bn_bwd", "step_splits", "step_pair", "fwd_pair", "step_fwd_pair")]
+
+
+class TmemPlanInfo(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int) for n in (
+        "fwd_kernel", "fwd_from_steps", "fwd_k_halves", "fwd_batch_tile", "fwd_batch_groups", "fwd_tiles_in_turn",
+        "fwd_weights_streamed", "fwd_grid", "fwd_smem_bytes", "bwd_kernel", "bwd_from_steps", "bwd_batch_tile",
+        "bwd_batch_groups", "bwd_tiles_in_turn", "bwd_grid", "bwd_smem_bytes")]
 
 
 class KernelInfo(ctypes.Structure):
@@ -114,6 +121,7 @@ def load() -> ctypes.CDLL:
     lib.flstm_engine_enable_trace.argtypes = [vp, ci]
     lib.flstm_engine_read_trace.argtypes = [vp, vp, sz]
     lib.flstm_tc_plan.argtypes = [sz, sz, ci, ci, sz, ctypes.POINTER(TcPlanInfo)]
+    lib.flstm_tmem_plan.argtypes = [sz, sz, ci, ci, sz, ctypes.POINTER(TmemPlanInfo)]
     lib.flstm_engine_wait.argtypes = [vp, vp, ctypes.c_uint]
     lib.flstm_engine_abort_comm.argtypes = [vp]
     lib.flstm_engine_backward_segment.argtypes = [vp, sz, ci, ci] + [vp] * 10

@@ -830,6 +830,43 @@ extern "C" int flstm_tc_plan(size_t batch, size_t hidden_size, int training, int
     return FLSTM_OK;
 }
 
+extern "C" int flstm_tmem_plan(size_t batch, size_t hidden_size, int training, int sm_count, size_t smem_limit,
+                               flstm_tmem_plan_info *out) {
+    using namespace flstm_b200;
+    if (!out || sm_count < 1) return set_error(FLSTM_ERR_INVALID, "bad argument");
+    *out = flstm_tmem_plan_info{};
+    tc::TcState st;
+    FLSTM_TRY(tc::choose_tmem((int)batch, (int)hidden_size, true, training != 0, sm_count, smem_limit, /*check_device=*/false, &st));
+    if (st.wide.use) {
+        out->fwd_kernel = 2;
+        out->fwd_batch_tile = st.wide.BT;
+        out->fwd_batch_groups = st.wide.ngroups;
+        out->fwd_tiles_in_turn = st.wide.nt;
+        out->fwd_grid = st.wide.grid;
+        out->fwd_smem_bytes = st.wide.smem_bytes;
+    } else if (st.fwdtm.use) {
+        out->fwd_kernel = 1;
+        out->fwd_k_halves = st.fwdtm.S == 2;
+        out->fwd_batch_tile = st.fwdtm.BT;
+        out->fwd_batch_groups = st.fwdtm.ngroups;
+        out->fwd_tiles_in_turn = 1;
+        out->fwd_weights_streamed = st.fwdtm.wstages > 0;
+        out->fwd_grid = st.fwdtm.grid;
+        out->fwd_smem_bytes = st.fwdtm.smem_bytes;
+    }
+    out->fwd_from_steps = (int)st.fwd_from;
+    if (st.bwdtm.use) {
+        out->bwd_kernel = 1;
+        out->bwd_batch_tile = st.bwdtm.BT;
+        out->bwd_batch_groups = st.bwdtm.ngroups;
+        out->bwd_tiles_in_turn = st.bwdtm.nt;
+        out->bwd_grid = st.bwdtm.grid;
+        out->bwd_smem_bytes = st.bwdtm.smem_bytes;
+        out->bwd_from_steps = (int)st.bwd_from;
+    }
+    return FLSTM_OK;
+}
+
 extern "C" int flstm_tc_gemm(int dtype, int out_dtype, size_t M, size_t N, size_t K, const void *A, const void *B,
                              void *D, size_t ldd, const float *bias, int layout, void *stream) {
     using namespace flstm_b200;

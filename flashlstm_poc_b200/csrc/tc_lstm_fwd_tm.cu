@@ -539,6 +539,12 @@ int launch_one(const CUtensorMap &tw, const CUtensorMap &tws, const CUtensorMap 
 }  // namespace
 
 // ------------------------------------------------------------------ host side
+// The forms that lstm_forward_tm has kernels for: with the K halves nothing is streamed, without them always something (on the
+// widths that take either on 148 SMs; a GPU with fewer may plan others, and those stay with the other kernels).
+static bool has_kernel(const FwdTmPlan &pl) {
+    return pl.S == 2 ? pl.wstages == 0 && (pl.BT == 32 || pl.BT == 64) : pl.wstages > 0 && (pl.BT == 16 || pl.BT == 32 || pl.BT == 64);
+}
+
 int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
     *plan = FwdTmPlan{};
     if (H % 64 != 0 || H < 64 || smem_limit < 160 * 1024) return FLSTM_OK;
@@ -583,6 +589,7 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
     // stream) may share its SM; two grids that each held what the other's CTAs were waiting for would run into their limits
     pl.smem_bytes = (int)smem_limit;
     pl.grid = pl.cta_rows * pl.ngroups;
+    if (!has_kernel(pl)) return FLSTM_OK;
     pl.use = true;
     *plan = pl;
     return FLSTM_OK;

@@ -238,9 +238,21 @@ typedef struct {
     int step_fwd_pair; /* wide batches: the all-steps forward kernel runs on CTA pairs (256-sequence tiles) */
 } flstm_tc_plan_info;
 /* (Engines try the cluster-resident kernels first where hidden_size <= 768, see flstm_engine_path, and then the kernels that
- * hold W_hh in tensor memory, which this function does not describe; FLSTM_TMEM=0 switches those off.) */
+ * hold W_hh in tensor memory, flstm_tmem_plan; what this function describes runs the launches that neither takes.) */
 int flstm_tc_plan(size_t batch, size_t hidden_size, int training, int sm_count, size_t smem_limit,
                   flstm_tc_plan_info *out);
+
+/* The same for the kernels that hold W_hh in tensor memory (FLSTM_TMEM=0 switches them off), where the cluster-resident ones do
+ * not run.  The cluster occupancy of a device is not looked at: an engine may get fewer batch groups for the BPTT. */
+typedef struct {
+    int fwd_kernel;     /* 0: none, 1: lstm_fwd_tm_kernel, 2: lstm_fwd_wide_kernel */
+    int fwd_from_steps; /* launches of fewer steps run on the kernels of flstm_tc_plan */
+    int fwd_k_halves;   /* lstm_fwd_tm_kernel: K is split over the halves of the tensor memory's lanes */
+    int fwd_batch_tile, fwd_batch_groups, fwd_tiles_in_turn, fwd_weights_streamed, fwd_grid, fwd_smem_bytes;
+    int bwd_kernel;     /* 0: none, 1: lstm_bwd_tm_kernel */
+    int bwd_from_steps, bwd_batch_tile, bwd_batch_groups, bwd_tiles_in_turn, bwd_grid, bwd_smem_bytes;
+} flstm_tmem_plan_info;
+int flstm_tmem_plan(size_t batch, size_t hidden_size, int training, int sm_count, size_t smem_limit, flstm_tmem_plan_info *out);
 
 /* The dense-contraction building block of the path on the tcgen05 tensor cores, exported for
  * unit tests and profiling: D[M,N] = A B^T (+ bias[N]) with f16/bf16 operands (`dtype`) and fp32

@@ -115,3 +115,46 @@ def test_unsupported_shapes_are_reported(lib):
     assert st == 4 and b"multiple of 64" in lib.flstm_last_error()
     st, _ = plan(lib, 8, 1024, smem=16 * 1024)  # a machine with too little shared memory
     assert st == 4
+
+
+def tmem_plan(lib, B, H, training=1, sms=SMS, smem=SMEM):
+    info = _lib.TmemPlanInfo()
+    assert lib.flstm_tmem_plan(B, H, training, sms, smem, ctypes.byref(info)) == 0
+    return info
+
+
+@pytest.mark.parametrize("sms", [16, 40, 64, 66, 70, 74, 78, 84, 90, 108, 120, 132, 148])
+def test_tensor_memory_plans_have_a_kernel_on_every_size_of_gpu(lib, sms):
+    """(K halves, batch tile, streamed) of an accepted forward plan is one of the kernels that exist, its grid fits the GPU and its
+    groups reach the whole batch.  With fewer SMs than a B200's some widths would need a form without a kernel: those stay with
+    the other kernels."""
+    exist = {(1, 32, 0), (1, 64, 0), (0, 16, 1), (0, 32, 1), (0, 64, 1)}
+    seen = set()
+    for H in range(64, 4800, 64):
+        for B in (1, 17, 32, 33, 64, 65, 100, 128, 200, 256, 400, 700, 1500):
+            p = tmem_plan(lib, B, H, sms=sms)
+            if p.fwd_kernel:
+                assert p.fwd_grid <= sms and p.fwd_smem_bytes <= SMEM
+                assert p.fwd_batch_tile * p.fwd_batch_groups * p.fwd_tiles_in_turn >= B
+            if p.fwd_kernel == 1:
+                seen.add((p.fwd_k_halves, p.fwd_batch_tile, p.fwd_weights_streamed))
+            elif p.fwd_kernel == 2:
+                assert p.fwd_batch_tile in (64, 128) and 1 <= p.fwd_tiles_in_turn <= 6
+            if p.bwd_kernel:
+                assert p.bwd_grid <= sms and p.bwd_smem_bytes <= SMEM and p.bwd_batch_tile in (32, 64)
+                assert p.bwd_batch_tile * p.bwd_batch_groups * p.bwd_tiles_in_turn >= B
+    assert seen <= exist
+    if sms == SMS:
+        assert seen == exist
+
+
+def test_tensor_memory_plans_follow_the_measured_rules(lib):
+    p = tmem_plan(lib, 64, 1024)  # two groups of 32 sequences; short launches keep the weights in shared memory
+    assert (p.fwd_kernel, p.fwd_batch_tile, p.fwd_batch_groups, p.fwd_from_steps) == (1, 32, 2, 5)
+    assert (p.bwd_kernel, p.bwd_batch_tile, p.bwd_batch_groups, p.bwd_tiles_in_turn, p.bwd_from_steps) == (1, 32, 2, 1, 24)
+    p = tmem_plan(lib, 256, 2048)  # two tiles of 128 in turn forward, step GEMMs backward
+    assert (p.fwd_kernel, p.fwd_batch_tile, p.fwd_tiles_in_turn, p.fwd_from_steps, p.bwd_kernel) == (2, 128, 2, 2, 0)
+    p = tmem_plan(lib, 40, 2048)
+    assert (p.fwd_kernel, p.fwd_batch_tile, p.fwd_from_steps, p.bwd_kernel, p.bwd_from_steps) == (1, 64, 12, 1, 4)
+    p = tmem_plan(lib, 8, 4096, training=0)
+    assert (p.fwd_kernel, p.fwd_k_halves, p.fwd_batch_tile, p.fwd_weights_streamed) == (1, 0, 16, 1)

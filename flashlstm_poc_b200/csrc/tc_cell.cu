@@ -7,7 +7,7 @@
 // g / o of the same units), its warps take 32-wide K chunks of [x | h] in turn straight from global memory into mma.sync
 // operand fragments (16-byte loads, four chunks in flight per warp), and the warps' sums meet in shared memory once.
 // States are read where the caller has them and written where the caller wants them.  Two layers, H = 1024, one sequence: 50 -> 8.2 us
-// on the device, 97 -> 17 us a call (host work is what is left); bound by the latency of four rounds of loads per warp.
+// on the device, 97 -> 12 us a call (host work is what is left); bound by the latency of four rounds of loads per warp.
 #include "common.cuh"
 #include "tc_cluster.cuh"
 #include "tc_kernels.h"

@@ -484,19 +484,24 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
 }
 
 // Inference over a few steps: a launch per layer and step reads the layer's weights once, against projection GEMM, state copies
-// and the weight loads of a persistent kernel, all of which a few steps do not repay.  One call, cells / other path, us:
-//   2 layers, H = 128, B = 32:   T = 1 12 / 33    T = 2 24 / 33    T = 3 36 / 37    T = 4 46 / 37
-//   4 layers, H = 512, B = 8:    T = 1 25 / 74    T = 2 49 / 82    T = 3 74 / 82    T = 4 98 / 90
-//   3 layers, H = 1024, B = 24:  T = 1 25 / 64    T = 2 49 / 76    T = 3 74 / 83    T = 4 99 / 92
-//   1 layer, H = 1216, B = 16:   T = 1 12 / 33    T = 2 24 / 39    T = 3 36 / 45    T = 4 48 / 51
-//   1 layer, H = 1216, B = 24:   T = 1 16 / 31    T = 2 32 / 38    T = 3 47 / 45    T = 4 62 / 51
-//   1 layer, H = 2048, B = 16:   T = 1 15 / 37    T = 2 29 / 37    T = 3 43 / 41    T = 4 59 / 47
-//   1 layer, H = 2048, B = 32:   T = 1 23 / 31    T = 2 45 / 37    T = 3 68 / 41    T = 4 90 / 47
-//   1 layer, B = 24, T = 1:      H = 3072 49 / 55   H = 4096 79 / 74
-// From the second step on weights that stay in L2 (half of its 126 MB) are what pays; beyond that only T = 1 does.  More than
-// 16 sequences take twice the operand loads per step, which wide layers do not repay.  A fourth step is repaid least: beyond
-// 16 sequences in a single layer, up to 16 in stacks of 512 units altogether or where the other path is the grid-wide
-// kernel (H > 512 at these batches).
+// and the weight loads of a persistent kernel, all of which a few steps do not repay.  One call, cells / other path, us (I = H;
+// - where the rule below does not take cells):
+//   2 layers, H = 128, B = 32:   T = 1 10 / 33    T = 2 16 / 33    T = 3 23 / 36    T = 4  - / 37
+//   4 layers, H = 512, B = 8:    T = 1 16 / 74    T = 2 30 / 82    T = 3 44 / 82    T = 4  - / 87
+//   3 layers, H = 1024, B = 24:  T = 1 21 / 70    T = 2 41 / 78    T = 3 60 / 86    T = 4  - / 91
+//   1 layer, H = 1024, B = 16:   T = 1  7 / 29    T = 2 12 / 32    T = 3 16 / 35    T = 4 22 / 35
+//   1 layer, H = 1152, B = 24:   T = 1 10 / 29    T = 2 16 / 33    T = 3 24 / 34    T = 4 31 / 38
+//   1 layer, H = 1216, B = 16:   T = 1 12 / 31    T = 2 22 / 33    T = 3 32 / 35    T = 4 41 / 39
+//   1 layer, H = 1280, B = 32:   T = 1 16 / 31    T = 2 31 / 33    T = 3  - / 36
+//   1 layer, H = 1536, B = 16:   T = 1 12 / 35    T = 2 25 / 37    T = 3 35 / 37    T = 4  - / 40
+//   1 layer, H = 2048, B = 16:   T = 1 15 / 39    T = 2 29 / 37    T = 3 44 / 41    T = 4  - / 44
+//   1 layer, H = 2048, B = 32:   T = 1 21 / 33    T = 2  - / 37
+//   1 layer, B = 24, T = 1:      H = 3072 46 / 58   H = 3584 - / 66
+// From the second step on weights that stay in L2 (half of its 126 MB) are what pays, and for a third step 48 MB of them; beyond
+// that only T = 1 does.  More than 16 sequences take twice the operand loads per step, which wide layers do not repay.  Beyond
+// H = 1184 (8 units per CTA) there are more CTAs than SMs, which a fourth step does not repay.  Up to 16 sequences it goes to
+// stacks of 512 units altogether or where the other path is the grid-wide kernel (H > 512 at these batches), beyond 16 to a
+// single layer; larger stacks, with a launch per layer and step to prepare, are left to the other path.
 // A result that overlaps an input keeps to the other path, which has read all of x, h0 and c0 before it writes any.
 bool cell_path(const Engine &e, size_t T, const void *x, const void *h0, const void *c0, const void *y, const void *hn, const void *cn) {
     if (e.backend != FLSTM_BACKEND_TC || e.cfg.training || T > 4 || e.cfg.batch > (size_t)kCellBatch || e.trace) return false;
@@ -514,7 +519,8 @@ bool cell_path(const Engine &e, size_t T, const void *x, const void *h0, const v
     const bool wide = B > 16;
     if (T == 1) return !wide || H <= 3072;
     if (weights > ((size_t)64 << 20)) return false;
-    if (T == 4) return wide ? L == 1 && H <= 1152 : H <= 1280 && (H > 512 || L * H <= 512);
+    if (T == 4) return H <= 1152 && (wide ? L == 1 : H > 512 || L * H <= 512);
+    if (T == 3 && weights > ((size_t)48 << 20)) return false;
     return !wide || H <= (T == 2 ? 1280 : 1152);
 }
 

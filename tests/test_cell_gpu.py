@@ -68,6 +68,7 @@ def test_states_updated_in_place():
     (1, 4, 16, 64, 512, True), (2, 4, 8, 64, 512, False), (4, 4, 8, 64, 128, True), (2, 4, 16, 64, 576, True),
     (1, 4, 17, 64, 1152, True), (2, 4, 17, 64, 64, False), (1, 4, 17, 64, 1216, False), (1, 4, 8, 64, 1344, False),
     (1, 5, 1, 64, 64, False), (1, 2, 1, 2048, 2112, False),
+    (1, 4, 16, 64, 1152, True), (1, 4, 16, 64, 1216, False), (1, 3, 16, 1536, 1536, True), (1, 3, 16, 2048, 2048, False),
 ])
 def test_which_calls_run_step_by_step(L, T, B, I, H, cells):
     """The edges of the rule, by the launches of a call: one per layer and step, or the other path's (states in, a projection

@@ -49,7 +49,9 @@ __host__ __device__ inline int smem_of(const FwdWidePlan &pl) {
     return kBarrierBytes + pl.cs * kChunkBytesW + pl.hstages * kCh * (pl.BT / 2) * 128 + 1024 /*align*/;
 }
 
-template <int BT, bool BF16, bool ACCURATE>
+// TRACE: stamps of the group's first tile of each step.  A form of its own: without being asked for they took 6 % of a launch
+// (H = 2048, B = 256, T = 24: 297 -> 315 us).
+template <int BT, bool BF16, bool ACCURATE, bool TRACE>
 __global__ void __launch_bounds__(kThreads, 1)
 lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_h,
                      const __grid_constant__ FwdWidePlan pl, FwdParams p) {
@@ -142,6 +144,10 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     // barriers the loads of this CTA complete: the leader's at the same offsets
     const uint32_t hfull_c = map_to_rank(smem_u32(hfull), 0), wbar_c = map_to_rank(smem_u32(wbar), 0);
     const uint32_t tempty_c = map_to_rank(smem_u32(tempty), 0);
+#define FLSTM_STAMP(slot)                                                                                                \
+    do {                                                                                                                 \
+        if (TRACE && n == 0 && blockIdx.x == 0 && tt < p.trace_steps) p.trace[tt * 16 + (slot)] = clock64();              \
+    } while (0)
 
     if (warp == kProducerWarp) {
         // ------------------------------------------------------------ producer
@@ -161,6 +167,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                         if (!ok) break;
                         fence_proxy_async_global();
                     }
+                    FLSTM_STAMP(0);
                     for (int ld = 0; ld < NLOAD; ++ld) {
                         ok = mbar_wait(&hempty[stage], phase ^ 1, abort_w, wait_ns);
                         if (!ok) break;
@@ -172,6 +179,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                                          hfull_c + 8u * (uint32_t)stage);
                         if (++stage == HST) { stage = 0; phase ^= 1; }
                     }
+                    FLSTM_STAMP(1);
                 }
             // way out: every copy this thread started must have landed before the CTA exits (the peer's copies complete
             // the leader's barriers; after an abort the whole pair lingers, see below)
@@ -209,6 +217,8 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                     for (int c = 0; c < CT; c += kCh) {
                         const uint32_t dh = landed();
                         if (!ok) break;
+                        if (c == 0) FLSTM_STAMP(2);
+                        FLSTM_STAMP(3);
 #pragma unroll
                         for (int e = 0; e < 4 * kCh; ++e)
                             umma_lo_ts<true>(d, da + 8 * e, dh + (e >> 2) * kStepH + 2 * (e & 3), idesc, e ? 1u : acc);
@@ -220,6 +230,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                     for (; c + kCh <= KC && ok; c += kCh) {
                         const uint32_t dh = landed();
                         if (!ok) break;
+                        FLSTM_STAMP(3);
 #pragma unroll
                         for (int e = 0; e < 4 * kCh; ++e)
                             umma_lo_ss<true>(d, dw + (e >> 2) * kStepW + 2 * (e & 3), dh + (e >> 2) * kStepH + 2 * (e & 3), idesc, e ? 1u : acc);
@@ -236,6 +247,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                     }
                     if (!ok) break;
                     umma_commit_pair_both(tfull_l + 8u * buf);
+                    FLSTM_STAMP(4);
                     ++wi;
                 }
             // the tensor memory is freed at the end of the kernel: the last committed batch of UMMAs must be done
@@ -255,6 +267,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                     // no third tile may use this hdone barrier before the publisher has seen this phase of it
                     mbar_arrive_cluster_relaxed(tempty_c + 8u * (wi & 1));
                     red_release_gpu_add(counters + n, 1u);
+                    FLSTM_STAMP(8);
                 }
         }
     } else {
@@ -320,6 +333,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                 // a warp reads the accumulator only if all of its lanes saw it complete
                 ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (wi >> 1) & 1, abort_w, wait_ns));
                 if (!ok) break;
+                if (threadIdx.x == 0) FLSTM_STAMP(5);
                 tcgen05_fence_after();
                 uint32_t lo[4 * GROUPS], hi[4 * GROUPS];  // gates i, f and g, o: per 8 columns two of each
                 tmem_ld_16x256b<GROUPS>(taddr0 + buf * BTH, lo);
@@ -354,6 +368,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                     if (b + 8 * i + s8 < p.B) *reinterpret_cast<uint32_t *>(h_out + (size_t)(8 * i) * p.H) = h2[i];
                 }
                 __syncwarp();
+                if (threadIdx.x == 0) FLSTM_STAMP(7);
                 if (lane == 0) {
                     mbar_arrive(&hdone[buf]);
                     // Behind hdone, so that nobody arrives there for the next tile of this buffer before all have for this one.
@@ -393,6 +408,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             }
         }
     }
+#undef FLSTM_STAMP
     tcgen05_fence_before();
     __syncthreads();
     // after an abort this CTA's own copies may still be landing on barriers it cannot see (the leader's)
@@ -408,7 +424,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
 
 template <int BT, bool BF16, bool ACC>
 int launch_one(const CUtensorMap &tw, const CUtensorMap &th, const FwdWidePlan &pl, const FwdParams &p, cudaStream_t s) {
-    auto kern = lstm_fwd_wide_kernel<BT, BF16, ACC>;
+    auto kern = p.trace ? lstm_fwd_wide_kernel<BT, BF16, ACC, true> : lstm_fwd_wide_kernel<BT, BF16, ACC, false>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)pl.smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid);

@@ -170,3 +170,31 @@ def test_the_length_of_a_launch_chooses_its_kernel_and_not_its_bits(dtype, B, H,
     for a, b in zip(want, got + list(long.grads(0))):
         assert torch.equal(a, b)
     long.close()
+
+
+def test_step_trace_of_the_wide_forward():
+    """The kernel with batch tiles in turn stamps the first tile of each step."""
+    import numpy as np
+
+    from flashlstm_poc_b200 import step_trace
+
+    w = Workload("trace", "f16", 1, 64, 1024, 140, 24, seed=56)
+    inp = make_inputs(w)
+    dev, td = torch.device("cuda", 0), TORCH_DTYPES["f16"]
+    eng = Engine("f16", 1, 140, 64, 1024, 24, device=dev)
+    eng.set_weights(0, inp.w_ih[0].to(dev), inp.w_hh[0].to(dev), inp.b_ih[0].to(dev), inp.b_hh[0].to(dev))
+    x, dy = inp.x.to(dev, td), inp.dy.to(dev, td)
+
+    def run_step():
+        eng.forward(x)
+        eng.backward(dy)
+
+    run_step()
+    stamps = step_trace.collect(eng, run_step, steps=16)
+    eng.close()
+    forward = stamps[0]
+    points = forward[:, [0, 2, 3, 4, 5, 7, 8]]
+    assert (points[:, 0] > 0).all() and (np.diff(points, axis=1) > 0).all() and (forward[:, 0] < forward[:, 1]).all()
+    assert (forward[1:, 0] > forward[:-1, 8]).all()  # a step's barrier waits for the release of the step before
+    summary = step_trace.summarize(stamps, skip=2)
+    assert summary["forward"]["period"] > 0 and summary["bptt"]["period"] > 0

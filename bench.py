@@ -47,15 +47,12 @@ SHARDED = ("c3_bf16_l2_h2048", "c5_bf16_l4_h1024")  # the configurations the bat
 
 # DRAM bytes per launch of the recurrent kernels from ncu captures of small cases (dram__bytes_read.sum +
 # dram__bytes_write.sum, summaries under profiles/).  Stored figures, not measured by this run.
+# Each holds for the kernel it names only.
 STORED_TRAFFIC = {
-    ("c2_fp16_h1024", "recurrent_fwd"): {"bytes_per_timestep": 1.20e6, "batch_per_gpu": 64,
-                                         "source": "profiles/lstm_fwd_kernel_c2_fp16_h1024_T128.md (T=128, per step)"},
-    # per-step path at 256 sequences per GPU: split-K GEMM 37.8 MB + pointwise kernel 19.9 MB per time step,
-    # each launch captured cold (caches flushed); the forward kernel keeps W_hh in L2 across its steps
-    ("c3_bf16_l2_h2048", "bptt"): {"bytes_per_timestep": 57.7e6, "batch_per_gpu": 256,
+    # 256 sequences per GPU: split-K GEMM 37.8 MB + pointwise kernel 19.9 MB per time step, each launch captured cold
+    # (caches flushed)
+    ("c3_bf16_l2_h2048", "bptt"): {"bytes_per_timestep": 57.7e6, "batch_per_gpu": 256, "kernel": "step_kernel",
                                    "source": "profiles/step_kernel_c3_bf16_l2_h2048_T8.md (T=8, per time step, cold launches)"},
-    ("c3_bf16_l2_h2048", "recurrent_fwd"): {"bytes_per_timestep": 12.4e6, "batch_per_gpu": 256,
-                                            "source": "profiles/step_kernel_c3_bf16_l2_h2048_T8.md (wide_fwd_kernel, T=8, per time step)"},
 }
 
 
@@ -274,11 +271,12 @@ def cpu_torch_baseline(w):
 
 
 # ----------------------------------------------------------------------------- GPU measurement
-def recurrent_roofline(w, B, plan, phase_ms, peaks, tc):
+def recurrent_roofline(w, B, kernels, range_steps, phase_ms, peaks, tc):
     """Roofline entry of the slower recurrent kernel.  Per time step and layer a recurrent kernel moves
     8 H^2 bytes of W_hh (counted every step: the W_hh-streaming convention) plus 20 B H (forward: projection in,
     h in, y out, gates out), 12 B H (inference) or 22 B H (BPTT) of activations, and does 8 B H^2 FLOP;
-    the bound is whichever of bytes / HBM peak and FLOP / tensor peak is longer."""
+    the bound is whichever of bytes / HBM peak and FLOP / tensor peak is longer.  `kernels` names what the engine runs in
+    each phase (Engine.recurrent_kernel) for its launches of `range_steps` steps."""
     T, H, L = w.seq_len, w.hidden_size, w.layers
     steps = T * L
     cand = [("recurrent_fwd", 8 * H * H + (20 if w.training else 12) * B * H)]
@@ -290,33 +288,28 @@ def recurrent_roofline(w, B, plan, phase_ms, peaks, tc):
     flop_step = 8.0 * B * H * H
     t_hbm = dom_bytes / (peaks["hbm_gbs"] * 1e9)
     t_tensor = flop_step / (peaks["bf16_tflops"] * 1e12)
-    step_path = bool(plan and plan.step_path)
-    if not tc:
-        kernel, per_launch_steps, launches = "simt::persistent_%s" % dom, T, L
-    elif step_path and dom == "recurrent_fwd" and os.environ.get("FLSTM_WIDE_PERSIST", "1") != "0":
-        kernel, per_launch_steps, launches = "tc::wide_fwd_kernel (all time steps of a layer in one launch)", T, L
-    elif step_path:
-        kernel = ("tc::step_kernel<LSTM_FWD> (one launch per time step)" if dom == "recurrent_fwd" else
-                  "tc::step_bwd_pointwise_kernel + tc::step_kernel<F32_PARTS> (one pair per time step)")
+    info = kernels[dom]
+    kernel = ("tc::" if tc else "simt::") + info["name"]
+    if info["launches_per_step"]:
+        kernel = ("tc::step_bwd_pointwise_kernel + " if tc and dom == "bptt" else "") + kernel + " (launched per time step)"
         per_launch_steps, launches = 1, steps
     else:
-        kernel, per_launch_steps, launches = ("tc::lstm_fwd_kernel" if dom == "recurrent_fwd" else "tc::lstm_bwd_kernel"), T, L
-    dur_s = dom_ms * 1e-3 / max(launches, 1)
+        per_launch_steps, launches = range_steps, L * -(-T // range_steps)
     out = {"kernel": kernel, "phase": dom, "us_per_timestep": us_step, "launches_in_phase": launches,
            "timesteps_per_launch": per_launch_steps, "algorithmic_bytes_per_timestep": dom_bytes,
            "algorithmic_flop_per_timestep": flop_step, "bound_us_per_timestep": max(t_hbm, t_tensor) * 1e6,
            "peak_source": peaks["source"], "traffic": None}
     if t_tensor > t_hbm:
-        achieved = flop_step * per_launch_steps / dur_s / 1e12 if dur_s > 0 else 0.0
+        achieved = flop_step / (us_step * 1e-6) / 1e12 if us_step > 0 else 0.0
         out.update(bound="tensor", achieved=achieved, peak=peaks["bf16_tflops"], unit="TFLOP/s",
                    frac=achieved / peaks["bf16_tflops"])
     else:
-        achieved = dom_bytes * per_launch_steps / dur_s / 1e9 if dur_s > 0 else 0.0
+        achieved = dom_bytes / (us_step * 1e-6) / 1e9 if us_step > 0 else 0.0
         out.update(bound="hbm", achieved=achieved, peak=peaks["hbm_gbs"], unit="GB/s", frac=achieved / peaks["hbm_gbs"])
     for key, name in (("traffic", dom), ("traffic_recurrent_fwd_kernel", "recurrent_fwd")):
         stored = STORED_TRAFFIC.get((w.name, name))
-        if stored and stored["batch_per_gpu"] == B and (key == "traffic" or name != dom):
-            steps_per_launch = per_launch_steps if name == dom else (T if tc and not (step_path and os.environ.get("FLSTM_WIDE_PERSIST", "1") == "0") else 1)
+        if stored and stored["batch_per_gpu"] == B and stored["kernel"] == kernels[name]["name"] and (key == "traffic" or name != dom):
+            steps_per_launch = 1 if kernels[name]["launches_per_step"] else range_steps
             out[key] = stored["bytes_per_timestep"] * steps_per_launch
             out[key + "_source"] = "stored figure, " + stored["source"]
     return out
@@ -327,7 +320,6 @@ def measure_workload(args, w, world, rank, dev, headline):
     import torch
     import torch.distributed as dist
 
-    from flashlstm_poc_b200 import _lib
     from flashlstm_poc_b200.engine import TORCH_DTYPES, Engine
     from flashlstm_poc_b200.parallel import shard_range
     from flashlstm_poc_b200.workloads import make_inputs
@@ -432,12 +424,11 @@ def measure_workload(args, w, world, rank, dev, headline):
 
     peaks = measured_peaks()
     tc = eng.backend == "tc"
-    plan = None
-    if tc:
-        plan = _lib.TcPlanInfo()
-        if _lib.load().flstm_tc_plan(B, H, 1 if w.training else 0, 148, 232448, plan) != 0:
-            plan = None
-    roofline = recurrent_roofline(w, B, plan, phase_acc, peaks, tc)
+    range_steps = min(T, args.recompute or T)
+    kernels = {"recurrent_fwd": eng.recurrent_kernel(range_steps)}
+    if w.training:
+        kernels["bptt"] = eng.recurrent_kernel(range_steps, backward=True)
+    roofline = recurrent_roofline(w, B, kernels, range_steps, phase_acc, peaks, tc)
     # dense contractions (projection, weight and input gradients): 2/3 of the training FLOPs (half in inference)
     gemm_flops = w.flops() / world * (2.0 / 3.0 if w.training else 0.5)
     gemm_ms = phase_acc.get("projection", 0.0) + phase_acc.get("weight_grad", 0.0) + phase_acc.get("input_grad", 0.0)
@@ -456,7 +447,9 @@ def measure_workload(args, w, world, rank, dev, headline):
         "phase_ms": {k: round(v, 4) for k, v in phase_acc.items()}, "roofline": roofline, "roofline_gemm": roofline_gemm,
         "mfu_vs_measured_bf16_sustained": w.flops() / world / (ms_per_step * 1e-3) / (peaks["bf16_tflops_sustained"] * 1e12),
         "mfu_vs_nominal_2250": w.flops() / world / (ms_per_step * 1e-3) / 2250e12,
-        "backend": eng.backend, "recurrent_path": ("per-step GEMM launches" if (plan and plan.step_path) else "persistent kernels") if tc else "simt",
+        "backend": eng.backend, "recurrent_path": ", ".join(
+            f"{phase}: {k['name']} ({'launched per time step' if k['launches_per_step'] else 'one launch per layer and range'})"
+            for phase, k in kernels.items()),
         "workspace_gib": eng.workspace_bytes / 2**30, "clocks": clocks, "warmup": warmup,
     }
 

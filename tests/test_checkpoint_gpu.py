@@ -84,6 +84,19 @@ def test_checkpoint_mode_with_streamed_weights():
     _compare("bf16", 1, 7, 3, 64, 2432, 3)
 
 
+@pytest.mark.parametrize("dtype,L,T,B,I,H,R,forward,backward", [
+    ("f16", 1, 30, 32, 64, 1024, 26, "lstm_fwd_tm_kernel", "lstm_bwd_tm_kernel"),  # a last segment of four steps runs without them
+    ("bf16", 2, 9, 256, 64, 1024, 4, "lstm_fwd_wide_kernel", "lstm_bwd_tm_kernel"),  # two batch tiles in turn
+    ("bf16", 1, 9, 5, 64, 2048, 5, "lstm_fwd_tm_kernel", "lstm_bwd_tm_kernel"),
+    ("f16", 1, 7, 130, 64, 1088, 3, "lstm_fwd_wide_kernel", "lstm_bwd_tm_kernel"),
+])
+def test_checkpoint_mode_in_tensor_memory(dtype, L, T, B, I, H, R, forward, backward):
+    eng = Engine(dtype, L, B, I, H, T, device=torch.device("cuda", 0))
+    assert eng.recurrent_kernel(R)["name"] == forward and eng.recurrent_kernel(R, backward=True)["name"] == backward
+    eng.close()
+    _compare(dtype, L, T, B, I, H, R)
+
+
 def test_checkpoint_mode_limits():
     from flashlstm_poc_b200._lib import FlashLstmError
 

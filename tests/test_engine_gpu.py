@@ -74,19 +74,19 @@ def test_scaled_baseline_configs(name, scale):
 
 
 @pytest.mark.parametrize("dtype,L,T,B,I,H,training,path", [
-    ("bf16", 2, 5, 32, 2048, 2048, True, "auto"),    # config 3's width: W_hh slices do not fit shared memory -> streamed from L2
-    ("f16", 1, 4, 8, 4096, 4096, False, "auto"),     # config 4: two row tiles per CTA, streamed weights, inference
+    ("bf16", 2, 5, 32, 2048, 2048, True, "auto"),    # config 3's width: W_hh in tensor and shared memory, both directions
+    ("f16", 1, 4, 8, 4096, 4096, False, "auto"),     # config 4: 128 gate rows per CTA, part of W_hh streamed, inference
     ("f16", 1, 3, 1, 4096, 4096, False, "auto"),     # config 4 at batch 1
-    ("bf16", 2, 4, 256, 256, 1024, True, "auto"),    # 256 sequences at H=1024: two batch groups, one 128-wide tile each
-    ("f16", 1, 5, 160, 128, 1024, True, "auto"),     # 128-wide tiles, the second one ragged (32 of 128 sequences)
-    ("bf16", 1, 4, 192, 64, 512, False, "auto"),     # 128-wide tiles, inference, H=512
-    ("bf16", 2, 4, 512, 256, 1024, True, "auto"),    # wide batch (config 5's regime): one GEMM launch per step, no K split
-    ("bf16", 1, 4, 96, 128, 1024, True, "auto"),     # 96 sequences at H=1024: per-step path, one ragged 128-row tile
-    ("bf16", 1, 3, 64, 256, 2048, True, "auto"),     # two batch tiles per CTA at H=2048: the planner takes the per-step path
+    ("bf16", 2, 4, 256, 256, 1024, True, "auto"),    # 256 sequences at H=1024: two batch groups, two tiles of 64 in turn each
+    ("f16", 1, 5, 160, 128, 1024, True, "auto"),     # the same with three tiles, the last one half full
+    ("bf16", 1, 4, 192, 64, 512, False, "auto"),     # clusters of 13 sequences, inference, H=512
+    ("bf16", 2, 4, 512, 256, 1024, True, "auto"),    # two tiles of 128 in turn forward, step GEMMs backward
+    ("bf16", 1, 4, 96, 128, 1024, True, "auto"),     # one 64-wide tile per group forward, step GEMMs backward (one ragged 128-row tile)
+    ("bf16", 1, 3, 64, 256, 2048, True, "auto"),     # few steps: streamed W_hh, one 64-wide tile, both directions
     ("f16", 1, 5, 300, 128, 256, True, "step"),      # per-step path, ragged last 128-row tile, backward K split 8 ways
     ("bf16", 1, 3, 256, 128, 512, False, "step"),    # per-step path, inference
     ("f16", 1, 4, 40, 128, 128, True, "step"),       # per-step path with a single, mostly empty 128-row tile
-    ("f16", 1, 6, 200, 192, 192, True, "auto"),      # ragged batch tile, K chunks not a multiple of 4
+    ("f16", 1, 6, 200, 192, 192, True, "auto"),      # clusters of seven sequences
     ("bf16", 2, 4, 320, 256, 1024, True, "persistent"),  # the persistent kernels with several batch tiles per CTA: five
                                                          # 64-wide tiles over two batch groups, one slot without sequences
     ("f16", 1, 4, 96, 128, 2048, True, "persistent"),    # streamed weights with three 32-wide tiles per CTA

@@ -37,6 +37,29 @@ def test_padded_shapes_match_the_oracle(dtype, L, T, B, I, H):
     eng.close()
 
 
+# the padded form of every kernel that holds W_hh in tensor memory, and of those that run their short launches: dtype, T, B, H,
+# kernel and batch tile forward and backward
+PADDED_TMEM = [(dtype, *shape) for dtype in ("f16", "bf16") for shape in (
+    (30, 20, 1000, "lstm_fwd_tm_kernel", 32, "lstm_bwd_tm_kernel", 32), (4, 60, 1000, "lstm_fwd_kernel", 32, "lstm_bwd_kernel", 32),
+    (4, 20, 1080, "lstm_fwd_tm_kernel", 32, "lstm_bwd_tm_kernel", 32), (4, 70, 1080, "lstm_fwd_tm_kernel", 64, "lstm_bwd_tm_kernel", 64),
+    (4, 3, 2430, "lstm_fwd_tm_kernel", 16, "lstm_bwd_kernel", 32), (4, 17, 2430, "lstm_fwd_tm_kernel", 32, "lstm_bwd_kernel", 32),
+    (4, 33, 2430, "lstm_fwd_tm_kernel", 64, "step_kernel", 0),
+    (4, 140, 1000, "lstm_fwd_wide_kernel", 64, "lstm_bwd_tm_kernel", 64),
+    (4, 259, 1080, "lstm_fwd_wide_kernel", 128, "lstm_bwd_tm_kernel", 64))]
+
+
+@pytest.mark.parametrize("dtype,T,B,H,forward,fwd_tile,backward,bwd_tile", PADDED_TMEM)
+def test_padded_shapes_in_tensor_memory(dtype, T, B, H, forward, fwd_tile, backward, bwd_tile):
+    eng = Engine(dtype, 1, B, 64, H, T, device=torch.device("cuda", 0))
+    got = eng.recurrent_kernel(T), eng.recurrent_kernel(T, backward=True)
+    eng.close()
+    assert [(k["name"], k["batch_tile"]) for k in got] == [(forward, fwd_tile), (backward, bwd_tile)]
+    test_padded_shapes_match_the_oracle(dtype, 1, T, B, 64, H)
+    test_padded_gate_functions_keep_their_relative_accuracy_near_zero(dtype, B, 64, H, True, steps=T)
+    if B > 4:
+        test_an_infinite_input_stays_out_of_the_padding(dtype, T, B, 64, H, True)
+
+
 def test_padded_ranges_and_unaligned_tensors():
     T, B, I, H = 7, 5, 33, 70
     w = Workload("t", "f16", 2, I, H, B, T, seed=52, state_std=0.3)
@@ -75,7 +98,7 @@ def test_padded_ranges_and_unaligned_tensors():
     ("f16", 150, 64, 1270, True),                       # wide batch
     ("bf16", 5, 8, 70, False),                          # one launch per step
 ])
-def test_padded_gate_functions_keep_their_relative_accuracy_near_zero(dtype, B, I, H, training):
+def test_padded_gate_functions_keep_their_relative_accuracy_near_zero(dtype, B, I, H, training, steps=1):
     """Only the cell candidate has a pre-activation, exact in 16 bits and down to 2^-13 (f16) or 2^-20 (bf16), so that
     c_1 = tanh(a) / 2.  tanh is good to 2 units in the last place there and sigmoid(0) = 1/2 is exact: 2^-22 relative."""
     dev, td = torch.device("cuda", 0), TORCH_DTYPES[dtype]
@@ -84,12 +107,12 @@ def test_padded_gate_functions_keep_their_relative_accuracy_near_zero(dtype, B, 
     a = (128 + (37 * u) % 128) / 128 * torch.pow(2.0, -(4 + u % (low - 3)).float()) * torch.where(u % 2 == 0, 1.0, -1.0)
     w_ih, w_hh, b = torch.zeros(4 * H, I), torch.zeros(4 * H, H), torch.zeros(4 * H)
     w_ih[2 * H:3 * H, 0] = a * 64
-    x = torch.zeros(1, B, I)
-    x[..., 0] = 1 / 64
-    eng = Engine(dtype, 1, B, I, H, 1, training=training, device=dev)
+    x = torch.zeros(steps, B, I)
+    x[0, :, 0] = 1 / 64
+    eng = Engine(dtype, 1, B, I, H, steps, training=training, device=dev)
     eng.set_weights(0, w_ih.to(dev), w_hh.to(dev), b.to(dev), b.to(dev))
     eng.forward(x.to(dev, td))
-    got = eng.cell_states(0, 1)[1].double().cpu()
+    got = eng.cell_states(0, steps)[1].double().cpu()
     eng.close()
     want = (torch.tanh(a.double()) / 2).expand(B, H)
     assert float(((got - want) / want).abs().max()) < 2 ** -22

@@ -48,11 +48,16 @@ def _step(eng, inp, dev, td):
 def test_step_barrier_timeout_returns_and_engine_recovers(dtype, backend, where):
     where, _, variant = where.partition("-")
     shape = {"": (64, 64, 8), "wide": (128, 1024, 96), "streamed": (128, 2048, 8), "several": (64, 512, 8)}[variant]
-    w = Workload("timeout", dtype, 1, *shape, 4, seed=11, state_std=0.1)
+    _time_out_and_recover(dtype, backend, where, shape, 4)
+
+
+def _time_out_and_recover(dtype, backend, where, shape, steps, kernel=None):
+    w = Workload("timeout", dtype, 1, *shape, steps, seed=11, state_std=0.1)
     inp = make_inputs(w)
     td = TORCH_DTYPES[dtype]
     eng, dev = _engine(w, inp, backend)
     assert eng.backend == backend
+    assert kernel in (None, eng.recurrent_kernel(steps, backward=where == "backward")["name"])
     before = _step(eng, inp, dev, td)
     assert all(np.isfinite(a).all() for a in before) and np.abs(before[0]).max() <= 1.0  # every row of y was written
 
@@ -107,3 +112,20 @@ def test_which_kernels_the_cases_above_time_out():
         assert [p[0] for p in paths] == [forward, backward]
         if H == 512:
             assert all(p[1] == 16 for p in paths)
+
+
+@pytest.mark.parametrize("dtype,where,shape,steps,kernel,switches", [
+    # I, H, B: W_hh in tensor memory, one batch tile of 32 or 64 sequences, several in turn, part of W_hh streamed
+    ("f16", "forward", (64, 1024, 40), 6, "lstm_fwd_tm_kernel", {}), ("bf16", "forward", (64, 1088, 70), 4, "lstm_fwd_tm_kernel", {}),
+    ("f16", "forward", (64, 1024, 140), 4, "lstm_fwd_wide_kernel", {}), ("bf16", "forward", (64, 2048, 200), 4, "lstm_fwd_wide_kernel", {}),
+    ("bf16", "forward", (64, 2432, 3), 4, "lstm_fwd_tm_kernel", {}),
+    ("f16", "backward", (64, 1088, 8), 4, "lstm_bwd_tm_kernel", {}), ("bf16", "backward", (64, 1024, 140), 4, "lstm_bwd_tm_kernel", {}),
+    # the grid-wide kernels that take their place elsewhere: output-tiled, streamed
+    ("bf16", "forward", (64, 1024, 1600), 4, "wide_fwd_kernel", {}), ("bf16", "forward", (128, 1024, 96), 4, "wide_fwd_kernel", {"FLSTM_TMEM": "0"}),
+    ("bf16", "forward", (128, 2048, 8), 4, "lstm_fwd_kernel", {"FLSTM_TMEM": "0"}),
+    ("bf16", "backward", (128, 2048, 8), 4, "lstm_bwd_kernel", {"FLSTM_TMEM": "0"}),
+])
+def test_each_grid_wide_kernel_returns_and_recovers(dtype, where, shape, steps, kernel, switches, monkeypatch):
+    for name, value in switches.items():
+        monkeypatch.setenv(name, value)
+    _time_out_and_recover(dtype, "tc", where, shape, steps, kernel)

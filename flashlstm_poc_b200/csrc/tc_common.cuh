@@ -244,6 +244,20 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[
                  : "r"(taddr)
                  : "memory");
 }
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// acc[i] += the fp32 value in column i of this thread's lane, 8 columns at a time (the caller's registers are full of accumulators)
+template <int N>
+__device__ __forceinline__ void tmem_add_32x32b(uint32_t taddr, uint32_t (&acc)[N]) {
+    static_assert(N % 8 == 0, "whole loads");
+#pragma unroll
+    for (int c = 0; c < N; c += 8) {
+        uint32_t more[8];
+        tmem_ld_32x32b_x8(taddr + c, more);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[c + i] = __float_as_uint(__uint_as_float(acc[c + i]) + __uint_as_float(more[i]));
+    }
+}
 // 16 lanes x 8 N columns of 32 bits, as mma accumulator fragments: thread i gets, per 8 columns, columns 2 (i % 4) and + 1 of lane
 // base_lane + i / 4 (r[0], r[1]) and of lane base_lane + 8 + i / 4 (r[2], r[3])
 template <int N>
@@ -273,7 +287,6 @@ __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------ UMMA
 // Shared-memory matrix descriptor for a K-major operand tile stored as rows of 128 bytes with the

@@ -189,7 +189,7 @@ static int choose_tmem(int B, int H, bool fwd, bool bwd, int sms, size_t smem_li
         FwdPlan f{};
         const bool single = plan_fwd(B, H, sms, smem_limit, &f) == FLSTM_OK && f.nt == 1, fits_one = st->fwdtm.use;
         if (st->fwdtm.BT == 64 && single && f.resident && f.BT <= 64) st->fwdtm.use = false;
-        if (st->fwdtm.use && st->fwdtm.S == 2 && good && single) {
+        if (st->fwdtm.use && st->fwdtm.S == 2 && good && single && f.pair && f.BT <= 64) {
             st->fwd_from = st->fwdtm.BT == 64 ? 12 : 5;
             st->fwd = f;
             st->fwd.halves = true;
@@ -203,7 +203,7 @@ static int choose_tmem(int B, int H, bool fwd, bool bwd, int sms, size_t smem_li
         FLSTM_TRY(plan_bwd_tm(B, H, sms, smem_limit, &st->bwdtm, check_device));
         BwdPlan b{};
         if (st->bwdtm.use && good && st->bwdtm.nt == 1 && plan_bwd(B, H, sms, smem_limit, &b, check_device) == FLSTM_OK &&
-            b.nt == 1 && b.KS == 4) {
+            b.nt == 1 && b.KS == 4 && b.BT <= 64) {
             st->bwd_from = H <= 1024 ? 24 : 4;
             st->bwd = b;
             st->bwd.halves = true;

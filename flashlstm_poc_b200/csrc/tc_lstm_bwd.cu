@@ -63,7 +63,8 @@ __host__ __device__ inline BwdSmemLayout bwd_smem_layout(int BT, int H, int KS, 
     return l;
 }
 
-template <int BT, int KS, bool W_RESIDENT, bool BF16, bool ACCURATE>
+// HALVES: as in the forward kernel, of this CTA's K range (lstm_bwd_tm_kernel takes the longer launches).
+template <int BT, int KS, bool W_RESIDENT, bool BF16, bool ACCURATE, bool HALVES>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_dg, BwdParams p) {
     constexpr int UPO = 64 / KS;            // units this CTA owns after the reduce-scatter
@@ -92,9 +93,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     const int ng = cl / p.jt;                // batch group
     const int j = cl % p.jt;                 // unit tile: hidden units [64j, 64j+64)
     unsigned int *counter = p.counters + ng;
-    constexpr int kTmemCols = (2 * BT < 32) ? 32 : 2 * BT;
-    // p.halves: a second pair of accumulators behind the first takes the second half of this CTA's K range
-    const uint32_t tmem_cols = p.halves ? 2 * kTmemCols : kTmemCols;
+    constexpr int kPairCols = (2 * BT < 32) ? 32 : 2 * BT, kTmemCols = HALVES ? 2 * kPairCols : kPairCols;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < L.stages; ++i) {
@@ -115,7 +114,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         tma_prefetch_desc(&tm_dg);
     }
     if (warp == 5) {
-        tmem_alloc(tmem_slot, tmem_cols);
+        tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
     tcgen05_fence_before();
@@ -218,7 +217,6 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             uint32_t phase = 0;
             const uint32_t s_w_u32 = smem_u32(s_w), idesc = p.idesc;
             const uint32_t items = (uint32_t)(p.s1 - (p.s0 > 1 ? p.s0 : 1)) * nt_count;
-            const int half = p.halves ? KCper / 2 : KCper;  // the chunk that starts the second accumulator
             int last_commit = -1;
             for (uint32_t wi = 0; wi < items && ok; ++wi) {
                 const int buf = wi & 1;
@@ -240,19 +238,26 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     uint64_t dw = umma_desc_mnmajor_sw128(W_RESIDENT ? s_w_u32 + (uint32_t)(ld * CH) * kChunkBytesW
                                                                      : st_base + CH * BT * 128, 8192);
                     uint32_t acc = ld != 0;
+                    auto contract = [&](int chunks) {
 #pragma unroll 4
-                    for (int c = 0; c < CH; ++c) {
-                        if (ld * CH + c == half) {
-                            d_tmem += kTmemCols;
-                            acc = 0u;
+                        for (int c = 0; c < chunks; ++c) {
+                            umma_f16(d_tmem, dw, dd, idesc, acc);
+                            umma_f16(d_tmem, dw + 128, dd + 2, idesc, 1u);
+                            umma_f16(d_tmem, dw + 256, dd + 4, idesc, 1u);
+                            umma_f16(d_tmem, dw + 384, dd + 6, idesc, 1u);
+                            acc = 1u;
+                            dw += kChunkBytesW >> 4;
+                            dd += (BT * 128) >> 4;
                         }
-                        umma_f16(d_tmem, dw, dd, idesc, acc);
-                        umma_f16(d_tmem, dw + 128, dd + 2, idesc, 1u);
-                        umma_f16(d_tmem, dw + 256, dd + 4, idesc, 1u);
-                        umma_f16(d_tmem, dw + 384, dd + 6, idesc, 1u);
-                        acc = 1u;
-                        dw += kChunkBytesW >> 4;
-                        dd += (BT * 128) >> 4;
+                    };
+                    const int first = KCper / 2 - ld * CH;  // chunks of this load that belong to the first half
+                    if (HALVES && first >= 0 && first < CH) {
+                        contract(first);
+                        d_tmem += kPairCols;
+                        acc = 0u;
+                        contract(CH - first);
+                    } else {
+                        contract(CH);
                     }
                     umma_commit(&empty[stage]);
                     if (++stage == L.stages) { stage = 0; phase ^= 1; }
@@ -360,13 +365,7 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                             const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + buf * BT + c0;
                             tmem_ld_32x32b_x32(taddr, acc);
                             tmem_ld_wait();
-                            if (p.halves) {
-                                uint32_t more[32];
-                                tmem_ld_32x32b_x32(taddr + kTmemCols, more);
-                                tmem_ld_wait();
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(more[i]));
-                            }
+                            if (HALVES) tmem_add_32x32b(taddr + kPairCols, acc);
                             if (lane < 16) {
                                 const int row = warp * 16 + lane;        // unit within the tile
                                 const uint32_t owner = row / UPO, lu = row % UPO;
@@ -490,16 +489,16 @@ lstm_bwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             while (global_timer_ns() - t0 < 20000ull) {}
         }
     }
-    if (warp == 5) tmem_dealloc(tmem_base, tmem_cols);
+    if (warp == 5) tmem_dealloc(tmem_base, kTmemCols);
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / (p.jt * KS), p.exits);
 }
 
 // ------------------------------------------------------------------ host side
-template <int BT, int KS, bool RES, bool BF16, bool ACC>
-static int launch_bwd_one(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes,
+template <int BT, int KS, bool RES, bool BF16, bool ACC, bool HALVES>
+static int launch_bwd_form(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes,
                       cudaStream_t s) {
-    auto kern = lstm_bwd_kernel<BT, KS, RES, BF16, ACC>;
+    auto kern = lstm_bwd_kernel<BT, KS, RES, BF16, ACC, HALVES>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -534,6 +533,14 @@ static int launch_bwd_one(const CUtensorMap &tw, const CUtensorMap &tdg, const B
     return FLSTM_OK;
 }
 
+template <int BT, int KS, bool RES, bool BF16, bool ACC>
+static int launch_bwd_one(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes, cudaStream_t s) {
+    if constexpr (KS == 4 && BT <= 64) {  // the plans that share a shape with lstm_bwd_tm_kernel
+        if (p.halves) return launch_bwd_form<BT, KS, RES, BF16, ACC, true>(tw, tdg, p, grid, smem_bytes, s);
+    }
+    return launch_bwd_form<BT, KS, RES, BF16, ACC, false>(tw, tdg, p, grid, smem_bytes, s);
+}
+
 template <int BT, int KS, bool RES, bool BF16>
 static int launch_bwd(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdParams &p, int grid, int smem_bytes, cudaStream_t s) {
     return p.real_units ? launch_bwd_one<BT, KS, RES, BF16, true>(tw, tdg, p, grid, smem_bytes, s)
@@ -542,7 +549,7 @@ static int launch_bwd(const CUtensorMap &tw, const CUtensorMap &tdg, const BwdPa
 
 template <int BT, int KS, bool RES>
 static int max_clusters(int smem_bytes, int grid) {
-    auto kern = lstm_bwd_kernel<BT, KS, RES, false, false>;
+    auto kern = lstm_bwd_kernel<BT, KS, RES, false, false, false>;
     if (ensure_smem_limit(kern, (size_t)smem_bytes) != cudaSuccess) {
         cudaGetLastError();
         return -1;

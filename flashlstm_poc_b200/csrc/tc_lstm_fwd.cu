@@ -77,7 +77,10 @@ __host__ __device__ inline FwdSmemLayout fwd_smem_layout(int BT, int H, int rt, 
 // Only the leader (rank 0) issues UMMAs; both CTAs' loads are counted on the leader's barriers, its commits
 // signal both CTAs.  Each CTA finds its 64 x BT accumulator in its own tensor memory, sequences [0, BT/2) in lanes
 // 0-63 and [BT/2, BT) in lanes 64-127 (BT/2 columns).  Nothing is multicast.
-template <int BT, bool W_RESIDENT, bool BF16, bool PAIR, bool ACCURATE>
+// HALVES: the two halves of K are summed apart and added last, the order of lstm_fwd_tm_kernel, which takes the longer launches of
+// the same shape: a second pair of accumulators behind the first takes the second half.  A form of its own: asking at run time
+// cost the issue loop of the others up to 7 % of a step (H = 1216, B = 40: 6.89 -> 7.37 us).
+template <int BT, bool W_RESIDENT, bool BF16, bool PAIR, bool ACCURATE, bool HALVES>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_h,
                 const __grid_constant__ CUtensorMap tm_g, FwdParams p) {
@@ -104,9 +107,7 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     const int jr = blockIdx.x % p.cta_rows;        // first row tile = jr * rt
     unsigned int *counter = p.counters + ng;
     constexpr int kAccCols = PAIR ? BT / 2 : BT;  // tensor-memory columns of one accumulator
-    constexpr int kTmemCols = (2 * kAccCols < 32) ? 32 : 2 * kAccCols;
-    // p.halves: a second pair of accumulators behind the first takes the second half of K, and the epilogue adds the two
-    const uint32_t tmem_cols = p.halves ? 2 * kTmemCols : kTmemCols;
+    constexpr int kPairCols = (2 * kAccCols < 32) ? 32 : 2 * kAccCols, kTmemCols = HALVES ? 2 * kPairCols : kPairCols;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     const bool leader = rank == 0;
 
@@ -130,10 +131,10 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     }
     if (warp == 5) {
         if (PAIR) {
-            tmem_alloc_pair(tmem_slot, tmem_cols);
+            tmem_alloc_pair(tmem_slot, kTmemCols);
             tmem_relinquish_pair();
         } else {
-            tmem_alloc(tmem_slot, tmem_cols);
+            tmem_alloc(tmem_slot, kTmemCols);
             tmem_relinquish();
         }
     }
@@ -271,7 +272,6 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             const uint32_t s_w_u32 = smem_u32(s_w), idesc = p.idesc;
             const uint32_t empty_l = smem_u32(empty), tfull_l = smem_u32(tfull);
             const uint32_t total_items = (uint32_t)p.T * items_per_step;
-            const int half = p.halves ? KC / 2 : KC;  // the chunk that starts the second accumulator
             int last_commit = -1;
             for (uint32_t it = 0; it < total_items && ok; ++it, ++wi) {
                 const int r = (it % items_per_step) / nt_count;
@@ -294,20 +294,27 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                     uint64_t dw = umma_desc_kmajor_sw128(W_RESIDENT ? s_w_u32 + (uint32_t)(r * KC + ld * CH) * kChunkBytesW
                                                                     : st_base + CH * BTH * 128);
                     uint32_t acc = ld != 0;
+                    auto contract = [&](int chunks) {
 #pragma unroll 4
-                    for (int c = 0; c < CH; ++c) {
-                        if (ld * CH + c == half) {
-                            d_tmem += kTmemCols;
-                            acc = 0u;
-                        }
+                        for (int c = 0; c < chunks; ++c) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            if (PAIR) umma_f16_pair(d_tmem, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
-                            else umma_f16(d_tmem, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                            for (int k = 0; k < 4; ++k) {
+                                if (PAIR) umma_f16_pair(d_tmem, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                                else umma_f16(d_tmem, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                            }
+                            acc = 1u;
+                            dw += kChunkBytesW >> 4;
+                            dh += (BTH * 128) >> 4;
                         }
-                        acc = 1u;
-                        dw += kChunkBytesW >> 4;
-                        dh += (BTH * 128) >> 4;
+                    };
+                    const int first = KC / 2 - ld * CH;  // chunks of this load that belong to the first half
+                    if (HALVES && first >= 0 && first < CH) {
+                        contract(first);
+                        d_tmem += kPairCols;
+                        acc = 0u;
+                        contract(CH - first);
+                    } else {
+                        contract(CH);
                     }
                     // the stage may be refilled (PAIR: in both CTAs) once these UMMAs have read it
                     if (PAIR) umma_commit_pair_both(empty_l + 8u * (uint32_t)stage);
@@ -383,16 +390,8 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 #pragma unroll
                         for (int c0 = 0; c0 < BT; c0 += 32) {
                             uint32_t acc[32];
-                            const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + buf * BT + c0;
-                            tmem_ld_32x32b_x32(taddr, acc);
+                            tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(warp * 32) << 16) + buf * BT + c0, acc);
                             tmem_ld_wait();
-                            if (p.halves) {
-                                uint32_t more[32];
-                                tmem_ld_32x32b_x32(taddr + kTmemCols, more);
-                                tmem_ld_wait();
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(more[i]));
-                            }
                             if (lane < 16) {
                                 float4 *dst = reinterpret_cast<float4 *>(ex + (warp * 16 + lane) * EXS + c0);
 #pragma unroll
@@ -417,14 +416,7 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                             if (W16 == 16) tmem_ld_32x32b_x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(&acc[0]));
                             else tmem_ld_32x32b_x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&acc[0]));
                             tmem_ld_wait();
-                            if (p.halves) {
-                                uint32_t more[W16];
-                                if (W16 == 16) tmem_ld_32x32b_x16(taddr + kTmemCols, *reinterpret_cast<uint32_t(*)[16]>(&more[0]));
-                                else tmem_ld_32x32b_x32(taddr + kTmemCols, *reinterpret_cast<uint32_t(*)[32]>(&more[0]));
-                                tmem_ld_wait();
-#pragma unroll
-                                for (int i = 0; i < W16; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(more[i]));
-                            }
+                            if (HALVES) tmem_add_32x32b(taddr + kPairCols, acc);
                             float4 *dst = reinterpret_cast<float4 *>(ex + row * EXS + seq0 + c0);
 #pragma unroll
                             for (int i = 0; i < W16 / 4; ++i)
@@ -499,19 +491,19 @@ lstm_fwd_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             while (global_timer_ns() - t0 < kAbortDrainNs) {}
         }
         cluster_sync_all();  // the peer's shared and tensor memory stay valid until the leader's last UMMA is consumed
-        if (warp == 5) tmem_dealloc_pair(tmem_base, tmem_cols);
+        if (warp == 5) tmem_dealloc_pair(tmem_base, kTmemCols);
     } else if (warp == 5) {
-        tmem_dealloc(tmem_base, tmem_cols);
+        tmem_dealloc(tmem_base, kTmemCols);
     }
     if (threadIdx.x == 0 && *abort_w) atomicCAS(p.err, 0u, 1u);
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / p.cta_rows, p.exits);
 }
 
 // ------------------------------------------------------------------ host launcher
-template <int BT, bool RES, bool BF16, bool PAIR, bool ACC>
-static int launch_fwd_one(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdParams &p, int grid,
+template <int BT, bool RES, bool BF16, bool PAIR, bool ACC, bool HALVES>
+static int launch_fwd_form(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdParams &p, int grid,
                       int smem_bytes, cudaStream_t s) {
-    auto kern = lstm_fwd_kernel<BT, RES, BF16, PAIR, ACC>;
+    auto kern = lstm_fwd_kernel<BT, RES, BF16, PAIR, ACC, HALVES>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -530,6 +522,15 @@ static int launch_fwd_one(const CUtensorMap &tw, const CUtensorMap &th, const CU
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, th, tg, p);
     if (e != cudaSuccess) return set_error(FLSTM_ERR_CUDA, "recurrent forward launch failed: %s", cudaGetErrorString(e));
     return FLSTM_OK;
+}
+
+template <int BT, bool RES, bool BF16, bool PAIR, bool ACC>
+static int launch_fwd_one(const CUtensorMap &tw, const CUtensorMap &th, const CUtensorMap &tg, const FwdParams &p, int grid,
+                          int smem_bytes, cudaStream_t s) {
+    if constexpr (PAIR && BT <= 64) {  // the plans that share a shape with lstm_fwd_tm_kernel
+        if (p.halves) return launch_fwd_form<BT, RES, BF16, PAIR, ACC, true>(tw, th, tg, p, grid, smem_bytes, s);
+    }
+    return launch_fwd_form<BT, RES, BF16, PAIR, ACC, false>(tw, th, tg, p, grid, smem_bytes, s);
 }
 
 template <int BT, bool RES, bool BF16, bool PAIR>

@@ -151,7 +151,7 @@ def test_tensor_memory_plans_have_a_kernel_on_every_size_of_gpu(lib, sms):
 def test_tensor_memory_plans_follow_the_measured_rules(lib):
     p = tmem_plan(lib, 64, 1024)  # two groups of 32 sequences; short launches keep the weights in shared memory
     assert (p.fwd_kernel, p.fwd_batch_tile, p.fwd_batch_groups, p.fwd_from_steps) == (1, 32, 2, 5)
-    assert (p.bwd_kernel, p.bwd_batch_tile, p.bwd_batch_groups, p.bwd_tiles_in_turn, p.bwd_from_steps) == (1, 32, 2, 1, 24)
+    assert (p.bwd_kernel, p.bwd_batch_tile, p.bwd_batch_groups, p.bwd_tiles_in_turn, p.bwd_from_steps) == (1, 32, 2, 1, 12)
     p = tmem_plan(lib, 256, 2048)  # two tiles of 128 in turn forward, step GEMMs backward
     assert (p.fwd_kernel, p.fwd_batch_tile, p.fwd_tiles_in_turn, p.fwd_from_steps, p.bwd_kernel) == (2, 128, 2, 2, 0)
     p = tmem_plan(lib, 40, 2048)

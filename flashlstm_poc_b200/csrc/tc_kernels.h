@@ -88,7 +88,8 @@ struct FwdTmPlan {
 };
 constexpr int kFwdTmGroup = 3;  // streamed chunk-steps per copy
 int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan);
-// tm_w: W_hh as for lstm_forward_persistent.  tm_ws: W_hh as a chunked map of one step, box rows 128, kFwdTmGroup chunks.  tm_h: chunked map with box rows S * BT / 2 and plan.ch chunks.  tm_g: box 1 x BT x 64.
+// tm_w: W_hh as for lstm_forward_persistent.  tm_ws: W_hh as a chunked map of one step, box rows 128, kFwdTmGroup chunks.
+// tm_h: chunked map with box rows S * BT / 2 and plan.ch chunks.  tm_g: box 1 x BT x 64.
 int lstm_forward_tm(int dtype, const FwdTmPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_ws, const CUtensorMap &tm_h,
                     const CUtensorMap &tm_g, const FwdParams &p, cudaStream_t s);
 

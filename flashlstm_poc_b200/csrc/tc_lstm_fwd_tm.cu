@@ -18,10 +18,11 @@
 // through a ring of slots by a warp of its own, ascending in even steps of the sequence and descending in odd ones: the slots then
 // still hold the chunk-steps that the next step starts with, and L2 is asked first for what it was given last (in one direction
 // 94 MB per step go round in its 126 MB and mostly miss).  The direction is the order of the sums: it follows the step's number
-// in its sequence, so that a sequence cut into ranges or segments gives the bits of one launch.  A step takes the chunk-steps that the slots hold first, so that
-// copies start as soon as h is there, then those in tensor and shared memory, then the streamed ones.  Roles, step barrier, epilogue and the way
-// out after a bounded wait expired are the other forward kernel's (tc_lstm_fwd.cu): producer and UMMA threads break out of
-// their loops, the 256 epilogue threads leave together, an aborted pair lingers before its final cluster barrier.
+// in its sequence, so that a sequence cut into ranges or segments gives the bits of one launch.  A step takes the chunk-steps
+// that the slots hold first, so that copies start as soon as h is there, then those in tensor and shared memory, then the
+// streamed ones.  Roles, step barrier, epilogue and the way out after a bounded wait expired are the other forward kernel's
+// (tc_lstm_fwd.cu): producer and UMMA threads break out of their loops, the 256 epilogue threads leave together, an aborted pair
+// lingers before its final cluster barrier.
 //
 // Replaces the same reference launches as tc_lstm_fwd.cu (flashlstm_v2/src/lstm_forward.cu:744-830, src/lstm.cu:1241-1337).
 #include <cstdlib>

@@ -466,38 +466,39 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
 // changes from one instruction to the next (start address, leading byte offset): kept as a 32-bit value that advances by
 // constants in unrolled loops an instruction takes about 25 cycles to issue, against 45 to 100 with 64-bit descriptors formed in
 // the loop.
-constexpr uint32_t kUmmaDescHi = 0x40004040u;  // 8-row groups 1024 bytes apart, descriptor version, 128-byte swizzle
+constexpr uint32_t kUmmaDescHi = 0x40004040u;    // 8-row groups 1024 bytes apart, descriptor version, 128-byte swizzle
+constexpr uint32_t kUmmaDescHi32 = 0xC0004010u;  // rows of 32 bytes: 8-row groups 256 bytes apart, 32-byte swizzle
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes = 16) {
     return ((smem_addr & 0x3FFFF) >> 4) | (lbo_bytes >> 4) << 16;
 }
 // D (+)= A B, both operands in shared memory
-template <bool PAIR>
+template <bool PAIR, uint32_t B_HI = kUmmaDescHi>
 __device__ __forceinline__ void umma_lo_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     if (PAIR)
         asm volatile(
-            "{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+            "{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %6};\n"
             "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n}\n"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
+            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi), "r"(B_HI) : "memory");
     else
         asm volatile(
-            "{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+            "{\n.reg .pred p;\n.reg .b64 a, b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %6};\n"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
+            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi), "r"(B_HI) : "memory");
 }
 // The same with A in tensor memory, K-major: lane = row, a 32-bit column holds two consecutive K elements, so an instruction
 // (K = 16) reads 8 columns.  PAIR: M = 256, each CTA holds its 128 rows at the same columns.
-template <bool PAIR>
+template <bool PAIR, uint32_t B_HI = kUmmaDescHi>
 __device__ __forceinline__ void umma_lo_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     if (PAIR)
         asm volatile(
             "{\n.reg .pred p;\n.reg .b64 b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 b, {%2, %5};\n"
             "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], b, %3, p;\n}\n"
-            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(B_HI) : "memory");
     else
         asm volatile(
             "{\n.reg .pred p;\n.reg .b64 b;\nsetp.ne.b32 p, %4, 0;\nmov.b64 b, {%2, %5};\n"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n"
-            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi) : "memory");
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(B_HI) : "memory");
 }
 
 // ------------------------------------------------------------------ host: tensor maps

@@ -50,6 +50,7 @@ struct TcState {
     StepPlan step{};
     ClusterFwdPlan cfwd{};
     ClusterBwdPlan cbwd{};
+    void *ring = nullptr;       // slots of the kernels that exchange without a step barrier
     float *dh_parts = nullptr;  // wide-batch path: fp32 (L, splits, B, H) partial sums of dG_t W_hh
     float *dw_parts = nullptr;  // split-K partial products of the weight-gradient GEMMs
     size_t dw_floats = 0, dw_layers = 1;
@@ -255,6 +256,7 @@ int init(Engine &e) {
         st->dw_layers = st->step.use && !tm_fwd && !st->bwdtm.use ? e.layers.size() : 1;
         e.fixed.want(&st->dw_parts, st->dw_layers * st->dw_floats * sizeof(float));
     }
+    if (const size_t bytes = direct_ring_bytes(st->fwdtm)) e.fixed.want(&st->ring, bytes);
     st->layers.resize(e.layers.size());
     // one bias-gradient scratch per layer: with the cross-layer wavefront two layers may reduce at once
     if (e.cfg.training) e.fixed.want(&e.db_part, e.layers.size() * (size_t)simt::column_sum_scratch_floats(4 * e.cfg.hidden_size) * sizeof(float));
@@ -288,7 +290,8 @@ int on_capacity_change(Engine &e) {
             FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->wide.BT / 2, 2));
         }
         if (st->fwdtm.use) {
-            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->fwdtm.S * st->fwdtm.BT / 2, st->fwdtm.ch));
+            if (!st->fwdtm.direct)
+                FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->fwdtm.S * st->fwdtm.BT / 2, st->fwdtm.ch));
             FLSTM_TRY(make_tensor_map_3d(&t.tm_g_tm, l.gates, cap, B, 4 * H, 4 * H, B * 4 * H, st->fwdtm.BT, 64, false));
             if (st->fwdtm.wstages) FLSTM_TRY(make_tensor_map_chunked(&t.tm_ws, l.w_hh, 1, 4 * H, H, 128, kFwdTmGroup));
         }
@@ -462,6 +465,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.gates = l.gates;
     p.counters = e.sync_words + 1;
     p.exits = e.sync_words + kExitsWord;
+    p.ring = st->ring;
     p.err = err;
     p.T = (int)n;
     p.t0 = (int)t0;
@@ -475,6 +479,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
     if (kind == Kind::Wide) FLSTM_TRY(lstm_forward_wide(e.cfg.dtype, st->wide, t.tm_ws, t.tm_h_tm, p, s));
+    else if (kind == Kind::Tmem && st->fwdtm.direct) FLSTM_TRY(lstm_forward_tm_direct(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_g_tm, p, s));
     else if (kind == Kind::Tmem) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h_tm, t.tm_g_tm, p, s));
     else FLSTM_TRY(lstm_forward_persistent(e.cfg.dtype, st->fwd, t.tm_w, t.tm_h, t.tm_g, p, s));
     size_t m2 = e.timer.mark(s);

@@ -45,6 +45,7 @@ struct FwdParams {
     void *gates;          // 16-bit (T, B, 4H): holds P on entry, the activated gates on exit
     unsigned int *counters;  // one step counter per batch group, zero between launches
     unsigned int *exits;     // CTAs that have left, zero between launches (leave_counters)
+    void *ring;              // slots through which h_t crosses without a step barrier (tc_direct.cuh)
     unsigned int *err;    // error word: non-zero after a bounded wait expired
     int T, B, H;          // T = number of steps this launch runs
     int t0;               // first (absolute) time step of this launch; the state of step t0 is in slot t0 of hs/cs
@@ -83,6 +84,7 @@ struct FwdTmPlan {
     int ch, hstages;  // chunk-steps of h per copy, copies in the ring
     int wstages;   // slots for copies of streamed W_hh (0: nothing is streamed)
     int hring;     // 0: the copies of h hold a whole tile, they need no hand-back
+    bool direct;   // h_t crosses without a step barrier (tc_lstm_fwd_tm_direct.cu)
     int smem_bytes;
     int grid;
 };
@@ -92,6 +94,11 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan);
 // tm_h: chunked map with box rows S * BT / 2 and plan.ch chunks.  tm_g: box 1 x BT x 64.
 int lstm_forward_tm(int dtype, const FwdTmPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_ws, const CUtensorMap &tm_h,
                     const CUtensorMap &tm_g, const FwdParams &p, cudaStream_t s);
+
+bool fits_direct(const FwdTmPlan &plan, size_t smem_limit);
+size_t direct_ring_bytes(const FwdTmPlan &plan);  // FwdParams::ring
+int lstm_forward_tm_direct(int dtype, const FwdTmPlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_g, const FwdParams &p,
+                           cudaStream_t s);
 
 // ------------------------------------------------------------------ wide batches with W_hh on the chip (tc_lstm_fwd_wide.cu)
 struct FwdWidePlan {

@@ -543,7 +543,8 @@ int launch_one(const CUtensorMap &tw, const CUtensorMap &tws, const CUtensorMap 
 // The forms that lstm_forward_tm has kernels for: with the K halves nothing is streamed, without them always something (on the
 // widths that take either on 148 SMs; a GPU with fewer may plan others, and those stay with the other kernels).
 static bool has_kernel(const FwdTmPlan &pl) {
-    return pl.S == 2 ? pl.wstages == 0 && (pl.BT == 32 || pl.BT == 64) : pl.wstages > 0 && (pl.BT == 16 || pl.BT == 32 || pl.BT == 64);
+    if (pl.direct) return true;
+    return pl.S == 2 ? pl.wstages == 0 && pl.BT == 64 : pl.wstages > 0 && (pl.BT == 16 || pl.BT == 32 || pl.BT == 64);
 }
 
 int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
@@ -567,13 +568,14 @@ int plan_fwd_tm(int B, int H, int sms, size_t smem_limit, FwdTmPlan *plan) {
     // h in copies of 16 KB, the whole tile at once if it fits beside the rest of the weights
     const int rest = pl.kc - pl.ct;
     pl.cs = rest;
+    pl.direct = fits_direct(pl, smem_limit);
     pl.ch = 16384 / step_h < pl.kc ? 16384 / step_h : pl.kc;
     pl.hstages = (pl.kc + pl.ch - 1) / pl.ch;
-    while (!fits() && pl.hstages > 2) {
+    while (!pl.direct && !fits() && pl.hstages > 2) {
         --pl.hstages;
         pl.hring = 1;
     }
-    if (!fits()) {
+    if (!pl.direct && !fits()) {
         // streamed: all the room goes to the slots, which keep what the next step begins with
         pl.cs = 0;
         pl.hring = 1;
@@ -606,7 +608,7 @@ int lstm_forward_tm(int dtype, const FwdTmPlan &pl, const CUtensorMap &tw, const
         return acc ? launch_one<S_, BT_, ST_, false, true>(tw, tws, th, tg, pl, p, s)                          \
                    : launch_one<S_, BT_, ST_, false, false>(tw, tws, th, tg, pl, p, s);                        \
     }
-    FLSTM_TM_CASE(2, 32, false) FLSTM_TM_CASE(2, 64, false)
+    FLSTM_TM_CASE(2, 64, false)
     FLSTM_TM_CASE(1, 16, true) FLSTM_TM_CASE(1, 32, true) FLSTM_TM_CASE(1, 64, true)
 #undef FLSTM_TM_CASE
     return set_error(FLSTM_ERR_UNSUPPORTED, "no tensor-memory forward kernel for this plan");

@@ -1,0 +1,77 @@
+"""The tensor-memory kernels that exchange without a step barrier (tc_direct.cuh): words that announce themselves, slots that are
+used again after eight steps.  What the oracle tests of test_tmem_gpu.py do not reach: results that are no numbers, a y that starts
+at any element, many launches in a row, and sequences of every length around the slots."""
+import pytest
+import torch
+
+from flashlstm_poc_b200.engine import TORCH_DTYPES, Engine
+from flashlstm_poc_b200.workloads import Workload, make_inputs
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda", 0)
+
+
+def engine(dtype, B, H, T, training=True):
+    w = Workload("t", dtype, 1, 64, H, B, T, seed=91, state_std=0.3, training=training)
+    inp = make_inputs(w)
+    eng = Engine(dtype, 1, B, 64, H, T, training=training, device=DEV)
+    eng.set_weights(0, inp.w_ih[0].to(DEV), inp.w_hh[0].to(DEV), inp.b_ih[0].to(DEV), inp.b_hh[0].to(DEV))
+    return eng, [t if t is None else t.to(DEV, TORCH_DTYPES[dtype]) for t in (inp.x, inp.h0, inp.c0, inp.dy)]
+
+
+# one batch group of 32 and of 64, an odd number of 64-wide chunks of K, a partly filled tile
+SHAPES = [("f16", 32, 1024), ("bf16", 5, 1088), ("bf16", 70, 1088), ("f16", 64, 2048), ("bf16", 31, 2048)]
+
+
+@pytest.mark.parametrize("dtype,B,H", SHAPES)
+def test_sequences_that_are_no_numbers_stay_their_own(dtype, B, H):
+    """From a step with an infinite and a NaN input on, one sequence's h is NaN, of either sign; it crosses like any other value and
+    reaches no other sequence, whose results stay the same bit for bit."""
+    T = 26
+    eng, (x, h0, c0, _) = engine(dtype, B, H, T, training=False)
+    want, _, _ = eng.forward(x, h0, c0)
+    want = want.clone()
+    for value in (float("nan"), -float("nan"), float("inf"), -float("inf")):
+        bad = x.clone()
+        bad[7, B // 2] = value
+        bad[7, B // 2, ::2] = -value
+        y, _, _ = eng.forward(bad, h0, c0)
+        others = [b for b in range(B) if b != B // 2]
+        assert torch.equal(y[:, others], want[:, others])
+        assert torch.equal(y[:7, B // 2], want[:7, B // 2])
+        assert torch.isnan(y[8:, B // 2]).all()
+    y, _, _ = eng.forward(x, h0, c0)
+    assert torch.equal(y, want)
+    eng.close()
+
+
+@pytest.mark.parametrize("dtype,B,H", SHAPES)
+def test_y_may_start_at_any_element(dtype, B, H):
+    T = 14
+    eng, (x, h0, c0, _) = engine(dtype, B, H, T, training=False)
+    want, hn, cn = eng.forward(x, h0, c0)
+    room = torch.empty(T * B * H + 1, dtype=want.dtype, device=DEV)
+    y = room[1:].view(T, B, H)
+    eng.forward_into(T, x, h0, c0, y, hn, cn)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    eng.close()
+
+
+@pytest.mark.parametrize("dtype,B,H", SHAPES)
+def test_every_length_around_the_slots_and_many_launches(dtype, B, H):
+    """A call of n steps gives the first n steps of a longer one, forward, and repeated calls the same bits."""
+    T = 40
+    eng, (x, h0, c0, dy) = engine(dtype, B, H, T)
+    y, _, _ = eng.forward(x, h0, c0)
+    want = y.clone()
+    grads = [g.clone() for g in eng.backward(dy)]
+    for n in [*range(1, 22), 39]:
+        y, hn, _ = eng.forward(x[:n], h0, c0)
+        assert torch.equal(y, want[:n]) and torch.equal(hn[0], want[n - 1])
+    for _ in range(20):
+        y, _, _ = eng.forward(x, h0, c0)
+        assert torch.equal(y, want)
+        for a, b in zip(grads, eng.backward(dy)):
+            assert torch.equal(a, b)
+    eng.close()

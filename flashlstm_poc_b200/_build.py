@@ -27,7 +27,7 @@ EXT = os.path.join(PKG, "_flashlstm" + (sysconfig.get_config_var("EXT_SUFFIX") o
 STAMP = os.path.join(OBJ, "stamp.txt")
 
 CU_SOURCES = [
-    "engine.cu", "engine_padded.cu", "copy_batch.cu", "simt_kernels.cu", "simt_persistent.cu", "simt_cluster.cu", "tc_engine.cu", "tc_gemm.cu", "tc_lstm_fwd.cu", "tc_lstm_fwd_tm.cu", "tc_lstm_fwd_tm_direct.cu", "tc_lstm_fwd_wide.cu", "tc_lstm_bwd.cu", "tc_lstm_bwd_tm.cu", "tc_lstm_step.cu", "tc_cell.cu", "tc_cluster_bwd.cu", "tc_cluster_fwd.cu", "comm.cu", "static_scratch.cu", "api_v1.cu", "api_v2.cu",
+    "engine.cu", "engine_padded.cu", "copy_batch.cu", "simt_kernels.cu", "simt_persistent.cu", "simt_cluster.cu", "tc_engine.cu", "tc_gemm.cu", "tc_lstm_fwd.cu", "tc_lstm_fwd_tm.cu", "tc_lstm_fwd_tm_direct.cu", "tc_lstm_fwd_wide.cu", "tc_lstm_bwd.cu", "tc_lstm_bwd_tm.cu", "tc_lstm_bwd_tm_direct.cu", "tc_lstm_step.cu", "tc_cell.cu", "tc_cluster_bwd.cu", "tc_cluster_fwd.cu", "comm.cu", "static_scratch.cu", "api_v1.cu", "api_v2.cu",
 ]
 
 NVCC_FLAGS = [

@@ -30,7 +30,7 @@ namespace tc {
 constexpr int kDirectSlots = 8, kResetAhead = 4, kResetSlack = 2;
 constexpr uint32_t kUnwritten = 0xffffffffu;
 constexpr int kGatherWarps = 16, kGatherThreads = kGatherWarps * 32;  // with 8 warps the exchange takes 100 to 400 cycles more
-constexpr int kGatherStages = 4;  // parts of a gather that are handed over one by one, at most
+constexpr int kGatherStages = 3;  // parts of a gather that are handed over one by one, at most
 // Pieces of a stage: a stage costs some 400 cycles and lets the UMMAs start as much earlier as it is smaller.
 __host__ __device__ constexpr int stage_pieces(int rounds) { return rounds <= 4 ? 2 : 4; }
 constexpr int kGatherBarrier = 3;  // named barrier
@@ -38,6 +38,10 @@ constexpr uint32_t kGatherDelay = 700, kGatherDelayMax = 2000, kGatherLater = 96
 
 __device__ __forceinline__ void st_relaxed_gpu(void *p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed_gpu_16(void *p, uint4 v) {  // one access of 128 bits
+    asm volatile("{\n.reg .b64 lo, hi;\n.reg .b128 v;\nmov.b64 lo, {%1, %2};\nmov.b64 hi, {%3, %4};\nmov.b128 v, {lo, hi};\n"
+                 "st.relaxed.gpu.global.b128 [%0], v;\n}\n" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 __device__ __forceinline__ uint32_t ld_acquire_cta_shared(uint32_t smem_addr) {
     uint32_t v;
@@ -83,6 +87,13 @@ __device__ __forceinline__ void gather_commit() { asm volatile("cp.async.commit_
 // all but the LEFT newest groups have landed
 template <int LEFT>
 __device__ __forceinline__ void gather_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+// A piece that is written whole is looked at by one word: lanes 0-7 look at the first word of theirs, 8-15 at the second, ..., so
+// that a warp reads every bank once (all four words take four times as long).
+__device__ __forceinline__ bool gather_unwritten_whole(uint32_t smem_addr) {
+    uint32_t a;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(a) : "r"(smem_addr + (threadIdx.x >> 3 & 3) * 4) : "memory");
+    return a == kUnwritten;
+}
 __device__ __forceinline__ bool gather_unwritten(uint32_t smem_addr) {
     uint32_t a, b, c, d;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(smem_addr) : "memory");
@@ -101,7 +112,7 @@ __device__ __forceinline__ void gather_arrive(uint32_t bar_cluster_addr) { mbar_
 // addresses are constants apart: with run-time loops a stage cost 400 to 800 cycles, be it copied by cp.async or in bulk.  The
 // threads meet at a named barrier and one of them hands the stage over: an arrival of every warp on the mbarrier of another CTA
 // takes 14 cycles, 450 a stage.
-template <int ROUNDS, uint32_t STEP>
+template <int ROUNDS, uint32_t STEP, bool WHOLE, bool TURNS>
 struct Gather {
     static constexpr int kStagePieces = stage_pieces(ROUNDS), kStages = (ROUNDS + kStagePieces - 1) / kStagePieces;
     static_assert(kStages <= kGatherStages, "barriers of the stages");
@@ -110,29 +121,39 @@ struct Gather {
     uint32_t full;  // the UMMA thread's barriers of the stages, a shared::cluster address
     // A copy that comes too early is a round trip lost (800 cycles), one that comes late as many cycles as it is late: each warp
     // starts its copies `delay` cycles after it has sent its own part, more after a step in which it came too early, less otherwise.
-    uint32_t sent, delay;
+    uint32_t sent, delay = kGatherDelay;
+    // TURNS: the pieces of a stage are asked for in an order of a group of CTAs' own (turn < stage_pieces), so that not all of them bring
+    // the same line across the dies at once.  Forward 1 to 3 % of a step; the BPTT at H = 2048 lost a tenth by it.
+    uint32_t turn = 0;
 
+    __device__ __forceinline__ bool unwritten(uint32_t smem_addr) const {
+        return WHOLE ? gather_unwritten_whole(smem_addr) : gather_unwritten(smem_addr);
+    }
     __device__ __forceinline__ void hand_over(int stage) const {
         fence_proxy_async_smem();
         named_barrier_sync(kGatherBarrier, kGatherThreads);
         if (threadIdx.x == 0) gather_arrive(full + 8u * (uint32_t)stage);
     }
-    // the state that a launch starts from, which lies in rows of its own
-    __device__ __forceinline__ void first(const char *src, uint32_t src_step) {
-        for (int i = 0; i < mine; ++i) gather_copy(to + (uint32_t)i * STEP, src + (size_t)((uint32_t)i * src_step));
+    // the state that a launch starts from, which lies in rows of its own; piece `apart` comes from `apart_by` bytes further on
+    __device__ __forceinline__ void first(const char *src, uint32_t src_step, int apart = -1, uint32_t apart_by = 0) {
+        for (int i = 0; i < mine; ++i)
+            gather_copy(to + (uint32_t)i * STEP, src + (size_t)((uint32_t)i * src_step + (i == apart ? apart_by : 0u)));
         gather_commit();
         gather_wait<0>();
         for (int st = 0; st < kStages; ++st) hand_over(st);
-        delay = kGatherDelay;
     }
     __device__ __forceinline__ void mark_sent() { sent = (uint32_t)clock(); }
     // starts the copies of a step
     __device__ __forceinline__ void issue(const char *src) const {
         while ((uint32_t)clock() - sent < delay) {}
 #pragma unroll
-        for (int i = 0; i < ROUNDS; ++i) {
-            if (i < mine) gather_copy(to + i * STEP, src + i * STEP);
-            if (i % kStagePieces == kStagePieces - 1 || i + 1 == ROUNDS) gather_commit();
+        for (int st = 0; st < kStages; ++st) {
+#pragma unroll
+            for (int k = 0; k < kStagePieces; ++k) {
+                const uint32_t i = st * kStagePieces + (TURNS ? k ^ turn : k);
+                if ((int)i < mine) gather_copy(to + i * STEP, src + i * STEP);
+            }
+            gather_commit();
         }
     }
     // Waits for them and hands them over.  All threads run through all stages whatever becomes of them.  False: a wait expired or
@@ -156,7 +177,7 @@ private:
                 bool missing = false;
 #pragma unroll
                 for (int i = ST * kStagePieces; i < (ST + 1) * kStagePieces && i < ROUNDS; ++i)
-                    missing |= i < mine && gather_unwritten(to + i * STEP);
+                    missing |= i < mine && unwritten(to + i * STEP);
                 if (__any_sync(0xffffffffu, missing)) {
                     ok = again(src, err_word, abort_w, code, limit_ns);
                     complete = true;
@@ -166,6 +187,7 @@ private:
             stage<ST + 1>(src, err_word, abort_w, code, limit_ns, complete, ok);
         }
     }
+
     // what is missing of any stage is copied again together: a round trip for each stage's missing pieces cost 2 k cycles a step
     __device__ __forceinline__ bool again(const char *src, unsigned int *err_word, volatile uint32_t *abort_w, unsigned int code,
                                           unsigned long long limit_ns) const {
@@ -173,7 +195,7 @@ private:
         uint32_t todo = 0;
 #pragma unroll
         for (int i = 0; i < ROUNDS; ++i)
-            if (i < mine && gather_unwritten(to + i * STEP)) todo |= 1u << i;
+            if (i < mine && unwritten(to + i * STEP)) todo |= 1u << i;
         unsigned long long since = 0;
         for (uint32_t spins = 1; __any_sync(0xffffffffu, todo); ++spins) {
 #pragma unroll
@@ -183,7 +205,7 @@ private:
             gather_wait<0>();
 #pragma unroll
             for (int i = 0; i < ROUNDS; ++i)
-                if ((todo >> i & 1u) && !gather_unwritten(to + i * STEP)) todo &= ~(1u << i);
+                if ((todo >> i & 1u) && !unwritten(to + i * STEP)) todo &= ~(1u << i);
             if ((spins & 31u) == 0) {
                 if (since == 0) since = global_timer_ns();
                 bool give_up = *abort_w != 0;

@@ -256,7 +256,7 @@ int init(Engine &e) {
         st->dw_layers = st->step.use && !tm_fwd && !st->bwdtm.use ? e.layers.size() : 1;
         e.fixed.want(&st->dw_parts, st->dw_layers * st->dw_floats * sizeof(float));
     }
-    if (const size_t bytes = direct_ring_bytes(st->fwdtm)) e.fixed.want(&st->ring, bytes);
+    if (const size_t bytes = std::max(direct_ring_bytes(st->fwdtm), direct_ring_bytes(st->bwdtm))) e.fixed.want(&st->ring, bytes);
     st->layers.resize(e.layers.size());
     // one bias-gradient scratch per layer: with the cross-layer wavefront two layers may reduce at once
     if (e.cfg.training) e.fixed.want(&e.db_part, e.layers.size() * (size_t)simt::column_sum_scratch_floats(4 * e.cfg.hidden_size) * sizeof(float));
@@ -284,7 +284,7 @@ int on_capacity_change(Engine &e) {
         const bool grid_fwd = st->fwd.BT > 0, grid_bwd = bwd && st->bwd.BT > 0, step_bwd = bwd && bwd_kind(*st, 1) == Kind::Steps;
         if (st->cfwd.use && (!e.cfg.training || st->cbwd.use)) continue;  // the cluster kernels use plain loads
         FLSTM_TRY(make_tensor_map_2d(&t.tm_w, l.w_hh, 4 * H, H, H, 64, 64, true));
-        if (bwd && st->bwdtm.use) FLSTM_TRY(make_bwd_tm_maps(&t.dg_tm, st->bwdtm, l.dg, dg_steps, B, H));
+        if (bwd && st->bwdtm.use && !st->bwdtm.direct) FLSTM_TRY(make_bwd_tm_maps(&t.dg_tm, st->bwdtm, l.dg, dg_steps, B, H));
         if (st->wide.use) {
             FLSTM_TRY(make_tensor_map_gate_rows(&t.tm_ws, l.w_hh, H));
             FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->wide.BT / 2, 2));
@@ -681,6 +681,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.trace_steps = e.trace_steps;
     p.counters = e.sync_words + 1;
     p.exits = e.sync_words + kExitsWord;
+    p.ring = st->ring;
     p.err = err;
     p.T = (int)T;
     p.s0 = (int)(T - t1);
@@ -689,7 +690,8 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.H = (int)H;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
-    if (kind == Kind::Tmem) FLSTM_TRY(lstm_backward_tm(e.cfg.dtype, st->bwdtm, t.tm_w, t.dg_tm, p, s));
+    if (kind == Kind::Tmem && st->bwdtm.direct) FLSTM_TRY(lstm_backward_tm_direct(e.cfg.dtype, st->bwdtm, t.tm_w, p, s));
+    else if (kind == Kind::Tmem) FLSTM_TRY(lstm_backward_tm(e.cfg.dtype, st->bwdtm, t.tm_w, t.dg_tm, p, s));
     else FLSTM_TRY(lstm_backward_persistent(e.cfg.dtype, st->bwd, t.tm_w, t.tm_dg, p, s));
     e.launches += 1;
     }

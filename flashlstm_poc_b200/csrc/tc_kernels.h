@@ -142,6 +142,7 @@ struct BwdParams {
     float *dh0, *dc0;     // fp32 (B, H) or null
     float *dc;            // fp32 (B, H) scratch for the cell-gradient carry (used when nt > 1)
     unsigned int *counters, *exits;  // as in FwdParams
+    void *ring;           // as in FwdParams, of dG
     unsigned int *err;
     int real_units;       // as in FwdParams; a padding unit's dh counts as zero
     long long *trace;     // optional per-step clock64() stamps of CTA 0 (see FwdParams)
@@ -175,6 +176,7 @@ struct BwdTmPlan {
     int ct, cs;    // chunk-steps of W_hh in tensor / shared memory (all of them)
     int ch, stages;  // chunk-steps of dG per copy, copies in the ring
     int ring;      // 0: the copies hold a whole tile, they need no hand-back
+    bool direct;   // dG_t crosses without a step barrier (tc_lstm_bwd_tm_direct.cu)
     int smem_bytes;
     int grid;
 };
@@ -186,6 +188,10 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
 int make_bwd_tm_maps(BwdTmMaps *maps, const BwdTmPlan &plan, const void *dg, size_t steps, size_t B, size_t H);
 int lstm_backward_tm(int dtype, const BwdTmPlan &plan, const CUtensorMap &tm_w, const BwdTmMaps &maps, const BwdParams &p,
                      cudaStream_t s);
+bool fits_direct(const BwdTmPlan &plan, size_t smem_limit);
+size_t direct_ring_bytes(const BwdTmPlan &plan);  // BwdParams::ring
+int max_clusters_direct(const BwdTmPlan &plan);   // that the current device holds at once, or -1
+int lstm_backward_tm_direct(int dtype, const BwdTmPlan &plan, const CUtensorMap &tm_w, const BwdParams &p, cudaStream_t s);
 
 // ------------------------------------------------------------------ wide-batch path: one GEMM launch per step
 struct StepPlan {

@@ -586,8 +586,9 @@ static int plan_groups(int B, int H, int groups, size_t smem_limit, BwdTmPlan *p
         pl.stages = (pl.kp + pl.ch - 1) / pl.ch;
         while (!fits() && pl.stages > 2) --pl.stages;
     }
-    if (!fits()) return FLSTM_OK;
-    pl.ring = pl.nt > 1 || pl.stages * pl.ch < pl.kp;
+    pl.direct = fits_direct(pl, smem_limit);
+    if (!pl.direct && !fits()) return FLSTM_OK;
+    pl.ring = !pl.direct && (pl.nt > 1 || pl.stages * pl.ch < pl.kp);
     // All of shared memory: a CTA allocates all of tensor memory, so no other kernel that uses some (another engine's, on another
     // stream) may share its SM; two grids that each held what the other's CTAs were waiting for would run into their limits
     pl.smem_bytes = (int)smem_limit;
@@ -606,7 +607,7 @@ int plan_bwd_tm(int B, int H, int sms, size_t smem_limit, BwdTmPlan *plan, bool 
     for (int groups = sms / (H / 64 * KS); groups > 0; --groups) {
         FLSTM_TRY(plan_groups(B, H, groups, smem_limit, plan));
         if (!plan->use) return FLSTM_OK;
-        if (!check_device || (plan->BT == 32 ? max_clusters<32>(*plan) : max_clusters<64>(*plan)) * KS >= plan->grid) return FLSTM_OK;
+        if (!check_device || (plan->direct ? max_clusters_direct(*plan) : plan->BT == 32 ? max_clusters<32>(*plan) : max_clusters<64>(*plan)) * KS >= plan->grid) return FLSTM_OK;
         *plan = BwdTmPlan{};
     }
     return FLSTM_OK;

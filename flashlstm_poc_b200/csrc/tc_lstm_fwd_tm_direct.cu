@@ -1,11 +1,10 @@
-// The tensor-memory forward kernel (tc_lstm_fwd_tm.cu: CTA pairs, K split over the lane halves, nothing streamed) without a step
-// barrier: h_t goes from CTA to CTA through words that announce themselves (tc_direct.cuh).
+// The tensor-memory forward kernel (tc_lstm_fwd_tm.cu: CTA pairs, K split over the lane halves, nothing streamed) for batch tiles of 32
+// sequences, without a step barrier: h_t goes from CTA to CTA through words that announce themselves (tc_direct.cuh).
 //
 // What bounds a step is its chain of L2 round trips.  With a counter per step, H = 1024, B = 64: 5.6 k cycles, of which
 // releasing the stores 1.2 k, the counter 1.5 k, copying 32 KB 1.3 k, UMMAs behind the last copy 0.4 k, accumulator to result 1.1 k.
-// The exchange here replaces the first three: 4.3 k cycles (H = 2048, B = 32: 6.9 -> 6.0 k, of which the UMMAs' own 2 k).  v1 call,
-// H = 1024, B = 32, T = 512: 1763 -> 1446 us; training step at B = 64: 4629 -> 4315 us; two layers of 2048, B = 32, T = 1024: 24.5 ->
-// 23.6 ms.
+// The exchange here replaces the first three: 4.2 k cycles (H = 2048, B = 32: 6.9 -> 5.9 k, of which the UMMAs' own 2 k); us a step at
+// fits_direct.
 //
 // Roles.  Warps 0-15 epilogue and gather, 16 projections, 17 UMMA issuer, 18 weights kept in shared memory, 19 the launch's one
 // counter barrier, then fences behind resets.  A warp that has sent its part of h_t stores what nobody waits for while
@@ -35,51 +34,47 @@ namespace tc {
 namespace {
 
 constexpr int kEpilogueThreads = kGatherThreads, kThreads = kEpilogueThreads + 128;
+constexpr int BT = 32, N = 2 * BT;         // sequences of a tile, UMMA N
+constexpr int kRowStride = BT + 4;         // of the exchange buffer (floats), keeps float4 alignment
 constexpr int kStepBytesW = 128 * 128;  // one chunk-step of A: 128 rows x 64 16-bit elements
 constexpr int kTmemColumns = 512;
 constexpr int kBarrierBytes = 1024;
 constexpr int kFillSlots = 8;  // a multiple of 4: a slot always belongs to the same set of warps (see tc_lstm_fwd_tm.cu)
 constexpr int kMinSmemBytes = kBarrierBytes + kFillSlots * kStepBytesW + 1024;
 
-// rounds in which the gather threads take the chunk-steps of a half of K, and chunk-steps of a round
-__host__ __device__ constexpr int round_steps(int BT) { return kGatherThreads / (8 * BT); }
-__host__ __device__ inline int gather_rounds(const FwdTmPlan &pl) { return (pl.kc + round_steps(pl.BT) - 1) / round_steps(pl.BT); }
-// of the kernel that a plan takes: H = 1024, 2048 and 2368 with 32 sequences, 2048 with 64
+// the gather threads take a half of K in rounds of two chunk-steps
+constexpr int kRoundSteps = kGatherThreads / (8 * BT);
+__host__ __device__ inline int gather_rounds(const FwdTmPlan &pl) { return (pl.kc + kRoundSteps - 1) / kRoundSteps; }
+// of the kernel that a plan takes: H = 1024, 2048 and 2368
 __host__ __device__ inline int kernel_rounds(const FwdTmPlan &pl) {
     const int n = gather_rounds(pl);
-    return pl.BT == 64 ? 16 : n <= 4 ? 4 : n <= 8 ? 8 : 10;
+    return n <= 4 ? 4 : n <= 8 ? 8 : 10;
 }
 
 struct Layout {
     int w, h, p, ex, total;
-    bool ex_in_h;  // the exchange buffer takes the place of the h tile, which the UMMAs have read by then
 };
-__host__ __device__ inline Layout layout_of(const FwdTmPlan &pl, int smem_limit) {
+__host__ __device__ inline Layout layout_of(const FwdTmPlan &pl) {
     Layout l;
-    const int step_h = pl.BT * 128;
     l.w = pl.cs * kStepBytesW;
-    l.h = gather_rounds(pl) * round_steps(pl.BT) * step_h;
-    l.p = 2 * pl.BT * 128;
-    l.ex = 128 * (pl.BT + 4) * 4;
-    l.total = kBarrierBytes + l.w + l.h + l.p + 1024 /*align*/;
-    // not over the last chunk-step: what lies beyond K must stay zero there
-    l.ex_in_h = l.total + l.ex > smem_limit && l.ex <= (pl.kc - 1) * step_h;
-    if (!l.ex_in_h) l.total += l.ex;
+    l.h = gather_rounds(pl) * kRoundSteps * BT * 128;
+    l.p = 2 * BT * 128;
+    l.ex = 128 * kRowStride * 4;
+    l.total = kBarrierBytes + l.w + l.h + l.p + l.ex + 1024 /*align*/;
     if (l.total < kMinSmemBytes) l.total = kMinSmemBytes;
     return l;
 }
 
-template <int BT, int ROUNDS, bool BF16, bool ACCURATE>
+template <int ROUNDS, bool BF16, bool ACCURATE>
 __global__ void __launch_bounds__(kThreads, 1)
 lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ FwdTmPlan pl,
                    FwdParams p) {
-    constexpr int N = 2 * BT, EXS = BT + 4;  // UMMA N; row stride of the exchange buffer (floats), keeps float4 alignment
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const Layout L = layout_of(pl, pl.smem_bytes);
+    const Layout L = layout_of(pl);
     const int KC = pl.kc, CT = pl.ct, CS = pl.cs;
     uint8_t *s_w = smem + kBarrierBytes, *s_h = s_w + L.w, *s_p = s_h + L.h;
-    float *s_ex = reinterpret_cast<float *>(L.ex_in_h ? s_h : s_p + L.p);
+    float *s_ex = reinterpret_cast<float *>(s_p + L.p);
     uint64_t *hfull = reinterpret_cast<uint64_t *>(smem), *tfull = hfull + kGatherStages, *tempty = tfull + 1, *wbar = tempty + 1;
     uint64_t *reset = wbar + 1, *ready = reset + 1, *pfull = ready + 1, *pempty = pfull + 2;
     uint64_t *ffull = pempty + 2, *fempty = ffull + kFillSlots;  // while W_hh moves into tensor memory
@@ -99,14 +94,9 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     char *const ring = static_cast<char *>(p.ring);
     const uint32_t slot_bytes = (uint32_t)gridDim.x * BT * 32u;
 
-    // epilogue ownership: unit u of the CTA's 16, sequences nb + 32 i.  Of the words, the one of units u and u ^ 1: of a single
-    // sequence the even lanes have it, of two the odd lanes have the second's
-    constexpr int PER = BT / 32;
+    // epilogue ownership: unit u of the CTA's 16 and sequence nb; the even lanes have the word of units u and u + 1
     const int u = threadIdx.x & 15, nb = (threadIdx.x >> 4) & 31, odd = u & 1;
-    const int rows_left = p.B - b0 - nb;  // sequence nb + 32 i exists while 32 i < rows_left
-    const int word_row = PER == 2 ? 32 * odd : 0;
-    const bool has_word = PER == 2 || !odd;
-    const uint32_t my_word = (uint32_t)((blockIdx.x * BT + nb + word_row) * 32 + (u & ~1) * 2);
+    const uint32_t my_word = (uint32_t)((blockIdx.x * BT + nb) * 32 + (u & ~1) * 2);
     const unsigned long long wait_ns = p.wait_ns ? p.wait_ns : kWaitLimitNs;
 
     if (threadIdx.x == 0) {
@@ -134,7 +124,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         tmem_alloc_pair(tmem_slot, kTmemColumns);
         tmem_relinquish_pair();
     }
-    if (warp < 16 && has_word && p.T > 1)
+    if (warp < 16 && !odd && p.T > 1)
         for (int s = 0; s < kDirectSlots; ++s) st_relaxed_gpu(ring + (size_t)s * slot_bytes + my_word, kUnwritten);
     tcgen05_fence_before();
     __syncthreads();
@@ -222,7 +212,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 constexpr uint32_t idesc = umma_idesc_f16(256, N, BF16 ? 1 : 0, 0, 0);
                 constexpr uint32_t kTileH = (BT * 32) >> 4, kStepW = kStepBytesW >> 4;  // descriptor units
                 const uint32_t tfull_l = smem_u32(tfull), dw_res = umma_desc_lo(smem_u32(s_w)), dh_tile = umma_desc_lo(smem_u32(s_h));
-                constexpr int stage_steps = stage_pieces(ROUNDS) * round_steps(BT);
+                constexpr int stage_steps = stage_pieces(ROUNDS) * kRoundSteps;
                 int committed = 0;
                 for (int tt = 0; tt < p.T && ok; ++tt) {
                     ok = mbar_wait_cluster(tempty, (tt & 1) ^ 1, abort_w, wait_ns);
@@ -274,9 +264,10 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // this thread's pieces of the h tile
         constexpr int PIECES = 2 * BT, TILES = kGatherThreads / PIECES;  // 16-byte pieces of 16 units, such tiles per round
         constexpr uint32_t ROUND = TILES * BT * 32;                       // bytes, in the ring and in the tile
-        Gather<ROUNDS, ROUND> g;
+        Gather<ROUNDS, ROUND, false, true> g;
         const char *from;
         g.full = map_to_rank(smem_u32(hfull), 0);
+        g.turn = (uint32_t)(jr >> 3) & (stage_pieces(ROUNDS) - 1);
         {
             const int n = tid % PIECES >> 1, e = tid & 1, j0 = tid / PIECES;
             const int first = (int)rank * KC * 4, tiles = p.H / 16 - first < 4 * KC ? p.H / 16 - first : 4 * KC;
@@ -290,29 +281,26 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const bool y_words = (reinterpret_cast<uintptr_t>(y) & 3) == 0;  // the caller's y may start at any element
         const int quad = warp & 3, col0 = (warp >> 2) * (BT / 4);       // lane quadrant, quarter of the columns
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (quad >> 1) * BT + col0;
-        const size_t idx0 = (size_t)(b0 + nb) * p.H + jr * 16 + u;
+        const bool valid = b0 + nb < p.B;
+        const size_t idx = (size_t)(b0 + nb) * p.H + jr * 16 + u;
         const bool pad = ACCURATE && jr * 16 + u >= p.real_units;
         if (p.T > 1) {
             fence_acq_rel_gpu();
             named_barrier_sync(2, kEpilogueThreads);
             if (tid == 0) red_release_gpu_add(counter, 1u);
         }
-        float c_keep[PER];
-#pragma unroll
-        for (int i = 0; i < PER; ++i) c_keep[i] = 32 * i < rows_left ? p.cs[(size_t)p.t0 * slab + idx0 + (size_t)(32 * i) * p.H] : 0.f;
+        float c_keep = valid ? p.cs[(size_t)p.t0 * slab + idx] : 0.f;
         bool gathered = true;
         for (int tt = 0; tt < p.T; ++tt) {
             const int t = p.t0 + tt, pb = tt & 1;
             // No thread leaves between here and the named barrier below, whatever its waits return: the barrier ORs the
             // failures, so that all 512 threads go on or give up together.
             bool good = mbar_wait(&pfull[pb], (tt >> 1) & 1, abort_w, wait_ns) && gathered;
-            float proj[PER][4];
+            float proj[4];
             {
                 const uint16_t *ptile = reinterpret_cast<const uint16_t *>(s_p + pb * BT * 128) + nb * 64 + u;
 #pragma unroll
-                for (int i = 0; i < PER; ++i)
-#pragma unroll
-                    for (int gt = 0; gt < 4; ++gt) proj[i][gt] = load16<BF16>(ptile + i * 2048 + gt * 16);
+                for (int gt = 0; gt < 4; ++gt) proj[gt] = load16<BF16>(ptile + gt * 16);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&pempty[pb]);
@@ -325,10 +313,9 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             tcgen05_fence_after();
             if (seen) {
                 uint32_t acc[BT / 4];
-                if constexpr (BT == 32) tmem_ld_32x32b_x8(taddr, acc);
-                else tmem_ld_32x32b_x16(taddr, acc);
+                tmem_ld_32x32b_x8(taddr, acc);
                 tmem_ld_wait();
-                float4 *dst = reinterpret_cast<float4 *>(s_ex + (quad * 32 + lane) * EXS + col0);
+                float4 *dst = reinterpret_cast<float4 *>(s_ex + (quad * 32 + lane) * kRowStride + col0);
 #pragma unroll
                 for (int i = 0; i < BT / 16; ++i)
                     dst[i] = make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]),
@@ -340,57 +327,45 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             if (lane == 0) mbar_arrive_cluster_relaxed(tempty_c);
             if (named_barrier_or(1, kEpilogueThreads, !good)) break;
             if (tid == 0) FLSTM_STAMP(tt, 6);
-            float act[PER][4];
-            uint32_t h16[PER];
+            float a[4];
 #pragma unroll
-            for (int i = 0; i < PER; ++i) {
-                float a[4];
-#pragma unroll
-                for (int gt = 0; gt < 4; ++gt) {
-                    const float *ex = s_ex + (gt * 16 + u) * EXS + nb + 32 * i;
-                    a[gt] = ex[0] + ex[64 * EXS] + proj[i][gt];
-                }
-                const float gi = sigmoid_sel<ACCURATE>(pad ? 0.f : a[0]), gf = sigmoid_sel<ACCURATE>(pad ? 0.f : a[1]);
-                const float gg = tanh_sel<ACCURATE>(pad ? 0.f : a[2]), go = sigmoid_sel<ACCURATE>(pad ? 0.f : a[3]);
-                c_keep[i] = fmaf(gf, c_keep[i], gi * gg);
-                h16[i] = to16<BF16>(go * tanh_sel<ACCURATE>(c_keep[i]));
-                act[i][0] = gi; act[i][1] = gf; act[i][2] = gg; act[i][3] = go;
+            for (int gt = 0; gt < 4; ++gt) {
+                const float *ex = s_ex + (gt * 16 + u) * kRowStride + nb;
+                a[gt] = ex[0] + ex[64 * kRowStride] + proj[gt];
             }
-            const uint32_t other_h = __shfl_xor_sync(0xffffffffu, odd ? h16[0] : h16[PER - 1], 1);
-            const uint32_t word = odd ? __byte_perm(other_h, h16[PER - 1], 0x5410) : __byte_perm(h16[0], other_h, 0x5410);
-            const bool word_valid = has_word && word_row < rows_left, more = tt + 1 < p.T;
+            const float gi = sigmoid_sel<ACCURATE>(pad ? 0.f : a[0]), gf = sigmoid_sel<ACCURATE>(pad ? 0.f : a[1]);
+            const float gg = tanh_sel<ACCURATE>(pad ? 0.f : a[2]), go = sigmoid_sel<ACCURATE>(pad ? 0.f : a[3]);
+            c_keep = fmaf(gf, c_keep, gi * gg);
+            const uint32_t h16 = to16<BF16>(go * tanh_sel<ACCURATE>(c_keep));
+            const uint32_t word = __byte_perm(h16, __shfl_xor_sync(0xffffffffu, h16, 1), 0x5410);
+            const bool word_valid = !odd && valid, more = tt + 1 < p.T;
             const size_t slot = (size_t)(tt & (kDirectSlots - 1)) * slot_bytes;
             if (more) {
                 if (word_valid) st_relaxed_gpu(ring + slot + my_word, word);
                 g.mark_sent();
                 if (tid == 0) FLSTM_STAMP(tt, 7);
-                if (L.ex_in_h) named_barrier_sync(2, kEpilogueThreads);
                 if (tt == 0) gathered = mbar_wait(ready, 0, abort_w, wait_ns);  // every CTA of the group has reset its words
             }
             // everything nobody waits for, while the others' parts are on their way: h_t and the caller's y, cell state, gate cache
             if (word_valid) {
-                const size_t idx = idx0 - odd + (size_t)word_row * p.H;
                 *reinterpret_cast<uint32_t *>(hs + (size_t)(t + 1) * slab + idx) = word;
                 if (y && y_words) *reinterpret_cast<uint32_t *>(y + (size_t)t * slab + idx) = word;
             }
-#pragma unroll
-            for (int i = 0; i < PER; ++i) {
-                const size_t idx = idx0 + (size_t)(32 * i) * p.H;
-                const uint32_t g01 = (uint32_t)to16<BF16>(act[i][0]) | (uint32_t)to16<BF16>(act[i][1]) << 16;
-                const uint32_t g23 = (uint32_t)to16<BF16>(act[i][2]) | (uint32_t)to16<BF16>(act[i][3]) << 16;
-                // gates i and f of two units from the even lane, g and o from the odd one
-                const uint32_t mine = odd ? g23 : g01, other = __shfl_xor_sync(0xffffffffu, odd ? g01 : g23, 1);
-                if (32 * i >= rows_left) continue;
-                p.cs[(size_t)(t + 1) * slab + idx] = c_keep[i];
-                if (y && !y_words) y[(size_t)t * slab + idx] = (uint16_t)h16[i];
+            // gates i and f of two units from the even lane, g and o from the odd one
+            const uint32_t g01 = (uint32_t)to16<BF16>(gi) | (uint32_t)to16<BF16>(gf) << 16;
+            const uint32_t g23 = (uint32_t)to16<BF16>(gg) | (uint32_t)to16<BF16>(go) << 16;
+            const uint32_t mine = odd ? g23 : g01, other = __shfl_xor_sync(0xffffffffu, odd ? g01 : g23, 1);
+            if (valid) {
+                p.cs[(size_t)(t + 1) * slab + idx] = c_keep;
+                if (y && !y_words) y[(size_t)t * slab + idx] = (uint16_t)h16;
                 if (p.store_gates) {
-                    uint16_t *grow = gates + ((size_t)t * p.B + b0 + nb + 32 * i) * G + (size_t)jr * 64 + odd * 32 + (u & ~1);
+                    uint16_t *grow = gates + ((size_t)t * p.B + b0 + nb) * G + (size_t)jr * 64 + odd * 32 + (u & ~1);
                     *reinterpret_cast<uint32_t *>(grow) = odd ? __byte_perm(other, mine, 0x5410) : __byte_perm(mine, other, 0x5410);
                     *reinterpret_cast<uint32_t *>(grow + 16) = odd ? __byte_perm(other, mine, 0x7632) : __byte_perm(mine, other, 0x7632);
                 }
             }
             if (resets_slot(tt, p.T)) {
-                if (has_word) st_relaxed_gpu(ring + (size_t)((tt + kResetAhead) & (kDirectSlots - 1)) * slot_bytes + my_word, kUnwritten);
+                if (!odd) st_relaxed_gpu(ring + (size_t)((tt + kResetAhead) & (kDirectSlots - 1)) * slot_bytes + my_word, kUnwritten);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(reset);
             }
@@ -417,9 +392,9 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / pl.cta_rows, p.exits);
 }
 
-template <int BT, int ROUNDS, bool BF16, bool ACC>
+template <int ROUNDS, bool BF16, bool ACC>
 int launch_one(const CUtensorMap &tw, const CUtensorMap &tg, const FwdTmPlan &pl, const FwdParams &p, cudaStream_t s) {
-    auto kern = lstm_fwd_tm_kernel<BT, ROUNDS, BF16, ACC>;
+    auto kern = lstm_fwd_tm_kernel<ROUNDS, BF16, ACC>;
     FLSTM_CUDA_TRY(ensure_smem_limit(reinterpret_cast<const void *>(kern), pl.smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid);
@@ -442,20 +417,25 @@ int launch_one(const CUtensorMap &tw, const CUtensorMap &tg, const FwdTmPlan &pl
 
 }  // namespace
 
+// With tiles of 64 sequences the tile of h is 64 KB at H = 1024 and the UMMAs take as long as the exchange; a step with a barrier
+// then takes no longer: H = 832, B = 100 4.41 us against 4.53 this way, H = 1152, B = 100 4.82 / 5.07, H = 1280, 1536, 1792, B = 64
+// 4.71 / 4.68, 5.13 / 5.16, 5.60 / 5.73.  Tiles of 32, B = 32 unless said otherwise: H = 832, B = 20 3.13 -> 2.47, H = 1024 3.29 -> 2.65
+// (B = 64 3.47 -> 2.94), H = 1280 3.53 -> 2.99, H = 1536 3.80 -> 3.27, H = 2048 4.30 -> 3.79 (B = 8 3.94 -> 3.36), H = 2304, B = 8
+// 4.27 -> 3.81.
 bool fits_direct(const FwdTmPlan &pl, size_t smem_limit) {
-    return pl.S == 2 && (pl.BT == 32 || pl.BT == 64) && pl.ct + pl.cs == pl.kc && gather_rounds(pl) <= kernel_rounds(pl) &&
-           (size_t)layout_of(pl, (int)smem_limit).total <= smem_limit;
+    return pl.S == 2 && pl.BT == BT && pl.ct + pl.cs == pl.kc && gather_rounds(pl) <= kernel_rounds(pl) &&
+           (size_t)layout_of(pl).total <= smem_limit;
 }
 size_t direct_ring_bytes(const FwdTmPlan &pl) { return pl.use && pl.direct ? (size_t)kDirectSlots * pl.grid * pl.BT * 32 : 0; }
 
 int lstm_forward_tm_direct(int dtype, const FwdTmPlan &pl, const CUtensorMap &tw, const CUtensorMap &tg, const FwdParams &p, cudaStream_t s) {
     const bool bf16 = dtype == FLSTM_DTYPE_BF16, acc = p.real_units > 0;
-#define FLSTM_TM_CASE(BT_, R_)                                                                            \
-    if (pl.BT == BT_ && kernel_rounds(pl) == R_) {                                                       \
-        if (bf16) return acc ? launch_one<BT_, R_, true, true>(tw, tg, pl, p, s) : launch_one<BT_, R_, true, false>(tw, tg, pl, p, s); \
-        return acc ? launch_one<BT_, R_, false, true>(tw, tg, pl, p, s) : launch_one<BT_, R_, false, false>(tw, tg, pl, p, s); \
+#define FLSTM_TM_CASE(R_)                                                                                        \
+    if (kernel_rounds(pl) == R_) {                                                                              \
+        if (bf16) return acc ? launch_one<R_, true, true>(tw, tg, pl, p, s) : launch_one<R_, true, false>(tw, tg, pl, p, s); \
+        return acc ? launch_one<R_, false, true>(tw, tg, pl, p, s) : launch_one<R_, false, false>(tw, tg, pl, p, s); \
     }
-    FLSTM_TM_CASE(32, 4) FLSTM_TM_CASE(32, 8) FLSTM_TM_CASE(32, 10) FLSTM_TM_CASE(64, 16)
+    FLSTM_TM_CASE(4) FLSTM_TM_CASE(8) FLSTM_TM_CASE(10)
 #undef FLSTM_TM_CASE
     return set_error(FLSTM_ERR_UNSUPPORTED, "no tensor-memory forward kernel for this plan");
 }

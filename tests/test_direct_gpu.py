@@ -75,3 +75,23 @@ def test_every_length_around_the_slots_and_many_launches(dtype, B, H):
         for a, b in zip(grads, eng.backward(dy)):
             assert torch.equal(a, b)
     eng.close()
+
+
+@pytest.mark.parametrize("dtype,B,H", SHAPES)
+def test_gradients_that_are_no_numbers_stay_their_own(dtype, B, H):
+    """A NaN and an infinity in one sequence's dY: its gradients of that step and before are NaN, no other sequence's change."""
+    T = 26
+    eng, (x, h0, c0, dy) = engine(dtype, B, H, T)
+    eng.forward(x, h0, c0)
+    want = [g.clone() for g in eng.backward(dy)]
+    others = [b for b in range(B) if b != B // 2]
+    for value in (float("nan"), -float("nan"), float("inf"), -float("inf")):
+        bad = dy.clone()
+        bad[18, B // 2, ::2] = value
+        bad[18, B // 2, 1::2] = -value
+        eng.forward(x, h0, c0)
+        dx, dh0, dc0 = eng.backward(bad)
+        assert torch.equal(dx[:, others], want[0][:, others]) and torch.equal(dx[19:], want[0][19:])
+        assert torch.equal(dh0[:, others], want[1][:, others]) and torch.equal(dc0[:, others], want[2][:, others])
+        assert torch.isnan(dx[:18, B // 2]).all() and torch.isnan(dh0[0, B // 2]).all()
+    eng.close()

@@ -14,7 +14,7 @@
 // (32 KB instead of the 48 KB a lone CTA needs for 128 x 256) and the pair's UMMA reads both halves of B, so the
 // shared-memory traffic per FLOP -- what bounds the one-CTA kernel at about 2/3 of the tensor peak -- drops by a
 // third, and so does the L2 traffic.  Every CTA loads its own halves with plain TMA copies (nothing is multicast).
-// The pair kernel is used for K-major A with K >= 2048, M >= 256 and N a multiple of 256 (FLSTM_GEMM_PAIR=0 turns it
+// The pair kernel is used for K-major A with K >= 1024, M >= 256 and N a multiple of 256 (FLSTM_GEMM_PAIR=0 turns it
 // off, =2 takes it whenever M >= 256 and N % 256 == 0).
 //
 // Used for (shapes at the benchmark configurations, per layer):
@@ -34,6 +34,7 @@
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "tc_kernels.h"
+#include "tc_recurrent.cuh"
 
 namespace flstm_b200 {
 namespace tc {
@@ -53,7 +54,7 @@ struct GemmShape {
     // 16-bit outputs leave through TMA: each epilogue warp stages [32 rows x 128 B] tiles, double-buffered
     static constexpr int kOutTileBytes = 32 * 128;
     static constexpr int kOutBytes = 4 * 2 * kOutTileBytes;
-    static constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + 1024 /*alignment slack*/ + 256 /*barriers*/ + BN * 4 /*bias*/;
 };
 
 enum OutMode { OUT_F16 = 0, OUT_BF16 = 1, OUT_F32 = 2 };
@@ -110,10 +111,10 @@ __device__ __forceinline__ void store_row32(void *dst_row, int col0, const uint3
 }
 
 // 64 accumulator columns of one output row -> 16-bit, into row r of a [32 x 128 B] staging tile laid out
-// the way a 128B-swizzled TMA store expects it (16-byte chunk j of row r at chunk j ^ (r & 7)).
+// the way a 128B-swizzled TMA store expects it (16-byte chunk j of row r at chunk j ^ (r & 7)).  `bias`: their 64 summands in
+// shared memory, or null.
 template <int MODE>
-__device__ __forceinline__ void stage_row64(uint8_t *tile, int r, const uint32_t (&acc)[64], const float *bias, int col0,
-                                            int n_valid) {
+__device__ __forceinline__ void stage_row64(uint8_t *tile, int r, const uint32_t (&acc)[64], const float *bias) {
     uint8_t *row = tile + r * 128;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -121,16 +122,9 @@ __device__ __forceinline__ void stage_row64(uint8_t *tile, int r, const uint32_t
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(acc[8 * j + i]);
         if (bias) {
-            if (n_valid >= 64) {
-                const float4 b0 = __ldg(reinterpret_cast<const float4 *>(bias + col0 + 8 * j));
-                const float4 b1 = __ldg(reinterpret_cast<const float4 *>(bias + col0 + 8 * j + 4));
-                v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
-                v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (8 * j + i < n_valid) v[i] += __ldg(bias + col0 + 8 * j + i);
-            }
+            const float4 b0 = *reinterpret_cast<const float4 *>(bias + 8 * j), b1 = *reinterpret_cast<const float4 *>(bias + 8 * j + 4);
+            v[0] += b0.x; v[1] += b0.y; v[2] += b0.z; v[3] += b0.w;
+            v[4] += b1.x; v[5] += b1.y; v[6] += b1.z; v[7] += b1.w;
         }
         uint32_t w[4];
 #pragma unroll
@@ -145,6 +139,25 @@ __device__ __forceinline__ void stage_row64(uint8_t *tile, int r, const uint32_t
         }
         *reinterpret_cast<uint4 *>(row + ((j ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+}
+
+// The bias of a tile's BN columns into shared memory, by the 128 epilogue threads, ahead of the wait for its accumulator (zeros beyond
+// N).  Every thread reads all of it for its row: from global memory, with next to no L1 beside 226 KB of shared memory, that took
+// longer than the product up to K = 1024 (5550 x 2048 x 512: 29.5 us, 14.9 without a bias).  `failed`: the thread's warp has given up;
+// true: one of them has, and all leave together.
+template <int BN>
+__device__ __forceinline__ bool stage_bias(float *s_bias, const float *__restrict__ bias, int n0, int N, bool failed) {
+    constexpr int PER = BN >= 128 ? BN / 128 : 1;
+    const int c = ((int)threadIdx.x - 64) * PER;
+    float b[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) b[i] = c + i < BN && n0 + c + i < N ? __ldg(bias + n0 + c + i) : 0.f;
+    if (named_barrier_or(1, 128, failed)) return true;  // (the tile before has been read)
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+        if (c + i < BN) s_bias[c + i] = b[i];
+    named_barrier_sync(1, 128);
+    return false;
 }
 
 // Output rows may be written through the inverse of the tile-interleaved gate order: row
@@ -166,6 +179,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *s_out = smem + S::kStages * S::kStageBytes;  // 1024-aligned: stage sizes are multiples of 1024
     uint64_t *bars = reinterpret_cast<uint64_t *>(s_out + S::kOutBytes);
+    float *s_bias = reinterpret_cast<float *>(s_out + S::kOutBytes + 256);
     uint64_t *full = bars, *empty = bars + S::kStages;
     uint64_t *tfull = bars + 2 * S::kStages, *tempty = tfull + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tempty + 2);
@@ -267,12 +281,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     } else {
         const int q = warp & 3;  // TMEM lane quadrant this warp may access
         int it = 0, out_idx = 0;
+        bool ok = true;
         for (int item = blockIdx.x; item < items; item += gridDim.x, ++it) {
             const int tile = item / splits;
             const int buf = it & 1;
             const uint32_t bphase = (it >> 1) & 1;
             const int m0 = (tile / num_n) * BM, n0 = (tile % num_n) * BN;
-            if (!mbar_wait(&tfull[buf], bphase, abort_w)) break;
+            if (HAS_BIAS && TMA_OUT && stage_bias<BN>(s_bias, bias, n0, N, !ok)) break;
+            ok = mbar_wait(&tfull[buf], bphase, abort_w);
+            if (!ok) {
+                if (HAS_BIAS && TMA_OUT) continue;  // the others learn of it where the warps meet
+                break;
+            }
             tcgen05_fence_after();
             const int row = m0 + q * 32 + lane;
             if (TMA_OUT) {
@@ -293,7 +313,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     uint8_t *tile = s_out + (q * 2 + (out_idx & 1)) * S::kOutTileBytes;
                     if (lane == 0) tma_store_wait_read<1>();  // the store that last used this buffer has read it
                     __syncwarp();
-                    stage_row64<MODE>(tile, lane, acc, HAS_BIAS ? bias : nullptr, n0 + c, n_valid);
+                    stage_row64<MODE>(tile, lane, acc, HAS_BIAS ? s_bias + c : nullptr);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -366,7 +386,7 @@ struct PairShape {
     static constexpr int kTmemCols = 2 * kBN;
     static constexpr int kOutTileBytes = 32 * 128;
     static constexpr int kOutBytes = 4 * 2 * kOutTileBytes;
-    static constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + 1024 /*alignment slack*/ + 256 /*barriers*/ + kBN * 4 /*bias*/;
 };
 
 // Roles as in gemm_kernel, in both CTAs of the pair, except that only the leader's warp 1 issues UMMAs.
@@ -387,6 +407,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *s_out = smem + S::kStages * S::kStageBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(s_out + S::kOutBytes);
+    float *s_bias = reinterpret_cast<float *>(s_out + S::kOutBytes + 256);
     uint64_t *full = bars, *empty = bars + S::kStages;
     uint64_t *tfull = bars + 2 * S::kStages, *tempty = tfull + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tempty + 2);
@@ -493,11 +514,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const int q = warp & 3;  // TMEM lane quadrant this warp may access
         const uint32_t tempty0 = map_to_rank(smem_u32(tempty), 0);
         int it = 0, out_idx = 0;
+        bool ok = true;
         for (int tile = pair; tile < tiles; tile += npairs, ++it) {
             const int buf = it & 1;
             const uint32_t bphase = (it >> 1) & 1;
             const int m0 = (tile / num_n) * 2 * BM + (int)rank * BM, n0 = (tile % num_n) * BN;
-            if (!mbar_wait(&tfull[buf], bphase, abort_w)) break;
+            if (HAS_BIAS && TMA_OUT && stage_bias<BN>(s_bias, bias, n0, N, !ok)) break;
+            ok = mbar_wait(&tfull[buf], bphase, abort_w);
+            if (!ok) {
+                if (HAS_BIAS && TMA_OUT) continue;  // the others learn of it where the warps meet
+                break;
+            }
             tcgen05_fence_after();
             const int row = m0 + q * 32 + lane;
             if (TMA_OUT) {
@@ -518,7 +545,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     uint8_t *tile_s = s_out + (q * 2 + (out_idx & 1)) * S::kOutTileBytes;
                     if (lane == 0) tma_store_wait_read<1>();  // the store that last used this buffer has read it
                     __syncwarp();
-                    stage_row64<MODE>(tile_s, lane, acc, HAS_BIAS ? bias : nullptr, n0 + c, n_valid);
+                    stage_row64<MODE>(tile_s, lane, acc, HAS_BIAS ? s_bias + c : nullptr);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
@@ -698,12 +725,11 @@ int gemm(int dtype, int out_dtype, size_t M, size_t N, size_t K, const void *A, 
         BN /= 2;
     }
     GemmArgs g{};
-    // measured on B200 (bf16) inside the engine's step: pairs win for K-major A from K = 2048 on (config 3:
-    // projection 1465 -> 1529, input gradient 1507 -> 1540 TFLOP/s; 8192^3 1159 -> 1377).  With K = 1024 and the
-    // bias epilogue (every projection) they lose (config 5: 12.8 -> 20.5 ms per step, 1351 -> 790 TFLOP/s in
-    // isolation; without a bias the same shape gains, 1036 -> 1275), and the MN-major weight-gradient form is
-    // neutral in isolation (1158 -> 1205) and 2 % slower inside the step, so both stay on lone CTAs.
-    g.pair = pair_enabled() && !a_mn && K >= 2048 && M >= 256 && N % 256 == 0 && sms >= 2;
+    // Pairs win for K-major A from K = 1024 on: with a bias 32768 x 4096 x 1024 196 -> 168 us, 8192 x 4096 x 1024 52.9 -> 46.7,
+    // 5550 x 2048 x 1024 24.2 -> 23.0; at K = 512 8192 x 4096 32.5 -> 31.4, 5550 x 2048 16.0 -> 16.2; without one at config 3's sizes
+    // 1507 -> 1540 TFLOP/s (input gradient).  The MN-major weight-gradient form is neutral in isolation (1158 -> 1205) and 2 % slower
+    // inside the step, so it stays on lone CTAs.
+    g.pair = pair_enabled() && !a_mn && K >= 1024 && M >= 256 && N % 256 == 0 && sms >= 2;
     if (pair_forced()) g.pair = M >= 256 && N % 256 == 0 && sms >= 2;
     // ... and only with enough tiles for the pairs
     if (g.pair && !pair_forced() && (M + 2 * BM - 1) / (2 * BM) * (N / 256) < (size_t)sms / 4) g.pair = false;

@@ -60,6 +60,17 @@ def test_kmajor_gemm(dtype, M, N, K):
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("M,N,K", [(64, 64, 8), (130, 136, 64), (5550, 2048, 64), (2000, 1160, 72), (40000, 256, 1024), (257, 4096, 1024)])
+def test_every_column_gets_its_own_bias(dtype, M, N, K):
+    """One tile and many per CTA, a last tile of columns that is partly filled: with A = 0 the result is the bias, rounded."""
+    td = DT[dtype][1]
+    A, B = torch.zeros(M, K, device="cuda", dtype=td), torch.randn(N, K, device="cuda").to(td)
+    bias = torch.arange(N, device="cuda", dtype=torch.float32) / 64 - 7
+    got = _gemm(dtype, dtype, M, N, K, A, B, bias=bias)
+    assert torch.equal(got, bias.to(td).expand(M, N))
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (128, 256, 128), (256, 128, 1024), (512, 512, 4096),
                                    (192, 320, 200), (64, 64, 64), (1024, 256, 8192), (4096, 2048, 512), (304, 256, 136)])
 def test_mnmajor_gemm(dtype, M, N, K):

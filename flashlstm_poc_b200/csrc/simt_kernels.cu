@@ -338,11 +338,67 @@ column_sum_partial_kernel(const T *__restrict__ dg, size_t R, size_t N, int spli
     }
 }
 
+// The same sums in the same order (row lane by row lane, split by split) from 16-byte loads, eight of them under way: what bounds it
+// is the traffic to memory, and 2-byte loads of one row at a time reached 3.7 of 6.5 TB/s (32768 x 4096 16-bit values: 72 -> 38 us;
+// 8192 x 4096: 19.4 -> 9.4; 5550 x 2048: 8.6 -> 6.6).
+template <typename T>
+__global__ void __launch_bounds__(256)
+column_sum_partial_wide_kernel(const T *__restrict__ dg, size_t R, size_t N, int splits, float *__restrict__ partial) {
+    constexpr int V = 16 / sizeof(T), W = 32 * V, AHEAD = 8;
+    __shared__ float part[8][W];
+    const int cl = (threadIdx.x % 32) * V, rl = threadIdx.x / 32;
+    const size_t col = (size_t)blockIdx.x * W + cl;
+    const size_t rows_per = (R + splits - 1) / splits;
+    const size_t r0 = (size_t)blockIdx.y * rows_per;
+    const size_t r1 = r0 + rows_per < R ? r0 + rows_per : R;
+    float s[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) s[v] = 0.f;
+    if (col < N) {
+        auto add = [&](const uint4 &q) {
+            const T *e = reinterpret_cast<const T *>(&q);
+#pragma unroll
+            for (int v = 0; v < V; ++v) s[v] += ld(e + v);
+        };
+        const T *src = dg + (r0 + rl) * N + col;
+        size_t r = r0 + rl;
+        for (; r + 8 * (AHEAD - 1) < r1; r += 8 * AHEAD, src += 8 * AHEAD * N) {
+            uint4 q[AHEAD];
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) q[i] = __ldcs(reinterpret_cast<const uint4 *>(src + i * 8 * N));
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) add(q[i]);
+        }
+        for (; r < r1; r += 8, src += 8 * N) add(*reinterpret_cast<const uint4 *>(src));
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) part[rl][cl + v] = s[v];
+    __syncthreads();
+    for (int c = threadIdx.x; c < W; c += 256) {
+        if ((size_t)blockIdx.x * W + c >= N) continue;
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += part[i][c];
+        partial[(size_t)blockIdx.y * N + (size_t)blockIdx.x * W + c] = t;
+    }
+}
+
+template <typename T>
+void column_sum_partial(const T *dg, size_t R, size_t N, int splits, float *partial, cudaStream_t s) {
+    constexpr size_t V = 16 / sizeof(T);
+    // columns in whole groups of 16 bytes, and rows enough that its few blocks do not count: 4096 x 1024 fp32 values 4.0 us the old way, 5.5
+    if (R >= 5120 && N % V == 0 && (reinterpret_cast<uintptr_t>(dg) & 15) == 0)
+        column_sum_partial_wide_kernel<<<dim3(ceil_div(N, 32 * V), splits), 256, 0, s>>>(dg, R, N, splits, partial);
+    else
+        column_sum_partial_kernel<<<dim3(ceil_div(N, 32), splits), 256, 0, s>>>(dg, R, N, splits, partial);
+}
+
 __global__ void column_sum_final_kernel(const float *__restrict__ partial, size_t N, int splits, float *__restrict__ out,
                                         int unperm_h, int accumulate) {
     const size_t col = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (col >= N) return;
     float t = 0.f;
+#pragma unroll 8
     for (int s = 0; s < splits; ++s) t += partial[(size_t)s * N + col];
     size_t o = col;
     if (unperm_h) {  // tile-interleaved gate order -> torch order
@@ -569,11 +625,10 @@ int column_sum_scratch_floats(size_t N) { return (int)(kColumnSumSplits * N); }
 int column_sum_two_pass(int dtype, const void *dg, size_t R, size_t N, float *scratch, float *out, int unperm_h,
                         cudaStream_t s, bool accumulate) {
     if (N == 0) return FLSTM_OK;
-    dim3 grid(ceil_div(N, 32), kColumnSumSplits);
     switch (dtype) {
-        case FLSTM_DTYPE_F32: column_sum_partial_kernel<<<grid, 256, 0, s>>>((const float *)dg, R, N, kColumnSumSplits, scratch); break;
-        case FLSTM_DTYPE_F16: column_sum_partial_kernel<<<grid, 256, 0, s>>>((const __half *)dg, R, N, kColumnSumSplits, scratch); break;
-        case FLSTM_DTYPE_BF16: column_sum_partial_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16 *)dg, R, N, kColumnSumSplits, scratch); break;
+        case FLSTM_DTYPE_F32: column_sum_partial((const float *)dg, R, N, kColumnSumSplits, scratch, s); break;
+        case FLSTM_DTYPE_F16: column_sum_partial((const __half *)dg, R, N, kColumnSumSplits, scratch, s); break;
+        case FLSTM_DTYPE_BF16: column_sum_partial((const __nv_bfloat16 *)dg, R, N, kColumnSumSplits, scratch, s); break;
         default: return set_error(FLSTM_ERR_INVALID, "column_sum: bad dtype %d", dtype);
     }
     FLSTM_TRY(check_launch("column_sum_partial"));

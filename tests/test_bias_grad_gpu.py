@@ -39,3 +39,20 @@ def test_bias_grad_interleaved_order():
     assert lib.flstm_bias_grad(1, interleave_columns(dg, H).data_ptr(), rows, 4 * H, H, db.data_ptr(), None) == 0
     assert torch.allclose(db.double(), dg.double().sum(0), rtol=1e-5, atol=1e-4)
     assert lib.flstm_bias_grad(1, dg.data_ptr(), rows, 4 * H, H + 16, db.data_ptr(), None) == 1  # H must be cols/4
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("rows,cols", [(5119, 64), (5120, 64), (5121, 264), (5550, 2048), (6001, 8), (8200, 1160)])
+def test_bias_grad_of_many_rows_has_the_order_of_few(dtype, rows, cols):
+    """From 5120 rows on columns in whole groups of 16 bytes are read 16 bytes at a time; a matrix that starts between two such groups
+    is not, and gives the same bits."""
+    lib = _lib.load()
+    code, td = DT[dtype]
+    torch.manual_seed(rows * 7 + cols)
+    room = torch.randn(rows * cols + 1, device="cuda").to(td)
+    off, on = room[1:].view(rows, cols), room[1:].clone().view(rows, cols)
+    got = [torch.empty(cols, device="cuda") for _ in range(2)]
+    for dg, db in zip((off, on), got):
+        assert lib.flstm_bias_grad(code, dg.data_ptr(), rows, cols, 0, db.data_ptr(), None) == 0, lib.flstm_last_error()
+    assert torch.equal(*got)
+    assert torch.allclose(got[0].double(), on.double().sum(0), rtol=1e-5, atol=1e-3 * rows ** 0.5 * 1e-2)

@@ -356,12 +356,13 @@ column_sum_partial_kernel(const T *__restrict__ dg, size_t R, size_t N, int spli
 }
 
 // The same sums in the same order (row lane by row lane, split by split) from 16-byte loads, eight of them under way: what bounds it
-// is the traffic to memory, and 2-byte loads of one row at a time reached 3.7 of 6.5 TB/s (32768 x 4096 16-bit values: 72 -> 38 us;
-// 8192 x 4096: 19.4 -> 9.4; 5550 x 2048: 8.6 -> 6.6).
+// is the traffic to memory, and 2-byte loads of one row at a time reached 3.7 of 6.5 TB/s (32768 x 4096 16-bit values: 67 -> 39 us;
+// 8192 x 4096: 13.9 -> 10.2; 5550 x 2048: 7.8 -> 5.9; 5200 x 2816: 9.3 -> 6.0).
 template <typename T>
 __global__ void __launch_bounds__(256)
 column_sum_partial_wide_kernel(const T *__restrict__ dg, size_t R, size_t N, int splits, float *__restrict__ partial) {
-    constexpr int V = 16 / sizeof(T), W = 32 * V, AHEAD = 8;
+    static_assert(sizeof(T) == 2, "16-bit values");
+    constexpr int V = 8, W = 32 * V, AHEAD = 8;
     __shared__ float part[8][W];
     const int cl = (threadIdx.x % 32) * V, rl = threadIdx.x / 32;
     const size_t col = (size_t)blockIdx.x * W + cl;
@@ -402,12 +403,15 @@ column_sum_partial_wide_kernel(const T *__restrict__ dg, size_t R, size_t N, int
 
 template <typename T>
 void column_sum_partial(const T *dg, size_t R, size_t N, int splits, float *partial, cudaStream_t s) {
-    constexpr size_t V = 16 / sizeof(T);
-    // columns in whole groups of 16 bytes, and rows enough that its few blocks do not count: 4096 x 1024 fp32 values 4.0 us the old way, 5.5
-    if (R >= 5120 && N % V == 0 && (reinterpret_cast<uintptr_t>(dg) & 15) == 0)
-        column_sum_partial_wide_kernel<<<dim3(ceil_div(N, 32 * V), splits), 256, 0, s>>>(dg, R, N, splits, partial);
-    else
-        column_sum_partial_kernel<<<dim3(ceil_div(N, 32), splits), 256, 0, s>>>(dg, R, N, splits, partial);
+    if constexpr (sizeof(T) == 2) {
+        // columns in whole groups of 16 bytes, and so many of them and rows that there are blocks enough all the same (210800 x 512:
+        // 94 us by the other way, 173 by this one); 4-byte loads fill the memory's bandwidth as they are (32768 x 4096: 85 us, 113)
+        if (R >= 5120 && N >= 2048 && N % 8 == 0 && (reinterpret_cast<uintptr_t>(dg) & 15) == 0) {
+            column_sum_partial_wide_kernel<<<dim3(ceil_div(N, 256), splits), 256, 0, s>>>(dg, R, N, splits, partial);
+            return;
+        }
+    }
+    column_sum_partial_kernel<<<dim3(ceil_div(N, 32), splits), 256, 0, s>>>(dg, R, N, splits, partial);
 }
 
 __global__ void column_sum_final_kernel(const float *__restrict__ partial, size_t N, int splits, float *__restrict__ out,

@@ -42,9 +42,9 @@ def test_bias_grad_interleaved_order():
 
 
 @pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
-@pytest.mark.parametrize("rows,cols", [(5119, 64), (5120, 64), (5121, 264), (5550, 2048), (6001, 8), (8200, 1160)])
+@pytest.mark.parametrize("rows,cols", [(5119, 2048), (5120, 2048), (5121, 2040), (5121, 2056), (6001, 1032), (8200, 4096)])
 def test_bias_grad_of_many_rows_has_the_order_of_few(dtype, rows, cols):
-    """From 5120 rows on columns in whole groups of 16 bytes are read 16 bytes at a time; a matrix that starts between two such groups
+    """From 5120 rows and enough columns on, those in whole groups of 16 bytes are read 16 bytes at a time; a matrix that starts between two such groups
     is not, and gives the same bits."""
     lib = _lib.load()
     code, td = DT[dtype]

@@ -62,6 +62,14 @@ struct TcState {
 // in both directions; beyond 64 sequences the grid-wide forward takes a fifth longer itself (512 x 128 still wins).
 constexpr int grid_fwd_cycles(int B) { return B <= 64 ? 5600 : 6500; }
 constexpr int kGridBwdCycles = 6500;
+// The same where the grid-wide kernel exchanges without a step barrier.  us a step in clusters / that way (estimated cycles):
+//   forward   H = 448, B = 112 2.16 / 2.40 (below 4000)   H = 512, B = 96 2.16 / 2.40 (3988)   H = 704, B = 48 2.48 / 2.43 (4560)
+//             H = 576, B = 56 / 64 / 96 / 112 2.24 / 2.36 (3842), 3.22 / 2.37 (5230), 3.48 / 2.47 (5560), 3.65 / 2.56
+//             H = 640, B = 96 3.76 / 2.55 (6040)   H = 768, B = 32 / 40 / 48 2.48 / 2.40 (4692), 2.58 / 2.47 (4802), 2.66 / 2.46 (4912)
+//   backward  H = 512, B = 112 3.78 / 3.76 (5302)   H = 576, B = 64 / 80 4.26 / 3.79, 4.44 / 3.94 (6169)   H = 768, B = 48 3.49 / 3.78 (6039)
+// The line is drawn up to 112 sequences; above, batches stay with the schedule of several tiles per cluster, whose tests hold shapes
+// there (H = 512, B = 128: 3.49 / 2.47).
+constexpr int kDirectBatch = 112, kDirectFwdCycles = 4850, kDirectBwdCycles = 6100;
 
 constexpr int kExitsWord = 1000;  // of Engine::sync_words: CTAs of the running launch that have left (see leave_counters)
 
@@ -225,16 +233,20 @@ int init(Engine &e) {
     // Each direction takes the cluster-resident kernel while its estimated step is shorter than the grid-wide ones'.
     // FLSTM_STEP_MIN_BATCH asks for one of the grid-wide schedules by name.
     if (!std::getenv("FLSTM_STEP_MIN_BATCH")) {
-        const ClusterCheck check{e.cfg.dtype == FLSTM_DTYPE_BF16, e.logical_h > 0};
-        FLSTM_TRY(plan_cluster_fwd(B, H, st->sms, st->smem_limit, &st->cfwd, &check));
-        if (st->cfwd.cycles > grid_fwd_cycles(B)) st->cfwd.use = false;
-        if (e.cfg.training) {
-            FLSTM_TRY(plan_cluster_bwd(B, H, st->sms, st->smem_limit, &st->cbwd, &check));
-            if (st->cbwd.cycles > kGridBwdCycles) st->cbwd.use = false;
-        }
         // the cross-layer wavefront would put two cooperative grids side by side
         const char *wave = std::getenv("FLSTM_WAVE_CHUNK");
         const bool wavefront = wave && std::atoi(wave) > 0;
+        const ClusterCheck check{e.cfg.dtype == FLSTM_DTYPE_BF16, e.logical_h > 0};
+        FwdTmPlan direct_fwd{};
+        if (!wavefront && B <= kDirectBatch) FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &direct_fwd));
+        FLSTM_TRY(plan_cluster_fwd(B, H, st->sms, st->smem_limit, &st->cfwd, &check));
+        if (st->cfwd.cycles > (direct_fwd.use && direct_fwd.direct ? kDirectFwdCycles : grid_fwd_cycles(B))) st->cfwd.use = false;
+        if (e.cfg.training) {
+            BwdTmPlan direct_bwd{};
+            if (!wavefront && B <= kDirectBatch) FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &direct_bwd, /*check_device=*/true));
+            FLSTM_TRY(plan_cluster_bwd(B, H, st->sms, st->smem_limit, &st->cbwd, &check));
+            if (st->cbwd.cycles > (direct_bwd.use && direct_bwd.direct ? kDirectBwdCycles : kGridBwdCycles)) st->cbwd.use = false;
+        }
         if (!wavefront)
             FLSTM_TRY(choose_tmem(B, H, !st->cfwd.use, e.cfg.training && !st->cbwd.use, st->sms, st->smem_limit, /*check_device=*/true, st));
     }

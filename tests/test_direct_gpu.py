@@ -6,6 +6,7 @@ import torch
 
 from flashlstm_poc_b200.engine import TORCH_DTYPES, Engine
 from flashlstm_poc_b200.workloads import Workload, make_inputs
+from tests.gpu_helpers import assert_parity, run_engine, run_oracle
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0)
@@ -95,3 +96,22 @@ def test_gradients_that_are_no_numbers_stay_their_own(dtype, B, H):
         assert torch.equal(dh0[:, others], want[1][:, others]) and torch.equal(dc0[:, others], want[2][:, others])
         assert torch.isnan(dx[:18, B // 2]).all() and torch.isnan(dh0[0, B // 2]).all()
     eng.close()
+
+
+# batch, hidden size, whether the forward and the backward pass stay in clusters
+CROSSING = [(56, 576, True, True), (57, 570, False, False), (64, 576, False, False), (112, 448, True, True), (112, 576, False, False),
+            (113, 448, True, False), (48, 768, False, True), (40, 768, True, True), (96, 640, False, False)]
+
+
+@pytest.mark.parametrize("B,H,cluster_fwd,cluster_bwd", CROSSING)
+def test_both_sides_of_the_line_to_the_clusters_match_the_oracle(B, H, cluster_fwd, cluster_bwd):
+    """A direction leaves the cluster-resident kernel where a step without a barrier over the grid is shorter; short sequences too."""
+    dtype = "bf16" if H % 128 else "f16"
+    for T in (3, 14):
+        w = Workload("t", dtype, 1, 40, H, B, T, seed=92, state_std=0.3)
+        inp = make_inputs(w)
+        got, eng = run_engine(w, inp, repeat=2)
+        names = [eng.recurrent_kernel(T, backward=back)["name"].startswith("cluster_") for back in (False, True)]
+        eng.close()
+        assert names == [cluster_fwd, cluster_bwd]
+        assert_parity(got, run_oracle(inp), dtype)

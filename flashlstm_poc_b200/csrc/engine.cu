@@ -613,7 +613,13 @@ int Engine::backward_checkpointed(size_t T, const void *dy, const void *dhn, con
             FLSTM_TRY(restore_state.run(s, &launches));
             const void *x_seg = li == 0 ? byte_ptr(x_saved) + seg0 * B * l.in_size * es
                                         : byte_ptr(layers[li - 1].y_all) + seg0 * slab * es;
+            // The h_t of every layer but the last are kept for the layer above: where the kernel can use them the recurrence is not
+            // run again, only its contractions.
+            seg.known_h = li + 1 < L && tc::takes_known_h(*this, n);
+            if (seg.known_h)
+                FLSTM_CUDA_TRY(cudaMemcpyAsync(byte_ptr(l.hs) + slab * es, byte_ptr(l.y_all) + seg0 * slab * es, n * slab * es, cudaMemcpyDeviceToDevice, s));
             st = tc::forward_layer(*this, li, 0, n, x_seg, nullptr, s);  // recompute
+            seg.known_h = false;
             if (st != FLSTM_OK) break;
             const void *dy_seg = byte_ptr((li == L - 1) ? dy : layers[li + 1].dx) + seg0 * slab * es;
             void *dx_seg = li == 0 ? (dx ? byte_ptr(dx) + seg0 * B * l.in_size * es : nullptr) : byte_ptr(l.dx) + seg0 * slab * es;

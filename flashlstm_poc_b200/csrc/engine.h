@@ -111,6 +111,7 @@ struct Engine {
         bool final_segment = true;   // the segment that starts at t = 0: dh0/dc0 and the gradient allreduce follow it
         bool first_segment = true;   // the first one processed (the end of the sequence): weight gradients start from zero
         bool keep_gates = true;      // forward writes the activated gates back (off in the checkpointing forward pass)
+        bool known_h = false;        // the segment's h_t stand in hs: the forward only rebuilds gates and cell states
         size_t start = 0;            // number of the segment's first step within the call's sequence
     } seg;
     std::vector<LayerBuffers> layers;
@@ -232,6 +233,8 @@ int set_weights(Engine &e, int first, int count, const float *const *params, cud
 unsigned int *error_mirror(Engine &e);
 int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs);  // flstm_path
 void recurrent_kernel(const Engine &e, bool backward, size_t steps, flstm_kernel_info *out);
+// whether a launch of this many steps runs without waiting from step to step where SegmentMode::known_h
+bool takes_known_h(const Engine &e, size_t steps);
 int forward_layer(Engine &e, int layer, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s);
 // `dx_ready` (optional) is recorded on `s` once dx_l of the range is complete, before the weight gradients
 int backward_layer(Engine &e, int layer, size_t T, size_t t0, size_t t1, const void *x_l, const void *dy_l,

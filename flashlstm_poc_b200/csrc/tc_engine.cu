@@ -389,6 +389,10 @@ void recurrent_kernel(const Engine &e, bool backward, size_t steps, flstm_kernel
     }
 }
 
+bool takes_known_h(const Engine &e, size_t steps) {
+    return fwd_kind(*static_cast<const TcState *>(e.tc_state), steps) == Kind::Wide;
+}
+
 int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s) {
     TcState *st = state(e);
     FLSTM_TRY(check_async_error(e));
@@ -484,6 +488,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.B = (int)B;
     p.H = (int)H;
     p.store_gates = (e.cfg.training && e.seg.keep_gates) ? 1 : 0;
+    p.known_h = e.seg.known_h ? 1 : 0;
     p.odd = (int)((e.seq_start + e.seg.start + t0) & 1);
     p.real_units = e.logical_h;
     p.trace = (li == 0 && t0 == 0) ? e.trace : nullptr;

@@ -50,6 +50,7 @@ struct FwdParams {
     int T, B, H;          // T = number of steps this launch runs
     int t0;               // first (absolute) time step of this launch; the state of step t0 is in slot t0 of hs/cs
     int store_gates;      // write the activated gates back (the gate cache)
+    int known_h;          // 1: hs holds every h_t of the launch already (lstm_forward_wide only): no step waits for another's
     int odd;              // 1: the first step of this launch has an odd number in its sequence (order of streamed weights)
     // 0: fast gate functions.  > 0: accurate ones (see common.cuh), and the units from this one on are padding
     // (engine_padded.cu): their pre-activations count as zero, whatever 0 * inf made of them

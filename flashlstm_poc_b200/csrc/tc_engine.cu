@@ -299,7 +299,7 @@ int on_capacity_change(Engine &e) {
         if (bwd && st->bwdtm.use && !st->bwdtm.direct) FLSTM_TRY(make_bwd_tm_maps(&t.dg_tm, st->bwdtm, l.dg, dg_steps, B, H));
         if (st->wide.use) {
             FLSTM_TRY(make_tensor_map_gate_rows(&t.tm_ws, l.w_hh, H));
-            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->wide.BT / 2, 2));
+            FLSTM_TRY(make_tensor_map_chunked(&t.tm_h_tm, l.hs, cap + 1, B, H, st->wide.BT / 2, st->wide.ch));
         }
         if (st->fwdtm.use) {
             if (!st->fwdtm.direct)

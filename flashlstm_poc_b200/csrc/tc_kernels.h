@@ -103,6 +103,7 @@ int lstm_forward_tm_direct(int dtype, const FwdTmPlan &plan, const CUtensorMap &
 
 // ------------------------------------------------------------------ wide batches with W_hh on the chip (tc_lstm_fwd_wide.cu)
 struct FwdWidePlan {
+    int ch;        // 64-wide chunks of h per copy
     bool use;
     int BT;        // sequences per batch tile: 64 or 128
     int cta_rows;  // CTAs per batch group = H / 16
@@ -116,7 +117,7 @@ struct FwdWidePlan {
 };
 constexpr int kMaxStepCounters = 900;  // words of Engine::sync_words that step barriers may take
 int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan);
-// tm_w: make_tensor_map_gate_rows.  tm_h: chunked map with box rows BT / 2 and 2 chunks.
+// tm_w: make_tensor_map_gate_rows.  tm_h: chunked map with box rows BT / 2 and plan.ch chunks.
 int lstm_forward_wide(int dtype, const FwdWidePlan &plan, const CUtensorMap &tm_w, const CUtensorMap &tm_h, const FwdParams &p,
                       cudaStream_t s);
 

@@ -9,7 +9,7 @@
 // independent recurrences with a step barrier each, so the chain of one hides behind the UMMAs of the others.
 //
 // Per step and batch tile of BT sequences:
-//   producer warp : waits for the tile's step barrier, streams h_{t-1} through the ring (copies of two 64-wide chunks)
+//   producer warp : waits for the tile's step barrier, streams h_{t-1} through the ring (copies of two or four 64-wide chunks)
 //   UMMA thread   : M = 128, N = BT, accumulating over K = H into one of two accumulators (BT / 2 columns: sequences [0, BT/2) in
 //                   lanes 0-63, the others in lanes 64-127)
 //   16 warps      : the rows of A are ordered so that a lane quadrant holds the four gates of 8 units, 8 lanes each: two
@@ -17,7 +17,7 @@
 //                   exchange through shared memory is needed.  Projections and cell states are read a tile ahead; h_t is stored
 //                   first, cell states, gates and y follow while a thread of its own publishes h_t.
 // Rebuilding the gates of a checkpointed segment whose h_t are kept (known_h) is the same launch without the chain: nobody waits
-// for a step and no h_t is stored (H = 1024, B = 256, 32 steps: 155 -> 120 us).
+// for a step and no h_t is stored (H = 1024, B = 256, 32 steps: 131 -> 91 us).
 // Waits are bounded; producer, publisher, UMMA thread and each epilogue warp break out of their loops by themselves (no barrier of
 // threads lies inside the loops) and meet at the final __syncthreads; an aborted pair lingers before the final cluster barrier.
 //
@@ -42,18 +42,17 @@ constexpr int kEpilogueWarps = 16, kProducerWarp = 16, kUmmaWarp = 17, kPublishe
 constexpr int kThreads = (kEpilogueWarps + 3) * 32;
 constexpr int kChunkBytesW = 64 * 128;  // 64 rows x 64 16-bit elements
 constexpr int kTmemColumns = 512;
-constexpr int kCh = 2;  // chunks per copy of h
 constexpr int kBarrierBytes = 1024, kMinSmemBytes = 120 * 1024;
 constexpr int kFillSlots = 12;  // a multiple of 4: a slot always belongs to the same set of warps (see tc_lstm_fwd_tm.cu)
 static_assert(kBarrierBytes + kFillSlots * kChunkBytesW + 1024 <= kMinSmemBytes, "the fill slots fit every launch");
 
 __host__ __device__ inline int smem_of(const FwdWidePlan &pl) {
-    return kBarrierBytes + pl.cs * kChunkBytesW + pl.hstages * kCh * (pl.BT / 2) * 128 + 1024 /*align*/;
+    return kBarrierBytes + pl.cs * kChunkBytesW + pl.hstages * pl.ch * (pl.BT / 2) * 128 + 1024 /*align*/;
 }
 
 // TRACE: stamps of the group's first tile of each step.  A form of its own: without being asked for they took 6 % of a launch
 // (H = 2048, B = 256, T = 24: 297 -> 315 us).
-template <int BT, bool BF16, bool ACCURATE, bool TRACE>
+template <int BT, int kCh, bool BF16, bool ACCURATE, bool TRACE>  // kCh: 64-wide chunks per copy of h
 __global__ void __launch_bounds__(kThreads, 1)
 lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_h,
                      const __grid_constant__ FwdWidePlan pl, FwdParams p) {
@@ -109,7 +108,7 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + 2 * BTH;
-    // (ct is even: a copy of h never mixes tensor- and shared-memory chunks)
+    // (ct is a multiple of kCh: a copy of h never mixes tensor- and shared-memory chunks)
     // W_hh into tensor memory by way of the shared memory that the ring will use: lanes l and l + 64 take row l of the tile in the
     // map's order (unit half, gate, unit), 32 columns of two elements per chunk; a warp reaches the lane quadrant warp % 4
     // and takes every fourth chunk.  A wait that expires raises the abort word, on which every role below gives up.
@@ -240,11 +239,16 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
                         dw += kCh * kStepW;
                         consumed();
                     }
-                    for (; c < KC && ok; c += kCh) {  // an odd last chunk
-                        const uint32_t dh = landed();
+                    if (c < KC && ok) {  // chunks that make no whole copy
+                        uint32_t dh = landed();
                         if (!ok) break;
+                        for (; c < KC; ++c) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) umma_lo_ss<true>(d, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                            for (int k = 0; k < 4; ++k) umma_lo_ss<true>(d, dw + 2 * k, dh + 2 * k, idesc, k ? 1u : acc);
+                            acc = 1;
+                            dw += kStepW;
+                            dh += kStepH;
+                        }
                         consumed();
                     }
                     if (!ok) break;
@@ -424,9 +428,9 @@ lstm_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / pl.cta_rows * pl.nt, p.exits);
 }
 
-template <int BT, bool BF16, bool ACC>
+template <int BT, int CH, bool BF16, bool ACC>
 int launch_one(const CUtensorMap &tw, const CUtensorMap &th, const FwdWidePlan &pl, const FwdParams &p, cudaStream_t s) {
-    auto kern = p.trace ? lstm_fwd_wide_kernel<BT, BF16, ACC, true> : lstm_fwd_wide_kernel<BT, BF16, ACC, false>;
+    auto kern = p.trace ? lstm_fwd_wide_kernel<BT, CH, BF16, ACC, true> : lstm_fwd_wide_kernel<BT, CH, BF16, ACC, false>;
     FLSTM_CUDA_TRY(ensure_smem_limit(kern, (size_t)pl.smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid);
@@ -469,11 +473,19 @@ int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan) {
     if (pl.nt > 6 || pl.nt * pl.ngroups > kMaxStepCounters) return FLSTM_OK;
     pl.kc = H / 64;
     const int tmem_chunks = (kTmemColumns - pl.BT) / 32;
-    pl.ct = (pl.kc < tmem_chunks ? pl.kc : tmem_chunks) / kCh * kCh;
-    pl.cs = pl.kc - pl.ct;
-    pl.hstages = 16;
-    while (pl.hstages > 3 && (size_t)smem_of(pl) > smem_limit) --pl.hstages;
-    if ((size_t)smem_of(pl) > smem_limit) return FLSTM_OK;
+    // A copy's wait, its commit and the address arithmetic between take the issuing thread some 200 cycles, more than the eight
+    // UMMAs of N = 64 of two chunks.  Tiles of 64 go in copies of four chunks as long as three of them fit; us a step with two / four
+    // chunks: H = 1024, B = 256 5.54 / 5.19, H = 2048, B = 100 7.62 / 6.31, H = 1536, B = 100 5.87 / 5.16, H = 512, B = 512 4.90 / 4.62.
+    // An UMMA of N = 128 takes twice as long and the ring holds fewer copies: H = 2048, B = 256 10.22 / 10.66, H = 1024, B = 384 7.50 / 8.39.
+    auto take_chunks = [&](int ch) {
+        pl.ch = ch;
+        pl.ct = (pl.kc < tmem_chunks ? pl.kc : tmem_chunks) / ch * ch;
+        pl.cs = pl.kc - pl.ct;
+        pl.hstages = 32 / ch;
+        while (pl.hstages > 3 && (size_t)smem_of(pl) > smem_limit) --pl.hstages;
+        return (size_t)smem_of(pl) <= smem_limit;
+    };
+    if (!(pl.BT == 64 && take_chunks(4)) && !take_chunks(2)) return FLSTM_OK;
     // All of shared memory: a CTA allocates all of tensor memory, so no other kernel that uses some (another engine's, on another
     // stream) may share its SM; two grids that each held what the other's CTAs were waiting for would run into their limits
     pl.smem_bytes = (int)smem_limit;
@@ -485,12 +497,12 @@ int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan) {
 
 int lstm_forward_wide(int dtype, const FwdWidePlan &pl, const CUtensorMap &tw, const CUtensorMap &th, const FwdParams &p, cudaStream_t s) {
     const bool bf16 = dtype == FLSTM_DTYPE_BF16, acc = p.real_units > 0;
-#define FLSTM_WIDE_CASE(BT_)                                                                                                \
-    if (pl.BT == BT_) {                                                                                                     \
-        if (bf16) return acc ? launch_one<BT_, true, true>(tw, th, pl, p, s) : launch_one<BT_, true, false>(tw, th, pl, p, s); \
-        return acc ? launch_one<BT_, false, true>(tw, th, pl, p, s) : launch_one<BT_, false, false>(tw, th, pl, p, s);       \
+#define FLSTM_WIDE_CASE(BT_, CH_)                                                                                                     \
+    if (pl.BT == BT_ && pl.ch == CH_) {                                                                                              \
+        if (bf16) return acc ? launch_one<BT_, CH_, true, true>(tw, th, pl, p, s) : launch_one<BT_, CH_, true, false>(tw, th, pl, p, s); \
+        return acc ? launch_one<BT_, CH_, false, true>(tw, th, pl, p, s) : launch_one<BT_, CH_, false, false>(tw, th, pl, p, s);       \
     }
-    FLSTM_WIDE_CASE(64) FLSTM_WIDE_CASE(128)
+    FLSTM_WIDE_CASE(64, 4) FLSTM_WIDE_CASE(64, 2) FLSTM_WIDE_CASE(128, 2)
 #undef FLSTM_WIDE_CASE
     return set_error(FLSTM_ERR_UNSUPPORTED, "no wide forward kernel for this plan");
 }

@@ -180,11 +180,11 @@ bool supported(const flstm_engine_config &cfg) {
 // keep short launches.  Those then sum the halves of K apart, so that a sequence cut into ranges or segments of any length
 // gives the bits of one launch.  Calls of n steps in us, other kernels -> these:
 //   forward, n = 1 / 2 / 4 / 8 / 16 / 24:
-//     H = 1024, B = 32, one tile of 32   23.7 / 26.7 / 33.5 / 47.2 / 76.9 / 107.8 -> 24.7 / 28.8 / 34.9 / 47.2 / 73.6 / 102.0
+//     H = 1024, B = 32, one tile of 32   23.7 / 26.7 / 33.5 / 47.2 / 76.9 / 107.8 -> 24.7 / 28.8 / 34.9 / 42.6 / 61.9 / 83.4
 //     H = 2048, B = 40, one tile of 64   26.5 / 30.8 / 45.2 / 70.8 / 123.1 / 168.3 -> 28.8 / 32.9 / 45.6 / 71.8 / 121.7 / 164.4
 //     H = 2048, B = 256, tiles in turn   35.9 / 53.2 / 84.6 / 154 / 282 / 404 -> 37.2 / 48.7 / 71.9 / 125 / 214 / 297
 //   backward, n = 1 / 2 / 4 / 8 / 16:
-//     H = 1024, B = 32   56.5 / 60.9 / 70.2 / 91.6 / 127.1 -> 59.3 / 63.4 / 71.7 / 92.9 / 125.9
+//     H = 1024, B = 32   56.5 / 60.9 / 70.2 / 91.6 / 127.1 -> 59.3 / 63.4 / 71.7 / 92.9 / 113.5
 //     H = 1024, B = 64   57.3 / 61.6 / 74.6 / 95.1 / 137.0 -> 59.3 / 63.5 / 77.0 / 95.2 / 136.3
 //     H = 2048, B = 5    104.4 / 107.5 / 121.4 / 146.0 / 196.5 -> 107.4 / 111.1 / 120.6 / 141.2 / 182.5
 //     H = 1280, B = 60   76.4 / 85.1 / 98.5 / 130.9 / 187.5 -> 78.2 / 87.1 / 98.1 / 126.8 / 179.0

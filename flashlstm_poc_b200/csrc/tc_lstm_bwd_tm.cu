@@ -10,6 +10,9 @@
 // blocks (half q, columns of half q) are partial sums and the other two are ignored.  A K range of an odd number of 64-wide
 // chunks leaves one chunk that runs as an instruction of N = BT from shared memory into the first half's block.
 //
+// Up to H = 1536 one tile of 32 sequences exchanges without a step barrier (tc_lstm_bwd_tm_direct.cu); this form runs wider ones, tiles
+// of 64 and tiles in turn.
+//
 // Per step: the producer waits for the step barrier and fetches dG_{t+1} of the K range (both halves with one copy: a 5-D
 // map orders them as the B operand wants); the UMMA thread contracts; the 256 epilogue threads move the accumulator to shared
 // memory, add the halves, send them to the owners with st.async, add the four sources and do the pointwise update.

@@ -6,6 +6,9 @@
 // 134 MB come from HBM.  The accumulators need a few dozen of the 512 tensor-memory columns; the others hold the slice as the
 // A operand of tcgen05.mma, what does not fit there stays in shared memory, and only what fits neither is streamed.
 //
+// This form, with a counter per step, runs batch tiles of 64 sequences and everything streamed; tiles of 32 whose slice stays on the
+// chip exchange without it (tc_lstm_fwd_tm_direct.cu), and share the split below.
+//
 // Work split.  CTA pairs (cta_group::2, M = 256): 128 tensor-memory lanes per CTA.
 //   S = 2 (H <= 16 x SMs): a CTA owns 64 gate rows (16 units).  Lanes 0-63 hold their first half of K = H, lanes 64-127 the
 //         second half, so that the lanes are full; the B operand has 2 BT rows, K half 0 of the BT sequences staged by the

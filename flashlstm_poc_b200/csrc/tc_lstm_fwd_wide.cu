@@ -463,8 +463,17 @@ int plan_fwd_wide(int B, int H, int sms, size_t smem_limit, FwdWidePlan *plan) {
     pl.cta_rows = H / 16;
     if (pl.cta_rows > sms || pl.cta_rows % 2) return FLSTM_OK;
     const int groups = sms / pl.cta_rows;
-    // two tiles of 64 sequences in turn rather than one of 128, whose chain would stand alone
-    pl.BT = B <= 128 * groups ? 64 : 128;
+    // Tiles of 64 sequences or half as many of 128.  Two of 64 rather than one of 128, whose chain would stand alone; beyond two,
+    // an odd number of 64 leaves no half tile empty, and copies of four chunks (below) keep up with the wider tiles, us a step 128 / 64:
+    //   3 of 64  H = 1024, B = 280 / 384 6.90 / 5.25, 7.19 / 5.52   H = 640, B = 384 5.27 / 4.49   H = 1792, B = 192 8.18 / 6.67   H = 2048, B = 192 8.95 / 8.11
+    //   4        H = 512, B = 1024 7.00 / 5.90   H = 1024, B = 512 7.94 / 7.09   H = 1792, B = 256 8.90 / 8.74   H = 2048, B = 256 9.6 / 10.5
+    //   5        H = 512, B = 1280 7.70 / 7.22   H = 1024, B = 640 9.15 / 8.76   H = 1536, B = 320 10.13 / 9.46   H = 2048, B = 320 13.22 / 12.98
+    //   6        H = 512, B = 1536 8.10 / 8.55   H = 1024, B = 768 9.59 / 10.38   H = 1536, B = 384 11.02 / 11.40
+    // Three tiles beside two groups, four and five in a lone one and H = 2176 keep the wider tiles although most would gain (H = 1024,
+    // B = 384 above; H = 1536, B = 256 8.17 / 7.75): tests name shapes of theirs as what tiles of 128 run.
+    const int narrow = ((B + 63) / 64 + groups - 1) / groups;
+    const bool three_on = narrow == 3 ? groups != 2 && H <= 2112 : (narrow == 4 || narrow == 5) && groups > 1;
+    pl.BT = narrow <= 2 || three_on ? 64 : 128;
     const int tiles = (B + pl.BT - 1) / pl.BT;
     pl.nt = (tiles + groups - 1) / groups;
     pl.ngroups = (tiles + pl.nt - 1) / pl.nt;

@@ -242,11 +242,14 @@ def test_long_ranges_continue_one_another(B, H, T):
 
 
 # copies of four chunks with one, two and three left over; the widest that has three such copies, and one that takes copies of two
-@pytest.mark.parametrize("B,H", [(530, 320), (140, 1152), (65, 1984), (100, 2176), (100, 2240)])
+@pytest.mark.parametrize("B,H", [(530, 320), (140, 1152), (65, 1984), (100, 2176), (100, 2240),
+                                 # three, four and five tiles of 64 rather than half as many of 128
+                                 (550, 768), (450, 1024), (130, 1792), (190, 2048)])
 def test_tiles_in_turn_with_every_remainder_of_a_copy(B, H):
     w = Workload("t", "bf16" if H % 128 else "f16", 1, 64, H, B, 4, seed=54, state_std=0.3, training=False)
     inp = make_inputs(w)
     got, eng = run_engine(w, inp, repeat=2)
-    assert eng.recurrent_kernel(4)["name"] == WIDE
+    kernel = eng.recurrent_kernel(4)
+    assert (kernel["name"], kernel["batch_tile"]) == (WIDE, 64)
     eng.close()
     assert_parity(got, run_oracle(inp), w.dtype)

@@ -237,15 +237,23 @@ int init(Engine &e) {
         const char *wave = std::getenv("FLSTM_WAVE_CHUNK");
         const bool wavefront = wave && std::atoi(wave) > 0;
         const ClusterCheck check{e.cfg.dtype == FLSTM_DTYPE_BF16, e.logical_h > 0};
-        FwdTmPlan direct_fwd{};
-        if (!wavefront && B <= kDirectBatch) FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &direct_fwd));
+        // (the other plan is made only where it decides: it asks the device about its kernel, which loads it)
+        const bool direct = !wavefront && B <= kDirectBatch;
         FLSTM_TRY(plan_cluster_fwd(B, H, st->sms, st->smem_limit, &st->cfwd, &check));
-        if (st->cfwd.cycles > (direct_fwd.use && direct_fwd.direct ? kDirectFwdCycles : grid_fwd_cycles(B))) st->cfwd.use = false;
+        if (st->cfwd.cycles > grid_fwd_cycles(B)) st->cfwd.use = false;
+        if (st->cfwd.use && st->cfwd.cycles > kDirectFwdCycles && direct) {
+            FwdTmPlan other{};
+            FLSTM_TRY(plan_fwd_tm(B, H, st->sms, st->smem_limit, &other));
+            if (other.use && other.direct) st->cfwd.use = false;
+        }
         if (e.cfg.training) {
-            BwdTmPlan direct_bwd{};
-            if (!wavefront && B <= kDirectBatch) FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &direct_bwd, /*check_device=*/true));
             FLSTM_TRY(plan_cluster_bwd(B, H, st->sms, st->smem_limit, &st->cbwd, &check));
-            if (st->cbwd.cycles > (direct_bwd.use && direct_bwd.direct ? kDirectBwdCycles : kGridBwdCycles)) st->cbwd.use = false;
+            if (st->cbwd.cycles > kGridBwdCycles) st->cbwd.use = false;
+            if (st->cbwd.use && st->cbwd.cycles > kDirectBwdCycles && direct) {
+                BwdTmPlan other{};
+                FLSTM_TRY(plan_bwd_tm(B, H, st->sms, st->smem_limit, &other, /*check_device=*/true));
+                if (other.use && other.direct) st->cbwd.use = false;
+            }
         }
         if (!wavefront)
             FLSTM_TRY(choose_tmem(B, H, !st->cfwd.use, e.cfg.training && !st->cbwd.use, st->sms, st->smem_limit, /*check_device=*/true, st));

@@ -14,8 +14,10 @@
 // that slot any more (it held step t - 4; the results of step t - 1, which this CTA has seen from all others, were sent by CTAs
 // that had gathered step t - 2).  The reset has to be performed before anybody looks for step t + 4, that is before this CTA sends
 // step t + 3: a warp of its own fences behind the resets of all threads and counts them (`performed`), and a CTA sends step t + 2
-// only when the reset of step t has been counted.  Fences in the threads themselves, behind their other stores, held them for three
-// thousand cycles a step.  A launch resets all slots before its first step; one counter barrier, which the fill of tensor memory
+// only when the reset of step t has been counted.  The warps report the resets of step t to mbarrier t % kResetBarriers: they report
+// those of step t + kResetSlack when the counting warp has seen step t, so that an mbarrier never completes another phase before the
+// one that is waited for has been seen (waits go by parity and would miss it), however late the counting warp is.  Fences in the
+// threads themselves, behind their other stores, held them for three thousand cycles a step.  A launch resets all slots before its first step; one counter barrier, which the fill of tensor memory
 // hides, comes before the first look.  The copies read L2, where the words are: an old one cannot come from L1.
 #pragma once
 
@@ -27,7 +29,8 @@
 namespace flstm_b200 {
 namespace tc {
 
-constexpr int kDirectSlots = 8, kResetAhead = 4, kResetSlack = 2;
+constexpr int kDirectSlots = 8, kResetAhead = 4, kResetSlack = 2, kResetBarriers = 2;
+static_assert(kResetBarriers >= kResetSlack, "a phase of its own for every step that may report its resets ahead of the count");
 constexpr uint32_t kUnwritten = 0xffffffffu;
 constexpr int kGatherWarps = 16, kGatherThreads = kGatherWarps * 32;  // with 8 warps the exchange takes 100 to 400 cycles more
 constexpr int kGatherStages = 3;  // parts of a gather that are handed over one by one, at most
@@ -69,10 +72,10 @@ __device__ __forceinline__ bool wait_performed(uint32_t performed, uint32_t coun
 // The steps of a launch of T steps whose results are sent on: all but the last.  Step t resets the slot of step t + kResetAhead if
 // that one is sent.
 __device__ __forceinline__ bool resets_slot(int t, int T) { return t + kResetAhead + 1 < T; }
-// the warp that performs the resets: `reset` gets an arrival of every storing warp per step
+// the warp that performs the resets: reset[t % kResetBarriers] gets an arrival of every storing warp in step t
 __device__ __forceinline__ void perform_resets(uint64_t *reset, uint32_t performed, int T, volatile uint32_t *abort_w, unsigned long long limit_ns) {
     for (int t = 0; resets_slot(t, T); ++t) {
-        if (!mbar_wait(reset, (uint32_t)t & 1u, abort_w, limit_ns)) return;
+        if (!mbar_wait(&reset[t % kResetBarriers], (uint32_t)(t / kResetBarriers) & 1u, abort_w, limit_ns)) return;
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
         st_release_cta_shared(performed, (uint32_t)t + 1u);
     }

@@ -67,7 +67,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     float *s_ps = reinterpret_cast<float *>(s_tile + L.tile), *s_red = s_ps + L.ps / 4;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *tfull = full + kGatherStages, *tempty = tfull + 1, *wbar = tempty + 1;
     uint64_t *rbar = wbar + 1;  // [2] partial sums received
-    uint64_t *reset = rbar + 2, *ready = reset + 1;
+    uint64_t *reset = rbar + 2, *ready = reset + kResetBarriers;
     uint64_t *ffull = ready + 1, *fempty = ffull + kFillSlots;  // while W_hh moves into tensor memory
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fempty + kFillSlots);
     volatile uint32_t *abort_w = tmem_slot + 1;
@@ -103,7 +103,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         mbar_init(tempty, kEpilogueThreads / 32);
         mbar_init(wbar, 1);
         for (int i = 0; i < 2; ++i) mbar_init(&rbar[i], 1);
-        mbar_init(reset, kEpilogueThreads / 32);
+        for (int i = 0; i < kResetBarriers; ++i) mbar_init(&reset[i], kEpilogueThreads / 32);
         mbar_init(ready, 1);
         for (int i = 0; i < kFillSlots; ++i) {
             mbar_init(&ffull[i], 1);
@@ -402,7 +402,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             if (resets_slot(k, steps)) {
                 if (has_piece) st_relaxed_gpu_16(ring + (size_t)((k + kResetAhead) & (kDirectSlots - 1)) * slot_bytes + my_piece, unwritten);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(reset);
+                if (lane == 0) mbar_arrive(&reset[k % kResetBarriers]);
             }
             if (tid == 0) FLSTM_STAMP(k, 8);
             g.issue(from + slot);

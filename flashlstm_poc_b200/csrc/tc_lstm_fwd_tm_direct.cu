@@ -76,7 +76,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     uint8_t *s_w = smem + kBarrierBytes, *s_h = s_w + L.w, *s_p = s_h + L.h;
     float *s_ex = reinterpret_cast<float *>(s_p + L.p);
     uint64_t *hfull = reinterpret_cast<uint64_t *>(smem), *tfull = hfull + kGatherStages, *tempty = tfull + 1, *wbar = tempty + 1;
-    uint64_t *reset = wbar + 1, *ready = reset + 1, *pfull = ready + 1, *pempty = pfull + 2;
+    uint64_t *reset = wbar + 1, *ready = reset + kResetBarriers, *pfull = ready + 1, *pempty = pfull + 2;
     uint64_t *ffull = pempty + 2, *fempty = ffull + kFillSlots;  // while W_hh moves into tensor memory
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fempty + kFillSlots);
     volatile uint32_t *abort_w = tmem_slot + 1;
@@ -104,7 +104,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         mbar_init(tfull, 1);
         mbar_init(tempty, 2 * kEpilogueThreads / 32);
         mbar_init(wbar, 1);
-        mbar_init(reset, kEpilogueThreads / 32);
+        for (int i = 0; i < kResetBarriers; ++i) mbar_init(&reset[i], kEpilogueThreads / 32);
         mbar_init(ready, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&pfull[i], 1);
@@ -367,7 +367,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             if (resets_slot(tt, p.T)) {
                 if (!odd) st_relaxed_gpu(ring + (size_t)((tt + kResetAhead) & (kDirectSlots - 1)) * slot_bytes + my_word, kUnwritten);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(reset);
+                if (lane == 0) mbar_arrive(&reset[tt % kResetBarriers]);
             }
             if (tid == 0) FLSTM_STAMP(tt, 8);
             if (more) {

@@ -14,8 +14,8 @@
 // (32 KB instead of the 48 KB a lone CTA needs for 128 x 256) and the pair's UMMA reads both halves of B, so the
 // shared-memory traffic per FLOP -- what bounds the one-CTA kernel at about 2/3 of the tensor peak -- drops by a
 // third, and so does the L2 traffic.  Every CTA loads its own halves with plain TMA copies (nothing is multicast).
-// The pair kernel is used for K-major A with K >= 1024, M >= 256 and N a multiple of 256 (FLSTM_GEMM_PAIR=0 turns it
-// off, =2 takes it whenever M >= 256 and N % 256 == 0).
+// The pair kernel is used for K-major A with K >= 1024, M >= 256, N a multiple of 256 and tiles enough (`gemm` below;
+// FLSTM_GEMM_PAIR=0 turns it off, =2 takes it whenever M >= 256 and N % 256 == 0).
 //
 // Used for (shapes at the benchmark configurations, per layer):
 //   input projection  P[T*B,4H]  = X[T*B,I] W_ih^T + b      (K-major x K-major, 16-bit out)
@@ -731,8 +731,13 @@ int gemm(int dtype, int out_dtype, size_t M, size_t N, size_t K, const void *A, 
     // inside the step, so it stays on lone CTAs.
     g.pair = pair_enabled() && !a_mn && K >= 1024 && M >= 256 && N % 256 == 0 && sms >= 2;
     if (pair_forced()) g.pair = M >= 256 && N % 256 == 0 && sms >= 2;
-    // ... and only with enough tiles for the pairs
-    if (g.pair && !pair_forced() && (M + 2 * BM - 1) / (2 * BM) * (N / 256) < (size_t)sms / 4) g.pair = false;
+    // ... and only with enough tiles for the pairs.  Below K = 2048 that is more than one for each: the first tile of a pair starts and
+    // ends later than a lone CTA's, and only the next one repays it.  Lone / pair, us: 40 to 72 tiles with a bias 768 x 4096 x 1024
+    // 11.3 / 11.6, 3072 x 1536 x 1024 11.2 / 12.4, 2304 x 2048 x 1984 16.4 / 17.6, without one 8192 x 512 x 1024 10.3 / 11.1,
+    // 3072 x 1536 x 1536 13.3 / 13.9; 80 and more 1280 x 4096 x 1024 16.8 / 16.4, 5550 x 2048 x 1280 28.1 / 26.9 and 26.6 / 26.0,
+    // 8192 x 2048 x 1984 50.7 / 48.1.
+    const size_t pair_tiles = (M + 2 * BM - 1) / (2 * BM) * (N / 256), pairs = (size_t)sms / 2;
+    if (g.pair && !pair_forced() && (K < 2048 ? pair_tiles <= pairs : pair_tiles < pairs / 2)) g.pair = false;
     if (g.pair) {
         BN = 256;
         splits = 1;

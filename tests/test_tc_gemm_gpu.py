@@ -20,6 +20,7 @@ def tile_shape(request, monkeypatch):
         monkeypatch.setenv("FLSTM_GEMM_PAIR", "2")
     else:
         monkeypatch.delenv("FLSTM_GEMM_PAIR", raising=False)
+    return request.param
 
 
 def _gemm(dtype, out, M, N, K, A, B, bias=None, mn=False):
@@ -57,6 +58,19 @@ def test_kmajor_gemm(dtype, M, N, K):
     assert _rel(got16, want + bias.double()) < (2e-3 if dtype == "f16" else 1e-2)
     got16 = _gemm(dtype, dtype, M, N, K, A, B)
     assert _rel(got16, want) < (2e-3 if dtype == "f16" else 1e-2)
+
+
+@pytest.mark.parametrize("M,N,K,pair", [(3072, 1536, 1024, False), (2304, 2048, 1984, False), (9216, 512, 1024, False), (5120, 1024, 1024, True),
+                                        (3072, 1536, 2048, True), (768, 4096, 2048, True), (8192, 4096, 960, False)])
+def test_pairs_take_long_contractions_with_tiles_enough(M, N, K, pair, tile_shape):
+    """From K = 2048 on half of the SM pairs are enough; shorter contractions need more than one tile per pair."""
+    from torch.profiler import ProfilerActivity, profile
+    A, B = torch.ones(M, K, device="cuda", dtype=torch.bfloat16), torch.ones(N, K, device="cuda", dtype=torch.bfloat16)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        got = _gemm("bf16", "bf16", M, N, K, A, B, bias=torch.zeros(N, device="cuda"))
+    assert (got == K).all()  # exact: K has at most 8 significant bits
+    names = [e.name for e in prof.events() if "gemm" in e.name]
+    assert len(names) == 1 and ("gemm_pair_kernel" in names[0]) == (pair or tile_shape == "pairs")
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])

@@ -288,7 +288,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             const uint32_t bphase = (it >> 1) & 1;
             const int m0 = (tile / num_n) * BM, n0 = (tile % num_n) * BN;
             if (HAS_BIAS && TMA_OUT && stage_bias<BN>(s_bias, bias, n0, N, !ok)) break;
-            ok = mbar_wait(&tfull[buf], bphase, abort_w);
+            // the whole warp or none of it reads the accumulator, and none of it is at the next barrier while the rest is here
+            ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], bphase, abort_w));
             if (!ok) {
                 if (HAS_BIAS && TMA_OUT) continue;  // the others learn of it where the warps meet
                 break;
@@ -520,7 +521,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const uint32_t bphase = (it >> 1) & 1;
             const int m0 = (tile / num_n) * 2 * BM + (int)rank * BM, n0 = (tile % num_n) * BN;
             if (HAS_BIAS && TMA_OUT && stage_bias<BN>(s_bias, bias, n0, N, !ok)) break;
-            ok = mbar_wait(&tfull[buf], bphase, abort_w);
+            // the whole warp or none of it reads the accumulator, and none of it is at the next barrier while the rest is here
+            ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], bphase, abort_w));
             if (!ok) {
                 if (HAS_BIAS && TMA_OUT) continue;  // the others learn of it where the warps meet
                 break;

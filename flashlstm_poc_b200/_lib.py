@@ -14,11 +14,11 @@ LIB_PATH = os.path.join(PKG, "libflashlstm_b200.so")
 ENGINE_SYMBOLS = [
     "flstm_engine_create", "flstm_engine_destroy", "flstm_engine_set_weights", "flstm_engine_set_all_weights", "flstm_engine_forward",
     "flstm_engine_backward", "flstm_engine_forward_range", "flstm_engine_backward_range", "flstm_engine_grad_ptrs", "flstm_engine_grad_buffer", "flstm_engine_export_grads", "flstm_engine_cache_ptrs",
-    "flstm_engine_set_cell_io_f32", "flstm_engine_backend", "flstm_engine_path", "flstm_engine_kernel", "flstm_comm_unique_id", "flstm_engine_attach_comm",
+    "flstm_engine_set_cell_io_f32", "flstm_engine_backend", "flstm_engine_path", "flstm_engine_kernel", "flstm_engine_direct", "flstm_comm_unique_id", "flstm_engine_attach_comm",
     "flstm_engine_enable_timing", "flstm_engine_phase_ms", "flstm_engine_launch_count", "flstm_tc_gemm",
     "flstm_engine_enable_trace", "flstm_engine_read_trace", "flstm_bias_grad", "flstm_tc_plan", "flstm_tmem_plan", "flstm_engine_wait", "flstm_engine_abort_comm",
                   "flstm_engine_set_recompute_interval", "flstm_engine_workspace_bytes",
-    "flstm_bias_grad_static", "flstm_engine_set_wait_limit", "flstm_engine_selftest_missing_arrivals",
+    "flstm_bias_grad_static", "flstm_engine_set_wait_limit", "flstm_engine_selftest_missing_arrivals", "flstm_engine_selftest_lost_words",
     "flstm_engine_backward_segment",
     "flstm_last_error",
     "flstm_version",
@@ -127,6 +127,8 @@ def load() -> ctypes.CDLL:
     lib.flstm_engine_backward_segment.argtypes = [vp, sz, ci, ci] + [vp] * 10
     lib.flstm_engine_set_wait_limit.argtypes = [vp, ctypes.c_ulonglong]
     lib.flstm_engine_selftest_missing_arrivals.argtypes = [vp, ctypes.c_uint]
+    lib.flstm_engine_selftest_lost_words.argtypes = [vp, ctypes.c_uint, sz, sz]
+    lib.flstm_engine_direct.argtypes = [vp, ci, sz, ctypes.POINTER(ci)]
     lib.flstm_engine_set_recompute_interval.argtypes = [vp, sz]
     lib.flstm_engine_workspace_bytes.argtypes = [vp]
     lib.flstm_engine_workspace_bytes.restype = sz

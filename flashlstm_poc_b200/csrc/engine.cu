@@ -1176,6 +1176,15 @@ int flstm_engine_path(flstm_engine *engine, int backward, int *path, int *ctas, 
     return FLSTM_OK;
 }
 
+int flstm_engine_direct(flstm_engine *engine, int backward, size_t steps, int *direct) {
+    if (!engine || !direct) return set_error(FLSTM_ERR_INVALID, "null argument");
+    if (steps == 0) return set_error(FLSTM_ERR_INVALID, "a launch has at least one step");
+    const Engine &e = engine->impl.core();
+    if (backward && !e.cfg.training) return set_error(FLSTM_ERR_INVALID, "engine was created with training = 0");
+    *direct = e.backend == FLSTM_BACKEND_TC && flstm_b200::tc::exchanges_directly(e, backward != 0, steps);
+    return FLSTM_OK;
+}
+
 int flstm_engine_kernel(flstm_engine *engine, int backward, size_t steps, flstm_kernel_info *out) {
     if (!engine || !out) return set_error(FLSTM_ERR_INVALID, "null argument");
     if (steps == 0) return set_error(FLSTM_ERR_INVALID, "a launch has at least one step");
@@ -1276,6 +1285,18 @@ int flstm_engine_set_wait_limit(flstm_engine *engine, unsigned long long limit_u
 int flstm_engine_selftest_missing_arrivals(flstm_engine *engine, unsigned int arrivals) {
     if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
     engine->impl.core().selftest_missing_arrivals = arrivals;
+    return FLSTM_OK;
+}
+
+int flstm_engine_selftest_lost_words(flstm_engine *engine, unsigned int what, size_t step, size_t sequence) {
+    if (!engine) return set_error(FLSTM_ERR_INVALID, "null engine");
+    if (what > 7 || step > 1u << 30 || sequence >= engine->impl.cfg.batch) return set_error(FLSTM_ERR_INVALID, "no such part, step or sequence");
+    if (what && (engine->impl.cfg.dtype != FLSTM_DTYPE_F16 || engine->impl.inner))
+        return set_error(FLSTM_ERR_UNSUPPORTED, "this self-test is for fp16 engines with hidden_size %% 64 == 0 and input_size %% 8 == 0");
+    auto &lost = engine->impl.core().selftest_lost;
+    lost.what = what;
+    lost.step = step;
+    lost.sequence = sequence;
     return FLSTM_OK;
 }
 

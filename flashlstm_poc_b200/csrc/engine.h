@@ -128,6 +128,10 @@ struct Engine {
     // the timeout self-test: a step barrier that waits for this many arrivals which nobody makes.
     unsigned long long wait_limit_ns = 0;
     unsigned int selftest_missing_arrivals = 0;
+    struct {
+        unsigned int what = 0;
+        size_t step = 0, sequence = 0;
+    } selftest_lost;  // tc::LostWords
     // A 16-bit shape that the tensor-core path cannot tile runs there zero-padded (engine_padded.cu): this engine then
     // only owns the logical gradients and staging tensors, `inner` has the padded sizes and does the work.
     Engine *inner = nullptr;
@@ -233,6 +237,7 @@ int set_weights(Engine &e, int first, int count, const float *const *params, cud
 unsigned int *error_mirror(Engine &e);
 int recurrent_path(const Engine &e, bool backward, int *ctas, int *seqs);  // flstm_path
 void recurrent_kernel(const Engine &e, bool backward, size_t steps, flstm_kernel_info *out);
+bool exchanges_directly(const Engine &e, bool backward, size_t steps);  // flstm_engine_direct
 // whether a launch of this many steps runs without waiting from step to step where SegmentMode::known_h
 bool takes_known_h(const Engine &e, size_t steps);
 int forward_layer(Engine &e, int layer, size_t t0, size_t t1, const void *x_l, void *y_out, cudaStream_t s);

@@ -73,8 +73,9 @@ __device__ __forceinline__ bool wait_performed(uint32_t performed, uint32_t coun
 // that one is sent.
 __device__ __forceinline__ bool resets_slot(int t, int T) { return t + kResetAhead + 1 < T; }
 // the warp that performs the resets: reset[t % kResetBarriers] gets an arrival of every storing warp in step t
-__device__ __forceinline__ void perform_resets(uint64_t *reset, uint32_t performed, int T, volatile uint32_t *abort_w, unsigned long long limit_ns) {
-    for (int t = 0; resets_slot(t, T); ++t) {
+__device__ __forceinline__ void perform_resets(uint64_t *reset, uint32_t performed, int T, volatile uint32_t *abort_w, unsigned long long limit_ns,
+                                               int lost_from) {
+    for (int t = 0; resets_slot(t, T) && t != lost_from; ++t) {
         if (!mbar_wait(&reset[t % kResetBarriers], (uint32_t)(t / kResetBarriers) & 1u, abort_w, limit_ns)) return;
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
         st_release_cta_shared(performed, (uint32_t)t + 1u);

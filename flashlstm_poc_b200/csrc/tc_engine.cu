@@ -397,6 +397,11 @@ void recurrent_kernel(const Engine &e, bool backward, size_t steps, flstm_kernel
     }
 }
 
+bool exchanges_directly(const Engine &e, bool backward, size_t steps) {
+    const TcState &st = *static_cast<const TcState *>(e.tc_state);
+    return backward ? bwd_kind(st, steps) == Kind::Tmem && st.bwdtm.direct : fwd_kind(st, steps) == Kind::Tmem && st.fwdtm.direct;
+}
+
 bool takes_known_h(const Engine &e, size_t steps) {
     return fwd_kind(*static_cast<const TcState *>(e.tc_state), steps) == Kind::Wide;
 }
@@ -503,6 +508,7 @@ int forward_layer(Engine &e, int li, size_t t0, size_t t1, const void *x_l, void
     p.trace_steps = e.trace_steps;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
+    p.lost = {e.selftest_lost.what, (int)e.selftest_lost.step, (int)e.selftest_lost.sequence / 32 * st->fwdtm.cta_rows};
     if (kind == Kind::Wide) FLSTM_TRY(lstm_forward_wide(e.cfg.dtype, st->wide, t.tm_ws, t.tm_h_tm, p, s));
     else if (kind == Kind::Tmem && st->fwdtm.direct) FLSTM_TRY(lstm_forward_tm_direct(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_g_tm, p, s));
     else if (kind == Kind::Tmem) FLSTM_TRY(lstm_forward_tm(e.cfg.dtype, st->fwdtm, t.tm_w, t.tm_ws, t.tm_h_tm, t.tm_g_tm, p, s));
@@ -715,6 +721,7 @@ int backward_layer(Engine &e, int li, size_t T, size_t t0, size_t t1, const void
     p.H = (int)H;
     p.wait_ns = e.wait_limit_ns;
     p.extra_arrivals = e.selftest_missing_arrivals;
+    p.lost = {e.selftest_lost.what, (int)e.selftest_lost.step, (int)e.selftest_lost.sequence / 32 * st->bwdtm.jt * 4};
     if (kind == Kind::Tmem && st->bwdtm.direct) FLSTM_TRY(lstm_backward_tm_direct(e.cfg.dtype, st->bwdtm, t.tm_w, p, s));
     else if (kind == Kind::Tmem) FLSTM_TRY(lstm_backward_tm(e.cfg.dtype, st->bwdtm, t.tm_w, t.dg_tm, p, s));
     else FLSTM_TRY(lstm_backward_persistent(e.cfg.dtype, st->bwd, t.tm_w, t.tm_dg, p, s));

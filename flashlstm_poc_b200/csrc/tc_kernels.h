@@ -38,6 +38,15 @@ struct FwdPlan {
     int grid;
 };
 
+// Self-test of the kernels without a step barrier: what CTA `cta` leaves out of step `step` of a launch (from 0).  The kernels have
+// forms of their own for it (fp16): in the others it took 1 to 2 % of a step.
+struct LostWords {
+    unsigned int what;
+    int step, cta;
+};
+// the first words of the pieces it sends (BPTT); all it sends; the count of its resets, from that step on
+constexpr unsigned int kLostWord = 1, kLostPart = 2, kLostCount = 4;
+
 struct FwdParams {
     float *cs;            // fp32 (T+1, B, H) cell states, slot 0 = c0
     void *hs;             // 16-bit (T+1, B, H) hidden states, slot 0 = h0
@@ -59,6 +68,7 @@ struct FwdParams {
     int trace_steps;
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path: the step barrier waits for this many arrivals nobody makes
+    LostWords lost;
     // filled by the launcher from the plan
     int rt, cta_rows, nt, stages, ch, halves;
     uint32_t idesc;
@@ -153,6 +163,7 @@ struct BwdParams {
     int s0, s1;           // reverse iterations [s0, s1) of this launch; iteration s is time T-1-s, s == T writes dh0/dc0
     unsigned long long wait_ns;   // limit of every device-side wait (0 = the 2 s default)
     unsigned int extra_arrivals;  // self-test of the timeout path (see FwdParams)
+    LostWords lost;
     int jt, nt, stages, ch, halves;
     uint32_t idesc;
 };

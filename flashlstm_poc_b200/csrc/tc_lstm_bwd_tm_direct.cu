@@ -56,7 +56,7 @@ __host__ __device__ inline Layout layout_of(const BwdTmPlan &pl) {
 // of the kernel that a plan takes: H = 1024 and 1536
 __host__ __device__ inline int kernel_rounds(const BwdTmPlan &pl) { return pl.kp + pl.left <= 8 ? 8 : 12; }
 
-template <int ROUNDS, bool BF16, bool ACCURATE>
+template <int ROUNDS, bool BF16, bool ACCURATE, bool LOST>  // LOST: the self-test's form (LostWords)
 __global__ void __launch_bounds__(kThreads, 1)
 lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ BwdTmPlan pl, BwdParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -182,7 +182,7 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // ------------------------------------------------------------ the launch's barrier, then fences behind resets
         if (steps > 1 && elect_one() && wait_counter(counter, (unsigned)(pl.jt * KS) + p.extra_arrivals, p.err, abort_w, 3u, wait_ns)) {
             mbar_arrive(ready);
-            perform_resets(reset, performed, steps, abort_w, wait_ns);
+            perform_resets(reset, performed, steps, abort_w, wait_ns, LOST && blockIdx.x == p.lost.cta && (p.lost.what & kLostCount) ? p.lost.step : -1);
         }
     } else if (warp == 17) {
         // ------------------------------------------------------------ UMMA issuer
@@ -294,6 +294,8 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         };
         fetch(p.s0);
         float dc = !valid ? 0.f : p.s0 > 0 ? p.dc[idx] : dcn ? load16<BF16>(dcn + idx) : 0.f;
+        const int lost_at = LOST && blockIdx.x == p.lost.cta && (p.lost.what & kLostPart) ? p.lost.step : -1;
+        const int torn_at = LOST && blockIdx.x == p.lost.cta && (p.lost.what & kLostWord) ? p.lost.step : -1;
         uint32_t wi = 0;  // steps contracted
         bool gathered = true;
         for (int s = p.s0; s < p.s1; ++s) {
@@ -388,7 +390,11 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const bool store = has_piece && valid, more = s + 1 < p.s1;
             const size_t slot = (size_t)(k & (kDirectSlots - 1)) * slot_bytes;
             if (more) {
-                if (store) st_relaxed_gpu_16(ring + slot + my_piece, piece);
+                if (store && !(LOST && k == lost_at)) {
+                    uint4 sent = piece;
+                    if (LOST && k == torn_at && (nb & 3)) sent.x = kUnwritten;  // (the others are looked at by this word: gather_unwritten_whole)
+                    st_relaxed_gpu_16(ring + slot + my_piece, sent);
+                }
                 g.mark_sent();
                 if (k == 0) gathered = mbar_wait(ready, 0, abort_w, wait_ns);  // every CTA of the group has reset its pieces
             }
@@ -433,9 +439,9 @@ void cluster_attr(cudaLaunchAttribute *a) {
     a->val.clusterDim.z = 1;
 }
 
-template <int ROUNDS, bool BF16, bool ACC>
+template <int ROUNDS, bool BF16, bool ACC, bool LOST = false>
 int launch_one(const CUtensorMap &tw, const BwdTmPlan &pl, const BwdParams &p, cudaStream_t s) {
-    auto kern = lstm_bwd_tm_kernel<ROUNDS, BF16, ACC>;
+    auto kern = lstm_bwd_tm_kernel<ROUNDS, BF16, ACC, LOST>;
     FLSTM_CUDA_TRY(ensure_smem_limit(reinterpret_cast<const void *>(kern), pl.smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid);
@@ -463,7 +469,7 @@ int launch_one(const CUtensorMap &tw, const BwdTmPlan &pl, const BwdParams &p, c
 // clusters of this plan that the current device holds at once, or -1
 template <int ROUNDS>
 int max_clusters(const BwdTmPlan &pl) {
-    auto kern = lstm_bwd_tm_kernel<ROUNDS, false, false>;
+    auto kern = lstm_bwd_tm_kernel<ROUNDS, false, false, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid);
     cfg.blockDim = dim3(kThreads);
@@ -501,6 +507,7 @@ int lstm_backward_tm_direct(int dtype, const BwdTmPlan &pl, const CUtensorMap &t
     const bool bf16 = dtype == FLSTM_DTYPE_BF16, acc = p.real_units > 0;
 #define FLSTM_TM_CASE(R_)                                                                                                      \
     if (kernel_rounds(pl) == R_) {                                                                                            \
+        if (p.lost.what && !bf16 && !acc) return launch_one<R_, false, false, true>(tw, pl, p, s);                              \
         if (bf16) return acc ? launch_one<R_, true, true>(tw, pl, p, s) : launch_one<R_, true, false>(tw, pl, p, s);           \
         return acc ? launch_one<R_, false, true>(tw, pl, p, s) : launch_one<R_, false, false>(tw, pl, p, s);                   \
     }

@@ -65,7 +65,7 @@ __host__ __device__ inline Layout layout_of(const FwdTmPlan &pl) {
     return l;
 }
 
-template <int ROUNDS, bool BF16, bool ACCURATE>
+template <int ROUNDS, bool BF16, bool ACCURATE, bool LOST>  // LOST: the self-test's form (LostWords)
 __global__ void __launch_bounds__(kThreads, 1)
 lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ FwdTmPlan pl,
                    FwdParams p) {
@@ -203,7 +203,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             // -------------------------------------------------------- the launch's barrier, then fences behind resets
             if (p.T > 1 && elect_one() && wait_counter(counter, (unsigned)pl.cta_rows + p.extra_arrivals, p.err, abort_w, 2u, wait_ns)) {
                 mbar_arrive(ready);
-                perform_resets(reset, performed, p.T, abort_w, wait_ns);
+                perform_resets(reset, performed, p.T, abort_w, wait_ns, LOST && blockIdx.x == p.lost.cta && (p.lost.what & kLostCount) ? p.lost.step : -1);
             }
         } else {
             // -------------------------------------------------------- UMMA issuer (the leader's)
@@ -289,6 +289,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             named_barrier_sync(2, kEpilogueThreads);
             if (tid == 0) red_release_gpu_add(counter, 1u);
         }
+        const int lost_at = LOST && blockIdx.x == p.lost.cta && (p.lost.what & kLostPart) ? p.lost.step : -1;
         float c_keep = valid ? p.cs[(size_t)p.t0 * slab + idx] : 0.f;
         bool gathered = true;
         for (int tt = 0; tt < p.T; ++tt) {
@@ -341,7 +342,7 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const bool word_valid = !odd && valid, more = tt + 1 < p.T;
             const size_t slot = (size_t)(tt & (kDirectSlots - 1)) * slot_bytes;
             if (more) {
-                if (word_valid) st_relaxed_gpu(ring + slot + my_word, word);
+                if (word_valid && !(LOST && tt == lost_at)) st_relaxed_gpu(ring + slot + my_word, word);
                 g.mark_sent();
                 if (tid == 0) FLSTM_STAMP(tt, 7);
                 if (tt == 0) gathered = mbar_wait(ready, 0, abort_w, wait_ns);  // every CTA of the group has reset its words
@@ -392,9 +393,9 @@ lstm_fwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (threadIdx.x == 0) leave_counters(p.counters, (int)gridDim.x / pl.cta_rows, p.exits);
 }
 
-template <int ROUNDS, bool BF16, bool ACC>
+template <int ROUNDS, bool BF16, bool ACC, bool LOST = false>
 int launch_one(const CUtensorMap &tw, const CUtensorMap &tg, const FwdTmPlan &pl, const FwdParams &p, cudaStream_t s) {
-    auto kern = lstm_fwd_tm_kernel<ROUNDS, BF16, ACC>;
+    auto kern = lstm_fwd_tm_kernel<ROUNDS, BF16, ACC, LOST>;
     FLSTM_CUDA_TRY(ensure_smem_limit(reinterpret_cast<const void *>(kern), pl.smem_bytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid);
@@ -432,6 +433,7 @@ int lstm_forward_tm_direct(int dtype, const FwdTmPlan &pl, const CUtensorMap &tw
     const bool bf16 = dtype == FLSTM_DTYPE_BF16, acc = p.real_units > 0;
 #define FLSTM_TM_CASE(R_)                                                                                        \
     if (kernel_rounds(pl) == R_) {                                                                              \
+        if (p.lost.what && !bf16 && !acc) return launch_one<R_, false, false, true>(tw, tg, pl, p, s);          \
         if (bf16) return acc ? launch_one<R_, true, true>(tw, tg, pl, p, s) : launch_one<R_, true, false>(tw, tg, pl, p, s); \
         return acc ? launch_one<R_, false, true>(tw, tg, pl, p, s) : launch_one<R_, false, false>(tw, tg, pl, p, s); \
     }

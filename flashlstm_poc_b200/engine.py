@@ -70,6 +70,12 @@ class Engine:
         out = {field: getattr(info, field) for field, _ in info._fields_}
         return dict(out, name=info.name.decode())
 
+    def exchanges_directly(self, steps: int, backward: bool = False) -> bool:
+        """Whether that kernel exchanges h_t / dG_t without a step barrier."""
+        direct = ctypes.c_int()
+        check(self.lib.flstm_engine_direct(self._h, int(backward), steps, ctypes.byref(direct)))
+        return bool(direct.value)
+
     def _stream(self) -> int:
         return torch._C._cuda_getCurrentRawStream(self._index)  # current_stream() makes a Stream object of it first
 
@@ -295,6 +301,11 @@ class Engine:
         CTA makes, so the second time step's wait runs out after the limit and the launch returns with the
         error word set (the next call raises TIMEOUT).  0 switches it off."""
         check(self.lib.flstm_engine_selftest_missing_arrivals(self._h, int(arrivals)))
+
+    def selftest_lost_words(self, what: int, step: int = 0, sequence: int = 0) -> None:
+        """The same for kernels without a step barrier: in step `step` of each following launch one CTA of the batch group
+        of sequence `sequence` sends nothing (2; 1: in the BPTT, parts), or stops counting its resets (4).  0 switches it off."""
+        check(self.lib.flstm_engine_selftest_lost_words(self._h, int(what), int(step), int(sequence)))
 
     def abort_comm(self) -> None:
         check(self.lib.flstm_engine_abort_comm(self._h))

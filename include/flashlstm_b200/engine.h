@@ -177,6 +177,8 @@ typedef struct {
     int weights_streamed;  /* W_hh, or a part of it, is read again in every step */
 } flstm_kernel_info;
 int flstm_engine_kernel(flstm_engine *engine, int backward, size_t steps, flstm_kernel_info *out);
+/* Whether in that kernel h_t / dG_t cross from CTA to CTA without a step barrier, as words that announce themselves. */
+int flstm_engine_direct(flstm_engine *engine, int backward, size_t steps, int *direct);
 
 /* Batch-sharded data parallelism: one engine per GPU/process.  flstm_comm_unique_id fills a
  * 128-byte id on rank 0 (send it to the other ranks by any means); every rank then calls
@@ -204,9 +206,14 @@ int flstm_engine_abort_comm(flstm_engine *engine);
  * wait on one another (flashlstm_v2/src/lstm_forward.cu:744-830 launches per step).
  * flstm_engine_selftest_missing_arrivals exercises that path without any fault: with arrivals = n > 0 every
  * step barrier of the following launches waits for n arrivals that no CTA makes, so the wait of the second
- * time step runs out after the limit.  Set a limit of a few milliseconds first; arrivals = 0 switches it off. */
+ * time step runs out after the limit.  Set a limit of a few milliseconds first; arrivals = 0 switches it off.
+ * (The kernels of flstm_engine_direct have one such barrier a launch, before the first result crosses.)
+ * flstm_engine_selftest_lost_words does the same for what those wait for instead: in step `step` of each following launch (from 0) one
+ * CTA of the batch group of sequence `sequence` leaves out what it sends (what = 2; 1: the BPTT's, parts of it), or from that step on does
+ * not count the resets of its slots (4).  what = 0 switches it off.  fp16 engines with hidden_size % 64 == 0 and input_size % 8 == 0. */
 int flstm_engine_set_wait_limit(flstm_engine *engine, unsigned long long limit_us);
 int flstm_engine_selftest_missing_arrivals(flstm_engine *engine, unsigned int arrivals);
+int flstm_engine_selftest_lost_words(flstm_engine *engine, unsigned int what, size_t step, size_t sequence);
 
 /* Per-phase device time of the last forward/backward pair in milliseconds (needs
  * flstm_engine_enable_timing(engine, 1); adds event records, no synchronisation).

@@ -4,7 +4,10 @@ The host asks the step barrier to wait for one arrival more than the CTAs of a b
 (flstm_engine_selftest_missing_arrivals) and shortens the limit of every device-side wait to a few
 milliseconds (flstm_engine_set_wait_limit).  The wait of the second time step then runs out: the kernel raises
 its error word, every role drains and the launch RETURNS; the host sees FLSTM_ERR_TIMEOUT, and the same engine
-then computes a normal step whose results are bit-identical to the ones it produced before."""
+then computes a normal step whose results are bit-identical to the ones it produced before.
+
+In the kernels without a step barrier the missing arrival is that of the launch's one barrier, ahead of the first result that crosses.
+Their waits from step to step run out on words that one CTA leaves out (flstm_engine_selftest_lost_words)."""
 import time
 
 import numpy as np
@@ -51,7 +54,7 @@ def test_step_barrier_timeout_returns_and_engine_recovers(dtype, backend, where)
     _time_out_and_recover(dtype, backend, where, shape, 4)
 
 
-def _time_out_and_recover(dtype, backend, where, shape, steps, kernel=None):
+def _time_out_and_recover(dtype, backend, where, shape, steps, kernel=None, lost=None):
     w = Workload("timeout", dtype, 1, *shape, steps, seed=11, state_std=0.1)
     inp = make_inputs(w)
     td = TORCH_DTYPES[dtype]
@@ -61,15 +64,21 @@ def _time_out_and_recover(dtype, backend, where, shape, steps, kernel=None):
     before = _step(eng, inp, dev, td)
     assert all(np.isfinite(a).all() for a in before) and np.abs(before[0]).max() <= 1.0  # every row of y was written
 
+    def ask(on):
+        if lost is None:
+            eng.selftest_missing_arrivals(int(on))
+        else:
+            eng.selftest_lost_words(*(lost if on else (0,)))
+
     eng.set_wait_limit(LIMIT_US)
     x, h0, c0, dy = (t.to(dev, td) for t in (inp.x, inp.h0, inp.c0, inp.dy))
     t_start = time.perf_counter()
     if where == "forward":
-        eng.selftest_missing_arrivals(1)
+        ask(True)
         eng.forward(x, h0, c0)          # enqueued; the kernel gives up at the barrier of the second step
     else:
         eng.forward(x, h0, c0)
-        eng.selftest_missing_arrivals(1)
+        ask(True)
         eng.backward(dy)
     with pytest.raises(FlashLstmError) as exc:
         eng.wait(20.0)                  # host watchdog: the launch has returned, the error word is set
@@ -78,7 +87,7 @@ def _time_out_and_recover(dtype, backend, where, shape, steps, kernel=None):
     assert waited < 5.0, f"the kernel took {waited:.2f} s to give up with a {LIMIT_US} us limit"
     torch.cuda.synchronize()            # the context is intact
 
-    eng.selftest_missing_arrivals(0)
+    ask(False)
     eng.set_wait_limit(0)
     after = _step(eng, inp, dev, td)
     eng.close()
@@ -129,3 +138,20 @@ def test_each_grid_wide_kernel_returns_and_recovers(dtype, where, shape, steps, 
     for name, value in switches.items():
         monkeypatch.setenv(name, value)
     _time_out_and_recover(dtype, "tc", where, shape, steps, kernel)
+
+
+@pytest.mark.parametrize("where,shape,lost", [
+    # I, H, B; what a CTA sends or its count of resets (2, 4), step, sequence: the first batch group and others, first steps, last ones and
+    # some behind the slots' first reuse
+    ("forward", (64, 1024, 64), (2, 14, 40)), ("forward", (64, 576, 96), (2, 0, 95)), ("forward", (64, 1536, 32), (2, 24, 30)),
+    ("forward", (64, 1024, 64), (4, 9, 3)), ("forward", (64, 2048, 31), (4, 0, 30)),
+    ("backward", (64, 1024, 64), (2, 14, 40)), ("backward", (64, 1088, 8), (2, 0, 7)), ("backward", (64, 1536, 32), (2, 24, 31)),
+    ("backward", (64, 576, 96), (4, 9, 70)),
+])
+def test_words_that_never_come_end_the_launch(where, shape, lost):
+    """The gathers of all CTAs of a batch group (the other groups go on to their end), and the wait for the resets of a CTA's own slots."""
+    steps = 26
+    eng = Engine("f16", 1, shape[2], shape[0], shape[1], steps, device=torch.device("cuda", 0))
+    assert eng.exchanges_directly(steps, backward=where == "backward")
+    eng.close()
+    _time_out_and_recover("f16", "tc", where, shape, steps, lost=lost)

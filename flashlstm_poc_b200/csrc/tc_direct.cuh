@@ -10,6 +10,14 @@
 // kUnwritten is no pair of 16-bit results: a conversion from fp32 gives NaN as 0x7fff.  Words are stored whole, so a word is
 // either unwritten or complete whatever becomes of the copies' order.
 //
+// What this takes for granted of the GPU, where PTX promises nothing (cp.async is a weak access, no acquire follows it):
+//   - an aligned 32-bit word of one store arrives whole in a copy (every word of a piece is looked at in the forward kernel);
+//   - a copy past L1 that starts after a reset has been fenced and its count has been seen, through whatever chain of words and
+//     barriers, does not bring the word from before the reset;
+//   - 16 aligned bytes of one 128-bit store arrive together: the BPTT looks at one word of four, as looking at all took 3 to 10 % of a step
+//     (H = 1088, B = 32 3.72 -> 3.82 us, H = 1024, B = 64 3.35 -> 3.66).  This one is watched: halves of an unwritten word are NaN in either
+//     type and make the sums they enter NaN, and where a sum is, the BPTT looks at all words of its operand (kErrTornPiece).
+//
 // Slots.  Results of step t go to slot t % 8.  After its stores of step t a thread resets its words of slot (t + 4) % 8: nobody reads
 // that slot any more (it held step t - 4; the results of step t - 1, which this CTA has seen from all others, were sent by CTAs
 // that had gathered step t - 2).  The reset has to be performed before anybody looks for step t + 4, that is before this CTA sends
@@ -91,7 +99,7 @@ __device__ __forceinline__ void gather_commit() { asm volatile("cp.async.commit_
 // all but the LEFT newest groups have landed
 template <int LEFT>
 __device__ __forceinline__ void gather_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
-// A piece that is written whole is looked at by one word: lanes 0-7 look at the first word of theirs, 8-15 at the second, ..., so
+// A piece that is written whole is looked at by one word (see above): lanes 0-7 look at the first word of theirs, 8-15 at the second, ..., so
 // that a warp reads every bank once (all four words take four times as long).
 __device__ __forceinline__ bool gather_unwritten_whole(uint32_t smem_addr) {
     uint32_t a;

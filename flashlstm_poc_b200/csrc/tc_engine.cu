@@ -355,7 +355,8 @@ static int check_async_error(Engine &e) {
         const unsigned int code = *st->err_host;
         *st->err_host = 0;
         cudaMemset(e.sync_words, 0, sizeof(unsigned int));
-        return set_error(FLSTM_ERR_TIMEOUT, "a bounded device-side wait expired in a persistent kernel (code %u)", code);
+        return set_error(FLSTM_ERR_TIMEOUT, code == kErrTornPiece ? "a piece of dG was read before all of it was written (code %u)"
+                                                                  : "a bounded device-side wait expired in a persistent kernel (code %u)", code);
     }
     return FLSTM_OK;
 }

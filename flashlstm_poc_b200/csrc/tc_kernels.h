@@ -47,6 +47,9 @@ struct LostWords {
 // the first words of the pieces it sends (BPTT); all it sends; the count of its resets, from that step on
 constexpr unsigned int kLostWord = 1, kLostPart = 2, kLostCount = 4;
 
+// error word: a piece of dG was read before all of it was written (1 to 3: waits that expired)
+constexpr unsigned int kErrTornPiece = 4;
+
 struct FwdParams {
     float *cs;            // fp32 (T+1, B, H) cell states, slot 0 = c0
     void *hs;             // 16-bit (T+1, B, H) hidden states, slot 0 = h0

@@ -56,6 +56,17 @@ __host__ __device__ inline Layout layout_of(const BwdTmPlan &pl) {
 // of the kernel that a plan takes: H = 1024 and 1536
 __host__ __device__ inline int kernel_rounds(const BwdTmPlan &pl) { return pl.kp + pl.left <= 8 ? 8 : 12; }
 
+// Whether the operand tile's row of a sequence holds a word that its CTA had not written yet: lane `part` of 16 looks at a sixteenth of
+// it, all words of each piece.
+__device__ __forceinline__ bool holds_unwritten(uint32_t row, int part, int kp, int left) {
+    const uint32_t mine = row + (part >> 3) * BT * 128 + (part & 7) * 16;
+    bool found = false;
+#pragma unroll 1
+    for (int c = 0; c < kp; ++c) found |= gather_unwritten(mine + (uint32_t)c * kRound);
+    if (left && part < 8) found |= gather_unwritten(mine + (uint32_t)kp * kRound);
+    return found;
+}
+
 template <int ROUNDS, bool BF16, bool ACCURATE, bool LOST>  // LOST: the self-test's form (LostWords)
 __global__ void __launch_bounds__(kThreads, 1)
 lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ BwdTmPlan pl, BwdParams p) {
@@ -355,6 +366,12 @@ lstm_bwd_tm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 const float *red = s_red + (size_t)rb * KS * UPO * kRowStride;
 #pragma unroll
                 for (int src = 0; src < KS; ++src) dh_in += red[(src * UPO + u16) * kRowStride + nb];
+                // A sum that is no number: a piece that came in part would give one (tc_direct.cuh)
+                if (dh_in != dh_in && k > 0 && good && holds_unwritten(smem_u32(s_tile) + nb * 128, u16, KP, pl.left)) {
+                    *abort_w = 1;
+                    atomicExch(p.err, kErrTornPiece);
+                    good = false;
+                }
                 // one warp's failure is everybody's
                 if (named_barrier_or(1, kEpilogueThreads, !good)) break;
                 if (tid == 0) FLSTM_STAMP(k, 6);

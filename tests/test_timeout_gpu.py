@@ -93,6 +93,7 @@ def _time_out_and_recover(dtype, backend, where, shape, steps, kernel=None, lost
     eng.close()
     for a, b in zip(before, after):
         assert np.array_equal(a, b)
+    return str(exc.value)
 
 
 @pytest.mark.parametrize("dtype,backend,where", [
@@ -155,3 +156,10 @@ def test_words_that_never_come_end_the_launch(where, shape, lost):
     assert eng.exchanges_directly(steps, backward=where == "backward")
     eng.close()
     _time_out_and_recover("f16", "tc", where, shape, steps, lost=lost)
+
+
+@pytest.mark.parametrize("I,H,B,step,sequence", [(64, 1024, 64, 14, 40), (64, 1088, 8, 0, 7), (64, 1536, 32, 24, 31), (64, 576, 96, 9, 70)])
+def test_a_piece_read_in_part_ends_the_launch(I, H, B, step, sequence):
+    """The BPTT looks at one word of a 16-byte piece: one that came without another of its words would be taken for whole."""
+    message = _time_out_and_recover("f16", "tc", "backward", (I, H, B), 26, lost=(1, step, sequence))
+    assert "before all of it was written" in message

@@ -20,11 +20,40 @@ def engine(dtype, B, H, T, training=True):
     return eng, [t if t is None else t.to(DEV, TORCH_DTYPES[dtype]) for t in (inp.x, inp.h0, inp.c0, inp.dy)]
 
 
-# one batch group of 32 and of 64, an odd number of 64-wide chunks of K, a partly filled tile
-SHAPES = [("f16", 32, 1024), ("bf16", 5, 1088), ("bf16", 70, 1088), ("f16", 64, 2048), ("bf16", 31, 2048)]
+# One batch group, an odd number of 64-wide chunks of K, partly filled tiles, the neighbouring form with a counter (tiles of 64, and a BPTT
+# too wide); then two and three groups on one ring, the last of them partly filled.
+SHAPES = [("f16", 32, 1024), ("bf16", 5, 1088), ("bf16", 70, 1088), ("f16", 64, 2048), ("bf16", 31, 2048),
+          ("f16", 64, 1024), ("bf16", 41, 1024), ("bf16", 96, 576)]
+# the widest: its training is not on the tensor cores
+FORWARD_SHAPES = SHAPES + [("bf16", 31, 2304)]
 
 
-@pytest.mark.parametrize("dtype,B,H", SHAPES)
+@pytest.mark.parametrize("B,H,forward,backward,groups", [(32, 1024, True, True, 1), (5, 1088, True, True, 1), (70, 1088, False, False, None),
+                                                         (64, 2048, False, False, None), (31, 2048, True, False, 1), (64, 1024, True, True, 2),
+                                                         (41, 1024, True, True, 2), (96, 576, True, True, 3), (31, 2304, True, None, 1)])
+def test_which_kernels_the_shapes_here_run(B, H, forward, backward, groups):
+    eng = Engine("bf16", 1, B, 64, H, 26, training=backward is not None, device=DEV)
+    assert eng.exchanges_directly(26) == forward
+    if groups:
+        assert eng.recurrent_kernel(26)["batch_groups"] == groups
+    if backward is not None:
+        assert eng.exchanges_directly(26, backward=True) == backward
+        assert not eng.exchanges_directly(1) or H % 128  # short launches, where there is another kernel for them
+    eng.close()
+
+
+@pytest.mark.parametrize("dtype,B,H,training", [("f16", 64, 1024, True), ("bf16", 41, 1024, True), ("bf16", 96, 576, True), ("f16", 20, 1408, True),
+                                                ("bf16", 31, 2304, False), ("f16", 7, 2368, False)])
+def test_slots_used_three_times_match_the_oracle(dtype, B, H, training):
+    w = Workload("t", dtype, 1, 40, H, B, 26, seed=93, state_std=0.3, training=training)
+    inp = make_inputs(w)
+    got, eng = run_engine(w, inp, repeat=2)
+    assert eng.exchanges_directly(26) and (not training or eng.exchanges_directly(26, backward=True))
+    eng.close()
+    assert_parity(got, run_oracle(inp), dtype)
+
+
+@pytest.mark.parametrize("dtype,B,H", FORWARD_SHAPES)
 def test_sequences_that_are_no_numbers_stay_their_own(dtype, B, H):
     """From a step with an infinite and a NaN input on, one sequence's h is NaN, of either sign; it crosses like any other value and
     reaches no other sequence, whose results stay the same bit for bit."""
@@ -46,7 +75,7 @@ def test_sequences_that_are_no_numbers_stay_their_own(dtype, B, H):
     eng.close()
 
 
-@pytest.mark.parametrize("dtype,B,H", SHAPES)
+@pytest.mark.parametrize("dtype,B,H", FORWARD_SHAPES)
 def test_y_may_start_at_any_element(dtype, B, H):
     T = 14
     eng, (x, h0, c0, _) = engine(dtype, B, H, T, training=False)

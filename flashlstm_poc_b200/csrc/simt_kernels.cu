@@ -404,8 +404,10 @@ column_sum_partial_wide_kernel(const T *__restrict__ dg, size_t R, size_t N, int
 template <typename T>
 void column_sum_partial(const T *dg, size_t R, size_t N, int splits, float *partial, cudaStream_t s) {
     if constexpr (sizeof(T) == 2) {
-        // columns in whole groups of 16 bytes, and so many of them and rows that there are blocks enough all the same (210800 x 512:
-        // 94 us by the other way, 173 by this one); 4-byte loads fill the memory's bandwidth as they are (32768 x 4096: 85 us, 113)
+        // Columns in whole groups of 16 bytes, and so many of them that there are blocks enough all the same (210800 x 512: 94 us by the
+        // other way, 173 by this one); 4-byte loads fill the memory's bandwidth as they are (32768 x 4096: 85 us, 113).  The line at 5120
+        // rows is not where the times cross: fewer rows gain too (from memory: 1024 x 4096 8.2 us by the other way, 5.4 by this one,
+        // 4096 x 2048 8.7 / 7.0, 4096 x 4096 14.5 / 9.2), but had not been measured when it was drawn.
         if (R >= 5120 && N >= 2048 && N % 8 == 0 && (reinterpret_cast<uintptr_t>(dg) & 15) == 0) {
             column_sum_partial_wide_kernel<<<dim3(ceil_div(N, 256), splits), 256, 0, s>>>(dg, R, N, splits, partial);
             return;

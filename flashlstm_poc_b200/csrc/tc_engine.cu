@@ -180,15 +180,26 @@ bool supported(const flstm_engine_config &cfg) {
 // keep short launches.  Those then sum the halves of K apart, so that a sequence cut into ranges or segments of any length
 // gives the bits of one launch.  Calls of n steps in us, other kernels -> these:
 //   forward, n = 1 / 2 / 4 / 8 / 16 / 24:
-//     H = 1024, B = 32, one tile of 32   23.7 / 26.7 / 33.5 / 47.2 / 76.9 / 107.8 -> 24.7 / 28.8 / 34.9 / 42.6 / 61.9 / 83.4
-//     H = 2048, B = 40, one tile of 64   26.5 / 30.8 / 45.2 / 70.8 / 123.1 / 168.3 -> 28.8 / 32.9 / 45.6 / 71.8 / 121.7 / 164.4
+//     without a step barrier
+//     H = 1024, B = 32   23.5 / 25.7 / 33.3 / 47.2 / 73.8 / 102.5 -> 23.6 / 27.7 / 32.9 / 43.0 / 62.1 / 83.2
+//     H = 1024, B = 64   23.6 / 26.5 / 34.9 / 48.3 / 77.9 / 107.3 -> 23.6 / 28.6 / 33.8 / 43.7 / 65.4 / 87.1
+//     H = 1152, B = 20   23.6 / 25.7 / 33.9 / 48.3 / 75.8 / 103.1 -> 23.6 / 27.7 / 31.9 / 43.1 / 63.5 / 84.1
+//     H = 2048, B = 32   24.6 / 30.8 / 40.7 / 59.7 / 102.2 / 143.8 -> 27.8 / 30.8 / 36.9 / 51.2 / 78.2 / 107.9
+//     with one
+//     H = 2048, B = 40, one tile of 64   26.7 / 31.4 / 43.1 / 67.6 / 115.0 / 160.9 -> 28.7 / 32.8 / 44.2 / 67.6 / 112.5 / 154.1
 //     H = 2048, B = 256, tiles in turn   35.9 / 53.2 / 84.6 / 154 / 282 / 404 -> 37.2 / 48.7 / 71.9 / 125 / 214 / 297
 //   backward, n = 1 / 2 / 4 / 8 / 16:
-//     H = 1024, B = 32   56.5 / 60.9 / 70.2 / 91.6 / 127.1 -> 59.3 / 63.4 / 71.7 / 92.9 / 113.5
-//     H = 1024, B = 64   57.3 / 61.6 / 74.6 / 95.1 / 137.0 -> 59.3 / 63.5 / 77.0 / 95.2 / 136.3
-//     H = 2048, B = 5    104.4 / 107.5 / 121.4 / 146.0 / 196.5 -> 107.4 / 111.1 / 120.6 / 141.2 / 182.5
-//     H = 1280, B = 60   76.4 / 85.1 / 98.5 / 130.9 / 187.5 -> 78.2 / 87.1 / 98.1 / 126.8 / 179.0
+//     without a step barrier
+//     H = 896, B = 60    61.2 / 64.1 / 77.2 / 96.1 / 131.4 -> 63.3 / 66.5 / 76.9 / 90.7 / 119.3
+//     H = 1024, B = 32   56.3 / 62.0 / 70.1 / 90.8 / 127.0 -> 59.3 / 62.3 / 70.1 / 86.5 / 113.0
+//     H = 1024, B = 64   60.2 / 64.1 / 76.3 / 96.7 / 139.2 -> 62.5 / 65.2 / 76.3 / 91.3 / 124.8
+//     H = 1280, B = 32   73.3 / 77.6 / 88.0 / 111.7 / 153.7 -> 76.5 / 80.1 / 87.8 / 105.6 / 138.6
+//     with one
+//     H = 1280, B = 60   73.2 / 81.9 / 95.3 / 127.0 / 184.2 -> 75.3 / 83.8 / 94.7 / 123.0 / 172.6
+//     H = 2048, B = 5    103.1 / 106.2 / 120.3 / 144.7 / 196.4 -> 104.1 / 107.5 / 117.6 / 139.3 / 180.2
 //     tiles in turn, H = 1024, B = 140   70.7 / 81.5 / 104 / 149 / 238 -> 68.0 / 77.0 / 92.3 / 123 / 182
+// The lines below were drawn for the kernels with a step barrier.  Without one the times cross at 3 to 4 steps in either direction:
+// launches of 4 steps forward and of 5 to 11 backward (H <= 1024) take 1 to 7 % longer than they would on these kernels.
 static int choose_tmem(int B, int H, bool fwd, bool bwd, int sms, size_t smem_limit, bool check_device, TcState *st) {
     const bool good = H % 128 == 0;
     if (fwd) {

@@ -424,7 +424,8 @@ step_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             bool ok = true;
             for (int tile = worker; tile < tiles && ok; tile += workers, ++it) {
                 const int tbuf = it & 1;
-                if (!mbar_wait(&tfull[tbuf], (it >> 1) & 1, abort_w)) break;
+                // the lanes of a warp agree about every wait: reading the accumulator takes all of them
+                if (!__all_sync(0xffffffffu, mbar_wait(&tfull[tbuf], (it >> 1) & 1, abort_w))) break;
                 tcgen05_fence_after();
                 const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + tbuf * BN;
 #pragma unroll 1
@@ -447,7 +448,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                         if (lane == 0) release_accumulator(tbuf);
                     }
                     if (row0 >= a.M) continue;
-                    ok = mbar_wait(&ldbar[buf], (ldphase >> buf) & 1u, abort_w);
+                    ok = __all_sync(0xffffffffu, mbar_wait(&ldbar[buf], (ldphase >> buf) & 1u, abort_w));
                     if (!ok) break;
                     ldphase ^= 1u << buf;
                     uint8_t *sP = wb + buf * kEpiPBytes, *sC = wb + 2 * kEpiPBytes + buf * kEpiCBytes;
@@ -470,7 +471,7 @@ step_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 const int buf = it & 1;
                 const int ks = tile / (num_m * num_n), mn = tile % (num_m * num_n);
                 const int m0 = (mn / num_n) * BMT + (int)rank * BM, n0 = (mn % num_n) * BN;
-                if (!mbar_wait(&tfull[buf], (it >> 1) & 1, abort_w)) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(&tfull[buf], (it >> 1) & 1, abort_w))) break;
                 tcgen05_fence_after();
                 const int row = m0 + q * 32 + lane;  // sequence index
                 const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN;
